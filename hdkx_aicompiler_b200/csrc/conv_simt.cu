@@ -60,132 +60,284 @@ __global__ void __launch_bounds__(kThreads) conv2d_direct_kernel(const TIn* __re
     }
 }
 
-// Register-tiled fp32 form of the same reduction: a block of 128 threads computes 64 output channels x kPT * 2 * kOT
-// consecutive output pixels (flattened over n, oh, ow), a thread kOT channels x kPT pixels. Every output element is still
-// ONE sequential chain acc = acc + x * w over rc, rh, rw with separately rounded multiply and add, so the bits are those
-// of the one-thread-per-output kernel above; only the number of loads per multiply changes (an input value serves kOT
-// channels, a weight kPT pixels). Weights of `rc_block` input channels at a time are staged in shared memory as
-// [rc][tap][64 channels], so a thread's weights are one or two 16-byte broadcast loads. kKW: the filter width at compile time (1, 3, 7) so that a filter row's loads are all
-// issued before its arithmetic; 0 = any.
-constexpr int kTileO = 64, kTileThreads = 128;
+// Register-tiled fp32 form of the same reduction, on packed pairs. A block computes kTO*kOG output channels x kTP*kPG
+// consecutive output pixels (flattened over n, oh, ow), a thread kTO x kTP of them. Every output element is still ONE
+// sequential chain acc = acc + x * w over rc, rh, rw with separately rounded multiply and add, so the bits are those of the
+// one-thread-per-output kernel above.
+//
+// What bounds it: the FMA pipe. Two roundings per term are two instructions, and a scalar multiply + add pair reaches only
+// 88 of the 128 lanes per clock of an SM (three register operands each, in a pure register loop); the packed f32x2 forms
+// reach 125, i.e. 62.5 terms per clock and SM = 36.4 TFLOP/s at 1.965 GHz, and leave half of the issue slots to the loads.
+// ptxas fuses mul.rn.f32x2 + add.rn.f32x2 into one fused multiply-add, which rounds once and changes the bits. The product
+// is therefore formed as fma(x, w, -0) with a -0 that is a kernel argument (fma(x, w, -0) is the rounded product for every
+// x and w, the signs of zeros included), which nothing can fold.
+// Measured, 128 -> 128 channels 3x3 at 28x28 and 32 images: 646 us with scalar arithmetic, 279 us = 26.6 TFLOP/s now (0.73 of
+// the packed bound; 2.65 blocks for each SM cost 12 % of it); ResNet-18 at 32 images 11.3 -> 4.6 ms. Weights doubled in
+// shared memory to spare the register moves, unrolling two stages and rolling the k loop up were slower.
+//
+// Half of the warps compute, the other half feed them: the im2col values of KC consecutive k = (rc, rh, rw) by 4-byte
+// cp.async (zeros outside the image and past the last k: acc + 0 is the identity, acc is never -0) and the weights through
+// registers, into a ring of kExactBufs shared-memory stages handed over with named barriers. With the same warps doing both, the
+// gather's dependent address arithmetic held up the FMA pipe (175 clocks per k where the arithmetic alone takes 140 with
+// one warp on a scheduler); as separate warps it runs in the issue slots that the packed instructions leave. A stage is
+// whole filter rows (four of 3 taps, two of 7, sixteen of 1), so that a row's pointer and bounds are found once and a tap
+// costs a bit test and the copy; other widths find every tap in a table.
+constexpr int kExactBufs = 3;
+constexpr int kExactMaxTaps = 64; // the table's size
 
-template <int kKW, int kOT, int kPT, typename Epilogue>
-__global__ void __launch_bounds__(kTileThreads) conv2d_tiled_f32_kernel(const float* __restrict__ data, const float* __restrict__ weight,
-                                                                        ConvDims d, int rc_block, Epilogue epi) {
-    static_assert(kOT == 4 || kOT == 8, "one or two float4 of weights per thread");
-    constexpr int kOG = kTileO / kOT;            // channel groups of a block
-    constexpr int kPG = kTileThreads / kOG;      // pixel groups of a block
-    constexpr int kTileP = kPG * kPT;
-    extern __shared__ __align__(16) float w_s[];  // [rc_block][KH*KW][kTileO]
-    const int KW = kKW > 0 ? kKW : d.KW;
-    const int taps = d.KH * KW;
-    const int plane_out = d.OH * d.OW;
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t mac2_exact(uint64_t acc, uint64_t x, uint64_t w, uint64_t neg_zero) {
+    uint64_t prod, sum;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(prod) : "l"(x), "l"(w), "l"(neg_zero));
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(sum) : "l"(acc), "l"(prod));
+    return sum;
+}
+// 4 bytes to shared memory: the value at src, or zero where !valid (src is not read then); nothing where !active
+__device__ __forceinline__ void cp_async4_zfill(uint32_t dst, const float* src, uint32_t valid, bool active) {
+    asm volatile(
+        "{\n\t.reg .pred ignore, act;\n\tsetp.eq.u32 ignore, %2, 0;\n\tsetp.ne.u32 act, %3, 0;\n\t"
+        "@act cp.async.ca.shared.global [%0], [%1], 4, ignore;\n\t}" ::"r"(dst), "l"(src), "r"(valid), "r"((uint32_t)active));
+}
+
+__device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void named_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+template <int kTO, int kTP, int kOG, int kPG>
+struct ExactTile {
+    static constexpr int kThreads = kOG * kPG;  // of each role
+    static constexpr int kO = kTO * kOG;
+    static constexpr int kP = kTP * kPG;
+};
+
+// kKW: the filter width at compile time (1, 3, 7; horizontal dilation 1), 0 = any
+template <int kKW, int kMul>
+struct ExactStage {
+    static constexpr int kRows = kMul * (kKW == 7 ? 2 : kKW == 3 ? 4 : 16);  // filter rows of a stage (kKW = 0: taps)
+    static constexpr int kK = kRows * (kKW > 0 ? kKW : 1);
+    static constexpr int kVec = kK % 4 == 0 ? 4 : 2;                 // weights of one global load
+};
+
+template <int kKW, int kTO, int kTP, int kOG, int kPG, int kMul, int kMinBlocks, typename Epilogue>
+__global__ void __launch_bounds__(2 * kOG * kPG, kMinBlocks)
+    conv2d_tiled_f32_kernel(const float* __restrict__ data, const float* __restrict__ weight, ConvDims d, float neg_zero_arg,
+                            Epilogue epi) {
+    using Tile = ExactTile<kTO, kTP, kOG, kPG>;
+    using Stage = ExactStage<kKW, kMul>;
+    constexpr int kT = Tile::kThreads, kTileO = Tile::kO, kTileP = Tile::kP, KC = Stage::kK, kVec = Stage::kVec;
+    // threads that share the gather of one pixel, and the filter rows each takes of a stage
+    constexpr int kShare = kT / kTileP > 1 ? kT / kTileP : 1;
+    constexpr int kSub = kShare < Stage::kRows ? kShare : Stage::kRows;
+    constexpr int kRowsPer = Stage::kRows / kSub;
+    constexpr int kWQ = kTileO * (KC / kVec);  // weight loads of a stage
+    constexpr int kWPer = (kWQ + kT - 1) / kT;
+    static_assert(kTO % 2 == 0 && kTP % 2 == 0 && kTileP <= kT && Stage::kRows % kSub == 0, "tile shape");
+    __shared__ __align__(16) float xs[kExactBufs][KC][kTileP];
+    __shared__ __align__(16) float ws[kExactBufs][KC][kTileO];
+    __shared__ int tap_off[kKW > 0 ? 1 : kExactMaxTaps];
+
+    const int K = d.C * d.KH * d.KW;
+    const int stages = (K + KC - 1) / KC;
+    const int plane_in = d.H * d.W, plane_out = d.OH * d.OW;
     const int64_t P = (int64_t)d.N * plane_out;
     const int o0 = blockIdx.y * kTileO;
     const int64_t p0 = (int64_t)blockIdx.x * kTileP;
-    const int pg = threadIdx.x % kPG;   // pixels p0 + pg + kPG e: consecutive lanes read consecutive pixels
-    const int og = threadIdx.x / kPG;   // channels o0 + kOT og ..
-    int ih0[kPT], iw0[kPT];
-    bool pix_ok[kPT];
-    const float* xn[kPT];
-#pragma unroll
-    for (int e = 0; e < kPT; ++e) {
-        const int64_t p = p0 + pg + kPG * e;
-        pix_ok[e] = p < P;
-        const int n = pix_ok[e] ? (int)(p / plane_out) : 0;
-        const int rem = pix_ok[e] ? (int)(p - (int64_t)n * plane_out) : 0;
-        const int oh = rem / d.OW, ow = rem - oh * d.OW;
-        ih0[e] = oh * d.SH - d.PH;
-        iw0[e] = ow * d.SW - d.PW;
-        xn[e] = data + (int64_t)n * d.C * d.H * d.W;
-    }
-    float acc[kOT][kPT];
-#pragma unroll
-    for (int j = 0; j < kOT; ++j)
-#pragma unroll
-        for (int e = 0; e < kPT; ++e) acc[j][e] = 0.0f;
-    const int64_t plane_in = (int64_t)d.H * d.W;
-    // 16-byte weight loads need every block's run to start on a 16-byte boundary
-    const bool w_vec = ((reinterpret_cast<uintptr_t>(weight) & 15u) == 0) && (((int64_t)d.C * taps) & 3) == 0 && ((rc_block * taps) & 3) == 0;
-    for (int c0 = 0; c0 < d.C; c0 += rc_block) {
-        const int nrc = (d.C - c0) < rc_block ? (d.C - c0) : rc_block;
-        __syncthreads();  // the previous block of weights has been used
-        // A channel's nrc * taps weights of this block are contiguous in the OIHW tensor. Consecutive threads take
-        // consecutive channels (distinct shared-memory banks) and 16 bytes each where the run allows it: with 4-byte
-        // loads every value costs a 32-byte sector of its own, which made the 512-channel layers weight-bound.
-        const int run = nrc * taps;
-        if (w_vec && (run & 3) == 0) {
-            for (int i = threadIdx.x; i < (run >> 2) * kTileO; i += kTileThreads) {
-                const int o = i % kTileO, jq = i / kTileO;
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (o0 + o < d.O) v = __ldg(reinterpret_cast<const float4*>(weight + ((int64_t)(o0 + o) * d.C + c0) * taps) + jq);
-                float* dst = w_s + (4 * jq) * kTileO + o;
-                dst[0] = v.x; dst[kTileO] = v.y; dst[2 * kTileO] = v.z; dst[3 * kTileO] = v.w;
-            }
-        } else {
-            for (int i = threadIdx.x; i < run * kTileO; i += kTileThreads) {
-                const int o = i % kTileO, j = i / kTileO;
-                w_s[i] = (o0 + o < d.O) ? __ldg(weight + ((int64_t)(o0 + o) * d.C + c0) * taps + j) : 0.0f;
-            }
-        }
+    const int tid = threadIdx.x % kT;
+    if (kKW == 0) {
+        for (int t = threadIdx.x; t < d.KH * d.KW; t += 2 * kT) tap_off[t] = (t / d.KW) * d.DH * d.W + (t % d.KW) * d.DW;
         __syncthreads();
-        for (int rc = 0; rc < nrc; ++rc) {
-            const float* wr = w_s + (rc * taps) * kTileO + og * kOT;
-            for (int rh = 0; rh < d.KH; ++rh) {
-                const float* row[kPT];
-                bool row_ok[kPT];
-#pragma unroll
-                for (int e = 0; e < kPT; ++e) {
-                    const int ih = ih0[e] + rh * d.DH;
-                    row_ok[e] = pix_ok[e] && ih >= 0 && ih < d.H;
-                    row[e] = xn[e] + (int64_t)(c0 + rc) * plane_in + (int64_t)(row_ok[e] ? ih : 0) * d.W;
-                }
-#pragma unroll
-                for (int rw = 0; rw < KW; ++rw) {
-                    float x[kPT];
-#pragma unroll
-                    for (int e = 0; e < kPT; ++e) {
-                        const int iw = iw0[e] + rw * d.DW;
-                        x[e] = (row_ok[e] && iw >= 0 && iw < d.W) ? __ldg(row[e] + iw) : 0.0f;
+    }
+    if (threadIdx.x >= kT) {
+    // gather role: pixel gp, kRowsPer consecutive filter rows (kKW = 0: taps) of every stage
+    const int gp = tid % kTileP, gsub = tid / kTileP;
+    const bool gather = kSub * kTileP == kT || gsub < kSub;
+    const int period = kKW > 0 ? d.KH : d.KH * d.KW;  // rows (taps) of one input channel
+    uint64_t inside = 0;                       // kKW = 0: taps inside the image; else filter columns inside it
+    int ih0 = -0x40000000;                     // no row of it is inside
+    const float* src = data;                   // the next row's first input (kKW = 0: the channel's plane at the first tap)
+    {
+        const int64_t p = p0 + gp;
+        if (gather && p < P) {
+            const int n = (int)(p / plane_out);
+            const int rem = (int)(p - (int64_t)n * plane_out);
+            const int oh = rem / d.OW, ow = rem - oh * d.OW;
+            const int iw0 = ow * d.SW - d.PW;
+            ih0 = oh * d.SH - d.PH;
+            src = data + (int64_t)n * d.C * plane_in + (int64_t)ih0 * d.W + iw0;
+            if (kKW > 0) {
+                for (int rw = 0; rw < kKW; ++rw)
+                    if (iw0 + rw >= 0 && iw0 + rw < d.W) inside |= 1ull << rw;
+            } else {
+                for (int rh = 0, t = 0; rh < d.KH; ++rh)
+                    for (int rw = 0; rw < d.KW; ++rw, ++t) {
+                        const int ih = ih0 + rh * d.DH, iw = iw0 + rw * d.DW;
+                        if (ih >= 0 && ih < d.H && iw >= 0 && iw < d.W) inside |= 1ull << t;
                     }
-                    float w[kOT];
-#pragma unroll
-                    for (int v = 0; v < kOT / 4; ++v) {
-                        const float4 wv = *reinterpret_cast<const float4*>(wr + (rh * KW + rw) * kTileO + 4 * v);
-                        w[4 * v] = wv.x; w[4 * v + 1] = wv.y; w[4 * v + 2] = wv.z; w[4 * v + 3] = wv.w;
-                    }
-#pragma unroll
-                    for (int j = 0; j < kOT; ++j)
-#pragma unroll
-                        for (int e = 0; e < kPT; ++e) acc[j][e] = __fadd_rn(acc[j][e], __fmul_rn(x[e], w[j]));
-                }
             }
         }
     }
-#pragma unroll
-    for (int e = 0; e < kPT; ++e) {
-        const int64_t p = p0 + pg + kPG * e;
-        if (p >= P) continue;
-        const int64_t n = p / plane_out, rem = p - n * plane_out;
-#pragma unroll
-        for (int j = 0; j < kOT; ++j) {
-            const int o = o0 + og * kOT + j;
-            if (o < d.O) epi(acc[j][e], (n * d.O + o) * plane_out + rem, o);
+    const int row_step = kKW > 0 ? d.DH * d.W : 0;                      // to the next row of the same channel
+    const int64_t wrap_step = (int64_t)plane_in - (int64_t)(period - 1) * row_step;  // from its last row to the next channel
+    int left = d.C * period;                                          // rows up to the end of K
+    int gt = 0, ih = ih0;
+    auto advance = [&](int rows) {  // a few rows ahead
+        const int c = rows / period, t = rows - c * period;
+        src += (int64_t)c * plane_in + (int64_t)t * row_step;
+        gt += t;
+        left -= rows;
+        if (gt >= period) {
+            gt -= period;
+            src += wrap_step - row_step;
         }
-    }
-}
+        ih = ih0 + gt * d.DH;
+    };
+    if (kSub > 1) advance(gsub * kRowsPer);
+    const uint32_t gdst0 = (uint32_t)__cvta_generic_to_shared(&xs[0][gsub * kRowsPer * (kKW > 0 ? kKW : 1)][gp]);
 
-template <int kOT, int kPT, typename Epilogue>
-void launch_tiled_f32(const float* data, const float* weight, const ConvDims& d, int rc_block, const Epilogue& epi, cudaStream_t s) {
-    constexpr int kTileP = (kTileThreads / (kTileO / kOT)) * kPT;
-    const int64_t P = (int64_t)d.N * d.OH * d.OW;
-    const dim3 grid((unsigned)((P + kTileP - 1) / kTileP), (unsigned)((d.O + kTileO - 1) / kTileO), 1u);
-    const size_t smem = (size_t)rc_block * d.KH * d.KW * kTileO * sizeof(float);
-    switch (d.KW) {
-        case 1: conv2d_tiled_f32_kernel<1, kOT, kPT, Epilogue><<<grid, kTileThreads, smem, s>>>(data, weight, d, rc_block, epi); break;
-        case 3: conv2d_tiled_f32_kernel<3, kOT, kPT, Epilogue><<<grid, kTileThreads, smem, s>>>(data, weight, d, rc_block, epi); break;
-        case 7: conv2d_tiled_f32_kernel<7, kOT, kPT, Epilogue><<<grid, kTileThreads, smem, s>>>(data, weight, d, rc_block, epi); break;
-        default: conv2d_tiled_f32_kernel<0, kOT, kPT, Epilogue><<<grid, kTileThreads, smem, s>>>(data, weight, d, rc_block, epi); break;
+    // row i (of kRowsPer) of the next stage into buffer `buf`; afterwards the state stands at the following row
+    auto gather_row = [&](int buf, int i) {
+        const uint32_t dst = gdst0 + (uint32_t)((buf * KC + i * (kKW > 0 ? kKW : 1)) * kTileP * 4);
+        if constexpr (kKW > 0) {
+            const uint32_t cols = ((unsigned)ih < (unsigned)d.H && left > 0) ? (uint32_t)inside : 0u;
+#pragma unroll
+            for (int rw = 0; rw < kKW; ++rw) cp_async4_zfill(dst + rw * kTileP * 4, src + rw, cols & (1u << rw), gather);
+        } else {
+            cp_async4_zfill(dst, src + tap_off[gt], left > 0 ? (uint32_t)(inside >> gt) & 1u : 0u, gather);
+        }
+        const bool wrap = ++gt == period;
+        gt = wrap ? 0 : gt;
+        ih = wrap ? ih0 : ih + d.DH;
+        src += wrap ? wrap_step : (int64_t)row_step;
+        --left;
+        if (kSub > 1 && i == kRowsPer - 1) advance(Stage::kRows - kRowsPer);
+    };
+    // weight role: up to kWPer loads of kVec consecutive k of one channel; consecutive threads take consecutive channels
+    const bool w_vec = K % kVec == 0 && (reinterpret_cast<uintptr_t>(weight) & (kVec * 4 - 1)) == 0;
+    float wreg[kWPer][kVec];
+    auto load_weights = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < kWPer; ++i) {
+            const int q = tid + i * kT;
+            const int o = o0 + q % kTileO, k = k0 + (q / kTileO) * kVec;
+#pragma unroll
+            for (int v = 0; v < kVec; ++v) wreg[i][v] = 0.0f;
+            if (o < d.O && k < K && (kWQ % kT == 0 || q < kWQ)) {
+                const float* src = weight + (int64_t)o * K + k;
+                if (w_vec && kVec == 4) {
+                    const float4 v = __ldg(reinterpret_cast<const float4*>(src));
+                    wreg[i][0] = v.x; wreg[i][1] = v.y; wreg[i][kVec - 2] = v.z; wreg[i][kVec - 1] = v.w;
+                } else if (w_vec) {
+                    const float2 v = __ldg(reinterpret_cast<const float2*>(src));
+                    wreg[i][0] = v.x; wreg[i][1] = v.y;
+                } else {
+#pragma unroll
+                    for (int v = 0; v < kVec; ++v)
+                        if (k + v < K) wreg[i][v] = __ldg(src + v);
+                }
+            }
+        }
+    };
+    auto store_weights = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < kWPer; ++i) {
+            const int q = tid + i * kT;
+            if (kWQ % kT != 0 && q >= kWQ) break;
+            float* dst = &ws[buf][(q / kTileO) * kVec][q % kTileO];
+#pragma unroll
+            for (int v = 0; v < kVec; ++v) dst[v * kTileO] = wreg[i][v];
+        }
+    };
+
+        load_weights(0);
+        int buf = 0;
+        for (int s = 0; s < stages; ++s) {
+            if (s >= kExactBufs) named_sync(1 + kExactBufs + buf, 2 * kT);  // the stage three back has been read
+#pragma unroll
+            for (int i = 0; i < kRowsPer; ++i) gather_row(buf, i);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            store_weights(buf);
+            load_weights((s + 1) * KC);
+            if (s > 0) {  // the previous stage has landed
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+                named_arrive(1 + (buf == 0 ? kExactBufs - 1 : buf - 1), 2 * kT);
+            }
+            buf = buf + 1 == kExactBufs ? 0 : buf + 1;
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        named_arrive(1 + (buf == 0 ? kExactBufs - 1 : buf - 1), 2 * kT);
+        return;
+    }
+
+    const int pg = tid % kPG, og = tid / kPG;
+    const uint64_t neg_zero = pack2(neg_zero_arg, neg_zero_arg);
+    uint64_t acc[kTO][kTP / 2];
+#pragma unroll
+    for (int j = 0; j < kTO; ++j)
+#pragma unroll
+        for (int e = 0; e < kTP / 2; ++e) acc[j][e] = 0ull;
+    int buf = 0;
+    for (int s = 0; s < stages; ++s) {
+        named_sync(1 + buf, 2 * kT);
+#pragma unroll
+        for (int k = 0; k < KC; ++k) {
+            uint64_t x[kTP / 2], w[kTO];
+            // the thread's pixels: groups of four consecutive ones kPG * 4 apart, then (kTP % 4 == 2) one pair
+#pragma unroll
+            for (int e = 0; e < kTP / 4; ++e) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&xs[buf][k][e * kPG * 4 + pg * 4]);
+                x[2 * e] = v.x;
+                x[2 * e + 1] = v.y;
+            }
+            if constexpr (kTP % 4 != 0) x[kTP / 2 - 1] = *reinterpret_cast<const uint64_t*>(&xs[buf][k][(kTP / 4) * kPG * 4 + pg * 2]);
+#pragma unroll
+            for (int j = 0; j < kTO / 4; ++j) {
+                const float4 v = *reinterpret_cast<const float4*>(&ws[buf][k][og * kTO + 4 * j]);
+                w[4 * j] = pack2(v.x, v.x);
+                w[4 * j + 1] = pack2(v.y, v.y);
+                w[4 * j + 2] = pack2(v.z, v.z);
+                w[4 * j + 3] = pack2(v.w, v.w);
+            }
+            if constexpr (kTO % 4 != 0) {
+                const float2 v = *reinterpret_cast<const float2*>(&ws[buf][k][og * kTO + kTO - 2]);
+                w[kTO - 2] = pack2(v.x, v.x);
+                w[kTO - 1] = pack2(v.y, v.y);
+            }
+#pragma unroll
+            for (int j = 0; j < kTO; ++j)
+#pragma unroll
+                for (int e = 0; e < kTP / 2; ++e) acc[j][e] = mac2_exact(acc[j][e], x[e], w[j], neg_zero);
+        }
+        if (s + kExactBufs < stages) named_arrive(1 + kExactBufs + buf, 2 * kT);
+        buf = buf + 1 == kExactBufs ? 0 : buf + 1;
+    }
+
+    // four consecutive pixels of one image are one 16-byte access where planes and pointers allow it
+    const bool vec = (plane_out & 3) == 0 && epi.aligned16();
+#pragma unroll
+    for (int g = 0; g < (kTP + 2) / 4; ++g) {
+        const bool quad = 4 * g + 4 <= kTP;
+        const int64_t p = p0 + g * kPG * 4 + pg * (quad ? 4 : 2);
+        if (p >= P) continue;
+#pragma unroll
+        for (int j = 0; j < kTO; ++j) {
+            const int o = o0 + og * kTO + j;
+            if (o >= d.O) continue;
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[j][2 * g]));
+            if (quad) asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2]), "=f"(v[3]) : "l"(acc[j][quad ? 2 * g + 1 : 0]));
+            if (quad && vec) {
+                const int64_t n = p / plane_out;
+                epi.four(v, (n * d.O + o) * plane_out + (p - n * plane_out), o);
+            } else {
+                for (int e = 0; e < (quad ? 4 : 2); ++e) {
+                    const int64_t n = (p + e) / plane_out;
+                    if (p + e < P) epi(v[e], (n * d.O + o) * plane_out + (p + e - n * plane_out), o);
+                }
+            }
+        }
     }
 }
 
@@ -201,6 +353,23 @@ struct EpilogueF32 {
         if (relu) v = v > 0.0f ? v : 0.0f;
         out[lin] = v;
     }
+    __device__ __forceinline__ bool aligned16() const {
+        return ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(residual)) & 15u) == 0;
+    }
+    // four consecutive outputs of channel o, the first at a multiple of four
+    __device__ __forceinline__ void four(const float* acc, int64_t lin, int o) const {
+        float4 v = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        if (bias) {
+            const float b = __ldg(bias + o);
+            v = make_float4(__fadd_rn(v.x, b), __fadd_rn(v.y, b), __fadd_rn(v.z, b), __fadd_rn(v.w, b));
+        }
+        if (residual) {
+            const float4 r = __ldg(reinterpret_cast<const float4*>(residual + lin));
+            v = make_float4(__fadd_rn(v.x, r.x), __fadd_rn(v.y, r.y), __fadd_rn(v.z, r.z), __fadd_rn(v.w, r.w));
+        }
+        if (relu) v = make_float4(v.x > 0.0f ? v.x : 0.0f, v.y > 0.0f ? v.y : 0.0f, v.z > 0.0f ? v.z : 0.0f, v.w > 0.0f ? v.w : 0.0f);
+        *reinterpret_cast<float4*>(out + lin) = v;
+    }
 };
 
 struct EpilogueS8 {
@@ -214,7 +383,7 @@ struct EpilogueS8 {
     }
 };
 
-// nn_dense / nn_gemm in reference order: acc = 0; acc += a[i,k]*b[j,k]; (*alpha); + (beta*)c[j]
+// nn_dense / nn_gemm in reference order, for what the packed kernel does not take: acc = 0; acc += a[i,k]*b[j,k]; (*alpha); + (beta*)c[j]
 // (include/te/topi/nn.h:48-101, src/relay/op/nn/dense.cc:34-61).
 __global__ void __launch_bounds__(kThreads) gemm_direct_kernel(const float* __restrict__ a, const float* __restrict__ b,
                                                                const float* __restrict__ c, float* __restrict__ out,
@@ -248,6 +417,69 @@ int grid_for(int64_t items) {
     return (int)blocks;
 }
 
+// Tile of the packed kernel. The sum over k is one chain per output and cannot be split, so a launch's parallelism is its
+// outputs: large tiles for large launches, smaller ones where they would leave SMs idle. The estimate is the number of
+// blocks on the busiest SM times the clocks a block takes there per k, as measured on the convolutions of ResNet-18 at 1, 8
+// and 32 images (`alone`: a single block on its SM, latencies showing; `shared`: per block when there are several).
+//   tile (channels x pixels)    64x128   64x96   32x64   16x32
+//   FMA-pipe bound                 128      96      32       8
+//   alone / shared             157/150 126/120   59/45   31/20.5
+struct ExactCost {
+    int tile_o, tile_p;
+    double alone, shared;
+};
+constexpr ExactCost kExactCosts[] = {
+    {64, 128, 157.0, 150.0}, {64, 96, 126.0, 120.0}, {32, 64, 59.0, 45.0}, {16, 32, 31.0, 20.5}};
+
+int pick_exact_tile(const ConvDims& d) {
+    const int64_t P = (int64_t)d.N * d.OH * d.OW;
+    int best = 0;
+    double best_cost = 0.0;
+    for (int i = 0; i < 4; ++i) {
+        const ExactCost& c = kExactCosts[i];
+        const int64_t blocks = ((P + c.tile_p - 1) / c.tile_p) * ((d.O + c.tile_o - 1) / c.tile_o);
+        const int64_t per_sm = (blocks + kNumSMs - 1) / kNumSMs;
+        const double cost = per_sm <= 1 ? c.alone : (double)per_sm * c.shared;
+        if (i == 0 || cost < best_cost) {
+            best = i;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+template <int kTO, int kTP, int kMul, int kMinBlocks>
+void launch_exact_tile(const float* data, const float* weight, const ConvDims& d, const EpilogueF32& epi, cudaStream_t s) {
+    using Tile = ExactTile<kTO, kTP, 8, 16>;
+    const int64_t P = (int64_t)d.N * d.OH * d.OW;
+    const dim3 grid((unsigned)((P + Tile::kP - 1) / Tile::kP), (unsigned)((d.O + Tile::kO - 1) / Tile::kO), 1u);
+    auto go = [&](auto kernel) { kernel<<<grid, 2 * Tile::kThreads, 0, s>>>(data, weight, d, -0.0f, epi); };
+    switch (d.DW == 1 ? d.KW : 0) {
+        case 1: go(conv2d_tiled_f32_kernel<1, kTO, kTP, 8, 16, kMul, kMinBlocks, EpilogueF32>); break;
+        case 3: go(conv2d_tiled_f32_kernel<3, kTO, kTP, 8, 16, kMul, kMinBlocks, EpilogueF32>); break;
+        case 7: go(conv2d_tiled_f32_kernel<7, kTO, kTP, 8, 16, kMul, kMinBlocks, EpilogueF32>); break;
+        default: go(conv2d_tiled_f32_kernel<0, kTO, kTP, 8, 16, kMul, kMinBlocks, EpilogueF32>); break;
+    }
+}
+
+// one thread per output for a handful of them, filters of more than 64 taps and extents beyond 32-bit offsets
+bool tiled_f32_ok(const ConvDims& d) {
+    const int64_t P = (int64_t)d.N * d.OH * d.OW;
+    return P * d.O >= 64 && d.KH * d.KW <= kExactMaxTaps && P <= 0x7fffffffll && (int64_t)d.H * d.W <= 0x3fffffffll &&
+           (int64_t)d.C * d.KH * d.KW <= 0x3fffffffll && (d.O + 15) / 16 <= 65535 &&
+           (int64_t)d.KH * d.DH * d.W + (int64_t)d.KW * d.DW <= 0x3fffffffll;
+}
+
+int32_t launch_tiled_f32(const float* data, const float* weight, const ConvDims& d, const EpilogueF32& epi, cudaStream_t s) {
+    switch (pick_exact_tile(d)) {
+        case 0: launch_exact_tile<8, 8, 1, 2>(data, weight, d, epi, s); break;
+        case 1: launch_exact_tile<8, 6, 1, 2>(data, weight, d, epi, s); break;
+        case 2: launch_exact_tile<4, 4, 2, 4>(data, weight, d, epi, s); break;
+        default: launch_exact_tile<2, 2, 4, 4>(data, weight, d, epi, s); break;
+    }
+    return check_launch("nn_conv2d (fp32, tiled)");
+}
+
 }  // namespace
 
 int32_t conv2d_fp32_exact(const float* data, const float* weight, const float* bias, const float* residual, float* out,
@@ -255,19 +487,7 @@ int32_t conv2d_fp32_exact(const float* data, const float* weight, const float* b
     const int64_t total = (int64_t)d.N * d.O * d.OH * d.OW;
     if (total == 0) return KXC_B200_OK;
     EpilogueF32 epi{bias, residual, out, relu};
-    const int taps = d.KH * d.KW;
-    // weights of up to 8 input channels per shared-memory block, within 40 KiB
-    int rc_block = (40 * 1024) / (taps * kTileO * (int)sizeof(float));
-    if (rc_block > 8) rc_block = 8;
-    if (rc_block > d.C) rc_block = d.C;
-    // the tiled kernel for anything that fills a few blocks; tiny problems and huge filters stay with one thread per output
-    const int64_t pixels = (int64_t)d.N * d.OH * d.OW;
-    if (rc_block >= 1 && total >= 4096 && (pixels + 15) / 16 <= 0x7fffffffll && (d.O + kTileO - 1) / kTileO <= 65535) {
-        // (a 4 x 2 shape with four times as many threads for the deep layers of a small batch was measured slower:
-        // 1.78 / 1.94 ms against 1.13 / 1.52 ms on the layer-3 / layer-4 convolutions of ResNet-18 at 32 images)
-        launch_tiled_f32<8, 4>(data, weight, d, rc_block, epi, s);
-        return check_launch("nn_conv2d (fp32, tiled)");
-    }
+    if (tiled_f32_ok(d)) return launch_tiled_f32(data, weight, d, epi, s);
     conv2d_direct_kernel<float, float, EpilogueF32><<<grid_for(total), kThreads, 0, s>>>(data, weight, d, epi);
     return check_launch("nn_conv2d (fp32)");
 }
@@ -285,6 +505,10 @@ int32_t gemm_fp32_exact(const float* a, const float* b, const float* c, float* o
                         cudaStream_t s) {
     const int64_t total = (int64_t)g.m * g.n;
     if (total == 0) return KXC_B200_OK;
+    // [M,K] x [N,K]^T + c is a 1x1 convolution over M images of one pixel, in the same order (32 x 1000 x 512: 76 -> 20 us)
+    const bool plain = !g.has_c || ((double)g.alpha == 1.0 && (double)g.beta == 1.0);
+    const ConvDims d{g.m, g.k, 1, 1, g.n, 1, 1, 1, 1, 0, 0, 1, 1, 1, 1};
+    if (g.transB && plain && g.k > 0 && tiled_f32_ok(d)) return launch_tiled_f32(a, b, d, EpilogueF32{g.has_c ? c : nullptr, nullptr, out, 0}, s);
     gemm_direct_kernel<<<grid_for(total), kThreads, 0, s>>>(a, b, c, out, g.m, g.n, g.k, g.alpha, g.beta, g.transB, g.has_c);
     return check_launch("nn_gemm (fp32)");
 }

@@ -164,6 +164,21 @@ def test_conv2d_fp32_mode_bit_exact(ops, rng, case):
     assert_bit_exact(got, conv_expect(x, w, b, None, True, s, p, d), f"conv fp32 {case}")
 
 
+# the tiles of the packed fp32 kernel (16x32, 32x64, 64x96, 64x128 channels x pixels), its filter widths (1, 3, 7, any),
+# reductions that end inside a stage, odd weight rows, planes of no multiple of four pixels
+@pytest.mark.parametrize("case", [
+    (1, 5, 21, 19, 17, 3, 3, 1, 1, 1), (1, 33, 20, 20, 64, 1, 1, 1, 0, 1), (5, 7, 27, 23, 65, 3, 3, 1, 1, 1),
+    (5, 3, 90, 94, 63, 7, 7, 2, 3, 1), (5, 18, 45, 44, 64, 1, 1, 1, 0, 1), (3, 5, 79, 81, 66, 3, 3, 1, 1, 1),
+    (5, 2, 57, 60, 64, 3, 3, 1, 1, 1), (4, 2, 63, 65, 70, 5, 5, 1, 2, 1), (5, 3, 56, 56, 64, 3, 3, 1, 2, 2),
+])
+def test_conv2d_fp32_tiles_bit_exact(ops, rng, case):
+    N, C, H, W, O, KH, KW, s, p, d = case
+    x, w, b = conv_inputs(rng, N, C, H, W, O, KH, KW)
+    res = rng.uniform(-1, 1, (N, O, port.conv_out_dim(H, KH, s, p, d), port.conv_out_dim(W, KW, s, p, d))).astype(f32)
+    got = host(ops.nn_conv2d(dev(x), dev(w), dev(b), (s, s), (p, p), (d, d), residual=dev(res), relu=True, precision="fp32"))
+    assert_bit_exact(got, conv_expect(x, w, b, res, True, s, p, d), f"conv fp32 {case}")
+
+
 @pytest.mark.parametrize("precision,tol,rounder", [("tf32", 1e-3, port.round_tf32), ("bf16", 1e-2, port.round_bf16)])
 @pytest.mark.parametrize("case", CONV_CASES)
 def test_conv2d_tensor_core(ops, rng, case, precision, tol, rounder):
