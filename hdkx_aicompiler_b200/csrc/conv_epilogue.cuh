@@ -101,7 +101,18 @@ __device__ __forceinline__ void requant_chunk(const TcParams& p, const uint32_t 
 }
 
 // Epilogue for one 32-column chunk held by one thread (= one output pixel, 32 consecutive channels).
-template <int kOutMode>
+// kSplit (three-pass tf32): the result may also leave as its tf32 high and low parts (TcParams::out_hi).
+__device__ __forceinline__ float tf32_rne(float x) {
+    uint32_t u = __float_as_uint(x);
+    if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0xfffu + ((u >> 13) & 1u)) & 0xffffe000u;
+    return __uint_as_float(u);
+}
+// (a non-finite value lives in the high part only: inf - inf would be NaN)
+__device__ __forceinline__ float tf32_low_part(float x, float hi) {
+    return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u ? 0.0f : tf32_rne(__fsub_rn(x, hi));
+}
+
+template <int kOutMode, bool kSplit = false>
 __device__ __forceinline__ void epilogue_chunk(const TcParams& p, const uint32_t (&v)[32], int c0, bool valid, int n,
                                                int oh, int ow) {
     if (!valid || c0 >= p.Cout) return;
@@ -222,6 +233,23 @@ __device__ __forceinline__ void epilogue_chunk(const TcParams& p, const uint32_t
                     if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0xfffu + ((u >> 13) & 1u)) & 0xffffe000u;
                     f[j] = __uint_as_float(u);
                 }
+            }
+            if constexpr (kSplit) {
+                if (p.out_hi != nullptr) {  // channel counts are multiples of 8 and the buffers aligned: 16-byte stores
+                    float* hi = p.out_hi + pix * p.Cout + c0;
+                    float* lo = hi + p.out_lo_offset;
+#pragma unroll
+                    for (int j = 0; j < 32; j += 4) {
+                        if (j >= nch) break;
+                        float h[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) h[k] = tf32_rne(f[j + k]);
+                        *reinterpret_cast<float4*>(hi + j) = make_float4(h[0], h[1], h[2], h[3]);
+                        *reinterpret_cast<float4*>(lo + j) = make_float4(tf32_low_part(f[j], h[0]), tf32_low_part(f[j + 1], h[1]),
+                                                                         tf32_low_part(f[j + 2], h[2]), tf32_low_part(f[j + 3], h[3]));
+                    }
+                }
+                if (p.out == nullptr) return;
             }
             if (vec) {
 #pragma unroll

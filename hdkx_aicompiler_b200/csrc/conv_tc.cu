@@ -34,15 +34,16 @@ constexpr int kTcThreads = 320;  // 2 control warps + 8 epilogue warps
 constexpr int kStoreBoxBytes = 32 * 128;
 constexpr int kSmemLimit = 227 * 1024;
 
-template <int KB_BYTES, int BN, int kCtas, int kMT = 1>
+template <int KB_BYTES, int BN, int kCtas, int kMT = 1, bool kX3 = false>
 struct StageGeom {
     static constexpr int kATileBytes = 128 * KB_BYTES;
-    static constexpr int kABytes = kMT * kATileBytes;  // kMT pixel tiles share one B tile
-    static constexpr int kBBytes = (BN / kCtas) * KB_BYTES;  // a CTA of a pair holds half of the B tile's rows
+    static constexpr int kABytes = (kX3 ? 2 : kMT) * kATileBytes;  // kMT pixel tiles share one B tile; x3: high, low part
+    static constexpr int kBTileBytes = (BN / kCtas) * KB_BYTES;  // a CTA of a pair holds half of the B tile's rows
+    static constexpr int kBBytes = (kX3 ? 2 : 1) * kBTileBytes;
     static constexpr int kStageBytes = kABytes + kBBytes;
     // per epilogue warp a 4 KiB box (32 pixels x 64 channels, SWIZZLE_128B) that TMA stores read; its first half
     // doubles as the staging tile of the per-thread store path
-    static constexpr int kEpilogueBytes = 8 * kStoreBoxBytes;
+    static constexpr int kEpilogueBytes = kX3 ? 0 : 8 * kStoreBoxBytes;
     static constexpr int kStagesRaw = (kSmemLimit - 2048 - kEpilogueBytes) / kStageBytes;
     static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
     static constexpr int kSmemBytes = kStages * kStageBytes + kEpilogueBytes + 1024;  // + slack to align the ring to 1024 B
@@ -61,13 +62,21 @@ struct StageGeom {
 // kMT = 2: a work item is TWO pixel tiles per CTA against one B tile. Their MMAs alternate between two
 // accumulators, which gives the tensor core two independent accumulate chains (a pair's M = 256 instruction has
 // a long dependent-issue latency) and halves the B traffic per pixel.
-template <MmaKind kKind, int KB_BYTES, int BN, int kOutMode, int kCtas, bool kDual = false, int kMT = 1>
+//
+// kX3 (three-pass tf32): every stage carries the high and low parts of both operands, so a tap's pixels and weights cross
+// L2 -> shared memory twice instead of three times and no partial sum leaves the chip. The B tile is [w_hi; w_lo] (2 BN
+// rows): ONE instruction of N = 2 BN multiplies a_hi with both and fills the accumulators hi*hi | hi*lo side by side, a
+// second of N = BN adds a_lo * w_hi to the latter. The two sums meet in one rounded fp32 add in the epilogue. An
+// instruction costs ~140 / 205 cycles at N = 128 / 256 and ~96 / 140 at 64 / 128 (operand fetch), so a stage of four K steps
+// is ~950 (BN 64) or ~1400 cycles (BN 128), just above the ~50 B/clk at which an SM's stage (48 / 64 KB) arrives.
+template <MmaKind kKind, int KB_BYTES, int BN, int kOutMode, int kCtas, bool kDual = false, int kMT = 1, bool kX3 = false>
 __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_constant__ TcParams p) {
-    using G = StageGeom<KB_BYTES, BN, kCtas, kMT>;
+    using G = StageGeom<KB_BYTES, BN, kCtas, kMT, kX3>;
     static_assert(!(kDual && kMT != 1), "the two-output kernel works on one pixel tile at a time");
+    static_assert(!kX3 || (kKind == MmaKind::TF32 && kCtas == 1 && !kDual && kMT == 1 && BN <= 128), "three-pass form: tf32, single CTAs");
     constexpr bool kPair = kCtas == 2;
     constexpr int kStages = G::kStages;
-    constexpr int kAccCols = (kDual ? 2 : kMT) * BN;  // TMEM columns of one accumulator buffer
+    constexpr int kAccCols = (kDual || kX3 ? 2 : kMT) * BN;  // TMEM columns of one accumulator buffer
     // two accumulator buffers (the epilogue of one work item overlaps the next item's main loop) where TMEM's 512
     // columns allow it, else one
     constexpr int kBufs = 2 * kAccCols <= 512 ? 2 : 1;
@@ -78,6 +87,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
     constexpr uint32_t kIdesc =
         make_instr_desc(kKind == MmaKind::F16 ? kFmtBF16 : (kKind == MmaKind::TF32 ? kFmtTF32 : kFmtS8),
                         kKind == MmaKind::I8 ? kAccS32 : kAccF32, BN, 128u * kCtas);
+    [[maybe_unused]] constexpr uint32_t kIdescWide = make_instr_desc(kFmtTF32, kAccF32, 2 * BN <= 256 ? 2 * BN : 256, 128u);  // x3: [w_hi; w_lo]
 
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[kStages];
@@ -137,8 +147,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
         if (lane == 0) {
             tma_prefetch_desc(&p.tmB);
             tma_prefetch_desc(&p.tmA[0]);
-            if constexpr (kDual) tma_prefetch_desc(&p.tmB2);
-            const uint32_t tx_bytes = (uint32_t)(kMT * rows_used * KB_BYTES + G::kBBytes);
+            if constexpr (kDual || kX3) tma_prefetch_desc(&p.tmB2);
+            const uint32_t tx_bytes = (uint32_t)((kX3 ? 2 : kMT) * rows_used * KB_BYTES + G::kBBytes);
             pdl_wait();  // the activations come from the previous kernel
             int stage = 0;
             uint32_t phase = 0;
@@ -190,6 +200,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                                     tma_load_4d(a_dst + t * G::kATileBytes, &p.tmA[map], full, cb * p.kb_elems, ow0[t] + cw, oh0[t] + ch,
                                                 n0[t]);
                                 tma_load_2d(a_dst + G::kABytes, &p.tmB, full, kb * p.kb_elems, co0);
+                                if constexpr (kX3) {
+                                    tma_load_4d(a_dst + G::kATileBytes, &p.tmA[map], full, cb * p.kb_elems, ow0[0] + cw, oh0[0] + ch,
+                                                n0[0] + p.N);
+                                    tma_load_2d(a_dst + G::kABytes + G::kBTileBytes, &p.tmB2, full, kb * p.kb_elems, co0);
+                                }
                             }
                             if (++stage == kStages) { stage = 0; phase ^= 1u; }
                         }
@@ -246,6 +261,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                     const uint64_t b_desc = make_smem_desc(a_addr + G::kABytes, KB_BYTES);
 #pragma unroll
                     for (int k = 0; k < KB_BYTES / 32; ++k) {
+                        if constexpr (kX3) {
+                            const uint64_t a_k = a_desc + (uint64_t)(2 * k), b_k = b_desc + (uint64_t)(2 * k);
+                            umma<kKind>(d_tmem, a_k, b_k, kIdescWide, (kb_local | k) != 0 ? 1u : 0u);
+                            umma<kKind>(d_tmem + (uint32_t)BN, a_k + (uint64_t)(G::kATileBytes >> 4), b_k, kIdesc, 1u);
+                        } else {
 #pragma unroll
                         for (int t = 0; t < kMT; ++t) {
                             // advancing 32 bytes along K inside the swizzle span = +2 in the (addr >> 4) field;
@@ -256,6 +276,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                                 umma_pair<kKind>(d_t, a_k, b_desc + (uint64_t)(2 * k), kIdesc, (kb_local | k) != 0 ? 1u : 0u);
                             else
                                 umma<kKind>(d_t, a_k, b_desc + (uint64_t)(2 * k), kIdesc, (kb_local | k) != 0 ? 1u : 0u);
+                        }
                         }
                     }
                     if constexpr (kPair) umma_commit_pair(smem_u32(&bar_empty[stage]), 3);
@@ -331,6 +352,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                 uint4 res_next[4] = {};
                 if (fast && has_res && (i + 1 < kChunksPerWarp) && (c0 + 32 < p.Cout))
                     residual_fetch_rows(ep, rows, c0 + 32, lane, res_next);
+                if constexpr (kX3) {
+                    uint32_t u[32];
+                    tmem_ld_32x32(t_addr + (uint32_t)(BN + i * 32), u);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j])));
+                }
                 tmem_ld_wait();
                 if (boxed) {
                     if ((i & 1) == 0) {  // a new 64-channel group: the previous store must have read the box
@@ -351,7 +379,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                 } else if (fast) {
                     if (c0 < p.Cout) epilogue_coalesced_bf16<32>(ep, v, c0, stage_tile, lane, rows, res_cur, has_res);
                 } else {
-                    epilogue_chunk<kOutMode>(p, v, c0, valid, n, oh, ow);
+                    epilogue_chunk<kOutMode, kX3>(p, v, c0, valid, n, oh, ow);
                 }
 #pragma unroll
                 for (int g = 0; g < 4; ++g) res_cur[g] = res_next[g];
@@ -421,10 +449,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
     if (threadIdx.x == 0 && *abort_ptr && p.status != nullptr) atomicExch(p.status, KXC_B200_ERR_DEVICE_WAIT);
 }
 
-template <MmaKind kKind, int KB_BYTES, int BN, int kOutMode, int kCtas, bool kDual = false, int kMT = 1>
+template <MmaKind kKind, int KB_BYTES, int BN, int kOutMode, int kCtas, bool kDual = false, int kMT = 1, bool kX3 = false>
 int32_t launch_one(const TcParams& p, cudaStream_t stream) {
-    using G = StageGeom<KB_BYTES, BN, kCtas, kMT>;
-    auto kernel = conv_igemm_kernel<kKind, KB_BYTES, BN, kOutMode, kCtas, kDual, kMT>;
+    using G = StageGeom<KB_BYTES, BN, kCtas, kMT, kX3>;
+    auto kernel = conv_igemm_kernel<kKind, KB_BYTES, BN, kOutMode, kCtas, kDual, kMT, kX3>;
     static PerDeviceOnce smem_once;
     static std::mutex units_mu;
     static int max_units[PerDeviceOnce::kMaxDevices] = {0};  // per device: clusters of two (kCtas = 2) resident at once
@@ -480,8 +508,24 @@ int32_t launch_by_out(const TcConfig& cfg, const TcParams& p, cudaStream_t s) {
     return fail(KXC_B200_ERR_INVALID, "tensor-core conv: output mode %d does not fit dtype %d", (int)cfg.out_mode, (int)cfg.dtype);
 }
 
+template <int KB_BYTES, int BN>
+int32_t launch_x3(const TcConfig& cfg, const TcParams& p, cudaStream_t s) {
+    switch (cfg.out_mode) {
+        case kOutNHWC_F32: return launch_one<MmaKind::TF32, KB_BYTES, BN, kOutNHWC_F32, 1, false, 1, true>(p, s);
+        case kOutNCHW_F32: return launch_one<MmaKind::TF32, KB_BYTES, BN, kOutNCHW_F32, 1, false, 1, true>(p, s);
+        default: return fail(KXC_B200_ERR_INVALID, "tensor-core conv: output mode %d has no three-pass form", (int)cfg.out_mode);
+    }
+}
+
 template <MmaKind kKind, int KB_BYTES>
 int32_t launch_by_bn(const TcConfig& cfg, const TcParams& p, cudaStream_t s) {
+    if (cfg.x3) {
+        if constexpr (kKind == MmaKind::TF32) {
+            if (cfg.ctas == 1 && cfg.mt == 1 && !cfg.dual && (cfg.bn == 64 || cfg.bn == 128))
+                return cfg.bn == 64 ? launch_x3<KB_BYTES, 64>(cfg, p, s) : launch_x3<KB_BYTES, 128>(cfg, p, s);
+        }
+        return fail(KXC_B200_ERR_INVALID, "tensor-core conv: no three-pass kernel for this configuration");
+    }
     if constexpr (KB_BYTES == 128 && kKind == MmaKind::F16) {
         if (cfg.dual) {
             if ((cfg.bn != 128 && cfg.bn != 192) || cfg.ctas != 1 || cfg.out_mode != kOutNHWC_BF16 || !p.vec_ok || (p.Cout & 31) != 0)
@@ -685,7 +729,8 @@ int32_t tc_setup_dual(TcParams* p, TcConfig* cfg, const void* act_nhwc, const vo
 
 int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_mode, const void* act_nhwc,
                       const void* w_packed, int N, int H, int W, int cpad, int Cout, int KH, int KW, int stride, int pad_h,
-                      int pad_w, int dil_h, int dil_w, int* status_word) {
+                      int pad_w, int dil_h, int dil_w, int* status_word, int map_images) {
+    if (map_images <= 0) map_images = N;
     const int eb = tc_elem_bytes(dtype);
     if (stride != 1 && stride != 2) return fail(KXC_B200_ERR_UNSUPPORTED, "tensor-core conv: stride %d", stride);
     const int row_bytes = cpad * eb;
@@ -762,7 +807,7 @@ int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_m
     const uint32_t box[4] = {(uint32_t)p->kb_elems, (uint32_t)p->BW, (uint32_t)p->BH, (uint32_t)p->BNI};
     uint8_t* base = const_cast<uint8_t*>(static_cast<const uint8_t*>(act_nhwc));
     if (stride == 1) {
-        const uint64_t dims[4] = {(uint64_t)cpad, (uint64_t)W, (uint64_t)H, (uint64_t)N};
+        const uint64_t dims[4] = {(uint64_t)cpad, (uint64_t)W, (uint64_t)H, (uint64_t)map_images};
         const uint64_t strides[3] = {(uint64_t)row_bytes, (uint64_t)W * row_bytes, (uint64_t)H * W * row_bytes};
         KXC_TRY(tc_make_tmap(&p->tmA[0], dtype, 4, base, dims, strides, box, kb_bytes));
         for (int i = 1; i < 4; ++i) p->tmA[i] = p->tmA[0];
@@ -775,7 +820,7 @@ int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_m
                 CUtensorMap* m = &p->tmA[hp * 2 + wp];
                 if (hc <= 0 || wc <= 0)
                     return fail(KXC_B200_ERR_UNSUPPORTED, "tensor-core conv: stride 2 over a %dx%d input", H, W);
-                const uint64_t dims[4] = {(uint64_t)cpad, (uint64_t)wc, (uint64_t)hc, (uint64_t)N};
+                const uint64_t dims[4] = {(uint64_t)cpad, (uint64_t)wc, (uint64_t)hc, (uint64_t)map_images};
                 const uint64_t strides[3] = {(uint64_t)2 * row_bytes, (uint64_t)2 * W * row_bytes, (uint64_t)H * W * row_bytes};
                 KXC_TRY(tc_make_tmap(m, dtype, 4, base + ((size_t)hp * W + wp) * row_bytes, dims, strides, box, kb_bytes));
             }
@@ -791,6 +836,30 @@ int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_m
         KXC_TRY(tc_status_word(&p->status));
     }
     return KXC_B200_OK;
+}
+
+int32_t tc_finish_x3(TcParams* p, TcConfig* cfg, const void* w_hi, const void* w_lo, int Cout, int k_elems) {
+    // The tile whose waves cost least: a stage takes ~950 cycles with 64 channels and ~1400 with 128 (see the kernel).
+    const long long m_tiles = (long long)p->tiles_w * p->tiles_h * p->tiles_n;
+    auto waves = [&](int bn) { return (m_tiles * ((Cout + bn - 1) / bn) + kNumSMs - 1) / kNumSMs; };
+    const int bn = Cout > 64 && waves(128) * 1400 <= waves(64) * 950 ? 128 : 64;
+    cfg->bn = bn; cfg->ctas = 1; cfg->mt = 1; cfg->dual = 0; cfg->x3 = 1;
+    p->tiles_c = (Cout + bn - 1) / bn;
+    const uint64_t ktot = (uint64_t)k_elems;
+    const uint64_t bdims[2] = {ktot, (uint64_t)Cout};
+    const uint64_t bstrides[1] = {ktot * 4};
+    const uint32_t bbox[2] = {(uint32_t)p->kb_elems, (uint32_t)bn};
+    KXC_TRY(tc_make_tmap(&p->tmB, kTcTF32, 2, const_cast<void*>(w_hi), bdims, bstrides, bbox, cfg->kb_bytes));
+    return tc_make_tmap(&p->tmB2, kTcTF32, 2, const_cast<void*>(w_lo), bdims, bstrides, bbox, cfg->kb_bytes);
+}
+
+int32_t tc_setup_conv_x3(TcParams* p, TcConfig* cfg, TcOutMode out_mode, const void* act_hi, const void* w_hi, const void* w_lo, int N,
+                         int H, int W, int cpad, int Cout, int KH, int KW, int stride, int pad_h, int pad_w, int dil_h, int dil_w) {
+    // The maps cover 2N images: an image's low part is addressed N images further on. A box that runs past image N reads
+    // low parts into rows that are not stored.
+    KXC_TRY(tc_setup_conv(p, cfg, kTcTF32, out_mode, act_hi, w_hi, N, H, W, cpad, Cout, KH, KW, stride, pad_h, pad_w, dil_h, dil_w, nullptr,
+                          2 * N));
+    return tc_finish_x3(p, cfg, w_hi, w_lo, Cout, KH * KW * cpad);
 }
 
 }  // namespace kxc_b200

@@ -67,6 +67,10 @@ struct alignas(64) TcParams {
     // TMA stores of the output (tc_bind_store): each epilogue warp's 32 pixels x 64 channels leave as one box
     CUtensorMap tmOut, tmOut2;
     int store_box;               // 1 when tmOut (and tmOut2 for the two-output form) are valid
+    // three-pass tf32 (TcConfig::x3), kOutNHWC_F32 only: the result also leaves split for the next contraction, the tf32
+    // high part at out_hi and the low part out_lo_offset elements after it (null: not wanted). `out` may then be null.
+    float* out_hi;
+    long long out_lo_offset;
 };
 
 struct TcConfig {
@@ -76,6 +80,9 @@ struct TcConfig {
     TcOutMode out_mode;
     int ctas = 1;  // 2: clusters of two CTAs share each B tile (tcgen05 cta_group::2, M = 256 per instruction)
     int dual = 0;  // 1: also computes the 1x1 convolution described by tmB2 / bias2 / out2 / relu2
+    // 1 (tf32 only): the operands come as tf32 high and low parts and hi*hi, hi*lo and lo*hi are summed in one launch. The
+    // low activations lie N images after the high ones (one tensor map covers both), tmB2 describes the low weights.
+    int x3 = 0;
     int mt = 1;    // 2: two pixel tiles per work item share each B tile (two accumulate chains in flight)
 };
 
@@ -105,10 +112,10 @@ int32_t static_scratch_status_word(int** out);
 // Fills tmA/tmB and the geometry of `p` for a regular convolution over an NHWC activation tensor
 // with `cpad` channels and weights packed as [Cout][KH][KW][cpad].
 // `status_word`: device int the kernel reports a run-out wait into; nullptr = the process-wide word
-// from tc_status_word().
+// from tc_status_word(). `map_images`: images the activation maps cover (0: N).
 int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_mode, const void* act_nhwc,
                       const void* w_packed, int N, int H, int W, int cpad, int Cout, int KH, int KW, int stride, int pad_h,
-                      int pad_w, int dil_h, int dil_w, int* status_word = nullptr);
+                      int pad_w, int dil_h, int dil_w, int* status_word = nullptr, int map_images = 0);
 
 // Whether a KHxKW convolution (stride, padding, dilation as given) can carry a 1x1 convolution of the same stride
 // and no padding as its second output, and the setup of that second output (call after tc_setup_conv, which it
@@ -119,6 +126,12 @@ bool tc_dual_applicable(TcDType dtype, TcOutMode out_mode, int cpad, int Cout, i
 // output, full 128-pixel tiles whose 32-pixel quarters are boxes of the output tensor, channel count a multiple of 64)
 // and sets p->store_box; otherwise leaves the per-thread store path in place. KXC_B200_TMA_STORE=0 disables it.
 int32_t tc_bind_store(TcParams* p, const TcConfig& cfg);
+// Three-pass tf32 form of tc_setup_conv: `act_hi` holds the high parts of N images followed at once by their low parts,
+// w_hi / w_lo the packed weights' parts. Output kOutNHWC_F32 or kOutNCHW_F32.
+int32_t tc_setup_conv_x3(TcParams* p, TcConfig* cfg, TcOutMode out_mode, const void* act_hi, const void* w_hi, const void* w_lo, int N,
+                         int H, int W, int cpad, int Cout, int KH, int KW, int stride, int pad_h, int pad_w, int dil_h, int dil_w);
+// The part of it that follows once the geometry and tmA are set: tile width, tmB / tmB2 over `k_elems` per output channel.
+int32_t tc_finish_x3(TcParams* p, TcConfig* cfg, const void* w_hi, const void* w_lo, int Cout, int k_elems);
 int32_t tc_setup_dual(TcParams* p, TcConfig* cfg, const void* act_nhwc, const void* w_packed, const void* w2_packed, int N,
                       int H, int W, int cpad, int Cout, int KH, int KW, int stride, int pad_h, int pad_w);
 

@@ -60,6 +60,54 @@ __global__ void nchw_to_nhwc_kernel(const TIn* __restrict__ in, TOut* __restrict
     }
 }
 
+// Both tf32 parts of every value in one pass over the input (three-pass tf32). Same grid and block.
+__global__ void nchw_to_nhwc_split_kernel(const float* __restrict__ in, float* __restrict__ hi, float* __restrict__ lo, int C, int HW, int cpad) {
+    __shared__ float tile[32][33];
+    const int n = blockIdx.z;
+    const int hw0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+    const float* src = in + (size_t)n * C * HW;
+    const size_t dst = (size_t)n * HW * cpad;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int c = c0 + threadIdx.y + 8 * k, hw = hw0 + threadIdx.x;
+        tile[threadIdx.y + 8 * k][threadIdx.x] = (c < C && hw < HW) ? src[(size_t)c * HW + hw] : 0.0f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int hw = hw0 + threadIdx.y + 8 * k, c = c0 + threadIdx.x;
+        if (hw < HW && c < cpad) {
+            const float v = tile[threadIdx.x][threadIdx.y + 8 * k];
+            hi[dst + (size_t)hw * cpad + c] = convert_to<float>(v);
+            lo[dst + (size_t)hw * cpad + c] = convert_to<Tf32Lo>(v).v;
+        }
+    }
+}
+
+// The same for rows that need no reordering: [rows, cols] -> two times [rows, cpad]. cols % 4 == 0 and cols == cpad take
+// 16-byte accesses (bound by memory: 4 bytes read and 8 written per value).
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ in, float* __restrict__ hi, float* __restrict__ lo, int64_t rows,
+                                                         int cols, int cpad) {
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (cols == cpad && (cols & 3) == 0) {
+        for (const int64_t total = rows * cols / 4; i < total; i += step) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(in) + i);
+            reinterpret_cast<float4*>(hi)[i] = make_float4(convert_to<float>(v.x), convert_to<float>(v.y), convert_to<float>(v.z), convert_to<float>(v.w));
+            reinterpret_cast<float4*>(lo)[i] = make_float4(convert_to<Tf32Lo>(v.x).v, convert_to<Tf32Lo>(v.y).v, convert_to<Tf32Lo>(v.z).v,
+                                                           convert_to<Tf32Lo>(v.w).v);
+        }
+        return;
+    }
+    for (const int64_t total = rows * cpad; i < total; i += step) {
+        const int c = (int)(i % cpad);
+        const int64_t r = i / cpad;
+        const float v = c < cols ? in[r * cols + c] : 0.0f;
+        hi[i] = convert_to<float>(v);
+        lo[i] = convert_to<Tf32Lo>(v).v;
+    }
+}
+
 // int8 form: 64 channels x 64 pixels per block, four bytes per thread on both sides (64-byte runs in HBM instead of the
 // 32-byte runs the element-wise kernel makes of 1-byte elements). grid (ceil(HW/64), ceil(cpad/64), N), block 256.
 // It is a batched byte transpose [C][HW] -> [HW][cpad] (rows c >= C read as zero), so it also serves NHWC -> NCHW with
@@ -209,6 +257,25 @@ int32_t nchw_to_nhwc(const void* in, void* out, TcDType dtype, int N, int C, int
             break;
     }
     return check_launch("nchw_to_nhwc");
+}
+
+int32_t nchw_to_nhwc_split(const float* in, float* hi, float* lo, int N, int C, int HW, int cpad, cudaStream_t s) {
+    if (N == 0) return KXC_B200_OK;
+    if (N > 65535) return fail(KXC_B200_ERR_UNSUPPORTED, "layout transform: batch %d exceeds the grid limit", N);
+    nchw_to_nhwc_split_kernel<<<dim3((HW + 31) / 32, (cpad + 31) / 32, N), dim3(32, 8), 0, s>>>(in, hi, lo, C, HW, cpad);
+    return check_launch("nchw_to_nhwc_split");
+}
+
+int32_t split_rows(const float* in, float* hi, float* lo, int64_t rows, int cols, int cpad, cudaStream_t s) {
+    if (rows * cpad == 0) return KXC_B200_OK;
+    const bool vec = cols == cpad && (cols & 3) == 0;
+    if (vec && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15u) != 0) {
+        // a caller's matrix that is not 16-byte aligned: element by element
+        KXC_TRY(convert_rows(in, hi, kTcTF32, rows, cols, cpad, s, false));
+        return convert_rows(in, lo, kTcTF32, rows, cols, cpad, s, true);
+    }
+    split_rows_kernel<<<grid_1d(vec ? rows * cols / 4 : rows * cpad, 256), 256, 0, s>>>(in, hi, lo, rows, cols, cpad);
+    return check_launch("split_rows");
 }
 
 int32_t nchw_to_nhwc_s8_subsample(const int8_t* in, int8_t* out, int N, int C, int H, int W, int OH, int OW, int stride, int cpad,

@@ -14,6 +14,10 @@ namespace kxc_b200 {
 // rounded away, nearest even), or int8 (copied).
 int32_t nchw_to_nhwc(const void* in, void* out, TcDType dtype, int N, int C, int HW, int cpad, cudaStream_t s, bool tf32_lo = false);
 
+// Three-pass tf32 operands: the tf32 rounding of every value (hi) and the tf32 rounding of what that dropped (lo).
+int32_t nchw_to_nhwc_split(const float* in, float* hi, float* lo, int N, int C, int HW, int cpad, cudaStream_t s);
+int32_t split_rows(const float* in, float* hi, float* lo, int64_t rows, int cols, int cpad, cudaStream_t s);
+
 // int8 NCHW -> NHWC of only the pixels a 1x1 convolution of stride `stride` without padding reads:
 // out[n][oh][ow][c] = in[n][c][oh*stride][ow*stride], channels zero-filled up to cpad (a multiple of 4).
 int32_t nchw_to_nhwc_s8_subsample(const int8_t* in, int8_t* out, int N, int C, int H, int W, int OH, int OW, int stride, int cpad,

@@ -271,10 +271,16 @@ __device__ __forceinline__ __nv_bfloat16 to_operand<__nv_bfloat16>(float v) { re
 template <>
 __device__ __forceinline__ float to_operand<float>(float v) { return round_tf32_rne(v); }
 
+// The tf32 rounding of what round_tf32_rne drops (a non-finite value lives in the high part only).
+__device__ __forceinline__ float tf32_dropped(float x) {
+    return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u ? 0.0f : round_tf32_rne(__fsub_rn(x, round_tf32_rne(x)));
+}
+
 // Stem input packing: NCHW fp32 [N,C<=4,H,W] -> [N][H+2*pad_h][Wp][4] operand type with a zero border,
 // so that the 8 consecutive pixels x 4 channels starting at an even column form one K block.
+// `lo` (fp32 storage only, may be null): a second packed tensor of what the tf32 rounding dropped.
 template <typename T>
-__global__ void __launch_bounds__(kThreads) stem_pack_kernel(const float* __restrict__ x, T* __restrict__ out, int N, int C,
+__global__ void __launch_bounds__(kThreads) stem_pack_kernel(const float* __restrict__ x, T* __restrict__ out, T* __restrict__ lo, int N, int C,
                                                              int H, int W, int Hp, int Wp, int pad_h, int pad_w) {
     // four consecutive packed pixels per thread (Wp is a multiple of 4): 12 independent loads in flight,
     // 32 or 64 contiguous bytes stored
@@ -306,18 +312,28 @@ __global__ void __launch_bounds__(kThreads) stem_pack_kernel(const float* __rest
         constexpr int kVecs = (int)(sizeof(T) * 16 / 16);
 #pragma unroll
         for (int q = 0; q < kVecs; ++q) reinterpret_cast<uint4*>(dst)[q] = reinterpret_cast<const uint4*>(v)[q];
+        if constexpr (sizeof(T) == 4) {
+            if (lo != nullptr) {
+                float* dlo = lo + (dst - out);
+#pragma unroll
+                for (int px = 0; px < 4; ++px)
+                    reinterpret_cast<float4*>(dlo)[px] = make_float4(tf32_dropped(f[px][0]), tf32_dropped(f[px][1]), tf32_dropped(f[px][2]),
+                                                                     tf32_dropped(f[px][3]));
+            }
+        }
     }
 }
 
 // Stem weights: OIHW fp32 [O,C<=4,KH,KW<=8] -> [O][KH][8][4] operand type, zero for kw >= KW or c >= C
 template <typename T>
-__global__ void stem_pack_weights_kernel(const float* __restrict__ w, T* __restrict__ out, int O, int C, int KH, int KW) {
+__global__ void stem_pack_weights_kernel(const float* __restrict__ w, T* __restrict__ out, int O, int C, int KH, int KW, int low) {
     const int total = O * KH * 32;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int c = i & 3, kw = (i >> 2) & 7;
         const int kh = (i >> 5) % KH, o = (i >> 5) / KH;
         float f = 0.0f;
         if (c < C && kw < KW) f = w[((o * C + c) * KH + kh) * KW + kw];
+        if constexpr (sizeof(T) == 4) f = low ? tf32_dropped(f) : f;
         out[i] = to_operand<T>(f);
     }
 }
@@ -392,20 +408,20 @@ int32_t nhwc_to_nchw_f32(const void* in, float* out, TcDType dt, int N, int C, i
 }
 
 int32_t stem_pack(const float* x, void* out, TcDType dt, int N, int C, int H, int W, int Hp, int Wp, int pad_h, int pad_w,
-                  cudaStream_t s) {
+                  cudaStream_t s, void* lo) {
     if (Wp % 4 != 0) return fail(KXC_B200_ERR_INVALID, "stem_pack: packed width %d must be a multiple of 4", Wp);
     const int64_t items = (int64_t)N * Hp * (Wp / 4);
     if (items == 0) return KXC_B200_OK;
     cudaError_t err = cudaSuccess;
     KXC_DISPATCH_ACT(dt, (err = launch_kernel(stem_pack_kernel<T>, dim3(grid_for(items, 16)), dim3(kThreads), 0, s, /*pdl=*/true, 1, x,
-                                              static_cast<T*>(out), N, C, H, W, Hp, Wp, pad_h, pad_w)));
+                                              static_cast<T*>(out), static_cast<T*>(lo), N, C, H, W, Hp, Wp, pad_h, pad_w)));
     if (err != cudaSuccess) return fail(KXC_B200_ERR_CUDA, "stem_pack launch: %s", cudaGetErrorString(err));
     return check_launch("stem_pack");
 }
 
-int32_t stem_pack_weights(const float* w, void* out, TcDType dt, int O, int C, int KH, int KW, cudaStream_t s) {
+int32_t stem_pack_weights(const float* w, void* out, TcDType dt, int O, int C, int KH, int KW, cudaStream_t s, bool tf32_lo) {
     KXC_DISPATCH_ACT(dt, (stem_pack_weights_kernel<T><<<grid_for((int64_t)O * KH * 32), kThreads, 0, s>>>(w, static_cast<T*>(out), O,
-                                                                                                          C, KH, KW)));
+                                                                                                          C, KH, KW, tf32_lo ? 1 : 0)));
     return check_launch("stem_pack_weights");
 }
 

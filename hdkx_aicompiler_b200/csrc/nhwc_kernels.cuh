@@ -17,7 +17,7 @@ int32_t eltwise_nhwc(const void* a, const void* b, void* out, TcDType dt, int64_
 int32_t nhwc_to_nchw_f32(const void* in, float* out, TcDType dt, int N, int C, int HW, cudaStream_t s);
 // Stem (few-channel, stride-2) input packing and its weight packing; see plan.cu.
 int32_t stem_pack(const float* x, void* out, TcDType dt, int N, int C, int H, int W, int Hp, int Wp, int pad_h, int pad_w,
-                  cudaStream_t s);
-int32_t stem_pack_weights(const float* w, void* out, TcDType dt, int O, int C, int KH, int KW, cudaStream_t s);
+                  cudaStream_t s, void* lo = nullptr);
+int32_t stem_pack_weights(const float* w, void* out, TcDType dt, int O, int C, int KH, int KW, cudaStream_t s, bool tf32_lo = false);
 
 }  // namespace kxc_b200

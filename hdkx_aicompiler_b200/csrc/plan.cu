@@ -56,6 +56,8 @@ struct Value {
     // storage of the internal (NHWC / row-major, operand dtype) copy
     size_t offset = 0, bytes = 0;
     bool has_storage = false;
+    bool split = false, plain = false;  // TF32X3 plans: the stored forms, of `elems` values each
+    size_t elems = 0;
     int first_step = -1, last_step = -1;
 };
 
@@ -98,10 +100,7 @@ struct Step {
     // conv / gemm
     TcParams params{};
     TcConfig cfg{};
-    // TF32X3 plans: the two correction passes (x_lo * w_hi, x_hi * w_lo) that run before `params` (x_hi * w_hi);
-    // src_input = the graph input this step reads through its NHWC copy (-1: an intermediate)
-    TcParams params_lohi{}, params_hilo{};
-    int src_input = -1;
+    int src_input = -1;  // the graph input this step reads through its copy or itself (-1: an intermediate)
     // pooling / misc geometry
     int N = 0, C = 0, H = 0, W = 0, OH = 0, OW = 0;
     kxc_b200_pool2d_attrs pool{};
@@ -122,11 +121,10 @@ int64_t numel_of(const std::vector<int64_t>& s) {
 struct kxc_b200_plan {
     int precision = KXC_B200_PREC_BF16;
     TcDType dtype = kTcBF16;
-    // KXC_B200_PREC_TF32X3: activations stay full fp32 in the arena; every convolution / dense step splits its
-    // input into tf32 high and low parts (x3_scratch) and runs three tensor-core passes into the same fp32 output
+    // KXC_B200_PREC_TF32X3: convolutions and dense layers multiply tf32 high and low parts in one launch. An activation is
+    // stored in the forms its consumers read (Value::split, Value::plain): the high parts followed by the low parts for a
+    // contraction, the full fp32 values for everything else (residuals, pooling).
     bool x3 = false;
-    void* x3_scratch = nullptr;
-    size_t x3_half_bytes = 0;  // the low part starts this many bytes into x3_scratch
     std::map<int, Value> values;
     std::vector<int> inputs, constants;
     std::vector<Node> nodes;
@@ -174,7 +172,6 @@ struct kxc_b200_plan {
         for (auto& g : graph_slots)
             if (g.exec) cudaGraphExecDestroy(g.exec);
         if (tail_buf) cudaFree(tail_buf);
-        if (x3_scratch) cudaFree(x3_scratch);
         if (arena) cudaFree(arena);
         if (weight_arena) cudaFree(weight_arena);
     }
@@ -193,6 +190,11 @@ struct kxc_b200_plan {
         return static_cast<uint8_t*>(arena) + v->offset;
     }
     int eb() const { return tc_elem_bytes(dtype); }
+    // TF32X3: where a value's full fp32 form lies (storage() is its high part when it is stored split)
+    void* plain(int id) {
+        Value* v = find(root_of(id));
+        return static_cast<uint8_t*>(storage(id)) + (x3 && v->split ? 8 * v->elems : 0);
+    }
 };
 
 namespace {
@@ -276,7 +278,7 @@ int sole_consumer(kxc_b200_plan* pl, int id) {
 }
 
 int32_t setup_stem(kxc_b200_plan* pl, Step& st, int N, int C, int H, int W, int O, int KH, int KW, int pad_h, int pad_w,
-                   const void* packed_in, const void* packed_w, TcOutMode out_mode) {
+                   const void* packed_in, const void* packed_w, const void* packed_w_lo, TcOutMode out_mode) {
     const TcDType dt = pl->dtype;
     const int eb = tc_elem_bytes(dt);
     TcParams& p = st.params;
@@ -296,20 +298,29 @@ int32_t setup_stem(kxc_b200_plan* pl, Step& st, int N, int C, int H, int W, int 
     const uint32_t box[4] = {32u, (uint32_t)p.BW, (uint32_t)p.BH, (uint32_t)p.BNI};
     uint8_t* base = const_cast<uint8_t*>(static_cast<const uint8_t*>(packed_in));
     for (int hp = 0; hp < 2; ++hp) {
-        const uint64_t dims[4] = {32, (uint64_t)OW, (uint64_t)((st.Hp - hp + 1) / 2), (uint64_t)N};
+        const uint64_t dims[4] = {32, (uint64_t)OW, (uint64_t)((st.Hp - hp + 1) / 2), (uint64_t)(pl->x3 ? 2 * N : N)};
         const uint64_t strides[3] = {2 * px, (uint64_t)2 * st.Wp * px, (uint64_t)st.Hp * st.Wp * px};
         CUtensorMap m;
         KXC_TRY(tc_make_tmap(&m, dt, 4, base + (size_t)hp * st.Wp * px, dims, strides, box, 32 * eb));
         p.tmA[hp * 2] = m;
         p.tmA[hp * 2 + 1] = m;
     }
+    KXC_TRY(tc_status_word(&p.status));
+    if (pl->x3) return tc_finish_x3(&p, &st.cfg, packed_w, packed_w_lo, O, KH * 32);
     const uint64_t ktot = (uint64_t)KH * 32;
     const uint64_t bdims[2] = {ktot, (uint64_t)O};
     const uint64_t bstr[1] = {ktot * eb};
     const uint32_t bbox[2] = {32u, (uint32_t)bn};
-    KXC_TRY(tc_make_tmap(&p.tmB, dt, 2, const_cast<void*>(packed_w), bdims, bstr, bbox, 32 * eb));
-    KXC_TRY(tc_status_word(&p.status));
-    return KXC_B200_OK;
+    return tc_make_tmap(&p.tmB, dt, 2, const_cast<void*>(packed_w), bdims, bstr, bbox, 32 * eb);
+}
+
+// TF32X3: a contraction's result leaves in the forms its consumers read.
+void bind_x3(kxc_b200_plan* pl, Step& st) {
+    if (st.out_is_graph_output) return;
+    Value* v = pl->find(pl->root_of(st.out));
+    st.params.out_hi = v->split ? static_cast<float*>(pl->storage(st.out)) : nullptr;
+    st.params.out_lo_offset = (long long)v->elems;
+    st.params.out = v->plain ? pl->plain(st.out) : nullptr;
 }
 
 }  // namespace
@@ -568,7 +579,7 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
             PackedWeight pw;
             pw.const_id = n.in[1];
             pw.O = (int)w->shape[0]; pw.C = (int)w->shape[1]; pw.KH = (int)w->shape[2]; pw.KW = (int)w->shape[3];
-            const bool stem = !pl->x3 && is_input(n.in[0]) && st.C <= 4 && n.conv.strides[0] == 2 && n.conv.strides[1] == 2 &&
+            const bool stem = is_input(n.in[0]) && st.C <= 4 && n.conv.strides[0] == 2 && n.conv.strides[1] == 2 &&
                               n.conv.dilation[0] == 1 && n.conv.dilation[1] == 1 && pw.KW <= 8 && st.W >= 8;
             if (stem) {
                 pw.mode = 1;
@@ -750,7 +761,9 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
         Value v;
         v.id = copy_id;
         v.kind = VKind::Intermediate;
-        v.bytes = stem ? (size_t)cv.N * cv.Hp * cv.Wp * 4 * eb : (size_t)cv.N * cv.H * cv.W * cv.cpad * eb;
+        v.elems = stem ? (size_t)cv.N * cv.Hp * cv.Wp * 4 : (size_t)cv.N * cv.H * cv.W * cv.cpad;
+        v.split = pl->x3;
+        v.bytes = v.elems * eb * (pl->x3 ? 2 : 1);
         pl->values[copy_id] = v;
         cv.out = copy_id;
         input_copy[key] = copy_id;
@@ -810,6 +823,20 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
         }
     }
 
+    // ---- TF32X3: the forms every activation is read in ----
+    if (pl->x3) {
+        for (auto& st : pl->steps) {
+            const bool contraction = st.kind == SKind::Conv || st.kind == SKind::Gemm;
+            auto reads = [&](int id, bool split) {
+                Value* v = id == -1 ? nullptr : pl->find(pl->root_of(id));
+                if (v && v->kind == VKind::Intermediate) (split ? v->split : v->plain) = true;
+            };
+            if (st.kind != SKind::InputNHWC && st.kind != SKind::InputStem) reads(st.in0, contraction);
+            reads(st.in1, false);
+            if (!contraction && st.out >= 0 && !st.out_is_graph_output) pl->find(pl->root_of(st.out))->plain = true;
+        }
+    }
+
     // ---- storage sizes and liveness ----
     for (size_t si = 0; si < pl->steps.size(); ++si) {
         Step& st = pl->steps[si];
@@ -824,7 +851,10 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
         touch(st.in1);
         if (st.out != -1 && !st.out_is_graph_output) {
             Value* v = pl->find(st.out);
-            if (v->id >= 0) v->bytes = (size_t)numel_of(v->shape) * eb;
+            if (v->id >= 0) {
+                v->elems = (size_t)numel_of(v->shape);
+                v->bytes = v->elems * eb * (pl->x3 ? (v->split ? 2 : 0) + (v->plain ? 1 : 0) : 1);
+            }
             touch(st.out);
         }
         if (st.out2 != -1) {
@@ -895,17 +925,6 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
             wtop += align_up(w.bytes, 1024);
         }
     }
-    if (pl->x3) {
-        // high / low halves of the largest convolution or dense input
-        size_t half = 0;
-        for (auto& st : pl->steps) {
-            if (st.kind == SKind::Conv) half = std::max(half, align_up((size_t)st.N * st.H * st.W * st.cpad * 4, 1024));
-            if (st.kind == SKind::Gemm) half = std::max(half, align_up((size_t)st.N * pl->weights[st.weight].cpad * 4, 1024));
-        }
-        pl->x3_half_bytes = half;
-        KXC_CUDA_TRY(cudaMalloc(&pl->x3_scratch, std::max<size_t>(2 * half, 1024)));
-    }
-
     // ---- tensor maps and launch parameters ----
     for (auto& st : pl->steps) {
         if (st.kind == SKind::Conv) {
@@ -938,7 +957,7 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
                 KXC_TRY(stem_direct_setup(&st.params, pl->storage(st.in0), pw.ptr, st.N, stem_oh, stem_ow, pw.KH, st.Hp, st.Wp));
                 st.cfg = TcConfig{dt, 64, 64, om};
             } else if (pw.mode == 1) {
-                KXC_TRY(setup_stem(pl, st, st.N, st.C, st.H, st.W, pw.O, pw.KH, pw.KW, st.pad_h, st.pad_w, pl->storage(st.in0), pw.ptr, om));
+                KXC_TRY(setup_stem(pl, st, st.N, st.C, st.H, st.W, pw.O, pw.KH, pw.KW, st.pad_h, st.pad_w, pl->storage(st.in0), pw.ptr, pw.ptr_lo, om));
             } else {
                 if (st.pool.strides[0] != st.pool.strides[1])
                     return fail(KXC_B200_ERR_UNSUPPORTED, "plan: nn_conv2d with different strides in h and w");
@@ -970,34 +989,18 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
                                           st.cpad, pw.O, pw.KH, pw.KW, st.pool.strides[0], st.pad_h, st.pad_w));
                     st.params.out2 = pl->storage(st.out2);
                     st.params.relu2 = st.relu2 ? 1 : 0;
+                } else if (pl->x3) {
+                    KXC_TRY(tc_setup_conv_x3(&st.params, &st.cfg, om, pl->storage(st.in0), pw.ptr, pw.ptr_lo, st.N, st.H, st.W, st.cpad, pw.O,
+                                             pw.KH, pw.KW, st.pool.strides[0], st.pad_h, st.pad_w, st.pool.pool_size[0], st.pool.pool_size[1]));
                 } else
                 KXC_TRY(tc_setup_conv(&st.params, &st.cfg, dt, om, pl->storage(st.in0), pw.ptr, st.N, st.H, st.W, st.cpad, pw.O,
                                       pw.KH, pw.KW, st.pool.strides[0], st.pad_h, st.pad_w, st.pool.pool_size[0], st.pool.pool_size[1]));
             }
             st.params.relu = st.relu ? 1 : 0;
             st.params.round_out_tf32 = (!st.out_is_graph_output && dt == kTcTF32 && !pl->x3) ? 1 : 0;
-            st.params.residual = st.in1 >= 0 ? pl->storage(st.in1) : nullptr;
+            st.params.residual = st.in1 >= 0 ? pl->plain(st.in1) : nullptr;
             st.params.out = st.out_is_graph_output ? nullptr : pl->storage(st.out);
-            if (pl->x3) {
-                // three passes, small terms first; each later pass adds the previous sum through its residual input
-                uint8_t* hi = static_cast<uint8_t*>(pl->x3_scratch);
-                uint8_t* lo = hi + pl->x3_half_bytes;
-                const void* act_hi = st.src_input >= 0 ? pl->storage(st.in0) : hi;  // a graph input's NHWC copy already holds the high part
-                TcConfig c2{};
-                KXC_TRY(tc_setup_conv(&st.params, &st.cfg, dt, om, act_hi, pw.ptr, st.N, st.H, st.W, st.cpad, pw.O, pw.KH, pw.KW,
-                                      st.pool.strides[0], st.pad_h, st.pad_w, st.pool.pool_size[0], st.pool.pool_size[1]));
-                KXC_TRY(tc_setup_conv(&st.params_lohi, &c2, dt, om, lo, pw.ptr, st.N, st.H, st.W, st.cpad, pw.O, pw.KH, pw.KW,
-                                      st.pool.strides[0], st.pad_h, st.pad_w, st.pool.pool_size[0], st.pool.pool_size[1]));
-                KXC_TRY(tc_setup_conv(&st.params_hilo, &c2, dt, om, act_hi, pw.ptr_lo, st.N, st.H, st.W, st.cpad, pw.O, pw.KH, pw.KW,
-                                      st.pool.strides[0], st.pad_h, st.pad_w, st.pool.pool_size[0], st.pool.pool_size[1]));
-                st.params.relu = st.relu ? 1 : 0;
-                st.params.out = st.out_is_graph_output ? nullptr : pl->storage(st.out);
-                st.params.residual = st.params.out;  // pass 3 adds the sum of passes 1 and 2
-                st.params_lohi.out = st.params.out;
-                st.params_lohi.residual = st.in1 >= 0 ? pl->storage(st.in1) : nullptr;
-                st.params_hilo.out = st.params.out;
-                st.params_hilo.residual = st.params.out;
-            }
+            if (pl->x3) bind_x3(pl, st);
             if (st.direct == 3) KXC_TRY(rowstack3x3_bind(&st.params));
             if (st.direct == 5) KXC_TRY(rowstack128_bind(&st.params));
             if (st.direct == 0 && pw.mode == 0 && !st.out_is_graph_output) KXC_TRY(tc_bind_store(&st.params, st.cfg));
@@ -1007,24 +1010,16 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
             TcOutMode om = st.out_is_graph_output ? kOutNHWC_F32 : (dt == kTcBF16 ? kOutNHWC_BF16 : kOutNHWC_F32);
             if (!st.out_is_graph_output && (pw.O % lanes))
                 return fail(KXC_B200_ERR_UNSUPPORTED, "plan: %d dense outputs must be a multiple of %d", pw.O, lanes);
-            KXC_TRY(tc_setup_conv(&st.params, &st.cfg, dt, om, pl->x3 ? pl->x3_scratch : pl->storage(st.in0), pw.ptr, st.N, 1, 1, pw.cpad,
-                                  pw.O, 1, 1, 1, 0, 0, 1, 1));
+            if (pl->x3)
+                KXC_TRY(tc_setup_conv_x3(&st.params, &st.cfg, om, pl->storage(st.in0), pw.ptr, pw.ptr_lo, st.N, 1, 1, pw.cpad, pw.O, 1, 1, 1, 0, 0,
+                                         1, 1));
+            else
+                KXC_TRY(tc_setup_conv(&st.params, &st.cfg, dt, om, pl->storage(st.in0), pw.ptr, st.N, 1, 1, pw.cpad, pw.O, 1, 1, 1, 0, 0, 1, 1));
             st.params.relu = 0;
             st.params.round_out_tf32 = (!st.out_is_graph_output && dt == kTcTF32 && !pl->x3) ? 1 : 0;
             st.params.residual = nullptr;
             st.params.out = st.out_is_graph_output ? nullptr : pl->storage(st.out);
-            if (pl->x3) {
-                uint8_t* hi = static_cast<uint8_t*>(pl->x3_scratch);
-                uint8_t* lo = hi + pl->x3_half_bytes;
-                TcConfig c2{};
-                KXC_TRY(tc_setup_conv(&st.params_lohi, &c2, dt, om, lo, pw.ptr, st.N, 1, 1, pw.cpad, pw.O, 1, 1, 1, 0, 0, 1, 1));
-                KXC_TRY(tc_setup_conv(&st.params_hilo, &c2, dt, om, hi, pw.ptr_lo, st.N, 1, 1, pw.cpad, pw.O, 1, 1, 1, 0, 0, 1, 1));
-                st.params.residual = st.params.out;
-                st.params_lohi.out = st.params.out;
-                st.params_lohi.residual = nullptr;
-                st.params_hilo.out = st.params.out;
-                st.params_hilo.residual = st.params.out;
-            }
+            if (pl->x3) bind_x3(pl, st);
         }
     }
     pl->finalized = true;
@@ -1075,6 +1070,14 @@ static int32_t plan_run_impl(kxc_b200_plan* pl, void** packed_args, void* stream
     return KXC_B200_OK;
 }
 
+// TF32X3: the split form of a value that a pooling or elementwise kernel has written in full.
+static int32_t split_x3(kxc_b200_plan* pl, int id, cudaStream_t s) {
+    Value* v = pl->find(pl->root_of(id));
+    if (!pl->x3 || !v->split) return KXC_B200_OK;
+    float* hi = static_cast<float*>(pl->storage(id));
+    return split_rows(static_cast<const float*>(pl->plain(id)), hi, hi + v->elems, (int64_t)(v->elems / 4), 4, 4, s);
+}
+
 static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream, cudaEvent_t* events) {
     if (!pl || !pl->finalized) return fail(KXC_B200_ERR_INVALID, "plan_run: plan is not finalized");
     if (pl->precision == KXC_B200_PREC_FP32) return run_exact(pl, packed_args, stream, events);
@@ -1108,6 +1111,7 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
                 case 0: KXC_TRY(pack_weights_ohwi(src, w.ptr_lo, dt, w.O, w.C, w.KH, w.KW, w.cpad, s, true)); break;
                 case 2: KXC_TRY(convert_rows(static_cast<const float*>(src), w.ptr_lo, dt, w.O, w.C, w.cpad, s, true)); break;
                 case 3: KXC_TRY(nchw_to_nhwc(src, w.ptr_lo, dt, 1, w.C, w.O, w.cpad, s, true)); break;
+                case 1: KXC_TRY(stem_pack_weights(static_cast<const float*>(src), w.ptr_lo, dt, w.O, w.C, w.KH, w.KW, s, true)); break;
                 default: return fail(KXC_B200_ERR_UNSUPPORTED, "plan: weight layout %d has no TF32X3 form", w.mode);
             }
         }
@@ -1129,11 +1133,18 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
         ++step_index;
         switch (st.kind) {
             case SKind::InputNHWC:
-                KXC_TRY(nchw_to_nhwc(arg_of(st.in0), pl->storage(st.out), dt, st.N, st.C, st.H * st.W, st.cpad, s));
+                if (pl->x3) {
+                    float* hi = static_cast<float*>(pl->storage(st.out));
+                    KXC_TRY(nchw_to_nhwc_split(static_cast<const float*>(arg_of(st.in0)), hi, hi + pl->find(st.out)->elems, st.N, st.C,
+                                               st.H * st.W, st.cpad, s));
+                } else {
+                    KXC_TRY(nchw_to_nhwc(arg_of(st.in0), pl->storage(st.out), dt, st.N, st.C, st.H * st.W, st.cpad, s));
+                }
                 break;
             case SKind::InputStem:
                 KXC_TRY(stem_pack(static_cast<const float*>(arg_of(st.in0)), pl->storage(st.out), dt, st.N, st.C, st.H, st.W, st.Hp,
-                                  st.Wp, st.pad_h, st.pad_w, s));
+                                  st.Wp, st.pad_h, st.pad_w, s,
+                                  pl->x3 ? static_cast<float*>(pl->storage(st.out)) + pl->find(st.out)->elems : nullptr));
                 break;
             case SKind::Conv:
             case SKind::Gemm: {
@@ -1144,31 +1155,7 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
                 p.reverse = (alternate_order && !pl->x3 && (tc_index++ & 1)) ? 1 : 0;
                 tc_finish_params(&p);
                 if (st.weight2 >= 0 && ((reinterpret_cast<uintptr_t>(p.bias2) | reinterpret_cast<uintptr_t>(p.out2)) & 15u)) p.vec_ok = 0;
-                if (pl->x3) {
-                    uint8_t* hi = static_cast<uint8_t*>(pl->x3_scratch);
-                    uint8_t* lo = hi + pl->x3_half_bytes;
-                    const bool gemm = st.kind == SKind::Gemm;
-                    const int cpad = gemm ? pl->weights[st.weight].cpad : st.cpad;
-                    if (st.src_input >= 0) {
-                        KXC_TRY(nchw_to_nhwc(arg_of(st.src_input), lo, dt, st.N, st.C, st.H * st.W, cpad, s, true));
-                    } else {
-                        const int64_t rows = gemm ? (int64_t)st.N : (int64_t)st.N * st.H * st.W;
-                        const float* src = static_cast<const float*>(pl->storage(st.in0));
-                        KXC_TRY(convert_rows(src, hi, dt, rows, cpad, cpad, s, false));
-                        KXC_TRY(convert_rows(src, lo, dt, rows, cpad, cpad, s, true));
-                    }
-                    TcParams q = st.params_lohi;
-                    if (st.out_is_graph_output) q.out = out_ptr;
-                    tc_finish_params(&q);
-                    KXC_TRY(tc_launch(st.cfg, q, s));
-                    q = st.params_hilo;
-                    if (st.out_is_graph_output) { q.out = out_ptr; q.residual = out_ptr; }
-                    tc_finish_params(&q);
-                    KXC_TRY(tc_launch(st.cfg, q, s));
-                    if (st.out_is_graph_output) p.residual = out_ptr;
-                    tc_finish_params(&p);
-                    KXC_TRY(tc_launch(st.cfg, p, s));
-                } else if (st.direct == 4) {
+                if (st.direct == 4) {
                     p.aux_in = arg_of(st.src_input);
                     KXC_TRY(stem_pool_nchw_launch(p, s));
                 } else if (st.direct == 2) {
@@ -1185,19 +1172,22 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
                 break;
             }
             case SKind::MaxPool:
-                KXC_TRY(maxpool_nhwc(pl->storage(st.in0), pl->storage(st.out), dt, st.N, st.H, st.W, st.C, st.OH, st.OW,
+                KXC_TRY(maxpool_nhwc(pl->plain(st.in0), pl->plain(st.out), dt, st.N, st.H, st.W, st.C, st.OH, st.OW,
                                      st.pool.pool_size[0], st.pool.pool_size[1], st.pool.strides[0], st.pool.strides[1],
                                      st.pool.padding[0], st.pool.padding[1], s));
+                KXC_TRY(split_x3(pl, st.out, s));
                 break;
             case SKind::Gap:
-                KXC_TRY(gap_nhwc(pl->storage(st.in0), pl->storage(st.out), dt, st.N, st.H * st.W, st.C, s));
+                KXC_TRY(gap_nhwc(pl->plain(st.in0), pl->plain(st.out), dt, st.N, st.H * st.W, st.C, s));
+                KXC_TRY(split_x3(pl, st.out, s));
                 break;
             case SKind::Eltwise:
-                KXC_TRY(eltwise_nhwc(pl->storage(st.in0), st.in1 >= 0 ? pl->storage(st.in1) : nullptr, pl->storage(st.out), dt,
+                KXC_TRY(eltwise_nhwc(pl->plain(st.in0), st.in1 >= 0 ? pl->plain(st.in1) : nullptr, pl->plain(st.out), dt,
                                      st.numel, st.relu ? 1 : 0, s));
+                KXC_TRY(split_x3(pl, st.out, s));
                 break;
             case SKind::ToNCHW:
-                KXC_TRY(nhwc_to_nchw_f32(pl->storage(st.in0), static_cast<float*>(out_ptr), dt, st.N, st.C, st.H * st.W, s));
+                KXC_TRY(nhwc_to_nchw_f32(pl->plain(st.in0), static_cast<float*>(out_ptr), dt, st.N, st.C, st.H * st.W, s));
                 break;
         }
     }

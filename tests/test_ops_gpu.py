@@ -510,6 +510,18 @@ def test_conv2d_tf32x3_meets_the_reference_tolerance_strictly(ops, rng, case):
         assert max_rel <= 1e-4, f"conv tf32x3 {case} bias={with_bias} res={with_res} relu={relu}: {max_abs:.3e} {max_rel:.3e}"
 
 
+# K blocks of 32 and 64 bytes, a 64-wide tile with one real channel in its last, stride 2, and (128 channels over 184 pixel
+# tiles) the 128-wide tile. The bound is the one above.
+@pytest.mark.parametrize("case", [(2, 8, 9, 7, 65, 3, 3, 1, 1, 1), (2, 16, 10, 11, 130, 3, 3, 2, 1, 1), (30, 32, 28, 28, 128, 1, 1, 1, 0, 1)])
+def test_conv2d_tf32x3_tiles(ops, rng, case):
+    N, C, H, W, O, KH, KW, s, p, d = case
+    x, w, b = conv_inputs(rng, N, C, H, W, O, KH, KW)
+    got = host(ops.nn_conv2d(dev(x), dev(w), dev(b), (s, s), (p, p), (d, d), relu=False, precision="tf32x3"))
+    assert ops.device_status() == 0
+    max_abs, max_rel = ref_metric(got, conv_expect(x, w, b, None, False, s, p, d))
+    assert max_rel <= 1e-4, f"conv tf32x3 {case}: {max_abs:.3e} {max_rel:.3e}"
+
+
 def test_conv2d_config1_tf32x3_vs_single_pass(ops, rng):
     """BASELINE config 1 (U(-1,1) data): the three-pass form is ~1000x closer to the fp32 reference than one pass."""
     x = rng.uniform(-1, 1, (1, 64, 56, 56)).astype(f32)

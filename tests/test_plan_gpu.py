@@ -206,7 +206,7 @@ def test_resnet18_plan(kxc, precision):
     assert got.shape == (N, 1000)
     # bf16: 20 convolutions in 17 launches (the stem kernel reads the fp32 input itself and also does the max pool; each
     # of the three 1x1 downsample convolutions rides in its block's first 3x3 launch) + gap + dense; flatten is a view.
-    # tf32: stem pack + 20 convolutions + max pool + gap + dense. tf32x3: input conversion instead of the stem pack.
+    # tf32 and tf32x3: stem pack + 20 convolutions + max pool + gap + dense.
     assert g.num_launches == (19 if precision == "bf16" else 24)
     hf = rs.build(N, weights)
     exact = ograph.run(hf, [x], workers=8)
