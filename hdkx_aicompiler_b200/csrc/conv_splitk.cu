@@ -1,0 +1,482 @@
+// Implicit-GEMM convolution / dense layer whose reduction is split over the CTAs of a cluster (see conv_tc.cuh for the GEMM
+// view). For launches with fewer tiles than SMs: the deep layers of a small batch are 8 to 64 tiles of 36 to 72 K blocks, and
+// one CTA walks its K blocks at the rate its own operand stream arrives (~50 B/clk), 16 to 24 us for 72 blocks whatever the
+// rest of the chip does. ResNet-18 bf16 on one image: 221 -> 130 us (layer 4: 24 -> 7.5 us per convolution, layer 3: 14.5 -> 7.4).
+//
+// One cluster = one output tile of 128 pixels x BN channels; CTA r of S takes the K blocks [r*K/S, (r+1)*K/S) through the same
+// TMA -> tcgen05.mma pipeline, writes its partial sums into its own (by then idle) operand ring, and after a cluster barrier
+// CTA r adds the r-th S-th of the rows of all S partials over distributed shared memory, in rank order, and applies the
+// epilogue. No partial sum touches global memory, nothing is atomic, and the result does not depend on timing.
+//
+//   warp 0      TMA producer; loads the weights of the first stages before it waits for the previous kernel (weights of a
+//               plan do not come from that kernel), so only the pixels are on the critical path of a layer
+//   warp 1      MMA issuer, TMEM owner
+//   warps 2..9  accumulator -> shared memory, then reduction and epilogue, 8 channels of one pixel per thread and step
+//
+// The shape of the launch (S, BN) comes from choose_split in conv_tc.cu. Waits are bounded as in conv_tc.cu; the cluster
+// barriers are reached by every thread of every CTA whether or not a wait ran out.
+#include "conv_tc.cuh"
+
+#include <cuda_bf16.h>
+
+#include <mutex>
+
+#include "common.cuh"
+#include "conv_epilogue.cuh"
+#include "sm100.cuh"
+
+namespace kxc_b200 {
+namespace {
+
+using namespace sm100;
+
+constexpr int kSplitThreads = 320;
+constexpr int kKB = 128;  // bytes of a K block
+constexpr int kSplitSmem = 227 * 1024 - 2048;
+
+template <int BN, bool kX3>
+struct SplitGeom {
+    static constexpr int kATile = 128 * kKB;
+    static constexpr int kBTile = BN * kKB;
+    static constexpr int kABytes = (kX3 ? 2 : 1) * kATile;
+    static constexpr int kStageBytes = kABytes + (kX3 ? 2 : 1) * kBTile;
+    static constexpr int kStagesRaw = (kSplitSmem - 1024) / kStageBytes;
+    static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
+    static constexpr int kSmemBytes = kStages * kStageBytes + 1024;
+};
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
+    return v;
+}
+
+// byte offset of the 16-byte piece `piece` of row `row` in a partial tile of BN fp32 columns (pieces rotate with the row, so
+// that both a warp of rows and a warp of pieces touch all banks)
+template <int BN>
+__device__ __forceinline__ uint32_t partial_off(int row, int piece) {
+    return (uint32_t)(row * BN * 4 + ((piece ^ (row & 7)) << 4));
+}
+
+// +bias -> +residual -> ReLU -> store of 8 consecutive channels of one pixel
+template <int kOutMode, bool kSplitOut>
+__device__ __forceinline__ void epilogue8(const TcParams& p, float (&f)[8], const float* bias, const void* residual, void* out_ptr, int relu,
+                                          int c0, int n, int oh, int ow) {
+    const int nch = p.Cout - c0 < 8 ? p.Cout - c0 : 8;
+    const size_t pix = ((size_t)n * p.OH + oh) * p.OW + ow;
+    if (bias != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (j < nch) f[j] = __fadd_rn(f[j], __ldg(bias + c0 + j));
+    }
+    if constexpr (kOutMode == kOutNCHW_F32) {
+        const size_t plane = (size_t)p.OH * p.OW;
+        const size_t off = ((size_t)n * p.Cout + c0) * plane + (size_t)oh * p.OW + ow;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (j < nch) {
+                float x = f[j];
+                if (residual != nullptr) x = __fadd_rn(x, __ldg(static_cast<const float*>(residual) + off + j * plane));
+                static_cast<float*>(out_ptr)[off + j * plane] = relu && !(x > 0.0f) ? 0.0f : x;
+            }
+    } else if constexpr (kOutMode == kOutNHWC_BF16) {
+        const bool vec = nch == 8 && (p.Cout & 7) == 0 && p.vec_ok;
+        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(out_ptr) + pix * p.Cout + c0;
+        if (residual != nullptr) {
+            const __nv_bfloat16* res = static_cast<const __nv_bfloat16*>(residual) + pix * p.Cout + c0;
+            if (vec) {
+                const uint4 r = __ldg(reinterpret_cast<const uint4*>(res));
+                const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    f[2 * k] = __fadd_rn(f[2 * k], bf16_lo(w[k]));
+                    f[2 * k + 1] = __fadd_rn(f[2 * k + 1], bf16_hi(w[k]));
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j < nch) f[j] = __fadd_rn(f[j], __bfloat162float(res[j]));
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = relu && !(f[j] > 0.0f) ? 0.0f : f[j];
+        if (vec) {
+            *reinterpret_cast<uint4*>(out) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (j < nch) out[j] = __float2bfloat16_rn(f[j]);
+        }
+    } else {  // kOutNHWC_F32
+        const size_t off = pix * p.Cout + c0;
+        const bool vec = nch == 8 && (p.Cout & 3) == 0 && p.vec_ok;
+        if (residual != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (j < nch) f[j] = __fadd_rn(f[j], __ldg(static_cast<const float*>(residual) + off + j));
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            f[j] = relu && !(f[j] > 0.0f) ? 0.0f : f[j];
+            if (p.round_out_tf32) f[j] = tf32_rne(f[j]);
+        }
+        auto store = [&](float* dst, const float (&v)[8], bool wide) {
+            if (wide) {
+                reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
+                reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j < nch) dst[j] = v[j];
+            }
+        };
+        if constexpr (kSplitOut) {
+            if (p.out_hi != nullptr) {
+                float h[8], l[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    h[j] = tf32_rne(f[j]);
+                    l[j] = tf32_low_part(f[j], h[j]);
+                }
+                store(p.out_hi + off, h, nch == 8 && (p.Cout & 3) == 0);
+                store(p.out_hi + p.out_lo_offset + off, l, nch == 8 && (p.Cout & 3) == 0);
+            }
+            if (out_ptr == nullptr) return;
+        }
+        store(static_cast<float*>(out_ptr) + off, f, vec);
+    }
+}
+
+// kDual, kX3: as in conv_tc.cu (second output through tmB2 / out2; high and low operand parts).
+template <MmaKind kKind, int BN, int kOutMode, bool kDual, bool kX3>
+__global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __grid_constant__ TcParams p) {
+    using G = SplitGeom<BN, kX3>;
+    static_assert(!(kDual && kX3), "one of the two");
+    static_assert((kDual ? 2 : 1) * 128 * BN * 4 <= G::kStages * G::kStageBytes, "the partial sums reuse the operand ring");
+    constexpr int kStages = G::kStages;
+    constexpr uint32_t kTmemCols = (kDual || kX3 ? 2 : 1) * BN;
+    constexpr uint32_t kFmt = kKind == MmaKind::F16 ? kFmtBF16 : kFmtTF32;
+    constexpr uint32_t kIdesc = make_instr_desc(kFmt, kAccF32, BN, 128u);
+    [[maybe_unused]] constexpr uint32_t kIdescWide = make_instr_desc(kFmt, kAccF32, 2 * BN <= 256 ? 2 * BN : 256, 128u);
+
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t bar_full[kStages];
+    __shared__ __align__(8) uint64_t bar_empty[kStages];
+    __shared__ __align__(8) uint64_t bar_acc;
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int abort_flag;
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const int rank = (int)cluster_cta_rank();
+    const int S = p.split;
+    const int tile = (int)blockIdx.x / S;
+
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < kStages; ++s) {
+            mbar_init(smem_u32(&bar_full[s]), 1);
+            mbar_init(smem_u32(&bar_empty[s]), 1);
+        }
+        mbar_init(smem_u32(&bar_acc), 1);
+        mbar_fence_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(&tmem_base_slot), kTmemCols);
+        tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = tmem_base_slot;
+    volatile int* abort_ptr = &abort_flag;
+    pdl_launch_dependents();
+
+    const int kb_main = p.taps_h * p.taps_w * p.cblocks;
+    const int kb_all = kb_main + (kDual ? p.cblocks : 0);
+    // The second output's few blocks go to the last rank alone: its sum is formed in the order of a launch of its own, and the
+    // main sum's parts are those of a launch without it (bit-identical either way).
+    const int kb0 = rank * kb_main / S, kb1 = rank == S - 1 ? kb_all : (rank + 1) * kb_main / S;
+    const int ct = tile % p.tiles_c;
+    int r = tile / p.tiles_c;
+    const int tw = r % p.tiles_w; r /= p.tiles_w;
+    const int th = r % p.tiles_h;
+    const int tn = r / p.tiles_h;
+    const int ow0 = tw * p.BW, oh0 = th * p.BH, n0 = tn * p.BNI;
+    const int rows_used = p.BW * p.BH * p.BNI;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            tma_prefetch_desc(&p.tmB);
+            tma_prefetch_desc(&p.tmA[0]);
+            if constexpr (kDual || kX3) tma_prefetch_desc(&p.tmB2);
+            const uint32_t tx_bytes = (uint32_t)((kX3 ? 2 : 1) * (rows_used * kKB + G::kBTile));
+            auto load_weights = [&](int kb, int stage) {
+                const uint32_t full = smem_u32(&bar_full[stage]);
+                const uint32_t dst = ring + (uint32_t)stage * G::kStageBytes + G::kABytes;
+                mbar_arrive_expect_tx(full, tx_bytes);
+                if (kDual && kb >= kb_main) {
+                    tma_load_2d(dst, &p.tmB2, full, (kb - kb_main) * p.kb_elems, ct * BN);
+                } else {
+                    tma_load_2d(dst, &p.tmB, full, kb * p.kb_elems, ct * BN);
+                    if constexpr (kX3) tma_load_2d(dst + G::kBTile, &p.tmB2, full, kb * p.kb_elems, ct * BN);
+                }
+            };
+            auto load_pixels = [&](int kb, int stage) {
+                int cb, kh, kw;
+                if (kDual && kb >= kb_main) {  // the 1x1 convolution reads the centre tap
+                    cb = kb - kb_main;
+                    kh = p.taps_h / 2;
+                    kw = p.taps_w / 2;
+                } else {
+                    const int tap = kb / p.cblocks;
+                    cb = kb - tap * p.cblocks;
+                    kh = tap / p.taps_w;
+                    kw = tap - kh * p.taps_w;
+                }
+                const int dh = kh * p.dil_h - p.pad_h, dw = kw * p.dil_w - p.pad_w;
+                int map = 0, ch = dh, cw = dw;
+                if (p.stride == 2) {
+                    const int hp = dh & 1, wp = dw & 1;
+                    map = hp * 2 + wp;
+                    ch = (dh - hp) >> 1;
+                    cw = (dw - wp) >> 1;
+                }
+                const uint32_t full = smem_u32(&bar_full[stage]);
+                const uint32_t dst = ring + (uint32_t)stage * G::kStageBytes;
+                tma_load_4d(dst, &p.tmA[map], full, cb * p.kb_elems, ow0 + cw, oh0 + ch, n0);
+                if constexpr (kX3) tma_load_4d(dst + G::kATile, &p.tmA[map], full, cb * p.kb_elems, ow0 + cw, oh0 + ch, n0 + p.N);
+            };
+            const int early = p.weights_ready ? (kb1 - kb0 < kStages ? kb1 - kb0 : kStages) : 0;
+            for (int i = 0; i < early; ++i) load_weights(kb0 + i, i);
+            pdl_wait();  // the pixels come from the previous kernel
+            for (int i = 0; i < early; ++i) load_pixels(kb0 + i, i);
+            int stage = early == kStages ? 0 : early;
+            uint32_t phase = early == kStages ? 1u : 0u;
+            for (int kb = kb0 + early; kb < kb1; ++kb) {
+                if (!mbar_wait_bounded(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_ptr)) break;
+                load_weights(kb, stage);
+                load_pixels(kb, stage);
+                if (++stage == kStages) { stage = 0; phase ^= 1u; }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            int stage = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int kb = kb0; kb < kb1; ++kb) {
+                if (!mbar_wait_bounded(smem_u32(&bar_full[stage]), phase, abort_ptr)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after_sync();
+                const bool second = kDual && kb >= kb_main;
+                const bool first_of_sum = kb == kb0 || (kDual && kb == kb_main);
+                const uint32_t d = tmem_base + (second ? (uint32_t)BN : 0u);
+                const uint32_t a_addr = ring + (uint32_t)stage * G::kStageBytes;
+                const uint64_t a_desc = make_smem_desc(a_addr, kKB), b_desc = make_smem_desc(a_addr + G::kABytes, kKB);
+#pragma unroll
+                for (int k = 0; k < kKB / 32; ++k) {
+                    const uint64_t a_k = a_desc + (uint64_t)(2 * k), b_k = b_desc + (uint64_t)(2 * k);
+                    const uint32_t accumulate = first_of_sum && k == 0 ? 0u : 1u;
+                    if constexpr (kX3) {
+                        umma<kKind>(d, a_k, b_k, kIdescWide, accumulate);
+                        umma<kKind>(d + (uint32_t)BN, a_k + (uint64_t)(G::kATile >> 4), b_k, kIdesc, 1u);
+                    } else {
+                        umma<kKind>(d, a_k, b_k, kIdesc, accumulate);
+                    }
+                }
+                umma_commit(smem_u32(&bar_empty[stage]));
+                if (++stage == kStages) { stage = 0; phase ^= 1u; }
+            }
+            if (ok) umma_commit(smem_u32(&bar_acc));
+        }
+    } else {
+        // this CTA's partial sums into its ring: every load has landed and every MMA has read it once bar_acc completes
+        const int quad = warp & 3, half = (warp - 2) >> 2;
+        const int row = quad * 32 + lane;
+        bool ok = mbar_wait_bounded(smem_u32(&bar_acc), 0, abort_ptr);
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) {
+            tc_fence_after_sync();
+#pragma unroll 1
+            for (int a = 0; a < (kDual ? 2 : 1); ++a) {
+                if (a == 1 && rank != S - 1) continue;
+#pragma unroll 1
+                for (int i = 0; i < BN / 64; ++i) {
+                    const int col = half * (BN / 2) + i * 32;
+                    const uint32_t t_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN + col);
+                    uint32_t v[32];
+                    tmem_ld_32x32(t_addr, v);
+                    if constexpr (kX3) {
+                        uint32_t u[32];
+                        tmem_ld_32x32(t_addr + (uint32_t)BN, u);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j])));
+                    } else {
+                        tmem_ld_wait();
+                    }
+#pragma unroll
+                    for (int g = 0; g < 8; ++g)
+                        st_shared_v4(ring + (uint32_t)(a * 128 * BN * 4) + partial_off<BN>(row, (col >> 2) + g),
+                                     make_uint4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]));
+                }
+            }
+            tc_fence_before_sync();
+        }
+    }
+    __syncwarp();
+    cluster_sync_all();  // the partial sums of all ranks are in place
+    // Every thread: one step per 8 channels of a pixel. The partial sums of a step are fetched together; a CTA's last fetch is
+    // followed by its arrival at the second barrier, so the epilogue's arithmetic and stores are not waited for by the others.
+    const bool live = warp >= 2 && !*abort_ptr;
+    if (live) pdl_wait();  // residual reads and output writes must not overtake earlier kernels
+    const int rows = (128 + S - 1) / S;
+    constexpr int kPieces = BN / 8;
+    const int box_hw = p.BH * p.BW;
+    const int items = rows * kPieces;
+    const int steps = (items * (kDual ? 2 : 1) + 255) / 256;
+#pragma unroll 1
+    for (int step = 0; step < steps; ++step) {
+        const int idx = step * 256 + (int)threadIdx.x - 64;
+        const int a = kDual ? idx / items : 0;
+        const int it = idx - a * items;
+        // neighbouring threads: neighbouring channels of a pixel (NHWC) or neighbouring pixels (NCHW)
+        const int piece = kOutMode == kOutNCHW_F32 ? it / rows : it % kPieces;
+        const int row = rank * rows + (kOutMode == kOutNCHW_F32 ? it % rows : it / kPieces);
+        const int n_l = row / box_hw;
+        const int rem = row - n_l * box_hw;
+        const int h_l = rem / p.BW;
+        const int n = n0 + n_l, oh = oh0 + h_l, ow = ow0 + rem - h_l * p.BW;
+        const int c0 = ct * BN + piece * 8;
+        const bool mine = live && idx < items * (kDual ? 2 : 1) && row < rows_used && n < p.N && oh < p.OH && ow < p.OW && c0 < p.Cout;
+        float f[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        if (mine) {
+            const uint32_t base = ring + (uint32_t)(a * 128 * BN * 4);
+            const uint32_t off0 = partial_off<BN>(row, 2 * piece), off1 = partial_off<BN>(row, 2 * piece + 1);
+            const int s_first = a == 1 ? S - 1 : 0;
+            float4 x[kMaxSplit], y[kMaxSplit];
+#pragma unroll
+            for (int s = 0; s < kMaxSplit; ++s) {
+                if (s < s_first || s >= S) continue;
+                x[s] = ld_cluster_f4(map_to_cta(base + off0, (uint32_t)s));
+                y[s] = ld_cluster_f4(map_to_cta(base + off1, (uint32_t)s));
+            }
+#pragma unroll
+            for (int s = 0; s < kMaxSplit; ++s) {
+                if (s < s_first || s >= S) continue;
+                f[0] += x[s].x; f[1] += x[s].y; f[2] += x[s].z; f[3] += x[s].w;
+                f[4] += y[s].x; f[5] += y[s].y; f[6] += y[s].z; f[7] += y[s].w;
+            }
+        }
+        if (step == steps - 1) {
+            __syncwarp();
+            cluster_arrive();
+        }
+        if (mine) {
+            if (kDual && a == 1)
+                epilogue8<kOutMode, false>(p, f, p.bias2, nullptr, p.out2, p.relu2, c0, n, oh, ow);
+            else
+                epilogue8<kOutMode, kX3>(p, f, p.bias, p.residual, p.out, p.relu, c0, n, oh, ow);
+        }
+    }
+    if (*abort_ptr) {  // loads already issued may still be landing (see conv_tc.cu)
+        const uint64_t t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+    }
+    __syncwarp();
+    cluster_wait();  // no CTA's shared memory goes while another still reads it
+    tc_fence_after_sync();
+    if (warp == 1) {
+        __syncwarp();
+        tmem_dealloc(tmem_base, kTmemCols);
+    }
+    if (threadIdx.x == 0 && *abort_ptr && p.status != nullptr) atomicExch(p.status, KXC_B200_ERR_DEVICE_WAIT);
+}
+
+template <MmaKind kKind, int BN, int kOutMode, bool kDual, bool kX3>
+int32_t launch_split(const TcParams& p, cudaStream_t s) {
+    using G = SplitGeom<BN, kX3>;
+    auto kernel = conv_splitk_kernel<kKind, BN, kOutMode, kDual, kX3>;
+    static PerDeviceOnce smem_once;
+    KXC_TRY(smem_opt_in(smem_once, kernel, G::kSmemBytes));
+    const int tiles = p.tiles_c * p.tiles_w * p.tiles_h * p.tiles_n;
+    KXC_CUDA_TRY(launch_kernel(kernel, dim3((unsigned)(tiles * p.split)), dim3(kSplitThreads), G::kSmemBytes, s, /*pdl=*/true, p.split, p));
+    return check_launch("conv_splitk_kernel");
+}
+
+template <MmaKind kKind, int kOutMode, bool kX3>
+int32_t launch_by_width(const TcConfig& cfg, const TcParams& p, cudaStream_t s) {
+    if constexpr (kKind == MmaKind::F16 && kOutMode == kOutNHWC_BF16) {
+        if (cfg.dual) {
+            return cfg.bn == 64 ? launch_split<kKind, 64, kOutMode, true, false>(p, s) : launch_split<kKind, 128, kOutMode, true, false>(p, s);
+        }
+    }
+    if (cfg.dual) return fail(KXC_B200_ERR_INVALID, "split-reduction conv: no two-output form for this configuration");
+    if constexpr (!kX3) {
+        if (cfg.bn == 256) return launch_split<kKind, 256, kOutMode, false, kX3>(p, s);
+    }
+    return cfg.bn == 64 ? launch_split<kKind, 64, kOutMode, false, kX3>(p, s) : launch_split<kKind, 128, kOutMode, false, kX3>(p, s);
+}
+
+}  // namespace
+
+int tc_split_capacity(int split) {
+    if (split < 2 || split > kMaxSplit) return 0;
+    static std::mutex mu;
+    static int known[PerDeviceOnce::kMaxDevices][kMaxSplit + 1] = {};  // clusters + 1
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= PerDeviceOnce::kMaxDevices) return 0;
+    std::lock_guard<std::mutex> lock(mu);
+    int& n = known[dev][split];
+    if (n == 0) {
+        using G = SplitGeom<64, false>;  // every form of the kernel takes an SM to itself
+        auto kernel = conv_splitk_kernel<MmaKind::F16, 64, kOutNHWC_BF16, false, false>;
+        cudaLaunchConfig_t lc = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)split;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        lc.gridDim = dim3((unsigned)(kNumSMs / split * split));
+        lc.blockDim = dim3(kSplitThreads);
+        lc.dynamicSmemBytes = G::kSmemBytes;
+        lc.attrs = attr;
+        lc.numAttrs = 1;
+        int found = 0;
+        if (cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, G::kSmemBytes) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&found, kernel, &lc) != cudaSuccess || found < 0) {
+            cudaGetLastError();
+            found = 0;
+        }
+        n = (found < kNumSMs / split ? found : kNumSMs / split) + 1;
+    }
+    return n - 1;
+}
+
+int32_t tc_launch_split(const TcConfig& cfg, const TcParams& p, cudaStream_t s) {
+    if (p.split < 2 || p.split > kMaxSplit || (cfg.bn != 64 && cfg.bn != 128 && (cfg.bn != 256 || cfg.x3 || cfg.dual)) || cfg.kb_bytes != kKB)
+        return fail(KXC_B200_ERR_INVALID, "split-reduction conv: %d parts, %d channels, %d-byte K blocks", p.split, cfg.bn, cfg.kb_bytes);
+    if (cfg.dtype == kTcBF16) {
+        switch (cfg.out_mode) {
+            case kOutNHWC_BF16: return launch_by_width<MmaKind::F16, kOutNHWC_BF16, false>(cfg, p, s);
+            case kOutNHWC_F32: return launch_by_width<MmaKind::F16, kOutNHWC_F32, false>(cfg, p, s);
+            case kOutNCHW_F32: return launch_by_width<MmaKind::F16, kOutNCHW_F32, false>(cfg, p, s);
+            default: break;
+        }
+    } else if (cfg.dtype == kTcTF32) {
+        switch (cfg.out_mode) {
+            case kOutNHWC_F32:
+                return cfg.x3 ? launch_by_width<MmaKind::TF32, kOutNHWC_F32, true>(cfg, p, s) : launch_by_width<MmaKind::TF32, kOutNHWC_F32, false>(cfg, p, s);
+            case kOutNCHW_F32:
+                return cfg.x3 ? launch_by_width<MmaKind::TF32, kOutNCHW_F32, true>(cfg, p, s) : launch_by_width<MmaKind::TF32, kOutNCHW_F32, false>(cfg, p, s);
+            default: break;
+        }
+    }
+    return fail(KXC_B200_ERR_INVALID, "split-reduction conv: output mode %d does not fit dtype %d", (int)cfg.out_mode, (int)cfg.dtype);
+}
+
+}  // namespace kxc_b200

@@ -578,6 +578,7 @@ int32_t launch_by_kb(const TcConfig& cfg, const TcParams& p, cudaStream_t s) {
 }  // namespace
 
 int32_t tc_launch(const TcConfig& cfg, const TcParams& p, cudaStream_t stream) {
+    if (p.split > 1) return tc_launch_split(cfg, p, stream);
     switch (cfg.dtype) {
         case kTcBF16: return launch_by_kb<MmaKind::F16>(cfg, p, stream);
         case kTcTF32: return launch_by_kb<MmaKind::TF32>(cfg, p, stream);
@@ -692,6 +693,55 @@ int32_t tc_bind_store(TcParams* p, const TcConfig& cfg) {
     return KXC_B200_OK;
 }
 
+namespace {
+// The weights of a split launch: boxes of cfg->bn rows x one K block of `k_elems` elements per output channel.
+int32_t weight_map(CUtensorMap* m, const TcConfig* cfg, const TcParams* p, const void* w, int k_elems) {
+    const uint64_t dims[2] = {(uint64_t)k_elems, (uint64_t)p->Cout};
+    const uint64_t strides[1] = {(uint64_t)k_elems * tc_elem_bytes(cfg->dtype)};
+    const uint32_t box[2] = {(uint32_t)p->kb_elems, (uint32_t)cfg->bn};
+    return tc_make_tmap(m, cfg->dtype, 2, const_cast<void*>(w), dims, strides, box, 128);
+}
+
+// Whether a set-up launch (tile width, store form and so on already chosen for the persistent kernel) is better off with its
+// reduction split over a cluster, and the set-up of that form. Modelled in cycles: a K block of 128 bytes per row costs what
+// its stage takes to arrive at ~50 B/clk per SM (x3: what its instructions take); ~1500 cycles per launch for filling the
+// pipeline and the epilogue, as much again for the cluster barriers and the exchange. It has to gain 10 %. A launch is kept to
+// the clusters that the chip holds at once (a dense layer of 16 tiles in clusters of eight that did not all fit: 8.8 -> 12 us).
+int32_t choose_split(TcParams* p, TcConfig* cfg, const void* w, const void* w_lo, int k_elems) {
+    p->split = 0;
+    if (cfg->dtype == kTcS8 || cfg->kb_bytes != 128) return KXC_B200_OK;
+    const long long m_tiles = (long long)p->tiles_w * p->tiles_h * p->tiles_n;
+    const int kb = p->taps_h * p->taps_w * p->cblocks;
+    if (kb < 12) return KXC_B200_OK;  // two or three microseconds as it is
+    auto stage_cycles = [&](int bn) {
+        return cfg->x3 ? (bn == 64 ? 950 : 1400) : (bn == 64 ? 490 : (bn == 128 ? 655 : (bn == 256 && cfg->ctas == 1 ? 980 : 800)));
+    };
+    const long long group = (long long)cfg->ctas * cfg->mt;
+    const long long items = p->tiles_c * ((m_tiles + group - 1) / group), slots = kNumSMs / cfg->ctas;
+    const long long whole = (items + slots - 1) / slots * kb * (cfg->mt == 2 ? 980 : stage_cycles(cfg->bn)) + 1500;
+    long long best = whole * 9 / 10;
+    int split = 0, width = 0;
+    for (int bn = 64; bn <= 256 && (bn == 64 || bn / 2 < p->Cout) && !(bn == 256 && cfg->x3); bn *= 2) {
+        const long long tiles = m_tiles * ((p->Cout + bn - 1) / bn);
+        for (int s = 2; s <= kMaxSplit && tiles * s <= kNumSMs; ++s) {
+            if (tiles > tc_split_capacity(s)) continue;
+            const long long span = (long long)((kb + s - 1) / s) * (bn == 256 ? 980 : stage_cycles(bn)) + 3000;
+            if (span < best) {
+                best = span;
+                split = s;
+                width = bn;
+            }
+        }
+    }
+    if (split == 0) return KXC_B200_OK;
+    p->split = split;
+    cfg->bn = width; cfg->ctas = 1; cfg->mt = 1;
+    p->tiles_c = (p->Cout + width - 1) / width;
+    KXC_TRY(weight_map(&p->tmB, cfg, p, w, k_elems));
+    return w_lo != nullptr ? weight_map(&p->tmB2, cfg, p, w_lo, k_elems) : KXC_B200_OK;
+}
+}  // namespace
+
 bool tc_dual_applicable(TcDType dtype, TcOutMode out_mode, int cpad, int Cout, int KH, int KW, int stride, int pad_h, int pad_w,
                         int dil_h, int dil_w) {
     // the second output's only tap must be the main filter's centre tap
@@ -702,6 +752,15 @@ bool tc_dual_applicable(TcDType dtype, TcOutMode out_mode, int cpad, int Cout, i
 int32_t tc_setup_dual(TcParams* p, TcConfig* cfg, const void* act_nhwc, const void* w_packed, const void* w2_packed, int N,
                       int H, int W, int cpad, int Cout, int KH, int KW, int stride, int pad_h, int pad_w) {
     KXC_TRY(tc_setup_conv(p, cfg, kTcBF16, kOutNHWC_BF16, act_nhwc, w_packed, N, H, W, cpad, Cout, KH, KW, stride, pad_h, pad_w, 1, 1));
+    if (p->split > 1) {  // the main sum's split is that of a launch without the second output (same bits)
+        cfg->dual = 1;
+        if (cfg->bn > 128) {  // (no 256-wide form of it: two narrower tiles, the same sums)
+            cfg->bn = 128;
+            p->tiles_c = (Cout + 127) / 128;
+            KXC_TRY(weight_map(&p->tmB, cfg, p, w_packed, KH * KW * cpad));
+        }
+        return weight_map(&p->tmB2, cfg, p, w2_packed, cpad);
+    }
     // The two accumulators of a buffer share TMEM: 128-wide tiles (two buffers of 2 x 128 columns), single CTAs. When
     // that leaves a launch with a second, mostly empty wave and 192-wide tiles fit one wave (256 -> 512 channels at 128
     // images: 196 tiles against 147 for 148 SMs), the 192-wide form is taken: one buffer of 2 x 192 columns, so the
@@ -714,7 +773,7 @@ int32_t tc_setup_dual(TcParams* p, TcConfig* cfg, const void* act_nhwc, const vo
         static const bool model = [] { const char* e = getenv("KXC_B200_TILE_MODEL"); return !(e != nullptr && e[0] == '0'); }();
         if (model && p->kb_elems * 2 == 128 && waves(t192) == 1 && waves(t128) >= 2) bn = 192;  // (192-wide tiles need 128-byte K blocks)
     }
-    cfg->bn = bn; cfg->ctas = 1; cfg->dual = 1;
+    cfg->bn = bn; cfg->ctas = 1; cfg->mt = 1; cfg->dual = 1;
     p->tiles_c = (Cout + bn - 1) / bn;
     const uint64_t ktot = (uint64_t)KH * KW * cpad;
     const uint64_t bdims[2] = {ktot, (uint64_t)Cout};
@@ -723,8 +782,7 @@ int32_t tc_setup_dual(TcParams* p, TcConfig* cfg, const void* act_nhwc, const vo
     KXC_TRY(tc_make_tmap(&p->tmB, kTcBF16, 2, const_cast<void*>(w_packed), bdims, bstrides, bbox, 128));
     const uint64_t b2dims[2] = {(uint64_t)cpad, (uint64_t)Cout};
     const uint64_t b2strides[1] = {(uint64_t)cpad * 2};
-    KXC_TRY(tc_make_tmap(&p->tmB2, kTcBF16, 2, const_cast<void*>(w2_packed), b2dims, b2strides, bbox, 128));
-    return KXC_B200_OK;
+    return tc_make_tmap(&p->tmB2, kTcBF16, 2, const_cast<void*>(w2_packed), b2dims, b2strides, bbox, 128);
 }
 
 int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_mode, const void* act_nhwc,
@@ -835,7 +893,7 @@ int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_m
     } else {
         KXC_TRY(tc_status_word(&p->status));
     }
-    return KXC_B200_OK;
+    return choose_split(p, cfg, w_packed, nullptr, KH * KW * cpad);
 }
 
 int32_t tc_finish_x3(TcParams* p, TcConfig* cfg, const void* w_hi, const void* w_lo, int Cout, int k_elems) {
@@ -850,7 +908,8 @@ int32_t tc_finish_x3(TcParams* p, TcConfig* cfg, const void* w_hi, const void* w
     const uint64_t bstrides[1] = {ktot * 4};
     const uint32_t bbox[2] = {(uint32_t)p->kb_elems, (uint32_t)bn};
     KXC_TRY(tc_make_tmap(&p->tmB, kTcTF32, 2, const_cast<void*>(w_hi), bdims, bstrides, bbox, cfg->kb_bytes));
-    return tc_make_tmap(&p->tmB2, kTcTF32, 2, const_cast<void*>(w_lo), bdims, bstrides, bbox, cfg->kb_bytes);
+    KXC_TRY(tc_make_tmap(&p->tmB2, kTcTF32, 2, const_cast<void*>(w_lo), bdims, bstrides, bbox, cfg->kb_bytes));
+    return choose_split(p, cfg, w_hi, w_lo, k_elems);
 }
 
 int32_t tc_setup_conv_x3(TcParams* p, TcConfig* cfg, TcOutMode out_mode, const void* act_hi, const void* w_hi, const void* w_lo, int N,

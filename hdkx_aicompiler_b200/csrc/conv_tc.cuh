@@ -71,6 +71,8 @@ struct alignas(64) TcParams {
     // high part at out_hi and the low part out_lo_offset elements after it (null: not wanted). `out` may then be null.
     float* out_hi;
     long long out_lo_offset;
+    int split;                   // 2..kMaxSplit: the reduction is split over clusters of that many CTAs (conv_splitk.cu); 0: it is not
+    int weights_ready;           // the packed weights were written long before this launch: they may be read ahead of its predecessor's end
 };
 
 struct TcConfig {
@@ -94,6 +96,12 @@ inline void tc_finish_params(TcParams* p) {
 
 // Launches the persistent kernel for the given configuration. `p` must be fully populated.
 int32_t tc_launch(const TcConfig& cfg, const TcParams& p, cudaStream_t stream);
+
+// conv_splitk.cu: launches with p.split > 1 (tc_launch passes them on).
+constexpr int kMaxSplit = 8;  // the largest portable cluster
+int32_t tc_launch_split(const TcConfig& cfg, const TcParams& p, cudaStream_t stream);
+// Clusters of `split` CTAs that the current device holds at once (whole GPCs' worth: fewer than 148 / split).
+int tc_split_capacity(int split);
 
 // Tile box selection: maximise the fraction of the 128 rows that are real output pixels.
 void tc_pick_tile(int N, int OH, int OW, int* BW, int* BH, int* BNI);

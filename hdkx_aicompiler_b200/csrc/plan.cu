@@ -1152,6 +1152,7 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
                 p.bias = st.bias_const >= 0 ? static_cast<const float*>(arg_of(st.bias_const)) : nullptr;
                 p.bias2 = st.bias2_const >= 0 ? static_cast<const float*>(arg_of(st.bias2_const)) : nullptr;
                 if (st.out_is_graph_output) p.out = out_ptr;
+                p.weights_ready = 1;  // packed by ordinary launches ahead of the run's first kernel
                 p.reverse = (alternate_order && !pl->x3 && (tc_index++ & 1)) ? 1 : 0;
                 tc_finish_params(&p);
                 if (st.weight2 >= 0 && ((reinterpret_cast<uintptr_t>(p.bias2) | reinterpret_cast<uintptr_t>(p.out2)) & 15u)) p.vec_ok = 0;
@@ -1325,6 +1326,7 @@ extern "C" int32_t kxc_b200_plan_launch_info(kxc_b200_plan* pl, int32_t index, c
             snprintf(buf, sizeof(buf), "%s c%d h%d w%d -> o%d k%dx%d s%d%s%s tile %dx%dx%d bn%d%s", st.direct == 4 ? "conv_stem_pool_nchw" : st.direct == 2 ? (st.fused_pool ? "conv_stem_pool" : "conv_stem_direct") : (st.direct == 3 ? "conv_rowstack" : (st.direct == 5 ? "conv_rowstack128" : (st.direct ? "conv_direct" : "conv_igemm"))), w.C, st.H, st.W, w.O, w.KH, w.KW,
                      p.stride, st.in1 >= 0 ? " +res" : "", st.relu ? " +relu" : "", p.BNI, p.BH, p.BW, st.cfg.bn,
                      st.cfg.ctas == 2 ? " pair" : (st.weight2 >= 0 ? " +1x1 second output" : (st.cfg.mt == 2 ? " x2 tiles" : "")));
+            if (p.split > 1) snprintf(buf + strlen(buf), sizeof(buf) - strlen(buf), " split%d", p.split);
             break;
         }
         case SKind::Gemm: {
@@ -1332,6 +1334,7 @@ extern "C" int32_t kxc_b200_plan_launch_info(kxc_b200_plan* pl, int32_t index, c
             fl = 2.0 * st.N * (double)w.O * w.C;
             by = (double)st.N * w.C * eb + (double)w.bytes + (double)st.N * w.O * (st.out_is_graph_output ? 4.0 : eb) + 4.0 * w.O;
             snprintf(buf, sizeof(buf), "dense_igemm m%d k%d -> n%d bn%d%s", st.N, w.C, w.O, st.cfg.bn, st.cfg.ctas == 2 ? " pair" : "");
+            if (st.params.split > 1) snprintf(buf + strlen(buf), sizeof(buf) - strlen(buf), " split%d", st.params.split);
             break;
         }
         case SKind::MaxPool:

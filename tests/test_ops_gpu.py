@@ -227,6 +227,23 @@ def test_conv2d_argument_errors(ops):
         ops.nn_conv2d(x, torch.zeros(2, 3, 1, 1, device="cuda"))
 
 
+# Reductions split over clusters of two to eight CTAs, 64 to 256 channels wide (conv_splitk.cu): ragged pixels and channels,
+# stride 2, dilation 2, K ranges that do not divide evenly. Bounds: those of the two tests of the whole reductions.
+@pytest.mark.parametrize("precision,rounder", [("tf32", port.round_tf32), ("bf16", port.round_bf16), ("tf32x3", None)])
+@pytest.mark.parametrize("case", [(1, 128, 9, 9, 64, 3, 3, 1, 1, 1), (9, 128, 13, 15, 100, 3, 3, 1, 1, 1), (2, 192, 21, 19, 70, 3, 3, 2, 1, 1),
+                                  (33, 128, 14, 13, 100, 3, 3, 1, 2, 2), (5, 1024, 7, 7, 40, 1, 1, 1, 0, 1), (25, 256, 14, 14, 264, 3, 3, 2, 1, 1)])
+def test_conv2d_split_reduction(ops, rng, case, precision, rounder):
+    N, C, H, W, O, KH, KW, s, p, d = case
+    x, w, b = conv_inputs(rng, N, C, H, W, O, KH, KW)
+    oh, ow = port.conv_out_dim(H, KH, s, p, d), port.conv_out_dim(W, KW, s, p, d)
+    res = rng.uniform(-1, 1, (N, O, oh, ow)).astype(f32)
+    got = host(ops.nn_conv2d(dev(x), dev(w), dev(b), (s, s), (p, p), (d, d), residual=dev(res), relu=True, precision=precision))
+    assert ops.device_status() == 0
+    max_abs, max_rel = ref_metric(got, conv_expect(x, w, b, res, True, s, p, d, rounder))
+    bound = 1e-4 if rounder is None else 2e-5 * max(1.0, np.sqrt(C * KH * KW) / 8)
+    assert min(max_abs, max_rel) <= bound, f"split conv {precision} {case}: {max_abs:.3e} {max_rel:.3e}"
+
+
 # ---------------------------------------------------------------- int8 conv + requantize
 def s8_inputs(rng, N, C, H, W, O, KH, KW):
     x = np.clip(np.round(rng.normal(0, 32, (N, C, H, W))), -128, 127).astype(np.int8)
