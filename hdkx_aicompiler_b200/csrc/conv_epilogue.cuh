@@ -124,8 +124,9 @@ __device__ __forceinline__ void epilogue_chunk(const TcParams& p, const uint32_t
         requant_chunk(p, v, c0, nch, qw);
         int8_t* out = static_cast<int8_t*>(p.out);
         if constexpr (kOutMode == kOutNHWC_S8) {
-            int8_t* dst = out + pix * p.Cout + c0;
-            if (nch == 32 && (p.Cout & 15) == 0 && p.vec_ok) {
+            const int pitch = p.out_pitch != 0 ? p.out_pitch : p.Cout;
+            int8_t* dst = out + pix * pitch + c0;
+            if (c0 + 32 <= pitch && (pitch & 15) == 0 && p.vec_ok) {  // (channels beyond Cout are zero and land in the padding)
                 reinterpret_cast<uint4*>(dst)[0] = make_uint4(qw[0], qw[1], qw[2], qw[3]);
                 reinterpret_cast<uint4*>(dst)[1] = make_uint4(qw[4], qw[5], qw[6], qw[7]);
             } else {

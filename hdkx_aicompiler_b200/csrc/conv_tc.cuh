@@ -71,6 +71,7 @@ struct alignas(64) TcParams {
     // high part at out_hi and the low part out_lo_offset elements after it (null: not wanted). `out` may then be null.
     float* out_hi;
     long long out_lo_offset;
+    int out_pitch;               // kOutNHWC_S8: channels per stored pixel (0: Cout), a multiple of 16
     int split;                   // 2..kMaxSplit: the reduction is split over clusters of that many CTAs (conv_splitk.cu); 0: it is not
     int weights_ready;           // the packed weights were written long before this launch: they may be read ahead of its predecessor's end
 };

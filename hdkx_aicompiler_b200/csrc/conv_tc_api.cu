@@ -196,15 +196,22 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     const size_t act_bytes = align_up((size_t)d.N * conv_h * conv_w * cpad, 1024);
     const size_t w_bytes = align_up((size_t)d.O * d.KH * d.KW * cpad, 1024);
     // Result layout. A thread of the epilogue owns one pixel, so its NCHW stores are single bytes whose neighbours in
-    // memory belong to the next pixel of the same tile row: runs of BW bytes. With the narrow tiles of the deep layers
-    // (BW <= 2) that costs more than the kernel itself (512 -> 512 channels at 7x7, 256 images: 100 us against 35 us for
-    // the NHWC form), so those layers store NHWC into the workspace and a byte transpose writes the reference layout.
+    // memory belong to the next pixel of the same tile row: runs of BW bytes. From 1 MiB of results on (and wherever BW <= 2)
+    // the kernel stores NHWC into the workspace instead, pixels padded to 16 channels, and a byte transpose writes the
+    // reference layout (128 -> 128 channels, 28x28, 256 images: 65 us of convolution with byte stores against 52 + 12). A
+    // smaller result is not worth the second launch.
     int bw = 0, bh = 0, bni = 0;
     tc_pick_tile(d.N, d.OH, d.OW, &bw, &bh, &bni);
-    const bool two_step = (bw <= 2 && (d.O & 15) == 0) || rowstack_ok;  // (the row-stacked kernel writes NHWC only)
-    const size_t out_bytes = two_step ? align_up((size_t)d.N * d.OH * d.OW * d.O, 1024) : 0;
+    const int out_pitch = (d.O + 15) / 16 * 16;
+    bool two_step = bw <= 2 || rowstack_ok || (long long)d.N * d.O * d.OH * d.OW >= (1 << 20);  // (the row-stacked kernel writes NHWC only)
+    const size_t out_bytes = two_step ? align_up((size_t)d.N * d.OH * d.OW * out_pitch, 1024) : 0;
     StreamScratch ws(s);
-    KXC_TRY(ws.alloc(act_bytes + w_bytes + out_bytes));
+    int32_t rc = ws.alloc(act_bytes + w_bytes + out_bytes);
+    if (rc != KXC_B200_OK && two_step && !rowstack_ok) {  // no room for the second copy of the result: byte stores
+        two_step = false;
+        rc = ws.alloc(act_bytes + w_bytes);
+    }
+    KXC_TRY(rc);
     uint8_t* act = static_cast<uint8_t*>(ws.ptr);
     uint8_t* wp = act + act_bytes;
     int8_t* out_nhwc = reinterpret_cast<int8_t*>(wp + w_bytes);
@@ -226,6 +233,7 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     p.multiplier = multiplier;
     p.shift = shift;
     p.out = two_step ? out_nhwc : out;
+    p.out_pitch = two_step ? out_pitch : 0;
     p.relu = relu;
     tc_finish_params(&p);
     if (rowstack_ok) {
@@ -233,7 +241,7 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     } else {
         KXC_TRY(tc_launch(cfg, p, s));
     }
-    if (two_step) return nhwc_to_nchw_s8(out_nhwc, out, d.N, d.O, d.OH * d.OW, s);
+    if (two_step) return nhwc_to_nchw_s8(out_nhwc, out, d.N, d.O, out_pitch, d.OH * d.OW, s);
     return KXC_B200_OK;
 }
 

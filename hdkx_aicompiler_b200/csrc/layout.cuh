@@ -23,8 +23,8 @@ int32_t split_rows(const float* in, float* hi, float* lo, int64_t rows, int cols
 int32_t nchw_to_nhwc_s8_subsample(const int8_t* in, int8_t* out, int N, int C, int H, int W, int OH, int OW, int stride, int cpad,
                                   cudaStream_t s);
 
-// int8 NHWC [N][HW][C] -> NCHW [N][C][HW] (the reference layout of a requantized result).
-int32_t nhwc_to_nchw_s8(const int8_t* in, int8_t* out, int N, int C, int HW, cudaStream_t s);
+// int8 NHWC [N][HW][C of pitch] -> NCHW [N][C][HW] (the reference layout of a requantized result).
+int32_t nhwc_to_nchw_s8(const int8_t* in, int8_t* out, int N, int C, int pitch, int HW, cudaStream_t s);
 
 // OIHW (fp32 or int8) -> [O][KH][KW][cpad] in the operand type.
 int32_t pack_weights_ohwi(const void* w, void* out, TcDType dtype, int O, int C, int KH, int KW, int cpad, cudaStream_t s, bool tf32_lo = false);

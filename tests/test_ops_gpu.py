@@ -268,6 +268,17 @@ def test_conv2d_s8_bit_exact(ops, rng, case, simt):
         assert np.array_equal(got, expect), f"s8 conv {case} relu={relu} simt={simt}: {np.count_nonzero(got != expect)} differ"
 
 
+# The byte transposes on both sides of the NCHW form: planes that are multiples of 16, of 4 and odd; channel counts that are not
+# multiples of 16 or 4; one, two and more column tiles; the result by way of NHWC (1 MiB and more) and without.
+@pytest.mark.parametrize("N,C,H,W,O", [(9, 72, 28, 28, 150), (3, 130, 30, 30, 400), (40, 64, 14, 14, 141), (27, 33, 25, 13, 133), (2, 48, 12, 12, 40),
+                                       (345, 128, 14, 14, 128)])
+def test_conv2d_s8_layouts(ops, rng, N, C, H, W, O):
+    x, w, b, m, sh = (dev(a) for a in s8_inputs(rng, N, C, H, W, O, 3, 3))
+    got = ops.nn_conv2d_s8(x, w, b, m, sh, (1, 1), (1, 1))
+    assert ops.device_status() == 0
+    assert torch.equal(got, ops.nn_conv2d_s8(x, w, b, m, sh, (1, 1), (1, 1), simt=True))
+
+
 # ---------------------------------------------------------------- dense / gemm
 @pytest.mark.parametrize("M,N,K", [(2, 2, 3), (2, 4, 3), (5, 11, 37), (33, 1000, 512), (130, 72, 200), (0, 4, 8)])
 def test_gemm_fp32_mode_bit_exact(ops, rng, M, N, K):
