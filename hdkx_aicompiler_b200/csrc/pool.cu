@@ -64,20 +64,21 @@ __global__ void __launch_bounds__(kThreads) pool_generic_kernel(const float* __r
 // two aligned 16-byte loads plus one scalar (the left neighbour) per row. Consecutive threads walk
 // consecutive column groups, so every input row is read in contiguous 32-byte pieces and every
 // output row is written as contiguous 16-byte vectors.
-template <bool kAddRelu>
+// (Index: 32 bits where the number of items allows it, for the two divisions)
+template <bool kAddRelu, typename Index>
 __global__ void __launch_bounds__(kThreads) maxpool_3x3s2p1_kernel(const float* __restrict__ x,
                                                                    const float* __restrict__ res,
                                                                    float* __restrict__ out, int64_t planes, int H, int W,
                                                                    int OH, int OW) {
     const int groups = OW >> 2;        // 4 outputs per group
     const int row_pairs = OH >> 1;     // OH is even when this kernel is chosen
-    const int64_t total = planes * row_pairs * groups;
+    const Index total = (Index)(planes * row_pairs * groups);
     const float pad_value = -1e30f;
-    for (int64_t lin = (int64_t)blockIdx.x * kThreads + threadIdx.x; lin < total; lin += (int64_t)gridDim.x * kThreads) {
-        const int g = (int)(lin % groups);
-        const int64_t t = lin / groups;
-        const int rp = (int)(t % row_pairs);
-        const int64_t plane = t / row_pairs;
+    for (Index lin = (Index)blockIdx.x * kThreads + threadIdx.x; lin < total; lin += (Index)gridDim.x * kThreads) {
+        const Index t = lin / (Index)groups;
+        const int g = (int)(lin - t * (Index)groups);
+        const int64_t plane = (int64_t)(t / (Index)row_pairs);
+        const int rp = (int)(t - (Index)plane * (Index)row_pairs);
         const int ow0 = g << 2;
         const int oh0 = rp << 1;
         const int iw0 = ow0 * 2;  // multiple of 8 -> 32-byte aligned in an aligned row
@@ -121,6 +122,55 @@ __global__ void __launch_bounds__(kThreads) maxpool_3x3s2p1_kernel(const float* 
             }
             __stcs(reinterpret_cast<float4*>(out + off), make_float4(o[0], o[1], o[2], o[3]));
         }
+    }
+}
+
+// ---- the same window over planes of any extent and alignment ------------------------------------
+// A thread produces one column of two output rows from 5 input rows x 3 columns with 4-byte loads (a warp's loads of one
+// row lie in one or two rows of the plane, so they share lines). What bound the generic kernel above at these shapes was
+// not memory but instructions: three 64-bit divisions and nine bounded loads for every output; 32-bit indices (the
+// launcher checks the range) and the shared rows leave a third of them.
+template <bool kAddRelu>
+__global__ void __launch_bounds__(kThreads) maxpool_3x3s2p1_ragged_kernel(const float* __restrict__ x, const float* __restrict__ res,
+                                                                          float* __restrict__ out, uint32_t total, int H, int W, int OH, int OW) {
+    const uint32_t row_pairs = (uint32_t)(OH + 1) >> 1;
+    const float pad_value = -1e30f;
+    const uint32_t lin = blockIdx.x * kThreads + threadIdx.x;
+    if (lin >= total) return;
+    const uint32_t t = lin / (uint32_t)OW;
+    const int ow = (int)(lin - t * (uint32_t)OW);
+    const uint32_t plane = t / row_pairs;
+    const int oh0 = (int)(t - plane * row_pairs) * 2;
+    const float* xp = x + (size_t)plane * H * W;
+    const int iw0 = ow * 2 - 1, ih0 = oh0 * 2 - 1;
+    const bool second = oh0 + 1 < OH;
+    const size_t off = ((size_t)plane * OH + oh0) * OW + ow;
+    float add0 = 0.0f, add1 = 0.0f;
+    if (kAddRelu) {
+        add0 = __ldcs(res + off);
+        if (second) add1 = __ldcs(res + off + OW);
+    }
+    float r[5][3];
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+        const int ih = ih0 + j;
+        const bool row_ok = ih >= 0 && ih < H;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int iw = iw0 + c;
+            r[j][c] = row_ok && iw >= 0 && iw < W ? __ldg(xp + (size_t)ih * W + iw) : pad_value;
+        }
+    }
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+        float m = -INFINITY;
+#pragma unroll
+        for (int rh = 0; rh < 3; ++rh)
+#pragma unroll
+            for (int rw = 0; rw < 3; ++rw) m = sel_max(m, r[2 * o + rh][rw]);
+        if (kAddRelu) m = relu1(__fadd_rn(m, o == 0 ? add0 : add1));
+        if (o == 0) __stcs(out + off, m);
+        else if (second) __stcs(out + off + OW, m);
     }
 }
 
@@ -218,8 +268,13 @@ int32_t launch_max_pool(const float* x, const float* res, float* out, const kxc_
         const int64_t items = pd.planes * (pd.OH / 2) * (pd.OW / 4);
         // one item per thread (no grid-stride iterations) up to 64 blocks per SM: the hardware block scheduler
         // balances these short kernels at a finer grain than a persistent loop would
-        maxpool_3x3s2p1_kernel<kAddRelu><<<grid_for(items, kThreads, 64), kThreads, 0, s>>>(x, res, out, pd.planes, pd.H,
-                                                                                           pd.W, pd.OH, pd.OW);
+        auto kernel = items < (1ll << 31) ? maxpool_3x3s2p1_kernel<kAddRelu, uint32_t> : maxpool_3x3s2p1_kernel<kAddRelu, int64_t>;
+        kernel<<<grid_for(items, kThreads, 64), kThreads, 0, s>>>(x, res, out, pd.planes, pd.H, pd.W, pd.OH, pd.OW);
+    } else if (d->kh == 3 && d->kw == 3 && d->stride_h == 2 && d->stride_w == 2 && d->pad_top == 1 && d->pad_left == 1 &&
+               pd.planes * ((pd.OH + 1) / 2) * pd.OW < (1ll << 31)) {
+        const int64_t items = pd.planes * ((pd.OH + 1) / 2) * pd.OW;
+        maxpool_3x3s2p1_ragged_kernel<kAddRelu><<<(unsigned)((items + kThreads - 1) / kThreads), kThreads, 0, s>>>(x, res, out, (uint32_t)items,
+                                                                                                                pd.H, pd.W, pd.OH, pd.OW);
     } else {
         const int64_t items = pd.planes * pd.OH * pd.OW;
         pool_generic_kernel<true, kAddRelu><<<grid_for(items, kThreads, 8), kThreads, 0, s>>>(x, res, out, pd);

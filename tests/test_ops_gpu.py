@@ -91,6 +91,18 @@ def test_max_pool_bit_exact(ops, rng, shape, k, s, p, ceil):
     assert_bit_exact(host(ops.nn_max_pool2d(dev(x), k, s, p, ceil)), port.max_pool2d(x, k, s, p, ceil), f"max_pool {shape}")
 
 
+# 3x3, stride 2, padding 1 over planes that the vector kernel refuses: odd heights and widths, one output row or column, ceil mode
+@pytest.mark.parametrize("shape,ceil", [((2, 3, 7, 9), False), ((3, 2, 14, 15), False), ((1, 5, 1, 1), False), ((2, 2, 2, 31), False), ((2, 3, 8, 11), True),
+                                        ((4, 33, 51, 57), False)])
+def test_max_pool_3x3s2_ragged_bit_exact(ops, rng, shape, ceil):
+    x = rng.uniform(-1, 1, shape).astype(f32)
+    x.ravel()[: min(x.size, SPECIALS.size)] = SPECIALS[: min(x.size, SPECIALS.size)]
+    expect = port.max_pool2d(x, (3, 3), (2, 2), (1, 1, 1, 1), ceil)
+    assert_bit_exact(host(ops.nn_max_pool2d(dev(x), (3, 3), (2, 2), (1, 1, 1, 1), ceil)), expect, f"max_pool {shape}")
+    res = rng.uniform(-1, 1, expect.shape).astype(f32)
+    assert_bit_exact(host(ops.max_pool2d_add_relu(dev(x), dev(res), (3, 3), (2, 2), (1, 1, 1, 1), ceil)), port.relu(port.add(expect, res)), f"chain {shape}")
+
+
 @pytest.mark.parametrize("shape,k,s,p,ceil", POOL_CASES)
 def test_avg_pool_bit_exact(ops, rng, shape, k, s, p, ceil):
     x = rng.uniform(-1, 1, shape).astype(f32)
