@@ -112,9 +112,19 @@ __device__ __forceinline__ float tf32_low_part(float x, float hi) {
     return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u ? 0.0f : tf32_rne(__fsub_rn(x, hi));
 }
 
+// kOutNCHW_F32: the chunk's residual values, fetched before the accumulator is waited for (one 4-byte load per channel: read
+// when they are needed, each waits out its own trip to memory).
+__device__ __forceinline__ void residual_fetch_nchw(const TcParams& p, int c0, bool valid, int n, int oh, int ow, float (&res)[32]) {
+    const size_t plane = (size_t)p.OH * p.OW;
+    const float* src = static_cast<const float*>(p.residual) + ((size_t)n * p.Cout + c0) * plane + (size_t)oh * p.OW + ow;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) res[j] = valid && c0 + j < p.Cout ? __ldg(src + (size_t)j * plane) : 0.0f;
+}
+
+// `nchw_res`: what residual_fetch_nchw read (kOutNCHW_F32 with a residual only).
 template <int kOutMode, bool kSplit = false>
 __device__ __forceinline__ void epilogue_chunk(const TcParams& p, const uint32_t (&v)[32], int c0, bool valid, int n,
-                                               int oh, int ow) {
+                                               int oh, int ow, const float (&nchw_res)[32]) {
     if (!valid || c0 >= p.Cout) return;
     const int nch = (p.Cout - c0) < 32 ? (p.Cout - c0) : 32;
     const size_t pix = ((size_t)n * p.OH + oh) * p.OW + ow;
@@ -265,18 +275,25 @@ __device__ __forceinline__ void epilogue_chunk(const TcParams& p, const uint32_t
             const size_t plane = (size_t)p.OH * p.OW;
             const size_t off = ((size_t)n * p.Cout + c0) * plane + (size_t)oh * p.OW + ow;
             float* out = static_cast<float*>(p.out) + off;
-            const float* res = p.residual ? static_cast<const float*>(p.residual) + off : nullptr;
+            const bool has_res = p.residual != nullptr;
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
                 if (j < nch) {
                     float x = f[j];
-                    if (res) x = __fadd_rn(x, __ldg(res + (size_t)j * plane));
+                    if (has_res) x = __fadd_rn(x, nchw_res[j]);
                     if (p.relu) x = x > 0.0f ? x : 0.0f;
                     out[(size_t)j * plane] = x;
                 }
             }
         }
     }
+}
+
+template <int kOutMode>
+__device__ __forceinline__ void epilogue_chunk(const TcParams& p, const uint32_t (&v)[32], int c0, bool valid, int n, int oh, int ow) {
+    static_assert(kOutMode != kOutNCHW_F32, "this layout's residual is fetched by the caller");
+    const float none[32] = {};
+    epilogue_chunk<kOutMode, false>(p, v, c0, valid, n, oh, ow, none);
 }
 
 // Hot-path epilogue (bf16 NHWC activations, channel count a multiple of 32, 16-byte aligned pointers):

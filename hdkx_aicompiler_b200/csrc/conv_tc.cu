@@ -329,6 +329,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
             const int col0 = half * kChunksPerWarp * 32;  // first column of this warp inside the tile
             const int c_base = ct * BN + col0;
             uint4 res_cur[4] = {};
+            float nchw_cur[32] = {}, nchw_next[32] = {};  // kOutNCHW_F32 only
+            if constexpr (kOutMode == kOutNCHW_F32) {
+                if (has_res && c_base < p.Cout) residual_fetch_nchw(p, c_base, valid, n, oh, ow, nchw_cur);
+            }
             RowMap rows;
             if (fast && !boxed) {
                 rows = make_row_map(pix, valid, lane);
@@ -352,6 +356,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                 uint4 res_next[4] = {};
                 if (fast && has_res && (i + 1 < kChunksPerWarp) && (c0 + 32 < p.Cout))
                     residual_fetch_rows(ep, rows, c0 + 32, lane, res_next);
+                if constexpr (kOutMode == kOutNCHW_F32) {
+                    if (has_res && i + 1 < kChunksPerWarp && c0 + 32 < p.Cout) residual_fetch_nchw(p, c0 + 32, valid, n, oh, ow, nchw_next);
+                }
                 if constexpr (kX3) {
                     uint32_t u[32];
                     tmem_ld_32x32(t_addr + (uint32_t)(BN + i * 32), u);
@@ -379,10 +386,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                 } else if (fast) {
                     if (c0 < p.Cout) epilogue_coalesced_bf16<32>(ep, v, c0, stage_tile, lane, rows, res_cur, has_res);
                 } else {
-                    epilogue_chunk<kOutMode, kX3>(p, v, c0, valid, n, oh, ow);
+                    epilogue_chunk<kOutMode, kX3>(p, v, c0, valid, n, oh, ow, nchw_cur);
                 }
 #pragma unroll
                 for (int g = 0; g < 4; ++g) res_cur[g] = res_next[g];
+                if constexpr (kOutMode == kOutNCHW_F32) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) nchw_cur[j] = nchw_next[j];
+                }
             }
             if constexpr (kDual) {
                 // second output: same rows and channels from the accumulator next to the main one; no residual
@@ -694,6 +705,38 @@ int32_t tc_bind_store(TcParams* p, const TcConfig& cfg) {
 }
 
 namespace {
+// Tile box of a launch that writes the reference's layout: a warp's 32 pixels leave as one 4-byte store per channel, in runs of
+// BW consecutive addresses (BW * BH when the box spans the rows), and every run costs its own 32-byte sectors. The box with
+// the fewest tiles may have runs of one to three pixels, so waves and sectors are weighed together: a tile's main loop is its K
+// blocks at the rate they arrive, its epilogue ~4 cycles per sector (stores and residual loads), which overlaps the next tile's
+// main loop. (9 x 72 x 45 x 51 -> 120 channels, tf32, with a residual: runs of 3 pixels, 41 us; full rows and the residual read
+// ahead of the accumulator, with two tiles per work item below, 27 us.)
+void pick_tile_nchw(int N, int OH, int OW, int Cout, int num_kb, int kb_bytes, int* BW, int* BH, int* BNI) {
+    const int bn_out = Cout <= 64 ? 64 : (Cout <= 128 ? 128 : 256);
+    const int tiles_c = (Cout + bn_out - 1) / bn_out;
+    const double main_loop = (double)num_kb * kb_bytes / 128.0 * (bn_out == 64 ? 490 : (bn_out == 128 ? 655 : 980));
+    double best = -1.0;
+    for (int bw = 1; bw <= OW && bw <= 128; ++bw) {
+        for (int bh = 1; bh <= OH && bw * bh <= 128; ++bh) {
+            int bn = 128 / (bw * bh);
+            if (bn > N) bn = N;
+            if (bn < 1) bn = 1;
+            const long long tiles = (long long)((OW + bw - 1) / bw) * ((OH + bh - 1) / bh) * ((N + bn - 1) / bn);
+            const long long waves = (tiles * tiles_c + kNumSMs - 1) / kNumSMs;
+            int run = bw == OW ? bw * bh : bw;
+            if (run > 32) run = 32;
+            const double epilogue = 4.0 * 1.5 * bn_out * 128.0 * (run / 8.0 + 0.9) / run;
+            const double slower = main_loop > epilogue ? main_loop : epilogue;
+            // (tiles as the tie-breaker: less work on the same number of waves)
+            const double cost = main_loop + (double)(waves - 1) * slower + epilogue + 1e-3 * (double)tiles;
+            if (best < 0.0 || cost < best) {
+                best = cost;
+                *BW = bw; *BH = bh; *BNI = bn;
+            }
+        }
+    }
+}
+
 // The weights of a split launch: boxes of cfg->bn rows x one K block of `k_elems` elements per output channel.
 int32_t weight_map(CUtensorMap* m, const TcConfig* cfg, const TcParams* p, const void* w, int k_elems) {
     const uint64_t dims[2] = {(uint64_t)k_elems, (uint64_t)p->Cout};
@@ -805,7 +848,10 @@ int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_m
     p->pad_h = pad_h; p->pad_w = pad_w; p->dil_h = dil_h; p->dil_w = dil_w;
     p->kb_elems = kb_bytes / eb;
     p->cblocks = row_bytes / kb_bytes;
-    tc_pick_tile(N, OH, OW, &p->BW, &p->BH, &p->BNI);
+    if (out_mode == kOutNCHW_F32)
+        pick_tile_nchw(N, OH, OW, Cout, KH * KW * p->cblocks, kb_bytes, &p->BW, &p->BH, &p->BNI);
+    else
+        tc_pick_tile(N, OH, OW, &p->BW, &p->BH, &p->BNI);
     p->tiles_w = (OW + p->BW - 1) / p->BW;
     p->tiles_h = (OH + p->BH - 1) / p->BH;
     p->tiles_n = (N + p->BNI - 1) / p->BNI;
