@@ -85,7 +85,7 @@ int32_t conv2d_tensor_core(const float* data, const float* weight, const float* 
         uint8_t* w_lo = w_hi + w_bytes;
         KXC_TRY(nchw_to_nhwc_split(data, act_hi, act_hi + act, d.N, d.C, d.H * d.W, cpad, s));
         KXC_TRY(pack_weights_ohwi(weight, w_hi, kTcTF32, d.O, d.C, d.KH, d.KW, cpad, s));
-        KXC_TRY(pack_weights_ohwi(weight, w_lo, kTcTF32, d.O, d.C, d.KH, d.KW, cpad, s, true));
+        KXC_TRY(pack_weights_ohwi(weight, w_lo, kTcTF32, d.O, d.C, d.KH, d.KW, cpad, s, true, true));
         TcParams p{};
         TcConfig cfg{};
         KXC_TRY(tc_setup_conv_x3(&p, &cfg, kOutNCHW_F32, act_hi, w_hi, w_lo, d.N, d.H, d.W, cpad, d.O, d.KH, d.KW, d.SH, d.PH, d.PW, d.DH,
@@ -107,7 +107,7 @@ int32_t conv2d_tensor_core(const float* data, const float* weight, const float* 
     uint8_t* act = static_cast<uint8_t*>(ws.ptr);
     uint8_t* wp = act + act_bytes;
     KXC_TRY(nchw_to_nhwc(data, act, dt, d.N, d.C, d.H * d.W, cpad, s));
-    KXC_TRY(pack_weights_ohwi(weight, wp, dt, d.O, d.C, d.KH, d.KW, cpad, s));
+    KXC_TRY(pack_weights_ohwi(weight, wp, dt, d.O, d.C, d.KH, d.KW, cpad, s, false, true));
     TcParams p{};
     TcConfig cfg{};
     KXC_TRY(tc_setup_conv(&p, &cfg, dt, kOutNCHW_F32, act, wp, d.N, d.H, d.W, cpad, d.O, d.KH, d.KW, d.SH, d.PH, d.PW, d.DH,
@@ -220,7 +220,8 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     } else {
         KXC_TRY(nchw_to_nhwc(data, act, dt, d.N, d.C, d.H * d.W, cpad, s));
     }
-    KXC_TRY(pack_weights_ohwi(weight, wp, dt, d.O, d.C, d.KH, d.KW, cpad, s));
+    // (the row-stacked kernel reads the weights ahead of its predecessor's end)
+    KXC_TRY(pack_weights_ohwi(weight, wp, dt, d.O, d.C, d.KH, d.KW, cpad, s, false, !rowstack_ok));
     TcParams p{};
     TcConfig cfg{};
     if (rowstack_ok) {
@@ -282,10 +283,10 @@ int32_t gemm_tensor_core(const float* a, const float* b, const float* c, float* 
     KXC_TRY(ws.alloc(a_bytes + b_bytes));
     uint8_t* ap = static_cast<uint8_t*>(ws.ptr);
     uint8_t* bp = ap + a_bytes;
-    KXC_TRY(convert_rows(a, ap, dt, g.m, g.k, kpad, s));
     if (g.transB) {
-        KXC_TRY(convert_rows(b, bp, dt, g.n, g.k, kpad, s));  // b is [N, K]
+        KXC_TRY(convert_rows_two(a, ap, g.m, b, bp, g.n, dt, g.k, kpad, s));  // b is [N, K]
     } else {
+        KXC_TRY(convert_rows(a, ap, dt, g.m, g.k, kpad, s));
         KXC_TRY(nchw_to_nhwc(b, bp, dt, 1, g.k, g.n, kpad, s));  // b is [K, N] -> [N, Kpad]
     }
     TcParams p{};

@@ -12,7 +12,12 @@ namespace kxc_b200 {
 // NCHW (fp32 or int8) -> NHWC with `cpad` channels (zero filled), converted to the tensor-core
 // operand type: bf16 (round to nearest even), tf32 kept in fp32 storage (low 13 mantissa bits
 // rounded away, nearest even), or int8 (copied).
-int32_t nchw_to_nhwc(const void* in, void* out, TcDType dtype, int N, int C, int HW, int cpad, cudaStream_t s, bool tf32_lo = false);
+int32_t nchw_to_nhwc(const void* in, void* out, TcDType dtype, int N, int C, int HW, int cpad, cudaStream_t s, bool tf32_lo = false,
+                     bool overlap = false);
+
+// convert_rows of two matrices with rows of the same length, in one launch where extents and addresses allow it.
+int32_t convert_rows_two(const float* a, void* out_a, int64_t rows_a, const float* b, void* out_b, int64_t rows_b, TcDType dtype, int cols,
+                         int cpad, cudaStream_t s);
 
 // Three-pass tf32 operands: the tf32 rounding of every value (hi) and the tf32 rounding of what that dropped (lo).
 int32_t nchw_to_nhwc_split(const float* in, float* hi, float* lo, int N, int C, int HW, int cpad, cudaStream_t s);
@@ -27,7 +32,8 @@ int32_t nchw_to_nhwc_s8_subsample(const int8_t* in, int8_t* out, int N, int C, i
 int32_t nhwc_to_nchw_s8(const int8_t* in, int8_t* out, int N, int C, int pitch, int HW, cudaStream_t s);
 
 // OIHW (fp32 or int8) -> [O][KH][KW][cpad] in the operand type.
-int32_t pack_weights_ohwi(const void* w, void* out, TcDType dtype, int O, int C, int KH, int KW, int cpad, cudaStream_t s, bool tf32_lo = false);
+int32_t pack_weights_ohwi(const void* w, void* out, TcDType dtype, int O, int C, int KH, int KW, int cpad, cudaStream_t s, bool tf32_lo = false,
+                          bool overlap = false);
 
 // Row-major [rows, cols] fp32 -> [rows, cpad] operand type (dense operands).
 int32_t convert_rows(const float* in, void* out, TcDType dtype, int64_t rows, int cols, int cpad, cudaStream_t s, bool tf32_lo = false);

@@ -1138,7 +1138,7 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
                     KXC_TRY(nchw_to_nhwc_split(static_cast<const float*>(arg_of(st.in0)), hi, hi + pl->find(st.out)->elems, st.N, st.C,
                                                st.H * st.W, st.cpad, s));
                 } else {
-                    KXC_TRY(nchw_to_nhwc(arg_of(st.in0), pl->storage(st.out), dt, st.N, st.C, st.H * st.W, st.cpad, s));
+                    KXC_TRY(nchw_to_nhwc(arg_of(st.in0), pl->storage(st.out), dt, st.N, st.C, st.H * st.W, st.cpad, s, false, true));
                 }
                 break;
             case SKind::InputStem:

@@ -18,7 +18,8 @@ PRECISIONS = {"fp32": PREC_FP32, "tf32": PREC_TF32, "bf16": PREC_BF16, "simt": P
 
 
 def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    # the raw handle: building a torch.cuda.Stream object for it costs as much as a small kernel's launch
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 
 def _req(t, dtype, name):
@@ -82,7 +83,7 @@ def nn_conv2d(data, weight, bias=None, strides=(1, 1), padding=(0, 0), dilation=
     if relu:
         flags |= RELU
     if out is None:
-        out = torch.empty((N, O, max(OH, 0), max(OW, 0)), dtype=torch.float32, device=data.device)
+        out = data.new_empty((N, O, max(OH, 0), max(OW, 0)))
     ptrs.append(out.data_ptr())
     desc = Conv2dDesc(N, C, H, W, O, KH, KW, sh, sw, ph, pw, dh, dw, flags, PRECISIONS[precision])
     check("nn_conv2d", load().kxc_b200_nn_conv2d(packed(*ptrs), desc, _stream(data)))
@@ -112,7 +113,7 @@ def nn_conv2d_s8(data, weight, bias, multiplier, shift, strides=(1, 1), padding=
     ph, pw = _pair(padding, 0)
     dh, dw = _pair(dilation, 1)
     OH, OW = conv_out_dim(H, KH, sh, ph, dh), conv_out_dim(W, KW, sw, pw, dw)
-    out = torch.empty((N, OH, OW, O) if nhwc else (N, O, OH, OW), dtype=torch.int8, device=data.device)
+    out = data.new_empty((N, OH, OW, O) if nhwc else (N, O, OH, OW))
     desc = Conv2dDesc(N, C, H, W, O, KH, KW, sh, sw, ph, pw, dh, dw, BIAS | (RELU if relu else 0) | (NHWC if nhwc else 0),
                       PREC_SIMT if simt else PREC_FP32)
     args = packed(data.data_ptr(), weight.data_ptr(), bias.data_ptr(), multiplier.data_ptr(), shift.data_ptr(),
@@ -141,7 +142,7 @@ def add(a, b, relu=False):
     for i, d in enumerate(b.shape):
         desc.shape_b[i] = d
     out_shape = torch.broadcast_shapes(a.shape, b.shape)
-    out = torch.empty(out_shape, dtype=torch.float32, device=a.device)
+    out = a.new_empty(out_shape)
     check("add", load().kxc_b200_add(packed(a.data_ptr(), b.data_ptr(), out.data_ptr()), desc, _stream(a)))
     return out
 
@@ -166,7 +167,7 @@ def _pool_desc(x, pool_size, strides, padding, ceil_mode, name):
 def nn_max_pool2d(x, pool_size, strides, padding=(0, 0, 0, 0), ceil_mode=False):
     x = _req(x, torch.float32, "nn_max_pool2d")
     desc, oshape = _pool_desc(x, pool_size, strides, padding, ceil_mode, "nn_max_pool2d")
-    out = torch.empty(oshape, dtype=torch.float32, device=x.device)
+    out = x.new_empty(oshape)
     check("nn_max_pool2d", load().kxc_b200_nn_max_pool2d(packed(x.data_ptr(), out.data_ptr()), desc, _stream(x)))
     return out
 
@@ -174,7 +175,7 @@ def nn_max_pool2d(x, pool_size, strides, padding=(0, 0, 0, 0), ceil_mode=False):
 def nn_avg_pool2d(x, pool_size, strides, padding=(0, 0, 0, 0), ceil_mode=False):
     x = _req(x, torch.float32, "nn_avg_pool2d")
     desc, oshape = _pool_desc(x, pool_size, strides, padding, ceil_mode, "nn_avg_pool2d")
-    out = torch.empty(oshape, dtype=torch.float32, device=x.device)
+    out = x.new_empty(oshape)
     check("nn_avg_pool2d", load().kxc_b200_nn_avg_pool2d(packed(x.data_ptr(), out.data_ptr()), desc, _stream(x)))
     return out
 
@@ -187,7 +188,7 @@ def max_pool2d_add_relu(x, residual, pool_size, strides, padding=(0, 0, 0, 0), c
     if tuple(residual.shape) != tuple(oshape):
         raise ValueError("max_pool2d_add_relu: residual must have the pooled shape")
     if out is None:
-        out = torch.empty(oshape, dtype=torch.float32, device=x.device)
+        out = x.new_empty(oshape)
     check("max_pool2d_add_relu",
           load().kxc_b200_max_pool2d_add_relu(packed(x.data_ptr(), residual.data_ptr(), out.data_ptr()), desc, _stream(x)))
     return out
@@ -198,7 +199,7 @@ def nn_global_avg_pool2d(x):
     if x.dim() != 4:
         raise ValueError("nn_global_avg_pool2d expects NCHW rank-4 input")
     N, C, H, W = x.shape
-    out = torch.empty((N, C, 1, 1), dtype=torch.float32, device=x.device)
+    out = x.new_empty((N, C, 1, 1))
     check("nn_global_avg_pool2d",
           load().kxc_b200_nn_global_avg_pool2d(packed(x.data_ptr(), out.data_ptr()), N, C, H, W, _stream(x)))
     return out
@@ -224,7 +225,7 @@ def reduce_mean(x, axes, keepdims=True):
     norm = sorted(a % x.dim() for a in axes)
     oshape = [1 if d in norm else n for d, n in enumerate(x.shape) if keepdims or d not in norm]
     desc = _lib.ReduceDesc(x.dim(), (_lib.i64 * 6)(*x.shape), len(axes), (_lib.i32 * 6)(*axes), 1 if keepdims else 0)
-    out = torch.empty(oshape, dtype=torch.float32, device=x.device)
+    out = x.new_empty(oshape)
     check("reduce_mean", load().kxc_b200_reduce_mean(packed(x.data_ptr(), out.data_ptr()), desc, _stream(x)))
     return out
 
@@ -249,7 +250,7 @@ def matmul(a, b, precision="tf32"):
         raise ValueError("matmul currently expects rank-2 inputs")
     if a.shape[1] != b.shape[0]:
         raise ValueError("matmul reduction dimension mismatch")
-    out = torch.empty((a.shape[0], b.shape[1]), dtype=torch.float32, device=a.device)
+    out = a.new_empty((a.shape[0], b.shape[1]))
     check("matmul", load().kxc_b200_matmul(packed(a.data_ptr(), b.data_ptr(), out.data_ptr()), a.shape[0], b.shape[1],
                                            a.shape[1], PRECISIONS[precision], _stream(a)))
     return out
@@ -339,7 +340,7 @@ def cast(x, dtype):
 
 def nn_flatten(x):
     x = _req(x, torch.float32, "nn_flatten")
-    out = torch.empty((x.shape[0], x.numel() // max(x.shape[0], 1)), dtype=torch.float32, device=x.device)
+    out = x.new_empty((x.shape[0], x.numel() // max(x.shape[0], 1)))
     check("nn_flatten", load().kxc_b200_nn_flatten(packed(x.data_ptr(), out.data_ptr()), x.numel(), _stream(x)))
     return out
 
@@ -351,7 +352,7 @@ def nn_dense(data, weight, precision="tf32"):
     Nn, K2 = weight.shape
     if K != K2:
         raise ValueError("nn_dense: inner dimensions differ")
-    out = torch.empty((M, Nn), dtype=torch.float32, device=data.device)
+    out = data.new_empty((M, Nn))
     desc = GemmDesc(M, Nn, K, 1.0, 1.0, 0, 1, 0, PRECISIONS[precision])
     check("nn_dense", load().kxc_b200_nn_gemm(packed(data.data_ptr(), weight.data_ptr(), out.data_ptr()), desc, _stream(data)))
     return out
@@ -363,7 +364,7 @@ def nn_gemm(a, b, c, alpha=1.0, beta=1.0, transA=0, transB=0, precision="tf32"):
     c = _req(c, torch.float32, "nn_gemm C")
     M, K = a.shape
     Nn = b.shape[0] if transB else b.shape[1]
-    out = torch.empty((M, Nn), dtype=torch.float32, device=a.device)
+    out = a.new_empty((M, Nn))
     desc = GemmDesc(M, Nn, K, float(alpha), float(beta), int(transA), int(transB), 1, PRECISIONS[precision])
     check("nn_gemm", load().kxc_b200_nn_gemm(packed(a.data_ptr(), b.data_ptr(), c.data_ptr(), out.data_ptr()), desc, _stream(a)))
     return out
