@@ -554,6 +554,19 @@ int32_t launch_by_bn(const TcConfig& cfg, const TcParams& p, cudaStream_t s) {
                                  : launch_one<kKind, KB_BYTES, 128, kOutNHWC_BF16, 1, false, 2>(p, s);
         }
     }
+    if constexpr (KB_BYTES == 128 && kKind != MmaKind::F16) {
+        if (cfg.mt == 2 && cfg.ctas == 1) {
+            if constexpr (kKind == MmaKind::I8) {
+                if (cfg.bn == 128 && cfg.out_mode == kOutNHWC_S8) return launch_one<kKind, KB_BYTES, 128, kOutNHWC_S8, 1, false, 2>(p, s);
+            } else if (cfg.out_mode == kOutNHWC_F32) {
+                if (cfg.bn == 64) return launch_one<kKind, KB_BYTES, 64, kOutNHWC_F32, 1, false, 2>(p, s);
+                if (cfg.bn == 128) return launch_one<kKind, KB_BYTES, 128, kOutNHWC_F32, 1, false, 2>(p, s);
+            } else if (cfg.out_mode == kOutNCHW_F32) {
+                if (cfg.bn == 64) return launch_one<kKind, KB_BYTES, 64, kOutNCHW_F32, 1, false, 2>(p, s);
+                if (cfg.bn == 128) return launch_one<kKind, KB_BYTES, 128, kOutNCHW_F32, 1, false, 2>(p, s);
+            }
+        }
+    }
     if (cfg.mt != 1) return fail(KXC_B200_ERR_INVALID, "tensor-core conv: no multi-tile kernel for this configuration");
     if constexpr (KB_BYTES == 128) {
         if (cfg.ctas == 2) {  // pairs exist for the wide tiles only (tc_setup_conv)
@@ -761,7 +774,7 @@ int32_t choose_split(TcParams* p, TcConfig* cfg, const void* w, const void* w_lo
     };
     const long long group = (long long)cfg->ctas * cfg->mt;
     const long long items = p->tiles_c * ((m_tiles + group - 1) / group), slots = kNumSMs / cfg->ctas;
-    const long long whole = (items + slots - 1) / slots * kb * (cfg->mt == 2 ? 980 : stage_cycles(cfg->bn)) + 1500;
+    const long long whole = (items + slots - 1) / slots * kb * (cfg->mt == 2 ? (cfg->bn == 64 ? 820 : 1100) : stage_cycles(cfg->bn)) + 1500;
     long long best = whole * 9 / 10;
     int split = 0, width = 0;
     for (int bn = 64; bn <= 256 && (bn == 64 || bn / 2 < p->Cout) && !(bn == 256 && cfg->x3); bn *= 2) {
@@ -906,6 +919,17 @@ int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_m
         return !(e != nullptr && e[0] == '1');
     }();
     cfg->mt = (mt_enabled && bn == 128 && dtype == kTcBF16 && out_mode == kOutNHWC_BF16 && kb_bytes == 128 && m_tiles >= 2 * ctas) ? 2 : 1;
+    // tf32 and int8: the tiles of such a launch arrive from L2 at 7 to 8 TB/s over the whole chip whatever the MMAs do, and two
+    // pixel tiles against one weight tile are 20 / 24 KB per tile instead of 24 / 32 (64 / 128 channels). Taken when the
+    // modelled makespan gains: a stage of two tiles costs 820 / 1100 cycles against 490 / 655 (the wider one meets its
+    // instructions' ~140 cycles). ResNet-18 tf32, 32 images: layer 1 42 -> 34 us per convolution, layer 2 31 -> 30; int8 128 -> 128,
+    // 28x28, 256 images: 52 -> 46.
+    if (mt_enabled && ctas == 1 && kb_bytes == 128 &&
+        ((dtype == kTcTF32 && (bn == 64 || bn == 128)) || (dtype == kTcS8 && bn == 128 && out_mode == kOutNHWC_S8))) {
+        const long long tc = (Cout + bn - 1) / bn;
+        auto waves = [](long long items) { return (items + kNumSMs - 1) / kNumSMs; };
+        if (waves((m_tiles + 1) / 2 * tc) * (bn == 64 ? 820 : 1100) < waves(m_tiles * tc) * (bn == 64 ? 490 : 655)) cfg->mt = 2;
+    }
     p->tiles_c = (Cout + bn - 1) / bn;
 
     const uint32_t box[4] = {(uint32_t)p->kb_elems, (uint32_t)p->BW, (uint32_t)p->BH, (uint32_t)p->BNI};
