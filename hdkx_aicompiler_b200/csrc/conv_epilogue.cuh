@@ -100,6 +100,31 @@ __device__ __forceinline__ void requant_chunk(const TcParams& p, const uint32_t 
     }
 }
 
+// The chunk's int8 results (four per word, bytes in channel order; the first `nch` are real) to one output pixel.
+template <int kOutMode>
+__device__ __forceinline__ void store_chunk_s8(const TcParams& p, const uint32_t (&qw)[8], int c0, int nch, int n, int oh, int ow) {
+    const size_t pix = ((size_t)n * p.OH + oh) * p.OW + ow;
+    int8_t* out = static_cast<int8_t*>(p.out);
+    if constexpr (kOutMode == kOutNHWC_S8) {
+        const int pitch = p.out_pitch != 0 ? p.out_pitch : p.Cout;
+        int8_t* dst = out + pix * pitch + c0;
+        if (c0 + 32 <= pitch && (pitch & 15) == 0 && p.vec_ok) {  // (channels beyond Cout are zero and land in the padding)
+            reinterpret_cast<uint4*>(dst)[0] = make_uint4(qw[0], qw[1], qw[2], qw[3]);
+            reinterpret_cast<uint4*>(dst)[1] = make_uint4(qw[4], qw[5], qw[6], qw[7]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                if (j < nch) dst[j] = (int8_t)(qw[j >> 2] >> (8 * (j & 3)));
+        }
+    } else {
+        const size_t plane = (size_t)p.OH * p.OW;
+        int8_t* dst = out + ((size_t)n * p.Cout + c0) * plane + (size_t)oh * p.OW + ow;
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            if (j < nch) dst[(size_t)j * plane] = (int8_t)(qw[j >> 2] >> (8 * (j & 3)));
+    }
+}
+
 // Epilogue for one 32-column chunk held by one thread (= one output pixel, 32 consecutive channels).
 // kSplit (three-pass tf32): the result may also leave as its tf32 high and low parts (TcParams::out_hi).
 __device__ __forceinline__ float tf32_rne(float x) {
@@ -132,25 +157,7 @@ __device__ __forceinline__ void epilogue_chunk(const TcParams& p, const uint32_t
     if constexpr (kOutMode == kOutNHWC_S8 || kOutMode == kOutNCHW_S8) {
         uint32_t qw[8];  // the chunk's 32 int8 results, four per word (bytes in channel order)
         requant_chunk(p, v, c0, nch, qw);
-        int8_t* out = static_cast<int8_t*>(p.out);
-        if constexpr (kOutMode == kOutNHWC_S8) {
-            const int pitch = p.out_pitch != 0 ? p.out_pitch : p.Cout;
-            int8_t* dst = out + pix * pitch + c0;
-            if (c0 + 32 <= pitch && (pitch & 15) == 0 && p.vec_ok) {  // (channels beyond Cout are zero and land in the padding)
-                reinterpret_cast<uint4*>(dst)[0] = make_uint4(qw[0], qw[1], qw[2], qw[3]);
-                reinterpret_cast<uint4*>(dst)[1] = make_uint4(qw[4], qw[5], qw[6], qw[7]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    if (j < nch) dst[j] = (int8_t)(qw[j >> 2] >> (8 * (j & 3)));
-            }
-        } else {
-            const size_t plane = (size_t)p.OH * p.OW;
-            int8_t* dst = out + ((size_t)n * p.Cout + c0) * plane + (size_t)oh * p.OW + ow;
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (j < nch) dst[(size_t)j * plane] = (int8_t)(qw[j >> 2] >> (8 * (j & 3)));
-        }
+        store_chunk_s8<kOutMode>(p, qw, c0, nch, n, oh, ow);
         return;
     } else {
         float f[32];

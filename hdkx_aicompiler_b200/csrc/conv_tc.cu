@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
     __shared__ __align__(8) uint64_t bar_acc_empty[2];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
+    [[maybe_unused]] __shared__ int requant_ok;
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -105,6 +106,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
+        if constexpr (kKind == MmaKind::I8) requant_ok = 1;
         for (int s = 0; s < kStages; ++s) {
             mbar_init(smem_u32(&bar_full[s]), 1);
             mbar_init(smem_u32(&bar_empty[s]), 1);
@@ -311,6 +313,24 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
         // (boxes are 64 channels wide: a warp needs an even number of 32-column chunks, which the 192-wide tile lacks)
         const bool boxed = fast && p.store_box && !has_res && (BN >= 128) && (kChunksPerWarp % 2 == 0);
         pdl_wait();  // residual reads and output writes must not overtake earlier kernels
+        // int8: the per-channel constants of the high-word requantize, prepared once per CTA in shared memory (the store boxes
+        // are not used by this type) instead of three loads, a shift and a select per value of every chunk. One channel whose
+        // shift or bias the short formula does not cover, or more channels than fit, and all chunks take the general one.
+        // (256 -> 256 channels, 14x14, 256 images: 31 -> 28 us)
+        [[maybe_unused]] const int4* q_tab = nullptr;
+        if constexpr (kKind == MmaKind::I8) {
+            const int padded = p.tiles_c * BN;
+            int4* tab = reinterpret_cast<int4*>(smem_raw + (ring - smem_u32(smem_raw)) + kStages * G::kStageBytes);
+            const int64_t max_abs_acc = 128ll * 128 * p.taps_h * p.taps_w * p.cblocks * p.kb_elems;
+            if (padded * (int)sizeof(int4) <= G::kEpilogueBytes && max_abs_acc < (1ll << 31)) {
+                for (int c = (int)threadIdx.x - 64; c < padded; c += 256) {
+                    if (c >= p.Cout) tab[c] = make_int4(0, 0, 0, 0);
+                    else if (!requant_prepare(__ldg(p.bias_i32 + c), __ldg(p.multiplier + c), __ldg(p.shift + c), max_abs_acc, &tab[c])) requant_ok = 0;
+                }
+                named_barrier(1, 256);
+                if (*(volatile int*)&requant_ok) q_tab = tab;
+            }
+        }
         int acc = 0;
         uint32_t acc_phase = 0;
         bool alive = true;
@@ -385,6 +405,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                     }
                 } else if (fast) {
                     if (c0 < p.Cout) epilogue_coalesced_bf16<32>(ep, v, c0, stage_tile, lane, rows, res_cur, has_res);
+                } else if (kKind == MmaKind::I8 && q_tab != nullptr) {
+                    if constexpr (kKind == MmaKind::I8) {
+                        if (valid && c0 < p.Cout) {
+                            const int32_t lo_cap = p.relu ? 0 : INT32_MIN;
+                            uint32_t qw[8];
+#pragma unroll
+                            for (int j = 0; j < 32; j += 4) {
+                                const uint32_t vv[4] = {v[j], v[j + 1], v[j + 2], v[j + 3]};
+                                const int4 qq[4] = {q_tab[c0 + j], q_tab[c0 + j + 1], q_tab[c0 + j + 2], q_tab[c0 + j + 3]};
+                                qw[j >> 2] = requant4_prepared(vv, qq, lo_cap);
+                            }
+                            store_chunk_s8<kOutMode>(p, qw, c0, p.Cout - c0 < 32 ? p.Cout - c0 : 32, n, oh, ow);
+                        }
+                    }
                 } else {
                     epilogue_chunk<kOutMode, kX3>(p, v, c0, valid, n, oh, ow, nchw_cur);
                 }

@@ -239,6 +239,18 @@ def test_conv2d_argument_errors(ops):
         ops.nn_conv2d(x, torch.zeros(2, 3, 1, 1, device="cuda"))
 
 
+# Two pixel tiles per work item (more than one wave of tf32 tiles, 64 and 128 channels), an odd number of tiles, full-row boxes in
+# the reference's layout and a residual read ahead of the accumulator. Bound: that of test_conv2d_tensor_core.
+@pytest.mark.parametrize("O", [64, 100])
+def test_conv2d_tf32_two_tiles(ops, rng, O):
+    x, w, b = conv_inputs(rng, 1, 32, 139, 139, O, 1, 1)
+    res = rng.uniform(-1, 1, (1, O, 139, 139)).astype(f32)
+    got = host(ops.nn_conv2d(dev(x), dev(w), dev(b), residual=dev(res), relu=True, precision="tf32"))
+    assert ops.device_status() == 0
+    max_abs, max_rel = ref_metric(got, conv_expect(x, w, b, res, True, 1, 0, 1, port.round_tf32))
+    assert min(max_abs, max_rel) <= 2e-5, f"{O} channels: {max_abs:.3e} {max_rel:.3e}"
+
+
 # Reductions split over clusters of two to eight CTAs, 64 to 256 channels wide (conv_splitk.cu): ragged pixels and channels,
 # stride 2, dilation 2, K ranges that do not divide evenly. Bounds: those of the two tests of the whole reductions.
 @pytest.mark.parametrize("precision,rounder", [("tf32", port.round_tf32), ("bf16", port.round_bf16), ("tf32x3", None)])
