@@ -953,7 +953,7 @@ int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_m
         return !(e != nullptr && e[0] == '1');
     }();
     cfg->mt = (mt_enabled && bn == 128 && dtype == kTcBF16 && out_mode == kOutNHWC_BF16 && kb_bytes == 128 && m_tiles >= 2 * ctas) ? 2 : 1;
-    // tf32 and int8: the tiles of such a launch arrive from L2 at 7 to 8 TB/s over the whole chip whatever the MMAs do, and two
+    // tf32 and int8: the tiles of such a launch reach shared memory at 7 to 8 TB/s over all SMs whatever the MMAs do, and two
     // pixel tiles against one weight tile are 20 / 24 KB per tile instead of 24 / 32 (64 / 128 channels). Taken when the
     // modelled makespan gains: a stage of two tiles costs 820 / 1100 cycles against 490 / 655 (the wider one meets its
     // instructions' ~140 cycles). ResNet-18 tf32, 32 images: layer 1 42 -> 34 us per convolution, layer 2 31 -> 30; int8 128 -> 128,

@@ -199,11 +199,13 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     // memory belong to the next pixel of the same tile row: runs of BW bytes. From 1 MiB of results on (and wherever BW <= 2)
     // the kernel stores NHWC into the workspace instead, pixels padded to 16 channels, and a byte transpose writes the
     // reference layout (128 -> 128 channels, 28x28, 256 images: 65 us of convolution with byte stores against 52 + 12). A
-    // smaller result is not worth the second launch.
+    // smaller result is not worth the second launch, and planes that are no multiple of four bytes have only the byte-wise
+    // transpose (33 -> 27 channels, 101x103, 132 images: 370 us with byte stores, 392 by way of NHWC).
     int bw = 0, bh = 0, bni = 0;
     tc_pick_tile(d.N, d.OH, d.OW, &bw, &bh, &bni);
     const int out_pitch = (d.O + 15) / 16 * 16;
-    bool two_step = bw <= 2 || rowstack_ok || (long long)d.N * d.O * d.OH * d.OW >= (1 << 20);  // (the row-stacked kernel writes NHWC only)
+    bool two_step = bw <= 2 || rowstack_ok ||
+                    ((long long)d.N * d.O * d.OH * d.OW >= (1 << 20) && ((long long)d.OH * d.OW & 3) == 0);  // (the row-stacked kernel writes NHWC only)
     const size_t out_bytes = two_step ? align_up((size_t)d.N * d.OH * d.OW * out_pitch, 1024) : 0;
     StreamScratch ws(s);
     int32_t rc = ws.alloc(act_bytes + w_bytes + out_bytes);
