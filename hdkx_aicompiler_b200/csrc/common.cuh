@@ -34,11 +34,15 @@ inline int32_t check_launch(const char* what) {
     return KXC_B200_OK;
 }
 
+// (A failed call also stays the thread's last error, which the next check_launch would take for its own launch's: it is cleared
+// where it is reported.)
 #define KXC_CUDA_TRY(expr)                                                                         \
     do {                                                                                           \
         cudaError_t _e = (expr);                                                                   \
-        if (_e != cudaSuccess)                                                                     \
+        if (_e != cudaSuccess) {                                                                   \
+            cudaGetLastError();                                                                    \
             return ::kxc_b200::fail(KXC_B200_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(_e)); \
+        }                                                                                          \
     } while (0)
 
 #define KXC_TRY(expr)                     \

@@ -53,6 +53,7 @@ struct StreamScratch {
         cudaError_t e = cudaMallocFromPoolAsync(&ptr, bytes, pool, stream);
         if (e != cudaSuccess) {
             ptr = nullptr;
+            cudaGetLastError();  // reported here: a launch after it (a caller's smaller request) has its own result
             return fail(KXC_B200_ERR_NOMEM, "workspace of %zu bytes: %s", bytes, cudaGetErrorString(e));
         }
         return KXC_B200_OK;

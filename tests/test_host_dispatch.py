@@ -1,0 +1,74 @@
+"""What the library's host code decides, checked without a GPU: its own objects are linked with tests/fake_cudart.cpp in place
+of the CUDA runtime, so a call through the C ABI runs up to its launches, which the fake checks against the grid limits and
+writes down, and calls of the runtime can be made to fail."""
+import ctypes
+import glob
+import os
+import subprocess
+
+import pytest
+
+from hdkx_aicompiler_b200 import _lib
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "hdkx_aicompiler_b200", "csrc")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    objects = ["build/" + os.path.basename(f)[:-3] + ".o" for f in sorted(glob.glob(os.path.join(CSRC, "*.cu")))]
+    subprocess.check_call(["make", "-s", "-j", str(min(16, os.cpu_count() or 4)), "-C", CSRC] + objects)
+    so = str(tmp_path_factory.mktemp("fake") / "libkxc_fake.so")
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I" + os.path.join(CUDA, "include"), "-o", so,
+                           os.path.join(ROOT, "tests", "fake_cudart.cpp")] + [os.path.join(CSRC, o) for o in objects] + ["-ldl", "-lpthread", "-lrt"])
+    lib = ctypes.CDLL(so)
+    for name, (res, args) in _lib.SYMBOLS.items():
+        fn = getattr(lib, name)
+        fn.restype, fn.argtypes = res, args
+    lib.fake_launches.restype = ctypes.c_char_p
+    lib.fake_pool_limit.argtypes = [ctypes.c_size_t]
+    return lib
+
+
+@pytest.fixture(autouse=True)
+def _clean(fake):
+    fake.fake_reset()
+
+
+def launches(fake):
+    return fake.fake_launches().decode().splitlines()
+
+
+def pointers(n):
+    return _lib.packed(*[(i + 1) << 40 for i in range(n)])
+
+
+def conv_s8(fake, n, c, h, w, o, k, s=1):
+    """nn_conv2d_s8 in the reference's layout: return code and message."""
+    d = _lib.Conv2dDesc(n, c, h, w, o, k, k, s, s, k // 2, k // 2, 1, 1, _lib.BIAS, _lib.PREC_FP32)
+    rc = fake.kxc_b200_nn_conv2d_s8(pointers(6), d, None)
+    return rc, fake.kxc_b200_last_error().decode()
+
+
+def test_s8_result_by_way_of_nhwc_falls_back_to_byte_stores(fake):
+    """No room for the second copy of a large result: the convolution writes the reference's layout itself. The failed
+    allocation must not be taken for the failure of the first launch after it."""
+    case = (256, 128, 28, 28, 128, 3)
+    assert conv_s8(fake, *case)[0] == 0
+    assert "transpose_bytes" in launches(fake)[-1]
+    fake.fake_reset()
+    operands = 256 * 28 * 28 * 128 + 128 * 9 * 128
+    fake.fake_pool_limit(operands + 4096)
+    rc, message = conv_s8(fake, *case)
+    assert rc == 0, message
+    assert "conv_igemm" in launches(fake)[-1]
+
+
+def test_refused_workspace_leaves_no_error_behind(fake):
+    fake.fake_pool_limit(1000)
+    rc, message = conv_s8(fake, 4, 64, 28, 28, 100, 3)
+    assert rc != 0 and "workspace" in message
+    fake.fake_pool_limit(1 << 40)
+    rc, message = conv_s8(fake, 4, 64, 28, 28, 100, 3)
+    assert rc == 0, message
