@@ -117,11 +117,12 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
 // 32-byte runs the element-wise kernel makes of 1-byte elements). grid (ceil(HW/64), ceil(cpad/64), N), block 256.
 // It is a batched byte transpose [C][HW] -> [HW][cpad] (rows c >= C read as zero), so it also serves NHWC -> NCHW with
 // the roles of the two extents exchanged (source rows `pitch` bytes apart); vec_out = 0 when the destination rows are not 4-byte multiples.
+// rows_on_x (here and in transpose_bytes_kernel): the first two grid dimensions are exchanged, see transpose_grid.
 __global__ void __launch_bounds__(256) nchw_to_nhwc_s8_kernel(const int8_t* __restrict__ in, int8_t* __restrict__ out, int C, int HW,
-                                                               int pitch, int cpad, int vec_in, int vec_out) {
+                                                               int pitch, int cpad, int vec_in, int vec_out, int rows_on_x) {
     __shared__ __align__(4) int8_t tile[64][68];
     const int n = blockIdx.z;
-    const int hw0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
+    const int hw0 = (int)(rows_on_x ? blockIdx.y : blockIdx.x) * 64, c0 = (int)(rows_on_x ? blockIdx.x : blockIdx.y) * 64;
     const int8_t* src = in + (size_t)n * C * pitch;
     int8_t* dst = out + (size_t)n * HW * cpad;
     const int q = threadIdx.x & 15, r = threadIdx.x >> 4;  // 16 four-byte columns x 16 rows per pass
@@ -169,9 +170,9 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_s8_kernel(const int8_t* __re
 // Tile 64 rows x TP columns. grid (ceil(W/TP), ceil(max(R, opitch)/64), batch), block 256.
 template <int V, int TP>
 __global__ void __launch_bounds__(256) transpose_bytes_kernel(const int8_t* __restrict__ in, int8_t* __restrict__ out, int R, int W, int pitch,
-                                                               int opitch) {
+                                                               int opitch, int rows_on_x) {
     __shared__ uint32_t tile[TP * 16];
-    const int w0 = blockIdx.x * TP, r0 = blockIdx.y * 64;
+    const int w0 = (int)(rows_on_x ? blockIdx.y : blockIdx.x) * TP, r0 = (int)(rows_on_x ? blockIdx.x : blockIdx.y) * 64;
     const int8_t* src = in + (int64_t)blockIdx.z * R * pitch;
     int8_t* dst = out + (int64_t)blockIdx.z * W * opitch;
     auto slot = [](int p, int q) { return p * 16 + (q ^ (((p >> 2) ^ (p >> 4)) & 15)); };
@@ -211,14 +212,22 @@ __global__ void __launch_bounds__(256) transpose_bytes_kernel(const int8_t* __re
     }
 }
 
+// Grid of a batched transpose: column tiles, row tiles, batch. The row tiles of a whole plane (NHWC -> NCHW: pixels) can be more
+// than the 65535 that the second dimension holds; they change places with the column tiles then, of which there are few.
+dim3 transpose_grid(int cols, int rows, int batch, int* rows_on_x) {
+    *rows_on_x = rows > 65535 ? 1 : 0;
+    return *rows_on_x ? dim3((unsigned)rows, (unsigned)cols, (unsigned)batch) : dim3((unsigned)cols, (unsigned)rows, (unsigned)batch);
+}
+
 // Batched byte transpose of `batch` matrices; false when the pitches or addresses do not suit the kernel above.
 bool transpose_bytes(const int8_t* in, int8_t* out, int batch, int R, int W, int pitch, int opitch, cudaStream_t s) {
     const uintptr_t a = reinterpret_cast<uintptr_t>(in);
     if ((pitch & 3) != 0 || (opitch & 3) != 0 || (a & 3u) != 0 || (reinterpret_cast<uintptr_t>(out) & 3u) != 0) return false;
     const bool wide = (pitch & 15) == 0 && (a & 15u) == 0;
     const int tp = W <= 64 ? 64 : (W <= 128 ? 128 : 256);
-    const dim3 grid((W + tp - 1) / tp, ((R > opitch ? R : opitch) + 63) / 64, batch);
-    auto go = [&](auto kernel) { kernel<<<grid, 256, 0, s>>>(in, out, R, W, pitch, opitch); };
+    int rows_on_x = 0;
+    const dim3 grid = transpose_grid((W + tp - 1) / tp, ((R > opitch ? R : opitch) + 63) / 64, batch, &rows_on_x);
+    auto go = [&](auto kernel) { kernel<<<grid, 256, 0, s>>>(in, out, R, W, pitch, opitch, rows_on_x); };
     if (wide) {
         if (tp == 64) go(transpose_bytes_kernel<16, 64>);
         else if (tp == 128) go(transpose_bytes_kernel<16, 128>);
@@ -344,8 +353,9 @@ int32_t nchw_to_nhwc(const void* in, void* out, TcDType dtype, int N, int C, int
             if (transpose_bytes(static_cast<const int8_t*>(in), static_cast<int8_t*>(out), N, C, HW, HW, cpad, s)) break;
             if ((cpad & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 3u) == 0) {
                 const int vec_in = ((HW & 3) == 0 && (reinterpret_cast<uintptr_t>(in) & 3u) == 0) ? 1 : 0;
-                nchw_to_nhwc_s8_kernel<<<dim3((HW + 63) / 64, (cpad + 63) / 64, N), 256, 0, s>>>(static_cast<const int8_t*>(in),
-                                                                                                static_cast<int8_t*>(out), C, HW, HW, cpad, vec_in, 1);
+                int rows_on_x = 0;
+                const dim3 g = transpose_grid((HW + 63) / 64, (cpad + 63) / 64, N, &rows_on_x);
+                nchw_to_nhwc_s8_kernel<<<g, 256, 0, s>>>(static_cast<const int8_t*>(in), static_cast<int8_t*>(out), C, HW, HW, cpad, vec_in, 1, rows_on_x);
             } else {
                 nchw_to_nhwc_kernel<int8_t, int8_t><<<grid, block, 0, s>>>(static_cast<const int8_t*>(in), static_cast<int8_t*>(out), C, HW, cpad, overlap ? 1 : 0);
             }
@@ -404,7 +414,9 @@ int32_t nhwc_to_nchw_s8(const int8_t* in, int8_t* out, int N, int C, int pitch, 
     if (!transpose_bytes(in, out, N, HW, C, pitch, HW, s)) {
         const int vec_in = ((pitch & 3) == 0 && (reinterpret_cast<uintptr_t>(in) & 3u) == 0) ? 1 : 0;
         const int vec_out = ((HW & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 3u) == 0) ? 1 : 0;
-        nchw_to_nhwc_s8_kernel<<<dim3((C + 63) / 64, (HW + 63) / 64, N), 256, 0, s>>>(in, out, HW, C, pitch, HW, vec_in, vec_out);
+        int rows_on_x = 0;
+        const dim3 g = transpose_grid((C + 63) / 64, (HW + 63) / 64, N, &rows_on_x);
+        nchw_to_nhwc_s8_kernel<<<g, 256, 0, s>>>(in, out, HW, C, pitch, HW, vec_in, vec_out, rows_on_x);
     }
     return check_launch("nhwc_to_nchw_s8");
 }

@@ -72,3 +72,11 @@ def test_refused_workspace_leaves_no_error_behind(fake):
     fake.fake_pool_limit(1 << 40)
     rc, message = conv_s8(fake, 4, 64, 28, 28, 100, 3)
     assert rc == 0, message
+
+
+# planes of more than 64 * 65535 pixels: the byte transposes' row tiles no longer fit the grid's second dimension; a plane that is
+# a multiple of four bytes takes the register transpose, an odd one (64 -> 64 channels, 3x3: always by way of NHWC) the byte-wise one
+@pytest.mark.parametrize("case", [(1, 16, 2048, 2048, 16, 1), (2, 8, 3000, 2000, 24, 3), (1, 64, 2049, 2049, 64, 3)])
+def test_s8_planes_beyond_the_second_grid_dimension(fake, case):
+    rc, message = conv_s8(fake, *case)
+    assert rc == 0, message

@@ -303,6 +303,14 @@ def test_conv2d_s8_layouts(ops, rng, N, C, H, W, O):
     assert torch.equal(got, ops.nn_conv2d_s8(x, w, b, m, sh, (1, 1), (1, 1), simt=True))
 
 
+# One plane of 4,194,308 pixels: its 64-row tiles are more than the second grid dimension holds
+def test_conv2d_s8_plane_beyond_the_second_grid_dimension(ops, rng):
+    x, w, b, m, sh = (dev(a) for a in s8_inputs(rng, 1, 3, 1048577, 4, 5, 1, 1))
+    got = ops.nn_conv2d_s8(x, w, b, m, sh)
+    assert ops.device_status() == 0
+    assert torch.equal(got, ops.nn_conv2d_s8(x, w, b, m, sh, simt=True))
+
+
 # ---------------------------------------------------------------- dense / gemm
 @pytest.mark.parametrize("M,N,K", [(2, 2, 3), (2, 4, 3), (5, 11, 37), (33, 1000, 512), (130, 72, 200), (0, 4, 8)])
 def test_gemm_fp32_mode_bit_exact(ops, rng, M, N, K):
