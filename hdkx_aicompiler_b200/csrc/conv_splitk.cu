@@ -450,7 +450,7 @@ int tc_split_capacity(int split) {
         if (cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, G::kSmemBytes) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&found, kernel, &lc) != cudaSuccess || found < 0) {
             cudaGetLastError();
-            found = 0;
+            return 0;  // not kept: the next call asks again
         }
         n = (found < kNumSMs / split ? found : kNumSMs / split) + 1;
     }

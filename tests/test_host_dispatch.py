@@ -51,6 +51,28 @@ def conv_s8(fake, n, c, h, w, o, k, s=1):
     return rc, fake.kxc_b200_last_error().decode()
 
 
+def conv(fake, precision, n, c, h, w, o, k, s=1, residual=False):
+    """nn_conv2d with a bias: return code and message."""
+    flags = _lib.BIAS | (_lib.RESIDUAL if residual else 0)
+    d = _lib.Conv2dDesc(n, c, h, w, o, k, k, s, s, k // 2, k // 2, 1, 1, flags, precision)
+    rc = fake.kxc_b200_nn_conv2d(pointers(4 + residual), d, None)
+    return rc, fake.kxc_b200_last_error().decode()
+
+
+# (first of the split-reduction tests: what a query answered is kept for the rest of the process)
+def test_failed_occupancy_query_is_asked_again(fake):
+    """How many clusters fit at once is asked once per size. A query that fails leaves that launch unsplit and no more."""
+    case = (_lib.PREC_BF16, 1, 512, 7, 7, 512, 3)
+    fake.fake_fail_occupancy(1000)
+    rc, message = conv(fake, *case)
+    assert rc == 0, message
+    assert "conv_igemm" in launches(fake)[-1]
+    fake.fake_reset()
+    rc, message = conv(fake, *case)
+    assert rc == 0, message
+    assert "conv_splitk" in launches(fake)[-1]
+
+
 def test_s8_result_by_way_of_nhwc_falls_back_to_byte_stores(fake):
     """No room for the second copy of a large result: the convolution writes the reference's layout itself. The failed
     allocation must not be taken for the failure of the first launch after it."""
