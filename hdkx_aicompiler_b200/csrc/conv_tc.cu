@@ -793,29 +793,41 @@ int32_t weight_map(CUtensorMap* m, const TcConfig* cfg, const TcParams* p, const
 }
 
 // Whether a set-up launch (tile width, store form and so on already chosen for the persistent kernel) is better off with its
-// reduction split over a cluster, and the set-up of that form. Modelled in cycles: a K block of 128 bytes per row costs what
-// its stage takes to arrive at ~50 B/clk per SM (x3: what its instructions take); ~1500 cycles per launch for filling the
-// pipeline and the epilogue, as much again for the cluster barriers and the exchange. It has to gain 10 %. A launch is kept to
-// the clusters that the chip holds at once (a dense layer of 16 tiles in clusters of eight that did not all fit: 8.8 -> 12 us).
+// reduction split over a cluster, and the set-up of that form: the cheaper of the two in modelled cycles, the split one 5 % ahead.
+// The figures are fits over 320 launches timed in every form that fits the chip (7 layers in a row, NHWC, and one layer
+// into NCHW; 16 to 144 K blocks; 1 to 96 images), in clocks of 1.9 GHz:
+//   a K block of 128 bytes per row     550 / 590 / 500 / 620 at 64 / 128 / 192 / 256 channels, 650 at 256 in the split kernel;
+//                                      760 with two bf16 pixel tiles, 820 / 1100 with two tf32 ones; three passes 830 / 1050, split 830 / 930
+//   what follows the last K block      unsplit 0 / 2000 / 4000 / 8000 (the epilogue of that many channels), 2800 more with two pixel
+//                                      tiles; split 3000 / 7000 / 13000 (both cluster barriers, the exchange of the partial
+//                                      sums over distributed shared memory and the epilogue, all of which grow with the width)
+// Over the same launches what this chooses is 0.3 % (NHWC) and 1.4 % (NCHW) behind the fastest form on average, and one launch
+// is behind the unsplit one by more than 1 %. (One figure for every width, 3000, made wide splits of short reductions slower than no split: bf16
+// 1024 -> 1024 1x1 at 7x7 and 24 images 14.7 us per layer in two parts of 256 channels, 11.3 unsplit; 256 -> 256 3x3 at
+// 14x14 and 32 images 19.4 and 17.8.) A launch is kept to the clusters that the chip holds at once (a dense layer of 16
+// tiles in clusters of eight that did not all fit: 8.8 -> 12 us).
 int32_t choose_split(TcParams* p, TcConfig* cfg, const void* w, const void* w_lo, int k_elems) {
     p->split = 0;
     if (cfg->dtype == kTcS8 || cfg->kb_bytes != 128) return KXC_B200_OK;
     const long long m_tiles = (long long)p->tiles_w * p->tiles_h * p->tiles_n;
     const int kb = p->taps_h * p->taps_w * p->cblocks;
     if (kb < 12) return KXC_B200_OK;  // two or three microseconds as it is
-    auto stage_cycles = [&](int bn) {
-        return cfg->x3 ? (bn == 64 ? 950 : 1400) : (bn == 64 ? 490 : (bn == 128 ? 655 : (bn == 256 && cfg->ctas == 1 ? 980 : 800)));
-    };
+    const bool wide_items = cfg->mt == 2;
+    const long long block = cfg->x3 ? (cfg->bn == 64 ? 830 : 1050)
+                            : wide_items ? (cfg->dtype == kTcBF16 ? 760 : (cfg->bn == 64 ? 820 : 1100))
+                                         : (cfg->bn == 64 ? 550 : (cfg->bn == 128 ? 590 : (cfg->bn == 192 ? 500 : 620)));
+    const long long tail = (cfg->bn == 64 ? 0 : (cfg->bn == 128 ? 2000 : (cfg->bn == 192 ? 4000 : 8000))) + (wide_items ? 2800 : 0);
     const long long group = (long long)cfg->ctas * cfg->mt;
     const long long items = p->tiles_c * ((m_tiles + group - 1) / group), slots = kNumSMs / cfg->ctas;
-    const long long whole = (items + slots - 1) / slots * kb * (cfg->mt == 2 ? (cfg->bn == 64 ? 820 : 1100) : stage_cycles(cfg->bn)) + 1500;
-    long long best = whole * 9 / 10;
+    long long best = ((items + slots - 1) / slots * kb * block + tail) * 95 / 100;
     int split = 0, width = 0;
     for (int bn = 64; bn <= 256 && (bn == 64 || bn / 2 < p->Cout) && !(bn == 256 && cfg->x3); bn *= 2) {
         const long long tiles = m_tiles * ((p->Cout + bn - 1) / bn);
+        const long long split_block = cfg->x3 ? (bn == 64 ? 830 : 930) : (bn == 64 ? 550 : (bn == 128 ? 590 : 650));
+        const long long split_tail = bn == 64 ? 3000 : (bn == 128 ? 7000 : 13000);
         for (int s = 2; s <= kMaxSplit && tiles * s <= kNumSMs; ++s) {
             if (tiles > tc_split_capacity(s)) continue;
-            const long long span = (long long)((kb + s - 1) / s) * (bn == 256 ? 980 : stage_cycles(bn)) + 3000;
+            const long long span = (long long)((kb + s - 1) / s) * split_block + split_tail;
             if (span < best) {
                 best = span;
                 split = s;

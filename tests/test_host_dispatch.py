@@ -102,3 +102,22 @@ def test_refused_workspace_leaves_no_error_behind(fake):
 def test_s8_planes_beyond_the_second_grid_dimension(fake, case):
     rc, message = conv_s8(fake, *case)
     assert rc == 0, message
+
+
+# Measured: the split form (two parts of 256 / 128 channels) takes 22.2, 28.2, 28.3 and 20.7 us where the whole reduction takes
+# 16.4, 23.3, 22.7 and 18.6
+@pytest.mark.parametrize("precision,case", [(_lib.PREC_TF32, (7, 42, 28, 30, 508, 3, 2)), (_lib.PREC_BF16, (6, 236, 22, 22, 313, 3, 1)),
+                                            (_lib.PREC_BF16, (13, 86, 47, 50, 230, 3, 2)), (_lib.PREC_TF32X3, (9, 50, 32, 35, 313, 3, 2))])
+def test_reductions_are_not_split_where_that_costs_time(fake, precision, case):
+    rc, message = conv(fake, precision, *case)
+    assert rc == 0, message
+    assert "conv_igemm" in launches(fake)[-1], launches(fake)[-1]
+
+
+# ... and stay split where it pays: 1 to 16 images of the deep layers (2.9 to 1.1 times as fast)
+@pytest.mark.parametrize("precision", [_lib.PREC_BF16, _lib.PREC_TF32, _lib.PREC_TF32X3])
+@pytest.mark.parametrize("case", [(1, 256, 14, 14, 256, 3), (1, 512, 7, 7, 512, 3), (8, 512, 7, 7, 512, 3), (16, 512, 7, 7, 512, 3)])
+def test_reductions_are_split_where_sms_would_idle(fake, precision, case):
+    rc, message = conv(fake, precision, *case)
+    assert rc == 0, message
+    assert "conv_splitk" in launches(fake)[-1], launches(fake)[-1]
