@@ -13,7 +13,7 @@
 //   warp 1      MMA issuer, TMEM owner
 //   warps 2..9  accumulator -> shared memory, then reduction and epilogue, 8 channels of one pixel per thread and step
 //
-// The shape of the launch (S, BN) comes from choose_split in conv_tc.cu. Waits are bounded as in conv_tc.cu; the cluster
+// The shape of the launch (S, BN) comes from choose_split or, with two outputs, tc_setup_dual in conv_tc.cu. Waits are bounded as in conv_tc.cu; the cluster
 // barriers are reached by every thread of every CTA whether or not a wait ran out.
 #include "conv_tc.cuh"
 
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __g
     const int kb_main = p.taps_h * p.taps_w * p.cblocks;
     const int kb_all = kb_main + (kDual ? p.cblocks : 0);
     // The second output's few blocks go to the last rank alone: its sum is formed in the order of a launch of its own, and the
-    // main sum's parts are those of a launch without it (bit-identical either way).
+    // main sum's parts are those of a launch without it in as many parts (bit-identical then).
     const int kb0 = rank * kb_main / S, kb1 = rank == S - 1 ? kb_all : (rank + 1) * kb_main / S;
     const int ct = tile % p.tiles_c;
     int r = tile / p.tiles_c;
@@ -411,9 +411,7 @@ int32_t launch_split(const TcParams& p, cudaStream_t s) {
 template <MmaKind kKind, int kOutMode, bool kX3>
 int32_t launch_by_width(const TcConfig& cfg, const TcParams& p, cudaStream_t s) {
     if constexpr (kKind == MmaKind::F16 && kOutMode == kOutNHWC_BF16) {
-        if (cfg.dual) {
-            return cfg.bn == 64 ? launch_split<kKind, 64, kOutMode, true, false>(p, s) : launch_split<kKind, 128, kOutMode, true, false>(p, s);
-        }
+        if (cfg.dual) return launch_split<kKind, 64, kOutMode, true, false>(p, s);  // (the only width of it, tc_setup_dual)
     }
     if (cfg.dual) return fail(KXC_B200_ERR_INVALID, "split-reduction conv: no two-output form for this configuration");
     if constexpr (!kX3) {
@@ -458,7 +456,7 @@ int tc_split_capacity(int split) {
 }
 
 int32_t tc_launch_split(const TcConfig& cfg, const TcParams& p, cudaStream_t s) {
-    if (p.split < 2 || p.split > kMaxSplit || (cfg.bn != 64 && cfg.bn != 128 && (cfg.bn != 256 || cfg.x3 || cfg.dual)) || cfg.kb_bytes != kKB)
+    if (p.split < 2 || p.split > kMaxSplit || (cfg.bn != 64 && (cfg.dual || (cfg.bn != 128 && (cfg.bn != 256 || cfg.x3)))) || cfg.kb_bytes != kKB)
         return fail(KXC_B200_ERR_INVALID, "split-reduction conv: %d parts, %d channels, %d-byte K blocks", p.split, cfg.bn, cfg.kb_bytes);
     if (cfg.dtype == kTcBF16) {
         switch (cfg.out_mode) {

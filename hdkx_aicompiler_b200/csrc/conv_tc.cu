@@ -854,13 +854,30 @@ bool tc_dual_applicable(TcDType dtype, TcOutMode out_mode, int cpad, int Cout, i
 int32_t tc_setup_dual(TcParams* p, TcConfig* cfg, const void* act_nhwc, const void* w_packed, const void* w2_packed, int N,
                       int H, int W, int cpad, int Cout, int KH, int KW, int stride, int pad_h, int pad_w) {
     KXC_TRY(tc_setup_conv(p, cfg, kTcBF16, kOutNHWC_BF16, act_nhwc, w_packed, N, H, W, cpad, Cout, KH, KW, stride, pad_h, pad_w, 1, 1));
-    if (p->split > 1) {  // the main sum's split is that of a launch without the second output (same bits)
-        cfg->dual = 1;
-        if (cfg->bn > 128) {  // (no 256-wide form of it: two narrower tiles, the same sums)
-            cfg->bn = 128;
-            p->tiles_c = (Cout + 127) / 128;
-            KXC_TRY(weight_map(&p->tmB, cfg, p, w_packed, KH * KW * cpad));
+    cfg->ctas = 1; cfg->mt = 1; cfg->dual = 1;
+    p->split = 0;  // (that of the main convolution alone)
+    const long long m_tiles = (long long)p->tiles_w * p->tiles_h * p->tiles_n;
+    auto waves = [](long long items) { return (items + kNumSMs - 1) / kNumSMs; };
+    // Split over clusters as in choose_split, by the clusters of this form and with the second output's K blocks behind the last
+    // rank's own. Its partial sums double the exchange, which leaves nothing to gain for tiles wider than 64 channels:
+    // 256 -> 512 at 14x14, block of four layers, us unsplit / 64 wide / 128 wide: one image 35.0 / 24.8 / 26.9, 8 images
+    // 35.5 / 30.9 / 32.9, 16 images 41.2 / 37.1 / 37.1, 24 images 45.3 / - / 45.3; 128 -> 256 at 28x28: 4 images
+    // 28.9 / 27.2 / 29.3, 8 images 33.1 / 31.5 / 33.3.
+    const int kb = KH * KW * p->cblocks;
+    const long long tiles64 = m_tiles * ((Cout + 63) / 64);
+    long long best = (waves(m_tiles * ((Cout + 127) / 128)) * (kb + p->cblocks) * 590 + 4000) * 95 / 100;
+    for (int s = 2; kb >= 12 && s <= kMaxSplit && tiles64 * s <= kNumSMs; ++s) {
+        if (tiles64 > tc_split_capacity(s)) continue;
+        const long long span = (long long)(kb - (s - 1) * kb / s + p->cblocks) * 550 + 4400;
+        if (span < best) {
+            best = span;
+            p->split = s;
         }
+    }
+    if (p->split > 1) {
+        cfg->bn = 64;
+        p->tiles_c = (Cout + 63) / 64;
+        KXC_TRY(weight_map(&p->tmB, cfg, p, w_packed, KH * KW * cpad));
         return weight_map(&p->tmB2, cfg, p, w2_packed, cpad);
     }
     // The two accumulators of a buffer share TMEM: 128-wide tiles (two buffers of 2 x 128 columns), single CTAs. When
@@ -869,13 +886,11 @@ int32_t tc_setup_dual(TcParams* p, TcConfig* cfg, const void* act_nhwc, const vo
     // epilogue no longer overlaps the next item's MMAs, which a CTA with a single work item does not miss.
     int bn = 128;
     {
-        const long long m_tiles = (long long)p->tiles_w * p->tiles_h * p->tiles_n;
-        auto waves = [](long long items) { return (items + kNumSMs - 1) / kNumSMs; };
         const long long t128 = m_tiles * ((Cout + 127) / 128), t192 = m_tiles * ((Cout + 191) / 192);
         static const bool model = [] { const char* e = getenv("KXC_B200_TILE_MODEL"); return !(e != nullptr && e[0] == '0'); }();
         if (model && p->kb_elems * 2 == 128 && waves(t192) == 1 && waves(t128) >= 2) bn = 192;  // (192-wide tiles need 128-byte K blocks)
     }
-    cfg->bn = bn; cfg->ctas = 1; cfg->mt = 1; cfg->dual = 1;
+    cfg->bn = bn;
     p->tiles_c = (Cout + bn - 1) / bn;
     const uint64_t ktot = (uint64_t)KH * KW * cpad;
     const uint64_t bdims[2] = {ktot, (uint64_t)Cout};

@@ -1,14 +1,16 @@
 """What the library's host code decides, checked without a GPU: its own objects are linked with tests/fake_cudart.cpp in place
 of the CUDA runtime, so a call through the C ABI runs up to its launches, which the fake checks against the grid limits and
 writes down, and calls of the runtime can be made to fail."""
+import contextlib
 import ctypes
 import glob
 import os
 import subprocess
 
 import pytest
+import torch
 
-from hdkx_aicompiler_b200 import _lib
+from hdkx_aicompiler_b200 import _lib, plan, resnet18
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "hdkx_aicompiler_b200", "csrc")
@@ -121,3 +123,58 @@ def test_reductions_are_split_where_sms_would_idle(fake, precision, case):
     rc, message = conv(fake, precision, *case)
     assert rc == 0, message
     assert "conv_splitk" in launches(fake)[-1], launches(fake)[-1]
+
+
+class DeviceTensor:
+    """What a plan asks of a constant: a shape and an address (that nothing reads)."""
+    is_cuda, dtype = True, torch.float32
+
+    def __init__(self, array):
+        self.shape = array.shape
+
+    def is_contiguous(self):
+        return True
+
+    def data_ptr(self):
+        return 1 << 40
+
+
+@pytest.fixture
+def compile_graph(fake, monkeypatch):
+    for name, (res, args) in plan._PLAN_SYMBOLS.items():
+        fn = getattr(fake, name)
+        fn.restype, fn.argtypes = res, args
+    monkeypatch.setattr(plan, "load", lambda: fake)
+    monkeypatch.setattr(_lib, "load", lambda: fake)
+    monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
+
+    def run(func, precision):
+        """The launches of one run of the compiled graph, with their clusters: (kernel, CTAs, CTAs of a cluster)."""
+        graph = plan.CompiledGraph(func, precision=precision, device="cpu")
+        fake.fake_reset()
+        rc = fake.kxc_b200_plan_run(graph.handle, _lib.packed(*[1 << 41] * len(func.params), *graph._const_ptrs, 1 << 42), None)
+        assert rc == 0, fake.kxc_b200_last_error()
+        out = []
+        for line in launches(fake):
+            words = line.split()
+            out.append((words[0], int(words[2]) * int(words[3]) * int(words[4]), int(words[-1])))
+        return graph, out
+
+    return run
+
+
+# clusters of 2..8 CTAs that the chip holds at once (fake_cudart.cpp answers the same)
+HELD = {2: 74, 3: 45, 4: 33, 5: 26, 6: 22, 7: 15, 8: 15}
+
+
+@pytest.mark.parametrize("precision", ["bf16", "tf32", "tf32x3"])
+def test_no_split_launch_of_a_network_needs_more_clusters_than_fit(compile_graph, precision):
+    weights = resnet18.make_weights(0)
+    two_outputs = 0
+    for n in list(range(1, 65)) + [80, 96, 128]:
+        graph, run = compile_graph(resnet18.build(n, weights, to_constant=DeviceTensor), precision)
+        for name, ctas, cluster in run:
+            if "conv_splitk" in name:
+                assert ctas <= 148 and ctas // cluster <= HELD[cluster], f"{n} images: {ctas // cluster} clusters of {cluster}"
+        two_outputs += sum("second output" in label and "split" in label for label, _, _ in graph.launch_info())
+    assert (two_outputs > 0) == (precision == "bf16")

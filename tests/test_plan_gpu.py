@@ -318,6 +318,22 @@ def test_downsample_block_two_output_kernel_is_bit_identical(kxc, monkeypatch, c
         assert np.isfinite(fused).all() and float(np.abs(fused).max()) > 0
 
 
+# The two-output launch chooses its own split: in two and four parts (the single launch's, so the bits are equal) at 8 images, none
+# at 32, where clusters of the main convolution's split would not all fit
+@pytest.mark.parametrize("cin,cout,hw,N,split", [(128, 256, 28, 8, "split2"), (256, 512, 14, 8, "split4"), (128, 256, 28, 32, "")])
+def test_downsample_block_split_of_the_two_output_kernel(kxc, monkeypatch, cin, cout, hw, N, split):
+    labels = []
+    compiled = kxc.plan.CompiledGraph.launch_info
+
+    def launch_info(graph):
+        labels.extend(l[0] for l in compiled(graph))
+        return compiled(graph)
+
+    monkeypatch.setattr(kxc.plan.CompiledGraph, "launch_info", launch_info)
+    test_downsample_block_two_output_kernel_is_bit_identical(kxc, monkeypatch, cin, cout, hw, N)
+    assert all(l.endswith("second output" + (" " + split if split else "")) for l in labels if "second output" in l)
+
+
 @pytest.mark.parametrize("n,h,w", [(2, 56, 56), (3, 30, 20), (1, 7, 5), (2, 14, 8), (1, 15, 9)])
 def test_64_channel_3x3_kernels_agree(kxc, monkeypatch, n, h, w):
     """Two 64 -> 64 3x3 layers (+bias, +relu, the second with a residual) through the row-stacked kernel (three filter
