@@ -6,7 +6,8 @@
 //   max pool  m = -inf; v = inb ? x : -1e30f; m = (m > v) ? m : v  (include/te/topi/nn.h:161-229)
 //   gap       s = 0; s = s + x over (h, w) in order; s / (float)(H*W)  (include/te/topi/nn.h:260-287)
 //   add/relu  one fp32 add, `x > 0 ? x : 0`  (include/te/topi/broadcast.h:90-109, nn.h:19-30)
-// with bf16 storage rounding (nearest even) applied when a result is written back as bf16.
+// with the storage's rounding (nearest even) applied when a result is written back: to bf16, to tf32 (fp32 storage of a tf32
+// plan), or none (three-pass tf32 plans keep full fp32 values).
 #include "nhwc_kernels.cuh"
 
 #include <cuda_bf16.h>
@@ -64,6 +65,17 @@ struct Vec<float> {
     __device__ static void store(float* p, const float (&f)[4]) {
         *reinterpret_cast<float4*>(p) = make_float4(rnd(f[0]), rnd(f[1]), rnd(f[2]), rnd(f[3]));
     }
+};
+
+// fp32 storage whose values are not tensor-core operands themselves (three-pass tf32 plans split them afterwards)
+struct FullF32 {
+    float v;
+};
+template <>
+struct Vec<FullF32> {
+    static constexpr int kLanes = 4;
+    __device__ static void load(const FullF32* p, float (&f)[4]) { Vec<float>::load(reinterpret_cast<const float*>(p), f); }
+    __device__ static void store(FullF32* p, const float (&f)[4]) { *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]); }
 };
 
 template <typename T>
@@ -359,42 +371,50 @@ int grid_for(int64_t items, int per_sm = 8) {
         return fail(KXC_B200_ERR_INVALID, "activation dtype"); \
     }
 
+// the same for results of pooling and elementwise kernels: `full` keeps fp32 storage unrounded
+#define KXC_DISPATCH_STORED(dtype, full, ...)                \
+    if ((dtype) == kTcTF32 && (full)) {                      \
+        using T = FullF32;                                   \
+        __VA_ARGS__;                                         \
+    } else                                                   \
+        KXC_DISPATCH_ACT(dtype, __VA_ARGS__)
+
 int32_t maxpool_nhwc(const void* x, void* out, TcDType dt, int N, int H, int W, int C, int OH, int OW, int KH, int KW, int SH,
-                     int SW, int PT, int PL, cudaStream_t s) {
+                     int SW, int PT, int PL, cudaStream_t s, bool full) {
     const int lanes = dt == kTcBF16 ? 8 : 4;
     if (C % lanes != 0) return fail(KXC_B200_ERR_UNSUPPORTED, "NHWC max pool: %d channels is not a multiple of %d", C, lanes);
     const int64_t items = (int64_t)N * OH * OW * (C / lanes);
     if (items == 0) return KXC_B200_OK;
     if (KH == 3 && KW == 3 && SH == 2 && SW == 2 && PT == 1 && PL == 1 && (OH % 2) == 0 && (OW % 2) == 0 && OH == (H + 2 - 3) / 2 + 1 &&
         OW == (W + 2 - 3) / 2 + 1) {
-        KXC_DISPATCH_ACT(dt, (maxpool3x3s2p1_nhwc_kernel<T><<<grid_for(items / 4, 16), kThreads, 0, s>>>(
+        KXC_DISPATCH_STORED(dt, full, (maxpool3x3s2p1_nhwc_kernel<T><<<grid_for(items / 4, 16), kThreads, 0, s>>>(
                                  static_cast<const T*>(x), static_cast<T*>(out), N, H, W, C, OH, OW)));
         return check_launch("maxpool3x3s2p1_nhwc");
     }
-    KXC_DISPATCH_ACT(dt, (maxpool_nhwc_kernel<T><<<grid_for(items, 16), kThreads, 0, s>>>(
+    KXC_DISPATCH_STORED(dt, full, (maxpool_nhwc_kernel<T><<<grid_for(items, 16), kThreads, 0, s>>>(
                              static_cast<const T*>(x), static_cast<T*>(out), N, H, W, C, OH, OW, KH, KW, SH, SW, PT, PL)));
     return check_launch("maxpool_nhwc");
 }
 
-int32_t gap_nhwc(const void* x, void* out, TcDType dt, int N, int HW, int C, cudaStream_t s) {
+int32_t gap_nhwc(const void* x, void* out, TcDType dt, int N, int HW, int C, cudaStream_t s, bool full) {
     const int lanes = dt == kTcBF16 ? 8 : 4;
     if (C % lanes != 0) return fail(KXC_B200_ERR_UNSUPPORTED, "NHWC global pool: %d channels is not a multiple of %d", C, lanes);
     const int64_t items = (int64_t)N * (C / lanes);
     if (items == 0) return KXC_B200_OK;
     cudaError_t err = cudaSuccess;
     const int blocks = (int)std::min<int64_t>((items + 31) / 32, (int64_t)kNumSMs * 16);
-    KXC_DISPATCH_ACT(dt, (err = launch_kernel(gap_nhwc_split_kernel<T>, dim3(blocks), dim3(kThreads), 0, s, /*pdl=*/true, 1,
+    KXC_DISPATCH_STORED(dt, full, (err = launch_kernel(gap_nhwc_split_kernel<T>, dim3(blocks), dim3(kThreads), 0, s, /*pdl=*/true, 1,
                                               static_cast<const T*>(x), static_cast<T*>(out), N, HW, C)));
     if (err != cudaSuccess) return fail(KXC_B200_ERR_CUDA, "gap_nhwc launch: %s", cudaGetErrorString(err));
     return check_launch("gap_nhwc");
 }
 
-int32_t eltwise_nhwc(const void* a, const void* b, void* out, TcDType dt, int64_t numel, int relu, cudaStream_t s) {
+int32_t eltwise_nhwc(const void* a, const void* b, void* out, TcDType dt, int64_t numel, int relu, cudaStream_t s, bool full) {
     const int lanes = dt == kTcBF16 ? 8 : 4;
     if (numel % lanes != 0) return fail(KXC_B200_ERR_UNSUPPORTED, "NHWC elementwise: %lld elements is not a multiple of %d", (long long)numel, lanes);
     const int64_t nvec = numel / lanes;
     if (nvec == 0) return KXC_B200_OK;
-    KXC_DISPATCH_ACT(dt, (eltwise_nhwc_kernel<T><<<grid_for(nvec, 16), kThreads, 0, s>>>(
+    KXC_DISPATCH_STORED(dt, full, (eltwise_nhwc_kernel<T><<<grid_for(nvec, 16), kThreads, 0, s>>>(
                              static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), nvec, relu)));
     return check_launch("eltwise_nhwc");
 }

@@ -1175,16 +1175,16 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
             case SKind::MaxPool:
                 KXC_TRY(maxpool_nhwc(pl->plain(st.in0), pl->plain(st.out), dt, st.N, st.H, st.W, st.C, st.OH, st.OW,
                                      st.pool.pool_size[0], st.pool.pool_size[1], st.pool.strides[0], st.pool.strides[1],
-                                     st.pool.padding[0], st.pool.padding[1], s));
+                                     st.pool.padding[0], st.pool.padding[1], s, pl->x3));
                 KXC_TRY(split_x3(pl, st.out, s));
                 break;
             case SKind::Gap:
-                KXC_TRY(gap_nhwc(pl->plain(st.in0), pl->plain(st.out), dt, st.N, st.H * st.W, st.C, s));
+                KXC_TRY(gap_nhwc(pl->plain(st.in0), pl->plain(st.out), dt, st.N, st.H * st.W, st.C, s, pl->x3));
                 KXC_TRY(split_x3(pl, st.out, s));
                 break;
             case SKind::Eltwise:
                 KXC_TRY(eltwise_nhwc(pl->plain(st.in0), st.in1 >= 0 ? pl->plain(st.in1) : nullptr, pl->plain(st.out), dt,
-                                     st.numel, st.relu ? 1 : 0, s));
+                                     st.numel, st.relu ? 1 : 0, s, pl->x3));
                 KXC_TRY(split_x3(pl, st.out, s));
                 break;
             case SKind::ToNCHW:

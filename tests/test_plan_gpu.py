@@ -126,6 +126,31 @@ def test_small_cnn_plan(kxc, rng, precision):
     assert np.array_equal(got, again)
 
 
+def test_tf32x3_plan_splits_unfused_results(kxc, rng):
+    """Three-pass plans store a value in the forms its consumers read: here the first convolution's result and the unfused add's
+    are read in full (add, pooling, residual) as well as in two parts (convolutions, dense), and the second convolution's has only
+    unfused readers. Bound: 1e-4 (the operators' own) for each of the four convolutions; one pooled or added value rounded to tf32 on
+    the way exceeds it."""
+    R = kxc.relay
+    N, C, H, O = 3, 16, 13, 32
+    w = lambda *s: R.Constant(cuda_const(rng.normal(0, np.sqrt(1.0 / np.prod(s[1:])), s).astype(f32)))  # noqa: E731
+    b = lambda n: R.Constant(cuda_const(rng.normal(0, 0.05, (n,)).astype(f32)))  # noqa: E731
+    conv = lambda e, ci, co, k: R.Call("nn_conv2d", [e, w(co, ci, k, k), b(co)], R.Conv2DAttrs((1, 1), (k // 2,) * 4, (1, 1), 1))  # noqa: E731
+    xv = R.Var("input", (N, C, H, H))
+    y = R.Call("nn_relu", [conv(xv, C, O, 3)])
+    c = conv(y, O, O, 3)
+    s = R.Call("add", [R.Call("nn_relu", [c]), R.Call("add", [c, y])])       # no convolution's epilogue takes these
+    t = R.Call("nn_relu", [R.Call("add", [conv(s, O, O, 1), s])])            # residual in full, operand in parts
+    p = R.Call("nn_max_pool2d", [t], R.MaxPool2DAttrs((2, 2), (1, 1, 1, 1), (1, 1), (3, 3), "NCHW", False))
+    g = R.Call("nn_flatten", [R.Call("nn_global_avg_pool2d", [R.Call("add", [conv(p, O, O, 3), p])])])
+    func = R.Function([xv], R.Call("nn_gemm", [g, w(24, O), b(24)], R.GemmAttrs(1.0, 1.0, 0, 1)))
+    x = rng.normal(0, 1, (N, C, H, H)).astype(f32)
+    got, plan = run_plan(kxc, func, x, "tf32x3")
+    assert sum("eltwise" in l[0] for l in plan.launch_info()) >= 2
+    max_abs, max_rel = ref_metric(got, ograph.run(host_func(func), [x]))
+    assert max_rel <= 4e-4, (max_abs, max_rel)
+
+
 def test_single_conv_plan_matches_per_op(kxc, rng):
     R = kxc.relay
     x = rng.uniform(-1, 1, (2, 64, 14, 14)).astype(f32)
