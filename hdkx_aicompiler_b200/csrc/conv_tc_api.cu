@@ -197,16 +197,23 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     const size_t act_bytes = align_up((size_t)d.N * conv_h * conv_w * cpad, 1024);
     const size_t w_bytes = align_up((size_t)d.O * d.KH * d.KW * cpad, 1024);
     // Result layout. A thread of the epilogue owns one pixel, so its NCHW stores are single bytes whose neighbours in
-    // memory belong to the next pixel of the same tile row: runs of BW bytes. From 1 MiB of results on (and wherever BW <= 2)
-    // the kernel stores NHWC into the workspace instead, pixels padded to 16 channels, and a byte transpose writes the
-    // reference layout (128 -> 128 channels, 28x28, 256 images: 65 us of convolution with byte stores against 52 + 12). A
-    // smaller result is not worth the second launch, and planes that are no multiple of four bytes have only the byte-wise
-    // transpose (33 -> 27 channels, 101x103, 132 images: 370 us with byte stores, 392 by way of NHWC).
+    // memory belong to the next pixel of the same tile row: runs of BW bytes. The other way is to store NHWC into the
+    // workspace, pixels padded to 16 channels, and to let a byte transpose write the reference layout, which costs a launch
+    // (1 to 3 us) and the result's bytes twice more. Measured, us with byte stores / by way of NHWC:
+    //   results of 1 MiB and more      96 -> 178 1x1 at 28x28, 229 images: 66 / 51; 128 -> 128 3x3 at 28x28, 256 images: 67 / 67;
+    //                                  smaller ones between 0.9 and 1.3 times; BW <= 2: 128 -> 401 1x1 at 13x13, 66 images: 34 / 23
+    //   ... planes no multiple of four (byte-wise transpose), BW > 2: 33 -> 27 3x3 at 101x103, 132 images: 333 / 386
+    //   below 1 MiB, boxes of one pixel per image: 32 -> 30 3x3 at 7x7, 256 images: 15.1 / 13.0
+    //   ... other boxes, also of BW <= 2: 128 -> 24 3x3 at 14x14, 148 images: 16.0 / 17.6; whole 16s of channels with BW <= 2:
+    //                                  from 13.2 / 15.1 (64 -> 48 at 14x14, 64 images) to 18.5 / 17.2 (256 -> 64 there)
     int bw = 0, bh = 0, bni = 0;
     tc_pick_tile(d.N, d.OH, d.OW, &bw, &bh, &bni);
     const int out_pitch = (d.O + 15) / 16 * 16;
-    bool two_step = bw <= 2 || rowstack_ok ||
-                    ((long long)d.N * d.O * d.OH * d.OW >= (1 << 20) && ((long long)d.OH * d.OW & 3) == 0);  // (the row-stacked kernel writes NHWC only)
+    const long long plane = (long long)d.OH * d.OW;
+    const bool narrow = bw <= 2;
+    bool two_step = rowstack_ok ||  // (the row-stacked kernel writes NHWC only)
+                    (narrow && ((d.O & 15) == 0 || bw * bh == 1)) ||
+                    (d.N * d.O * plane >= (1 << 20) && ((plane & 3) == 0 || narrow));
     const size_t out_bytes = two_step ? align_up((size_t)d.N * d.OH * d.OW * out_pitch, 1024) : 0;
     StreamScratch ws(s);
     int32_t rc = ws.alloc(act_bytes + w_bytes + out_bytes);

@@ -98,6 +98,18 @@ def test_refused_workspace_leaves_no_error_behind(fake):
     assert rc == 0, message
 
 
+# How a result in the reference's layout leaves (True: by way of NHWC), see conv2d_s8_dispatch: tile boxes two columns wide or less with
+# channels that are no multiple of 16, odd and even planes, below and above 1 MiB, one pixel per image; wider boxes
+@pytest.mark.parametrize("case,by_way_of_nhwc", [
+    ((64, 128, 7, 7, 100, 3), False), ((148, 128, 14, 14, 24, 3), False), ((16, 64, 14, 14, 50, 3), False), ((66, 128, 13, 13, 401, 1), True),
+    ((64, 512, 7, 7, 500, 1), True), ((256, 32, 7, 7, 30, 3), True), ((128, 64, 5, 5, 33, 3), True), ((64, 128, 7, 7, 96, 3), True),
+    ((229, 96, 28, 28, 178, 1), True), ((132, 33, 101, 103, 27, 3), False), ((2, 48, 12, 12, 40, 3), False)])
+def test_s8_result_route(fake, case, by_way_of_nhwc):
+    rc, message = conv_s8(fake, *case)
+    assert rc == 0, message
+    assert ("conv_igemm" not in launches(fake)[-1]) == by_way_of_nhwc
+
+
 # planes of more than 64 * 65535 pixels: the byte transposes' row tiles no longer fit the grid's second dimension; a plane that is
 # a multiple of four bytes takes the register transpose, an odd one (64 -> 64 channels, 3x3: always by way of NHWC) the byte-wise one
 @pytest.mark.parametrize("case", [(1, 16, 2048, 2048, 16, 1), (2, 8, 3000, 2000, 24, 3), (1, 64, 2049, 2049, 64, 3)])

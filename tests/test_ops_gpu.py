@@ -303,6 +303,15 @@ def test_conv2d_s8_layouts(ops, rng, N, C, H, W, O):
     assert torch.equal(got, ops.nn_conv2d_s8(x, w, b, m, sh, (1, 1), (1, 1), simt=True))
 
 
+# Tile boxes of at most two columns, channels that are no multiple of 16: odd and even planes, below and above 1 MiB of results
+@pytest.mark.parametrize("N,C,H,W,O", [(64, 64, 7, 7, 100), (16, 64, 14, 14, 50), (66, 64, 13, 13, 101), (129, 33, 7, 7, 30), (33, 32, 9, 9, 246)])
+def test_conv2d_s8_narrow_boxes(ops, rng, N, C, H, W, O):
+    x, w, b, m, sh = (dev(a) for a in s8_inputs(rng, N, C, H, W, O, 3, 3))
+    got = ops.nn_conv2d_s8(x, w, b, m, sh, (1, 1), (1, 1))
+    assert ops.device_status() == 0
+    assert torch.equal(got, ops.nn_conv2d_s8(x, w, b, m, sh, (1, 1), (1, 1), simt=True))
+
+
 # One plane of 4,194,308 pixels: its 64-row tiles are more than the second grid dimension holds
 def test_conv2d_s8_plane_beyond_the_second_grid_dimension(ops, rng):
     x, w, b, m, sh = (dev(a) for a in s8_inputs(rng, 1, 3, 1048577, 4, 5, 1, 1))
