@@ -268,6 +268,23 @@ def test_conv2d_split_reduction(ops, rng, case, precision, rounder):
     assert min(max_abs, max_rel) <= bound, f"split conv {precision} {case}: {max_abs:.3e} {max_rel:.3e}"
 
 
+# Tile boxes of results in the reference's layout, chosen by the runs of their stores: whole rows, rows wider than a tile, one
+# column, one pixel per image, several images per box; a residual read chunk by chunk ahead of the accumulator (32, 64 and more
+# channels, a last chunk that is partly there). Bound: that of test_conv2d_tensor_core.
+@pytest.mark.parametrize("precision,rounder", [("tf32", port.round_tf32), ("bf16", port.round_bf16)])
+@pytest.mark.parametrize("case", [(1, 16, 3, 200, 40, 3), (3, 16, 150, 1, 33, 3), (2, 32, 5, 131, 70, 1), (9, 16, 3, 3, 65, 3), (130, 32, 1, 1, 96, 1),
+                                  (1, 32, 45, 51, 130, 1), (5, 8, 28, 30, 31, 3)])
+def test_conv2d_nchw_boxes(ops, rng, case, precision, rounder):
+    N, C, H, W, O, k = case
+    x, w, b = conv_inputs(rng, N, C, H, W, O, k, k)
+    res = rng.uniform(-1, 1, (N, O, H, W)).astype(f32)
+    got = host(ops.nn_conv2d(dev(x), dev(w), dev(b), (1, 1), (k // 2, k // 2), residual=dev(res), relu=True, precision=precision))
+    assert ops.device_status() == 0
+    max_abs, max_rel = ref_metric(got, conv_expect(x, w, b, res, True, 1, k // 2, 1, rounder))
+    bound = 2e-5 * max(1.0, np.sqrt(C * k * k) / 8)
+    assert min(max_abs, max_rel) <= bound, f"{precision} {case}: {max_abs:.3e} {max_rel:.3e}"
+
+
 # ---------------------------------------------------------------- int8 conv + requantize
 def s8_inputs(rng, N, C, H, W, O, KH, KW):
     x = np.clip(np.round(rng.normal(0, 32, (N, C, H, W))), -128, 127).astype(np.int8)
