@@ -792,6 +792,13 @@ int32_t weight_map(CUtensorMap* m, const TcConfig* cfg, const TcParams* p, const
     return tc_make_tmap(m, cfg->dtype, 2, const_cast<void*>(w), dims, strides, box, 128);
 }
 
+// Whether `tiles` clusters of s CTAs run at once. Clusters of an odd number of CTAs leave halves of SM pairs behind, and behind a
+// kernel that is still draining the last two did not start with the others: 44 of 45 clusters of three took 1 to 17 us longer
+// than the same parts in fewer clusters do, 25 and 26 of 26 clusters of five 2 and 5 us; 32 of 33 clusters of four 0.3.
+bool split_fits(long long tiles, int s) {
+    return tiles * s <= kNumSMs && tiles <= tc_split_capacity(s) - ((s & 1) != 0 ? 2 : 0);
+}
+
 // Whether a set-up launch (tile width, store form and so on already chosen for the persistent kernel) is better off with its
 // reduction split over a cluster, and the set-up of that form: the cheaper of the two in modelled cycles, the split one 5 % ahead.
 // The figures are fits over 320 launches timed in every form that fits the chip (7 layers in a row, NHWC, and one layer
@@ -804,8 +811,8 @@ int32_t weight_map(CUtensorMap* m, const TcConfig* cfg, const TcParams* p, const
 // Over the same launches what this chooses is 0.3 % (NHWC) and 1.4 % (NCHW) behind the fastest form on average, and one launch
 // is behind the unsplit one by more than 1 %. (One figure for every width, 3000, made wide splits of short reductions slower than no split: bf16
 // 1024 -> 1024 1x1 at 7x7 and 24 images 14.7 us per layer in two parts of 256 channels, 11.3 unsplit; 256 -> 256 3x3 at
-// 14x14 and 32 images 19.4 and 17.8.) A launch is kept to the clusters that the chip holds at once (a dense layer of 16
-// tiles in clusters of eight that did not all fit: 8.8 -> 12 us).
+// 14x14 and 32 images 19.4 and 17.8.) A launch is kept to the clusters that the chip holds at once (split_fits; a dense
+// layer of 16 tiles in clusters of eight that did not all fit: 8.8 -> 12 us).
 int32_t choose_split(TcParams* p, TcConfig* cfg, const void* w, const void* w_lo, int k_elems) {
     p->split = 0;
     if (cfg->dtype == kTcS8 || cfg->kb_bytes != 128) return KXC_B200_OK;
@@ -825,8 +832,8 @@ int32_t choose_split(TcParams* p, TcConfig* cfg, const void* w, const void* w_lo
         const long long tiles = m_tiles * ((p->Cout + bn - 1) / bn);
         const long long split_block = cfg->x3 ? (bn == 64 ? 830 : 930) : (bn == 64 ? 550 : (bn == 128 ? 590 : 650));
         const long long split_tail = bn == 64 ? 3000 : (bn == 128 ? 7000 : 13000);
-        for (int s = 2; s <= kMaxSplit && tiles * s <= kNumSMs; ++s) {
-            if (tiles > tc_split_capacity(s)) continue;
+        for (int s = 2; s <= kMaxSplit; ++s) {
+            if (!split_fits(tiles, s)) continue;
             const long long span = (long long)((kb + s - 1) / s) * split_block + split_tail;
             if (span < best) {
                 best = span;
@@ -866,8 +873,8 @@ int32_t tc_setup_dual(TcParams* p, TcConfig* cfg, const void* act_nhwc, const vo
     const int kb = KH * KW * p->cblocks;
     const long long tiles64 = m_tiles * ((Cout + 63) / 64);
     long long best = (waves(m_tiles * ((Cout + 127) / 128)) * (kb + p->cblocks) * 590 + 4000) * 95 / 100;
-    for (int s = 2; kb >= 12 && s <= kMaxSplit && tiles64 * s <= kNumSMs; ++s) {
-        if (tiles64 > tc_split_capacity(s)) continue;
+    for (int s = 2; kb >= 12 && s <= kMaxSplit; ++s) {
+        if (!split_fits(tiles64, s)) continue;
         const long long span = (long long)(kb - (s - 1) * kb / s + p->cblocks) * 550 + 4400;
         if (span < best) {
             best = span;

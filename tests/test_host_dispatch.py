@@ -190,3 +190,10 @@ def test_no_split_launch_of_a_network_needs_more_clusters_than_fit(compile_graph
                 assert ctas <= 148 and ctas // cluster <= HELD[cluster], f"{n} images: {ctas // cluster} clusters of {cluster}"
         two_outputs += sum("second output" in label and "split" in label for label, _, _ in graph.launch_info())
     assert (two_outputs > 0) == (precision == "bf16")
+
+
+def test_clusters_of_an_odd_size_keep_two_in_reserve(fake):
+    """22 pixel tiles by two of 256 channels in three parts are 44 of the 45 clusters that fit: measured slower than no split."""
+    rc, message = conv(fake, _lib.PREC_BF16, 2, 219, 33, 36, 463, 3)
+    assert rc == 0, message
+    assert "conv_igemm" in launches(fake)[-1], launches(fake)[-1]
