@@ -202,8 +202,7 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     // (1 to 3 us) and the result's bytes twice more. Measured, us with byte stores / by way of NHWC:
     //   results of 1 MiB and more      96 -> 178 1x1 at 28x28, 229 images: 66 / 51; 128 -> 128 3x3 at 28x28, 256 images: 67 / 67;
     //                                  smaller ones between 0.9 and 1.3 times; BW <= 2: 128 -> 401 1x1 at 13x13, 66 images: 34 / 23
-    //   ... planes no multiple of four (byte-wise transpose), BW > 2 or few channels: 33 -> 27 3x3 at 101x103, 132 images:
-    //                                  333 / 386; BW 1, 96 -> 26 3x3 at 27x27, 160 images: 44.6 / 47.3
+    //   ... planes no multiple of four (byte-wise transpose), BW > 2: 33 -> 27 3x3 at 101x103, 132 images: 333 / 386
     //   below 1 MiB, boxes of one pixel per image: 32 -> 30 3x3 at 7x7, 256 images: 15.1 / 13.0
     //   ... other boxes, also of BW <= 2: 128 -> 24 3x3 at 14x14, 148 images: 16.0 / 17.6; whole 16s of channels with BW <= 2:
     //                                  from 13.2 / 15.1 (64 -> 48 at 14x14, 64 images) to 18.5 / 17.2 (256 -> 64 there)
@@ -214,7 +213,7 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     const bool narrow = bw <= 2;
     bool two_step = rowstack_ok ||  // (the row-stacked kernel writes NHWC only)
                     (narrow && ((d.O & 15) == 0 || bw * bh == 1)) ||
-                    (d.N * d.O * plane >= (1 << 20) && ((plane & 3) == 0 || (narrow && d.O >= 64)));
+                    (d.N * d.O * plane >= (1 << 20) && ((plane & 3) == 0 || narrow));
     const size_t out_bytes = two_step ? align_up((size_t)d.N * d.OH * d.OW * out_pitch, 1024) : 0;
     StreamScratch ws(s);
     int32_t rc = ws.alloc(act_bytes + w_bytes + out_bytes);
