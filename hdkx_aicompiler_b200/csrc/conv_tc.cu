@@ -792,11 +792,14 @@ int32_t weight_map(CUtensorMap* m, const TcConfig* cfg, const TcParams* p, const
     return tc_make_tmap(m, cfg->dtype, 2, const_cast<void*>(w), dims, strides, box, 128);
 }
 
-// Whether `tiles` clusters of s CTAs run at once. Clusters of an odd number of CTAs leave halves of SM pairs behind, and behind a
-// kernel that is still draining the last two did not start with the others: 44 of 45 clusters of three took 1 to 17 us longer
-// than the same parts in fewer clusters do, 25 and 26 of 26 clusters of five 2 and 5 us; 32 of 33 clusters of four 0.3.
-bool split_fits(long long tiles, int s) {
-    return tiles * s <= kNumSMs && tiles <= tc_split_capacity(s) - ((s & 1) != 0 ? 2 : 0);
+// Whether `tiles` clusters of s CTAs fit on the chip at once, and the cycles that the last ones start later. Clusters of an odd
+// number of CTAs leave halves of SM pairs behind: behind a kernel that is still draining, 44 of 45 clusters of three took 1 to
+// 17 us longer than fewer clusters do, 25 and 26 of 26 clusters of five 2 and 5 us (32 of 33 clusters of four 0.3); behind one
+// that leaves the shared memory free, nothing.
+bool split_fits(long long tiles, int s, long long* late) {
+    const int held = tc_split_capacity(s);
+    *late = (s & 1) != 0 && tiles > held - 2 ? 3800 : 0;
+    return tiles * s <= kNumSMs && tiles <= held;
 }
 
 // Whether a set-up launch (tile width, store form and so on already chosen for the persistent kernel) is better off with its
@@ -833,8 +836,9 @@ int32_t choose_split(TcParams* p, TcConfig* cfg, const void* w, const void* w_lo
         const long long split_block = cfg->x3 ? (bn == 64 ? 830 : 930) : (bn == 64 ? 550 : (bn == 128 ? 590 : 650));
         const long long split_tail = bn == 64 ? 3000 : (bn == 128 ? 7000 : 13000);
         for (int s = 2; s <= kMaxSplit; ++s) {
-            if (!split_fits(tiles, s)) continue;
-            const long long span = (long long)((kb + s - 1) / s) * split_block + split_tail;
+            long long late = 0;
+            if (!split_fits(tiles, s, &late)) continue;
+            const long long span = (long long)((kb + s - 1) / s) * split_block + split_tail + late;
             if (span < best) {
                 best = span;
                 split = s;
@@ -874,8 +878,9 @@ int32_t tc_setup_dual(TcParams* p, TcConfig* cfg, const void* act_nhwc, const vo
     const long long tiles64 = m_tiles * ((Cout + 63) / 64);
     long long best = (waves(m_tiles * ((Cout + 127) / 128)) * (kb + p->cblocks) * 590 + 4000) * 95 / 100;
     for (int s = 2; kb >= 12 && s <= kMaxSplit; ++s) {
-        if (!split_fits(tiles64, s)) continue;
-        const long long span = (long long)(kb - (s - 1) * kb / s + p->cblocks) * 550 + 4400;
+        long long late = 0;
+        if (!split_fits(tiles64, s, &late)) continue;
+        const long long span = (long long)(kb - (s - 1) * kb / s + p->cblocks) * 550 + 4400 + late;
         if (span < best) {
             best = span;
             p->split = s;
