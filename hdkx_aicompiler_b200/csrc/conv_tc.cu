@@ -755,9 +755,12 @@ namespace {
 // Tile box of a launch that writes the reference's layout: a warp's 32 pixels leave as one 4-byte store per channel, in runs of
 // BW consecutive addresses (BW * BH when the box spans the rows), and every run costs its own 32-byte sectors. The box with
 // the fewest tiles may have runs of one to three pixels, so waves and sectors are weighed together: a tile's main loop is its K
-// blocks at the rate they arrive, its epilogue ~4 cycles per sector (stores and residual loads), which overlaps the next tile's
-// main loop. (9 x 72 x 45 x 51 -> 120 channels, tf32, with a residual: runs of 3 pixels, 41 us; full rows and the residual read
-// ahead of the accumulator, with two tiles per work item below, 27 us.)
+// blocks at the rate they arrive, its epilogue 80 cycles per channel or, if that is more, 12 per sector of a warp's store, which
+// overlaps the next tile's main loop. Runs of 8 to 32 pixels took the same time per tile (62 to 66 cycles per channel at 256
+// channels without a residual; 88, 95 and 107 at 32, 16 and 8 with one), runs of 4 twice that. Among 60 launches timed with up to 30
+// boxes each, a cost per sector alone traded whole waves for longer runs: 31 -> 331 1x1 stride 2, 56x54, 61 images, 1x14x9 boxes
+// 52 us and 1x4x27 60; 20 -> 463 on 101x103, 53 images, 158 and 172. In launches of one wave the box hardly matters (64 -> 64
+// 3x3 at 56x56, one image: 11.0 to 11.3 us from 128 down to 28 pixels a box).
 void pick_tile_nchw(int N, int OH, int OW, int Cout, int num_kb, int kb_bytes, int* BW, int* BH, int* BNI) {
     const int bn_out = Cout <= 64 ? 64 : (Cout <= 128 ? 128 : 256);
     const int tiles_c = (Cout + bn_out - 1) / bn_out;
@@ -772,10 +775,11 @@ void pick_tile_nchw(int N, int OH, int OW, int Cout, int num_kb, int kb_bytes, i
             const long long waves = (tiles * tiles_c + kNumSMs - 1) / kNumSMs;
             int run = bw == OW ? bw * bh : bw;
             if (run > 32) run = 32;
-            const double epilogue = 4.0 * 1.5 * bn_out * 128.0 * (run / 8.0 + 0.9) / run;
+            const double sectors = 32.0 * (run / 8.0 + 0.9) / run;
+            const double epilogue = bn_out * (12.0 * sectors > 80.0 ? 12.0 * sectors : 80.0);
             const double slower = main_loop > epilogue ? main_loop : epilogue;
-            // (tiles as the tie-breaker: less work on the same number of waves)
-            const double cost = main_loop + (double)(waves - 1) * slower + epilogue + 1e-3 * (double)tiles;
+            // (tie-breakers: longer runs, then fewer tiles on the same number of waves)
+            const double cost = main_loop + (double)(waves - 1) * slower + epilogue + 10.0 * sectors + 1e-3 * (double)tiles;
             if (best < 0.0 || cost < best) {
                 best = cost;
                 *BW = bw; *BH = bh; *BNI = bn;

@@ -5,12 +5,14 @@ import contextlib
 import ctypes
 import glob
 import os
+import re
 import subprocess
 
+import numpy as np
 import pytest
 import torch
 
-from hdkx_aicompiler_b200 import _lib, plan, resnet18
+from hdkx_aicompiler_b200 import _lib, plan, relay, resnet18
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "hdkx_aicompiler_b200", "csrc")
@@ -201,3 +203,16 @@ def test_nearly_all_clusters_of_an_odd_size_cost_more(fake):
     rc, message = conv(fake, _lib.PREC_TF32X3, 11, 317, 23, 20, 42, 3)
     assert rc == 0, message
     assert "conv_splitk" in launches(fake)[-1] and launches(fake)[-1].endswith("cluster 3"), launches(fake)[-1]
+
+
+# Measured: 52 and 158 us with boxes of few waves (1x14x9, 7x1x18), 60 and 172 with whole rows
+@pytest.mark.parametrize("n,c,h,w,o,waves", [(61, 31, 56, 54, 331, 5), (53, 20, 101, 103, 463, 17)])
+def test_nchw_boxes_do_not_trade_waves_for_longer_runs(compile_graph, n, c, h, w, o, waves):
+    x = relay.Var("input", (n, c, h, w))
+    conv = relay.Call("nn_conv2d", [x, relay.Constant(DeviceTensor(np.empty((o, c, 1, 1)))), relay.Constant(DeviceTensor(np.empty(o)))],
+                      relay.Conv2DAttrs((2, 2), (0, 0, 0, 0), (1, 1), 1))
+    graph, _ = compile_graph(relay.Function([x], relay.Call("nn_relu", [conv])), "bf16")
+    label = graph.launch_info()[-1][0]
+    bni, bh, bw = (int(v) for v in re.search(r"tile (\d+)x(\d+)x(\d+)", label).groups())
+    tiles = -(-n // bni) * -(-((h + 1) // 2) // bh) * -(-((w + 1) // 2) // bw) * -(-o // 256)
+    assert -(-tiles // 148) <= waves, label
