@@ -952,6 +952,12 @@ int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_m
     {
         const long long mt = (long long)p->tiles_w * p->tiles_h * p->tiles_n;
         while (bn > 64 && mt * ((Cout + bn - 1) / bn) < 32) bn /= 2;
+        // Into the reference's layout a narrower tile is the better one as long as all are resident at once: their K blocks
+        // arrive at nearly the same rate, and the epilogue that follows the last one is half as long. (252 -> 160 1x1 at 9x9,
+        // tf32, 42 images: 10.1 us 64 wide, 14.8 256 wide; 84 -> 433 1x1 at 7x10, bf16, 12 images: 7.2 and 8.6 128 wide.)
+        if (out_mode == kOutNCHW_F32) {
+            while (bn > 64 && mt * ((Cout + bn / 2 - 1) / (bn / 2)) <= kNumSMs) bn /= 2;
+        }
     }
     // CTA pairs (tcgen05 cta_group::2): each CTA fetches half of the B tile, which relieves the L2 -> shared-memory
     // fill rate that bounds the wide tiles. KXC_B200_CTA_PAIR=0 switches them off (for measurements).
