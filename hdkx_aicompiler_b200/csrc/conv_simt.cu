@@ -71,8 +71,8 @@ __global__ void __launch_bounds__(kThreads) conv2d_direct_kernel(const TIn* __re
 // ptxas fuses mul.rn.f32x2 + add.rn.f32x2 into one fused multiply-add, which rounds once and changes the bits. The product
 // is therefore formed as fma(x, w, -0) with a -0 that is a kernel argument (fma(x, w, -0) is the rounded product for every
 // x and w, the signs of zeros included), which nothing can fold.
-// Measured, 128 -> 128 channels 3x3 at 28x28 and 32 images: 646 us with scalar arithmetic, 279 us = 26.6 TFLOP/s now (0.73 of
-// the packed bound; 2.65 blocks for each SM cost 12 % of it); ResNet-18 at 32 images 11.3 -> 4.6 ms. Weights doubled in
+// Measured, 128 -> 128 channels 3x3 at 28x28 and 32 images: 646 us with scalar arithmetic, 275 us = 26.9 TFLOP/s now (0.74 of
+// the packed bound; 2.65 blocks for each SM cost 12 % of it); ResNet-18 at 32 images 11.3 -> 4.5 ms. Weights doubled in
 // shared memory to spare the register moves, unrolling two stages and rolling the k loop up were slower.
 //
 // Half of the warps compute, the other half feed them: the im2col values of KC consecutive k = (rc, rh, rw) by 4-byte
@@ -314,27 +314,58 @@ __global__ void __launch_bounds__(2 * kOG * kPG, kMinBlocks)
         buf = buf + 1 == kExactBufs ? 0 : buf + 1;
     }
 
-    // four consecutive pixels of one image are one 16-byte access where planes and pointers allow it
+    // Four consecutive pixels of one image are one 16-byte access where planes and pointers allow it. A pixel's place is found once
+    // for all channels, and the residual of four channels is fetched before the first of their results is stored: with a 64-bit
+    // division and one load in flight per result, short reductions were nothing but epilogue (19 -> 476 channels 1x1 over 81x81,
+    // 18 images, with a residual: 625 us, now 301; over 80x82 418 and 277). All channels at once were slower in long ones
+    // (128 -> 128 3x3 at 28x28, 32 images: 280 against 275 us, for registers), lanes that trade pixels so that a warp stores whole
+    // rows in all of them (715 us).
     const bool vec = (plane_out & 3) == 0 && epi.aligned16();
+    const int64_t image_step = (int64_t)d.O * plane_out;
 #pragma unroll
     for (int g = 0; g < (kTP + 2) / 4; ++g) {
         const bool quad = 4 * g + 4 <= kTP;
-        const int64_t p = p0 + g * kPG * 4 + pg * (quad ? 4 : 2);
-        if (p >= P) continue;
+        const int width = quad ? 4 : 2;
+        const bool whole = quad && vec;
+        int64_t base[4] = {-1, -1, -1, -1};  // where the thread's pixels lie in channel 0; -1: nowhere
 #pragma unroll
-        for (int j = 0; j < kTO; ++j) {
-            const int o = o0 + og * kTO + j;
-            if (o >= d.O) continue;
-            float v[4] = {0.f, 0.f, 0.f, 0.f};
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[j][2 * g]));
-            if (quad) asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2]), "=f"(v[3]) : "l"(acc[j][quad ? 2 * g + 1 : 0]));
-            if (quad && vec) {
-                const int64_t n = p / plane_out;
-                epi.four(v, (n * d.O + o) * plane_out + (p - n * plane_out), o);
-            } else {
-                for (int e = 0; e < (quad ? 4 : 2); ++e) {
-                    const int64_t n = (p + e) / plane_out;
-                    if (p + e < P) epi(v[e], (n * d.O + o) * plane_out + (p + e - n * plane_out), o);
+        for (int e = 0; e < width; ++e) {
+            const uint32_t p = (uint32_t)p0 + g * kPG * 4 + pg * width + e;  // (P is below 2^31)
+            const uint32_t n = p / (uint32_t)plane_out;
+            if (p < (uint32_t)P) base[e] = n * image_step + (p - n * plane_out);
+        }
+        if (base[0] < 0) continue;
+        constexpr int kBatch = kTO < 4 ? kTO : 4;  // channels whose residual is in flight together
+#pragma unroll
+        for (int j0 = 0; j0 < kTO; j0 += kBatch) {
+            float r[kBatch][4] = {};
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int o = o0 + og * kTO + j0 + i;
+                if (o >= d.O) continue;
+                if (whole) {
+                    epi.fetch4(r[i], base[0] + (int64_t)o * plane_out);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < width; ++e)
+                        if (base[e] >= 0) r[i][e] = epi.fetch(base[e] + (int64_t)o * plane_out);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int o = o0 + og * kTO + j0 + i;
+                if (o >= d.O) continue;
+                float v[4] = {0.f, 0.f, 0.f, 0.f};
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[j0 + i][2 * g]));
+                if (quad) asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2]), "=f"(v[3]) : "l"(acc[j0 + i][quad ? 2 * g + 1 : 0]));
+#pragma unroll
+                for (int e = 0; e < width; ++e) v[e] = epi.finish(v[e], r[i][e], o);
+                if (whole) {
+                    *reinterpret_cast<float4*>(epi.out + base[0] + (int64_t)o * plane_out) = make_float4(v[0], v[1], v[2], v[3]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < width; ++e)
+                        if (base[e] >= 0) epi.out[base[e] + (int64_t)o * plane_out] = v[e];
                 }
             }
         }
@@ -346,29 +377,23 @@ struct EpilogueF32 {
     const float* residual;
     float* out;
     int relu;
-    __device__ __forceinline__ void operator()(float acc, int64_t lin, int o) const {
-        float v = acc;
-        if (bias) v = __fadd_rn(v, __ldg(bias + o));
-        if (residual) v = __fadd_rn(v, __ldg(residual + lin));
-        if (relu) v = v > 0.0f ? v : 0.0f;
-        out[lin] = v;
+    __device__ __forceinline__ float fetch(int64_t lin) const { return residual ? __ldg(residual + lin) : 0.0f; }
+    __device__ __forceinline__ void fetch4(float (&r)[4], int64_t lin) const {  // lin: a multiple of four
+        if (residual) {
+            const float4 q = __ldg(reinterpret_cast<const float4*>(residual + lin));
+            r[0] = q.x; r[1] = q.y; r[2] = q.z; r[3] = q.w;
+        }
     }
+    // the result of channel o: r as fetched
+    __device__ __forceinline__ float finish(float v, float r, int o) const {
+        if (bias) v = __fadd_rn(v, __ldg(bias + o));
+        if (residual) v = __fadd_rn(v, r);
+        if (relu) v = v > 0.0f ? v : 0.0f;
+        return v;
+    }
+    __device__ __forceinline__ void operator()(float acc, int64_t lin, int o) const { out[lin] = finish(acc, fetch(lin), o); }
     __device__ __forceinline__ bool aligned16() const {
         return ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(residual)) & 15u) == 0;
-    }
-    // four consecutive outputs of channel o, the first at a multiple of four
-    __device__ __forceinline__ void four(const float* acc, int64_t lin, int o) const {
-        float4 v = make_float4(acc[0], acc[1], acc[2], acc[3]);
-        if (bias) {
-            const float b = __ldg(bias + o);
-            v = make_float4(__fadd_rn(v.x, b), __fadd_rn(v.y, b), __fadd_rn(v.z, b), __fadd_rn(v.w, b));
-        }
-        if (residual) {
-            const float4 r = __ldg(reinterpret_cast<const float4*>(residual + lin));
-            v = make_float4(__fadd_rn(v.x, r.x), __fadd_rn(v.y, r.y), __fadd_rn(v.z, r.z), __fadd_rn(v.w, r.w));
-        }
-        if (relu) v = make_float4(v.x > 0.0f ? v.x : 0.0f, v.y > 0.0f ? v.y : 0.0f, v.z > 0.0f ? v.z : 0.0f, v.w > 0.0f ? v.w : 0.0f);
-        *reinterpret_cast<float4*>(out + lin) = v;
     }
 };
 
