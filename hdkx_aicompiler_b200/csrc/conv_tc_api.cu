@@ -213,7 +213,7 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     const bool narrow = bw <= 2;
     bool two_step = rowstack_ok ||  // (the row-stacked kernel writes NHWC only)
                     (narrow && ((d.O & 15) == 0 || bw * bh == 1)) ||
-                    (d.N * d.O * plane >= (1 << 20) && ((plane & 3) == 0 || narrow));
+                    (plane * d.N * d.O >= (1 << 20) && ((plane & 3) == 0 || narrow));
     const size_t out_bytes = two_step ? align_up((size_t)d.N * d.OH * d.OW * out_pitch, 1024) : 0;
     StreamScratch ws(s);
     int32_t rc = ws.alloc(act_bytes + w_bytes + out_bytes);
