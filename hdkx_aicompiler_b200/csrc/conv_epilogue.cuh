@@ -8,6 +8,7 @@
 #include <climits>
 
 #include "conv_tc.cuh"
+#include "tf32.cuh"
 
 namespace kxc_b200 {
 
@@ -125,18 +126,6 @@ __device__ __forceinline__ void store_chunk_s8(const TcParams& p, const uint32_t
     }
 }
 
-// Epilogue for one 32-column chunk held by one thread (= one output pixel, 32 consecutive channels).
-// kSplit (three-pass tf32): the result may also leave as its tf32 high and low parts (TcParams::out_hi).
-__device__ __forceinline__ float tf32_rne(float x) {
-    uint32_t u = __float_as_uint(x);
-    if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0xfffu + ((u >> 13) & 1u)) & 0xffffe000u;
-    return __uint_as_float(u);
-}
-// (a non-finite value lives in the high part only: inf - inf would be NaN)
-__device__ __forceinline__ float tf32_low_part(float x, float hi) {
-    return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u ? 0.0f : tf32_rne(__fsub_rn(x, hi));
-}
-
 // kOutNCHW_F32: the chunk's residual values, fetched before the accumulator is waited for (one 4-byte load per channel: read
 // when they are needed, each waits out its own trip to memory).
 __device__ __forceinline__ void residual_fetch_nchw(const TcParams& p, int c0, bool valid, int n, int oh, int ow, float (&res)[32]) {
@@ -146,6 +135,8 @@ __device__ __forceinline__ void residual_fetch_nchw(const TcParams& p, int c0, b
     for (int j = 0; j < 32; ++j) res[j] = valid && c0 + j < p.Cout ? __ldg(src + (size_t)j * plane) : 0.0f;
 }
 
+// Epilogue for one 32-column chunk held by one thread (= one output pixel, 32 consecutive channels).
+// kSplit (three-pass tf32): the result may also leave as its tf32 high and low parts (TcParams::out_hi).
 // `nchw_res`: what residual_fetch_nchw read (kOutNCHW_F32 with a residual only).
 template <int kOutMode, bool kSplit = false>
 __device__ __forceinline__ void epilogue_chunk(const TcParams& p, const uint32_t (&v)[32], int c0, bool valid, int n,
@@ -246,14 +237,10 @@ __device__ __forceinline__ void epilogue_chunk(const TcParams& p, const uint32_t
             }
             if (p.round_out_tf32) {  // activation that feeds another tf32 contraction: store what it will read
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    uint32_t u = __float_as_uint(f[j]);
-                    if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0xfffu + ((u >> 13) & 1u)) & 0xffffe000u;
-                    f[j] = __uint_as_float(u);
-                }
+                for (int j = 0; j < 32; ++j) f[j] = tf32_rne(f[j]);
             }
             if constexpr (kSplit) {
-                if (p.out_hi != nullptr) {  // channel counts are multiples of 8 and the buffers aligned: 16-byte stores
+                if (p.out_hi != nullptr) {  // channel counts are multiples of 4 and the buffers aligned: 16-byte stores
                     float* hi = p.out_hi + pix * p.Cout + c0;
                     float* lo = hi + p.out_lo_offset;
 #pragma unroll

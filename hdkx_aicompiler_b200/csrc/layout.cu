@@ -6,33 +6,25 @@
 
 #include "common.cuh"
 #include "sm100.cuh"
+#include "tf32.cuh"
 
 namespace kxc_b200 {
 namespace {
-
-__device__ __forceinline__ float round_tf32_rne(float x) {
-    uint32_t u = __float_as_uint(x);
-    if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0xfffu + ((u >> 13) & 1u)) & 0xffffe000u;
-    return __uint_as_float(u);
-}
 
 template <typename TOut>
 __device__ __forceinline__ TOut convert_to(float v);
 template <>
 __device__ __forceinline__ __nv_bfloat16 convert_to<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 template <>
-__device__ __forceinline__ float convert_to<float>(float v) { return round_tf32_rne(v); }
+__device__ __forceinline__ float convert_to<float>(float v) { return tf32_rne(v); }
 
-// What single-pass tf32 drops: the tf32 rounding of (v - tf32(v)). a*b ~ a_hi*b_hi + a_hi*b_lo + a_lo*b_hi then carries
-// about 21 bits of each operand instead of 11.
+// what single-pass tf32 drops
 struct Tf32Lo {
     float v;
 };
 template <>
 __device__ __forceinline__ Tf32Lo convert_to<Tf32Lo>(float v) {
-    const float hi = round_tf32_rne(v);
-    // inf - inf would be NaN: a non-finite value lives in the high part only
-    return Tf32Lo{(__float_as_uint(v) & 0x7f800000u) == 0x7f800000u ? 0.0f : round_tf32_rne(__fsub_rn(v, hi))};
+    return Tf32Lo{tf32_low_part(v, tf32_rne(v))};
 }
 
 template <typename TIn, typename TOut>

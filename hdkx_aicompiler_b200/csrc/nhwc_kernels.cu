@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "sm100.cuh"
+#include "tf32.cuh"
 
 namespace kxc_b200 {
 namespace {
@@ -57,13 +58,8 @@ struct Vec<float> {
     }
     // fp32 storage holds tf32 operands: every stored activation is rounded (nearest even) to the 10-bit
     // mantissa the tensor cores read, so that what the next contraction sees is well defined
-    __device__ static float rnd(float x) {
-        uint32_t u = __float_as_uint(x);
-        if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0xfffu + ((u >> 13) & 1u)) & 0xffffe000u;
-        return __uint_as_float(u);
-    }
     __device__ static void store(float* p, const float (&f)[4]) {
-        *reinterpret_cast<float4*>(p) = make_float4(rnd(f[0]), rnd(f[1]), rnd(f[2]), rnd(f[3]));
+        *reinterpret_cast<float4*>(p) = make_float4(tf32_rne(f[0]), tf32_rne(f[1]), tf32_rne(f[2]), tf32_rne(f[3]));
     }
 };
 
@@ -271,22 +267,14 @@ __global__ void nhwc_to_nchw_kernel(const T* __restrict__ in, float* __restrict_
     }
 }
 
-__device__ __forceinline__ float round_tf32_rne(float x) {
-    uint32_t u = __float_as_uint(x);
-    if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0xfffu + ((u >> 13) & 1u)) & 0xffffe000u;
-    return __uint_as_float(u);
-}
 template <typename T>
 __device__ __forceinline__ T to_operand(float v);
 template <>
 __device__ __forceinline__ __nv_bfloat16 to_operand<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 template <>
-__device__ __forceinline__ float to_operand<float>(float v) { return round_tf32_rne(v); }
+__device__ __forceinline__ float to_operand<float>(float v) { return tf32_rne(v); }
 
-// The tf32 rounding of what round_tf32_rne drops (a non-finite value lives in the high part only).
-__device__ __forceinline__ float tf32_dropped(float x) {
-    return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u ? 0.0f : round_tf32_rne(__fsub_rn(x, round_tf32_rne(x)));
-}
+__device__ __forceinline__ float tf32_dropped(float x) { return tf32_low_part(x, tf32_rne(x)); }
 
 // Stem input packing: NCHW fp32 [N,C<=4,H,W] -> [N][H+2*pad_h][Wp][4] operand type with a zero border,
 // so that the 8 consecutive pixels x 4 channels starting at an even column form one K block.
