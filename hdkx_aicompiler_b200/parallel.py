@@ -1,7 +1,9 @@
 """Data-parallel plumbing for the operator path: contiguous batch shards and the one exchange step.
 
 Every image is independent through all 49 calls of the graph, so rank r of G simply owns images
-[r*N/G, (r+1)*N/G) with replicated weights. The only communication is the reference's
+[r*N/G, (r+1)*N/G) with replicated weights. (Independent, not bit for bit the same in every batch: bf16, tf32 and three-pass
+plans may split a layer's sums by the number of tiles of the batch, so N/G images can differ from the same images among N in
+the last bits of a sum. The fp32 plan gives equal bits.) The only communication is the reference's
 `device.gather_to_worker0`: concatenate the per-worker shards on dim 0, in worker order, into worker 0
 (CpuCCLBackend::GatherToWorker0 / ConcatFirstDim, src/base/disco/ccl_cpu.cc:274-294, :134-174).
 Works on any torch.distributed backend (NCCL on GPUs, gloo on CPU for the tests).

@@ -8,13 +8,14 @@ Precisions and what they cost in accuracy, measured on ResNet-18 with the benchm
 magnitude ~300) against the reference's fp32 arithmetic, worst element of the logits:
 
     "fp32"    CUDA cores in the reference's operation order            bit-identical
-    "tf32x3"  three tf32 tensor-core passes per contraction            8e-2 absolute, 2.6e-4 of the logit scale
+    "tf32x3"  three tf32 tensor-core passes per contraction            2e-3 to 8e-3 absolute, 0.7e-5 to 2.5e-5 of the scale
     "tf32"    one pass, operands rounded to tf32                       1.7e-1 absolute, 5.2e-4 of the logit scale
     "bf16"    bf16 activations and weights, fp32 accumulate            1.4 absolute, 4.2e-3 of the logit scale
 
 "tf32x3" removes the operand rounding (a single layer then agrees to ~2e-5), but not the rounding inside the tensor
 core's own fp32 accumulation, which truncates as it aligns the partial products of a long reduction; over twenty
-layers that is what remains, so only "fp32" reproduces the reference to the last bits.
+layers that is what remains (the lower figures at two images, whose reductions are split over several accumulators, the
+higher ones at 32), so only "fp32" reproduces the reference to the last bits.
 """
 import ctypes
 
