@@ -764,7 +764,7 @@ namespace {
 void pick_tile_nchw(int N, int OH, int OW, int Cout, int num_kb, int kb_bytes, int* BW, int* BH, int* BNI) {
     const int bn_out = Cout <= 64 ? 64 : (Cout <= 128 ? 128 : 256);
     const int tiles_c = (Cout + bn_out - 1) / bn_out;
-    const double main_loop = (double)num_kb * kb_bytes / 128.0 * (bn_out == 64 ? 490 : (bn_out == 128 ? 655 : 980));
+    const double main_loop = (double)num_kb * kb_bytes / 128.0 * (bn_out == 64 ? 550 : (bn_out == 128 ? 590 : 620));  // (choose_split's figures)
     double best = -1.0;
     for (int bw = 1; bw <= OW && bw <= 128; ++bw) {
         for (int bh = 1; bh <= OH && bw * bh <= 128; ++bh) {
