@@ -73,7 +73,9 @@ struct alignas(64) TcParams {
     long long out_lo_offset;
     int out_pitch;               // kOutNHWC_S8: channels per stored pixel (0: Cout), a multiple of 16
     int split;                   // 2..kMaxSplit: the reduction is split over clusters of that many CTAs (conv_splitk.cu); 0: it is not
-    int weights_ready;           // the packed weights were written long before this launch: they may be read ahead of its predecessor's end
+    // the packed weights were written long before this launch: they may be read ahead of its predecessor's end (set before the
+    // set-up functions, which weigh it)
+    int weights_ready;
 };
 
 struct TcConfig {

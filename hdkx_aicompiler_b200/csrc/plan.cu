@@ -927,6 +927,7 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
     }
     // ---- tensor maps and launch parameters ----
     for (auto& st : pl->steps) {
+        st.params.weights_ready = 1;  // packed by ordinary launches ahead of the run's first kernel
         if (st.kind == SKind::Conv) {
             PackedWeight& pw = pl->weights[st.weight];
             Value* ov = pl->find(st.out);
@@ -1152,7 +1153,6 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
                 p.bias = st.bias_const >= 0 ? static_cast<const float*>(arg_of(st.bias_const)) : nullptr;
                 p.bias2 = st.bias2_const >= 0 ? static_cast<const float*>(arg_of(st.bias2_const)) : nullptr;
                 if (st.out_is_graph_output) p.out = out_ptr;
-                p.weights_ready = 1;  // packed by ordinary launches ahead of the run's first kernel
                 p.reverse = (alternate_order && !pl->x3 && (tc_index++ & 1)) ? 1 : 0;
                 tc_finish_params(&p);
                 if (st.weight2 >= 0 && ((reinterpret_cast<uintptr_t>(p.bias2) | reinterpret_cast<uintptr_t>(p.out2)) & 15u)) p.vec_ok = 0;

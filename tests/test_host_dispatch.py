@@ -229,6 +229,19 @@ def test_nchw_tiles_are_narrow_while_all_are_resident(compile_graph, precision, 
     assert "bn64" in graph.launch_info()[-1][0]
 
 
+def test_operators_split_only_what_also_pays_behind_their_own_conversions(fake, compile_graph):
+    """The same convolution by itself and as a graph whose weights were packed long before: 14.0 us whole against 16.1 in two parts for
+    the operator, while a layer of the graph gains by the split."""
+    rc, message = conv(fake, _lib.PREC_TF32, 30, 42, 11, 11, 113, 3)
+    assert rc == 0, message
+    assert "conv_igemm" in launches(fake)[-1], launches(fake)[-1]
+    x = relay.Var("input", (30, 42, 11, 11))
+    call = relay.Call("nn_conv2d", [x, relay.Constant(DeviceTensor(np.empty((113, 42, 3, 3)))), relay.Constant(DeviceTensor(np.empty(113)))],
+                      relay.Conv2DAttrs((1, 1), (1, 1, 1, 1), (1, 1), 1))
+    graph, _ = compile_graph(relay.Function([x], relay.Call("nn_relu", [call])), "tf32")
+    assert "split" in graph.launch_info()[-1][0]
+
+
 def test_nchw_boxes_keep_long_runs_where_stores_would_outlast_the_main_loop(compile_graph):
     """135 K blocks do not hide the epilogue of one-column boxes: 204 us with 14x9x1, 174 with rows of 37."""
     x = relay.Var("input", (14, 457, 36, 37))
