@@ -375,6 +375,7 @@ __global__ void __launch_bounds__(kThreads8, 1) conv3x3_rowstack_s8_kernel(const
         if (lane == 0) {
             tma_prefetch_desc(&p.tmA[0]);
             tma_prefetch_desc(&p.tmB);
+            if (!p.weights_ready) pdl_wait();  // weights that the previous kernel packs
             mbar_arrive_expect_tx(smem_u32(&bar_w), kWeightBytes8);
             for (int kw = 0; kw < 3; ++kw)
                 for (int r = 0; r < 3; ++r)

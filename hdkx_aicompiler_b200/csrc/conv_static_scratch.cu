@@ -134,8 +134,8 @@ extern "C" int32_t kxc_b200_nn_conv2d_static_scratch(void** packed_args, const k
     KXC_TRY(scratch_for_current_device(&sc));
     unsigned char* act = sc.base;
     unsigned char* wp = sc.base + act_bytes;
-    KXC_TRY(nchw_to_nhwc(data, act, dt, d.N, d.C, d.H * d.W, cpad, s));
-    KXC_TRY(pack_weights_ohwi(weight, wp, dt, d.O, d.C, d.KH, d.KW, cpad, s));
+    const WeightPack pack{weight, wp, nullptr, d.O, d.C, d.KH * d.KW, cpad};
+    KXC_TRY(convert_operands(data, act, nullptr, dt, d.N, d.C, d.H * d.W, cpad, &pack, s, true));
     TcParams p{};
     TcConfig cfg{};
     KXC_TRY(tc_setup_conv(&p, &cfg, dt, kOutNCHW_F32, act, wp, d.N, d.H, d.W, cpad, d.O, d.KH, d.KW, d.SH, d.PH, d.PW, d.DH, d.DW,

@@ -84,9 +84,8 @@ int32_t conv2d_tensor_core(const float* data, const float* weight, const float* 
         float* act_hi = static_cast<float*>(ws.ptr);
         uint8_t* w_hi = static_cast<uint8_t*>(ws.ptr) + align_up(2 * act * 4, 1024);
         uint8_t* w_lo = w_hi + w_bytes;
-        KXC_TRY(nchw_to_nhwc_split(data, act_hi, act_hi + act, d.N, d.C, d.H * d.W, cpad, s));
-        KXC_TRY(pack_weights_ohwi(weight, w_hi, kTcTF32, d.O, d.C, d.KH, d.KW, cpad, s));
-        KXC_TRY(pack_weights_ohwi(weight, w_lo, kTcTF32, d.O, d.C, d.KH, d.KW, cpad, s, true, true));
+        const WeightPack pack{weight, w_hi, w_lo, d.O, d.C, d.KH * d.KW, cpad};
+        KXC_TRY(convert_operands(data, act_hi, act_hi + act, kTcTF32, d.N, d.C, d.H * d.W, cpad, &pack, s, true));
         TcParams p{};
         TcConfig cfg{};
         KXC_TRY(tc_setup_conv_x3(&p, &cfg, kOutNCHW_F32, act_hi, w_hi, w_lo, d.N, d.H, d.W, cpad, d.O, d.KH, d.KW, d.SH, d.PH, d.PW, d.DH,
@@ -107,8 +106,8 @@ int32_t conv2d_tensor_core(const float* data, const float* weight, const float* 
     KXC_TRY(ws.alloc(act_bytes + w_bytes));
     uint8_t* act = static_cast<uint8_t*>(ws.ptr);
     uint8_t* wp = act + act_bytes;
-    KXC_TRY(nchw_to_nhwc(data, act, dt, d.N, d.C, d.H * d.W, cpad, s));
-    KXC_TRY(pack_weights_ohwi(weight, wp, dt, d.O, d.C, d.KH, d.KW, cpad, s, false, true));
+    const WeightPack pack{weight, wp, nullptr, d.O, d.C, d.KH * d.KW, cpad};
+    KXC_TRY(convert_operands(data, act, nullptr, dt, d.N, d.C, d.H * d.W, cpad, &pack, s, true));
     TcParams p{};
     TcConfig cfg{};
     KXC_TRY(tc_setup_conv(&p, &cfg, dt, kOutNCHW_F32, act, wp, d.N, d.H, d.W, cpad, d.O, d.KH, d.KW, d.SH, d.PH, d.PW, d.DH,
@@ -166,6 +165,7 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
         TcParams p{};
         if (rowstack_ok) {
             KXC_TRY(rowstack3x3_s8_setup(&p, data, weight, d.N, d.H, d.W));
+            p.weights_ready = 1;
             p.bias_i32 = bias;
             p.multiplier = multiplier;
             p.shift = shift;
@@ -225,13 +225,12 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     uint8_t* act = static_cast<uint8_t*>(ws.ptr);
     uint8_t* wp = act + act_bytes;
     int8_t* out_nhwc = reinterpret_cast<int8_t*>(wp + w_bytes);
+    const WeightPack pack{weight, wp, nullptr, d.O, d.C, d.KH * d.KW, cpad};
     if (subsample) {
-        KXC_TRY(nchw_to_nhwc_s8_subsample(data, reinterpret_cast<int8_t*>(act), d.N, d.C, in_h, in_w, d.OH, d.OW, d.SH, cpad, s));
+        KXC_TRY(convert_operands_s8_subsample(data, reinterpret_cast<int8_t*>(act), d.N, d.C, in_h, in_w, d.OH, d.OW, d.SH, cpad, &pack, s, true));
     } else {
-        KXC_TRY(nchw_to_nhwc(data, act, dt, d.N, d.C, d.H * d.W, cpad, s));
+        KXC_TRY(convert_operands(data, act, nullptr, dt, d.N, d.C, d.H * d.W, cpad, &pack, s, true));
     }
-    // (the row-stacked kernel reads the weights ahead of its predecessor's end)
-    KXC_TRY(pack_weights_ohwi(weight, wp, dt, d.O, d.C, d.KH, d.KW, cpad, s, false, !rowstack_ok));
     TcParams p{};
     TcConfig cfg{};
     if (rowstack_ok) {
@@ -275,7 +274,7 @@ int32_t gemm_tensor_core(const float* a, const float* b, const float* c, float* 
         if (g.transB)
             KXC_TRY(split_rows(b, b_hi, b_lo, g.n, g.k, kpad, s));
         else
-            KXC_TRY(nchw_to_nhwc_split(b, b_hi, b_lo, 1, g.k, g.n, kpad, s));
+            KXC_TRY(convert_operands(b, b_hi, b_lo, kTcTF32, 1, g.k, g.n, kpad, nullptr, s, false));
         TcParams p{};
         TcConfig cfg{};
         KXC_TRY(tc_setup_conv_x3(&p, &cfg, kOutNHWC_F32, a_hi, b_hi, b_lo, g.m, 1, 1, kpad, g.n, 1, 1, 1, 0, 0, 1, 1));
@@ -297,7 +296,7 @@ int32_t gemm_tensor_core(const float* a, const float* b, const float* c, float* 
         KXC_TRY(convert_rows_two(a, ap, g.m, b, bp, g.n, dt, g.k, kpad, s));  // b is [N, K]
     } else {
         KXC_TRY(convert_rows(a, ap, dt, g.m, g.k, kpad, s));
-        KXC_TRY(nchw_to_nhwc(b, bp, dt, 1, g.k, g.n, kpad, s));  // b is [K, N] -> [N, Kpad]
+        KXC_TRY(convert_operands(b, bp, nullptr, dt, 1, g.k, g.n, kpad, nullptr, s, true));  // b is [K, N] -> [N, Kpad]
     }
     TcParams p{};
     TcConfig cfg{};

@@ -32,53 +32,98 @@ __device__ __forceinline__ TOut convert_elem(TIn v) { return convert_to<TOut>((f
 template <>
 __device__ __forceinline__ int8_t convert_elem<int8_t, int8_t>(int8_t v) { return v; }
 
-// `overlap` (here and in pack_weights_kernel): the next kernel's CTAs may set themselves up while this one runs; they wait for its
-// end before they read. Never for weights that a kernel reads ahead of its predecessor's end: those of a plan
-// (TcParams::weights_ready) and of the row-stacked kernels.
-// grid (ceil(HW/32), ceil(cpad/32), N), block (32, 8)
-template <typename TIn, typename TOut>
-__global__ void nchw_to_nhwc_kernel(const TIn* __restrict__ in, TOut* __restrict__ out, int C, int HW, int cpad, int overlap) {
-    if (overlap) sm100::pdl_launch_dependents();
-    __shared__ TIn tile[32][33];
-    const int n = blockIdx.z;
-    const int hw0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-    const TIn* src = in + (size_t)n * C * HW;
-    TOut* dst = out + (size_t)n * HW * cpad;
+// Weights OIHW -> [O][KH*KW][cpad] (channels c >= C zero): a thread takes the whole filter of one output channel and kVec input
+// channels, so that its reads are consecutive words and its stores are whole 32-bit words side by side with its neighbours'.
+template <typename TIn, typename TOut, bool kSplit>
+__device__ __forceinline__ void pack_weights_block(const TIn* __restrict__ w, TOut* __restrict__ out, TOut* __restrict__ lo, int64_t groups, int C,
+                                                   int taps, int cpad, int64_t block) {
+    constexpr int kVec = 4 / (int)sizeof(TOut);
+    const int64_t g = block * 256 + threadIdx.x;
+    if (g >= groups) return;
+    const int per_row = cpad / kVec;
+    const int o = (int)(g / per_row), c0 = (int)(g - (int64_t)o * per_row) * kVec;
+    const TIn* src = w + ((int64_t)o * C + c0) * taps;
+    TOut* dst = out + (int64_t)o * taps * cpad + c0;
+    const int64_t lo_off = kSplit ? lo - out : 0;
+#pragma unroll 9
+    for (int t = 0; t < taps; ++t) {
+        alignas(4) TOut v[kVec];
+        [[maybe_unused]] TOut l[kVec];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int c = c0 + threadIdx.y + 8 * k, hw = hw0 + threadIdx.x;
-        tile[threadIdx.y + 8 * k][threadIdx.x] = (c < C && hw < HW) ? src[(size_t)c * HW + hw] : (TIn)0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int hw = hw0 + threadIdx.y + 8 * k, c = c0 + threadIdx.x;
-        if (hw < HW && c < cpad) dst[(size_t)hw * cpad + c] = convert_elem<TIn, TOut>(tile[threadIdx.x][threadIdx.y + 8 * k]);
+        for (int e = 0; e < kVec; ++e) {
+            const TIn x = c0 + e < C ? __ldg(src + (int64_t)e * taps + t) : (TIn)0;
+            v[e] = convert_elem<TIn, TOut>(x);
+            if constexpr (kSplit) l[e] = convert_to<Tf32Lo>(x).v;
+        }
+        *reinterpret_cast<uint32_t*>(dst + (int64_t)t * cpad) = *reinterpret_cast<const uint32_t*>(v);
+        if constexpr (kSplit) dst[lo_off + (int64_t)t * cpad] = l[0];
     }
 }
 
-// Both tf32 parts of every value in one pass over the input (three-pass tf32). Same grid and block.
-__global__ void nchw_to_nhwc_split_kernel(const float* __restrict__ in, float* __restrict__ hi, float* __restrict__ lo, int C, int HW, int cpad) {
-    __shared__ float tile[32][33];
-    const int n = blockIdx.z;
-    const int hw0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-    const float* src = in + (size_t)n * C * HW;
-    const size_t dst = (size_t)n * HW * cpad;
+struct PackArgs {
+    const void* w = nullptr;
+    void* out = nullptr;
+    void* lo = nullptr;   // three-pass tf32: the low parts
+    int64_t groups = 0;   // threads that have work (pack_weights_block)
+    int C = 0, taps = 0, cpad = 0;
+    unsigned blocks = 0;
+};
+
+// Activations NCHW fp32 -> NHWC of the operand type and, in the first blocks of the same launch, the weights of the convolution
+// that follows. One launch instead of two (each cost 2 to 3 us of launch and drain beside 2 to 5 us of work: conv 72 -> 120 3x3
+// at 45x51, 9 images, tf32: 38.9 -> 32.3 us a call). A block turns kCT channels x 2048 / kCT pixels through shared memory with
+// eight loads in flight per thread; stores are channel pairs, 128 or 256 bytes per pixel (kCT = 64; 32 for fewer channels).
+// Bound by memory: 4 bytes read and 2, 4 or 8 written per value.
+//
+// Programmatic launch on both sides: the blocks wait for the previous kernel before they touch memory, and with `overlap` then
+// let the next kernel's CTAs set themselves up. Weights packed here are not TcParams::weights_ready for the kernel after it (it
+// waits before it reads them); those of a plan come from launches before this one, which have ended by the time its blocks let
+// go. A launch that packs a plan's weights does not let go early: the kernel after the next may read them ahead.
+template <typename TOut, bool kSplit, int kCT>
+__global__ void __launch_bounds__(256) convert_operands_kernel(const float* __restrict__ in, TOut* __restrict__ out, TOut* __restrict__ lo, int C,
+                                                               int HW, int cpad, int tiles_hw, int tiles_c, PackArgs pack, int overlap) {
+    constexpr int kPT = 2048 / kCT;
+    sm100::pdl_wait();
+    if (overlap) sm100::pdl_launch_dependents();
+    if (blockIdx.x < pack.blocks) {
+        pack_weights_block<float, TOut, kSplit>(static_cast<const float*>(pack.w), static_cast<TOut*>(pack.out), static_cast<TOut*>(pack.lo),
+                                                pack.groups, pack.C, pack.taps, pack.cpad, blockIdx.x);
+        return;
+    }
+    __shared__ float tile[kCT][kPT + 1];
+    unsigned t = blockIdx.x - pack.blocks;
+    const int hw0 = (int)(t % (unsigned)tiles_hw) * kPT;
+    t /= (unsigned)tiles_hw;
+    const int c0 = (int)(t % (unsigned)tiles_c) * kCT;
+    const int n = (int)(t / (unsigned)tiles_c);
+    const float* src = in + ((int64_t)n * C + c0) * HW + hw0;
+    const int64_t dst = ((int64_t)n * HW + hw0) * cpad + c0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int c = c0 + threadIdx.y + 8 * k, hw = hw0 + threadIdx.x;
-        tile[threadIdx.y + 8 * k][threadIdx.x] = (c < C && hw < HW) ? src[(size_t)c * HW + hw] : 0.0f;
+    for (int k = 0; k < 8; ++k) {
+        const int i = (int)threadIdx.x + 256 * k, p = i % kPT, c = i / kPT;
+        tile[c][p] = (c0 + c < C && hw0 + p < HW) ? __ldg(src + (int64_t)c * HW + p) : 0.0f;
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int hw = hw0 + threadIdx.y + 8 * k, c = c0 + threadIdx.x;
-        if (hw < HW && c < cpad) {
-            const float v = tile[threadIdx.x][threadIdx.y + 8 * k];
-            hi[dst + (size_t)hw * cpad + c] = convert_to<float>(v);
-            lo[dst + (size_t)hw * cpad + c] = convert_to<Tf32Lo>(v).v;
+        const int i = (int)threadIdx.x + 256 * k, c = i % (kCT / 2) * 2, p = i / (kCT / 2);
+        if (hw0 + p >= HW || c0 + c >= cpad) continue;  // (cpad is even)
+        const float x = tile[c][p], y = tile[c + 1][p];
+        const int64_t at = dst + (int64_t)p * cpad + c;
+        if constexpr (sizeof(TOut) == 2) {
+            *reinterpret_cast<__nv_bfloat162*>(out + at) = __nv_bfloat162(convert_to<TOut>(x), convert_to<TOut>(y));
+        } else {
+            *reinterpret_cast<float2*>(out + at) = make_float2(convert_to<float>(x), convert_to<float>(y));
+            if constexpr (kSplit) *reinterpret_cast<float2*>(lo + at) = make_float2(convert_to<Tf32Lo>(x).v, convert_to<Tf32Lo>(y).v);
         }
     }
+}
+
+// Weights alone: constants of a plan, packed once.
+template <typename TIn, typename TOut, bool kSplit>
+__global__ void __launch_bounds__(256) pack_weights_kernel(PackArgs pack) {
+    pack_weights_block<TIn, TOut, kSplit>(static_cast<const TIn*>(pack.w), static_cast<TOut*>(pack.out), static_cast<TOut*>(pack.lo), pack.groups,
+                                          pack.C, pack.taps, pack.cpad, blockIdx.x);
 }
 
 // The same for rows that need no reordering: [rows, cols] -> two times [rows, cpad]. cols % 4 == 0 and cols == cpad take
@@ -106,15 +151,13 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
 }
 
 // int8 form: 64 channels x 64 pixels per block, four bytes per thread on both sides (64-byte runs in HBM instead of the
-// 32-byte runs the element-wise kernel makes of 1-byte elements). grid (ceil(HW/64), ceil(cpad/64), N), block 256.
+// 32-byte runs an element-wise kernel makes of 1-byte elements). Tiles ceil(HW/64) x ceil(cpad/64) x N, block 256.
 // It is a batched byte transpose [C][HW] -> [HW][cpad] (rows c >= C read as zero), so it also serves NHWC -> NCHW with
 // the roles of the two extents exchanged (source rows `pitch` bytes apart); vec_out = 0 when the destination rows are not 4-byte multiples.
-// rows_on_x (here and in transpose_bytes_kernel): the first two grid dimensions are exchanged, see transpose_grid.
-__global__ void __launch_bounds__(256) nchw_to_nhwc_s8_kernel(const int8_t* __restrict__ in, int8_t* __restrict__ out, int C, int HW,
-                                                               int pitch, int cpad, int vec_in, int vec_out, int rows_on_x) {
+__device__ __forceinline__ void transpose_s8_tile(const int8_t* __restrict__ in, int8_t* __restrict__ out, int C, int HW, int pitch, int cpad,
+                                                  int vec_in, int vec_out, int hw_tile, int c_tile, int n) {
     __shared__ __align__(4) int8_t tile[64][68];
-    const int n = blockIdx.z;
-    const int hw0 = (int)(rows_on_x ? blockIdx.y : blockIdx.x) * 64, c0 = (int)(rows_on_x ? blockIdx.x : blockIdx.y) * 64;
+    const int hw0 = hw_tile * 64, c0 = c_tile * 64;
     const int8_t* src = in + (size_t)n * C * pitch;
     int8_t* dst = out + (size_t)n * HW * cpad;
     const int q = threadIdx.x & 15, r = threadIdx.x >> 4;  // 16 four-byte columns x 16 rows per pass
@@ -159,14 +202,14 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_s8_kernel(const int8_t* __re
 // shared memory, as above, held the kernel to 3 TB/s: 17 us for 25.7 MB in and out, this one 12 to 13), reads V bytes of four
 // rows at a time and parks whole words in shared memory; word (column p, quad q) lies at q ^ f(p), so that a warp's stores,
 // whose columns are V apart, fall on 16 banks and its reads, one column per 16 lanes, on 32.
-// Tile 64 rows x TP columns. grid (ceil(W/TP), ceil(max(R, opitch)/64), batch), block 256.
+// Tile 64 rows x TP columns: ceil(W/TP) x ceil(max(R, opitch)/64) x batch of them, block 256.
 template <int V, int TP>
-__global__ void __launch_bounds__(256) transpose_bytes_kernel(const int8_t* __restrict__ in, int8_t* __restrict__ out, int R, int W, int pitch,
-                                                               int opitch, int rows_on_x) {
+__device__ __forceinline__ void transpose_bytes_tile(const int8_t* __restrict__ in, int8_t* __restrict__ out, int R, int W, int pitch, int opitch,
+                                                     int w_tile, int r_tile, int batch) {
     __shared__ uint32_t tile[TP * 16];
-    const int w0 = (int)(rows_on_x ? blockIdx.y : blockIdx.x) * TP, r0 = (int)(rows_on_x ? blockIdx.x : blockIdx.y) * 64;
-    const int8_t* src = in + (int64_t)blockIdx.z * R * pitch;
-    int8_t* dst = out + (int64_t)blockIdx.z * W * opitch;
+    const int w0 = w_tile * TP, r0 = r_tile * 64;
+    const int8_t* src = in + (int64_t)batch * R * pitch;
+    int8_t* dst = out + (int64_t)batch * W * opitch;
     auto slot = [](int p, int q) { return p * 16 + (q ^ (((p >> 2) ^ (p >> 4)) & 15)); };
     constexpr int kWords = V / 4, kVecs = TP / V;
 #pragma unroll
@@ -204,42 +247,13 @@ __global__ void __launch_bounds__(256) transpose_bytes_kernel(const int8_t* __re
     }
 }
 
-// Grid of a batched transpose: column tiles, row tiles, batch. The row tiles of a whole plane (NHWC -> NCHW: pixels) can be more
-// than the 65535 that the second dimension holds; they change places with the column tiles then, of which there are few.
-dim3 transpose_grid(int cols, int rows, int batch, int* rows_on_x) {
-    *rows_on_x = rows > 65535 ? 1 : 0;
-    return *rows_on_x ? dim3((unsigned)rows, (unsigned)cols, (unsigned)batch) : dim3((unsigned)cols, (unsigned)rows, (unsigned)batch);
-}
-
-// Batched byte transpose of `batch` matrices; false when the pitches or addresses do not suit the kernel above.
-bool transpose_bytes(const int8_t* in, int8_t* out, int batch, int R, int W, int pitch, int opitch, cudaStream_t s) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(in);
-    if ((pitch & 3) != 0 || (opitch & 3) != 0 || (a & 3u) != 0 || (reinterpret_cast<uintptr_t>(out) & 3u) != 0) return false;
-    const bool wide = (pitch & 15) == 0 && (a & 15u) == 0;
-    const int tp = W <= 64 ? 64 : (W <= 128 ? 128 : 256);
-    int rows_on_x = 0;
-    const dim3 grid = transpose_grid((W + tp - 1) / tp, ((R > opitch ? R : opitch) + 63) / 64, batch, &rows_on_x);
-    auto go = [&](auto kernel) { kernel<<<grid, 256, 0, s>>>(in, out, R, W, pitch, opitch, rows_on_x); };
-    if (wide) {
-        if (tp == 64) go(transpose_bytes_kernel<16, 64>);
-        else if (tp == 128) go(transpose_bytes_kernel<16, 128>);
-        else go(transpose_bytes_kernel<16, 256>);
-    } else {
-        if (tp == 64) go(transpose_bytes_kernel<4, 64>);
-        else if (tp == 128) go(transpose_bytes_kernel<4, 128>);
-        else go(transpose_bytes_kernel<4, 256>);
-    }
-    return true;
-}
-
 // int8 NCHW -> NHWC of the pixels a 1x1 convolution of stride `st` (no padding) reads: out[n][p][c] =
-// in[n][c][(p / OW) * st][(p % OW) * st], p = oh * OW + ow. grid (ceil(OH*OW/64), ceil(cpad/64), N), block 256: the same
+// in[n][c][(p / OW) * st][(p % OW) * st], p = oh * OW + ow. Tiles ceil(OH*OW/64) x ceil(cpad/64) x N, block 256: the same
 // 64 x 64 byte transpose as above with gathered source pixels; the rows the convolution skips are never touched.
-__global__ void __launch_bounds__(256) nchw_to_nhwc_s8_subsample_kernel(const int8_t* __restrict__ in, int8_t* __restrict__ out, int C,
-                                                                         int H, int W, int OH, int OW, int st, int cpad) {
+__device__ __forceinline__ void subsample_s8_tile(const int8_t* __restrict__ in, int8_t* __restrict__ out, int C, int H, int W, int OH, int OW,
+                                                  int st, int cpad, int p_tile, int c_tile, int n) {
     __shared__ __align__(4) int8_t tile[64][68];
-    const int n = blockIdx.z;
-    const int p0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
+    const int p0 = p_tile * 64, c0 = c_tile * 64;
     const int P = OH * OW;
     const int8_t* src = in + (size_t)n * C * H * W;
     int8_t* dst = out + (size_t)n * P * cpad;
@@ -275,18 +289,37 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_s8_subsample_kernel(const in
     }
 }
 
-template <typename TIn, typename TOut>
-__global__ void pack_weights_kernel(const TIn* __restrict__ w, TOut* __restrict__ out, int O, int C, int KH, int KW, int cpad, int overlap) {
+// How the tiles of an int8 transposition are turned
+enum TransposeForm : int { kTurnBytes, kTurnWords, kTurnVectors, kTurnSubsampled };
+
+struct TransposeArgs {
+    const int8_t* in;
+    int8_t* out;
+    int R, W, pitch, opitch;  // R rows of `pitch` bytes, W of them used -> W rows of `opitch` bytes
+    int vec_in, vec_out;      // kTurnBytes
+    int H, OH, OW, stride;    // kTurnSubsampled (W: the input's columns)
+    int tiles_w, tiles_r;
+};
+
+// The int8 counterpart of convert_operands_kernel: the activations' byte transposition and the weights of the same convolution.
+// Also the way back (results NHWC -> NCHW, without weights). (128 -> 128 3x3 at 28x28, 256 images: 74.0 -> 68.6 us a call.)
+template <int kForm, int TP>
+__global__ void __launch_bounds__(256) transpose_bytes_kernel(TransposeArgs a, PackArgs pack, int overlap) {
+    sm100::pdl_wait();
     if (overlap) sm100::pdl_launch_dependents();
-    const int64_t total = (int64_t)O * KH * KW * cpad;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int c = (int)(i % cpad);
-        int64_t t = i / cpad;
-        const int kw = (int)(t % KW); t /= KW;
-        const int kh = (int)(t % KH);
-        const int o = (int)(t / KH);
-        out[i] = c < C ? convert_elem<TIn, TOut>(w[(((int64_t)o * C + c) * KH + kh) * KW + kw]) : convert_elem<TIn, TOut>((TIn)0);
+    if (blockIdx.x < pack.blocks) {
+        pack_weights_block<int8_t, int8_t, false>(static_cast<const int8_t*>(pack.w), static_cast<int8_t*>(pack.out), nullptr, pack.groups, pack.C,
+                                                  pack.taps, pack.cpad, blockIdx.x);
+        return;
     }
+    unsigned t = blockIdx.x - pack.blocks;
+    const int tw = (int)(t % (unsigned)a.tiles_w);
+    t /= (unsigned)a.tiles_w;
+    const int tr = (int)(t % (unsigned)a.tiles_r), n = (int)(t / (unsigned)a.tiles_r);
+    if constexpr (kForm == kTurnVectors) transpose_bytes_tile<16, TP>(a.in, a.out, a.R, a.W, a.pitch, a.opitch, tw, tr, n);
+    else if constexpr (kForm == kTurnWords) transpose_bytes_tile<4, TP>(a.in, a.out, a.R, a.W, a.pitch, a.opitch, tw, tr, n);
+    else if constexpr (kForm == kTurnBytes) transpose_s8_tile(a.in, a.out, a.R, a.W, a.pitch, a.opitch, a.vec_in, a.vec_out, tw, tr, n);
+    else subsample_s8_tile(a.in, a.out, a.R, a.H, a.W, a.OH, a.OW, a.stride, a.opitch, tw, tr, n);
 }
 
 template <typename TOut>
@@ -325,42 +358,81 @@ int grid_1d(int64_t items, int threads) {
     return (int)b;
 }
 
-}  // namespace
-
-int32_t nchw_to_nhwc(const void* in, void* out, TcDType dtype, int N, int C, int HW, int cpad, cudaStream_t s, bool tf32_lo, bool overlap) {
-    if (N == 0) return KXC_B200_OK;
-    if (N > 65535) return fail(KXC_B200_ERR_UNSUPPORTED, "layout transform: batch %d exceeds the grid limit", N);
-    const dim3 grid((HW + 31) / 32, (cpad + 31) / 32, N), block(32, 8);
-    switch (dtype) {
-        case kTcBF16:
-            nchw_to_nhwc_kernel<float, __nv_bfloat16><<<grid, block, 0, s>>>(static_cast<const float*>(in), static_cast<__nv_bfloat16*>(out), C, HW, cpad, overlap ? 1 : 0);
-            break;
-        case kTcTF32:
-            if (tf32_lo)
-                nchw_to_nhwc_kernel<float, Tf32Lo><<<grid, block, 0, s>>>(static_cast<const float*>(in), static_cast<Tf32Lo*>(out), C, HW, cpad, overlap ? 1 : 0);
-            else
-                nchw_to_nhwc_kernel<float, float><<<grid, block, 0, s>>>(static_cast<const float*>(in), static_cast<float*>(out), C, HW, cpad, overlap ? 1 : 0);
-            break;
-        case kTcS8:
-            if (transpose_bytes(static_cast<const int8_t*>(in), static_cast<int8_t*>(out), N, C, HW, HW, cpad, s)) break;
-            if ((cpad & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 3u) == 0) {
-                const int vec_in = ((HW & 3) == 0 && (reinterpret_cast<uintptr_t>(in) & 3u) == 0) ? 1 : 0;
-                int rows_on_x = 0;
-                const dim3 g = transpose_grid((HW + 63) / 64, (cpad + 63) / 64, N, &rows_on_x);
-                nchw_to_nhwc_s8_kernel<<<g, 256, 0, s>>>(static_cast<const int8_t*>(in), static_cast<int8_t*>(out), C, HW, HW, cpad, vec_in, 1, rows_on_x);
-            } else {
-                nchw_to_nhwc_kernel<int8_t, int8_t><<<grid, block, 0, s>>>(static_cast<const int8_t*>(in), static_cast<int8_t*>(out), C, HW, cpad, overlap ? 1 : 0);
-            }
-            break;
-    }
-    return check_launch("nchw_to_nhwc");
+template <typename T>
+PackArgs pack_args(const WeightPack* w) {
+    PackArgs p;
+    if (w == nullptr || (int64_t)w->O * w->taps * w->cpad == 0) return p;
+    p.w = w->w; p.out = w->out; p.lo = w->lo;
+    p.C = w->C; p.taps = w->taps; p.cpad = w->cpad;
+    p.groups = (int64_t)w->O * (w->cpad / (4 / (int)sizeof(T)));
+    p.blocks = (unsigned)((p.groups + 255) / 256);
+    return p;
 }
 
-int32_t nchw_to_nhwc_split(const float* in, float* hi, float* lo, int N, int C, int HW, int cpad, cudaStream_t s) {
+// Tiles of an activation conversion and the blocks that pack weights, as one grid dimension.
+int32_t one_dim_grid(int64_t tiles_a, int64_t tiles_b, int64_t batch, unsigned pack_blocks, unsigned* grid) {
+    const int64_t blocks = tiles_a * tiles_b * batch + pack_blocks;
+    if (blocks > 0x7fffffffll) return fail(KXC_B200_ERR_UNSUPPORTED, "layout transform: %lld tiles exceed the grid limit", (long long)blocks);
+    *grid = (unsigned)blocks;
+    return KXC_B200_OK;
+}
+
+template <typename TOut, bool kSplit>
+int32_t launch_convert(const float* in, void* out, void* lo, int N, int C, int HW, int cpad, const WeightPack* w, cudaStream_t s, bool overlap) {
+    const PackArgs pack = pack_args<TOut>(w);
+    auto go = [&](auto kernel, int ct) -> int32_t {
+        const int tiles_hw = (int)(((int64_t)HW + 2048 / ct - 1) / (2048 / ct)), tiles_c = (cpad + ct - 1) / ct;
+        unsigned grid = 0;
+        KXC_TRY(one_dim_grid(tiles_hw, tiles_c, N, pack.blocks, &grid));
+        KXC_CUDA_TRY(launch_kernel(kernel, dim3(grid), dim3(256), 0, s, /*pdl=*/true, 1, in, static_cast<TOut*>(out), static_cast<TOut*>(lo), C, HW,
+                                   cpad, tiles_hw, tiles_c, pack, overlap ? 1 : 0));
+        return check_launch("convert_operands");
+    };
+    return cpad <= 32 ? go(convert_operands_kernel<TOut, kSplit, 32>, 32) : go(convert_operands_kernel<TOut, kSplit, 64>, 64);
+}
+
+// Byte transposition of `batch` matrices, by words turned in registers where pitches and addresses allow it.
+int32_t launch_transpose(const int8_t* in, int8_t* out, int batch, int R, int W, int pitch, int opitch, const WeightPack* w, cudaStream_t s,
+                         bool overlap) {
+    const PackArgs pack = pack_args<int8_t>(w);
+    const uintptr_t ia = reinterpret_cast<uintptr_t>(in), oa = reinterpret_cast<uintptr_t>(out);
+    TransposeArgs a{};
+    a.in = in; a.out = out; a.R = R; a.W = W; a.pitch = pitch; a.opitch = opitch;
+    auto go = [&](auto kernel, int tp, int rows) -> int32_t {
+        a.tiles_w = (int)(((int64_t)W + tp - 1) / tp);
+        a.tiles_r = (int)(((int64_t)rows + 63) / 64);
+        unsigned grid = 0;
+        KXC_TRY(one_dim_grid(a.tiles_w, a.tiles_r, batch, pack.blocks, &grid));
+        KXC_CUDA_TRY(launch_kernel(kernel, dim3(grid), dim3(256), 0, s, /*pdl=*/true, 1, a, pack, overlap ? 1 : 0));
+        return check_launch("transpose_bytes");
+    };
+    if ((pitch & 3) == 0 && (opitch & 3) == 0 && (ia & 3u) == 0 && (oa & 3u) == 0) {
+        const int rows = R > opitch ? R : opitch;
+        const bool wide = (pitch & 15) == 0 && (ia & 15u) == 0;
+        if (W <= 64) return wide ? go(transpose_bytes_kernel<kTurnVectors, 64>, 64, rows) : go(transpose_bytes_kernel<kTurnWords, 64>, 64, rows);
+        if (W <= 128) return wide ? go(transpose_bytes_kernel<kTurnVectors, 128>, 128, rows) : go(transpose_bytes_kernel<kTurnWords, 128>, 128, rows);
+        return wide ? go(transpose_bytes_kernel<kTurnVectors, 256>, 256, rows) : go(transpose_bytes_kernel<kTurnWords, 256>, 256, rows);
+    }
+    a.vec_in = (pitch & 3) == 0 && (ia & 3u) == 0;
+    a.vec_out = (opitch & 3) == 0 && (oa & 3u) == 0;
+    return go(transpose_bytes_kernel<kTurnBytes, 64>, 64, opitch);
+}
+
+}  // namespace
+
+int32_t convert_operands(const void* in, void* out, void* lo, TcDType dtype, int N, int C, int HW, int cpad, const WeightPack* w, cudaStream_t s,
+                         bool overlap) {
     if (N == 0) return KXC_B200_OK;
     if (N > 65535) return fail(KXC_B200_ERR_UNSUPPORTED, "layout transform: batch %d exceeds the grid limit", N);
-    nchw_to_nhwc_split_kernel<<<dim3((HW + 31) / 32, (cpad + 31) / 32, N), dim3(32, 8), 0, s>>>(in, hi, lo, C, HW, cpad);
-    return check_launch("nchw_to_nhwc_split");
+    const float* f = static_cast<const float*>(in);
+    switch (dtype) {
+        case kTcBF16: return launch_convert<__nv_bfloat16, false>(f, out, nullptr, N, C, HW, cpad, w, s, overlap);
+        case kTcTF32:
+            return lo != nullptr ? launch_convert<float, true>(f, out, lo, N, C, HW, cpad, w, s, overlap)
+                                 : launch_convert<float, false>(f, out, nullptr, N, C, HW, cpad, w, s, overlap);
+        case kTcS8: return launch_transpose(static_cast<const int8_t*>(in), static_cast<int8_t*>(out), N, C, HW, HW, cpad, w, s, overlap);
+    }
+    return fail(KXC_B200_ERR_INVALID, "convert_operands: dtype");
 }
 
 int32_t convert_rows_two(const float* a, void* out_a, int64_t rows_a, const float* b, void* out_b, int64_t rows_b, TcDType dtype, int cols,
@@ -391,46 +463,43 @@ int32_t split_rows(const float* in, float* hi, float* lo, int64_t rows, int cols
     return check_launch("split_rows");
 }
 
-int32_t nchw_to_nhwc_s8_subsample(const int8_t* in, int8_t* out, int N, int C, int H, int W, int OH, int OW, int stride, int cpad,
-                                  cudaStream_t s) {
+int32_t convert_operands_s8_subsample(const int8_t* in, int8_t* out, int N, int C, int H, int W, int OH, int OW, int stride, int cpad,
+                                      const WeightPack* w, cudaStream_t s, bool overlap) {
     if (N == 0 || C == 0 || OH == 0 || OW == 0) return KXC_B200_OK;
     if ((cpad & 3) != 0 || (reinterpret_cast<uintptr_t>(out) & 3u) != 0 || N > 65535 || (long long)H * W > 0x7fffffffll)
-        return fail(KXC_B200_ERR_UNSUPPORTED, "nchw_to_nhwc_s8_subsample: %d padded channels, %d images", cpad, N);
-    nchw_to_nhwc_s8_subsample_kernel<<<dim3((OH * OW + 63) / 64, (cpad + 63) / 64, N), 256, 0, s>>>(in, out, C, H, W, OH, OW, stride, cpad);
-    return check_launch("nchw_to_nhwc_s8_subsample");
+        return fail(KXC_B200_ERR_UNSUPPORTED, "convert_operands_s8_subsample: %d padded channels, %d images", cpad, N);
+    const PackArgs pack = pack_args<int8_t>(w);
+    TransposeArgs a{};
+    a.in = in; a.out = out; a.R = C; a.W = W; a.opitch = cpad;
+    a.H = H; a.OH = OH; a.OW = OW; a.stride = stride;
+    a.tiles_w = (OH * OW + 63) / 64;
+    a.tiles_r = (cpad + 63) / 64;
+    unsigned grid = 0;
+    KXC_TRY(one_dim_grid(a.tiles_w, a.tiles_r, N, pack.blocks, &grid));
+    KXC_CUDA_TRY(launch_kernel(transpose_bytes_kernel<kTurnSubsampled, 64>, dim3(grid), dim3(256), 0, s, /*pdl=*/true, 1, a, pack, overlap ? 1 : 0));
+    return check_launch("convert_operands_s8_subsample");
 }
 
 int32_t nhwc_to_nchw_s8(const int8_t* in, int8_t* out, int N, int C, int pitch, int HW, cudaStream_t s) {
     if (N == 0 || C == 0 || HW == 0) return KXC_B200_OK;
     // source rows = pixels (C bytes of `pitch`), destination rows = channels (HW bytes each)
-    if (!transpose_bytes(in, out, N, HW, C, pitch, HW, s)) {
-        const int vec_in = ((pitch & 3) == 0 && (reinterpret_cast<uintptr_t>(in) & 3u) == 0) ? 1 : 0;
-        const int vec_out = ((HW & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 3u) == 0) ? 1 : 0;
-        int rows_on_x = 0;
-        const dim3 g = transpose_grid((C + 63) / 64, (HW + 63) / 64, N, &rows_on_x);
-        nchw_to_nhwc_s8_kernel<<<g, 256, 0, s>>>(in, out, HW, C, pitch, HW, vec_in, vec_out, rows_on_x);
-    }
-    return check_launch("nhwc_to_nchw_s8");
+    return launch_transpose(in, out, N, HW, C, pitch, HW, nullptr, s, false);
 }
 
-int32_t pack_weights_ohwi(const void* w, void* out, TcDType dtype, int O, int C, int KH, int KW, int cpad, cudaStream_t s, bool tf32_lo, bool overlap) {
-    const int64_t total = (int64_t)O * KH * KW * cpad;
-    const int grid = grid_1d(total, 256);
+int32_t pack_weights_ohwi(const WeightPack& w, TcDType dtype, cudaStream_t s) {
+    auto go = [&](auto kernel, const PackArgs& p) -> int32_t {
+        if (p.blocks == 0) return KXC_B200_OK;
+        kernel<<<p.blocks, 256, 0, s>>>(p);
+        return check_launch("pack_weights");
+    };
     switch (dtype) {
-        case kTcBF16:
-            pack_weights_kernel<float, __nv_bfloat16><<<grid, 256, 0, s>>>(static_cast<const float*>(w), static_cast<__nv_bfloat16*>(out), O, C, KH, KW, cpad, overlap ? 1 : 0);
-            break;
+        case kTcBF16: return go(pack_weights_kernel<float, __nv_bfloat16, false>, pack_args<__nv_bfloat16>(&w));
         case kTcTF32:
-            if (tf32_lo)
-                pack_weights_kernel<float, Tf32Lo><<<grid, 256, 0, s>>>(static_cast<const float*>(w), static_cast<Tf32Lo*>(out), O, C, KH, KW, cpad, overlap ? 1 : 0);
-            else
-                pack_weights_kernel<float, float><<<grid, 256, 0, s>>>(static_cast<const float*>(w), static_cast<float*>(out), O, C, KH, KW, cpad, overlap ? 1 : 0);
-            break;
-        case kTcS8:
-            pack_weights_kernel<int8_t, int8_t><<<grid, 256, 0, s>>>(static_cast<const int8_t*>(w), static_cast<int8_t*>(out), O, C, KH, KW, cpad, overlap ? 1 : 0);
-            break;
+            return w.lo != nullptr ? go(pack_weights_kernel<float, float, true>, pack_args<float>(&w))
+                                   : go(pack_weights_kernel<float, float, false>, pack_args<float>(&w));
+        case kTcS8: return go(pack_weights_kernel<int8_t, int8_t, false>, pack_args<int8_t>(&w));
     }
-    return check_launch("pack_weights");
+    return fail(KXC_B200_ERR_INVALID, "pack_weights: dtype");
 }
 
 int32_t convert_rows(const float* in, void* out, TcDType dtype, int64_t rows, int cols, int cpad, cudaStream_t s, bool tf32_lo) {

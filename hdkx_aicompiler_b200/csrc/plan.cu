@@ -1100,18 +1100,17 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
         const void* src = arg_of(w.const_id);
         if (src == w.source) continue;
         switch (w.mode) {
-            case 0: KXC_TRY(pack_weights_ohwi(src, w.ptr, dt, w.O, w.C, w.KH, w.KW, w.cpad, s)); break;
+            case 0: KXC_TRY(pack_weights_ohwi(WeightPack{src, w.ptr, w.ptr_lo, w.O, w.C, w.KH * w.KW, w.cpad}, dt, s)); break;
             case 1: KXC_TRY(stem_pack_weights(static_cast<const float*>(src), w.ptr, dt, w.O, w.C, w.KH, w.KW, s)); break;
             case 4: KXC_TRY(stem_direct_pack_weights(static_cast<const float*>(src), w.ptr, w.O, w.C, w.KH, w.KW, s)); break;
             case 5: KXC_TRY(stem_stacked_pack_weights(static_cast<const float*>(src), w.ptr, w.O, w.C, w.KW, s)); break;
             case 2: KXC_TRY(convert_rows(static_cast<const float*>(src), w.ptr, dt, w.O, w.C, w.cpad, s)); break;
-            case 3: KXC_TRY(nchw_to_nhwc(src, w.ptr, dt, 1, w.C, w.O, w.cpad, s)); break;
+            case 3: KXC_TRY(convert_operands(src, w.ptr, w.ptr_lo, dt, 1, w.C, w.O, w.cpad, nullptr, s, false)); break;
         }
         if (pl->x3) {
             switch (w.mode) {
-                case 0: KXC_TRY(pack_weights_ohwi(src, w.ptr_lo, dt, w.O, w.C, w.KH, w.KW, w.cpad, s, true)); break;
+                case 0: case 3: break;  // both parts at once, above
                 case 2: KXC_TRY(convert_rows(static_cast<const float*>(src), w.ptr_lo, dt, w.O, w.C, w.cpad, s, true)); break;
-                case 3: KXC_TRY(nchw_to_nhwc(src, w.ptr_lo, dt, 1, w.C, w.O, w.cpad, s, true)); break;
                 case 1: KXC_TRY(stem_pack_weights(static_cast<const float*>(src), w.ptr_lo, dt, w.O, w.C, w.KH, w.KW, s, true)); break;
                 default: return fail(KXC_B200_ERR_UNSUPPORTED, "plan: weight layout %d has no TF32X3 form", w.mode);
             }
@@ -1134,13 +1133,9 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
         ++step_index;
         switch (st.kind) {
             case SKind::InputNHWC:
-                if (pl->x3) {
-                    float* hi = static_cast<float*>(pl->storage(st.out));
-                    KXC_TRY(nchw_to_nhwc_split(static_cast<const float*>(arg_of(st.in0)), hi, hi + pl->find(st.out)->elems, st.N, st.C,
-                                               st.H * st.W, st.cpad, s));
-                } else {
-                    KXC_TRY(nchw_to_nhwc(arg_of(st.in0), pl->storage(st.out), dt, st.N, st.C, st.H * st.W, st.cpad, s, false, true));
-                }
+                KXC_TRY(convert_operands(arg_of(st.in0), pl->storage(st.out),
+                                         pl->x3 ? static_cast<float*>(pl->storage(st.out)) + pl->find(st.out)->elems : nullptr, dt, st.N, st.C,
+                                         st.H * st.W, st.cpad, nullptr, s, true));
                 break;
             case SKind::InputStem:
                 KXC_TRY(stem_pack(static_cast<const float*>(arg_of(st.in0)), pl->storage(st.out), dt, st.N, st.C, st.H, st.W, st.Hp,

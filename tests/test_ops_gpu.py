@@ -268,6 +268,29 @@ def test_conv2d_split_reduction(ops, rng, case, precision, rounder):
     assert min(max_abs, max_rel) <= bound, f"split conv {precision} {case}: {max_abs:.3e} {max_rel:.3e}"
 
 
+# The conversion of both operands in one launch: blocks of 32 and 64 channels, a last block of either kind that is partly there,
+# planes shorter than a block's pixels and of no multiple of them, odd channel counts (pairs), filters of 1, 9 and 49 taps, more
+# filters than one block of threads takes; in a captured graph the launch follows an allocation instead of a kernel.
+# Bounds: that of test_conv2d_tensor_core, and 1e-4 for three passes.
+@pytest.mark.parametrize("precision,rounder", [("tf32", port.round_tf32), ("bf16", port.round_bf16), ("tf32x3", None)])
+@pytest.mark.parametrize("case", [(1, 1, 1, 1, 1, 1), (3, 7, 5, 13, 300, 1), (2, 33, 9, 11, 40, 3), (2, 65, 8, 8, 24, 3), (1, 131, 6, 7, 20, 7)])
+def test_conv2d_operand_conversion(ops, rng, case, precision, rounder):
+    N, C, H, W, O, k = case
+    x, w, b = conv_inputs(rng, N, C, H, W, O, k, k)
+    args = [dev(v) for v in (x, w, b)]
+    got = host(ops.nn_conv2d(*args, padding=(k // 2, k // 2), precision=precision))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        again = ops.nn_conv2d(*args, padding=(k // 2, k // 2), precision=precision)
+    graph.replay()
+    assert_bit_exact(host(again), got, f"captured {precision} {case}")
+    del graph
+    assert ops.device_status() == 0
+    max_abs, max_rel = ref_metric(got, conv_expect(x, w, b, None, False, 1, k // 2, 1, rounder))
+    bound = 1e-4 if rounder is None else 2e-5 * max(1.0, np.sqrt(C * k * k) / 8)
+    assert min(max_abs, max_rel) <= bound, f"{precision} {case}: {max_abs:.3e} {max_rel:.3e}"
+
+
 # Tile boxes of results in the reference's layout, chosen by the runs of their stores: whole rows, rows wider than a tile, one
 # column, one pixel per image, several images per box; a residual read chunk by chunk ahead of the accumulator (32, 64 and more
 # channels, a last chunk that is partly there). Bound: that of test_conv2d_tensor_core.
