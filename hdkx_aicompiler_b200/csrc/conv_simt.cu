@@ -72,17 +72,20 @@ __global__ void __launch_bounds__(kThreads) conv2d_direct_kernel(const TIn* __re
 // is therefore formed as fma(x, w, -0) with a -0 that is a kernel argument (fma(x, w, -0) is the rounded product for every
 // x and w, the signs of zeros included), which nothing can fold.
 // Measured, 128 -> 128 channels 3x3 at 28x28 and 32 images: 646 us with scalar arithmetic, 275 us = 26.9 TFLOP/s now (0.74 of
-// the packed bound; 2.65 blocks for each SM cost 12 % of it); ResNet-18 at 32 images 11.3 -> 4.5 ms. Weights doubled in
-// shared memory to spare the register moves, unrolling two stages and rolling the k loop up were slower.
+// the packed bound at 1.965 GHz, but the pipe is busy for 97 % of the clocks on an SM that holds three blocks: the clock falls
+// to 1.63 GHz under it). ResNet-18 at 32 images 11.3 -> 4.4 ms. Weights doubled in shared memory or channels and pixels paired
+// crosswise to spare the register moves, unrolling two stages and rolling the k loop up gained nothing.
 //
 // Half of the warps compute, the other half feed them: the im2col values of KC consecutive k = (rc, rh, rw) by 4-byte
-// cp.async (zeros outside the image and past the last k: acc + 0 is the identity, acc is never -0) and the weights through
-// registers, into a ring of kExactBufs shared-memory stages handed over with named barriers. With the same warps doing both, the
+// cp.async (zeros outside the image and past the last k: acc + 0 is the identity, acc is never -0) and the weights, into a ring of
+// shared-memory stages handed over with named barriers. Filters of width 3 and 7 copy their weights in the same way and keep
+// the copies of kBufs - 2 stages in flight: small tiles alone on their SM were bound by one stage's way from L2
+// (512 -> 512 3x3 at 7x7, one image: 55 us, 51 with them, 37 on 16x16 tiles). The others, whose K is
+// short, take them through registers a stage ahead (4-byte copies there: 10 to 25 % slower). With the same warps doing both, the
 // gather's dependent address arithmetic held up the FMA pipe (175 clocks per k where the arithmetic alone takes 140 with
 // one warp on a scheduler); as separate warps it runs in the issue slots that the packed instructions leave. A stage is
 // whole filter rows (four of 3 taps, two of 7, sixteen of 1), so that a row's pointer and bounds are found once and a tap
 // costs a bit test and the copy; other widths find every tap in a table.
-constexpr int kExactBufs = 3;
 constexpr int kExactMaxTaps = 64; // the table's size
 
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
@@ -118,25 +121,45 @@ template <int kKW, int kMul>
 struct ExactStage {
     static constexpr int kRows = kMul * (kKW == 7 ? 2 : kKW == 3 ? 4 : 16);  // filter rows of a stage (kKW = 0: taps)
     static constexpr int kK = kRows * (kKW > 0 ? kKW : 1);
-    static constexpr int kVec = kK % 4 == 0 ? 4 : 2;                 // weights of one global load
+    // a warp copies the weights of kWK consecutive k of 32 / kWK channels: 8 to 32 bytes in a row on the global side, and rows
+    // of the stage that are 32 / kWK words longer than its channels spread them over all banks
+    static constexpr bool kAsync = kKW >= 3;
+    static constexpr int kWK = kK % 8 == 0 ? 8 : kK % 4 == 0 ? 4 : 2;
+    static constexpr int kWO = kAsync ? 32 / kWK : 0;
+    static constexpr int kVec = kK % 4 == 0 ? 4 : 2;  // through registers: weights of one global load
 };
 
-template <int kKW, int kTO, int kTP, int kOG, int kPG, int kMul, int kMinBlocks, typename Epilogue>
-__global__ void __launch_bounds__(2 * kOG * kPG, kMinBlocks)
+template <int kKW, int kTO, int kTP, int kOG, int kPG, int kMul, int kDeep>
+struct ExactSmem {
+    using Tile = ExactTile<kTO, kTP, kOG, kPG>;
+    using Stage = ExactStage<kKW, kMul>;
+    static constexpr int kBufs = Stage::kAsync ? kDeep : 3;
+    static constexpr int kWPitch = Tile::kO + Stage::kWO;
+    static constexpr int kXs = Stage::kK * Tile::kP, kWs = Stage::kK * kWPitch;  // words of a buffer
+    static constexpr int kBytes = kBufs * (kXs + kWs) * 4;
+};
+
+template <int kKW, int kTO, int kTP, int kOG, int kPG, int kMul, int kDeep, typename Epilogue>
+__global__ void __launch_bounds__(2 * kOG * kPG, 2)
     conv2d_tiled_f32_kernel(const float* __restrict__ data, const float* __restrict__ weight, ConvDims d, float neg_zero_arg,
                             Epilogue epi) {
     using Tile = ExactTile<kTO, kTP, kOG, kPG>;
     using Stage = ExactStage<kKW, kMul>;
-    constexpr int kT = Tile::kThreads, kTileO = Tile::kO, kTileP = Tile::kP, KC = Stage::kK, kVec = Stage::kVec;
+    using Smem = ExactSmem<kKW, kTO, kTP, kOG, kPG, kMul, kDeep>;
+    constexpr int kBufs = Smem::kBufs, kVec = Stage::kVec;
+    constexpr int kT = Tile::kThreads, kTileO = Tile::kO, kTileP = Tile::kP, KC = Stage::kK, kWPitch = Smem::kWPitch;
+    constexpr int kLag = kBufs - 2;  // stages whose copies are in flight behind the one that is handed over
     // threads that share the gather of one pixel, and the filter rows each takes of a stage
     constexpr int kShare = kT / kTileP > 1 ? kT / kTileP : 1;
     constexpr int kSub = kShare < Stage::kRows ? kShare : Stage::kRows;
     constexpr int kRowsPer = Stage::kRows / kSub;
-    constexpr int kWQ = kTileO * (KC / kVec);  // weight loads of a stage
-    constexpr int kWPer = (kWQ + kT - 1) / kT;
-    static_assert(kTO % 2 == 0 && kTP % 2 == 0 && kTileP <= kT && Stage::kRows % kSub == 0, "tile shape");
-    __shared__ __align__(16) float xs[kExactBufs][KC][kTileP];
-    __shared__ __align__(16) float ws[kExactBufs][KC][kTileO];
+    constexpr int kWLoads = kTileO * KC / (Stage::kAsync ? 1 : kVec);  // weight copies (loads) of a stage
+    constexpr int kWPer = (kWLoads + kT - 1) / kT;
+    static_assert(kTO % 2 == 0 && kTP % 2 == 0 && kTileP <= kT && Stage::kRows % kSub == 0 && kTileO % 8 == 0, "tile shape");
+    static_assert(kBufs >= 3 && 2 * kBufs < 16, "ring: two named barriers a buffer");
+    extern __shared__ __align__(16) float exact_smem[];
+    float* const xs = exact_smem;                     // [kBufs][KC][kTileP]
+    float* const ws = exact_smem + kBufs * Smem::kXs;  // [kBufs][KC][kWPitch]
     __shared__ int tap_off[kKW > 0 ? 1 : kExactMaxTaps];
 
     const int K = d.C * d.KH * d.KW;
@@ -195,7 +218,7 @@ __global__ void __launch_bounds__(2 * kOG * kPG, kMinBlocks)
         ih = ih0 + gt * d.DH;
     };
     if (kSub > 1) advance(gsub * kRowsPer);
-    const uint32_t gdst0 = (uint32_t)__cvta_generic_to_shared(&xs[0][gsub * kRowsPer * (kKW > 0 ? kKW : 1)][gp]);
+    const uint32_t gdst0 = (uint32_t)__cvta_generic_to_shared(xs + gsub * kRowsPer * (kKW > 0 ? kKW : 1) * kTileP + gp);
 
     // row i (of kRowsPer) of the next stage into buffer `buf`; afterwards the state stands at the following row
     auto gather_row = [&](int buf, int i) {
@@ -214,61 +237,90 @@ __global__ void __launch_bounds__(2 * kOG * kPG, kMinBlocks)
         --left;
         if (kSub > 1 && i == kRowsPer - 1) advance(Stage::kRows - kRowsPer);
     };
-    // weight role: up to kWPer loads of kVec consecutive k of one channel; consecutive threads take consecutive channels
-    const bool w_vec = K % kVec == 0 && (reinterpret_cast<uintptr_t>(weight) & (kVec * 4 - 1)) == 0;
-    float wreg[kWPer][kVec];
-    auto load_weights = [&](int k0) {
+    int buf = 0;
+    auto hand_over = [&](int s) {  // stage s - kLag has landed
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (s >= kLag) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kLag) : "memory");
+            named_arrive(1 + (buf >= kLag ? buf - kLag : buf - kLag + kBufs), 2 * kT);
+        }
+        buf = buf + 1 == kBufs ? 0 : buf + 1;
+    };
+    if constexpr (Stage::kAsync) {
+        // weights: a warp copies blocks of kWK consecutive k of kWO channels; the pointers advance by a stage at a time
+        const float* wsrc[kWPer];
+        uint32_t wdst[kWPer];
+        int wleft[kWPer];  // k up to the end of K; 0: no such channel
 #pragma unroll
         for (int i = 0; i < kWPer; ++i) {
-            const int q = tid + i * kT;
-            const int o = o0 + q % kTileO, k = k0 + (q / kTileO) * kVec;
-#pragma unroll
-            for (int v = 0; v < kVec; ++v) wreg[i][v] = 0.0f;
-            if (o < d.O && k < K && (kWQ % kT == 0 || q < kWQ)) {
-                const float* src = weight + (int64_t)o * K + k;
-                if (w_vec && kVec == 4) {
-                    const float4 v = __ldg(reinterpret_cast<const float4*>(src));
-                    wreg[i][0] = v.x; wreg[i][1] = v.y; wreg[i][kVec - 2] = v.z; wreg[i][kVec - 1] = v.w;
-                } else if (w_vec) {
-                    const float2 v = __ldg(reinterpret_cast<const float2*>(src));
-                    wreg[i][0] = v.x; wreg[i][1] = v.y;
-                } else {
-#pragma unroll
-                    for (int v = 0; v < kVec; ++v)
-                        if (k + v < K) wreg[i][v] = __ldg(src + v);
-                }
-            }
+            const int block = tid / 32 + i * (kT / 32), l = tid & 31;
+            const int k = block % (KC / Stage::kWK) * Stage::kWK + l % Stage::kWK;
+            const int o = block / (KC / Stage::kWK) * Stage::kWO + l / Stage::kWK;
+            const bool there = o < kTileO && o0 + o < d.O;
+            wsrc[i] = there ? weight + (int64_t)(o0 + o) * K + k : weight;
+            wdst[i] = (uint32_t)__cvta_generic_to_shared(ws + k * kWPitch + o);
+            wleft[i] = there ? K - k : 0;
         }
-    };
-    auto store_weights = [&](int buf) {
-#pragma unroll
-        for (int i = 0; i < kWPer; ++i) {
-            const int q = tid + i * kT;
-            if (kWQ % kT != 0 && q >= kWQ) break;
-            float* dst = &ws[buf][(q / kTileO) * kVec][q % kTileO];
-#pragma unroll
-            for (int v = 0; v < kVec; ++v) dst[v * kTileO] = wreg[i][v];
-        }
-    };
-
-        load_weights(0);
-        int buf = 0;
         for (int s = 0; s < stages; ++s) {
-            if (s >= kExactBufs) named_sync(1 + kExactBufs + buf, 2 * kT);  // the stage three back has been read
+            if (s >= kBufs) named_sync(1 + kBufs + buf, 2 * kT);  // the stage that lay here has been read
+#pragma unroll
+            for (int i = 0; i < kWPer; ++i) {
+                const bool in_tile = kWLoads % kT == 0 || tid + i * kT < kWLoads;
+                cp_async4_zfill(wdst[i] + (uint32_t)(buf * Smem::kWs * 4), wsrc[i], wleft[i] > 0 ? 1u : 0u, in_tile);
+                wsrc[i] += wleft[i] > 0 ? KC : 0;
+                wleft[i] -= KC;
+            }
 #pragma unroll
             for (int i = 0; i < kRowsPer; ++i) gather_row(buf, i);
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            store_weights(buf);
-            load_weights((s + 1) * KC);
-            if (s > 0) {  // the previous stage has landed
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-                named_arrive(1 + (buf == 0 ? kExactBufs - 1 : buf - 1), 2 * kT);
-            }
-            buf = buf + 1 == kExactBufs ? 0 : buf + 1;
+            hand_over(s);
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        named_arrive(1 + (buf == 0 ? kExactBufs - 1 : buf - 1), 2 * kT);
-        return;
+    } else {
+        // through registers: up to kWPer loads of kVec consecutive k of one channel; consecutive threads take consecutive channels
+        const bool w_vec = K % kVec == 0 && (reinterpret_cast<uintptr_t>(weight) & (kVec * 4 - 1)) == 0;
+        float wreg[kWPer][kVec];
+        auto load_weights = [&](int k0) {
+#pragma unroll
+            for (int i = 0; i < kWPer; ++i) {
+                const int q = tid + i * kT;
+                const int o = o0 + q % kTileO, k = k0 + (q / kTileO) * kVec;
+#pragma unroll
+                for (int v = 0; v < kVec; ++v) wreg[i][v] = 0.0f;
+                if (o < d.O && k < K && (kWLoads % kT == 0 || q < kWLoads)) {
+                    const float* src = weight + (int64_t)o * K + k;
+                    if (w_vec && kVec == 4) {
+                        const float4 v = __ldg(reinterpret_cast<const float4*>(src));
+                        wreg[i][0] = v.x; wreg[i][1] = v.y; wreg[i][kVec - 2] = v.z; wreg[i][kVec - 1] = v.w;
+                    } else if (w_vec) {
+                        const float2 v = __ldg(reinterpret_cast<const float2*>(src));
+                        wreg[i][0] = v.x; wreg[i][1] = v.y;
+                    } else {
+#pragma unroll
+                        for (int v = 0; v < kVec; ++v)
+                            if (k + v < K) wreg[i][v] = __ldg(src + v);
+                    }
+                }
+            }
+        };
+        load_weights(0);
+        for (int s = 0; s < stages; ++s) {
+            if (s >= kBufs) named_sync(1 + kBufs + buf, 2 * kT);
+#pragma unroll
+            for (int i = 0; i < kRowsPer; ++i) gather_row(buf, i);
+#pragma unroll
+            for (int i = 0; i < kWPer; ++i) {
+                const int q = tid + i * kT;
+                if (kWLoads % kT != 0 && q >= kWLoads) break;
+                float* dst = ws + (buf * KC + (q / kTileO) * kVec) * kWPitch + q % kTileO;
+#pragma unroll
+                for (int v = 0; v < kVec; ++v) dst[v * kWPitch] = wreg[i][v];
+            }
+            load_weights((s + 1) * KC);
+            hand_over(s);
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    for (int s = stages > kLag ? stages - kLag : 0; s < stages; ++s) named_arrive(1 + s % kBufs, 2 * kT);
+    return;
     }
 
     const int pg = tid % kPG, og = tid / kPG;
@@ -287,21 +339,21 @@ __global__ void __launch_bounds__(2 * kOG * kPG, kMinBlocks)
             // the thread's pixels: groups of four consecutive ones kPG * 4 apart, then (kTP % 4 == 2) one pair
 #pragma unroll
             for (int e = 0; e < kTP / 4; ++e) {
-                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&xs[buf][k][e * kPG * 4 + pg * 4]);
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(xs + (buf * KC + k) * kTileP + e * kPG * 4 + pg * 4);
                 x[2 * e] = v.x;
                 x[2 * e + 1] = v.y;
             }
-            if constexpr (kTP % 4 != 0) x[kTP / 2 - 1] = *reinterpret_cast<const uint64_t*>(&xs[buf][k][(kTP / 4) * kPG * 4 + pg * 2]);
+            if constexpr (kTP % 4 != 0) x[kTP / 2 - 1] = *reinterpret_cast<const uint64_t*>(xs + (buf * KC + k) * kTileP + (kTP / 4) * kPG * 4 + pg * 2);
 #pragma unroll
             for (int j = 0; j < kTO / 4; ++j) {
-                const float4 v = *reinterpret_cast<const float4*>(&ws[buf][k][og * kTO + 4 * j]);
+                const float4 v = *reinterpret_cast<const float4*>(ws + (buf * KC + k) * kWPitch + og * kTO + 4 * j);
                 w[4 * j] = pack2(v.x, v.x);
                 w[4 * j + 1] = pack2(v.y, v.y);
                 w[4 * j + 2] = pack2(v.z, v.z);
                 w[4 * j + 3] = pack2(v.w, v.w);
             }
             if constexpr (kTO % 4 != 0) {
-                const float2 v = *reinterpret_cast<const float2*>(&ws[buf][k][og * kTO + kTO - 2]);
+                const float2 v = *reinterpret_cast<const float2*>(ws + (buf * KC + k) * kWPitch + og * kTO + kTO - 2);
                 w[kTO - 2] = pack2(v.x, v.x);
                 w[kTO - 1] = pack2(v.y, v.y);
             }
@@ -310,8 +362,8 @@ __global__ void __launch_bounds__(2 * kOG * kPG, kMinBlocks)
 #pragma unroll
                 for (int e = 0; e < kTP / 2; ++e) acc[j][e] = mac2_exact(acc[j][e], x[e], w[j], neg_zero);
         }
-        if (s + kExactBufs < stages) named_arrive(1 + kExactBufs + buf, 2 * kT);
-        buf = buf + 1 == kExactBufs ? 0 : buf + 1;
+        if (s + kBufs < stages) named_arrive(1 + kBufs + buf, 2 * kT);
+        buf = buf + 1 == kBufs ? 0 : buf + 1;
     }
 
     // Four consecutive pixels of one image are one 16-byte access where planes and pointers allow it. A pixel's place is found once
@@ -444,24 +496,27 @@ int grid_for(int64_t items) {
 
 // Tile of the packed kernel. The sum over k is one chain per output and cannot be split, so a launch's parallelism is its
 // outputs: large tiles for large launches, smaller ones where they would leave SMs idle. The estimate is the number of
-// blocks on the busiest SM times the clocks a block takes there per k, as measured on the convolutions of ResNet-18 at 1, 8
-// and 32 images (`alone`: a single block on its SM, latencies showing; `shared`: per block when there are several).
-//   tile (channels x pixels)    64x128   64x96   32x64   16x32
-//   FMA-pipe bound                 128      96      32       8
-//   alone / shared             157/150 126/120   59/45   31/20.5
+// blocks on the busiest SM times the clocks a block takes there per k (`alone`: a single block on its SM, latencies showing;
+// `shared`: per block when there are several). Filters of width 3 and 7: fits over 156 convolutions of 1 to 64 images timed
+// with every tile, 4 to 7 % off (10 % at 16x16); what they choose is 0.1 % behind the fastest tile on average and 1.08 times as
+// fast as the best of the first four tiles. The others, where the epilogue weighs as much as the sum: as measured on ResNet-18.
+//   tile (channels x pixels)    64x128   64x96  32x64  16x32  16x16  32x96  32x32  32x128
+//   FMA-pipe bound                 128      96     32      8      4     48     16      64
 struct ExactCost {
     int tile_o, tile_p;
     double alone, shared;
 };
-constexpr ExactCost kExactCosts[] = {
-    {64, 128, 157.0, 150.0}, {64, 96, 126.0, 120.0}, {32, 64, 59.0, 45.0}, {16, 32, 31.0, 20.5}};
+constexpr ExactCost kExactCosts[] = {{64, 128, 157.0, 150.0}, {64, 96, 126.0, 120.0}, {32, 64, 59.0, 45.0}, {16, 32, 31.0, 20.5}};
+constexpr ExactCost kExactWideCosts[] = {{64, 128, 162.8, 153.6}, {64, 96, 127.2, 120.0}, {32, 64, 49.2, 46.4}, {16, 32, 21.7, 18.4},
+                                         {16, 16, 14.8, 11.8},    {32, 96, 71.2, 67.2},   {32, 32, 32.1, 27.2}, {32, 128, 88.2, 83.2}};
 
-int pick_exact_tile(const ConvDims& d) {
+template <int kCount>
+int pick_exact_tile(const ConvDims& d, const ExactCost (&costs)[kCount]) {
     const int64_t P = (int64_t)d.N * d.OH * d.OW;
     int best = 0;
     double best_cost = 0.0;
-    for (int i = 0; i < 4; ++i) {
-        const ExactCost& c = kExactCosts[i];
+    for (int i = 0; i < kCount; ++i) {
+        const ExactCost& c = costs[i];
         const int64_t blocks = ((P + c.tile_p - 1) / c.tile_p) * ((d.O + c.tile_o - 1) / c.tile_o);
         const int64_t per_sm = (blocks + kNumSMs - 1) / kNumSMs;
         const double cost = per_sm <= 1 ? c.alone : (double)per_sm * c.shared;
@@ -473,17 +528,35 @@ int pick_exact_tile(const ConvDims& d) {
     return best;
 }
 
-template <int kTO, int kTP, int kMul, int kMinBlocks>
-void launch_exact_tile(const float* data, const float* weight, const ConvDims& d, const EpilogueF32& epi, cudaStream_t s) {
-    using Tile = ExactTile<kTO, kTP, 8, 16>;
+template <int kKW, int kTO, int kTP, int kOG, int kPG, int kMul, int kDeep>
+int32_t launch_exact(const float* data, const float* weight, const ConvDims& d, const EpilogueF32& epi, cudaStream_t s) {
+    using Tile = ExactTile<kTO, kTP, kOG, kPG>;
+    constexpr int kBytes = ExactSmem<kKW, kTO, kTP, kOG, kPG, kMul, kDeep>::kBytes;
+    auto kernel = conv2d_tiled_f32_kernel<kKW, kTO, kTP, kOG, kPG, kMul, kDeep, EpilogueF32>;
+    static PerDeviceOnce smem_once;
+    KXC_TRY(smem_opt_in(smem_once, kernel, kBytes));
     const int64_t P = (int64_t)d.N * d.OH * d.OW;
     const dim3 grid((unsigned)((P + Tile::kP - 1) / Tile::kP), (unsigned)((d.O + Tile::kO - 1) / Tile::kO), 1u);
-    auto go = [&](auto kernel) { kernel<<<grid, 2 * Tile::kThreads, 0, s>>>(data, weight, d, -0.0f, epi); };
-    switch (d.DW == 1 ? d.KW : 0) {
-        case 1: go(conv2d_tiled_f32_kernel<1, kTO, kTP, 8, 16, kMul, kMinBlocks, EpilogueF32>); break;
-        case 3: go(conv2d_tiled_f32_kernel<3, kTO, kTP, 8, 16, kMul, kMinBlocks, EpilogueF32>); break;
-        case 7: go(conv2d_tiled_f32_kernel<7, kTO, kTP, 8, 16, kMul, kMinBlocks, EpilogueF32>); break;
-        default: go(conv2d_tiled_f32_kernel<0, kTO, kTP, 8, 16, kMul, kMinBlocks, EpilogueF32>); break;
+    kernel<<<grid, 2 * Tile::kThreads, kBytes, s>>>(data, weight, d, -0.0f, epi);
+    return check_launch("nn_conv2d (fp32, tiled)");
+}
+
+template <int kKW>
+int32_t launch_exact_width(const float* data, const float* weight, const ConvDims& d, const EpilogueF32& epi, cudaStream_t s) {
+    if constexpr (kKW >= 3) {
+        switch (pick_exact_tile(d, kExactWideCosts)) {
+            case 4: return launch_exact<kKW, 2, 2, 8, 8, 4, 5>(data, weight, d, epi, s);
+            case 5: return launch_exact<kKW, 4, 6, 8, 16, 1, 4>(data, weight, d, epi, s);
+            case 6: return launch_exact<kKW, 4, 2, 8, 16, 2, 5>(data, weight, d, epi, s);
+            case 7: return launch_exact<kKW, 4, 8, 8, 16, 1, 4>(data, weight, d, epi, s);
+            default: break;
+        }
+    }
+    switch (kKW >= 3 ? pick_exact_tile(d, kExactWideCosts) : pick_exact_tile(d, kExactCosts)) {
+        case 0: return launch_exact<kKW, 8, 8, 8, 16, 1, 3>(data, weight, d, epi, s);
+        case 1: return launch_exact<kKW, 8, 6, 8, 16, 1, 3>(data, weight, d, epi, s);
+        case 2: return launch_exact<kKW, 4, 4, 8, 16, 2, 5>(data, weight, d, epi, s);
+        default: return launch_exact<kKW, 2, 2, 8, 16, 4, 5>(data, weight, d, epi, s);
     }
 }
 
@@ -496,13 +569,12 @@ bool tiled_f32_ok(const ConvDims& d) {
 }
 
 int32_t launch_tiled_f32(const float* data, const float* weight, const ConvDims& d, const EpilogueF32& epi, cudaStream_t s) {
-    switch (pick_exact_tile(d)) {
-        case 0: launch_exact_tile<8, 8, 1, 2>(data, weight, d, epi, s); break;
-        case 1: launch_exact_tile<8, 6, 1, 2>(data, weight, d, epi, s); break;
-        case 2: launch_exact_tile<4, 4, 2, 4>(data, weight, d, epi, s); break;
-        default: launch_exact_tile<2, 2, 4, 4>(data, weight, d, epi, s); break;
+    switch (d.DW == 1 ? d.KW : 0) {
+        case 1: return launch_exact_width<1>(data, weight, d, epi, s);
+        case 3: return launch_exact_width<3>(data, weight, d, epi, s);
+        case 7: return launch_exact_width<7>(data, weight, d, epi, s);
+        default: return launch_exact_width<0>(data, weight, d, epi, s);
     }
-    return check_launch("nn_conv2d (fp32, tiled)");
 }
 
 }  // namespace

@@ -191,6 +191,17 @@ def test_conv2d_fp32_tiles_bit_exact(ops, rng, case):
     assert_bit_exact(got, conv_expect(x, w, b, res, True, s, p, d), f"conv fp32 {case}")
 
 
+# its tiles for filters of width 3 and 7 only (16x16, 32x32, 32x96, 32x128): fewer stages than the ring holds, reductions that end
+# inside a stage, channels beyond the last
+@pytest.mark.parametrize("case", [
+    (1, 5, 6, 7, 17, 3, 3, 2, 1, 1), (1, 61, 6, 7, 17, 3, 3, 1, 1, 1), (1, 3, 9, 5, 20, 7, 7, 1, 3, 1), (2, 5, 28, 43, 17, 3, 3, 1, 1, 1),
+    (4, 3, 18, 34, 18, 7, 7, 1, 3, 1), (2, 7, 50, 48, 33, 3, 3, 1, 1, 1), (3, 2, 33, 48, 33, 7, 7, 1, 3, 1), (4, 7, 50, 36, 33, 3, 3, 1, 1, 1),
+    (3, 2, 46, 53, 35, 7, 7, 1, 3, 1),
+])
+def test_conv2d_fp32_wide_filter_tiles_bit_exact(ops, rng, case):
+    test_conv2d_fp32_tiles_bit_exact(ops, rng, case)
+
+
 @pytest.mark.parametrize("precision,tol,rounder", [("tf32", 1e-3, port.round_tf32), ("bf16", 1e-2, port.round_bf16)])
 @pytest.mark.parametrize("case", CONV_CASES)
 def test_conv2d_tensor_core(ops, rng, case, precision, tol, rounder):
