@@ -1,5 +1,7 @@
-// 3x3 / stride-1 / pad-1 convolution for 128 -> 128 channel layers (bf16 NHWC): the row-stacked form of
-// conv_rowstack.cu on CTA pairs, with the weights resident in shared memory.
+// 3x3 / stride-1 / pad-1 convolution for 128 -> 128 channel layers (bf16 NHWC) and 64 -> 64 channel layers (tf32 NHWC): the
+// row-stacked form of conv_rowstack.cu on CTA pairs, with the weights resident in shared memory. 64 tf32 and 128 bf16 channels are
+// the same 256 bytes per pixel, so both share everything up to the accumulator; what follows is about the bf16 layers, the tf32
+// ones differ as said at the end.
 //
 // The general implicit-GEMM kernel reads every input pixel nine times (one box per filter tap) and the weights once per
 // work item: at 128 channels that is ~440 KB of L2 -> shared-memory traffic per 128-pixel tile, and the measured fill
@@ -21,6 +23,13 @@
 // warps 2..17 epilogue with TMA-loaded residual boxes and TMA-stored output boxes of 64 channels); pair protocol as in
 // conv_tc.cu (loads of both CTAs count on the leader's barriers, commits arrive on both CTAs' barriers, the peer's epilogue
 // warps release accumulators on the leader's barrier). Every wait is bounded. No multicast loads.
+//
+// tf32, 64 -> 64: the 192 stacked rows are all output channels, so pairs are not halved and a halo is fetched once: ~46 KB per
+// 112-pixel tile and 24 instructions, against 360 KB (nine boxes and the weights of two tiles) and 72 in the general kernel, which
+// was bound by the tiles' way into shared memory. Results are 256 bytes per pixel: each group of four epilogue warps owns a box
+// of 32 channels (128-byte rows), and residual boxes come in a ring of three such planes. ResNet-18 layer 1, per launch without /
+// with residual, us: one image 6.9 / 7.6 -> 6.0 / 6.1, 4: 10.8 / 12.3 -> 7.4 / 7.6, 32: 32.8 / 34.6 -> 19.8 / 21.2, 256: 204 / 207 -> 150 / 134
+// (5 us per tile pair at 32 images: ~320 KB through shared memory per tile, as much a clock as the bf16 forms reach).
 #include "conv_rowstack.cuh"
 
 #include <mutex>
@@ -43,26 +52,34 @@ constexpr int kEpiWarps = 8;
 constexpr int kCh = 64 / (kEpiWarps / 4);
 constexpr int kEpiThreads = kEpiWarps * 32;
 constexpr int kThreads = 64 + kEpiThreads;
-constexpr int kC = 128;               // input channels: two planes of 64 (128-byte rows)
-constexpr int kO = 128;               // output channels, in two halves of kOH
-constexpr int kOH = 64;
-constexpr int kBN = 3 * kOH;          // MMA N: the three filter rows of one half side by side
+constexpr int kOH = 64;               // output channels of a work item
+constexpr int kBN = 3 * kOH;          // MMA N: their three filter rows side by side
 constexpr int kTileW = 8;
 constexpr int kRows = 16;
 constexpr int kOutRows = kRows - 2;
 constexpr int kHaloW = kTileW + 2;
-constexpr int kPlaneBytes = kHaloW * kRows * 128;   // 20480: one 64-channel plane of a halo
+constexpr int kPlaneBytes = kHaloW * kRows * 128;   // 20480: one plane (128 bytes per pixel) of a halo
 constexpr int kHaloBytes = 2 * kPlaneBytes;         // 40960
 constexpr int kBRows = kBN / 2;                     // 96 stacked weight rows per CTA
 constexpr int kWBlockBytes = kBRows * 128;          // 12288: one (tap column, plane) block of this CTA's rows
 constexpr int kWeightBytes = 3 * 2 * kWBlockBytes;  // 73728
 constexpr int kStages = 2;
 constexpr int kAccStride = 256;
-constexpr int kBoxBytes = kTileW * kOutRows * 128;  // 14336: 8 x 14 pixels x 64 channels
-constexpr int kResBufs = 2;
-constexpr int kOutBufs = 2;
-constexpr int kSmemBytes = kWeightBytes + kStages * kHaloBytes + (kResBufs + kOutBufs) * kBoxBytes + 1024;
-static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
+constexpr int kBoxBytes = kTileW * kOutRows * 128;  // 14336: 8 x 14 pixels x 64 channels (tf32: 32)
+
+template <bool kF32>
+struct Geom {
+    static constexpr int kC = kF32 ? 64 : 128;       // input channels: two planes
+    static constexpr int kPlaneC = kC / 2;
+    static constexpr int kHalves = kF32 ? 1 : 2;
+    static constexpr int kO = kHalves * kOH;         // output channels
+    static constexpr int kBoxC = kF32 ? 32 : 64;     // channels of a residual or output box
+    static constexpr int kResBufs = kF32 ? 3 : 2;    // boxes
+    static constexpr int kOutBufs = 2;               // boxes (tf32: one per group of warps)
+    static constexpr int kResWarps = kF32 ? 4 : kEpiWarps;  // warps that read a residual box
+    static constexpr int kSmemBytes = kWeightBytes + kStages * kHaloBytes + (kResBufs + kOutBufs) * kBoxBytes + 1024;
+    static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
+};
 
 template <int kN>
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&v)[kN]) {
@@ -71,9 +88,12 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&v)[kN]) 
     else tmem_ld_32x16(taddr, v);
 }
 
+template <bool kF32>
 __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const __grid_constant__ TcParams p) {
+    using G = Geom<kF32>;
+    constexpr int kC = G::kC, kPlaneC = G::kPlaneC, kResBufs = G::kResBufs, kOutBufs = G::kOutBufs;
     constexpr uint32_t kTmemCols = 2 * kAccStride;
-    constexpr uint32_t kIdesc = make_instr_desc(kFmtBF16, kAccF32, kBN, 256u);
+    constexpr uint32_t kIdesc = make_instr_desc(kF32 ? kFmtTF32 : kFmtBF16, kAccF32, kBN, 256u);
 
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bar_w;
@@ -90,8 +110,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
     const int lane = threadIdx.x & 31;
     const uint32_t w_smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t halo_smem = w_smem + kWeightBytes;
-    const uint32_t res_smem = halo_smem + kStages * kHaloBytes;
-    const uint32_t out_smem = res_smem + kResBufs * kBoxBytes;
+    const uint32_t out_smem = halo_smem + kStages * kHaloBytes;
+    const uint32_t res_smem = out_smem + kOutBufs * kBoxBytes;
     const bool has_res = p.residual != nullptr;
     const uint32_t cta_rank = cluster_cta_rank();
     const bool leader = cta_rank == 0;
@@ -109,7 +129,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
         }
         for (int b = 0; b < kResBufs; ++b) {
             mbar_init(smem_u32(&bar_res_full[b]), 1);
-            mbar_init(smem_u32(&bar_res_empty[b]), kEpiWarps);
+            mbar_init(smem_u32(&bar_res_empty[b]), G::kResWarps);
         }
         mbar_fence_init();
     }
@@ -125,14 +145,15 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
     volatile int* abort_ptr = &abort_flag;
     pdl_launch_dependents();
 
-    // Work split: pair q of Q (Q even) works on channel half q & 1 and on the tile pairs q/2, q/2 + Q/2, ...; CTA `rank`
-    // of the pair takes tile 2 * tile_pair + rank. A tile index beyond the last tile loads zeros and stores nothing.
+    // Work split: pair q of Q (Q even) works on channel half q & 1 and on the tile pairs q/2, q/2 + Q/2, ... (tf32: there is one
+    // half, tile pairs q, q + Q, ...); CTA `rank` of the pair takes tile 2 * tile_pair + rank. A tile index beyond the last tile
+    // loads zeros and stores nothing.
     const int total_tiles = p.tiles_w * p.tiles_h * p.tiles_n;
     const int tile_pairs = (total_tiles + 1) >> 1;
     const int pair_id = (int)(blockIdx.x >> 1);
-    const int half = pair_id & 1;
-    const int first_tp = pair_id >> 1;
-    const int tp_step = (int)(gridDim.x >> 2);
+    const int half = kF32 ? 0 : pair_id & 1;
+    const int first_tp = pair_id / G::kHalves;
+    const int tp_step = (int)(gridDim.x / (2 * G::kHalves));
 
     if (warp == 0) {
         if (lane == 0) {
@@ -149,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
                         const int s0 = (int)cta_rank * kBRows + 32 * j;  // first stacked row of the box
                         const int r = s0 / kOH, co0 = s0 % kOH;
                         tma_load_2d_pair(w_smem + (uint32_t)((kw * 2 + pl) * kWBlockBytes + 32 * j * 128), &p.tmB, wbar,
-                                         (r * 3 + kw) * kC + pl * 64, half * kOH + co0);
+                                         (r * 3 + kw) * kC + pl * kPlaneC, half * kOH + co0);
                     }
             pdl_wait();  // the weights are constants; the activations come from the previous kernel
             int stage = 0, rb = 0;
@@ -166,14 +187,18 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
                 const uint32_t dst = halo_smem + (uint32_t)(stage * kHaloBytes);
                 // tensor map dimensions: channel, ROW, column, image
                 tma_load_4d_pair(dst, &p.tmA[0], full0, 0, th * kOutRows - 1, tw * kTileW - 1, tn);
-                tma_load_4d_pair(dst + kPlaneBytes, &p.tmA[0], full0, 64, th * kOutRows - 1, tw * kTileW - 1, tn);
+                tma_load_4d_pair(dst + kPlaneBytes, &p.tmA[0], full0, kPlaneC, th * kOutRows - 1, tw * kTileW - 1, tn);
                 if (++stage == kStages) { stage = 0; phase ^= 1u; }
-                if (has_res) {  // this CTA's own residual box (its own barrier)
-                    if (!mbar_wait_bounded(smem_u32(&bar_res_empty[rb]), rphase ^ 1u, abort_ptr)) break;
+                bool ok = true;
+                for (int g = 0; ok && has_res && g < kOH / G::kBoxC; ++g) {  // this CTA's own residual boxes (its own barriers)
+                    ok = mbar_wait_bounded(smem_u32(&bar_res_empty[rb]), rphase ^ 1u, abort_ptr);
+                    if (!ok) break;
                     mbar_arrive_expect_tx(smem_u32(&bar_res_full[rb]), kBoxBytes);
-                    tma_load_4d(res_smem + rb * kBoxBytes, &p.tmA[1], smem_u32(&bar_res_full[rb]), half * kOH, th * kOutRows, tw * kTileW, tn);
+                    tma_load_4d(res_smem + rb * kBoxBytes, &p.tmA[1], smem_u32(&bar_res_full[rb]), half * kOH + g * G::kBoxC, th * kOutRows,
+                                tw * kTileW, tn);
                     if (++rb == kResBufs) { rb = 0; rphase ^= 1u; }
                 }
+                if (!ok) break;
             }
         }
     } else if (warp == 1) {
@@ -197,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
                     for (int k = 0; k < 8; ++k) {
                         const uint32_t a_lo = a_lo0 + (uint32_t)(((k >> 2) * kPlaneBytes + kw * (kRows * 128) + (k & 3) * 32) >> 4);
                         const uint32_t b_lo = b_lo0 + (uint32_t)(((kw * 2 + (k >> 2)) * kWBlockBytes + (k & 3) * 32) >> 4);
-                        umma_f16_split_pair(d, a_lo, hi, b_lo, hi, kIdesc, (kw | k) != 0 ? 1u : 0u);
+                        umma_split_pair<kF32 ? MmaKind::TF32 : MmaKind::F16>(d, a_lo, hi, b_lo, hi, kIdesc, (kw | k) != 0 ? 1u : 0u);
                     }
                 }
                 umma_commit_pair(smem_u32(&bar_empty[stage]), 3);
@@ -212,7 +237,10 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
         const int c0 = ((warp - 2) >> 2) * kCh;  // channels [c0, c0 + kCh) of the pair's half
         const int h_l = lane & 15;              // accumulator row = input row of the tile
         const int w_l = 2 * quad + (lane >> 4);
-        const bool issuer = threadIdx.x == 64;  // the epilogue thread that owns the TMA stores' async groups
+        // the epilogue thread that owns the TMA stores' async groups, its barriers and their threads (tf32: of each group of warps)
+        const int group = kF32 ? (warp - 2) >> 2 : 0;
+        constexpr int kStoreThreads = kF32 ? kEpiThreads / 2 : kEpiThreads;
+        const bool issuer = threadIdx.x == 64 + group * kStoreThreads;
         const bool in_box = (h_l >= 1) && (h_l <= kOutRows);
         const uint32_t box_row = (uint32_t)(w_l * kOutRows + (h_l - 1));
         const uint32_t row_off = box_row * 128u;
@@ -223,7 +251,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
 #pragma unroll
         for (int j = 0; j < kCh; ++j) bias[j] = p.bias != nullptr ? __ldg(p.bias + half * kOH + c0 + j) : 0.0f;
         pdl_wait();
-        int acc = 0, rb = 0, ob = 0;
+        int acc = 0, rb = group, ob = group;
         uint32_t acc_phase = 0, rphase = 0;
         for (int tp = first_tp; tp < tile_pairs; tp += tp_step) {
             int r = 2 * tp + (int)cta_rank;
@@ -255,6 +283,15 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
                 if (!bad) {
                     if (in_box) {
                         const uint32_t base = res_smem + rb * kBoxBytes + row_off;
+                        if constexpr (kF32) {
+#pragma unroll
+                            for (int g = 0; g < 8; ++g) {
+                                const uint4 rv = ld_shared_v4(base + (((uint32_t)g ^ sw) << 4));
+                                const uint32_t w[4] = {rv.x, rv.y, rv.z, rv.w};
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) f[4 * g + k] = __fadd_rn(f[4 * g + k], __uint_as_float(w[k]));
+                            }
+                        } else
 #pragma unroll
                         for (int g = 0; g < kCh / 8; ++g) {
                             const uint4 rv = ld_shared_v4(base + ((((uint32_t)((c0 >> 3) + g)) ^ sw) << 4));
@@ -268,18 +305,31 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
                     }
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&bar_res_empty[rb]));
-                    if (++rb == kResBufs) { rb = 0; rphase ^= 1u; }
+                    rb += G::kO / G::kHalves / G::kBoxC;
+                    if (rb >= kResBufs) { rb -= kResBufs; rphase ^= 1u; }
                 }
             }
             if (p.relu) {
 #pragma unroll
                 for (int j = 0; j < kCh; ++j) f[j] = f[j] > 0.0f ? f[j] : 0.0f;
             }
-            // the output box used two tiles ago must have been read by its TMA store before it is overwritten
-            if (issuer) bulk_wait_group_read<kOutBufs - 1>();
-            if (named_barrier_or(1, kEpiThreads, bad)) break;
+            if constexpr (kF32) {
+                if (p.round_out_tf32) {
+#pragma unroll
+                    for (int j = 0; j < kCh; ++j) f[j] = tf32_rne(f[j]);
+                }
+            }
+            // the output box must have been read by its TMA store, of two tiles (tf32: one) ago, before it is overwritten
+            if (issuer) bulk_wait_group_read<kF32 ? 0 : kOutBufs - 1>();
+            if (named_barrier_or(1 + 2 * group, kStoreThreads, bad)) break;
             if (in_box) {
                 const uint32_t base = out_smem + ob * kBoxBytes + row_off;
+                if constexpr (kF32) {
+#pragma unroll
+                    for (int g = 0; g < 8; ++g)
+                        st_shared_v4(base + (((uint32_t)g ^ sw) << 4), make_uint4(__float_as_uint(f[4 * g]), __float_as_uint(f[4 * g + 1]),
+                                                                                  __float_as_uint(f[4 * g + 2]), __float_as_uint(f[4 * g + 3])));
+                } else
 #pragma unroll
                 for (int g = 0; g < kCh / 8; ++g) {
                     uint4 o;
@@ -291,12 +341,13 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
                 }
             }
             fence_proxy_async_shared();
-            named_barrier(2, kEpiThreads);
+            named_barrier(2 + 2 * group, kStoreThreads);
             if (issuer) {  // pixels beyond the image's last row or column are clipped by the store
-                if (n < p.N) tma_store_4d(&p.tmA[2], out_smem + ob * kBoxBytes, half * kOH, th * kOutRows, tw * kTileW, n);
+                if (n < p.N)
+                    tma_store_4d(&p.tmA[2], out_smem + ob * kBoxBytes, half * kOH + group * G::kBoxC, th * kOutRows, tw * kTileW, n);
                 bulk_commit_group();  // (an empty group for the missing second tile keeps the group count in step)
             }
-            ob ^= 1;
+            if constexpr (!kF32) ob ^= 1;  // (two boxes per group where there is no residual: no change)
             acc ^= 1;
             if (acc == 0) acc_phase ^= 1u;
         }
@@ -321,56 +372,61 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
 }  // namespace
 
 bool rowstack128_applicable(TcDType dtype, int C, int O, int KH, int KW, int stride, int pad_h, int pad_w, int dil_h, int dil_w) {
-    return dtype == kTcBF16 && C == kC && O == kO && KH == 3 && KW == 3 && stride == 1 && pad_h == 1 && pad_w == 1 && dil_h == 1 &&
-           dil_w == 1;
+    const int ch = dtype == kTcBF16 ? Geom<false>::kC : dtype == kTcTF32 ? Geom<true>::kC : 0;
+    return ch != 0 && C == ch && O == ch && KH == 3 && KW == 3 && stride == 1 && pad_h == 1 && pad_w == 1 && dil_h == 1 && dil_w == 1;
 }
 
-int32_t rowstack128_setup(TcParams* p, const void* act_nhwc, const void* w_packed, int N, int H, int W) {
-    p->N = N; p->OH = H; p->OW = W; p->Cout = kO;
+int32_t rowstack128_setup(TcParams* p, TcDType dtype, const void* act_nhwc, const void* w_packed, int N, int H, int W) {
+    const int ch = dtype == kTcBF16 ? Geom<false>::kC : Geom<true>::kC, eb = tc_elem_bytes(dtype);
+    p->N = N; p->OH = H; p->OW = W; p->Cout = ch;
     p->taps_h = 3; p->taps_w = 3; p->stride = 1; p->pad_h = 1; p->pad_w = 1; p->dil_h = 1; p->dil_w = 1;
-    p->cblocks = 2; p->kb_elems = 64;
+    p->cblocks = 2; p->kb_elems = 128 / eb;
     p->BW = kTileW; p->BH = kOutRows; p->BNI = 1;
     p->tiles_w = (W + kTileW - 1) / kTileW;
     p->tiles_h = (H + kOutRows - 1) / kOutRows;
     p->tiles_n = N;
-    p->tiles_c = 2;
-    const uint64_t px = kC * 2;
-    // dimensions: channel, ROW, column, image -> a box lands in shared memory as [column][row][64 channels]
-    const uint64_t dims[4] = {(uint64_t)kC, (uint64_t)H, (uint64_t)W, (uint64_t)N};
+    p->tiles_c = ch / kOH;
+    const uint64_t px = (uint64_t)ch * eb;
+    // dimensions: channel, ROW, column, image -> a box lands in shared memory as [column][row][128 bytes of channels]
+    const uint64_t dims[4] = {(uint64_t)ch, (uint64_t)H, (uint64_t)W, (uint64_t)N};
     const uint64_t strides[3] = {(uint64_t)W * px, px, (uint64_t)H * W * px};
-    const uint32_t box[4] = {64u, (uint32_t)kRows, (uint32_t)kHaloW, 1u};
-    KXC_TRY(tc_make_tmap(&p->tmA[0], kTcBF16, 4, const_cast<void*>(act_nhwc), dims, strides, box, 128));
+    const uint32_t box[4] = {(uint32_t)p->kb_elems, (uint32_t)kRows, (uint32_t)kHaloW, 1u};
+    KXC_TRY(tc_make_tmap(&p->tmA[0], dtype, 4, const_cast<void*>(act_nhwc), dims, strides, box, 128));
     for (int i = 1; i < 4; ++i) p->tmA[i] = p->tmA[0];
-    const uint64_t ktot = (uint64_t)9 * kC;
-    const uint64_t bdims[2] = {ktot, (uint64_t)kO};
-    const uint64_t bstr[1] = {ktot * 2};
-    const uint32_t bbox[2] = {64u, 32u};
-    KXC_TRY(tc_make_tmap(&p->tmB, kTcBF16, 2, const_cast<void*>(w_packed), bdims, bstr, bbox, 128));
+    const uint64_t ktot = (uint64_t)9 * ch;
+    const uint64_t bdims[2] = {ktot, (uint64_t)ch};
+    const uint64_t bstr[1] = {ktot * eb};
+    const uint32_t bbox[2] = {(uint32_t)p->kb_elems, 32u};
+    KXC_TRY(tc_make_tmap(&p->tmB, dtype, 2, const_cast<void*>(w_packed), bdims, bstr, bbox, 128));
     KXC_TRY(tc_status_word(&p->status));
     return KXC_B200_OK;
 }
 
-int32_t rowstack128_bind(TcParams* p) {
-    // tmA[1]: residual boxes (loads), tmA[2]: output boxes (stores): 8 x 14 pixels x 64 channels of the 128
+int32_t rowstack128_bind(TcParams* p, TcDType dtype) {
+    // tmA[1]: residual boxes (loads), tmA[2]: output boxes (stores): 8 x 14 pixels x 128 bytes, half of the channels
     if (p->out == nullptr) return fail(KXC_B200_ERR_INVALID, "row-stacked 128-channel conv: no output tensor");
-    const uint64_t px = kO * 2;
-    const uint64_t dims[4] = {(uint64_t)kO, (uint64_t)p->OH, (uint64_t)p->OW, (uint64_t)p->N};
+    const uint64_t px = (uint64_t)p->Cout * tc_elem_bytes(dtype);
+    const uint64_t dims[4] = {(uint64_t)p->Cout, (uint64_t)p->OH, (uint64_t)p->OW, (uint64_t)p->N};
     const uint64_t strides[3] = {(uint64_t)p->OW * px, px, (uint64_t)p->OH * p->OW * px};
-    const uint32_t box[4] = {(uint32_t)kOH, (uint32_t)kOutRows, (uint32_t)kTileW, 1u};
-    KXC_TRY(tc_make_tmap(&p->tmA[2], kTcBF16, 4, p->out, dims, strides, box, 128));
+    const uint32_t box[4] = {(uint32_t)(128 / tc_elem_bytes(dtype)), (uint32_t)kOutRows, (uint32_t)kTileW, 1u};
+    KXC_TRY(tc_make_tmap(&p->tmA[2], dtype, 4, p->out, dims, strides, box, 128));
     if (p->residual != nullptr)
-        KXC_TRY(tc_make_tmap(&p->tmA[1], kTcBF16, 4, const_cast<void*>(p->residual), dims, strides, box, 128));
+        KXC_TRY(tc_make_tmap(&p->tmA[1], dtype, 4, const_cast<void*>(p->residual), dims, strides, box, 128));
     return KXC_B200_OK;
 }
 
-int32_t rowstack128_launch(const TcParams& p, cudaStream_t stream) {
+namespace {
+template <bool kF32>
+int32_t launch(const TcParams& p, cudaStream_t stream) {
+    using G = Geom<kF32>;
+    constexpr int kSmemBytes = G::kSmemBytes;
     static PerDeviceOnce smem_once;
     static std::mutex units_mu;
     static int max_pairs[PerDeviceOnce::kMaxDevices] = {0};  // per device: clusters of two resident at once
     int dev = 0;
-    auto kernel = conv3x3_rowstack128_kernel;
+    auto kernel = conv3x3_rowstack128_kernel<kF32>;
     KXC_TRY(smem_opt_in(smem_once, kernel, kSmemBytes, &dev));
-    if (!p.vec_ok || p.out == nullptr) return fail(KXC_B200_ERR_INVALID, "row-stacked 128-channel conv: pointers must be 16-byte aligned");
+    if ((!kF32 && !p.vec_ok) || p.out == nullptr) return fail(KXC_B200_ERR_INVALID, "row-stacked 128-channel conv: pointers must be 16-byte aligned");
     const long long tiles = (long long)p.tiles_w * p.tiles_h * p.tiles_n;
     if (tiles <= 0) return KXC_B200_OK;
     int pairs;
@@ -397,9 +453,14 @@ int32_t rowstack128_launch(const TcParams& p, cudaStream_t stream) {
         pairs = max_pairs[dev];
     }
     const long long tile_pairs = (tiles + 1) / 2;
-    if (2 * tile_pairs < pairs) pairs = (int)(2 * tile_pairs);
+    if (G::kHalves * tile_pairs < pairs) pairs = (int)(G::kHalves * tile_pairs);
     KXC_CUDA_TRY(launch_kernel(kernel, dim3(2 * pairs), dim3(kThreads), kSmemBytes, stream, /*pdl=*/true, 2, p));
     return check_launch("conv3x3_rowstack128_kernel");
+}
+}  // namespace
+
+int32_t rowstack128_launch(TcDType dtype, const TcParams& p, cudaStream_t stream) {
+    return dtype == kTcTF32 ? launch<true>(p, stream) : launch<false>(p, stream);
 }
 
 }  // namespace kxc_b200

@@ -325,16 +325,17 @@ void bind_x3(kxc_b200_plan* pl, Step& st) {
 
 }  // namespace
 
-// The 128 -> 128 channel 3x3 layers: the row-stacked CTA-pair kernel with resident weights or the implicit-GEMM kernel.
-// Measured per launch at 28 x 28 (ms, row-stacked against implicit GEMM): without a residual 0.191 / 0.215 at 1024 images
-// and 0.033 / 0.037 at 128; with a residual 0.235 / 0.227 at 1024, 0.127 / 0.121-0.125 at 512, 0.067-0.068 / 0.070-0.072
-// at 256 and 0.037-0.039 / 0.040-0.041 at 128. So: always without a residual, with one up to 256 images of 28 x 28. KXC_B200_ROWSTACK128 = 0: never, 2: always (A/B runs); read at every
-// plan build.
-static bool rowstack128_wanted(bool has_residual, long long pixels) {
+// The 128 -> 128 (bf16) and 64 -> 64 (tf32) channel 3x3 layers: the row-stacked CTA-pair kernel with resident weights or the
+// implicit-GEMM kernel. bf16, measured per launch at 28 x 28 (ms, row-stacked against implicit GEMM): without a residual 0.191 / 0.215
+// at 1024 images and 0.033 / 0.037 at 128; with a residual 0.235 / 0.227 at 1024, 0.127 / 0.121-0.125 at 512, 0.067-0.068 /
+// 0.070-0.072 at 256 and 0.037-0.039 / 0.040-0.041 at 128. So: always without a residual, with one up to 256 images of 28 x 28.
+// tf32: always (figures at the kernel, 1 to 256 images of 56 x 56). KXC_B200_ROWSTACK128 = 0: never, 2: always (A/B runs); read
+// at every plan build.
+static bool rowstack128_wanted(TcDType dtype, bool has_residual, long long pixels) {
     const char* e = getenv("KXC_B200_ROWSTACK128");
     if (e != nullptr && e[0] == '0') return false;
     if (e != nullptr && e[0] == '2') return true;
-    return !has_residual || pixels <= 256ll * 28 * 28;
+    return dtype == kTcTF32 || !has_residual || pixels <= 256ll * 28 * 28;
 }
 
 static int32_t finalize_exact(kxc_b200_plan* pl);
@@ -971,12 +972,12 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
                     st.direct = 3;
                     KXC_TRY(rowstack3x3_setup(&st.params, pl->storage(st.in0), pw.ptr, st.N, st.H, st.W));
                     st.cfg = TcConfig{dt, 128, 64, om};
-                } else if (rowstack128_wanted(st.in1 >= 0, (long long)st.N * st.H * st.W) && !st.out_is_graph_output && !pl->x3 &&
+                } else if (rowstack128_wanted(dt, st.in1 >= 0, (long long)st.N * st.H * st.W) && !st.out_is_graph_output && !pl->x3 &&
                            st.weight2 < 0 &&
                            rowstack128_applicable(dt, st.C, pw.O, pw.KH, pw.KW, st.pool.strides[0], st.pad_h, st.pad_w,
                                                   st.pool.pool_size[0], st.pool.pool_size[1])) {
                     st.direct = 5;
-                    KXC_TRY(rowstack128_setup(&st.params, pl->storage(st.in0), pw.ptr, st.N, st.H, st.W));
+                    KXC_TRY(rowstack128_setup(&st.params, dt, pl->storage(st.in0), pw.ptr, st.N, st.H, st.W));
                     st.cfg = TcConfig{dt, 128, 192, om};
                     st.cfg.ctas = 2;
                 } else if (direct_mode > 0 && !st.out_is_graph_output &&
@@ -1003,7 +1004,7 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
             st.params.out = st.out_is_graph_output ? nullptr : pl->storage(st.out);
             if (pl->x3) bind_x3(pl, st);
             if (st.direct == 3) KXC_TRY(rowstack3x3_bind(&st.params));
-            if (st.direct == 5) KXC_TRY(rowstack128_bind(&st.params));
+            if (st.direct == 5) KXC_TRY(rowstack128_bind(&st.params, dt));
             if (st.direct == 0 && pw.mode == 0 && !st.out_is_graph_output) KXC_TRY(tc_bind_store(&st.params, st.cfg));
             (void)ov;
         } else if (st.kind == SKind::Gemm) {
@@ -1159,7 +1160,7 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
                 } else if (st.direct == 3) {
                     KXC_TRY(rowstack3x3_launch(p, s));
                 } else if (st.direct == 5) {
-                    KXC_TRY(rowstack128_launch(p, s));
+                    KXC_TRY(rowstack128_launch(dt, p, s));
                 } else if (st.direct == 1) {
                     KXC_TRY(direct3x3_launch(p, s));
                 } else {
@@ -1318,7 +1319,7 @@ extern "C" int32_t kxc_b200_plan_launch_info(kxc_b200_plan* pl, int32_t index, c
                                                 : ((w.mode == 1 || w.mode == 4) ? (double)st.N * st.Hp * st.Wp * 4 * eb : (double)st.N * st.H * st.W * st.cpad * eb);
             by = in_bytes + (double)w.bytes + out_elems * (st.fused_pool ? 0.25 : 1.0) * (st.out_is_graph_output ? 4.0 : eb) +
                  (st.in1 >= 0 ? out_elems * eb : 0.0) + 4.0 * w.O;
-            snprintf(buf, sizeof(buf), "%s c%d h%d w%d -> o%d k%dx%d s%d%s%s tile %dx%dx%d bn%d%s", st.direct == 4 ? "conv_stem_pool_nchw" : st.direct == 2 ? (st.fused_pool ? "conv_stem_pool" : "conv_stem_direct") : (st.direct == 3 ? "conv_rowstack" : (st.direct == 5 ? "conv_rowstack128" : (st.direct ? "conv_direct" : "conv_igemm"))), w.C, st.H, st.W, w.O, w.KH, w.KW,
+            snprintf(buf, sizeof(buf), "%s c%d h%d w%d -> o%d k%dx%d s%d%s%s tile %dx%dx%d bn%d%s", st.direct == 4 ? "conv_stem_pool_nchw" : st.direct == 2 ? (st.fused_pool ? "conv_stem_pool" : "conv_stem_direct") : (st.direct == 3 ? "conv_rowstack" : (st.direct == 5 ? (pl->dtype == kTcTF32 ? "conv_rowstack_tf32" : "conv_rowstack128") : (st.direct ? "conv_direct" : "conv_igemm"))), w.C, st.H, st.W, w.O, w.KH, w.KW,
                      p.stride, st.in1 >= 0 ? " +res" : "", st.relu ? " +relu" : "", p.BNI, p.BH, p.BW, st.cfg.bn,
                      st.cfg.ctas == 2 ? " pair" : (st.weight2 >= 0 ? " +1x1 second output" : (st.cfg.mt == 2 ? " x2 tiles" : "")));
             if (p.split > 1) snprintf(buf + strlen(buf), sizeof(buf) - strlen(buf), " split%d", p.split);

@@ -444,6 +444,41 @@ def test_128_channel_3x3_kernels_agree(kxc, monkeypatch, n, h, w):
     assert float(np.abs(outs["rowstack128"] - outs["igemm"]).max()) <= 2e-2 * scale
 
 
+# The tf32 form, 64 -> 64 channels: the same three layers at the same kinds of sizes (one tile, an odd number of them, ragged rows and
+# columns, several work items per pair, so that the ring of residual planes wraps). Bound: the test above's five roundings of an
+# activation, at 2^-11 each.
+@pytest.mark.parametrize("n,h,w", [(2, 28, 28), (3, 30, 20), (1, 7, 5), (3, 14, 8), (1, 15, 9), (50, 30, 28)])
+def test_64_channel_tf32_kernels_agree(kxc, monkeypatch, n, h, w):
+    R = kxc.relay
+    rng = np.random.default_rng(7)
+    x = rng.uniform(-1, 1, (n, 64, h, w)).astype(f32)
+    ws = [rng.normal(0, (2 / 576) ** 0.5, (64, 64, 3, 3)).astype(f32) for _ in range(3)]
+    bs = [rng.normal(0, 0.1, (64,)).astype(f32) for _ in range(3)]
+
+    def build(to):
+        xv = R.Var("input", x.shape)
+        conv = lambda d, i: R.Call("nn_conv2d", [d, R.Constant(to(ws[i])), R.Constant(to(bs[i]))],
+                                   R.Conv2DAttrs((1, 1), (1, 1, 1, 1), (1, 1), 1))
+        y0 = R.Call("nn_relu", [conv(xv, 0)])
+        y1 = R.Call("nn_relu", [conv(y0, 1)])
+        return R.Function([xv], R.Call("nn_relu", [R.Call("nn_relu", [R.Call("add", [conv(y1, 2), y0])])]))
+
+    outs = {}
+    for name, flag in (("rowstack", "2"), ("igemm", "0")):
+        monkeypatch.setenv("KXC_B200_ROWSTACK128", flag)
+        outs[name], g = run_plan(kxc, build(cuda_const), x, "tf32")
+        kinds = [l[0].split()[0] for l in g.launch_info()]
+        assert kinds.count("conv_rowstack_tf32") == (3 if flag == "2" else 0)
+    from hdkx_aicompiler_b200 import ops
+    assert ops.device_status() == 0
+    bound = 5 * 2.0 ** -11
+    if n <= 3:
+        emu = ograph.run(build(lambda a: a), [x], operand_round=port.round_tf32, workers=4)
+        for name, got in outs.items():
+            assert float(np.abs(got - emu).max()) <= bound * float(np.abs(emu).max()), name
+    assert float(np.abs(outs["rowstack"] - outs["igemm"]).max()) <= bound * float(np.abs(outs["igemm"]).max())
+
+
 @pytest.mark.parametrize("precision", ["bf16", "tf32"])
 def test_resnet18_stem_plan(kxc, precision):
     """The packed-stem path alone (7x7 stride-2 convolution over 3 channels + bias + relu): against the oracle on
