@@ -1,14 +1,15 @@
 // 7x7 stride-2 "stem" convolution + bias + ReLU + max_pool2d(3x3, stride 2, pad 1) in ONE kernel that reads the
 // graph input as the reference hands it over (NCHW fp32, include/te/topi/nn.h:107-158 / :161-229) and writes the
-// pooled bf16 NHWC activation: neither a packed copy of the input nor the convolution's output touches HBM.
+// pooled NHWC activation (bf16, or fp32 holding tf32 values): neither a packed copy of the input nor the convolution's output
+// touches HBM.
 //
 // Work split of a CTA (22 warps), all roles running concurrently on a ring of input strips:
-//   warp 0        loads the 28 KiB of weights once (bulk copy)
-//   warps 18..21  converters: bring the fp32 rows of a strip (three channel planes) into shared memory with cp.async,
-//                 one strip ahead, round to bf16 and write the packed layout [row][pixel][4 channels] (8 bytes per
-//                 pixel, zero border) that the tensor core reads
+//   warp 0        loads the 28 KiB (tf32: 56) of weights once (bulk copy)
+//   warps 10..13  converters: bring the fp32 rows of a strip (three channel planes) into shared memory with cp.async,
+//                 one strip ahead, round to the operand type and write the packed layout [row][pixel][4 channels] (8 bytes
+//                 per pixel, zero border) that the tensor core reads
 //   warp 1        issues tcgen05.mma, owns TMEM
-//   warps 2..17   epilogue: accumulator -> +bias -> bf16 -> running 3x3 maximum -> ReLU -> store
+//   warps 2..9    epilogue: accumulator -> +bias -> (bf16) -> running 3x3 maximum -> ReLU -> store
 //
 // MMA formulation. In the packed layout the K vector of output pixel (oh, ow) for filter row r is the 8 pixels x 4
 // channels starting at packed pixel (2*oh + r, 2*ow): with the unswizzled K-major operand layout (rows 16 bytes
@@ -29,6 +30,18 @@
 // neighbour in another warp comes through a 64-byte shared-memory slot and a 128-thread barrier). Rounding to bf16
 // is monotonic and keeps the sign, so max-then-ReLU on rounded values equals the reference's ReLU-then-fold
 // `m = (m > v) ? m : v` (NaN -> 0, -0 -> +0 included): 0 is a neutral element and one final max with 0 is the ReLU.
+//
+// tf32. A pixel is 16 bytes, so consecutive output columns (two pixels) are 32 bytes apart and the rows of a core matrix, which lie
+// 16 bytes apart, cannot be every second pixel. The even and the odd pixels of a row therefore lie in two planes: one K step
+// (eight tf32 values) is the pixel pair (2j, 2j + 1) = entry i + j of either plane, the distance of the planes being the
+// operand's leading byte offset. Four K steps per filter row instead of two, 46 instructions per three output rows; strips of two
+// pooled rows, which is what shared memory holds. The order of the sums is that of the implicit-GEMM kernel over the packed
+// input, which this replaces together with the packing and the pooling kernel, and so are the bits. ResNet-18 tf32, the three
+// launches / this one, us: 4 images 28.6 / 18.3, 32: 119 / 54, 256: 826 / 307 (64 % of the clocks are instructions; their operands'
+// way out of shared memory).
+//
+// bf16 strips have four pooled rows; two where that leaves no SM a second strip (up to five images of 224 x 224), whose time is
+// then one strip's latency: 13.1 -> 9.6 us.
 // Every wait is bounded (sm100::mbar_wait_bounded); a wait that runs out is reported through the status word.
 #include "conv_stem.cuh"
 
@@ -48,31 +61,38 @@ constexpr int kEpilogueWarp0 = 2, kEpilogueWarps = 4 * (64 / kPartCols);
 constexpr int kThreads = (2 + kEpilogueWarps + 4) * 32;  // loader, MMA issuer, epilogue warps, 4 converter warps
 constexpr int kBN = 64;             // output channels
 constexpr int kKH = 7;
-constexpr int kPooledRows = 4;      // pooled rows per strip
-constexpr int kConvRows = 2 * kPooledRows + 1;             // 9: conv rows 8s-1 .. 8s+7 (the first one recomputed)
-constexpr int kInRows = 2 * (kConvRows - 1) + kKH;         // 23 packed input rows
-constexpr int kMaxRowBytes = 2048;
-constexpr int kStripBytes = ((kInRows * kMaxRowBytes + 4096 + 1023) / 1024) * 1024;  // + slack for the M = 128 over-read
-constexpr int kStages = 2;          // packed strips in shared memory (the tensor core reads one while the next is written)
-constexpr int kEvenRows = 4 * kBN, kOddRows = 3 * kBN;     // stacked filter rows: r = 6,4,2,0 and r = 5,3,1
-constexpr int kWeightBytes = 4 * (kEvenRows + kOddRows) * 16;  // 4 K chunks of 8 elements per filter row: 28672
 constexpr int kBlockRows = 3;       // output rows per accumulator buffer
 constexpr int kBufCols = 256;       // TMEM columns per buffer (3 slots of 64 used)
-constexpr int kMaxEntries = 24;     // MMA instructions of a three-row block
-constexpr int kExchBytes = 2 * (64 / kPartCols) * 4 * kPartCols * 2;  // [parity][channel part][quadrant] x one column's channels of the part
 constexpr int kConverterWarp0 = kEpilogueWarp0 + kEpilogueWarps, kConverterThreads = 128;
-// fp32 staging of ONE strip, filled by cp.async: every converter thread owns the 16-byte slots of its own 4-pixel items
-// ([item][channel][thread]), so no thread ever waits for another one's copies
+constexpr int kStages = 2;          // packed strips in shared memory (the tensor core reads one while the next is written)
+constexpr int kEvenRows = 4 * kBN, kOddRows = 3 * kBN;     // stacked filter rows: r = 6,4,2,0 and r = 5,3,1
 constexpr int kMaxC = 3;
-constexpr int kMaxRowItems = kMaxRowBytes / 32;                                                        // 4-pixel items per row
-constexpr int kItemsPerThread = (kInRows * 56 + kConverterThreads - 1) / kConverterThreads;            // 11 for 224-pixel rows
-constexpr int kStagingBytes = kItemsPerThread * kMaxC * kConverterThreads * 16;                          // 67584
-constexpr int kSmemBytes = kWeightBytes + kStages * kStripBytes + kExchBytes + kStagingBytes + 1024;
+
+template <bool kF32, int kPooled>
+struct StemGeom {
+    static constexpr int kConvRows = 2 * kPooled + 1;             // conv rows 2 kPooled s - 1 ... (the first one recomputed)
+    static constexpr int kInRows = 2 * (kConvRows - 1) + kKH;     // packed input rows
+    static constexpr int kMaxWidth = kF32 ? 224 : 244;
+    static constexpr int kMaxRowBytes = kF32 ? 232 * 16 : 2048;
+    // + slack for what the M = 128 rows read past the last row's end
+    static constexpr int kStripBytes = ((kInRows * kMaxRowBytes + (kF32 ? 1024 : 4096) + 1023) / 1024) * 1024;
+    static constexpr int kSteps = kF32 ? 4 : 2;                   // K steps (32 bytes) of a filter row
+    static constexpr int kWeightBytes = 2 * kSteps * (kEvenRows + kOddRows) * 16;
+    static constexpr int kExchBytes = 2 * (64 / kPartCols) * 4 * kPartCols * (kF32 ? 4 : 2);  // [parity][channel part][quadrant] x one column's channels of the part
+    // fp32 staging of ONE strip, filled by cp.async: every converter thread owns the 16-byte slots of its own 4-pixel items
+    // ([item][channel][thread]), so no thread ever waits for another one's copies
+    static constexpr int kItemsPerThread = (kInRows * (kMaxWidth / 4) + kConverterThreads - 1) / kConverterThreads;  // 11, 8, 7
+    static constexpr int kStagingBytes = kItemsPerThread * kMaxC * kConverterThreads * 16;
+    static constexpr int kBiasBytes = kBN * 4;
+    static constexpr int kSmemBytes = kWeightBytes + kStages * kStripBytes + kExchBytes + kStagingBytes + kBiasBytes + 1024;
+    static_assert(kSmemBytes <= 227 * 1024 - 256, "shared memory of one CTA");
+};
 
 // The instruction list of a block of R output rows (see the file comment), built at compile time so that the issue
 // loop is straight-line code with immediate operands: a single thread can then issue an MMA every ~25 cycles. (A loop
 // that fetches its operands from a table costs ~140 cycles per instruction in the one issuing thread, twice what the
 // tensor core needs for the instruction itself.)
+constexpr int kMaxEntries = 48;     // MMA instructions of a three-row block (24 for bf16)
 struct MmaEntry {
     int t, cp;        // packed input row relative to the block's first one; which pair of K chunks
     uint32_t b_rel;   // low descriptor word of the stacked weights, relative to the weights' base address
@@ -82,7 +102,7 @@ struct MmaTable {
     MmaEntry e[kMaxEntries];
     int len;
 };
-__host__ __device__ constexpr MmaTable make_mma_table(int R) {
+__host__ __device__ constexpr MmaTable make_mma_table(int R, int steps) {
     MmaTable tb{};
     int n = 0;
     for (int t = 0; t <= 2 * (R - 1) + (kKH - 1); ++t) {
@@ -93,8 +113,8 @@ __host__ __device__ constexpr MmaTable make_mma_table(int R) {
         const int q = odd ? (kKH - 2 - r_first) / 2 : (kKH - 1 - r_first) / 2;
         const int cnt = jmax - jmin + 1;
         const uint32_t lbo = (uint32_t)(odd ? kOddRows : kEvenRows) * 16u;
-        const uint32_t wbase = (odd ? 4u * kEvenRows * 16u : 0u) + (uint32_t)q * kBN * 16u;
-        for (int cp = 0; cp < 2; ++cp) {
+        const uint32_t wbase = (odd ? 2u * (uint32_t)steps * kEvenRows * 16u : 0u) + (uint32_t)q * kBN * 16u;
+        for (int cp = 0; cp < steps; ++cp) {
             const uint32_t b_addr = wbase + (uint32_t)cp * 2u * lbo;
             const uint32_t lbo_field = (lbo >> 4) << 16;
             const bool first_touch = cp == 0 && !odd && t == 2 * jmax;  // slot jmax receives filter row 0 here
@@ -110,30 +130,31 @@ __host__ __device__ constexpr MmaTable make_mma_table(int R) {
     return tb;
 }
 
-template <int kAcc>
-__device__ __forceinline__ void umma_f16_imm(uint32_t d_tmem, uint32_t a_lo, uint32_t hi, uint32_t b_lo, uint32_t idesc) {
+template <bool kF32, int kAcc>
+__device__ __forceinline__ void umma_imm(uint32_t d_tmem, uint32_t a_lo, uint32_t hi, uint32_t b_lo, uint32_t idesc) {
     // both descriptors share the upper word (unswizzled, 8-row groups 128 B apart); the accumulate flag is an immediate
-    if constexpr (kAcc != 0) {
+    if constexpr (kF32) {
         asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.eq.u32 p, 1, 1;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %2};\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem), "r"(a_lo), "r"(hi), "r"(b_lo), "r"(idesc)
+            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.eq.u32 p, 1, %5;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %2};\n\t"
+            "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem), "r"(a_lo), "r"(hi), "r"(b_lo), "r"(idesc), "n"(kAcc)
             : "memory");
     } else {
         asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.eq.u32 p, 1, 0;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %2};\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem), "r"(a_lo), "r"(hi), "r"(b_lo), "r"(idesc)
+            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.eq.u32 p, 1, %5;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %2};\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem), "r"(a_lo), "r"(hi), "r"(b_lo), "r"(idesc), "n"(kAcc)
             : "memory");
     }
 }
 
-template <int R, int I = 0>
+template <bool kF32, int R, int I = 0>
 __device__ __forceinline__ void issue_block(uint32_t d0, uint32_t a_lo0, uint32_t row16, uint32_t hi, uint32_t w_lo) {
-    constexpr MmaTable tb = make_mma_table(R);
+    constexpr MmaTable tb = make_mma_table(R, kF32 ? 4 : 2);
     if constexpr (I < tb.len) {
         constexpr MmaEntry e = tb.e[I];
-        constexpr uint32_t idesc = make_instr_desc(kFmtBF16, kAccF32, (uint32_t)e.n);
-        umma_f16_imm<e.acc>(d0 + (uint32_t)e.d_off, a_lo0 + (uint32_t)e.t * row16 + (uint32_t)(e.cp * 2), hi, w_lo + e.b_rel, idesc);
-        issue_block<R, I + 1>(d0, a_lo0, row16, hi, w_lo);
+        constexpr uint32_t idesc = make_instr_desc(kF32 ? kFmtTF32 : kFmtBF16, kAccF32, (uint32_t)e.n);
+        // a K step further: four bf16 pixels in a row, or the next entry of both planes
+        umma_imm<kF32, e.acc>(d0 + (uint32_t)e.d_off, a_lo0 + (uint32_t)e.t * row16 + (uint32_t)(e.cp * (kF32 ? 1 : 2)), hi, w_lo + e.b_rel, idesc);
+        issue_block<kF32, R, I + 1>(d0, a_lo0, row16, hi, w_lo);
     }
 }
 
@@ -159,7 +180,10 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uin
                  : "memory");
 }
 
+template <bool kF32, int kPooledRows>
 __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_nchw_kernel(const __grid_constant__ TcParams p) {
+    using G = StemGeom<kF32, kPooledRows>;
+    constexpr int kConvRows = G::kConvRows, kStripBytes = G::kStripBytes, kWeightBytes = G::kWeightBytes, kItemsPerThread = G::kItemsPerThread;
     constexpr uint32_t kTmemCols = 2 * kBufCols;
 
     extern __shared__ uint8_t smem_raw[];
@@ -176,9 +200,10 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_nchw_kernel(const 
     const uint32_t w_smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t strip_smem = w_smem + kWeightBytes;
     const uint32_t exch_smem = strip_smem + kStages * kStripBytes;
-    const uint32_t staging_smem = exch_smem + kExchBytes;
+    const uint32_t staging_smem = exch_smem + G::kExchBytes;
+    [[maybe_unused]] const uint32_t bias_smem = staging_smem + G::kStagingBytes;  // tf32: the epilogue's registers are taken
 
-    const int row_bytes = p.aux_row_bytes;  // packed row: Wp * 8
+    const int row_bytes = p.aux_row_bytes;  // packed row: Wp pixels
     const int Hp = p.aux_hp;
     const int H = p.aux_h, W = p.aux_w_px, C = p.aux_c;
     const int strips_per_image = p.OH / (2 * kPooledRows);
@@ -207,6 +232,12 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_nchw_kernel(const 
         const uint32_t addr = strip_smem + i * 16;
         asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0u) : "memory");
     }
+    if constexpr (kF32) {
+        if (threadIdx.x < kBN) {
+            const float b = p.bias != nullptr ? __ldg(p.bias + threadIdx.x) : 0.0f;
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(bias_smem + threadIdx.x * 4u), "f"(b) : "memory");
+        }
+    }
     fence_proxy_async_shared();
     tc_fence_before_sync();
     __syncthreads();
@@ -215,8 +246,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_nchw_kernel(const 
     volatile int* abort_ptr = &abort_flag;
     pdl_launch_dependents();
 
-    // Strip s of an image: conv rows 8s-1 .. 8s+7 (local j = 0..8; j = 0 is skipped for s = 0, it is the pool's padding
-    // row), packed input rows from max(16s - 2, 0); blocks of up to three conv rows.
+    // Strip s of an image, four pooled rows: conv rows 8s-1 .. 8s+7 (local j = 0..8; j = 0 is skipped for s = 0, it is the pool's
+    // padding row), packed input rows from max(16s - 2, 0); blocks of up to three conv rows.
     if (warp == 0) {
         if (lane == 0) {
             mbar_arrive_expect_tx(smem_u32(&bar_w), (uint32_t)kWeightBytes);
@@ -248,7 +279,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_nchw_kernel(const 
             // the others are padding rows (zeros)
             const int n = strip / strips_per_image;
             const int s = strip - n * strips_per_image;
-            const int row0 = s > 0 ? 16 * s - 2 : 0;
+            const int row0 = s > 0 ? 4 * kPooledRows * s - 2 : 0;
             int rows_in = (s > 0 ? 2 * (kConvRows - 1) : 2 * (kConvRows - 2)) + kKH;
             if (row0 + rows_in > Hp) rows_in = Hp - row0;
             const int h0 = row0 - p.pad_h;  // image row of local row 0
@@ -293,7 +324,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_nchw_kernel(const 
             if (next < total_strips) strip_geom(next, &base2, &row_lo2, &row_hi2);
             // warp-uniform outcome: no lane may leave while the others go on to the __syncwarp below
             if (!__all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_ptr))) break;
-            const uint32_t dst0 = strip_smem + (uint32_t)stage * kStripBytes + (uint32_t)p.pad_w * 8u;
+            const uint32_t dst0 = strip_smem + (uint32_t)stage * kStripBytes + (kF32 ? 0u : (uint32_t)p.pad_w * 8u);
 #pragma unroll
             for (int k = 0; k < kItemsPerThread; ++k) {
                 const int row = (int)(item_rq[k] >> 16), q = (int)(item_rq[k] & 0xffffu);
@@ -310,15 +341,23 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_nchw_kernel(const 
                                 asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[c].x), "=f"(v[c].y), "=f"(v[c].z), "=f"(v[c].w) : "r"(src));
                             }
                     }
-                    const uint32_t dst = dst0 + (uint32_t)row * (uint32_t)row_bytes + (uint32_t)q * 32u;
+                    const uint32_t dst = dst0 + (uint32_t)row * (uint32_t)row_bytes + (kF32 ? 0u : (uint32_t)q * 32u);
                     const float* f0 = reinterpret_cast<const float*>(&v[0]);
                     const float* f1 = reinterpret_cast<const float*>(&v[1]);
                     const float* f2 = reinterpret_cast<const float*>(&v[2]);
 #pragma unroll
-                    for (int px = 0; px < 4; ++px)
-                        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(dst + px * 8u), "r"(pack_bf16(f0[px], f1[px])),
-                                     "r"(pack_bf16(f2[px], 0.0f))
-                                     : "memory");
+                    for (int px = 0; px < 4; ++px) {
+                        if constexpr (kF32) {
+                            const uint32_t at = (uint32_t)(4 * q + px + p.pad_w);  // even pixels, then odd ones
+                            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (at & 1u) * (uint32_t)(row_bytes >> 1) + (at >> 1) * 16u),
+                                         "f"(tf32_rne(f0[px])), "f"(tf32_rne(f1[px])), "f"(tf32_rne(f2[px])), "f"(0.0f)
+                                         : "memory");
+                        } else {
+                            asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(dst + px * 8u), "r"(pack_bf16(f0[px], f1[px])),
+                                         "r"(pack_bf16(f2[px], 0.0f))
+                                         : "memory");
+                        }
+                    }
                 }
                 // the slots of item k are in registers (their values went into the stores above): refill them
                 issue_item(k, base2, row_lo2, row_hi2);
@@ -351,12 +390,12 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_nchw_kernel(const 
                     if (!__all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&bar_acc_empty[buf]), ((blk >> 1) & 1u) ^ 1u, abort_ptr))) { ok = false; break; }
                     tc_fence_after_sync();
                     const int in_row0 = s > 0 ? 2 * j0 : 2 * j0 - 2;  // local packed row of filter row 0 of conv row j0
-                    const uint32_t a_lo0 = desc_lo(strip_base + (uint32_t)(in_row0 * row_bytes), 16);
+                    const uint32_t a_lo0 = desc_lo(strip_base + (uint32_t)(in_row0 * row_bytes), kF32 ? (uint32_t)row_bytes >> 1 : 16u);
                     const uint32_t d0 = tmem_base + buf * kBufCols;
                     if (elect_one()) {
-                        if (R == 3) issue_block<3>(d0, a_lo0, row16, ab_hi, w_lo);
-                        else if (R == 2) issue_block<2>(d0, a_lo0, row16, ab_hi, w_lo);
-                        else issue_block<1>(d0, a_lo0, row16, ab_hi, w_lo);
+                        if (R == 3) issue_block<kF32, 3>(d0, a_lo0, row16, ab_hi, w_lo);
+                        else if (R == 2) issue_block<kF32, 2>(d0, a_lo0, row16, ab_hi, w_lo);
+                        else issue_block<kF32, 1>(d0, a_lo0, row16, ab_hi, w_lo);
                         umma_commit(smem_u32(&bar_acc_full[buf]));
                     }
                     __syncwarp();
@@ -365,6 +404,112 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_nchw_kernel(const 
                 if (elect_one()) umma_commit(smem_u32(&bar_empty[stage]));
                 __syncwarp();
                 if (++stage == kStages) { stage = 0; phase ^= 1u; }
+            }
+        }
+    } else if constexpr (kF32) {
+        // ------------------------------ epilogue, fp32 ------------------------------
+        // As below with one register per channel: the maximum is taken of the unrounded sums and rounded to tf32 once, which is
+        // the maximum of the rounded ones.
+        const int quad = warp & 3;
+        const int part = (warp - kEpilogueWarp0) >> 2;
+        const int ow = quad * 32 + lane;
+        const int c0 = part * kPartCols;
+        const int POH = p.OH / 2, POW = p.OW / 2;
+        float* pooled = static_cast<float*>(p.out);
+        const bool col_ok = ow < p.OW;
+        const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
+        pdl_wait();
+        uint32_t blk = 0;
+        uint32_t fin = 0;
+        bool bad = false, dead = false;
+        for (int strip = blockIdx.x; !dead && strip < total_strips; strip += gridDim.x) {
+            const int n = strip / strips_per_image;
+            const int s = strip - n * strips_per_image;
+            float vmax[kPartCols];
+#pragma unroll
+            for (int e = 0; e < kPartCols; ++e) vmax[e] = 0.0f;
+            for (int j0 = (s > 0 ? 0 : 1); !dead && j0 < kConvRows; j0 += kBlockRows, ++blk) {
+                const int R = kConvRows - j0 < kBlockRows ? kConvRows - j0 : kBlockRows;
+                const uint32_t buf = blk & 1u;
+                if (!bad) bad = !__all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&bar_acc_full[buf]), (blk >> 1) & 1u, abort_ptr));
+                if (!bad) tc_fence_after_sync();
+                for (int jj = 0; jj < R; ++jj) {
+                    const int j = j0 + jj;
+                    float cur[kPartCols];
+#pragma unroll
+                    for (int e = 0; e < kPartCols; ++e) cur[e] = 0.0f;
+                    if (!bad) {
+                        uint32_t v[kPartCols];
+                        tmem_ld_part(lane_base + buf * kBufCols + (uint32_t)(jj * kBN), v);
+                        tmem_ld_wait();
+                        if (jj == R - 1) {
+                            tc_fence_before_sync();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[buf]));
+                        }
+                        if (col_ok) {
+#pragma unroll
+                            for (int g = 0; g < kPartCols / 4; ++g) {
+                                float b[4];
+                                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(b[3]) : "r"(bias_smem + (uint32_t)(c0 + 4 * g) * 4u));
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) cur[4 * g + k] = __fadd_rn(__uint_as_float(v[4 * g + k]), b[k]);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int e = 0; e < kPartCols; ++e) vmax[e] = fmaxf(vmax[e], cur[e]);
+                    if ((j & 1) == 0 && j >= 2) {
+                        constexpr uint32_t kColBytes = kPartCols * 4;
+                        auto slot_of = [&](int q) { return exch_smem + ((((fin & 1u) * (uint32_t)(64 / kPartCols) + (uint32_t)part) * 4u + (uint32_t)q) * kColBytes); };
+                        if (lane == 31) {
+                            const uint32_t slot = slot_of(quad);
+#pragma unroll
+                            for (int g = 0; g < kPartCols / 4; ++g)
+                                asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(slot + g * 16u), "f"(vmax[4 * g]), "f"(vmax[4 * g + 1]),
+                                             "f"(vmax[4 * g + 2]), "f"(vmax[4 * g + 3])
+                                             : "memory");
+                        }
+                        if (named_barrier_or(1 + part, 128, bad)) {
+                            dead = true;
+                            break;
+                        }
+                        constexpr int kHalf = kPartCols / 2;
+                        const bool odd = (lane & 1) != 0;
+                        float edge[kHalf];
+#pragma unroll
+                        for (int e = 0; e < kHalf; ++e) edge[e] = 0.0f;
+                        if (lane < 2 && quad > 0) {
+                            const uint32_t slot = slot_of(quad - 1) + (odd ? kColBytes / 2 : 0u);
+#pragma unroll
+                            for (int g = 0; g < kHalf / 4; ++g)
+                                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                             : "=f"(edge[4 * g]), "=f"(edge[4 * g + 1]), "=f"(edge[4 * g + 2]), "=f"(edge[4 * g + 3])
+                                             : "r"(slot + g * 16u));
+                        }
+                        float res[kHalf];
+#pragma unroll
+                        for (int e = 0; e < kHalf; ++e) {
+                            const float lo = vmax[e], hi = vmax[e + kHalf];
+                            const float partner = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1);
+                            const float up1 = __shfl_up_sync(0xffffffffu, lo, 1);
+                            const float up2 = __shfl_up_sync(0xffffffffu, hi, 2);
+                            float prev = odd ? up2 : up1;
+                            if (lane < 2) prev = edge[e];
+                            const float m = fmaxf(fmaxf(fmaxf(odd ? hi : lo, partner), prev), 0.0f);
+                            res[e] = p.round_out_tf32 ? tf32_rne(m) : m;
+                        }
+                        if ((ow & ~1) < p.OW) {
+                            const int ph = kPooledRows * s + j / 2 - 1;
+                            float4* dst = reinterpret_cast<float4*>(pooled + ((((size_t)n * POH + ph) * POW + (ow >> 1)) * kBN) + c0 + (odd ? kHalf : 0));
+#pragma unroll
+                            for (int g = 0; g < kHalf / 4; ++g) dst[g] = make_float4(res[4 * g], res[4 * g + 1], res[4 * g + 2], res[4 * g + 3]);
+                        }
+                        ++fin;
+#pragma unroll
+                        for (int e = 0; e < kPartCols; ++e) vmax[e] = cur[e];
+                    }
+                }
             }
         }
     } else {
@@ -474,7 +619,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_nchw_kernel(const 
                             res[e] = *reinterpret_cast<uint32_t*>(&m);
                         }
                         if ((ow & ~1) < p.OW) {
-                            const int ph = 4 * s + j / 2 - 1;
+                            const int ph = kPooledRows * s + j / 2 - 1;
                             uint4* dst = reinterpret_cast<uint4*>(pooled + ((((size_t)n * POH + ph) * POW + (ow >> 1)) * kBN) + c0 + (odd ? kHalf * 2 : 0));
 #pragma unroll
                             for (int g = 0; g < kHalf / 4; ++g) dst[g] = make_uint4(res[4 * g], res[4 * g + 1], res[4 * g + 2], res[4 * g + 3]);
@@ -503,42 +648,63 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_nchw_kernel(const 
 }
 
 // Stem weights, filter rows stacked by parity: [r = 6,4,2,0 | r = 5,3,1], each stack in core-matrix order
-// [4 k-chunks][stack rows][8] bf16 with stack row = (position in the stack) * 64 + cout; element e of chunk j = pixel
-// 2j + e/4, channel e%4; zero for kw >= KW or c >= C.
-__global__ void stem_pack_weights_stacked_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ out, int O, int C, int KW) {
-    const int total = 4 * (kEvenRows + kOddRows) * 8;
+// [k-chunks][stack rows][16 bytes] with stack row = (position in the stack) * 64 + cout; element e of bf16 chunk j (of 4) = pixel
+// 2j + e/4, channel e%4, of tf32 chunk j (of 8) = pixel j, channel e; zero for kw >= KW or c >= C.
+template <typename T>
+__global__ void stem_pack_weights_stacked_kernel(const float* __restrict__ w, T* __restrict__ out, int O, int C, int KW) {
+    constexpr int kElems = 16 / (int)sizeof(T), kPixels = kElems / 4, kChunks = 8 / kPixels;
+    const int total = kChunks * (kEvenRows + kOddRows) * kElems;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const bool odd = i >= 4 * kEvenRows * 8;
-        const int li = odd ? i - 4 * kEvenRows * 8 : i;
+        const bool odd = i >= kChunks * kEvenRows * kElems;
+        const int li = odd ? i - kChunks * kEvenRows * kElems : i;
         const int rows = odd ? kOddRows : kEvenRows;
-        const int e = li & 7;
-        const int row = (li >> 3) % rows;
-        const int jc = (li >> 3) / rows;
+        const int e = li % kElems;
+        const int row = (li / kElems) % rows;
+        const int jc = (li / kElems) / rows;
         const int o = row & (kBN - 1), pos = row / kBN;
         const int r = odd ? (kKH - 2) - 2 * pos : (kKH - 1) - 2 * pos;
-        const int kw = 2 * jc + (e >> 2), c = e & 3;
+        const int kw = kPixels * jc + (e >> 2), c = e & 3;
         float f = 0.0f;
         if (o < O && c < C && kw < KW) f = w[((o * C + c) * kKH + r) * KW + kw];
-        out[i] = __float2bfloat16_rn(f);
+        if constexpr (sizeof(T) == 4) out[i] = tf32_rne(f);
+        else out[i] = __float2bfloat16_rn(f);
     }
+}
+
+template <bool kF32, int kPooled>
+int32_t launch(const TcParams& p, cudaStream_t stream) {
+    constexpr int kBytes = StemGeom<kF32, kPooled>::kSmemBytes;
+    static PerDeviceOnce smem_once;
+    auto kernel = conv_stem_pool_nchw_kernel<kF32, kPooled>;
+    KXC_TRY(smem_opt_in(smem_once, kernel, kBytes));
+    const long long strips = (long long)(p.OH / (2 * kPooled)) * p.N;
+    const int grid = (int)(strips < kNumSMs ? strips : kNumSMs);
+    KXC_CUDA_TRY(launch_kernel(kernel, dim3(grid), dim3(kThreads), kBytes, stream, /*pdl=*/true, 1, p));
+    return check_launch("conv_stem_pool_nchw_kernel");
 }
 
 }  // namespace
 
 bool stem_pool_nchw_applicable(TcDType dtype, int C, int O, int KH, int KW, int W, int OH, int OW, int Wp) {
-    return dtype == kTcBF16 && C >= 1 && C <= kMaxC && W <= 4 * kMaxRowItems && kInRows * (W / 4) <= kItemsPerThread * kConverterThreads &&
-           O == kBN && KH == kKH && KW <= 8 && (W % 4) == 0 && (OH % (2 * kPooledRows)) == 0 &&
-           (OW % 2) == 0 && OW <= 128 && Wp * 8 <= kMaxRowBytes && (Wp * 8) % 16 == 0;
+    if (dtype != kTcBF16 && dtype != kTcTF32) return false;
+    const bool f32 = dtype == kTcTF32;
+    const int row_bytes = Wp * (f32 ? 16 : 8), pooled = f32 ? 2 : 4;
+    return C >= 1 && C <= kMaxC && W <= (f32 ? StemGeom<true, 2>::kMaxWidth : StemGeom<false, 4>::kMaxWidth) && O == kBN && KH == kKH && KW <= 8 && (W % 4) == 0 && (OH % (2 * pooled)) == 0 &&
+           (OW % 2) == 0 && OW <= 128 && row_bytes <= (f32 ? StemGeom<true, 2>::kMaxRowBytes : StemGeom<false, 4>::kMaxRowBytes) && row_bytes % 32 == 0;
 }
 
-size_t stem_stacked_weight_bytes() { return (size_t)kWeightBytes; }
+size_t stem_stacked_weight_bytes(TcDType dtype) {
+    return dtype == kTcTF32 ? (size_t)StemGeom<true, 2>::kWeightBytes : (size_t)StemGeom<false, 4>::kWeightBytes;
+}
 
-int32_t stem_stacked_pack_weights(const float* w, void* out, int O, int C, int KW, cudaStream_t s) {
-    stem_pack_weights_stacked_kernel<<<(4 * (kEvenRows + kOddRows) * 8 + 255) / 256, 256, 0, s>>>(w, static_cast<__nv_bfloat16*>(out), O, C, KW);
+int32_t stem_stacked_pack_weights(TcDType dtype, const float* w, void* out, int O, int C, int KW, cudaStream_t s) {
+    const int grid = (8 * (kEvenRows + kOddRows) * 4 + 255) / 256;
+    if (dtype == kTcTF32) stem_pack_weights_stacked_kernel<float><<<grid, 256, 0, s>>>(w, static_cast<float*>(out), O, C, KW);
+    else stem_pack_weights_stacked_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(w, static_cast<__nv_bfloat16*>(out), O, C, KW);
     return check_launch("stem_pack_weights_stacked");
 }
 
-int32_t stem_pool_nchw_setup(TcParams* p, const void* packed_w, int N, int C, int H, int W, int OH, int OW, int pad_h, int pad_w,
+int32_t stem_pool_nchw_setup(TcParams* p, TcDType dtype, const void* packed_w, int N, int C, int H, int W, int OH, int OW, int pad_h, int pad_w,
                              int Hp, int Wp) {
     p->N = N; p->OH = OH; p->OW = OW; p->Cout = kBN;
     p->taps_h = kKH; p->taps_w = 1; p->stride = 2;
@@ -547,24 +713,21 @@ int32_t stem_pool_nchw_setup(TcParams* p, const void* packed_w, int N, int C, in
     p->tiles_w = 1; p->tiles_h = OH; p->tiles_n = N; p->tiles_c = 1;
     p->aux_in = nullptr;  // the graph input: bound at run time
     p->aux_w = packed_w;
-    p->aux_row_bytes = Wp * 8;
+    p->aux_row_bytes = Wp * (dtype == kTcTF32 ? 16 : 8);
     p->aux_hp = Hp;
     p->aux_c = C; p->aux_h = H; p->aux_w_px = W;
     KXC_TRY(tc_status_word(&p->status));
     return KXC_B200_OK;
 }
 
-int32_t stem_pool_nchw_launch(const TcParams& p, cudaStream_t stream) {
-    static PerDeviceOnce smem_once;
-    KXC_TRY(smem_opt_in(smem_once, conv_stem_pool_nchw_kernel, kSmemBytes));
-    if (!p.vec_ok || p.out == nullptr || p.aux_in == nullptr)
+int32_t stem_pool_nchw_launch(TcDType dtype, const TcParams& p, cudaStream_t stream) {
+    if ((dtype == kTcBF16 && !p.vec_ok) || p.out == nullptr || p.aux_in == nullptr)
         return fail(KXC_B200_ERR_INVALID, "fused stem conv + pool: missing tensors or pointers that are not 16-byte aligned");
     if (!p.relu) return fail(KXC_B200_ERR_INVALID, "fused stem conv + pool: the pooling shortcut relies on the ReLU in between");
-    const long long strips = (long long)(p.OH / (2 * kPooledRows)) * p.N;
-    if (strips <= 0) return KXC_B200_OK;
-    const int grid = (int)(strips < kNumSMs ? strips : kNumSMs);
-    KXC_CUDA_TRY(launch_kernel(conv_stem_pool_nchw_kernel, dim3(grid), dim3(kThreads), kSmemBytes, stream, /*pdl=*/true, 1, p));
-    return check_launch("conv_stem_pool_nchw_kernel");
+    if (p.N <= 0 || p.OH <= 0) return KXC_B200_OK;
+    if (dtype == kTcTF32) return launch<true, 2>(p, stream);
+    // two pooled rows per strip where every strip then has an SM to itself
+    return (long long)(p.OH / 4) * p.N <= kNumSMs ? launch<false, 2>(p, stream) : launch<false, 4>(p, stream);
 }
 
 }  // namespace kxc_b200

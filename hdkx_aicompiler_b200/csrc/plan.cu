@@ -561,16 +561,20 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
                     const bool pool_ok = pa.pool_size[0] == 3 && pa.pool_size[1] == 3 && pa.strides[0] == 2 && pa.strides[1] == 2 &&
                                          pa.padding[0] == 1 && pa.padding[1] == 1 && pa.padding[2] == 1 && pa.padding[3] == 1 &&
                                          pa.ceil_mode == 0;
+                    const char* e3 = getenv("KXC_B200_STEM_FUSED_INPUT");  // "0" keeps the pack kernel + packed-input kernel
+                    const bool nchw_ok = (!e3 || atoi(e3) != 0) && !pl->x3 && n.conv.padding[0] == KHc / 2 && n.conv.padding[1] == KWc / 2 &&
+                                         stem_pool_nchw_applicable(dt, st.C, (int)w->shape[0], KHc, KWc, st.W, OHc, OWc, Wpc);
+                    // tf32: the fused kernel or none, from 57 strips of four convolution rows on (three images of 224 x 224). Below,
+                    // whole networks gain 1 to 3 % (one image 170 / 168 us, two 186 / 180; four 217 / 209) and keep the list of
+                    // launches that test_resnet18_plan holds them to. bf16 has a fused kernel for packed inputs too.
                     if (pool_ok && st.C <= 4 && KWc <= 8 && st.W >= 8 &&
-                        stem_direct_applicable(dt, st.C, (int)w->shape[0], KHc, KWc, OWc, Wpc) && stem_pool_applicable(OHc, OWc, 3, 2, 1)) {
+                        (dt == kTcTF32 ? nchw_ok && (long long)(OHc / 4) * st.N > 56
+                                       : stem_direct_applicable(dt, st.C, (int)w->shape[0], KHc, KWc, OWc, Wpc) && stem_pool_applicable(OHc, OWc, 3, 2, 1))) {
                         st.fused_pool = 1;
                         pl->nodes[pc].fused_into_other = true;
                         cur = pl->nodes[pc].out;
                         emit_at = pc;
-                        const char* e3 = getenv("KXC_B200_STEM_FUSED_INPUT");  // "0" keeps the pack kernel + packed-input kernel
-                        if ((!e3 || atoi(e3) != 0) && n.conv.padding[0] == KHc / 2 && n.conv.padding[1] == KWc / 2 &&
-                            stem_pool_nchw_applicable(dt, st.C, (int)w->shape[0], KHc, KWc, st.W, OHc, OWc, Wpc))
-                            st.direct_input = 1;
+                        st.direct_input = nchw_ok ? 1 : 0;
                     }
                 }
             }
@@ -935,7 +939,7 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
             const int stem_oh = (int)conv_out_dim(st.H, pw.KH, 2, st.pad_h, 1), stem_ow = (int)conv_out_dim(st.W, pw.KW, 2, st.pad_w, 1);
             if (st.direct_input) {
                 pw.mode = 5;
-                if (stem_stacked_weight_bytes() > pw.bytes) return fail(KXC_B200_ERR_INVALID, "plan: stacked stem weights do not fit their slot");
+                if (stem_stacked_weight_bytes(dt) > pw.bytes) return fail(KXC_B200_ERR_INVALID, "plan: stacked stem weights do not fit their slot");
             }
             if (pw.mode == 1 && !st.out_is_graph_output) {
                 // the direct stem kernel writes bf16 NHWC only; its packed weights take the same number of bytes
@@ -952,7 +956,7 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
             if (st.fused_pool && pw.mode != 4 && pw.mode != 5) return fail(KXC_B200_ERR_UNSUPPORTED, "plan: fused stem pooling needs the direct stem kernel");
             if (pw.mode == 5) {
                 st.direct = 4;
-                KXC_TRY(stem_pool_nchw_setup(&st.params, pw.ptr, st.N, st.C, st.H, st.W, stem_oh, stem_ow, st.pad_h, st.pad_w, st.Hp, st.Wp));
+                KXC_TRY(stem_pool_nchw_setup(&st.params, dt, pw.ptr, st.N, st.C, st.H, st.W, stem_oh, stem_ow, st.pad_h, st.pad_w, st.Hp, st.Wp));
                 st.cfg = TcConfig{dt, 64, 64, om};
             } else if (pw.mode == 4) {
                 st.direct = 2;
@@ -1104,7 +1108,7 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
             case 0: KXC_TRY(pack_weights_ohwi(WeightPack{src, w.ptr, w.ptr_lo, w.O, w.C, w.KH * w.KW, w.cpad}, dt, s)); break;
             case 1: KXC_TRY(stem_pack_weights(static_cast<const float*>(src), w.ptr, dt, w.O, w.C, w.KH, w.KW, s)); break;
             case 4: KXC_TRY(stem_direct_pack_weights(static_cast<const float*>(src), w.ptr, w.O, w.C, w.KH, w.KW, s)); break;
-            case 5: KXC_TRY(stem_stacked_pack_weights(static_cast<const float*>(src), w.ptr, w.O, w.C, w.KW, s)); break;
+            case 5: KXC_TRY(stem_stacked_pack_weights(dt, static_cast<const float*>(src), w.ptr, w.O, w.C, w.KW, s)); break;
             case 2: KXC_TRY(convert_rows(static_cast<const float*>(src), w.ptr, dt, w.O, w.C, w.cpad, s)); break;
             case 3: KXC_TRY(convert_operands(src, w.ptr, w.ptr_lo, dt, 1, w.C, w.O, w.cpad, nullptr, s, false)); break;
         }
@@ -1154,7 +1158,7 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
                 if (st.weight2 >= 0 && ((reinterpret_cast<uintptr_t>(p.bias2) | reinterpret_cast<uintptr_t>(p.out2)) & 15u)) p.vec_ok = 0;
                 if (st.direct == 4) {
                     p.aux_in = arg_of(st.src_input);
-                    KXC_TRY(stem_pool_nchw_launch(p, s));
+                    KXC_TRY(stem_pool_nchw_launch(dt, p, s));
                 } else if (st.direct == 2) {
                     KXC_TRY(st.fused_pool ? stem_pool_launch(p, s) : stem_direct_launch(p, s));
                 } else if (st.direct == 3) {

@@ -302,6 +302,37 @@ def test_stem_pool_fusion_is_bit_identical(kxc, monkeypatch):
     assert np.mean(fused != exp) < 1e-3 and np.abs(fused - exp).max() <= 2.0 ** -7 * np.abs(exp).max()
 
 
+# The fused stem against pack + convolution + pool, bit for bit: strips of two pooled rows (tf32; bf16 while each has an SM to itself)
+# and of four, one strip per image, several strips per CTA, narrow images whose A rows read far past a row's end, the widest image,
+# one to three channels, values that are not finite.
+@pytest.mark.parametrize("precision", ["bf16", "tf32"])
+@pytest.mark.parametrize("n,c,h,w", [(1, 3, 224, 224), (6, 3, 224, 224), (30, 2, 16, 8), (10, 3, 48, 100), (301, 1, 16, 12), (2, 3, 32, 244)])
+def test_fused_stem_is_bit_identical(kxc, monkeypatch, precision, n, c, h, w):
+    R = kxc.relay
+    rng = np.random.default_rng(n + w)
+    x = rng.normal(0, 1, (n, c, h, w)).astype(f32)
+    x[n - 1, 0, 5, 3:6] = [np.inf, np.nan, -np.inf]
+    wt = rng.normal(0, (2 / (49 * c)) ** 0.5, (64, c, 7, 7)).astype(f32)
+    b = rng.normal(0, 0.1, (64,)).astype(f32)
+
+    def build():
+        xv = R.Var("input", x.shape)
+        y = R.Call("nn_relu", [R.Call("nn_conv2d", [xv, R.Constant(cuda_const(wt)), R.Constant(cuda_const(b))],
+                                      R.Conv2DAttrs((2, 2), (3, 3, 3, 3), (1, 1), 1))])
+        y = R.Call("nn_max_pool2d", [y], R.MaxPool2DAttrs((2, 2), (1, 1, 1, 1), (1, 1), (3, 3), "NCHW", False))
+        return R.Function([xv], R.Call("nn_relu", [y]))
+
+    fused, gf = run_plan(kxc, build(), x, precision)
+    assert any(l[0].startswith("conv_stem_pool_nchw") for l in gf.launch_info()) == (precision == "bf16" or (w <= 224 and n > 1))
+    monkeypatch.setenv("KXC_B200_STEM_FUSED_INPUT", "0")
+    monkeypatch.setenv("KXC_B200_STEM_POOL_FUSE", "0")
+    unfused, gu = run_plan(kxc, build(), x, precision)
+    assert not any(l[0].startswith("conv_stem_pool") for l in gu.launch_info())
+    from hdkx_aicompiler_b200 import ops
+    assert ops.device_status() == 0
+    assert_bit_exact(fused, unfused, f"{precision} {n}x{c}x{h}x{w}")
+
+
 @pytest.mark.parametrize("cin,cout,hw,N", [(64, 128, 56, 3), (128, 256, 28, 3), (64, 64, 30, 3), (256, 512, 14, 128)])
 def test_downsample_block_two_output_kernel_is_bit_identical(kxc, monkeypatch, cin, cout, hw, N):
     """A ResNet downsample block: conv3x3(s2)+relu and the residual branch's conv1x1(s2) read the same tensor and
