@@ -72,7 +72,8 @@ struct PackArgs {
 // Activations NCHW fp32 -> NHWC of the operand type and, in the first blocks of the same launch, the weights of the convolution
 // that follows. One launch instead of two (each cost 2 to 3 us of launch and drain beside 2 to 5 us of work: conv 72 -> 120 3x3
 // at 45x51, 9 images, tf32: 38.9 -> 32.3 us a call). A block turns kCT channels x 2048 / kCT pixels through shared memory with
-// eight loads in flight per thread; stores are channel pairs, 128 or 256 bytes per pixel (kCT = 64; 32 for fewer channels).
+// eight loads in flight per thread; stores are channel pairs, 128 bytes per pixel (kCT = 64 for more than 32 bf16 channels, which are
+// padded to whole 64s then, else 32: fp32 counts are padded to 32s, 66 channels at 23x22, 43 images: 5.7 us with 64, 4.7 with 32).
 // Bound by memory: 4 bytes read and 2, 4 or 8 written per value.
 //
 // Programmatic launch on both sides: the blocks wait for the previous kernel before they touch memory, and with `overlap` then
@@ -388,7 +389,10 @@ int32_t launch_convert(const float* in, void* out, void* lo, int N, int C, int H
                                    cpad, tiles_hw, tiles_c, pack, overlap ? 1 : 0));
         return check_launch("convert_operands");
     };
-    return cpad <= 32 ? go(convert_operands_kernel<TOut, kSplit, 32>, 32) : go(convert_operands_kernel<TOut, kSplit, 64>, 64);
+    if constexpr (sizeof(TOut) == 2) {
+        if (cpad > 32) return go(convert_operands_kernel<TOut, kSplit, 64>, 64);
+    }
+    return go(convert_operands_kernel<TOut, kSplit, 32>, 32);
 }
 
 // Byte transposition of `batch` matrices, by words turned in registers where pitches and addresses allow it.
