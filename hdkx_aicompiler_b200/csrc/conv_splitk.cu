@@ -4,14 +4,19 @@
 // rest of the chip does. ResNet-18 bf16 on one image: 221 -> 130 us (layer 4: 24 -> 7.5 us per convolution, layer 3: 14.5 -> 7.4).
 //
 // One cluster = one output tile of 128 pixels x BN channels; CTA r of S takes the K blocks [r*K/S, (r+1)*K/S) through the same
-// TMA -> tcgen05.mma pipeline, writes its partial sums into its own (by then idle) operand ring, and after a cluster barrier
-// CTA r adds the r-th S-th of the rows of all S partials over distributed shared memory, in rank order, and applies the
-// epilogue. No partial sum touches global memory, nothing is atomic, and the result does not depend on timing.
+// TMA -> tcgen05.mma pipeline and owns the r-th S-th of the rows. It writes its partial sums into its own (by then idle) operand
+// ring; each warp sends the rows of its 32 x 32 piece to their owners as bulk copies between the CTAs' shared memories, counted on the
+// owner's mbarrier, and the owner adds the S parts in rank order and applies the epilogue. No partial sum touches global memory,
+// nothing is atomic, and the result does not depend on timing.
+// The other ways to exchange them were slower: owners that fetch the parts after a cluster barrier, a few 16-byte loads per
+// thread in flight (whole networks, us before / now: bf16 one image 127.3 / 121.0, 8: 161.9 / 155.7; tf32 one image 168.0 / 157.8,
+// 4: 204.0 / 189.5, 32: 491.6 / 476.7), and 16-byte st.async from the accumulator to the owners (slower than the fetches from two
+// images on, tf32 32: 524).
 //
 //   warp 0      TMA producer; loads the weights of the first stages before it waits for the previous kernel (weights of a
 //               plan do not come from that kernel), so only the pixels are on the critical path of a layer
 //   warp 1      MMA issuer, TMEM owner
-//   warps 2..9  accumulator -> shared memory, then reduction and epilogue, 8 channels of one pixel per thread and step
+//   warps 2..9  accumulator -> shared memory -> owners, then reduction and epilogue, 8 channels of one pixel per thread and step
 //
 // The shape of the launch (S, BN) comes from choose_split or, with two outputs, tc_setup_dual in conv_tc.cu. Waits are bounded as in conv_tc.cu; the cluster
 // barriers are reached by every thread of every CTA whether or not a wait ran out.
@@ -34,73 +39,132 @@ constexpr int kSplitThreads = 320;
 constexpr int kKB = 128;  // bytes of a K block
 constexpr int kSplitSmem = 227 * 1024 - 2048;
 
-template <int BN, bool kX3>
+template <int BN, bool kX3, bool kDual = false>
 struct SplitGeom {
     static constexpr int kATile = 128 * kKB;
     static constexpr int kBTile = BN * kKB;
     static constexpr int kABytes = (kX3 ? 2 : 1) * kATile;
     static constexpr int kStageBytes = kABytes + (kX3 ? 2 : 1) * kBTile;
-    static constexpr int kStagesRaw = (kSplitSmem - 1024) / kStageBytes;
+    // A CTA's own sums: [BN / 32][128 rows][128 bytes], at the start of the ring. What it receives: [BN / 32][other ranks][rows][128
+    // bytes], at most 7 x 16 or 6 x 19 rows (256 channels: up to 3 x 32), one rank more with a second output.
+    static constexpr int kSumBytes = 128 * BN * 4;
+    static constexpr int kMaxParts = BN == 256 ? 4 : kMaxSplit;
+    static constexpr int kRecvRows = kDual ? 133 : (BN == 256 ? 96 : 114);
+    static constexpr int kRecvBytes = kRecvRows * BN * 4;
+    // It lies behind the ring, ready from the start, where that costs one of eight stages; else behind the CTA's own sums, from when
+    // the cluster's MMAs have read the rings (128 channels with five of seven stages and a buffer: 2 to 3 % slower in long reductions).
+    static constexpr bool kOwnBuffer = BN == 64 && !kX3;
+    static constexpr int kStagesRaw = (kSplitSmem - 1024 - (kOwnBuffer ? kRecvBytes : 0)) / kStageBytes;
     static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
-    static constexpr int kSmemBytes = kStages * kStageBytes + 1024;
+    static constexpr int kRecvOffset = kOwnBuffer ? kStages * kStageBytes : kSumBytes;
+    static constexpr int kUsed = kRecvOffset + kRecvBytes > kStages * kStageBytes ? kRecvOffset + kRecvBytes : kStages * kStageBytes;
+    static constexpr int kSmemBytes = kUsed + 1024;
+    static_assert(kSmemBytes <= kSplitSmem && (kDual ? 2 : 1) * kSumBytes <= (kOwnBuffer ? kStages * kStageBytes : kSumBytes), "shared memory of one CTA");
 };
 
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
-    return v;
+// `bytes` (a multiple of 16) into a CTA of the cluster, counted on the mbarrier `cluster_bar` of that CTA
+__device__ __forceinline__ void bulk_copy_to_cta(uint32_t cluster_dst, uint32_t src, uint32_t bytes, uint32_t cluster_bar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(cluster_dst), "r"(src),
+                 "r"(bytes), "r"(cluster_bar)
+                 : "memory");
 }
 
-// byte offset of the 16-byte piece `piece` of row `row` in a partial tile of BN fp32 columns (pieces rotate with the row, so
-// that both a warp of rows and a warp of pieces touch all banks)
-template <int BN>
-__device__ __forceinline__ uint32_t partial_off(int row, int piece) {
-    return (uint32_t)(row * BN * 4 + ((piece ^ (row & 7)) << 4));
-}
+// byte offset of 16-byte piece 0..7 in a row of 32 sums (pieces rotate with the row's place in its owner's share, so that both a
+// warp of rows and a warp of pieces touch all banks)
+__device__ __forceinline__ uint32_t piece_off(int local_row, int piece) { return (uint32_t)((piece ^ (local_row & 7)) << 4); }
 
-// +bias -> +residual -> ReLU -> store of 8 consecutive channels of one pixel
-template <int kOutMode, bool kSplitOut>
-__device__ __forceinline__ void epilogue8(const TcParams& p, float (&f)[8], const float* bias, const void* residual, void* out_ptr, int relu,
-                                          int c0, int n, int oh, int ow) {
-    const int nch = p.Cout - c0 < 8 ? p.Cout - c0 : 8;
-    const size_t pix = ((size_t)n * p.OH + oh) * p.OW + ow;
+// 8 consecutive channels [c0, c0 + 8) of one pixel: a thread's share of a step
+struct Item {
+    bool mine;
+    int second, piece, local, row;  // second output; piece of 8 columns; row of the owner's share, of the tile
+    int c0, n, oh, ow;
+};
+
+// what the epilogue of an item reads from global memory, fetched while the sums are still on their way
+template <int kOutMode>
+struct Ahead {
+    float bias[8];
+    uint32_t res[kOutMode == kOutNHWC_BF16 ? 4 : 8];  // bf16 pairs or fp32
+};
+
+template <int kOutMode>
+__device__ __forceinline__ void fetch_ahead(const TcParams& p, const Item& it, const float* bias, const void* residual, Ahead<kOutMode>& a) {
+    if (!it.mine) return;
+    const int nch = p.Cout - it.c0 < 8 ? p.Cout - it.c0 : 8;
+    const size_t pix = ((size_t)it.n * p.OH + it.oh) * p.OW + it.ow;
     if (bias != nullptr) {
+        if (nch == 8 && p.vec_ok) {
+            const float4 x = __ldg(reinterpret_cast<const float4*>(bias + it.c0)), y = __ldg(reinterpret_cast<const float4*>(bias + it.c0) + 1);
+            a.bias[0] = x.x; a.bias[1] = x.y; a.bias[2] = x.z; a.bias[3] = x.w;
+            a.bias[4] = y.x; a.bias[5] = y.y; a.bias[6] = y.z; a.bias[7] = y.w;
+        } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (j < nch) f[j] = __fadd_rn(f[j], __ldg(bias + c0 + j));
+            for (int j = 0; j < 8; ++j) a.bias[j] = j < nch ? __ldg(bias + it.c0 + j) : 0.0f;
+        }
     }
-    if constexpr (kOutMode == kOutNCHW_F32) {
-        const size_t plane = (size_t)p.OH * p.OW;
-        const size_t off = ((size_t)n * p.Cout + c0) * plane + (size_t)oh * p.OW + ow;
+    if (residual == nullptr) return;
+    if constexpr (kOutMode == kOutNHWC_BF16) {
+        const __nv_bfloat16* res = static_cast<const __nv_bfloat16*>(residual) + pix * p.Cout + it.c0;
+        if (nch == 8 && (p.Cout & 7) == 0 && p.vec_ok) {
+            const uint4 r = __ldg(reinterpret_cast<const uint4*>(res));
+            a.res[0] = r.x; a.res[1] = r.y; a.res[2] = r.z; a.res[3] = r.w;
+        } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (j < nch) {
-                float x = f[j];
-                if (residual != nullptr) x = __fadd_rn(x, __ldg(static_cast<const float*>(residual) + off + j * plane));
-                static_cast<float*>(out_ptr)[off + j * plane] = relu && !(x > 0.0f) ? 0.0f : x;
-            }
-    } else if constexpr (kOutMode == kOutNHWC_BF16) {
-        const bool vec = nch == 8 && (p.Cout & 7) == 0 && p.vec_ok;
-        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(out_ptr) + pix * p.Cout + c0;
-        if (residual != nullptr) {
-            const __nv_bfloat16* res = static_cast<const __nv_bfloat16*>(residual) + pix * p.Cout + c0;
-            if (vec) {
-                const uint4 r = __ldg(reinterpret_cast<const uint4*>(res));
-                const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    f[2 * k] = __fadd_rn(f[2 * k], bf16_lo(w[k]));
-                    f[2 * k + 1] = __fadd_rn(f[2 * k + 1], bf16_hi(w[k]));
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (j < nch) f[j] = __fadd_rn(f[j], __bfloat162float(res[j]));
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t lo = 2 * k < nch ? __ldg(reinterpret_cast<const unsigned short*>(res) + 2 * k) : 0u;
+                const uint32_t hi = 2 * k + 1 < nch ? __ldg(reinterpret_cast<const unsigned short*>(res) + 2 * k + 1) : 0u;
+                a.res[k] = lo | (hi << 16);
             }
         }
+    } else {
+        const size_t plane = kOutMode == kOutNCHW_F32 ? (size_t)p.OH * p.OW : 1;
+        const float* res = static_cast<const float*>(residual) + (kOutMode == kOutNCHW_F32 ? ((size_t)it.n * p.Cout + it.c0) * plane + (size_t)it.oh * p.OW + it.ow
+                                                                                           : pix * p.Cout + it.c0);
+        if (kOutMode == kOutNHWC_F32 && nch == 8 && (p.Cout & 3) == 0 && p.vec_ok) {
+            const uint4 x = __ldg(reinterpret_cast<const uint4*>(res)), y = __ldg(reinterpret_cast<const uint4*>(res) + 1);
+            a.res[0] = x.x; a.res[1] = x.y; a.res[2] = x.z; a.res[3] = x.w;
+            a.res[4] = y.x; a.res[5] = y.y; a.res[6] = y.z; a.res[7] = y.w;
+        } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] = relu && !(f[j] > 0.0f) ? 0.0f : f[j];
-        if (vec) {
+            for (int j = 0; j < 8; ++j) a.res[j] = j < nch ? __float_as_uint(__ldg(res + j * plane)) : 0u;
+        }
+    }
+}
+
+// +bias -> +residual -> ReLU -> store of an item
+template <int kOutMode, bool kSplitOut>
+__device__ __forceinline__ void epilogue8(const TcParams& p, float (&f)[8], const Ahead<kOutMode>& a, bool has_bias, bool has_res, void* out_ptr,
+                                          int relu, const Item& it) {
+    const int c0 = it.c0;
+    const int nch = p.Cout - c0 < 8 ? p.Cout - c0 : 8;
+    const size_t pix = ((size_t)it.n * p.OH + it.oh) * p.OW + it.ow;
+    if (has_bias) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = __fadd_rn(f[j], a.bias[j]);
+    }
+    if (has_res) {
+        if constexpr (kOutMode == kOutNHWC_BF16) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                f[2 * k] = __fadd_rn(f[2 * k], bf16_lo(a.res[k]));
+                f[2 * k + 1] = __fadd_rn(f[2 * k + 1], bf16_hi(a.res[k]));
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) f[j] = __fadd_rn(f[j], __uint_as_float(a.res[j]));
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = relu && !(f[j] > 0.0f) ? 0.0f : f[j];
+    if constexpr (kOutMode == kOutNCHW_F32) {
+        const size_t plane = (size_t)p.OH * p.OW;
+        float* out = static_cast<float*>(out_ptr) + ((size_t)it.n * p.Cout + c0) * plane + (size_t)it.oh * p.OW + it.ow;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (j < nch) out[j * plane] = f[j];
+    } else if constexpr (kOutMode == kOutNHWC_BF16) {
+        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(out_ptr) + pix * p.Cout + c0;
+        if (nch == 8 && (p.Cout & 7) == 0 && p.vec_ok) {
             *reinterpret_cast<uint4*>(out) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
         } else {
 #pragma unroll
@@ -109,16 +173,10 @@ __device__ __forceinline__ void epilogue8(const TcParams& p, float (&f)[8], cons
         }
     } else {  // kOutNHWC_F32
         const size_t off = pix * p.Cout + c0;
-        const bool vec = nch == 8 && (p.Cout & 3) == 0 && p.vec_ok;
-        if (residual != nullptr) {
+        const bool whole = nch == 8 && (p.Cout & 3) == 0;
+        if (p.round_out_tf32) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (j < nch) f[j] = __fadd_rn(f[j], __ldg(static_cast<const float*>(residual) + off + j));
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            f[j] = relu && !(f[j] > 0.0f) ? 0.0f : f[j];
-            if (p.round_out_tf32) f[j] = tf32_rne(f[j]);
+            for (int j = 0; j < 8; ++j) f[j] = tf32_rne(f[j]);
         }
         auto store = [&](float* dst, const float (&v)[8], bool wide) {
             if (wide) {
@@ -138,21 +196,20 @@ __device__ __forceinline__ void epilogue8(const TcParams& p, float (&f)[8], cons
                     h[j] = tf32_rne(f[j]);
                     l[j] = tf32_low_part(f[j], h[j]);
                 }
-                store(p.out_hi + off, h, nch == 8 && (p.Cout & 3) == 0);
-                store(p.out_hi + p.out_lo_offset + off, l, nch == 8 && (p.Cout & 3) == 0);
+                store(p.out_hi + off, h, whole);
+                store(p.out_hi + p.out_lo_offset + off, l, whole);
             }
             if (out_ptr == nullptr) return;
         }
-        store(static_cast<float*>(out_ptr) + off, f, vec);
+        store(static_cast<float*>(out_ptr) + off, f, whole && p.vec_ok);
     }
 }
 
 // kDual, kX3: as in conv_tc.cu (second output through tmB2 / out2; high and low operand parts).
 template <MmaKind kKind, int BN, int kOutMode, bool kDual, bool kX3>
 __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __grid_constant__ TcParams p) {
-    using G = SplitGeom<BN, kX3>;
+    using G = SplitGeom<BN, kX3, kDual>;
     static_assert(!(kDual && kX3), "one of the two");
-    static_assert((kDual ? 2 : 1) * 128 * BN * 4 <= G::kStages * G::kStageBytes, "the partial sums reuse the operand ring");
     constexpr int kStages = G::kStages;
     constexpr uint32_t kTmemCols = (kDual || kX3 ? 2 : 1) * BN;
     constexpr uint32_t kFmt = kKind == MmaKind::F16 ? kFmtBF16 : kFmtTF32;
@@ -163,6 +220,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __g
     __shared__ __align__(8) uint64_t bar_full[kStages];
     __shared__ __align__(8) uint64_t bar_empty[kStages];
     __shared__ __align__(8) uint64_t bar_acc;
+    __shared__ __align__(8) uint64_t bar_recv;
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
@@ -172,6 +230,10 @@ __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __g
     const int rank = (int)cluster_cta_rank();
     const int S = p.split;
     const int tile = (int)blockIdx.x / S;
+    const int rows = (128 + S - 1) / S;  // of an owner; the last one may have fewer
+    const int my_rows = 128 - rank * rows < rows ? 128 - rank * rows : rows;
+    const int parts = S - 1 + (kDual ? 1 : 0);  // received per 32 columns: the other ranks' in order, the last rank's second output
+    const uint32_t recv = ring + (uint32_t)G::kRecvOffset;
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -180,7 +242,9 @@ __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __g
             mbar_init(smem_u32(&bar_empty[s]), 1);
         }
         mbar_init(smem_u32(&bar_acc), 1);
+        mbar_init(smem_u32(&bar_recv), 1);
         mbar_fence_init();
+        mbar_arrive_expect_tx(smem_u32(&bar_recv), (uint32_t)((rank == S - 1 ? S - 1 : parts) * my_rows * BN * 4));
     }
     if (warp == 1) {
         tmem_alloc(smem_u32(&tmem_base_slot), kTmemCols);
@@ -191,6 +255,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __g
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
     volatile int* abort_ptr = &abort_flag;
+    // First cluster barrier: every CTA's receive buffer and its mbarrier are ready. Arrived at here, or when the ring is idle.
+    if constexpr (G::kOwnBuffer) cluster_arrive();
     pdl_launch_dependents();
 
     const int kb_main = p.taps_h * p.taps_w * p.cblocks;
@@ -294,20 +360,33 @@ __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __g
             if (ok) umma_commit(smem_u32(&bar_acc));
         }
     } else {
-        // this CTA's partial sums into its ring: every load has landed and every MMA has read it once bar_acc completes
+        // this CTA's partial sums into its ring and on to the owners of their rows: every load has landed and every MMA has read it
+        // once bar_acc completes
         const int quad = warp & 3, half = (warp - 2) >> 2;
         const int row = quad * 32 + lane;
+        const int local = row % rows;
+        pdl_wait();  // residual reads and output writes must not overtake earlier kernels
         bool ok = mbar_wait_bounded(smem_u32(&bar_acc), 0, abort_ptr);
         ok = __all_sync(0xffffffffu, ok);
-        if (ok) {
-            tc_fence_after_sync();
+        if constexpr (!G::kOwnBuffer) cluster_arrive();
+        tc_fence_after_sync();
+        // lanes 0 to 2: the owners of the warp's rows, and the rows of them
+        const int owner = quad * 32 / rows + lane;
+        const int from = owner * rows > quad * 32 ? owner * rows : quad * 32;
+        const int upto = (owner + 1) * rows < quad * 32 + 32 ? (owner + 1) * rows : quad * 32 + 32;
+        const bool sends = lane < 3 && from < upto && from < 128 && owner != rank;
+        const uint32_t to = map_to_cta(recv, sends ? (uint32_t)owner : 0u), to_bar = map_to_cta(smem_u32(&bar_recv), sends ? (uint32_t)owner : 0u);
+        const int slot = rank < owner ? rank : rank - 1;  // of this rank among the owner's parts
+        bool ready = false;
 #pragma unroll 1
-            for (int a = 0; a < (kDual ? 2 : 1); ++a) {
-                if (a == 1 && rank != S - 1) continue;
+        for (int a = 0; a < (kDual ? 2 : 1); ++a) {
+            if (a == 1 && rank != S - 1) continue;
 #pragma unroll 1
-                for (int i = 0; i < BN / 64; ++i) {
-                    const int col = half * (BN / 2) + i * 32;
-                    const uint32_t t_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN + col);
+            for (int i = 0; i < BN / 64; ++i) {
+                const int cg = half * (BN / 64) + i;  // 32 columns
+                const uint32_t t_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN + cg * 32);
+                const uint32_t own = ring + (uint32_t)(a * G::kSumBytes + cg * 128 * 128);
+                if (ok) {
                     uint32_t v[32];
                     tmem_ld_32x32(t_addr, v);
                     if constexpr (kX3) {
@@ -321,74 +400,104 @@ __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __g
                     }
 #pragma unroll
                     for (int g = 0; g < 8; ++g)
-                        st_shared_v4(ring + (uint32_t)(a * 128 * BN * 4) + partial_off<BN>(row, (col >> 2) + g),
-                                     make_uint4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]));
+                        st_shared_v4(own + (uint32_t)(row * 128) + piece_off(local, g), make_uint4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]));
                 }
+                fence_proxy_async_shared();
+                __syncwarp();
+                if (!ready) cluster_wait();
+                ready = true;
+                if (ok && sends)
+                    bulk_copy_to_cta(to + (uint32_t)(((cg * parts + (a == 1 ? S - 1 : slot)) * rows + from - owner * rows) * 128),
+                                     own + (uint32_t)(from * 128), (uint32_t)((upto - from) * 128), to_bar);
+                __syncwarp();
             }
-            tc_fence_before_sync();
         }
+        tc_fence_before_sync();
     }
-    __syncwarp();
-    cluster_sync_all();  // the partial sums of all ranks are in place
-    // Every thread: one step per 8 channels of a pixel. The partial sums of a step are fetched together; a CTA's last fetch is
-    // followed by its arrival at the second barrier, so the epilogue's arithmetic and stores are not waited for by the others.
-    const bool live = warp >= 2 && !*abort_ptr;
-    if (live) pdl_wait();  // residual reads and output writes must not overtake earlier kernels
-    const int rows = (128 + S - 1) / S;
+    // Every thread: one item of 8 channels per step, its bias and residual fetched a step (or the exchange) ahead.
     constexpr int kPieces = BN / 8;
     const int box_hw = p.BH * p.BW;
-    const int items = rows * kPieces;
-    const int steps = (items * (kDual ? 2 : 1) + 255) / 256;
+    const int items = my_rows * kPieces;
+    auto item_of = [&](int step) {
+        Item it;
+        int idx = step * 256 + (int)threadIdx.x - 64;
+        it.mine = idx < items * (kDual ? 2 : 1);
+        it.second = kDual ? idx / items : 0;
+        idx -= it.second * items;
+        // neighbouring threads: neighbouring channels of a pixel (NHWC) or neighbouring pixels (NCHW)
+        it.piece = kOutMode == kOutNCHW_F32 ? idx / my_rows : idx % kPieces;
+        it.local = kOutMode == kOutNCHW_F32 ? idx % my_rows : idx / kPieces;
+        it.row = rank * rows + it.local;
+        const int n_l = it.row / box_hw;
+        const int rem = it.row - n_l * box_hw;
+        const int h_l = rem / p.BW;
+        it.n = n0 + n_l;
+        it.oh = oh0 + h_l;
+        it.ow = ow0 + rem - h_l * p.BW;
+        it.c0 = ct * BN + it.piece * 8;
+        it.mine = it.mine && it.row < rows_used && it.n < p.N && it.oh < p.OH && it.ow < p.OW && it.c0 < p.Cout;
+        return it;
+    };
+    auto fetch = [&](const Item& it, Ahead<kOutMode>& a) {
+        fetch_ahead<kOutMode>(p, it, kDual && it.second ? p.bias2 : p.bias, kDual && it.second ? nullptr : p.residual, a);
+    };
+    Item cur{};
+    Ahead<kOutMode> ahead{};
+    bool live = false;
+    if (warp >= 2) {
+        cur = item_of(0);
+        fetch(cur, ahead);
+        live = mbar_wait_bounded(smem_u32(&bar_recv), 0, abort_ptr);
+        asm volatile("fence.acq_rel.cluster;" ::: "memory");
+        live = !named_barrier_or(1, 256, !live);  // ... and the CTA's own sums are in place
+    } else {
+        __syncwarp();
+        if constexpr (!G::kOwnBuffer) cluster_arrive();
+        cluster_wait();
+    }
+    // Second cluster barrier: this CTA has what it waited for, or has given up. The epilogue's arithmetic and stores are not waited
+    // for by the others; nobody's shared memory goes while parts are read out of it or on their way to it.
+    __syncwarp();
+    cluster_arrive();
+    const int steps = live ? (items * (kDual ? 2 : 1) + 255) / 256 : 0;
 #pragma unroll 1
     for (int step = 0; step < steps; ++step) {
-        const int idx = step * 256 + (int)threadIdx.x - 64;
-        const int a = kDual ? idx / items : 0;
-        const int it = idx - a * items;
-        // neighbouring threads: neighbouring channels of a pixel (NHWC) or neighbouring pixels (NCHW)
-        const int piece = kOutMode == kOutNCHW_F32 ? it / rows : it % kPieces;
-        const int row = rank * rows + (kOutMode == kOutNCHW_F32 ? it % rows : it / kPieces);
-        const int n_l = row / box_hw;
-        const int rem = row - n_l * box_hw;
-        const int h_l = rem / p.BW;
-        const int n = n0 + n_l, oh = oh0 + h_l, ow = ow0 + rem - h_l * p.BW;
-        const int c0 = ct * BN + piece * 8;
-        const bool mine = live && idx < items * (kDual ? 2 : 1) && row < rows_used && n < p.N && oh < p.OH && ow < p.OW && c0 < p.Cout;
-        float f[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        if (mine) {
-            const uint32_t base = ring + (uint32_t)(a * 128 * BN * 4);
-            const uint32_t off0 = partial_off<BN>(row, 2 * piece), off1 = partial_off<BN>(row, 2 * piece + 1);
-            const int s_first = a == 1 ? S - 1 : 0;
-            float4 x[kMaxSplit], y[kMaxSplit];
-#pragma unroll
-            for (int s = 0; s < kMaxSplit; ++s) {
-                if (s < s_first || s >= S) continue;
-                x[s] = ld_cluster_f4(map_to_cta(base + off0, (uint32_t)s));
-                y[s] = ld_cluster_f4(map_to_cta(base + off1, (uint32_t)s));
-            }
-#pragma unroll
-            for (int s = 0; s < kMaxSplit; ++s) {
-                if (s < s_first || s >= S) continue;
-                f[0] += x[s].x; f[1] += x[s].y; f[2] += x[s].z; f[3] += x[s].w;
-                f[4] += y[s].x; f[5] += y[s].y; f[6] += y[s].z; f[7] += y[s].w;
+        const Item next = item_of(step + 1);
+        Ahead<kOutMode> next_ahead{};
+        fetch(next, next_ahead);
+        if (cur.mine) {
+            float f[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+            const int cg = cur.piece >> 2;
+            const uint32_t off0 = piece_off(cur.local, 2 * (cur.piece & 3)), off1 = piece_off(cur.local, 2 * (cur.piece & 3) + 1);
+            auto add = [&](uint32_t at) {
+                const uint4 x = ld_shared_v4(at + off0), y = ld_shared_v4(at + off1);
+                f[0] += __uint_as_float(x.x); f[1] += __uint_as_float(x.y); f[2] += __uint_as_float(x.z); f[3] += __uint_as_float(x.w);
+                f[4] += __uint_as_float(y.x); f[5] += __uint_as_float(y.y); f[6] += __uint_as_float(y.z); f[7] += __uint_as_float(y.w);
+            };
+            const uint32_t own = ring + (uint32_t)(cur.second * G::kSumBytes + (cg * 128 + cur.row) * 128);
+            const uint32_t got = recv + (uint32_t)((cg * parts * rows + cur.local) * 128);
+            if (kDual && cur.second) {
+                add(rank == S - 1 ? own : got + (uint32_t)((S - 1) * rows * 128));
+                epilogue8<kOutMode, false>(p, f, ahead, p.bias2 != nullptr, false, p.out2, p.relu2, cur);
+            } else {
+#pragma unroll 4
+                for (int s = 0; s < S; ++s) add(s == rank ? own : got + (uint32_t)((s < rank ? s : s - 1) * rows * 128));
+                epilogue8<kOutMode, kX3>(p, f, ahead, p.bias != nullptr, p.residual != nullptr, p.out, p.relu, cur);
             }
         }
-        if (step == steps - 1) {
-            __syncwarp();
-            cluster_arrive();
-        }
-        if (mine) {
-            if (kDual && a == 1)
-                epilogue8<kOutMode, false>(p, f, p.bias2, nullptr, p.out2, p.relu2, c0, n, oh, ow);
-            else
-                epilogue8<kOutMode, kX3>(p, f, p.bias, p.residual, p.out, p.relu, c0, n, oh, ow);
-        }
+        cur = next;
+        ahead = next_ahead;
     }
     if (*abort_ptr) {  // loads already issued may still be landing (see conv_tc.cu)
         const uint64_t t0 = global_timer_ns();
         while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
     }
     __syncwarp();
-    cluster_wait();  // no CTA's shared memory goes while another still reads it
+    cluster_wait();
+    if (*abort_ptr) {  // ... and so may parts that the others sent before they arrived
+        const uint64_t t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+    }
     tc_fence_after_sync();
     if (warp == 1) {
         __syncwarp();
@@ -399,7 +508,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __g
 
 template <MmaKind kKind, int BN, int kOutMode, bool kDual, bool kX3>
 int32_t launch_split(const TcParams& p, cudaStream_t s) {
-    using G = SplitGeom<BN, kX3>;
+    using G = SplitGeom<BN, kX3, kDual>;
+    if (p.split > G::kMaxParts) return fail(KXC_B200_ERR_INVALID, "split-reduction conv: %d parts of %d channels", p.split, BN);
     auto kernel = conv_splitk_kernel<kKind, BN, kOutMode, kDual, kX3>;
     static PerDeviceOnce smem_once;
     KXC_TRY(smem_opt_in(smem_once, kernel, G::kSmemBytes));

@@ -813,14 +813,18 @@ bool split_fits(long long tiles, int s, long long* late) {
 //   a K block of 128 bytes per row     550 / 590 / 500 / 620 at 64 / 128 / 192 / 256 channels, 650 at 256 in the split kernel;
 //                                      760 with two bf16 pixel tiles, 820 / 1100 with two tf32 ones; three passes 830 / 1050, split 830 / 930
 //   what follows the last K block      unsplit 0 / 2000 / 4000 / 8000 (the epilogue of that many channels), 2800 more with two pixel
-//                                      tiles; split 3000 / 7000 / 13000 (both cluster barriers, the exchange of the partial
-//                                      sums over distributed shared memory and the epilogue, all of which grow with the width);
+//                                      tiles; split 3000 / 5500 / 10000 (the exchange of the partial sums over distributed shared
+//                                      memory and the epilogue, which grow with the width; refitted over 170 layers when the
+//                                      exchange changed, 7000 / 13000 before: 0.1 % behind the fastest form, 0.5 with the old ones;
+//                                      tf32 512 -> 512 1x1 at 7x7, 32 images: 14.0 unsplit, 11.7 in two parts of 128 channels);
+//                                      7000 and 13000 still into the reference's layout, whose 4-byte stores weigh more (tf32 66
+//                                      channels 3x3 stride 2 at 23x22, 43 images: 16.4 unsplit, 18.4 split by the lower figures);
 //                                      4000 more into the reference's layout, for more than 64 channels, when the weights cannot
 //                                      be fetched ahead of the previous kernel's end (87 operator calls: 14 were slower than
 //                                      unsplit without it, tf32 42 -> 113 3x3 at 11x11, 30 images, 16.1 against 14.0 us; 5 with it;
 //                                      427 -> 36 1x1 at 8x7, 7 images, 11.6 split, 12.4 unsplit)
-// Over the same launches what this chooses is 0.3 % (NHWC) and 1.4 % (NCHW) behind the fastest form on average, and one launch
-// is behind the unsplit one by more than 1 %. (One figure for every width, 3000, made wide splits of short reductions slower than no split: bf16
+// Into NCHW what this chooses was 1.4 % behind the fastest form on average, and one launch behind the unsplit one by more than
+// 1 %. (One figure for every width, 3000, made wide splits of short reductions slower than no split: bf16
 // 1024 -> 1024 1x1 at 7x7 and 24 images 14.7 us per layer in two parts of 256 channels, 11.3 unsplit; 256 -> 256 3x3 at
 // 14x14 and 32 images 19.4 and 17.8.) A launch is kept to the clusters that the chip holds at once (split_fits; a dense
 // layer of 16 tiles in clusters of eight that did not all fit: 8.8 -> 12 us).
@@ -838,13 +842,14 @@ int32_t choose_split(TcParams* p, TcConfig* cfg, const void* w, const void* w_lo
     const long long group = (long long)cfg->ctas * cfg->mt;
     const long long items = p->tiles_c * ((m_tiles + group - 1) / group), slots = kNumSMs / cfg->ctas;
     long long best = ((items + slots - 1) / slots * kb * block + tail) * 95 / 100;
-    const long long cold = cfg->out_mode == kOutNCHW_F32 && !p->weights_ready && p->Cout > 64 ? 4000 : 0;
+    const bool nchw = cfg->out_mode == kOutNCHW_F32;
+    const long long cold = nchw && !p->weights_ready && p->Cout > 64 ? 4000 : 0;
     int split = 0, width = 0;
     for (int bn = 64; bn <= 256 && (bn == 64 || bn / 2 < p->Cout) && !(bn == 256 && cfg->x3); bn *= 2) {
         const long long tiles = m_tiles * ((p->Cout + bn - 1) / bn);
         const long long split_block = cfg->x3 ? (bn == 64 ? 830 : 930) : (bn == 64 ? 550 : (bn == 128 ? 590 : 650));
-        const long long split_tail = bn == 64 ? 3000 : (bn == 128 ? 7000 : 13000);
-        for (int s = 2; s <= kMaxSplit; ++s) {
+        const long long split_tail = bn == 64 ? 3000 : (nchw ? (bn == 128 ? 7000 : 13000) : (bn == 128 ? 5500 : 10000));
+        for (int s = 2; s <= (bn == 256 ? 4 : kMaxSplit); ++s) {  // (what shared memory holds of the parts)
             long long late = 0;
             if (!split_fits(tiles, s, &late)) continue;
             const long long span = (long long)((kb + s - 1) / s) * split_block + split_tail + cold + late;
