@@ -118,6 +118,10 @@ def check(name, rc):
         raise KxcError(name, rc, last_error())
 
 
+_PACKED_TYPES = [ctypes.c_void_p * n for n in range(9)]
+
+
 def packed(*ptrs):
     """void** packed_args from raw addresses."""
-    return (ctypes.c_void_p * len(ptrs))(*ptrs)
+    n = len(ptrs)
+    return (_PACKED_TYPES[n] if n < 9 else ctypes.c_void_p * n)(*ptrs)

@@ -645,28 +645,42 @@ int32_t tc_launch(const TcConfig& cfg, const TcParams& p, cudaStream_t stream) {
     return fail(KXC_B200_ERR_INVALID, "tensor-core conv: unknown dtype");
 }
 
-void tc_pick_tile(int N, int OH, int OW, int* BW, int* BH, int* BNI) {
-    double best = -1.0;
-    int bw_best = 1, bh_best = 1, bn_best = 1;
-    for (int bw = 1; bw <= OW && bw <= 128; ++bw) {
-        for (int bh = 1; bh <= OH && bw * bh <= 128; ++bh) {
-            int bn = 128 / (bw * bh);
+namespace {
+// What the two searches over tile boxes look up instead of dividing in every one of up to 620 boxes (an operator call spent 2 to
+// 7 us of host time on them): tiles over the rows by box height, and images per box and tiles over the images by box area.
+struct BoxTables {
+    int tiles_h[129], bni[129], tiles_n[129];
+    BoxTables(int N, int OH) {
+        for (int bh = 1; bh <= 128 && bh <= OH; ++bh) tiles_h[bh] = (OH + bh - 1) / bh;
+        for (int area = 1; area <= 128; ++area) {
+            int bn = 128 / area;
             if (bn > N) bn = N;
-            if (bn > 128) bn = 128;
             if (bn < 1) bn = 1;
-            const long long tiles = (long long)((OW + bw - 1) / bw) * ((OH + bh - 1) / bh) * ((N + bn - 1) / bn);
-            const double eff = (double)N * OH * OW / ((double)tiles * 128.0);
-            // prefer higher efficiency; on ties the box with the most pixels per image (neighbouring filter
-            // taps of one tile then re-read the same cache lines), then the squarer one (smaller halo)
-            const int area = bw * bh, area_best = bw_best * bh_best;
-            const int skew = bw > bh ? bw - bh : bh - bw, skew_best = bw_best > bh_best ? bw_best - bh_best : bh_best - bw_best;
-            if (eff > best + 1e-9 || (eff > best - 1e-9 && (area > area_best || (area == area_best && skew < skew_best)))) {
-                best = eff;
-                bw_best = bw; bh_best = bh; bn_best = bn;
+            bni[area] = bn;
+            tiles_n[area] = (N + bn - 1) / bn;
+        }
+    }
+};
+}  // namespace
+
+void tc_pick_tile(int N, int OH, int OW, int* BW, int* BH, int* BNI) {
+    const BoxTables tables(N, OH);
+    long long best = -1;
+    int bw_best = 1, bh_best = 1, area_best = 0, skew_best = 0;
+    for (int bw = 1; bw <= OW && bw <= 128; ++bw) {
+        const long long tiles_w = (OW + bw - 1) / bw;
+        for (int bh = 1, area = bw; bh <= OH && area <= 128; ++bh, area += bw) {
+            const long long tiles = tiles_w * tables.tiles_h[bh] * tables.tiles_n[area];
+            // prefer fewer tiles, i.e. more of the 128 rows in use; on ties the box with the most pixels per image (neighbouring
+            // filter taps of one tile then re-read the same cache lines), then the squarer one (smaller halo)
+            const int skew = bw > bh ? bw - bh : bh - bw;
+            if (best < 0 || tiles < best || (tiles == best && (area > area_best || (area == area_best && skew < skew_best)))) {
+                best = tiles;
+                bw_best = bw; bh_best = bh; area_best = area; skew_best = skew;
             }
         }
     }
-    *BW = bw_best; *BH = bh_best; *BNI = bn_best;
+    *BW = bw_best; *BH = bh_best; *BNI = tables.bni[bw_best * bh_best];
 }
 
 int32_t tc_make_tmap(CUtensorMap* out, TcDType dtype, int rank, void* base, const uint64_t* dims,
@@ -765,24 +779,29 @@ void pick_tile_nchw(int N, int OH, int OW, int Cout, int num_kb, int kb_bytes, i
     const int bn_out = Cout <= 64 ? 64 : (Cout <= 128 ? 128 : 256);
     const int tiles_c = (Cout + bn_out - 1) / bn_out;
     const double main_loop = (double)num_kb * kb_bytes / 128.0 * (bn_out == 64 ? 550 : (bn_out == 128 ? 590 : 620));  // (choose_split's figures)
+    const BoxTables tables(N, OH);
     double best = -1.0;
     for (int bw = 1; bw <= OW && bw <= 128; ++bw) {
-        for (int bh = 1; bh <= OH && bw * bh <= 128; ++bh) {
-            int bn = 128 / (bw * bh);
-            if (bn > N) bn = N;
-            if (bn < 1) bn = 1;
-            const long long tiles = (long long)((OW + bw - 1) / bw) * ((OH + bh - 1) / bh) * ((N + bn - 1) / bn);
+        const long long tiles_w = (OW + bw - 1) / bw;
+        int run = 0;
+        double epilogue = 0.0, slower = 0.0, once = 0.0;
+        for (int bh = 1, area = bw; bh <= OH && area <= 128; ++bh, area += bw) {
+            const long long tiles = tiles_w * tables.tiles_h[bh] * tables.tiles_n[area];
             const long long waves = (tiles * tiles_c + kNumSMs - 1) / kNumSMs;
-            int run = bw == OW ? bw * bh : bw;
-            if (run > 32) run = 32;
-            const double sectors = 32.0 * (run / 8.0 + 0.9) / run;
-            const double epilogue = bn_out * (12.0 * sectors > 80.0 ? 12.0 * sectors : 80.0);
-            const double slower = main_loop > epilogue ? main_loop : epilogue;
+            int r = bw == OW ? area : bw;
+            if (r > 32) r = 32;
+            if (r != run) {
+                run = r;
+                const double sectors = 32.0 * (run / 8.0 + 0.9) / run;
+                epilogue = bn_out * (12.0 * sectors > 80.0 ? 12.0 * sectors : 80.0);
+                slower = main_loop > epilogue ? main_loop : epilogue;
+                once = 10.0 * sectors;
+            }
             // (tie-breakers: longer runs, then fewer tiles on the same number of waves)
-            const double cost = main_loop + (double)(waves - 1) * slower + epilogue + 10.0 * sectors + 1e-3 * (double)tiles;
+            const double cost = main_loop + (double)(waves - 1) * slower + epilogue + once + 1e-3 * (double)tiles;
             if (best < 0.0 || cost < best) {
                 best = cost;
-                *BW = bw; *BH = bh; *BNI = bn;
+                *BW = bw; *BH = bh; *BNI = tables.bni[area];
             }
         }
     }

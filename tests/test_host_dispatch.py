@@ -249,3 +249,44 @@ def test_nchw_boxes_keep_long_runs_where_stores_would_outlast_the_main_loop(comp
                       relay.Conv2DAttrs((1, 1), (1, 1, 1, 1), (1, 1), 1))
     graph, _ = compile_graph(relay.Function([x], relay.Call("nn_relu", [call])), "tf32")
     assert "x37 " in graph.launch_info()[-1][0], graph.launch_info()[-1][0]
+
+
+def test_geometries_are_remembered_by_value():
+    """Descriptors kept per shape and attributes (ops._per_geometry): lists and tuples are the same key, every attribute is part of
+    it, a refused geometry is refused again, and one that was written to by its user would show in the next call."""
+    from hdkx_aicompiler_b200 import ops
+    shapes = torch.Size((2, 3, 9, 8)), torch.Size((5, 3, 3, 3))
+    key = lambda *v: tuple(ops._key(e) for e in v)
+    seen = set()
+    for strides, padding, dilation, flags, precision in [([1, 1], (1, 1), (1, 1), 0, "tf32"), ((1, 1), [np.int64(1), 1.0], (1, 1), 0, "tf32"),
+                                                         ((2, 1), (1, 1), (1, 1), 0, "tf32"), ((1, 1), (0, 1), (1, 1), 0, "tf32"),
+                                                         ((1, 1), (1, 1), (2, 1), 0, "tf32"), ((1, 1), (1, 1), (1, 1), 1, "tf32"),
+                                                         ((1, 1), (1, 1), (1, 1), 0, "bf16"), (None, None, None, 0, "tf32")]:
+        desc, out, bias = ops._conv2d_geometry(*shapes, 1, *key(strides, padding, dilation), flags, precision)
+        sh, sw = ops._pair(strides, 1)
+        ph, pw = ops._pair(padding, 0)
+        dh, dw = ops._pair(dilation, 1)
+        assert [getattr(desc, f[0]) for f in desc._fields_] == [2, 3, 9, 8, 5, 3, 3, sh, sw, ph, pw, dh, dw, flags, ops.PRECISIONS[precision]]
+        assert tuple(out) == (2, 5, ops.conv_out_dim(9, 3, sh, ph, dh), ops.conv_out_dim(8, 3, sw, pw, dw)) and tuple(bias) == (5,)
+        seen.add(id(desc))
+    assert len(seen) == 7
+    for _ in range(2):
+        with pytest.raises(ValueError):
+            ops._conv2d_geometry(torch.Size((2, 4, 9, 8)), shapes[1], 1, None, None, None, 0, "tf32")
+    small = ops._pool_geometry(shapes[0], (3, 3), (2, 2), (1, 1, 1, 1), False, "p")
+    assert ops._pool_geometry(shapes[0], (3, 3), (2, 2), (1, 1), False, "p")[1] == small[1] == (2, 3, 5, 4)
+    assert ops._pool_geometry(shapes[0], (2, 3), (2, 2), (1, 0, 0, 0), True, "p")[1] == (2, 3, 5, 4)
+
+
+# Tile boxes are found with look-ups instead of divisions; what they are has not changed: the box with the fewest tiles, of those the
+# one with the most pixels, of those the squarest
+@pytest.mark.parametrize("n,oh,ow", [(1, 1, 1), (1, 7, 7), (3, 5, 200), (2, 300, 3), (129, 13, 15), (1024, 56, 56), (70000, 1, 1)])
+def test_tile_box_search(fake, n, oh, ow):
+    best = min((-(-ow // bw) * -(-oh // bh) * -(-n // max(1, min(128 // (bw * bh), n))), -bw * bh, abs(bw - bh), bw, bh)
+               for bw in range(1, min(ow, 128) + 1) for bh in range(1, min(oh, 128 // bw) + 1))
+    box = [ctypes.c_int(0) for _ in range(3)]
+    pick = getattr(fake, "_ZN8kxc_b20012tc_pick_tileEiiiPiS0_S0_")
+    pick.restype, pick.argtypes = None, [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_int)] * 3
+    pick(n, oh, ow, *[ctypes.byref(b) for b in box])
+    bw, bh, bni = (b.value for b in box)
+    assert (bw, bh, bni) == (best[3], best[4], max(1, min(128 // (bw * bh), n)))
