@@ -135,6 +135,48 @@ __device__ __forceinline__ void residual_fetch_nchw(const TcParams& p, int c0, b
     for (int j = 0; j < 32; ++j) res[j] = valid && c0 + j < p.Cout ? __ldg(src + (size_t)j * plane) : 0.0f;
 }
 
+// The reference's layout, results of less than 4 GiB: one chunk of a pixel by 32-bit byte offsets from the tensors' bases, the bias
+// from shared memory. `off` is the pixel's place in the chunk's first channel, `step` the bytes of a plane, `nch` the chunk's
+// channels. (64-bit addresses, a bound check per channel and per-channel bias loads made ~800 instructions of a chunk, and the eight
+// epilogue warps bound whole launches. us per launch before / now: 72 -> 120 3x3 at 45x51, 9 images, tf32 23.4 / 19.1, with a residual
+// 26.3 / 23.3; 95 -> 120 1x1 at 33x36, 50 images 21.3 / 12.9, 30.4 / 25.0; 64 -> 256 1x1 at 56x56, 20 images, bf16 35.1 / 25.3. All of a
+// tile's residual values in flight at once spilled registers (43 us for the second), the next tile's first ones fetched before a
+// tile ends changed nothing, other cache hints neither.)
+__device__ __forceinline__ void nchw_fetch32(const char* residual, uint32_t off, uint32_t step, int nch, float (&res)[32]) {
+    if (nch >= 32) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j, off += step) res[j] = __ldg(reinterpret_cast<const float*>(residual + off));
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j, off += step)
+            if (j < nch) res[j] = __ldg(reinterpret_cast<const float*>(residual + off));
+    }
+}
+template <bool kPart>
+__device__ __forceinline__ void nchw_store32_part(char* out, uint32_t off, uint32_t step, int nch, const uint32_t (&v)[32], uint32_t bias_smem,
+                                                  bool has_bias, const float (&res)[32], bool has_res, bool relu) {
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+        if (kPart && 4 * g >= nch) break;
+        float b[4];
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(b[3]) : "r"(bias_smem + 16u * g));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float x = __uint_as_float(v[4 * g + k]);
+            if (has_bias) x = __fadd_rn(x, b[k]);
+            if (has_res) x = __fadd_rn(x, res[4 * g + k]);
+            if (relu) x = fmaxf(x, 0.0f);  // (NaN and -0 give 0, as x > 0 ? x : 0 does)
+            if (!kPart || 4 * g + k < nch) *reinterpret_cast<float*>(out + off) = x;
+            off += step;
+        }
+    }
+}
+__device__ __forceinline__ void nchw_store32(char* out, uint32_t off, uint32_t step, int nch, const uint32_t (&v)[32], uint32_t bias_smem,
+                                             bool has_bias, const float (&res)[32], bool has_res, bool relu) {
+    if (nch >= 32) nchw_store32_part<false>(out, off, step, nch, v, bias_smem, has_bias, res, has_res, relu);
+    else nchw_store32_part<true>(out, off, step, nch, v, bias_smem, has_bias, res, has_res, relu);
+}
+
 // Epilogue for one 32-column chunk held by one thread (= one output pixel, 32 consecutive channels).
 // kSplit (three-pass tf32): the result may also leave as its tf32 high and low parts (TcParams::out_hi).
 // `nchw_res`: what residual_fetch_nchw read (kOutNCHW_F32 with a residual only).

@@ -34,7 +34,7 @@ constexpr int kTcThreads = 320;  // 2 control warps + 8 epilogue warps
 constexpr int kStoreBoxBytes = 32 * 128;
 constexpr int kSmemLimit = 227 * 1024;
 
-template <int KB_BYTES, int BN, int kCtas, int kMT = 1, bool kX3 = false>
+template <int KB_BYTES, int BN, int kCtas, int kMT = 1, bool kX3 = false, bool kNchw = false>
 struct StageGeom {
     static constexpr int kATileBytes = 128 * KB_BYTES;
     static constexpr int kABytes = (kX3 ? 2 : kMT) * kATileBytes;  // kMT pixel tiles share one B tile; x3: high, low part
@@ -43,7 +43,8 @@ struct StageGeom {
     static constexpr int kStageBytes = kABytes + kBBytes;
     // per epilogue warp a 4 KiB box (32 pixels x 64 channels, SWIZZLE_128B) that TMA stores read; its first half
     // doubles as the staging tile of the per-thread store path
-    static constexpr int kEpilogueBytes = kX3 ? 0 : 8 * kStoreBoxBytes;
+    // (or, into the reference's layout, holds the bias; the three-pass kernels have no other use for it)
+    static constexpr int kEpilogueBytes = kX3 ? (kNchw ? kStoreBoxBytes : 0) : 8 * kStoreBoxBytes;
     static constexpr int kStagesRaw = (kSmemLimit - 2048 - kEpilogueBytes) / kStageBytes;
     static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
     static constexpr int kSmemBytes = kStages * kStageBytes + kEpilogueBytes + 1024;  // + slack to align the ring to 1024 B
@@ -71,7 +72,7 @@ struct StageGeom {
 // is ~950 (BN 64) or ~1400 cycles (BN 128), just above the ~50 B/clk at which an SM's stage (48 / 64 KB) arrives.
 template <MmaKind kKind, int KB_BYTES, int BN, int kOutMode, int kCtas, bool kDual = false, int kMT = 1, bool kX3 = false>
 __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_constant__ TcParams p) {
-    using G = StageGeom<KB_BYTES, BN, kCtas, kMT, kX3>;
+    using G = StageGeom<KB_BYTES, BN, kCtas, kMT, kX3, kOutMode == kOutNCHW_F32>;
     static_assert(!(kDual && kMT != 1), "the two-output kernel works on one pixel tile at a time");
     static_assert(!kX3 || (kKind == MmaKind::TF32 && kCtas == 1 && !kDual && kMT == 1 && BN <= 128), "three-pass form: tf32, single CTAs");
     constexpr bool kPair = kCtas == 2;
@@ -331,6 +332,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                 if (*(volatile int*)&requant_ok) q_tab = tab;
             }
         }
+        // The reference's layout: the bias in shared memory (the store boxes are not used here either), padded to whole tiles
+        [[maybe_unused]] const uint32_t bias_tab = ring + (uint32_t)(kStages * G::kStageBytes);
+        [[maybe_unused]] bool small_nchw = false;  // nchw_store32's conditions
+        if constexpr (kOutMode == kOutNCHW_F32) {
+            const int padded = p.tiles_c * BN;
+            small_nchw = padded * 4 <= G::kEpilogueBytes && (unsigned long long)p.N * p.Cout * p.OH * p.OW < (1ull << 30);
+            if (small_nchw) {
+                float* tab = reinterpret_cast<float*>(smem_raw + (bias_tab - smem_u32(smem_raw)));
+                for (int c = (int)threadIdx.x - 64; c < padded; c += 256) tab[c] = p.bias != nullptr && c < p.Cout ? __ldg(p.bias + c) : 0.0f;
+                named_barrier(1, 256);
+            }
+        }
         int acc = 0;
         uint32_t acc_phase = 0;
         bool alive = true;
@@ -350,8 +363,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
             const int c_base = ct * BN + col0;
             uint4 res_cur[4] = {};
             float nchw_cur[32] = {}, nchw_next[32] = {};  // kOutNCHW_F32 only
+            [[maybe_unused]] const uint32_t nchw_step = (uint32_t)(p.OH * p.OW) * 4u;
+            [[maybe_unused]] const uint32_t nchw_off = small_nchw ? (uint32_t)(n * p.Cout + c_base) * nchw_step + (uint32_t)(oh * p.OW + ow) * 4u : 0u;
             if constexpr (kOutMode == kOutNCHW_F32) {
-                if (has_res && c_base < p.Cout) residual_fetch_nchw(p, c_base, valid, n, oh, ow, nchw_cur);
+                if (has_res && c_base < p.Cout) {
+                    if (!small_nchw) residual_fetch_nchw(p, c_base, valid, n, oh, ow, nchw_cur);
+                    else if (valid) nchw_fetch32(static_cast<const char*>(p.residual), nchw_off, nchw_step, p.Cout - c_base, nchw_cur);
+                }
             }
             RowMap rows;
             if (fast && !boxed) {
@@ -368,6 +386,34 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                 tc_fence_after_sync();
             }
             const uint32_t t_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * kAccCols + t * BN + col0);
+            if (kOutMode == kOutNCHW_F32 && small_nchw) {
+                if constexpr (kOutMode == kOutNCHW_F32) {
+                    // unrolled: the two chunks of residual values in flight then need not be moved
+#pragma unroll
+                    for (int i = 0; i < kChunksPerWarp; ++i) {
+                        const int c0 = c_base + i * 32;
+                        if (c0 >= p.Cout) break;
+                        uint32_t v[32];
+                        tmem_ld_32x32(t_addr + (uint32_t)(i * 32), v);
+                        float(&res)[32] = i & 1 ? nchw_next : nchw_cur;
+                        float(&res_ahead)[32] = i & 1 ? nchw_cur : nchw_next;
+                        if (has_res && valid && i + 1 < kChunksPerWarp && c0 + 32 < p.Cout)
+                            nchw_fetch32(static_cast<const char*>(p.residual), nchw_off + (uint32_t)(i + 1) * 32u * nchw_step, nchw_step, p.Cout - c0 - 32, res_ahead);
+                        if constexpr (kX3) {
+                            uint32_t u[32];
+                            tmem_ld_32x32(t_addr + (uint32_t)(BN + i * 32), u);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j])));
+                        }
+                        tmem_ld_wait();
+                        if (valid)
+                            nchw_store32(static_cast<char*>(p.out), nchw_off + (uint32_t)i * 32u * nchw_step, nchw_step, p.Cout - c0, v,
+                                         bias_tab + (uint32_t)c0 * 4u, p.bias != nullptr, res, has_res, p.relu != 0);
+                        __syncwarp();
+                    }
+                }
+            } else
 #pragma unroll 1
             for (int i = 0; i < kChunksPerWarp; ++i) {
                 const int c0 = c_base + i * 32;
@@ -496,7 +542,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
 
 template <MmaKind kKind, int KB_BYTES, int BN, int kOutMode, int kCtas, bool kDual = false, int kMT = 1, bool kX3 = false>
 int32_t launch_one(const TcParams& p, cudaStream_t stream) {
-    using G = StageGeom<KB_BYTES, BN, kCtas, kMT, kX3>;
+    using G = StageGeom<KB_BYTES, BN, kCtas, kMT, kX3, kOutMode == kOutNCHW_F32>;
     auto kernel = conv_igemm_kernel<kKind, KB_BYTES, BN, kOutMode, kCtas, kDual, kMT, kX3>;
     static PerDeviceOnce smem_once;
     static std::mutex units_mu;

@@ -250,6 +250,24 @@ def test_conv2d_argument_errors(ops):
         ops.nn_conv2d(x, torch.zeros(2, 3, 1, 1, device="cuda"))
 
 
+# More channels than the bias table in shared memory holds (64-bit epilogue); whole and partial chunks either side of a tile in the other
+# form, with and without bias and residual, -0 and NaN sums. Bound: that of test_conv2d_tensor_core.
+@pytest.mark.parametrize("precision,rounder", [("tf32", port.round_tf32), ("tf32x3", None)])
+@pytest.mark.parametrize("O", [31, 64, 97, 8250])
+def test_conv2d_nchw_epilogues(ops, rng, O, precision, rounder):
+    x, w, b = conv_inputs(rng, 2, 8, 9, 7, O, 1, 1)
+    x[1, :, 3, 3], w[0] = -0.0, np.abs(w[0])
+    x[0, 2, 1, 1] = np.nan
+    res = rng.uniform(-1, 1, (2, O, 9, 7)).astype(f32)
+    for bias, r, relu in [(None, None, False), (b, None, True), (b, res, True), (None, res, False)]:
+        got = host(ops.nn_conv2d(dev(x), dev(w), None if bias is None else dev(bias), residual=None if r is None else dev(r), relu=relu, precision=precision))
+        assert ops.device_status() == 0
+        exp = conv_expect(x, w, bias, r, relu, 1, 0, 1, rounder)
+        assert np.array_equal(np.isnan(got), np.isnan(exp))
+        max_abs, max_rel = ref_metric(np.nan_to_num(got), np.nan_to_num(exp))
+        assert min(max_abs, max_rel) <= (1e-4 if rounder is None else 2e-5), f"{precision} {O}: {max_abs:.3e} {max_rel:.3e}"
+
+
 # Two pixel tiles per work item (more than one wave of tf32 tiles, 64 and 128 channels), an odd number of tiles, full-row boxes in
 # the reference's layout and a residual read ahead of the accumulator. Bound: that of test_conv2d_tensor_core.
 @pytest.mark.parametrize("O", [64, 100])
