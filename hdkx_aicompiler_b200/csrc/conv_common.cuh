@@ -44,6 +44,9 @@ int32_t conv2d_tensor_core(const float* data, const float* weight, const float* 
                            const ConvDims& d, int relu, int precision, cudaStream_t s);
 int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32_t* bias, const int32_t* multiplier,
                            const int32_t* shift, int8_t* out, const ConvDims& d, int relu, int force_simt, int nhwc, cudaStream_t s);
+// gemm_small.cu: tf32 / bf16 dense layers of few tiles in one launch (has_c with alpha = beta = 1, or no c)
+bool gemm_small_applicable(const float* a, const float* b, const float* out, const kxc_b200_gemm_desc& g);
+int32_t gemm_small(const float* a, const float* b, const float* c, float* out, const kxc_b200_gemm_desc& g, cudaStream_t s);
 int32_t gemm_tensor_core(const float* a, const float* b, const float* c, float* out, const kxc_b200_gemm_desc& g,
                          cudaStream_t s);
 

@@ -261,6 +261,7 @@ int32_t gemm_tensor_core(const float* a, const float* b, const float* c, float* 
     // alpha = beta = 1 form is fused into the tensor-core epilogue.
     if ((g.has_c && ((double)g.alpha != 1.0 || (double)g.beta != 1.0)) || g.m > 65535 * 128)
         return gemm_fp32_exact(a, b, c, out, g, s);
+    if (gemm_small_applicable(a, b, out, g)) return gemm_small(a, b, g.has_c ? c : nullptr, out, g, s);
     if (g.precision == KXC_B200_PREC_TF32X3) {
         const int kpad = tc_channel_pad(kTcTF32, g.k);
         const size_t a_elems = (size_t)g.m * kpad;  // the low part of A follows its high part at once (tc_setup_conv_x3)

@@ -425,6 +425,43 @@ def test_gemm_tensor_core(ops, rng, M, N, K, precision, tol, rounder):
     assert ops.device_status() == 0
 
 
+# The one-launch kernel for few tiles: edges of its 32 x 16 tiles, k that ends inside a warp's part, a vector, a pass; a second pass of
+# one and of 512; rows that are not 16-byte aligned (odd k, an offset base); and the sizes either side of its rule, where the
+# tensor-core path begins (300 tiles, 152 for two passes; k = 1025). Bound: that of test_gemm_tensor_core; the sums themselves are fp32.
+@pytest.mark.parametrize("precision,rounder", [("tf32", port.round_tf32), ("bf16", port.round_bf16)])
+@pytest.mark.parametrize("M,N,K,offset", [(1, 1, 1, 0), (32, 16, 64, 0), (33, 17, 65, 0), (31, 47, 511, 0), (40, 15, 512, 1), (7, 30, 513, 0),
+                                          (65, 33, 1024, 0), (3, 1000, 96, 1), (128, 1184, 20, 0), (128, 1185, 20, 0), (20, 40, 1025, 0), (97, 590, 520, 0), (97, 600, 520, 0)])
+def test_gemm_few_tiles(ops, rng, M, N, K, offset, precision, rounder):
+    a = rng.normal(size=(M, K)).astype(f32)
+    b = rng.normal(0, np.sqrt(2.0 / K), (N, K)).astype(f32)
+    c = rng.normal(size=N).astype(f32)
+    a_dev = torch.zeros(M * K + offset, device="cuda")[offset:].view(M, K).copy_(dev(a))
+    exact = rounder(a).astype(np.float64) @ rounder(b).astype(np.float64).T
+    for got, exp in [(ops.nn_gemm(a_dev, dev(b), dev(c), transB=1, precision=precision), exact + c), (ops.nn_dense(a_dev, dev(b), precision=precision), exact)]:
+        assert ops.device_status() == 0
+        err = np.abs(host(got) - exp) / np.maximum(1.0, np.abs(exp))
+        assert err.max() <= 2e-5 * max(1.0, np.sqrt(K) / 8), f"{precision} {M}x{N}x{K}: {err.max():.3e}"
+
+
+# The result over an operand: the one-launch kernel reads the operands while it stores, so the call takes the path that converts them first.
+def test_gemm_result_over_an_operand(ops, rng):
+    from hdkx_aicompiler_b200._lib import check, load, packed
+    a, b = rng.normal(size=(70, 48)).astype(f32), rng.normal(size=(48, 48)).astype(f32)
+    expect = host(ops.nn_dense(dev(a), dev(b)))
+    x, w = dev(a), dev(b)
+    desc = ops._gemm_desc(70, 48, 48, 1.0, 1.0, 0, 1, 0, ops.PRECISIONS["tf32"])
+    check("nn_dense", load().kxc_b200_nn_gemm(packed(x.data_ptr(), w.data_ptr(), x.data_ptr()), desc, torch.cuda.current_stream().cuda_stream))
+    got = host(x)[:, :48]
+    assert (np.abs(got - expect) / np.maximum(1.0, np.abs(expect))).max() <= 4e-5  # the bound above, once for each path
+
+
+@pytest.mark.parametrize("n,offset", [(1, 0), (1023, 0), (4099, 0), (4099, 1), (1 << 20, 0), ((1 << 20) + 1, 0)])
+def test_flatten_sizes(ops, rng, n, offset):
+    x = rng.normal(size=n).astype(f32)
+    got = ops.nn_flatten(torch.zeros(n + offset, device="cuda")[offset:].copy_(dev(x)).view(1, n, 1))
+    assert_bit_exact(host(got), x.reshape(1, n), f"flatten {n}")
+
+
 def test_gemm_transA_rejected(ops):
     from hdkx_aicompiler_b200 import KxcError
     z = torch.zeros(2, 2, device="cuda")
