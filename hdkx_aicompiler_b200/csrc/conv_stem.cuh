@@ -25,7 +25,8 @@ int32_t stem_pool_launch(const TcParams& p, cudaStream_t stream);
 
 // conv_stem_fused.cu: the same convolution + bias + ReLU + max_pool2d(3x3, s2, p1), reading the NCHW fp32 graph
 // input directly (the packed layout exists only in shared memory) and issuing row-stacked MMAs. `p.aux_in` is the
-// fp32 input (bound at run time), `p.out` the pooled bf16 NHWC tensor. Bit-identical to stem_pool_launch.
+// fp32 input (bound at run time), `p.out` the pooled NHWC tensor (bf16, or fp32 holding tf32 values). The bf16 form is
+// bit-identical to stem_pool_launch, the tf32 form to the implicit-GEMM stem and its pooling.
 bool stem_pool_nchw_applicable(TcDType dtype, int C, int O, int KH, int KW, int W, int OH, int OW, int Wp);
 size_t stem_stacked_weight_bytes(TcDType dtype);
 // OIHW fp32 -> filter rows stacked by parity in core-matrix order
