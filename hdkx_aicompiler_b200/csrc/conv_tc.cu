@@ -369,6 +369,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                 if (has_res && c_base < p.Cout) {
                     if (!small_nchw) residual_fetch_nchw(p, c_base, valid, n, oh, ow, nchw_cur);
                     else if (valid) nchw_fetch32(static_cast<const char*>(p.residual), nchw_off, nchw_step, p.Cout - c_base, nchw_cur);
+                    __syncwarp();  // (lanes beyond the image's edge skipped the loads; the reads of tensor memory want the whole warp)
                 }
             }
             RowMap rows;
@@ -399,6 +400,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                         float(&res_ahead)[32] = i & 1 ? nchw_cur : nchw_next;
                         if (has_res && valid && i + 1 < kChunksPerWarp && c0 + 32 < p.Cout)
                             nchw_fetch32(static_cast<const char*>(p.residual), nchw_off + (uint32_t)(i + 1) * 32u * nchw_step, nchw_step, p.Cout - c0 - 32, res_ahead);
+                        __syncwarp();
                         if constexpr (kX3) {
                             uint32_t u[32];
                             tmem_ld_32x32(t_addr + (uint32_t)(BN + i * 32), u);

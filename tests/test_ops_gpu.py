@@ -337,6 +337,22 @@ def test_conv2d_nchw_boxes(ops, rng, case, precision, rounder):
     assert min(max_abs, max_rel) <= bound, f"{precision} {case}: {max_abs:.3e} {max_rel:.3e}"
 
 
+# Boxes whose warps reach over the image's edge (lanes without a pixel skip the residual's loads and meet the others again before the
+# accumulator is read): two chunks of channels per warp and their second parts, two pixel tiles per item with a ragged one behind.
+# Bounds: that of test_conv2d_tensor_core, and 1e-4 for three passes.
+@pytest.mark.parametrize("precision,rounder,case", [("tf32x3", None, (2, 16, 11, 13, 130, 3)), ("tf32x3", None, (3, 32, 5, 131, 100, 1)),
+                                                    ("tf32", port.round_tf32, (9, 40, 45, 51, 100, 1)), ("bf16", port.round_bf16, (7, 64, 45, 51, 200, 1))])
+def test_conv2d_nchw_residual_beyond_the_edge(ops, rng, case, precision, rounder):
+    N, C, H, W, O, k = case
+    x, w, b = conv_inputs(rng, N, C, H, W, O, k, k)
+    res = rng.uniform(-1, 1, (N, O, H, W)).astype(f32)
+    got = host(ops.nn_conv2d(dev(x), dev(w), dev(b), (1, 1), (k // 2, k // 2), residual=dev(res), relu=True, precision=precision))
+    assert ops.device_status() == 0
+    max_abs, max_rel = ref_metric(got, conv_expect(x, w, b, res, True, 1, k // 2, 1, rounder))
+    bound = 1e-4 if rounder is None else 2e-5 * max(1.0, np.sqrt(C * k * k) / 8)
+    assert min(max_abs, max_rel) <= bound, f"{precision} {case}: {max_abs:.3e} {max_rel:.3e}"
+
+
 # ---------------------------------------------------------------- int8 conv + requantize
 def s8_inputs(rng, N, C, H, W, O, KH, KW):
     x = np.clip(np.round(rng.normal(0, 32, (N, C, H, W))), -128, 127).astype(np.int8)
