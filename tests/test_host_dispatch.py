@@ -12,6 +12,7 @@ import numpy as np
 import pytest
 import torch
 
+import dispatch_cases
 from hdkx_aicompiler_b200 import _lib, plan, relay, resnet18
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -290,3 +291,43 @@ def test_tile_box_search(fake, n, oh, ow):
     pick(n, oh, ow, *[ctypes.byref(b) for b in box])
     bw, bh, bni = (b.value for b in box)
     assert (bw, bh, bni) == (best[3], best[4], max(1, min(128 // (bw * bh), n)))
+
+
+# The layers whose split exchanges test_plan_gpu.py runs do take the forms they are listed for: every size of a cluster
+@pytest.mark.parametrize("precision,case,split,width", dispatch_cases.SPLIT_LAYERS)
+def test_split_layers_take_the_form_they_stand_for(compile_graph, precision, case, split, width):
+    n, c, h, w, o, k = case
+    graph, run = compile_graph(dispatch_cases.split_layer(relay, case, DeviceTensor, np.empty((o, c, k, k)), np.empty(o)), precision)
+    label = next(l[0] for l in graph.launch_info() if l[0].startswith("conv"))
+    assert label.endswith(f"split{split}") and f"bn{width} " in label, label
+    assert any("conv_splitk" in name and cluster == split for name, _, cluster in run)
+
+
+def test_split_layers_cover_every_cluster_and_width():
+    forms = {(split, width) for _, _, split, width in dispatch_cases.SPLIT_LAYERS}
+    assert {split for split, _ in forms} == set(range(2, 9)) and {(2, 256), (3, 256), (4, 256)} <= forms
+
+
+# ... and the shapes of test_conv2d_split_reduction and test_gemm_few_rows_split: CTAs of a cluster, 1 where the reduction is not split
+@pytest.mark.parametrize("precision,case,split", [(_lib.PREC_TF32, (1, 128, 9, 9, 64, 3, 1), 8), (_lib.PREC_TF32, (9, 128, 13, 15, 100, 3, 1), 3),
+                                                             (_lib.PREC_TF32, (2, 192, 21, 19, 70, 3, 2), 8), (_lib.PREC_TF32, (5, 1024, 7, 7, 40, 1, 1), 8),
+                                                             (_lib.PREC_TF32, (25, 256, 14, 14, 264, 3, 2), 3), (_lib.PREC_BF16, (1, 128, 9, 9, 64, 3, 1), 6),
+                                                             (_lib.PREC_BF16, (9, 128, 13, 15, 100, 3, 1), 1), (_lib.PREC_BF16, (2, 192, 21, 19, 70, 3, 2), 7),
+                                                             (_lib.PREC_BF16, (5, 1024, 7, 7, 40, 1, 1), 8), (_lib.PREC_BF16, (25, 256, 14, 14, 264, 3, 2), 2),
+                                                             (_lib.PREC_TF32X3, (1, 128, 9, 9, 64, 3, 1), 8), (_lib.PREC_TF32X3, (9, 128, 13, 15, 100, 3, 1), 6),
+                                                             (_lib.PREC_TF32X3, (2, 192, 21, 19, 70, 3, 2), 8), (_lib.PREC_TF32X3, (5, 1024, 7, 7, 40, 1, 1), 8),
+                                                             (_lib.PREC_TF32X3, (25, 256, 14, 14, 264, 3, 2), 3)])
+def test_operator_reductions_by_cluster(fake, precision, case, split):
+    rc, message = conv(fake, precision, *case)
+    assert rc == 0, message
+    last = launches(fake)[-1]
+    assert last.endswith(f"cluster {split}") and ("conv_splitk" in last) == (split > 1), last
+
+
+@pytest.mark.parametrize("precision,m,n,k,split", [(_lib.PREC_TF32, 1, 4096, 1024, 4), (_lib.PREC_TF32, 3, 3000, 1056, 5), (_lib.PREC_TF32, 7, 200, 2048, 8),
+                                                          (_lib.PREC_TF32, 2, 1000, 1600, 6), (_lib.PREC_BF16, 1, 4096, 1024, 2), (_lib.PREC_BF16, 3, 3000, 1056, 5),
+                                                          (_lib.PREC_BF16, 7, 200, 2048, 8), (_lib.PREC_BF16, 2, 1000, 1600, 5)])
+def test_dense_layers_of_few_rows_are_split(fake, precision, m, n, k, split):
+    rc = fake.kxc_b200_nn_gemm(pointers(4), _lib.GemmDesc(m, n, k, 1.0, 1.0, 0, 1, 1, precision), None)
+    assert rc == 0, fake.kxc_b200_last_error().decode()
+    assert "conv_splitk" in launches(fake)[-1] and launches(fake)[-1].endswith(f"cluster {split}"), launches(fake)[-1]

@@ -460,6 +460,21 @@ def test_gemm_few_tiles(ops, rng, M, N, K, offset, precision, rounder):
 
 
 # The result over an operand: the one-launch kernel reads the operands while it stores, so the call takes the path that converts them first.
+# Dense layers of one, three and seven rows by way of a split reduction: tiles of which all but a few rows are empty, fewer rows than CTAs
+# of a cluster. Bound: that of test_gemm_tensor_core.
+@pytest.mark.parametrize("precision,rounder", [("tf32", port.round_tf32), ("bf16", port.round_bf16)])
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 1024), (3, 3000, 1056), (7, 200, 2048), (2, 1000, 1600)])
+def test_gemm_few_rows_split(ops, rng, M, N, K, precision, rounder):
+    a = rng.normal(size=(M, K)).astype(f32)
+    b = rng.normal(0, np.sqrt(2.0 / K), (N, K)).astype(f32)
+    c = rng.normal(size=N).astype(f32)
+    exp = rounder(a).astype(np.float64) @ rounder(b).astype(np.float64).T + c
+    got = host(ops.nn_gemm(dev(a), dev(b), dev(c), transB=1, precision=precision))
+    assert ops.device_status() == 0
+    err = np.abs(got - exp) / np.maximum(1.0, np.abs(exp))
+    assert err.max() <= 2e-5 * max(1.0, np.sqrt(K) / 8), f"{precision} {M}x{N}x{K}: {err.max():.3e}"
+
+
 def test_gemm_result_over_an_operand(ops, rng):
     from hdkx_aicompiler_b200._lib import check, load, packed
     a, b = rng.normal(size=(70, 48)).astype(f32), rng.normal(size=(48, 48)).astype(f32)

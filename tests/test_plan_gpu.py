@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 import torch
 
+import dispatch_cases
 from conftest import assert_bit_exact, assert_close, ref_metric
 from oracle import graph as ograph
 from oracle import port
@@ -388,6 +389,28 @@ def test_downsample_block_split_of_the_two_output_kernel(kxc, monkeypatch, cin, 
     monkeypatch.setattr(kxc.plan.CompiledGraph, "launch_info", launch_info)
     test_downsample_block_two_output_kernel_is_bit_identical(kxc, monkeypatch, cin, cout, hw, N)
     assert all(l.endswith("second output" + (" " + split if split else "")) for l in labels if "second output" in l)
+
+
+# Every form of a split reduction (conv_splitk.cu): what each cluster's CTAs send one another and add up. Bounds: that of
+# test_conv2d_tensor_core for the sums (1e-4 for three passes) and, since both sides store them rounded, one step of the stored type where
+# they lie on either side of a boundary (2^-7 of the value with the 8 bits of bf16, 2^-10 with the 11 of tf32). Sums that are off by less
+# than 1e-3 of a step rarely do: at most one result in a hundred.
+@pytest.mark.parametrize("precision,case,split,width", dispatch_cases.SPLIT_LAYERS)
+def test_split_layers(kxc, precision, case, split, width):
+    n, c, h, w, o, k = case
+    rng = np.random.default_rng(23)
+    x = rng.uniform(-1, 1, (n, c, h, w)).astype(f32)
+    wt, bs = rng.normal(0, (2 / (k * k * c)) ** 0.5, (o, c, k, k)).astype(f32), rng.normal(0, 0.1, (o,)).astype(f32)
+    got, g = run_plan(kxc, dispatch_cases.split_layer(kxc.relay, case, cuda_const, wt, bs), x, precision)
+    from hdkx_aicompiler_b200 import ops
+    assert ops.device_status() == 0
+    label = next(l[0] for l in g.launch_info() if l[0].startswith("conv"))
+    assert label.endswith(f"split{split}") and f"bn{width} " in label, label
+    expect = ograph.run(dispatch_cases.split_layer(kxc.relay, case, lambda a: a, wt, bs), [x], operand_round=ROUND.get(precision), workers=8)
+    max_abs, max_rel = ref_metric(got, expect)
+    bound = 1e-4 if precision == "tf32x3" else 2e-5 * max(1.0, np.sqrt(c * k * k) / 8) + {"bf16": 2.0 ** -7, "tf32": 2.0 ** -10}[precision]
+    assert min(max_abs, max_rel) <= bound, f"{precision} {case}: {max_abs:.3e} {max_rel:.3e}"
+    assert precision == "tf32x3" or np.mean(got != expect) <= 1e-2, f"{precision} {case}: {np.mean(got != expect):.2e} of the results differ"
 
 
 @pytest.mark.parametrize("n,h,w", [(2, 56, 56), (3, 30, 20), (1, 7, 5), (2, 14, 8), (1, 15, 9)])
