@@ -331,3 +331,17 @@ def test_dense_layers_of_few_rows_are_split(fake, precision, m, n, k, split):
     rc = fake.kxc_b200_nn_gemm(pointers(4), _lib.GemmDesc(m, n, k, 1.0, 1.0, 0, 1, 1, precision), None)
     assert rc == 0, fake.kxc_b200_last_error().decode()
     assert "conv_splitk" in launches(fake)[-1] and launches(fake)[-1].endswith(f"cluster {split}"), launches(fake)[-1]
+
+
+# The tiles of the packed fp32 kernel that test_ops_gpu.py runs: all of them, and those of test_conv2d_fp32_wide_filter_tiles_bit_exact
+@pytest.mark.parametrize("case,width,tile", dispatch_cases.FP32_TILES + [
+    ((1, 5, 6, 7, 17, 3, 3, 2, 1, 1), 3, "16x16"), ((1, 61, 6, 7, 17, 3, 3, 1, 1, 1), 3, "16x16"), ((1, 3, 9, 5, 20, 7, 7, 1, 3, 1), 7, "16x16"),
+    ((2, 5, 28, 43, 17, 3, 3, 1, 1, 1), 3, "32x32"), ((4, 3, 18, 34, 18, 7, 7, 1, 3, 1), 7, "32x32"), ((2, 7, 50, 48, 33, 3, 3, 1, 1, 1), 3, "32x96"),
+    ((3, 2, 33, 48, 33, 7, 7, 1, 3, 1), 7, "32x96"), ((4, 7, 50, 36, 33, 3, 3, 1, 1, 1), 3, "32x128"), ((3, 2, 46, 53, 35, 7, 7, 1, 3, 1), 7, "32x128"),
+])
+def test_fp32_tiles_are_those_the_gpu_tests_name(fake, case, width, tile):
+    n, c, h, w, o, kh, kw, s, p, d = case
+    desc = _lib.Conv2dDesc(n, c, h, w, o, kh, kw, s, s, p, p, d, d, _lib.BIAS | _lib.RESIDUAL | _lib.RELU, _lib.PREC_FP32)
+    assert fake.kxc_b200_nn_conv2d(pointers(5), desc, None) == 0, fake.kxc_b200_last_error().decode()
+    to, tp, og, pg = (int(v) for v in re.search(r"tiled_f32_kernelILi%dELi(\d+)ELi(\d+)ELi(\d+)ELi(\d+)E" % width, launches(fake)[-1]).groups())
+    assert f"{to * og}x{tp * pg}" == tile, launches(fake)[-1]

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 import torch
 
+import dispatch_cases
 from conftest import assert_bit_exact, assert_close, ref_metric
 from oracle import port
 
@@ -176,7 +177,7 @@ def test_conv2d_fp32_mode_bit_exact(ops, rng, case):
     assert_bit_exact(got, conv_expect(x, w, b, None, True, s, p, d), f"conv fp32 {case}")
 
 
-# the tiles of the packed fp32 kernel (16x32, 32x64, 64x96, 64x128 channels x pixels), its filter widths (1, 3, 7, any),
+# tiles of the packed fp32 kernel (test_conv2d_fp32_every_tile_bit_exact has them all), its filter widths (1, 3, 7, any),
 # reductions that end inside a stage, odd weight rows, planes of no multiple of four pixels
 @pytest.mark.parametrize("case", [
     (1, 5, 21, 19, 17, 3, 3, 1, 1, 1), (1, 33, 20, 20, 64, 1, 1, 1, 0, 1), (5, 7, 27, 23, 65, 3, 3, 1, 1, 1),
@@ -199,6 +200,12 @@ def test_conv2d_fp32_tiles_bit_exact(ops, rng, case):
     (3, 2, 46, 53, 35, 7, 7, 1, 3, 1),
 ])
 def test_conv2d_fp32_wide_filter_tiles_bit_exact(ops, rng, case):
+    test_conv2d_fp32_tiles_bit_exact(ops, rng, case)
+
+
+# every tile of every width
+@pytest.mark.parametrize("case", [case for case, _, _ in dispatch_cases.FP32_TILES])
+def test_conv2d_fp32_every_tile_bit_exact(ops, rng, case):
     test_conv2d_fp32_tiles_bit_exact(ops, rng, case)
 
 
