@@ -32,8 +32,11 @@ __device__ __forceinline__ float round_operand(float x) {
     else return tf32_rne(x);
 }
 
-template <bool kBF16>
-__global__ void __launch_bounds__(kThreads) gemm_small_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ c,
+// kBlocks: resident per SM, what the rule below counts on. (128 registers, tf32 with or without the bound; bf16 takes 161 for one block,
+// which is faster while there is a tile per SM, 32x2016x512 6.0 / 6.3 us and 32x2016x1024 10.4 / 11.2, but would be two waves beyond that,
+// 128x1000x512 11.1 / 9.2.)
+template <bool kBF16, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks) gemm_small_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ c,
                                                               float* __restrict__ out, int M, int N, int K, int vec) {
     extern __shared__ __align__(16) float rows[];  // kTM rows of a, then kTN rows of b
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -119,10 +122,19 @@ __global__ void __launch_bounds__(kThreads) gemm_small_kernel(const float* __res
 
 }  // namespace
 
-// While all tiles are resident at once, two blocks per SM for one pass over k and one for two. Device time of the other path / this
-// one (tf32, us; the other path also takes the host 9 to 15 per call): 32x1000x512 9.2 / 6.5, 128x1000x512 9.5 / 9.9, 300x256x64
-// 7.3 / 7.2, 900x100x300 13.0 / 9.0, 32x1000x1024 10.9 / 11.1; beyond the line 128x1000x1024 11.5 / 17.4. A result that overlaps an
-// operand needs the other path, which has read both (into its workspace) before it stores anything.
+// While all tiles are resident at once, two blocks per SM for one pass over k and one for two: then a call of the operator, which is
+// bound by its host side, always gains. On the device alone, in a captured graph or behind a full queue, it gains with one pass and a
+// tile per SM and trades otherwise. us, a call / its device time, other path : this one:
+//                    tf32                          bf16
+//   32x1008x512      13.5 / 9.1 : 8.2 / 6.1        12.9 / 8.1 : 8.5 / 5.9
+//   128x1000x512     13.6 / 10.3 : 9.8 / 9.4       12.9 / 9.0 : 9.6 / 9.2
+//   32x3200x64       12.5 / 5.9 : 8.2 / 7.2        12.9 / 5.5 : 8.4 / 6.7
+//   32x1008x640      13.5 / 9.3 : 9.8 / 9.5        12.7 / 8.8 : 9.3 / 9.0
+//   32x1008x1024     14.0 / 10.6 : 10.9 / 10.7     14.0 / 9.4 : 10.5 / 10.3
+//   32x128x1024      13.1 / 8.6 : 10.7 / 10.6      13.5 / 7.9 : 10.3 / 10.2
+//   32x2016x1024     16.5 / 12.8 : 11.1 / 10.8     13.9 / 11.1 : 10.6 / 10.4
+//   128x1000x1024, beyond the line: 11.5 : 17.4 on the device
+// A result that overlaps an operand needs the other path, which has read both (into its workspace) before it stores anything.
 bool gemm_small_applicable(const float* a, const float* b, const float* out, const kxc_b200_gemm_desc& g) {
     auto overlaps = [&](const float* x, int64_t rows) {
         const auto o = reinterpret_cast<uintptr_t>(out), q = reinterpret_cast<uintptr_t>(x);
@@ -142,8 +154,9 @@ int32_t gemm_small(const float* a, const float* b, const float* c, float* out, c
         KXC_CUDA_TRY(launch_kernel(kernel, grid, dim3(kThreads), kSmemBytes, s, /*pdl=*/true, 1, a, b, c, out, g.m, g.n, g.k, vec));
         return check_launch("gemm_small");
     };
-    static PerDeviceOnce once_bf16, once_tf32;
-    return g.precision == KXC_B200_PREC_BF16 ? go(gemm_small_kernel<true>, once_bf16) : go(gemm_small_kernel<false>, once_tf32);
+    static PerDeviceOnce once_bf16, once_bf16_two, once_tf32;
+    if (g.precision != KXC_B200_PREC_BF16) return go(gemm_small_kernel<false, 2>, once_tf32);
+    return (int64_t)grid.x * grid.y <= kNumSMs ? go(gemm_small_kernel<true, 1>, once_bf16) : go(gemm_small_kernel<true, 2>, once_bf16_two);
 }
 
 }  // namespace kxc_b200

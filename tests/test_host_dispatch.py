@@ -333,6 +333,22 @@ def test_dense_layers_of_few_rows_are_split(fake, precision, m, n, k, split):
     assert "conv_splitk" in launches(fake)[-1] and launches(fake)[-1].endswith(f"cluster {split}"), launches(fake)[-1]
 
 
+# Which dense layers take one launch on the CUDA cores (rule and figures at gemm_small_applicable): up to two tiles of 32 x 16 per SM
+# with up to 512 k, one with up to 1024. bf16: blocks of one per SM while that is enough (the template's last argument)
+@pytest.mark.parametrize("precision", [_lib.PREC_TF32, _lib.PREC_BF16])
+@pytest.mark.parametrize("m,n,k,blocks", [(1, 1, 1, 1), (32, 2368, 512, 1), (33, 1184, 512, 1), (32, 2369, 512, 2), (128, 1184, 20, 2), (64, 2368, 512, 2),
+                                          (128, 1185, 20, 0), (32, 2368, 1024, 1), (97, 592, 513, 1), (97, 593, 513, 0), (20, 40, 1025, 0)])
+def test_dense_layers_of_few_tiles_in_one_launch(fake, precision, m, n, k, blocks):
+    rc = fake.kxc_b200_nn_gemm(pointers(4), _lib.GemmDesc(m, n, k, 1.0, 1.0, 0, 1, 1, precision), None)
+    assert rc == 0, fake.kxc_b200_last_error().decode()
+    lines = launches(fake)
+    if blocks == 0:
+        assert not any("gemm_small" in line for line in lines), lines
+    else:
+        kernel = "gemm_small_kernelILb0ELi2EE" if precision == _lib.PREC_TF32 else f"gemm_small_kernelILb1ELi{blocks}EE"
+        assert len(lines) == 1 and kernel in lines[0], lines
+
+
 # The tiles of the packed fp32 kernel that test_ops_gpu.py runs: all of them, and those of test_conv2d_fp32_wide_filter_tiles_bit_exact
 @pytest.mark.parametrize("case,width,tile", dispatch_cases.FP32_TILES + [
     ((1, 5, 6, 7, 17, 3, 3, 2, 1, 1), 3, "16x16"), ((1, 61, 6, 7, 17, 3, 3, 1, 1, 1), 3, "16x16"), ((1, 3, 9, 5, 20, 7, 7, 1, 3, 1), 7, "16x16"),
