@@ -564,11 +564,10 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
                     const char* e3 = getenv("KXC_B200_STEM_FUSED_INPUT");  // "0" keeps the pack kernel + packed-input kernel
                     const bool nchw_ok = (!e3 || atoi(e3) != 0) && !pl->x3 && n.conv.padding[0] == KHc / 2 && n.conv.padding[1] == KWc / 2 &&
                                          stem_pool_nchw_applicable(dt, st.C, (int)w->shape[0], KHc, KWc, st.W, OHc, OWc, Wpc);
-                    // tf32: the fused kernel or none, from 57 strips of four convolution rows on (three images of 224 x 224). Below,
-                    // whole networks gain 1 to 3 % (one image 170 / 168 us, two 186 / 180; four 217 / 209) and keep the list of
-                    // launches that test_resnet18_plan holds them to. bf16 has a fused kernel for packed inputs too.
+                    // tf32: the fused kernel wherever it applies, or none (whole networks without / with it, us: one image 153.2 / 151.7, two
+                    // 168.5 / 163.7, three 184.1 / 177.7, four 192.9 / 185.0). bf16 has a fused kernel for packed inputs too.
                     if (pool_ok && st.C <= 4 && KWc <= 8 && st.W >= 8 &&
-                        (dt == kTcTF32 ? nchw_ok && (long long)(OHc / 4) * st.N > 56
+                        (dt == kTcTF32 ? nchw_ok
                                        : stem_direct_applicable(dt, st.C, (int)w->shape[0], KHc, KWc, OWc, Wpc) && stem_pool_applicable(OHc, OWc, 3, 2, 1))) {
                         st.fused_pool = 1;
                         pl->nodes[pc].fused_into_other = true;
