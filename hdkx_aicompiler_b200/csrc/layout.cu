@@ -32,21 +32,32 @@ __device__ __forceinline__ TOut convert_elem(TIn v) { return convert_to<TOut>((f
 template <>
 __device__ __forceinline__ int8_t convert_elem<int8_t, int8_t>(int8_t v) { return v; }
 
-// Weights OIHW -> [O][KH*KW][cpad] (channels c >= C zero): a thread takes the whole filter of one output channel and kVec input
-// channels, so that its reads are consecutive words and its stores are whole 32-bit words side by side with its neighbours'.
+// Weights OIHW -> [O][KH*KW][cpad] (channels c >= C zero): a thread takes up to kPackTaps taps of one output channel and kVec input
+// channels, so that its reads are consecutive words and its stores are whole 32-bit words side by side with its neighbours'. One way to
+// memory and back bounds it. (With a thread per whole filter there was one after the other for every nine taps, on few blocks where
+// the channels are few. us a call, so / now: 3 -> 32 channels 31x31 at 64x64, bf16 442 / 332, int8 424 / 326; 3 -> 64 11x11, tf32 52.5 / 46.3;
+// 3 -> 64 7x7 stride 2 at 224x224, bf16 27.0 / 23.2. Filters of up to nine taps as before.)
+constexpr int kPackTaps = 9;
 template <typename TIn, typename TOut, bool kSplit>
 __device__ __forceinline__ void pack_weights_block(const TIn* __restrict__ w, TOut* __restrict__ out, TOut* __restrict__ lo, int64_t groups, int C,
-                                                   int taps, int cpad, int64_t block) {
+                                                   int taps, int cpad, unsigned group_blocks, unsigned block) {
     constexpr int kVec = 4 / (int)sizeof(TOut);
-    const int64_t g = block * 256 + threadIdx.x;
+    int first = 0;
+    if (block >= group_blocks) {
+        const unsigned piece = block / group_blocks;
+        block -= piece * group_blocks;
+        first = (int)piece * kPackTaps;
+    }
+    const int64_t g = (int64_t)block * 256 + threadIdx.x;
     if (g >= groups) return;
     const int per_row = cpad / kVec;
     const int o = (int)(g / per_row), c0 = (int)(g - (int64_t)o * per_row) * kVec;
-    const TIn* src = w + ((int64_t)o * C + c0) * taps;
-    TOut* dst = out + (int64_t)o * taps * cpad + c0;
+    const TIn* src = w + ((int64_t)o * C + c0) * taps + first;
+    TOut* dst = out + ((int64_t)o * taps + first) * cpad + c0;
     const int64_t lo_off = kSplit ? lo - out : 0;
+    const int count = taps - first < kPackTaps ? taps - first : kPackTaps;
 #pragma unroll 9
-    for (int t = 0; t < taps; ++t) {
+    for (int t = 0; t < count; ++t) {
         alignas(4) TOut v[kVec];
         [[maybe_unused]] TOut l[kVec];
 #pragma unroll
@@ -64,9 +75,9 @@ struct PackArgs {
     const void* w = nullptr;
     void* out = nullptr;
     void* lo = nullptr;   // three-pass tf32: the low parts
-    int64_t groups = 0;   // threads that have work (pack_weights_block)
+    int64_t groups = 0;   // threads that have work (pack_weights_block), for every kPackTaps taps
     int C = 0, taps = 0, cpad = 0;
-    unsigned blocks = 0;
+    unsigned group_blocks = 0, blocks = 0;
 };
 
 // Activations NCHW fp32 -> NHWC of the operand type and, in the first blocks of the same launch, the weights of the convolution
@@ -88,7 +99,7 @@ __global__ void __launch_bounds__(256) convert_operands_kernel(const float* __re
     if (overlap) sm100::pdl_launch_dependents();
     if (blockIdx.x < pack.blocks) {
         pack_weights_block<float, TOut, kSplit>(static_cast<const float*>(pack.w), static_cast<TOut*>(pack.out), static_cast<TOut*>(pack.lo),
-                                                pack.groups, pack.C, pack.taps, pack.cpad, blockIdx.x);
+                                                pack.groups, pack.C, pack.taps, pack.cpad, pack.group_blocks, blockIdx.x);
         return;
     }
     __shared__ float tile[kCT][kPT + 1];
@@ -124,7 +135,7 @@ __global__ void __launch_bounds__(256) convert_operands_kernel(const float* __re
 template <typename TIn, typename TOut, bool kSplit>
 __global__ void __launch_bounds__(256) pack_weights_kernel(PackArgs pack) {
     pack_weights_block<TIn, TOut, kSplit>(static_cast<const TIn*>(pack.w), static_cast<TOut*>(pack.out), static_cast<TOut*>(pack.lo), pack.groups,
-                                          pack.C, pack.taps, pack.cpad, blockIdx.x);
+                                          pack.C, pack.taps, pack.cpad, pack.group_blocks, blockIdx.x);
 }
 
 // The same for rows that need no reordering: [rows, cols] -> two times [rows, cpad]. cols % 4 == 0 and cols == cpad take
@@ -310,7 +321,7 @@ __global__ void __launch_bounds__(256) transpose_bytes_kernel(TransposeArgs a, P
     if (overlap) sm100::pdl_launch_dependents();
     if (blockIdx.x < pack.blocks) {
         pack_weights_block<int8_t, int8_t, false>(static_cast<const int8_t*>(pack.w), static_cast<int8_t*>(pack.out), nullptr, pack.groups, pack.C,
-                                                  pack.taps, pack.cpad, blockIdx.x);
+                                                  pack.taps, pack.cpad, pack.group_blocks, blockIdx.x);
         return;
     }
     unsigned t = blockIdx.x - pack.blocks;
@@ -366,7 +377,8 @@ PackArgs pack_args(const WeightPack* w) {
     p.w = w->w; p.out = w->out; p.lo = w->lo;
     p.C = w->C; p.taps = w->taps; p.cpad = w->cpad;
     p.groups = (int64_t)w->O * (w->cpad / (4 / (int)sizeof(T)));
-    p.blocks = (unsigned)((p.groups + 255) / 256);
+    p.group_blocks = (unsigned)((p.groups + 255) / 256);
+    p.blocks = p.group_blocks * (unsigned)((w->taps + kPackTaps - 1) / kPackTaps);
     return p;
 }
 

@@ -361,3 +361,16 @@ def test_fp32_tiles_are_those_the_gpu_tests_name(fake, case, width, tile):
     assert fake.kxc_b200_nn_conv2d(pointers(5), desc, None) == 0, fake.kxc_b200_last_error().decode()
     to, tp, og, pg = (int(v) for v in re.search(r"tiled_f32_kernelILi%dELi(\d+)ELi(\d+)ELi(\d+)ELi(\d+)E" % width, launches(fake)[-1]).groups())
     assert f"{to * og}x{tp * pg}" == tile, launches(fake)[-1]
+
+
+# Weights are packed by a thread per nine taps of a filter: blocks of the launch that converts both operands (961 taps: 107 pieces)
+@pytest.mark.parametrize("precision", [_lib.PREC_TF32, _lib.PREC_BF16, _lib.PREC_TF32X3])
+def test_large_filters_are_packed_in_pieces(fake, precision):
+    blocks = {}
+    for k in (1, 3, 5, 31):
+        fake.fake_reset()
+        rc, message = conv(fake, precision, 1, 3, 64, 64, 32, k)
+        assert rc == 0, message
+        assert "convert_operands" in launches(fake)[0]
+        blocks[k] = int(launches(fake)[0].split(" grid ")[1].split()[0])
+    assert blocks[1] == blocks[3] and blocks[5] == blocks[3] + 2 and blocks[31] == blocks[3] + 106, blocks

@@ -384,6 +384,28 @@ def test_conv2d_s8_bit_exact(ops, rng, case, simt):
         assert np.array_equal(got, expect), f"s8 conv {case} relu={relu} simt={simt}: {np.count_nonzero(got != expect)} differ"
 
 
+# Weights packed by several threads per filter (9 taps each): a last piece that is partly there, one tap behind whole pieces, int8 (four
+# channels per thread) with and without a stride. Bounds: those of test_conv2d_tensor_core and 1e-4 for three passes; int8 equal.
+@pytest.mark.parametrize("precision", ["tf32", "bf16", "tf32x3", "s8"])
+@pytest.mark.parametrize("N,C,H,W,O,KH,KW", [(2, 3, 12, 17, 33, 5, 5), (1, 5, 14, 13, 20, 11, 11), (1, 40, 9, 11, 70, 2, 5), (2, 2, 31, 8, 9, 19, 1)])
+def test_conv2d_weights_of_large_filters(ops, rng, N, C, H, W, O, KH, KW, precision):
+    pad = (KH // 2, KW // 2)
+    if precision == "s8":
+        x, w, b, m, sh = s8_inputs(rng, N, C, H, W, O, KH, KW)
+        for relu in (True, False):
+            got = host(ops.nn_conv2d_s8(dev(x), dev(w), dev(b), dev(m), dev(sh), padding=pad, relu=relu))
+            assert np.array_equal(got, port.conv2d_s8_requant(x, w, b, m, sh, relu, (1, 1), pad))
+        return
+    rounder = {"tf32": port.round_tf32, "bf16": port.round_bf16, "tf32x3": None}[precision]
+    x, w, b = conv_inputs(rng, N, C, H, W, O, KH, KW)
+    got = host(ops.nn_conv2d(dev(x), dev(w), dev(b), padding=pad, precision=precision))
+    assert ops.device_status() == 0
+    rounded = (x, w) if rounder is None else (rounder(x), rounder(w))
+    max_abs, max_rel = ref_metric(got, port.conv2d(*rounded, b, (1, 1), pad))
+    bound = 1e-4 if rounder is None else 2e-5 * max(1.0, np.sqrt(C * KH * KW) / 8)
+    assert min(max_abs, max_rel) <= bound, f"{precision}: {max_abs:.3e} {max_rel:.3e}"
+
+
 # The byte transposes on both sides of the NCHW form: planes that are multiples of 16, of 4 and odd; channel counts that are not
 # multiples of 16 or 4; one, two and more column tiles; the result by way of NHWC (1 MiB and more) and without.
 @pytest.mark.parametrize("N,C,H,W,O", [(9, 72, 28, 28, 150), (3, 130, 30, 30, 400), (40, 64, 14, 14, 141), (27, 33, 25, 13, 133), (2, 48, 12, 12, 40),
