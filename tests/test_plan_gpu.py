@@ -3,6 +3,7 @@ same Relay-style graph call by call."""
 import numpy as np
 import pytest
 import torch
+import torch.nn.functional as F
 
 import dispatch_cases
 from conftest import assert_bit_exact, assert_close, ref_metric
@@ -332,6 +333,61 @@ def test_fused_stem_is_bit_identical(kxc, monkeypatch, precision, n, c, h, w):
     from hdkx_aicompiler_b200 import ops
     assert ops.device_status() == 0
     assert_bit_exact(fused, unfused, f"{precision} {n}x{c}x{h}x{w}")
+
+
+def conv64(x, w, b, stride, pad):
+    """A convolution in 64-bit arithmetic, independent of this library and of the oracle's fp32."""
+    k = w.shape[2]
+    cols = [F.unfold(x[i:i + 4].double(), k, padding=pad, stride=stride) for i in range(0, len(x), 4)]
+    y = torch.cat([w.double().flatten(1) @ c for c in cols]) + (0 if b is None else b.double().view(-1, 1))
+    return y.view(len(x), len(w), (x.shape[2] + 2 * pad - k) // stride + 1, -1)
+
+
+# Against 64-bit arithmetic on the unrounded operands, as a share of the logits' norm: operand rounding sets the level, whatever the order of
+# the sums. Measured over 3 seeds and 1 to 32 images: tf32 4.5e-4 to 5.0e-4, bf16 3.4e-3 to 4.0e-3, three passes 0.7e-5 to 2.6e-5; bounds 1.5
+# times the largest.
+@pytest.mark.parametrize("precision,bound", [("tf32", 7.5e-4), ("bf16", 6e-3), ("tf32x3", 4e-5)])
+@pytest.mark.parametrize("n", [1, 4, 32])
+def test_resnet18_against_64_bits(kxc, precision, bound, n):
+    rs = kxc.resnet18
+    weights = rs.make_weights(seed=n)
+    t = {name: cuda_const(a) for name, a in weights}
+    x = torch.from_numpy(np.random.default_rng(n).normal(0, 1, (n, 3, 224, 224)).astype(f32)).cuda()
+    got = kxc.plan.CompiledGraph(rs.build(n, weights, to_constant=cuda_const), precision).run(x).double()
+    assert kxc.ops.device_status() == 0
+    conv = lambda y, name, s, p: conv64(y, t[name + ".weight"], t[name + ".bias"], s, p)  # noqa: E731
+    y = F.max_pool2d(conv(x, "conv1", 2, 3).relu(), 3, 2, 1)
+    for stage in range(1, 5):
+        for block in range(2):
+            s, name = (2 if stage > 1 and block == 0 else 1), f"layer{stage}.{block}"
+            z = conv(conv(y, name + ".conv1", s, 1).relu(), name + ".conv2", 1, 1)
+            y = (z + (conv(y, name + ".downsample", s, 0) if name + ".downsample.weight" in t else y)).relu()
+    exact = y.mean((2, 3)) @ t["fc.weight"].double().T + t["fc.bias"].double()
+    err = ((got - exact).norm() / exact.norm()).item()
+    print(f"resnet18 {precision} {n} images against 64 bits: {err:.3e}")
+    assert err <= bound
+
+
+# One layer's stored results, read back through an identity: the share that is not the rounding of the 64-bit sum (a sum that is off by
+# the order of its terms falls on the other side of a rounding boundary). Row-stacked, general and split kernels. Measured: tf32 1.2e-3
+# to 2.8e-3, bf16 0.8e-4 to 1.4e-4; bounds three times the largest.
+@pytest.mark.parametrize("precision,kernel,n,c,hw", [("tf32", "conv_rowstack_tf32", 4, 64, 56), ("tf32", "conv_rowstack_tf32", 3, 64, 23),
+                                                     ("bf16", "conv_rowstack128", 4, 128, 28), ("tf32", "conv_igemm", 2, 256, 14),
+                                                     ("bf16", "conv_igemm", 2, 256, 14), ("tf32", "conv_igemm", 1, 512, 7), ("bf16", "conv_igemm", 1, 512, 7)])
+def test_layers_against_64_bits(kxc, precision, kernel, n, c, hw):
+    R = kxc.relay
+    rng = np.random.default_rng(5)
+    x, w = rng.normal(0, 1, (n, c, hw, hw)).astype(f32), rng.normal(0, (2 / (9 * c)) ** 0.5, (c, c, 3, 3)).astype(f32)
+    eye, zero = np.eye(c, dtype=f32).reshape(c, c, 1, 1), np.zeros(c, f32)
+    xv = R.Var("input", x.shape)
+    conv = lambda y, f, p: R.Call("nn_conv2d", [y, R.Constant(cuda_const(f)), R.Constant(cuda_const(zero))],  # noqa: E731
+                                  R.Conv2DAttrs((1, 1), (p,) * 4, (1, 1), 1))
+    got, g = run_plan(kxc, R.Function([xv], conv(R.Call("nn_relu", [conv(xv, w, 1)]), eye, 0)), x, precision)
+    assert next(l[0] for l in g.launch_info() if l[0].startswith("conv")).startswith(kernel + " ")
+    exact = conv64(cuda_const(ROUND[precision](x)), cuda_const(ROUND[precision](w)), None, 1, 1).relu()
+    share = np.mean(got != ROUND[precision](exact.float().cpu().numpy()))
+    print(f"{kernel} {precision} {n}x{c}x{hw}: {share:.2e}")
+    assert share <= {"tf32": 8.4e-3, "bf16": 4.2e-4}[precision]
 
 
 @pytest.mark.parametrize("cin,cout,hw,N", [(64, 128, 56, 3), (128, 256, 28, 3), (64, 64, 30, 3), (256, 512, 14, 128)])
