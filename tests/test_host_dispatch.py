@@ -286,7 +286,8 @@ def test_tile_box_search(fake, n, oh, ow):
     best = min((-(-ow // bw) * -(-oh // bh) * -(-n // max(1, min(128 // (bw * bh), n))), -bw * bh, abs(bw - bh), bw, bh)
                for bw in range(1, min(ow, 128) + 1) for bh in range(1, min(oh, 128 // bw) + 1))
     box = [ctypes.c_int(0) for _ in range(3)]
-    pick = getattr(fake, "_ZN8kxc_b20012tc_pick_tileEiiiPiS0_S0_")
+    symbols = subprocess.run(["nm", "-D", "--defined-only", fake._name], check=True, capture_output=True, text=True).stdout
+    pick = getattr(fake, next(line.split()[-1] for line in symbols.splitlines() if "tc_pick_tile" in line))
     pick.restype, pick.argtypes = None, [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_int)] * 3
     pick(n, oh, ow, *[ctypes.byref(b) for b in box])
     bw, bh, bni = (b.value for b in box)
