@@ -27,50 +27,6 @@ __device__ __forceinline__ Tf32Lo convert_to<Tf32Lo>(float v) {
     return Tf32Lo{tf32_low_part(v, tf32_rne(v))};
 }
 
-template <typename TIn, typename TOut>
-__device__ __forceinline__ TOut convert_elem(TIn v) { return convert_to<TOut>((float)v); }
-template <>
-__device__ __forceinline__ int8_t convert_elem<int8_t, int8_t>(int8_t v) { return v; }
-
-// Weights OIHW -> [O][KH*KW][cpad] (channels c >= C zero): a thread takes up to kPackTaps taps of one output channel and kVec input
-// channels, so that its reads are consecutive words and its stores are whole 32-bit words side by side with its neighbours'. One way to
-// memory and back bounds it. (With a thread per whole filter there was one after the other for every nine taps, on few blocks where
-// the channels are few. us a call, so / now: 3 -> 32 channels 31x31 at 64x64, bf16 442 / 332, int8 424 / 326; 3 -> 64 11x11, tf32 52.5 / 46.3;
-// 3 -> 64 7x7 stride 2 at 224x224, bf16 27.0 / 23.2. Filters of up to nine taps as before.)
-constexpr int kPackTaps = 9;
-template <typename TIn, typename TOut, bool kSplit>
-__device__ __forceinline__ void pack_weights_block(const TIn* __restrict__ w, TOut* __restrict__ out, TOut* __restrict__ lo, int64_t groups, int C,
-                                                   int taps, int cpad, unsigned group_blocks, unsigned block) {
-    constexpr int kVec = 4 / (int)sizeof(TOut);
-    int first = 0;
-    if (block >= group_blocks) {
-        const unsigned piece = block / group_blocks;
-        block -= piece * group_blocks;
-        first = (int)piece * kPackTaps;
-    }
-    const int64_t g = (int64_t)block * 256 + threadIdx.x;
-    if (g >= groups) return;
-    const int per_row = cpad / kVec;
-    const int o = (int)(g / per_row), c0 = (int)(g - (int64_t)o * per_row) * kVec;
-    const TIn* src = w + ((int64_t)o * C + c0) * taps + first;
-    TOut* dst = out + ((int64_t)o * taps + first) * cpad + c0;
-    const int64_t lo_off = kSplit ? lo - out : 0;
-    const int count = taps - first < kPackTaps ? taps - first : kPackTaps;
-#pragma unroll 9
-    for (int t = 0; t < count; ++t) {
-        alignas(4) TOut v[kVec];
-        [[maybe_unused]] TOut l[kVec];
-#pragma unroll
-        for (int e = 0; e < kVec; ++e) {
-            const TIn x = c0 + e < C ? __ldg(src + (int64_t)e * taps + t) : (TIn)0;
-            v[e] = convert_elem<TIn, TOut>(x);
-            if constexpr (kSplit) l[e] = convert_to<Tf32Lo>(x).v;
-        }
-        *reinterpret_cast<uint32_t*>(dst + (int64_t)t * cpad) = *reinterpret_cast<const uint32_t*>(v);
-        if constexpr (kSplit) dst[lo_off + (int64_t)t * cpad] = l[0];
-    }
-}
-
 // n / d for n < 2^31, d >= 1 by a multiplication (Granlund and Montgomery, "Division by invariant integers using multiplication", 1994). A
 // conversion's blocks find their tile in a one-dimensional grid, and two divisions held up the loads of every block (us on the device, with them /
 // so: int8 96 -> 178 1x1 at 28x28, 229 images 52.5 / 51.8, 128 -> 128 3x3 at 28x28, 256 images 67.9 / 66.8, 128 -> 64 3x3 stride 2 at 57x57,
@@ -89,10 +45,62 @@ struct PackArgs {
     const void* w = nullptr;
     void* out = nullptr;
     void* lo = nullptr;   // three-pass tf32: the low parts
-    int64_t groups = 0;   // threads that have work (pack_weights_block), for every kPackTaps taps
+    int64_t groups = 0;   // threads that have work for every piece of a filter (pack_weights_block)
     int C = 0, taps = 0, cpad = 0;
-    unsigned group_blocks = 0, blocks = 0;
+    int per_thread = 0;       // taps
+    Divisor pieces, per_row;  // of a filter; groups of channels of an output channel
+    unsigned blocks = 0;
 };
+
+// Weights OIHW -> [O][KH*KW][cpad] (channels c >= C zero): a thread takes some taps (PackArgs::per_thread) of one output channel and kVec
+// input channels, so that its reads are consecutive words, about ten of them in flight at once, and its stores are whole 32-bit words side
+// by side with its neighbours'. The warps of the pieces of 32 groups are neighbours: they read the same sectors. One way to memory and
+// back bounds it. (With a thread per whole filter there was one after the other for every nine taps, on few blocks where the channels are
+// few: 3 -> 32 channels 31x31 at 64x64, bf16 442 us a call so, 333 now, int8 428 and 326; 3 -> 64 7x7 stride 2 at 224x224, bf16 28.5 and 24.7.)
+// Nine taps of fp32, five of bf16, three of int8, but nine where that still makes 48 blocks: 100 -> 200 3x3 at 41x43, 16 images, int8 36 us a
+// call with nine and 28 with three, since the convolution's CTAs, set up meanwhile, leave less room to a conversion that takes long; 256 ->
+// 256 3x3 at 14x14, 16 images, 14.9 with nine and 16.4 with three, whose blocks cost more than their shorter chain gains.
+template <typename T>
+constexpr int kPackTaps = sizeof(T) == 4 ? 9 : sizeof(T) == 2 ? 5 : 3;
+template <typename TIn, typename TOut, bool kSplit>
+__device__ __forceinline__ void pack_weights_block(const TIn* __restrict__ w, TOut* __restrict__ out, TOut* __restrict__ lo, const PackArgs& a,
+                                                   unsigned block) {
+    constexpr int kVec = 4 / (int)sizeof(TOut);
+    const unsigned warp = block * 8 + threadIdx.x / 32, set = a.pieces.quotient(warp);
+    const int64_t g = (int64_t)set * 32 + threadIdx.x % 32;
+    if (g >= a.groups) return;
+    const int C = a.C, taps = a.taps, cpad = a.cpad, first = (int)(warp - set * a.pieces.d) * a.per_thread;
+    const int o = a.groups < 1ll << 31 ? (int)a.per_row.quotient((unsigned)g) : (int)(g / a.per_row.d);
+    const int c0 = (int)(g - (int64_t)o * a.per_row.d) * kVec;
+    const TIn* src = w + ((int64_t)o * C + c0) * taps + first;
+    TOut* dst = out + ((int64_t)o * taps + first) * cpad + c0;
+    [[maybe_unused]] const int64_t lo_off = kSplit ? lo - out : 0;
+    if constexpr (kVec == 4) {  // (a loop: the registers of 36 loads would cost the transposition blocks)
+        const int count = taps - first < a.per_thread ? taps - first : a.per_thread;
+#pragma unroll 9
+        for (int t = 0; t < count; ++t) {
+            alignas(4) TOut v[kVec];
+#pragma unroll
+            for (int e = 0; e < kVec; ++e) v[e] = c0 + e < C ? __ldg(src + (int64_t)e * taps + t) : (TIn)0;
+            *reinterpret_cast<uint32_t*>(dst + (int64_t)t * cpad) = *reinterpret_cast<const uint32_t*>(v);
+        }
+    } else {
+        TIn x[kPackTaps<TOut>][kVec];
+#pragma unroll
+        for (int t = 0; t < kPackTaps<TOut>; ++t)
+#pragma unroll
+            for (int e = 0; e < kVec; ++e) x[t][e] = first + t < taps && c0 + e < C ? __ldg(src + (int64_t)e * taps + t) : (TIn)0;
+#pragma unroll
+        for (int t = 0; t < kPackTaps<TOut>; ++t) {
+            if (first + t >= taps) break;
+            alignas(4) TOut v[kVec];
+#pragma unroll
+            for (int e = 0; e < kVec; ++e) v[e] = convert_to<TOut>(x[t][e]);
+            *reinterpret_cast<uint32_t*>(dst + (int64_t)t * cpad) = *reinterpret_cast<const uint32_t*>(v);
+            if constexpr (kSplit) dst[lo_off + (int64_t)t * cpad] = convert_to<Tf32Lo>(x[t][0]).v;
+        }
+    }
+}
 
 // Activations NCHW fp32 -> NHWC of the operand type and, in the first blocks of the same launch, the weights of the convolution
 // that follows. One launch instead of two (each cost 2 to 3 us of launch and drain beside 2 to 5 us of work: conv 72 -> 120 3x3
@@ -113,7 +121,7 @@ __global__ void __launch_bounds__(256) convert_operands_kernel(const float* __re
     if (overlap) sm100::pdl_launch_dependents();
     if (blockIdx.x < pack.blocks) {
         pack_weights_block<float, TOut, kSplit>(static_cast<const float*>(pack.w), static_cast<TOut*>(pack.out), static_cast<TOut*>(pack.lo),
-                                                pack.groups, pack.C, pack.taps, pack.cpad, pack.group_blocks, blockIdx.x);
+                                                pack, blockIdx.x);
         return;
     }
     __shared__ float tile[kCT][kPT + 1];
@@ -148,8 +156,7 @@ __global__ void __launch_bounds__(256) convert_operands_kernel(const float* __re
 // Weights alone: constants of a plan, packed once.
 template <typename TIn, typename TOut, bool kSplit>
 __global__ void __launch_bounds__(256) pack_weights_kernel(PackArgs pack) {
-    pack_weights_block<TIn, TOut, kSplit>(static_cast<const TIn*>(pack.w), static_cast<TOut*>(pack.out), static_cast<TOut*>(pack.lo), pack.groups,
-                                          pack.C, pack.taps, pack.cpad, pack.group_blocks, blockIdx.x);
+    pack_weights_block<TIn, TOut, kSplit>(static_cast<const TIn*>(pack.w), static_cast<TOut*>(pack.out), static_cast<TOut*>(pack.lo), pack, blockIdx.x);
 }
 
 // The same for rows that need no reordering: [rows, cols] -> two times [rows, cpad]. cols % 4 == 0 and cols == cpad take
@@ -334,8 +341,7 @@ __global__ void __launch_bounds__(256) transpose_bytes_kernel(TransposeArgs a, P
     sm100::pdl_wait();
     if (overlap) sm100::pdl_launch_dependents();
     if (blockIdx.x < pack.blocks) {
-        pack_weights_block<int8_t, int8_t, false>(static_cast<const int8_t*>(pack.w), static_cast<int8_t*>(pack.out), nullptr, pack.groups, pack.C,
-                                                  pack.taps, pack.cpad, pack.group_blocks, blockIdx.x);
+        pack_weights_block<int8_t, int8_t, false>(static_cast<const int8_t*>(pack.w), static_cast<int8_t*>(pack.out), nullptr, pack, blockIdx.x);
         return;
     }
     const unsigned t = blockIdx.x - pack.blocks;
@@ -389,9 +395,11 @@ PackArgs pack_args(const WeightPack* w) {
     if (w == nullptr || (int64_t)w->O * w->taps * w->cpad == 0) return p;
     p.w = w->w; p.out = w->out; p.lo = w->lo;
     p.C = w->C; p.taps = w->taps; p.cpad = w->cpad;
-    p.groups = (int64_t)w->O * (w->cpad / (4 / (int)sizeof(T)));
-    p.group_blocks = (unsigned)((p.groups + 255) / 256);
-    p.blocks = p.group_blocks * (unsigned)((w->taps + kPackTaps - 1) / kPackTaps);
+    p.per_row = Divisor((unsigned)(w->cpad / (4 / (int)sizeof(T))));
+    p.groups = (int64_t)w->O * p.per_row.d;
+    p.per_thread = sizeof(T) == 1 && p.groups >= 48 * 256 ? 9 : kPackTaps<T>;  // (reasons at pack_weights_block)
+    p.pieces = Divisor((unsigned)((w->taps + p.per_thread - 1) / p.per_thread));
+    p.blocks = (unsigned)(((p.groups + 31) / 32 * p.pieces.d + 7) / 8);
     return p;
 }
 

@@ -364,9 +364,10 @@ def test_fp32_tiles_are_those_the_gpu_tests_name(fake, case, width, tile):
     assert f"{to * og}x{tp * pg}" == tile, launches(fake)[-1]
 
 
-# Weights are packed by a thread per nine taps of a filter: blocks of the launch that converts both operands (961 taps: 107 pieces)
-@pytest.mark.parametrize("precision", [_lib.PREC_TF32, _lib.PREC_BF16, _lib.PREC_TF32X3])
-def test_large_filters_are_packed_in_pieces(fake, precision):
+# Weights are packed by a thread per nine taps of a filter (fp32; five of bf16): blocks of the launch that converts both operands. 256
+# channel groups in eight warps make one block per piece of the filters.
+@pytest.mark.parametrize("precision,taps", [(_lib.PREC_TF32, 9), (_lib.PREC_BF16, 5), (_lib.PREC_TF32X3, 9)])
+def test_large_filters_are_packed_in_pieces(fake, precision, taps):
     blocks = {}
     for k in (1, 3, 5, 31):
         fake.fake_reset()
@@ -374,4 +375,5 @@ def test_large_filters_are_packed_in_pieces(fake, precision):
         assert rc == 0, message
         assert "convert_operands" in launches(fake)[0]
         blocks[k] = int(launches(fake)[0].split(" grid ")[1].split()[0])
-    assert blocks[1] == blocks[3] and blocks[5] == blocks[3] + 2 and blocks[31] == blocks[3] + 106, blocks
+    for k in (3, 5, 31):
+        assert blocks[k] - blocks[1] == -(-k * k // taps) - 1, blocks

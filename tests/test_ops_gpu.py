@@ -384,10 +384,12 @@ def test_conv2d_s8_bit_exact(ops, rng, case, simt):
         assert np.array_equal(got, expect), f"s8 conv {case} relu={relu} simt={simt}: {np.count_nonzero(got != expect)} differ"
 
 
-# Weights packed by several threads per filter (9 taps each): a last piece that is partly there, one tap behind whole pieces, int8 (four
-# channels per thread) with and without a stride. Bounds: those of test_conv2d_tensor_core and 1e-4 for three passes; int8 equal.
+# Weights packed by several threads per filter (9, 5 or 3 taps each): a last piece that is partly there, one tap behind whole pieces,
+# groups of channels that end inside a warp, int8 (four channels per thread, nine taps for many filters). Bounds: those of
+# test_conv2d_tensor_core and 1e-4 for three passes; int8 equal.
 @pytest.mark.parametrize("precision", ["tf32", "bf16", "tf32x3", "s8"])
-@pytest.mark.parametrize("N,C,H,W,O,KH,KW", [(2, 3, 12, 17, 33, 5, 5), (1, 5, 14, 13, 20, 11, 11), (1, 40, 9, 11, 70, 2, 5), (2, 2, 31, 8, 9, 19, 1)])
+@pytest.mark.parametrize("N,C,H,W,O,KH,KW", [(2, 3, 12, 17, 33, 5, 5), (1, 5, 14, 13, 20, 11, 11), (1, 40, 9, 11, 70, 2, 5), (2, 2, 31, 8, 9, 19, 1),
+                                             (1, 130, 5, 6, 400, 5, 5)])
 def test_conv2d_weights_of_large_filters(ops, rng, N, C, H, W, O, KH, KW, precision):
     pad = (KH // 2, KW // 2)
     if precision == "s8":
