@@ -73,10 +73,10 @@ __global__ void __launch_bounds__(kThreads) conv2d_direct_kernel(const TIn* __re
 // ptxas fuses mul.rn.f32x2 + add.rn.f32x2 into one fused multiply-add, which rounds once and changes the bits. The product
 // is therefore formed as fma(x, w, -0) with a -0 that is a kernel argument (fma(x, w, -0) is the rounded product for every
 // x and w, the signs of zeros included), which nothing can fold.
-// Measured, 128 -> 128 channels 3x3 at 28x28 and 32 images: 646 us with scalar arithmetic, 275 us = 26.9 TFLOP/s now (0.74 of
-// the packed bound at 1.965 GHz, but the pipe is busy for 97 % of the clocks on an SM that holds three blocks: the clock falls
-// to 1.63 GHz under it). ResNet-18 at 32 images 11.3 -> 4.4 ms. Weights doubled in shared memory or channels and pixels paired
-// crosswise to spare the register moves, unrolling two stages and rolling the k loop up gained nothing.
+// Measured, 128 -> 128 channels 3x3 at 28x28 and 32 images: 646 us with scalar arithmetic, 275 us = 26.9 TFLOP/s now, 0.74 of
+// the packed bound at 1.965 GHz. ncu: the pipe is busy for 97 % of the clocks on the SMs that work throughout and 85 % on average, as
+// there are 2.65 blocks for each SM, two of them at a time, at 1.89 GHz. ResNet-18 at 32 images 11.3 -> 4.4 ms. Weights doubled in shared
+// memory or channels and pixels paired crosswise to spare the register moves, unrolling two stages and rolling the k loop up gained nothing.
 //
 // Half of the warps compute, the other half feed them: the im2col values of KC consecutive k = (rc, rh, rw) by 4-byte
 // cp.async (zeros outside the image and past the last k: acc + 0 is the identity, acc is never -0) and the weights, into a ring of

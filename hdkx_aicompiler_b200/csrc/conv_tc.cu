@@ -822,7 +822,9 @@ namespace {
 // channels without a residual; 88, 95 and 107 at 32, 16 and 8 with one), runs of 4 twice that. Among 60 launches timed with up to 30
 // boxes each, a cost per sector alone traded whole waves for longer runs: 31 -> 331 1x1 stride 2, 56x54, 61 images, 1x14x9 boxes
 // 52 us and 1x4x27 60; 20 -> 463 on 101x103, 53 images, 158 and 172. In launches of one wave the box hardly matters (64 -> 64
-// 3x3 at 56x56, one image: 11.0 to 11.3 us from 128 down to 28 pixels a box).
+// 3x3 at 56x56, one image: 11.0 to 11.3 us from 128 down to 28 pixels a box). All of these were measured with 64-bit addresses in the
+// epilogue; nchw_store32 takes up to 0.6 of its time (95 -> 120 1x1 at 33x36, 50 images 21.3 -> 12.9 us a launch), so the weights given to
+// it here are too high by as much and have not been fitted again.
 void pick_tile_nchw(int N, int OH, int OW, int Cout, int num_kb, int kb_bytes, int* BW, int* BH, int* BNI) {
     const int bn_out = Cout <= 64 ? 64 : (Cout <= 128 ? 128 : 256);
     const int tiles_c = (Cout + bn_out - 1) / bn_out;
@@ -891,7 +893,8 @@ bool split_fits(long long tiles, int s, long long* late) {
 //                                      unsplit without it, tf32 42 -> 113 3x3 at 11x11, 30 images, 16.1 against 14.0 us; 5 with it;
 //                                      427 -> 36 1x1 at 8x7, 7 images, 11.6 split, 12.4 unsplit)
 // Into NCHW what this chooses was 1.4 % behind the fastest form on average, and one launch behind the unsplit one by more than
-// 1 %. (One figure for every width, 3000, made wide splits of short reductions slower than no split: bf16
+// 1 %, both with the epilogue of 64-bit addresses, which unsplit launches below 4 GiB have left since (nchw_store32): the unsplit tails
+// and the figures into NCHW have not been fitted again. (One figure for every width, 3000, made wide splits of short reductions slower than no split: bf16
 // 1024 -> 1024 1x1 at 7x7 and 24 images 14.7 us per layer in two parts of 256 channels, 11.3 unsplit; 256 -> 256 3x3 at
 // 14x14 and 32 images 19.4 and 17.8.) A launch is kept to the clusters that the chip holds at once (split_fits; a dense
 // layer of 16 tiles in clusters of eight that did not all fit: 8.8 -> 12 us).
