@@ -849,8 +849,8 @@ int32_t cm_setup(CmParams* p, TcDType dtype, const CmPlan& plan, const void* act
     p->loads = t.loads; p->groups = 0;
     for (int l = 0; l < t.loads; ++l) {
         p->load_map[l] = (unsigned char)t.map[l];
-        p->load_h[l] = (short)t.h[l];
-        p->load_w[l] = (short)t.w[l];
+        p->load_h[l] = t.h[l];
+        p->load_w[l] = t.w[l];
         const int end = l + 1 < t.loads ? t.first[l + 1] : t.taps;
         for (int j = t.first[l]; j < end; j += c.group) {
             CmParams::Group& w = p->group[p->groups++];

@@ -44,7 +44,7 @@ struct alignas(64) CmParams {
     const void* residual;
     void* out;
     int* status;
-    short load_h[kMaxLoads], load_w[kMaxLoads];  // first row and column of the box, from the tile's first pixel
+    int load_h[kMaxLoads], load_w[kMaxLoads];  // first row and column of the box, from the tile's first pixel (paddings and dilations have 24 bits)
     unsigned char load_map[kMaxLoads];
     Group group[kMaxTaps + 1];
 };

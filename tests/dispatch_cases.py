@@ -64,6 +64,13 @@ CHMAJOR = [
     ("s8", (5, 31, 64, 64, 64, 3, 3, 1, 1, 1), True), ("s8", (1, 12, 41, 41, 129, 7, 3, 2, 3, 2), False),
 ]
 
+# ... and with taps further than 2^15 pixels from their result: precision, images, channels, h, w, output channels, filter, stride, padding, dilation
+CHMAJOR_FAR = [
+    ("s8", 1, 16, 1, 50000, 32, (1, 3), 1, (0, 0), (1, 17000)), ("s8", 1, 16, 1, 64, 8, (1, 3), 1, (0, 33000), (1, 1)), ("s8", 1, 3, 40005, 1, 5, (3, 1), 1, (0, 0), (20000, 1)),
+    ("s8", 1, 20, 3, 70003, 33, (1, 3), 2, (0, 0), (1, 34000)), ("tf32", 1, 64, 1, 50000, 128, (1, 3), 1, (0, 0), (1, 17000)),
+    ("tf32", 1, 64, 1, 40000, 128, (1, 3), 1, (0, 33000), (1, 1)),
+]
+
 # Layers of a plan that it takes, NHWC results: (images, channels, h, w, output channels, k, stride). chmajor_layers is that layer, a second one
 # of its output channels with the first one's result as residual (1x1, stride 1), and a pooling that keeps its result NHWC.
 CHMAJOR_LAYERS = [

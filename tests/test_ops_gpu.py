@@ -469,6 +469,22 @@ def test_conv2d_channel_major(ops, rng, precision, case, vec):
             assert min(max_abs, max_rel) <= 2e-5 * max(1.0, np.sqrt(C * KH * KW) / 8), f"{name} {case}: {max_abs:.3e} {max_rel:.3e}"
 
 
+# Taps further than 2^15 pixels from their result, by dilation or by padding; bounds of test_conv2d_channel_major
+@pytest.mark.parametrize("precision,N,C,H,W,O,k,s,p,d", dispatch_cases.CHMAJOR_FAR)
+def test_conv2d_taps_far_from_their_pixel(ops, rng, precision, N, C, H, W, O, k, s, p, d):
+    if precision == "s8":
+        x, w, b, m, sh = (dev(a) for a in s8_inputs(rng, N, C, H, W, O, *k))
+        got = ops.nn_conv2d_s8(x, w, b, m, sh, (s, s), p, d)
+        assert ops.device_status() == 0
+        assert torch.equal(got, ops.nn_conv2d_s8(x, w, b, m, sh, (s, s), p, d, simt=True))
+        return
+    x, w, b = conv_inputs(rng, N, C, H, W, O, *k)
+    got = host(ops.nn_conv2d(dev(x), dev(w), dev(b), (s, s), p, d, precision=precision))
+    assert ops.device_status() == 0
+    max_abs, max_rel = ref_metric(got, port.conv2d(port.round_tf32(x), port.round_tf32(w), b, (s, s), p, d))
+    assert min(max_abs, max_rel) <= 2e-5 * max(1.0, np.sqrt(C * k[0] * k[1]) / 8), f"{max_abs:.3e} {max_rel:.3e}"
+
+
 # One plane of 4,194,308 pixels: its 64-row tiles are more than the second grid dimension holds
 def test_conv2d_s8_plane_beyond_the_second_grid_dimension(ops, rng):
     x, w, b, m, sh = (dev(a) for a in s8_inputs(rng, 1, 3, 1048577, 4, 5, 1, 1))
