@@ -620,6 +620,9 @@ int32_t launch_kind(const CmParams& p, cudaStream_t stream) {
 }
 
 int div_up(int a, int b) { return (a + b - 1) / b; }
+long long tiles(const CmGeometry& g, int BW, int BH, int BNI) {
+    return (long long)div_up(g.Cout, kM) * div_up(g.OW, BW) * div_up(g.OH, BH) * div_up(g.N, BNI);
+}
 int floor_half(int v) { return (v - (v & 1)) / 2; }
 
 // The taps of a filter as loads: those that share a box (all of them at stride 1, those of one row and column parity at stride 2) or
@@ -700,7 +703,7 @@ bool box_cost(const CmGeometry& g, const Grouping& t, int staging, int BW, int B
     b->w_slots = w_slots < kMaxSlots ? w_slots : kMaxSlots;
     int groups = 0;
     for (int l = 0; l < t.loads; ++l) groups += div_up((l + 1 < t.loads ? t.first[l + 1] : t.taps) - t.first[l], b->group);
-    const long long items = (long long)div_up(g.Cout, kM) * div_up(g.OW, BW) * div_up(g.OH, BH) * div_up(g.N, BNI);
+    const long long items = tiles(g, BW, BH, BNI);
     // What a tile costs: its rows at the rate the copies reach shared memory, or its instructions, which fetch 128 + n rows of 32 bytes at
     // 64 bytes a clock, and the hand-over of a group; then its epilogue, which overlaps the next tile. (Boxes chosen so over 200 drawn layers.)
     const double fill = (double)g.cblocks * ((double)t.loads * rows_px + (double)t.taps * rows_w) * 2.6;
@@ -765,9 +768,10 @@ bool choose(CmPlan* plan, TcDType dtype, const ConvDims& d) {
 
 }  // namespace
 
-// Integers take this form wherever it applies: of 210 drawn layers (device time of a call) it was the faster one in all but five, by 1.25
-// in the geometric mean (91 -> 427 1x1 at 58x59, 169 images: 683 -> 254 us; 48x51, 40 -> 123 3x3, 18 images: 22.0 -> 23.6), and a result needs
-// no second copy. With fp32 results the pixel-major kernel has less to hand over per K block, splits long reductions of few tiles over
+// Integers take this form wherever it applies: of 260 drawn layers (device time of a call, against the pixel-major forms of results in planes: byte
+// stores, or NHWC and a transposition) it was the faster one by 1.32 in the geometric mean; seven lost more than 2 %, 1x1 layers to 32 and fewer
+// channels up to 6 % (53 -> 8 of stride 2 at 80x78, 68 images: 19.2 -> 20.4), 180 -> 17 3x3 at 16x16, 51 images 12.6 -> 15.4, 64 -> 64 3x3 at 12x13,
+// 165 images 12.2 -> 14.0. A model of the pixel-major forms, fitted to the same layers, chose worse than not choosing. With fp32 results the pixel-major kernel has less to hand over per K block, splits long reductions of few tiles over
 // clusters and takes 64 channels at a time, so modelled clocks decide. Its model ends with the last K block; 30 clocks per channel of a
 // tile stand for the epilogue of an unsplit one. Over 227 drawn layers (tf32 and bf16, with and without a residual) the choice was 1.6 %
 // behind the faster form and 4 % ahead of the pixel-major kernel alone; one layer lost 12 % by it, 24 -> 30 3x3 at 92x95, 32 images, whose few
@@ -813,8 +817,7 @@ const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcO
         if (out_mode == kOutNCHW_F32) {
             const double epilogue = p.split > 1 ? 0.0 : 30.0 * (d.O < cfg.bn ? d.O : cfg.bn);
             const CmChoice& c = e.plan.c;
-            const long long items = (long long)div_up(d.O, kM) * div_up(d.OW, c.BW) * div_up(d.OH, c.BH) * div_up(d.N, c.BNI);
-            const double ahead = d.KH * d.KW == 1 && items <= kNumSMs ? 2800.0 : 1000.0;
+            const double ahead = d.KH * d.KW == 1 && tiles(e.plan.g, c.BW, c.BH, c.BNI) <= kNumSMs ? 2800.0 : 1000.0;
             e.use = rc == KXC_B200_OK && (d.O > 32 || e.plan.g.cblocks > 1) && c.cost + ahead < cfg.clocks + epilogue;
         } else {
             const double ahead = d.KH * d.KW == 1 ? (p.split > 1 ? 1.15 : 0.80) : (d.SH == 1 && p.split <= 2 ? 0.83 : 0.95);
@@ -826,14 +829,19 @@ const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcO
     return e.use ? &e.plan : nullptr;
 }
 
-int32_t cm_setup(CmParams* p, TcDType dtype, const CmPlan& plan, const void* act_nhwc, const void* w_packed, int cpad, int* status_word) {
+int cm_weight_pad(TcDType t, int c, const CmPlan& plan) {
+    const int e128 = kRow / tc_elem_bytes(t);
+    return tiles(plan.g, plan.c.BW, plan.c.BH, plan.c.BNI) > kNumSMs ? div_up(c, e128) * e128 : cm_channel_pad(t, c);
+}
+
+int32_t cm_setup(CmParams* p, TcDType dtype, const CmPlan& plan, const void* act_nhwc, const void* w_packed, int cpad, int w_cpad, int* status_word) {
     const CmGeometry& g = plan.g;
     const CmChoice& c = plan.c;
     Grouping t;
     if (!group_taps(g, c.shared != 0, &t)) return fail(KXC_B200_ERR_INVALID, "channel-major conv: %dx%d filter", g.KH, g.KW);
     const int eb = tc_elem_bytes(dtype);
-    const uint64_t px = (uint64_t)cpad * eb;
-    if (px % 16 != 0) return fail(KXC_B200_ERR_INVALID, "channel-major conv: %d padded channels x %d bytes", cpad, eb);
+    const uint64_t px = (uint64_t)cpad * eb, tap = (uint64_t)w_cpad * eb;
+    if (px % 16 != 0 || tap % 16 != 0) return fail(KXC_B200_ERR_INVALID, "channel-major conv: %d, %d padded channels x %d bytes", cpad, w_cpad, eb);
     p->N = g.N; p->OH = g.OH; p->OW = g.OW; p->Cout = g.Cout;
     p->kb_elems = g.kb_elems; p->cblocks = g.cblocks; p->last_steps = g.last_steps;
     p->BW = c.BW; p->BH = c.BH; p->BNI = c.BNI; p->HB = c.HB; p->WB = c.WB; p->n_cols = c.n;
@@ -874,8 +882,8 @@ int32_t cm_setup(CmParams* p, TcDType dtype, const CmPlan& plan, const void* act
         const uint64_t strides[3] = {px * s, px * s * g.W, px * g.H * g.W};
         KXC_TRY(tc_make_tmap(&p->tmA[par], dtype, 4, base + ((size_t)hp * g.W + wp) * px, dims, strides, box, kRow));
     }
-    const uint64_t wdims[3] = {(uint64_t)cpad, (uint64_t)g.Cout, (uint64_t)(g.KH * g.KW)};
-    const uint64_t wstr[2] = {px * g.KH * g.KW, px};
+    const uint64_t wdims[3] = {(uint64_t)w_cpad, (uint64_t)g.Cout, (uint64_t)(g.KH * g.KW)};
+    const uint64_t wstr[2] = {tap * g.KH * g.KW, tap};
     const uint32_t wbox[3] = {(uint32_t)g.kb_elems, (uint32_t)rows_w, 1u};
     KXC_TRY(tc_make_tmap(&p->tmW, dtype, 3, const_cast<void*>(w_packed), wdims, wstr, wbox, kRow));
     p->status = status_word;

@@ -1,6 +1,6 @@
 // Convolution with the output channels as the MMA's rows (conv_chmajor.cu): into the reference's layout bf16 and tf32 operands with fp32
-// results, int8 with requantized ones; into NHWC bf16 and tf32. Activations NHWC, weights [Cout][KH * KW][cpad], both of the operand type, `cpad` channels in
-// multiples of 16 bytes.
+// results, int8 with requantized ones; into NHWC bf16 and tf32. Activations NHWC of `cpad` channels, weights [Cout][KH * KW][w_cpad], both of the operand
+// type and in multiples of 16 bytes.
 #pragma once
 
 #include <cuda.h>
@@ -66,13 +66,18 @@ struct CmPlan {
 // last choices, which depend on the geometry and the device alone; valid until the thread's next call.
 const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcOutMode out_mode = kOutNCHW_F32);
 // `status_word`: as in tc_setup_conv.
-int32_t cm_setup(CmParams* p, TcDType dtype, const CmPlan& plan, const void* act_nhwc, const void* w_packed, int cpad, int* status_word = nullptr);
+int32_t cm_setup(CmParams* p, TcDType dtype, const CmPlan& plan, const void* act_nhwc, const void* w_packed, int cpad, int w_cpad, int* status_word = nullptr);
 int32_t cm_launch(TcDType dtype, const CmParams& p, cudaStream_t stream);
 
-// Channels an operand of this form is padded to.
+// Channels that an operator pads its pixels to: whole 32-byte sectors (pixels of 16 bytes more made the copies up to twice as long: tf32 1 -> 76
+// 5x5 at 46x44, 28 images, a call 31.7 -> 21.1 us; int8 44 -> 46 3x3 of stride 2 at 53x56, 85 images 31.6 -> 23.5; none of 420 drawn layers lost 2 %).
 inline int cm_channel_pad(TcDType t, int c) {
-    const int e16 = 16 / tc_elem_bytes(t);
-    return (c + e16 - 1) / e16 * e16;
+    const int e32 = 32 / tc_elem_bytes(t);
+    return (c + e32 - 1) / e32 * e32;
 }
+// ... and its filters' taps. Of a launch with more tiles than SMs, which loads them once per tile: whole rows of 128 bytes, the copies' unit
+// (int8, a call, with sectors / so: 11 -> 137 5x5 at 20x19, 235 images 98.3 / 50.1 us, 16 -> 158 5x5 at 63x65, 18 images 65.2 / 39.0). One wave
+// does not earn back the longer packing (64 -> 32 3x3 at 8x11, one image 7.3 / 7.6).
+int cm_weight_pad(TcDType t, int c, const CmPlan& plan);
 
 }  // namespace kxc_b200

@@ -135,12 +135,12 @@ extern "C" int32_t kxc_b200_nn_conv2d_static_scratch(void** packed_args, const k
     KXC_TRY(scratch_for_current_device(&sc));
     unsigned char* act = sc.base;
     unsigned char* wp = sc.base + act_bytes;
-    if (const CmPlan* cm = cm_wanted(dt, d, 0)) {  // (its operands are padded less and fit where these do)
+    if (const CmPlan* cm = cm_wanted(dt, d, 0)) {  // (its operands, filters in sectors too, are padded no further and fit where these do)
         const int cm_pad = cm_channel_pad(dt, d.C);
         const WeightPack pack{weight, wp, nullptr, d.O, d.C, d.KH * d.KW, cm_pad};
         KXC_TRY(convert_operands(data, act, nullptr, dt, d.N, d.C, d.H * d.W, cm_pad, &pack, s, true));
         CmParams p{};
-        KXC_TRY(cm_setup(&p, dt, *cm, act, wp, cm_pad, sc.status));
+        KXC_TRY(cm_setup(&p, dt, *cm, act, wp, cm_pad, cm_pad, sc.status));
         p.bias = bias;
         p.residual = residual;
         p.out = out;

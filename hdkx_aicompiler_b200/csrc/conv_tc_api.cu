@@ -122,17 +122,18 @@ int32_t conv2d_tensor_core(const float* data, const float* weight, const float* 
     const int eb = tc_elem_bytes(dt);
     const CmPlan* cm = cm_wanted(dt, d, 0);
     const int cpad = cm != nullptr ? cm_channel_pad(dt, d.C) : tc_channel_pad(dt, d.C);
+    const int w_cpad = cm != nullptr ? cm_weight_pad(dt, d.C, *cm) : cpad;
     const size_t act_bytes = align_up((size_t)d.N * d.H * d.W * cpad * eb, 1024);
-    const size_t w_bytes = align_up((size_t)d.O * d.KH * d.KW * cpad * eb, 1024);
+    const size_t w_bytes = align_up((size_t)d.O * d.KH * d.KW * w_cpad * eb, 1024);
     StreamScratch ws(s);
     KXC_TRY(ws.alloc(act_bytes + w_bytes));
     uint8_t* act = static_cast<uint8_t*>(ws.ptr);
     uint8_t* wp = act + act_bytes;
-    const WeightPack pack{weight, wp, nullptr, d.O, d.C, d.KH * d.KW, cpad};
+    const WeightPack pack{weight, wp, nullptr, d.O, d.C, d.KH * d.KW, w_cpad};
     KXC_TRY(convert(act, nullptr, dt, cpad, &pack));
     if (cm != nullptr) {
         CmParams p{};
-        KXC_TRY(cm_setup(&p, dt, *cm, act, wp, cpad));
+        KXC_TRY(cm_setup(&p, dt, *cm, act, wp, cpad, w_cpad));
         p.bias = bias;
         p.residual = residual;
         p.out = out;
@@ -223,20 +224,20 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     const int in_h = d.H, in_w = d.W;
     const int conv_h = subsample ? d.OH : d.H, conv_w = subsample ? d.OW : d.W;  // the tensor the kernel convolves
     if (const CmPlan* cm = cm_wanted(dt, subsample ? without_stride(d) : d, 0)) {
-        const int cm_pad = cm_channel_pad(dt, d.C);
+        const int cm_pad = cm_channel_pad(dt, d.C), w_cpad = cm_weight_pad(dt, d.C, *cm);
         const size_t cm_act = align_up((size_t)d.N * conv_h * conv_w * cm_pad, 1024);
         StreamScratch ws(s);
-        KXC_TRY(ws.alloc(cm_act + align_up((size_t)d.O * d.KH * d.KW * cm_pad, 1024)));
+        KXC_TRY(ws.alloc(cm_act + align_up((size_t)d.O * d.KH * d.KW * w_cpad, 1024)));
         uint8_t* act = static_cast<uint8_t*>(ws.ptr);
         uint8_t* wp = act + cm_act;
-        const WeightPack pack{weight, wp, nullptr, d.O, d.C, d.KH * d.KW, cm_pad};
+        const WeightPack pack{weight, wp, nullptr, d.O, d.C, d.KH * d.KW, w_cpad};
         if (subsample) {
             KXC_TRY(convert_operands_s8_subsample(data, reinterpret_cast<int8_t*>(act), d.N, d.C, in_h, in_w, d.OH, d.OW, d.SH, cm_pad, &pack, s, true));
         } else {
             KXC_TRY(convert_operands(data, act, nullptr, dt, d.N, d.C, d.H * d.W, cm_pad, &pack, s, true));
         }
         CmParams p{};
-        KXC_TRY(cm_setup(&p, dt, *cm, act, wp, cm_pad));
+        KXC_TRY(cm_setup(&p, dt, *cm, act, wp, cm_pad, w_cpad));
         p.bias_i32 = bias;
         p.multiplier = multiplier;
         p.shift = shift;

@@ -1010,7 +1010,7 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
                                              pw.KH, pw.KW, st.pool.strides[0], st.pad_h, st.pad_w, st.pool.pool_size[0], st.pool.pool_size[1]));
                 } else if (const CmPlan* cm = cm_wanted(dt, conv_dims(st, pw), st.params.weights_ready, om)) {
                     st.direct = 6;
-                    KXC_TRY(cm_setup(&st.cm, dt, *cm, pl->storage(st.in0), pw.ptr, st.cpad));
+                    KXC_TRY(cm_setup(&st.cm, dt, *cm, pl->storage(st.in0), pw.ptr, st.cpad, st.cpad));
                     st.cm.relu = st.relu ? 1 : 0;
                     st.cm.pixels = !st.out_is_graph_output;
                     st.cm.round_out_tf32 = !st.out_is_graph_output && dt == kTcTF32 ? 1 : 0;
