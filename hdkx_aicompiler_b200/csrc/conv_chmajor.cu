@@ -784,7 +784,8 @@ bool choose(CmPlan* plan, TcDType dtype, const ConvDims& d) {
 // measured. 3x3 layers, whose pixels the pixel-major kernel loads nine times over, are ahead of their model: tf32 128 -> 128 at 28x28 and
 // 256 -> 256 at 14x14 gained up to the line, 512 -> 512 at 7x7 (two images to a tile, the weights' rows bound both forms) lost where the model said
 // so: 32 images 39.7 / 77.1 us, 256 images 103.5 / 154.0. Split reductions of 1x1 layers lose 8 to 17 % up to a ratio of 1 (64 x 768 -> 160 at 7x7
-// 14.2 / 15.2) and gain from 1.15 on, longer splits of wider filters are level there. ResNet-18 tf32 32 images 476.8 / 419.6 us, 64: 739 / 661, 256:
+// 14.2 / 15.2) and gain from 1.15 on. Splits of wider filters over three and more CTAs keep what the models call level: 40 drawn layers of
+// ratios 0.86 to 1.02 were 0.985 to 1.43 times as fast here, bf16 192 -> 160 3x3 at 13x11, 28 images, 18.9 / 15.2 us, at 0.997. ResNet-18 tf32 32 images 476.8 / 419.6 us, 64: 739 / 661, 256:
 // 2156 / 2028; bf16 32: 265.7 / 254.2, 128: 552 / 545. bf16 layers of stride 2 keep the pixel-major kernel: with a 1x1 layer beside
 // them they are one launch of it (two outputs), and alone they give the same bits as there.
 const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcOutMode out_mode) {
@@ -820,7 +821,7 @@ const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcO
             const double ahead = d.KH * d.KW == 1 && tiles(e.plan.g, c.BW, c.BH, c.BNI) <= kNumSMs ? 2800.0 : 1000.0;
             e.use = rc == KXC_B200_OK && (d.O > 32 || e.plan.g.cblocks > 1) && c.cost + ahead < cfg.clocks + epilogue;
         } else {
-            const double ahead = d.KH * d.KW == 1 ? (p.split > 1 ? 1.15 : 0.80) : (d.SH == 1 && p.split <= 2 ? 0.83 : 0.95);
+            const double ahead = d.KH * d.KW == 1 ? (p.split > 1 ? 1.15 : 0.80) : (p.split > 2 ? 1.0 : (d.SH == 1 ? 0.83 : 0.95));
             e.use = rc == KXC_B200_OK && cfg.clocks >= ahead * e.plan.c.cost && !(dtype == kTcBF16 && d.SH == 2);
         }
         // (what a failed query of the device decided is not kept)

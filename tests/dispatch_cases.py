@@ -7,7 +7,7 @@ tests run the same shapes."""
 # (and among 8 when there are fewer than 8); last tiles of 32 to 96 channels.
 SPLIT_LAYERS = [
     ("bf16", (50, 1024, 14, 9, 32, 1), 2, 64), ("bf16", (64, 768, 7, 7, 160, 1), 2, 128), ("bf16", (40, 768, 14, 9, 32, 1), 3, 64),
-    ("bf16", (5, 768, 7, 7, 1600, 1), 3, 128), ("bf16", (33, 512, 9, 7, 288, 3), 3, 256), ("bf16", (24, 768, 14, 9, 32, 1), 4, 64),
+    ("bf16", (5, 768, 7, 7, 1600, 1), 3, 128), ("bf16", (28, 192, 13, 11, 160, 3), 3, 256), ("bf16", (33, 512, 9, 7, 288, 3), 3, 256), ("bf16", (24, 768, 14, 9, 32, 1), 4, 64),
     ("bf16", (3, 1536, 7, 7, 1600, 1), 4, 128), ("bf16", (20, 256, 13, 11, 160, 3), 4, 256), ("bf16", (24, 128, 8, 16, 32, 3), 5, 64),
     ("bf16", (5, 128, 7, 7, 1024, 3), 5, 128), ("bf16", (2, 768, 7, 7, 32, 1), 6, 64), ("bf16", (18, 128, 13, 11, 96, 3), 6, 128),
     ("bf16", (1, 192, 9, 7, 64, 3), 7, 64), ("bf16", (4, 192, 4, 6, 32, 3), 7, 64), ("bf16", (1, 192, 3, 3, 32, 3), 7, 64),
