@@ -785,9 +785,14 @@ bool choose(CmPlan* plan, TcDType dtype, const ConvDims& d) {
 // 256 -> 256 at 14x14 gained up to the line, 512 -> 512 at 7x7 (two images to a tile, the weights' rows bound both forms) lost where the model said
 // so: 32 images 39.7 / 77.1 us, 256 images 103.5 / 154.0. Split reductions of 1x1 layers lose 8 to 17 % up to a ratio of 1 (64 x 768 -> 160 at 7x7
 // 14.2 / 15.2) and gain from 1.15 on. Splits of wider filters over three and more CTAs keep what the models call level: 40 drawn layers of
-// ratios 0.86 to 1.02 were 0.985 to 1.43 times as fast here, bf16 192 -> 160 3x3 at 13x11, 28 images, 18.9 / 15.2 us, at 0.997. ResNet-18 tf32 32 images 476.8 / 419.6 us, 64: 739 / 661, 256:
-// 2156 / 2028; bf16 32: 265.7 / 254.2, 128: 552 / 545. bf16 layers of stride 2 keep the pixel-major kernel: with a 1x1 layer beside
-// them they are one launch of it (two outputs), and alone they give the same bits as there.
+// ratios 0.86 to 1.02 were 0.985 to 1.43 times as fast here, bf16 192 -> 160 3x3 at 13x11, 28 images, 18.9 / 15.2 us, at 0.997. Launches of one channel
+// block that read and write more than they multiply are the epilogue's, of which 32 channels use a quarter: tf32 1x1 layers up to a ratio
+// of 1.5 (32 -> 32 at 90x88, 45 images 161.8 / 225.8, 32 -> 40 at 76x79, 56 images 160.8 / 174.1; all 23 drawn ones lost) and 3x3 layers of 17 to 32 channels
+// from about 100 tiles on (32 -> 32 at 40x42, 61 images 66.9 / 81.2, 0.82 to 1.10; fewer tiles 1.04 to 1.18), bf16 1x1 layers of 17 to 32 channels and more
+// than one wave (64 -> 32 at 95x95, 33 images 92.4 / 100.4, 0.92 to 0.95; 16 channels gain 16 to 23 %). Of 626 drawn layers these lines
+// let 178 through, which were 1.13 times as fast (nine lost more than 3 %, the worst bf16 480 -> 416 1x1 at 33x31, 8 images, 34.8 / 39.6).
+// ResNet-18 tf32 32 images 476.8 / 419.6 us, 64: 739 / 661, 256: 2156 / 2028; bf16 32: 265.7 / 254.2, 128: 552 / 545. bf16 layers of stride 2
+// keep the pixel-major kernel: with a 1x1 layer beside them they are one launch of it (two outputs), and alone they give the same bits as there.
 const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcOutMode out_mode) {
     struct Entry {
         int key[17] = {-1};
@@ -822,7 +827,14 @@ const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcO
             e.use = rc == KXC_B200_OK && (d.O > 32 || e.plan.g.cblocks > 1) && c.cost + ahead < cfg.clocks + epilogue;
         } else {
             const double ahead = d.KH * d.KW == 1 ? (p.split > 1 ? 1.15 : 0.80) : (p.split > 2 ? 1.0 : (d.SH == 1 ? 0.83 : 0.95));
-            e.use = rc == KXC_B200_OK && cfg.clocks >= ahead * e.plan.c.cost && !(dtype == kTcBF16 && d.SH == 2);
+            const long long items = tiles(e.plan.g, e.plan.c.BW, e.plan.c.BH, e.plan.c.BNI);
+            const bool few = d.O > 16 && d.O <= 32;  // channels
+            bool stays = dtype == kTcBF16 && d.SH == 2;
+            if (e.plan.g.cblocks == 1 && d.SH == 1) {
+                if (dtype == kTcTF32) stays = d.KH * d.KW == 1 ? cfg.clocks < 1.5 * e.plan.c.cost : few && d.KH * d.KW <= 9 && items > 100;
+                else if (few && d.KH * d.KW == 1 && items > kNumSMs) stays = true;
+            }
+            e.use = rc == KXC_B200_OK && cfg.clocks >= ahead * e.plan.c.cost && !stays;
         }
         // (what a failed query of the device decided is not kept)
         if (rc != KXC_B200_OK || tc_split_capacity(2) <= 0) e.key[0] = -1;
