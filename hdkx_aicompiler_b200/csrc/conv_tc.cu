@@ -963,8 +963,10 @@ int32_t tc_setup_dual(TcParams* p, TcConfig* cfg, const void* act_nhwc, const vo
     // rank's own. Its partial sums double the exchange, which leaves nothing to gain for tiles wider than 64 channels:
     // 256 -> 512 at 14x14, block of four layers, us unsplit / 64 wide / 128 wide: one image 35.0 / 24.8 / 26.9, 8 images
     // 35.5 / 30.9 / 32.9, 16 images 41.2 / 37.1 / 37.1, 24 images 45.3 / - / 45.3; 128 -> 256 at 28x28: 4 images
-    // 28.9 / 27.2 / 29.3, 8 images 33.1 / 31.5 / 33.3. Short reductions need a margin: 64 -> 128 at 56x56, nine K blocks, whole
-    // ResNet-18 at one image 115.8 / 111.8; without the margin 2 gained 2 %, 3 1 % (and lost the bits of two launches), from 4 on level.
+    // 28.9 / 27.2 / 29.3, 8 images 33.1 / 31.5 / 33.3. Of short reductions (nine K blocks: 3x3
+    // over 64 channels) only parts of two K blocks pay, and the margin leaves those: of 85 drawn blocks (32 to 512 outputs, 8x8 to 109x109, 1 to
+    // 42 images; blocks of four layers) 56 split into five and more parts were 1.06 to 1.25 times as fast, 1.15 in the mean; 12 in three parts 0.95 to
+    // 1.11, 17 in two 0.92 to 0.99 and one 1.03. ResNet-18 at one image 115.8 / 111.8 us.
     const int kb = KH * KW * p->cblocks;
     const long long tiles64 = m_tiles * ((Cout + 63) / 64);
     long long best = (waves(m_tiles * ((Cout + 127) / 128)) * (kb + p->cblocks) * 590 + 4000) * 95 / 100;
