@@ -2,6 +2,7 @@
 import ctypes
 import functools
 import os
+import warnings
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _LIB_NAME = "libkxc_b200.so"
@@ -113,17 +114,39 @@ _NATIVE_ENTRIES = ["nn_conv2d", "nn_conv2d_s8", "nn_max_pool2d", "nn_avg_pool2d"
                    "nn_global_avg_pool2d", "plan_run"]  # in the order of native.cpp
 
 
-@functools.lru_cache(maxsize=None)
-def native():
-    """The operators' calls in native code (csrc/native.cpp), bound to the library's functions; built with it, there is no call without it."""
+def load_native():
+    """The operators' calls in native code (csrc/native.cpp), bound to the library's functions. ImportError where the file is missing or
+    belongs to another torch or Python than this process's."""
+    import torch
+
     lib = load()
+    how = "run `python -c 'import __graft_entry__ as g; g.build()'` or `make -C hdkx_aicompiler_b200/csrc`"
     try:
         from . import _native
     except ImportError as e:
-        raise ImportError(f"{os.path.join(_HERE, '_native.so')} is not usable ({e}): run `python -c 'import __graft_entry__ as g; g.build()'` "
-                          f"or `make -C hdkx_aicompiler_b200/csrc`") from e
+        raise ImportError(f"{os.path.join(_HERE, '_native.so')} is not usable ({e}): {how}") from e
+    if _native.torch_version != torch.__version__:
+        raise ImportError(f"{_native.__file__} was built with torch {_native.torch_version}, not {torch.__version__}: {how}")
     _native.bind(*[ctypes.cast(getattr(lib, "kxc_b200_" + name), vp).value for name in _NATIVE_ENTRIES])
     return _native
+
+
+class _NoNativeCalls:
+    """Answers None to every call, as native.cpp does to what is not ordinary: the callers go their general way."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+@functools.lru_cache(maxsize=None)
+def native():
+    """load_native(), or, with one warning, what leaves every call to the general path: the same kernels, about 3 us more of the
+    host's time a call."""
+    try:
+        return load_native()
+    except ImportError as e:
+        warnings.warn(f"operator calls are made from Python: {e}", RuntimeWarning, stacklevel=3)
+        return _NoNativeCalls()
 
 
 def last_error():

@@ -338,4 +338,14 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Operator calls in nativ
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__native(void) {
+    const char* here = Py_GetVersion();  // "3.12.3 (...": the binary interface is that of the first two numbers
+    const size_t minor = strcspn(strchr(PY_VERSION, '.') + 1, ".") + (size_t)(strchr(PY_VERSION, '.') + 1 - PY_VERSION);
+    if (strncmp(here, PY_VERSION, minor) != 0 || (here[minor] >= '0' && here[minor] <= '9')) {
+        PyErr_Format(PyExc_ImportError, "built for Python " PY_VERSION ", not %.10s", here);
+        return nullptr;
+    }
+    PyObject* m = PyModule_Create(&module);
+    if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", KXC_TORCH_VERSION) != 0) Py_CLEAR(m);
+    return m;
+}
