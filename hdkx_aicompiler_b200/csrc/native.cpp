@@ -54,6 +54,7 @@ const at::Tensor* plain(PyObject* o, at::ScalarType type, int rank) {
     return &t;
 }
 void* address(const at::Tensor& t) { return const_cast<void*>(t.const_data_ptr()); }
+void* result_address(const at::Tensor& t) { return t.mutable_data_ptr(); }  // (memory shared with a lazy clone becomes its own first)
 
 // `n` plain whole numbers of a tuple or list.
 bool numbers(PyObject* o, int n, int32_t* out) {
@@ -124,7 +125,7 @@ PyObject* conv2d(PyObject*, PyObject* const* a, Py_ssize_t n) {
     } else {
         out = at::empty(at::IntArrayRef(dims, 4), x->options().requires_grad(false));
     }
-    ptrs[at] = address(out);
+    ptrs[at] = result_address(out);
     const kxc_b200_conv2d_desc desc = {(int32_t)x->size(0), (int32_t)x->size(1), (int32_t)x->size(2), (int32_t)x->size(3), (int32_t)w->size(0),
                                        (int32_t)w->size(2), (int32_t)w->size(3), s[0], s[1], p[0], p[1], d[0], d[1], flags, (int32_t)PyLong_AsLong(a[8])};
     return call(*x, out, [&](void* stream) { return lib.conv2d(ptrs, &desc, stream); });
@@ -149,7 +150,7 @@ PyObject* conv2d_s8(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t oh = (h + 2 * p[0] - ((kh - 1) * d[0] + 1)) / s[0] + 1, ow = (wd + 2 * p[1] - ((kw - 1) * d[1] + 1)) / s[1] + 1;
     const int64_t dims[4] = {x->size(0), nhwc ? oh : o, nhwc ? ow : oh, nhwc ? o : ow};
     const at::Tensor out = at::empty(at::IntArrayRef(dims, 4), x->options().requires_grad(false));
-    void* ptrs[6] = {address(*x), address(*w), address(*q[0]), address(*q[1]), address(*q[2]), address(out)};
+    void* ptrs[6] = {address(*x), address(*w), address(*q[0]), address(*q[1]), address(*q[2]), result_address(out)};
     const int32_t flags = KXC_B200_BIAS | (relu ? KXC_B200_RELU : 0) | (nhwc ? KXC_B200_NHWC : 0);
     const kxc_b200_conv2d_desc desc = {(int32_t)x->size(0), (int32_t)x->size(C), (int32_t)h, (int32_t)wd, (int32_t)o, (int32_t)kh, (int32_t)kw, s[0], s[1], p[0], p[1],
                                        d[0], d[1], flags, simt ? KXC_B200_PREC_SIMT : KXC_B200_PREC_FP32};
@@ -184,7 +185,7 @@ PyObject* pool(Entry entry, PyObject* const* a, Py_ssize_t n, bool chain) {
     } else {
         out = at::empty(at::IntArrayRef(dims, 4), x->options().requires_grad(false));
     }
-    ptrs[at] = address(out);
+    ptrs[at] = result_address(out);
     const kxc_b200_pool2d_desc desc = {(int32_t)x->size(0), (int32_t)x->size(1), (int32_t)x->size(2), (int32_t)x->size(3), k[0], k[1], s[0], s[1], p[0], p[1], p[2], p[3], ceil_mode ? 1 : 0};
     return call(*x, out, [&](void* stream) { return entry(ptrs, &desc, stream); });
     END_HANDLE_TH_ERRORS
@@ -200,7 +201,7 @@ PyObject* global_avg_pool2d(PyObject*, PyObject* o) {
     if (x == nullptr || !small(*x)) Py_RETURN_NONE;
     const int64_t dims[4] = {x->size(0), x->size(1), 1, 1};
     const at::Tensor out = at::empty(at::IntArrayRef(dims, 4), x->options().requires_grad(false));
-    void* ptrs[2] = {address(*x), address(out)};
+    void* ptrs[2] = {address(*x), result_address(out)};
     return call(*x, out, [&](void* stream) {
         return lib.gap(ptrs, (int32_t)x->size(0), (int32_t)x->size(1), (int32_t)x->size(2), (int32_t)x->size(3), stream);
     });
@@ -212,7 +213,7 @@ PyObject* flatten(PyObject*, PyObject* o) {
     if (x == nullptr || x->dim() < 1) Py_RETURN_NONE;
     const int64_t dims[2] = {x->size(0), x->numel() / x->size(0)};
     const at::Tensor out = at::empty(at::IntArrayRef(dims, 2), x->options().requires_grad(false));
-    void* ptrs[2] = {address(*x), address(out)};
+    void* ptrs[2] = {address(*x), result_address(out)};
     return call(*x, out, [&](void* stream) { return lib.flatten(ptrs, x->numel(), stream); });
     END_HANDLE_TH_ERRORS
 }
@@ -221,7 +222,7 @@ PyObject* relu(PyObject*, PyObject* o) {
     const at::Tensor* x = ordinary_state() ? plain(o, at::kFloat, -1) : nullptr;
     if (x == nullptr) Py_RETURN_NONE;
     const at::Tensor out = at::empty(x->sizes(), x->options().requires_grad(false));
-    void* ptrs[2] = {address(*x), address(out)};
+    void* ptrs[2] = {address(*x), result_address(out)};
     return call(*x, out, [&](void* stream) { return lib.relu(ptrs, x->numel(), stream); });
     END_HANDLE_TH_ERRORS
 }
@@ -237,7 +238,7 @@ PyObject* softmax(PyObject*, PyObject* const* a, Py_ssize_t n) {
     for (int i = 0; i < desc.rank; ++i) desc.shape[i] = x->size(i);
     desc.axis = (int32_t)axis;
     const at::Tensor out = at::empty(x->sizes(), x->options().requires_grad(false));
-    void* ptrs[2] = {address(*x), address(out)};
+    void* ptrs[2] = {address(*x), result_address(out)};
     return call(*x, out, [&](void* stream) { return lib.softmax(ptrs, &desc, stream); });
     END_HANDLE_TH_ERRORS
 }
@@ -258,7 +259,7 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
     const int64_t dims[2] = {a->size(0), b->size(trans ? 0 : 1)};
     const at::Tensor out = at::empty(at::IntArrayRef(dims, 2), a->options().requires_grad(false));
-    ptrs[at] = address(out);
+    ptrs[at] = result_address(out);
     const kxc_b200_gemm_desc desc = {(int32_t)dims[0], (int32_t)dims[1], (int32_t)a->size(1), 1.0f, 1.0f, 0, trans ? 1 : 0, has_c ? 1 : 0, (int32_t)PyLong_AsLong(args[4])};
     return call(*a, out, [&](void* stream) { return lib.gemm(ptrs, &desc, stream); });
     END_HANDLE_TH_ERRORS
@@ -281,7 +282,7 @@ PyObject* plan_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
         args[i] = address(*t);
     }
     memcpy(args + inputs, PyBytes_AS_STRING(a[1]), (size_t)constants * sizeof(void*));
-    args[inputs + constants] = address(*out);
+    args[inputs + constants] = result_address(*out);
     void* handle = PyLong_Check(a[0]) ? PyLong_AsVoidPtr(a[0]) : nullptr;
     if (handle == nullptr) {
         PyErr_Clear();

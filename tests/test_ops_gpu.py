@@ -941,6 +941,21 @@ def test_native_calls_refuse_what_the_general_path_refuses(ops, rng, monkeypatch
     torch.cuda.synchronize()
 
 
+def test_results_into_a_lazy_clone_leave_its_source_alone(ops, rng):
+    """Memory that `out` shares until it is written: the source keeps its values, the clone gets the result."""
+    x, w, b = (dev(a) for a in conv_inputs(rng, 2, 5, 9, 8, 7, 3, 3))
+    a, r = torch.rand(2, 5, 9, 8, device="cuda"), torch.rand(2, 5, 5, 4, device="cuda")
+    from hdkx_aicompiler_b200 import plan, relay
+    v = relay.Var("input", (2, 5, 9, 8))
+    graph = plan.CompiledGraph(relay.Function([v], relay.Call("nn_conv2d", [v, relay.Constant(w), relay.Constant(b)], relay.Conv2DAttrs((1, 1), (1,) * 4, (1, 1), 1))), "bf16")
+    for call, shape in ((lambda out: ops.nn_conv2d(x, w, b, (1, 1), (1, 1), out=out), (2, 7, 9, 8)),
+                        (lambda out: ops.max_pool2d_add_relu(a, r, (3, 3), (2, 2), (1, 1, 1, 1), out=out), (2, 5, 5, 4)), (lambda out: graph.run(a, out=out), (2, 7, 9, 8))):
+        source = torch.full(shape, 7.0, device="cuda")
+        clone = torch._lazy_clone(source)
+        expect = call(torch.empty(shape, device="cuda"))
+        assert torch.equal(call(clone), expect) and torch.equal(clone, expect) and bool((source == 7).all())
+
+
 def test_native_calls_leave_modes_and_subclasses_alone(ops):
     from torch.utils._python_dispatch import TorchDispatchMode
 
