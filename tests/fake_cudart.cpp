@@ -16,6 +16,7 @@ std::map<const void*, std::string> kernels;
 std::string log_text;
 size_t pool_limit = SIZE_MAX;
 int occupancy_failures = 0;
+int encoded = 0;  // tensor maps since fake_reset
 cudaError_t last = cudaSuccess;
 uintptr_t next_address = 1ull << 40;
 
@@ -38,6 +39,7 @@ cudaError_t launch(const void* func, dim3 g, dim3 b, size_t smem, unsigned clust
 }
 CUresult encode(CUtensorMap* m, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                 CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill) {
+    ++encoded;
     memset(m, 0, sizeof(*m));
     return CUDA_SUCCESS;
 }
@@ -49,10 +51,12 @@ void fake_reset(void) {
     log_text.clear();
     pool_limit = SIZE_MAX;
     occupancy_failures = 0;
+    encoded = 0;
     last = cudaSuccess;
 }
 void fake_pool_limit(size_t bytes) { pool_limit = bytes; }
 void fake_fail_occupancy(int times) { occupancy_failures = times; }
+int fake_encoded(void) { return encoded; }
 const char* fake_launches(void) { return log_text.c_str(); }
 
 // ---- the runtime
