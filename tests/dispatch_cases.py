@@ -7,7 +7,7 @@ tests run the same shapes."""
 # (and among 8 when there are fewer than 8); last tiles of 32 to 96 channels.
 SPLIT_LAYERS = [
     ("bf16", (50, 1024, 14, 9, 32, 1), 2, 64), ("bf16", (64, 768, 7, 7, 160, 1), 2, 128), ("bf16", (40, 768, 14, 9, 32, 1), 3, 64),
-    ("bf16", (5, 768, 7, 7, 1600, 1), 3, 128), ("bf16", (28, 192, 13, 11, 160, 3), 3, 256), ("bf16", (33, 512, 9, 7, 288, 3), 3, 256), ("bf16", (24, 768, 14, 9, 32, 1), 4, 64),
+    ("bf16", (5, 768, 7, 7, 1600, 1), 3, 128), ("bf16", (28, 192, 13, 11, 160, 3), 3, 256), ("bf16", (24, 768, 14, 9, 32, 1), 4, 64),
     ("bf16", (3, 1536, 7, 7, 1600, 1), 4, 128), ("bf16", (20, 256, 13, 11, 160, 3), 4, 256), ("bf16", (24, 128, 8, 16, 32, 3), 5, 64),
     ("bf16", (5, 128, 7, 7, 1024, 3), 5, 128), ("bf16", (2, 768, 7, 7, 32, 1), 6, 64), ("bf16", (18, 128, 13, 11, 96, 3), 6, 128),
     ("bf16", (1, 192, 9, 7, 64, 3), 7, 64), ("bf16", (4, 192, 4, 6, 32, 3), 7, 64), ("bf16", (1, 192, 3, 3, 32, 3), 7, 64),
@@ -21,6 +21,7 @@ SPLIT_LAYERS = [
     ("tf32x3", (5, 512, 7, 7, 1600, 1), 3, 128), ("tf32x3", (3, 512, 7, 7, 1600, 1), 4, 128), ("tf32x3", (24, 768, 14, 9, 32, 1), 5, 64),
     ("tf32x3", (5, 768, 7, 7, 1024, 1), 5, 128), ("tf32x3", (40, 768, 7, 7, 96, 1), 6, 128), ("tf32x3", (1, 512, 1, 1, 32, 1), 8, 64),
     ("tf32x3", (28, 1024, 7, 7, 96, 1), 8, 128),
+    ("bf16", (33, 512, 9, 7, 288, 3), 3, 256),
 ]
 
 
@@ -46,6 +47,15 @@ FP32_TILES = [
     ((1, 3, 5, 6, 16, 7, 7, 1, 3, 1), 7, "16x16"), ((3, 3, 20, 21, 17, 7, 7, 1, 3, 1), 7, "16x32"), ((3, 3, 28, 29, 17, 7, 7, 1, 3, 1), 7, "32x32"),
     ((3, 3, 40, 41, 17, 7, 7, 1, 3, 1), 7, "32x64"), ((3, 3, 40, 41, 33, 7, 7, 1, 3, 1), 7, "32x96"), ((5, 3, 40, 41, 33, 7, 7, 1, 3, 1), 7, "32x128"),
     ((3, 3, 57, 58, 33, 7, 7, 1, 3, 1), 7, "64x96"),
+]
+
+# int8 filters of 81 taps, which it does not take: (images, channels, h, w, output channels, k), whether the result leaves by way of NHWC.
+# Results below and from 1 MiB on, planes that are multiples of 16, of 4 and odd, channels that are multiples of 16, of 4 and odd, boxes of two
+# and fewer columns and wider ones, one pixel per image.
+S8_LARGE_FILTERS = [
+    ((64, 20, 7, 7, 100, 9), False), ((16, 24, 14, 14, 50, 9), False), ((2, 48, 12, 12, 40, 9), False), ((5, 3, 41, 43, 33, 9), False),
+    ((66, 24, 13, 13, 401, 9), True), ((256, 16, 7, 7, 30, 9), True), ((128, 17, 5, 5, 33, 9), True), ((64, 40, 7, 7, 96, 9), True),
+    ((29, 12, 28, 28, 178, 9), True), ((9, 33, 30, 30, 400, 9), True), ((40, 8, 14, 14, 141, 9), True), ((4, 130, 48, 48, 128, 9), True),
 ]
 
 # Convolutions that the channel-major kernel takes: precision, (images, channels, h, w, output channels, kh, kw, stride, pad, dilation),

@@ -408,8 +408,8 @@ def test_conv2d_weights_of_large_filters(ops, rng, N, C, H, W, O, KH, KW, precis
     assert min(max_abs, max_rel) <= bound, f"{precision}: {max_abs:.3e} {max_rel:.3e}"
 
 
-# The byte transposes on both sides of the NCHW form: planes that are multiples of 16, of 4 and odd; channel counts that are not
-# multiples of 16 or 4; one, two and more column tiles; the result by way of NHWC (1 MiB and more) and without.
+# The byte transpose in front of the NCHW form: planes that are multiples of 16, of 4 and odd; channel counts that are not multiples of 16
+# or 4; one, two and more column tiles; results by words (planes whose rows are multiples of four) and by bytes.
 @pytest.mark.parametrize("N,C,H,W,O", [(9, 72, 28, 28, 150), (3, 130, 30, 30, 400), (40, 64, 14, 14, 141), (27, 33, 25, 13, 133), (2, 48, 12, 12, 40),
                                        (345, 128, 14, 14, 128)])
 def test_conv2d_s8_layouts(ops, rng, N, C, H, W, O):
@@ -419,13 +419,24 @@ def test_conv2d_s8_layouts(ops, rng, N, C, H, W, O):
     assert torch.equal(got, ops.nn_conv2d_s8(x, w, b, m, sh, (1, 1), (1, 1), simt=True))
 
 
-# Tile boxes of at most two columns, channels that are no multiple of 16: odd and even planes, below and above 1 MiB of results
+# Small odd and even planes, several images to a tile, channels that are no multiple of 16, below and above 1 MiB of results
 @pytest.mark.parametrize("N,C,H,W,O", [(64, 64, 7, 7, 100), (16, 64, 14, 14, 50), (66, 64, 13, 13, 101), (129, 33, 7, 7, 30), (33, 32, 9, 9, 246)])
 def test_conv2d_s8_narrow_boxes(ops, rng, N, C, H, W, O):
     x, w, b, m, sh = (dev(a) for a in s8_inputs(rng, N, C, H, W, O, 3, 3))
     got = ops.nn_conv2d_s8(x, w, b, m, sh, (1, 1), (1, 1))
     assert ops.device_status() == 0
     assert torch.equal(got, ops.nn_conv2d_s8(x, w, b, m, sh, (1, 1), (1, 1), simt=True))
+
+
+# Filters of more taps than the channel-major kernel lists: results by byte stores, and by way of NHWC and a byte transpose
+@pytest.mark.parametrize("case,by_way_of_nhwc", dispatch_cases.S8_LARGE_FILTERS)
+def test_conv2d_s8_filters_beyond_the_channel_major_kernel(ops, rng, case, by_way_of_nhwc):
+    N, C, H, W, O, k = case
+    x, w, b, m, sh = (dev(a) for a in s8_inputs(rng, N, C, H, W, O, k, k))
+    for relu in (True, False):
+        got = ops.nn_conv2d_s8(x, w, b, m, sh, (1, 1), (k // 2, k // 2), relu=relu)
+        assert ops.device_status() == 0
+        assert torch.equal(got, ops.nn_conv2d_s8(x, w, b, m, sh, (1, 1), (k // 2, k // 2), relu=relu, simt=True))
 
 
 # 1x1 convolutions of stride 2: only the pixels they read are converted. Odd and even extents, one row, one column, channels below, at and
