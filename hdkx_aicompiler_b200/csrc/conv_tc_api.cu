@@ -163,13 +163,6 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     const int stem_wp = ((d.W + 2 * d.PW > 2 * (d.OW - 1) + 8 ? d.W + 2 * d.PW : 2 * (d.OW - 1) + 8) + 3) / 4 * 4;
     const bool stem_ok = !force_simt && tc_shape_ok(d) && d.SH == 2 && d.SW == 2 && d.DH == 1 && d.DW == 1 &&
                          stem_direct_s8_applicable(d.C, d.O, d.KH, d.KW, 2, 1, d.W, d.OW, stem_wp);
-    // 64 -> 64 channels, 3x3, stride 1: the row-stacked kernel (one box load per tile instead of nine)
-    static const bool rowstack_enabled = [] {
-        const char* e = getenv("KXC_B200_ROWSTACK_S8");
-        return !(e != nullptr && e[0] == '0');
-    }();
-    const bool rowstack_ok = rowstack_enabled && !force_simt && tc_shape_ok(d) &&
-                             rowstack3x3_s8_applicable(d.C, d.O, d.KH, d.KW, d.SH == d.SW ? d.SH : 0, d.PH, d.PW, d.DH, d.DW);
     auto run_stem = [&](bool nhwc_layout) -> int32_t {
         const size_t x_bytes = align_up((size_t)d.N * stem_hp * stem_wp * 8, 1024);
         const size_t w_bytes = align_up(stem_direct_weight_bytes(d.KH), 1024);
@@ -195,7 +188,12 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
         if (cpad != d.C || (d.O & 15) != 0 || !aligned16(data) || !aligned16(weight) || !aligned16(out))
             return fail(KXC_B200_ERR_INVALID, "nn_conv2d_s8: NHWC operands need C = 32/64/128k channels, O a multiple of 16 and 16-byte aligned pointers");
         TcParams p{};
-        if (rowstack_ok) {
+        // 64 -> 64 channels, 3x3, stride 1: the row-stacked kernel (one box load per tile instead of nine)
+        static const bool rowstack_enabled = [] {
+            const char* e = getenv("KXC_B200_ROWSTACK_S8");
+            return !(e != nullptr && e[0] == '0');
+        }();
+        if (rowstack_enabled && rowstack3x3_s8_applicable(d.C, d.O, d.KH, d.KW, d.SH, d.PH, d.PW, d.DH, d.DW)) {
             KXC_TRY(rowstack3x3_s8_setup(&p, data, weight, d.N, d.H, d.W));
             p.weights_ready = 1;
             p.bias_i32 = bias;
@@ -220,22 +218,21 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     if (force_simt || !tc_shape_ok(d)) return conv2d_s8_exact(data, weight, bias, multiplier, shift, out, d, relu, s);
     if (stem_ok) return run_stem(false);
     // (a quarter of the conversion and of the kernel's loads for the downsample branches of a ResNet)
-    const bool subsample = subsampled(d) && (cpad & 3) == 0;
-    const int in_h = d.H, in_w = d.W;
-    const int conv_h = subsample ? d.OH : d.H, conv_w = subsample ? d.OW : d.W;  // the tensor the kernel convolves
-    if (const CmPlan* cm = cm_wanted(dt, subsample ? without_stride(d) : d, 0)) {
+    const bool subsample = subsampled(d);
+    const ConvDims dc = subsample ? without_stride(d) : d;  // what the kernel convolves
+    auto convert = [&](uint8_t* act, int pad, const WeightPack* pack) {
+        return subsample ? convert_operands_s8_subsample(data, reinterpret_cast<int8_t*>(act), d.N, d.C, d.H, d.W, d.OH, d.OW, d.SH, pad, pack, s, true)
+                         : convert_operands(data, act, nullptr, dt, d.N, d.C, d.H * d.W, pad, pack, s, true);
+    };
+    if (const CmPlan* cm = cm_wanted(dt, dc, 0)) {
         const int cm_pad = cm_channel_pad(dt, d.C), w_cpad = cm_weight_pad(dt, d.C, *cm);
-        const size_t cm_act = align_up((size_t)d.N * conv_h * conv_w * cm_pad, 1024);
+        const size_t cm_act = align_up((size_t)d.N * dc.H * dc.W * cm_pad, 1024);
         StreamScratch ws(s);
         KXC_TRY(ws.alloc(cm_act + align_up((size_t)d.O * d.KH * d.KW * w_cpad, 1024)));
         uint8_t* act = static_cast<uint8_t*>(ws.ptr);
         uint8_t* wp = act + cm_act;
         const WeightPack pack{weight, wp, nullptr, d.O, d.C, d.KH * d.KW, w_cpad};
-        if (subsample) {
-            KXC_TRY(convert_operands_s8_subsample(data, reinterpret_cast<int8_t*>(act), d.N, d.C, in_h, in_w, d.OH, d.OW, d.SH, cm_pad, &pack, s, true));
-        } else {
-            KXC_TRY(convert_operands(data, act, nullptr, dt, d.N, d.C, d.H * d.W, cm_pad, &pack, s, true));
-        }
+        KXC_TRY(convert(act, cm_pad, &pack));
         CmParams p{};
         KXC_TRY(cm_setup(&p, dt, *cm, act, wp, cm_pad, w_cpad));
         p.bias_i32 = bias;
@@ -245,31 +242,28 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
         p.relu = relu;
         return cm_launch(dt, p, s);
     }
-    // What is left: filters of more taps than the channel-major kernel lists, results of 2^32 elements and more.
-    const size_t act_bytes = align_up((size_t)d.N * conv_h * conv_w * cpad, 1024);
+    // What is left: filters of more taps than the channel-major kernel lists or too far apart for its boxes, results of 2^32 elements and more.
+    const size_t act_bytes = align_up((size_t)d.N * dc.H * dc.W * cpad, 1024);
     const size_t w_bytes = align_up((size_t)d.O * d.KH * d.KW * cpad, 1024);
     // Result layout. A thread of the epilogue owns one pixel, so its NCHW stores are single bytes whose neighbours in
     // memory belong to the next pixel of the same tile row: runs of BW bytes. The other way is to store NHWC into the
     // workspace, pixels padded to 16 channels, and to let a byte transpose write the reference layout, which costs a launch
-    // (1 to 3 us) and the result's bytes twice more. Measured, us with byte stores / by way of NHWC:
-    //   results of 1 MiB and more      96 -> 178 1x1 at 28x28, 229 images: 66 / 51; 128 -> 128 3x3 at 28x28, 256 images: 67 / 67;
-    //                                  smaller ones between 0.9 and 1.3 times; BW <= 2: 128 -> 401 1x1 at 13x13, 66 images: 34 / 23
-    //   ... planes no multiple of four (byte-wise transpose), BW > 2: 33 -> 27 3x3 at 101x103, 132 images: 333 / 386
-    //   below 1 MiB, boxes of one pixel per image: 32 -> 30 3x3 at 7x7, 256 images: 15.1 / 13.0
-    //   ... other boxes, also of BW <= 2: 128 -> 24 3x3 at 14x14, 148 images: 16.0 / 17.6; whole 16s of channels with BW <= 2:
-    //                                  from 13.2 / 15.1 (64 -> 48 at 14x14, 64 images) to 18.5 / 17.2 (256 -> 64 there)
+    // (1 to 3 us) and the result's bytes twice more. Measured on 60 filters of 81 and 121 taps, us a call with byte stores / by way of NHWC:
+    //   narrow boxes (BW <= 2)         24 -> 401 at 13x13, 66 images: 80.3 / 71.5; 17 -> 33 at 5x5, 128 images: 36.3 / 34.3; 20 -> 100 at 7x7, 64
+    //                                  images (two pixels to an image's box, odd channels) 34.5 / 35.1
+    //   results of 1 MiB and more      3 -> 210 at 20x17, 88 images: 110.3 / 97.1, others between 0.95 and 1.03 times; planes no multiple of four
+    //                                  (byte-wise transpose): 3 -> 223 at 39x42, 112 images 303 / 340
+    //   smaller ones                   32.9 / 33.7 to 47.2 / 49.4
     int bw = 0, bh = 0, bni = 0;
     tc_pick_tile(d.N, d.OH, d.OW, &bw, &bh, &bni);
     const int out_pitch = (d.O + 15) / 16 * 16;
     const long long plane = (long long)d.OH * d.OW;
     const bool narrow = bw <= 2;
-    bool two_step = rowstack_ok ||  // (the row-stacked kernel writes NHWC only)
-                    (narrow && ((d.O & 15) == 0 || bw * bh == 1)) ||
-                    (plane * d.N * d.O >= (1 << 20) && ((plane & 3) == 0 || narrow));
+    bool two_step = (narrow && ((d.O & 15) == 0 || bw * bh == 1)) || (plane * d.N * d.O >= (1 << 20) && ((plane & 3) == 0 || narrow));
     const size_t out_bytes = two_step ? align_up((size_t)d.N * d.OH * d.OW * out_pitch, 1024) : 0;
     StreamScratch ws(s);
     int32_t rc = ws.alloc(act_bytes + w_bytes + out_bytes);
-    if (rc != KXC_B200_OK && two_step && !rowstack_ok) {  // no room for the second copy of the result: byte stores
+    if (rc != KXC_B200_OK && two_step) {  // no room for the second copy of the result: byte stores
         two_step = false;
         rc = ws.alloc(act_bytes + w_bytes);
     }
@@ -278,19 +272,11 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     uint8_t* wp = act + act_bytes;
     int8_t* out_nhwc = reinterpret_cast<int8_t*>(wp + w_bytes);
     const WeightPack pack{weight, wp, nullptr, d.O, d.C, d.KH * d.KW, cpad};
-    if (subsample) {
-        KXC_TRY(convert_operands_s8_subsample(data, reinterpret_cast<int8_t*>(act), d.N, d.C, in_h, in_w, d.OH, d.OW, d.SH, cpad, &pack, s, true));
-    } else {
-        KXC_TRY(convert_operands(data, act, nullptr, dt, d.N, d.C, d.H * d.W, cpad, &pack, s, true));
-    }
+    KXC_TRY(convert(act, cpad, &pack));
     TcParams p{};
     TcConfig cfg{};
-    if (rowstack_ok) {
-        KXC_TRY(rowstack3x3_s8_setup(&p, act, wp, d.N, d.H, d.W));
-    } else {
-        KXC_TRY(tc_setup_conv(&p, &cfg, dt, two_step ? kOutNHWC_S8 : kOutNCHW_S8, act, wp, d.N, conv_h, conv_w, cpad, d.O, d.KH, d.KW,
-                              subsample ? 1 : d.SH, d.PH, d.PW, d.DH, d.DW));
-    }
+    KXC_TRY(tc_setup_conv(&p, &cfg, dt, two_step ? kOutNHWC_S8 : kOutNCHW_S8, act, wp, d.N, dc.H, dc.W, cpad, d.O, d.KH, d.KW, dc.SH, d.PH, d.PW, d.DH,
+                          d.DW));
     p.bias_i32 = bias;
     p.multiplier = multiplier;
     p.shift = shift;
@@ -298,11 +284,7 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
     p.out_pitch = two_step ? out_pitch : 0;
     p.relu = relu;
     tc_finish_params(&p);
-    if (rowstack_ok) {
-        KXC_TRY(rowstack3x3_s8_launch(p, s));
-    } else {
-        KXC_TRY(tc_launch(cfg, p, s));
-    }
+    KXC_TRY(tc_launch(cfg, p, s));
     if (two_step) return nhwc_to_nchw_s8(out_nhwc, out, d.N, d.O, out_pitch, d.OH * d.OW, s);
     return KXC_B200_OK;
 }

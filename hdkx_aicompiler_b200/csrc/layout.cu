@@ -503,18 +503,15 @@ int32_t split_rows(const float* in, float* hi, float* lo, int64_t rows, int cols
     return check_launch("split_rows");
 }
 
-int32_t convert_operands_subsample(const void* in, void* out, void* lo, TcDType dtype, int N, int C, int H, int W, int OH, int OW, int stride, int cpad,
+int32_t convert_operands_subsample(const float* in, void* out, void* lo, TcDType dtype, int N, int C, int H, int W, int OH, int OW, int stride, int cpad,
                                    const WeightPack* w, cudaStream_t s, bool overlap) {
     if (N == 0) return KXC_B200_OK;
-    if (dtype == kTcS8)
-        return convert_operands_s8_subsample(static_cast<const int8_t*>(in), static_cast<int8_t*>(out), N, C, H, W, OH, OW, stride, cpad, w, s, overlap);
     if (N > 65535 || (long long)H * W > 0x7fffffffll) return fail(KXC_B200_ERR_UNSUPPORTED, "layout transform: %d images of %dx%d", N, H, W);
     PixelArgs px;
     px.plane = H * W; px.W = W; px.st = stride; px.by_ow = Divisor((unsigned)OW);
-    const float* f = static_cast<const float*>(in);
-    if (dtype == kTcBF16) return launch_convert<__nv_bfloat16, false, true>(f, out, nullptr, N, C, OH * OW, cpad, w, s, overlap, px);
-    return lo != nullptr ? launch_convert<float, true, true>(f, out, lo, N, C, OH * OW, cpad, w, s, overlap, px)
-                         : launch_convert<float, false, true>(f, out, nullptr, N, C, OH * OW, cpad, w, s, overlap, px);
+    if (dtype == kTcBF16) return launch_convert<__nv_bfloat16, false, true>(in, out, nullptr, N, C, OH * OW, cpad, w, s, overlap, px);
+    return lo != nullptr ? launch_convert<float, true, true>(in, out, lo, N, C, OH * OW, cpad, w, s, overlap, px)
+                         : launch_convert<float, false, true>(in, out, nullptr, N, C, OH * OW, cpad, w, s, overlap, px);
 }
 
 int32_t convert_operands_s8_subsample(const int8_t* in, int8_t* out, int N, int C, int H, int W, int OH, int OW, int stride, int cpad,

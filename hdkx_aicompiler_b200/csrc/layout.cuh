@@ -31,8 +31,8 @@ int32_t convert_operands(const void* in, void* out, void* lo, TcDType dtype, int
 int32_t convert_operands_s8_subsample(const int8_t* in, int8_t* out, int N, int C, int H, int W, int OH, int OW, int stride, int cpad,
                                       const WeightPack* weights, cudaStream_t s, bool overlap);
 
-// Either, by type: `lo` as for convert_operands.
-int32_t convert_operands_subsample(const void* in, void* out, void* lo, TcDType dtype, int N, int C, int H, int W, int OH, int OW, int stride, int cpad,
+// bf16 and tf32: `lo` as for convert_operands.
+int32_t convert_operands_subsample(const float* in, void* out, void* lo, TcDType dtype, int N, int C, int H, int W, int OH, int OW, int stride, int cpad,
                                    const WeightPack* weights, cudaStream_t s, bool overlap);
 
 // convert_rows of two matrices with rows of the same length, in one launch where extents and addresses allow it.
