@@ -771,21 +771,27 @@ bool choose(CmPlan* plan, TcDType dtype, const ConvDims& d) {
 // Integers take this form wherever it applies: of 260 drawn layers (device time of a call, against the pixel-major forms of results in planes: byte
 // stores, or NHWC and a transposition) it was the faster one by 1.32 in the geometric mean; seven lost more than 2 %, 1x1 layers to 32 and fewer
 // channels up to 6 % (53 -> 8 of stride 2 at 80x78, 68 images: 19.2 -> 20.4), 180 -> 17 3x3 at 16x16, 51 images 12.6 -> 15.4, 64 -> 64 3x3 at 12x13,
-// 165 images 12.2 -> 14.0. A model of the pixel-major forms, fitted to the same layers, chose worse than not choosing. With fp32 results the pixel-major kernel has less to hand over per K block, splits long reductions of few tiles over
+// 165 images 12.2 -> 14.0. A model of the pixel-major forms, fitted to the same layers, chose worse than not choosing.
+//
+// With fp32 results into planes the pixel-major kernel has less to hand over per K block, splits long reductions of few tiles over
 // clusters and takes 64 channels at a time, so modelled clocks decide. Its model ends with the last K block; 30 clocks per channel of a
-// tile stand for the epilogue of an unsplit one. Over 227 drawn layers (tf32 and bf16, with and without a residual) the choice was 1.6 %
-// behind the faster form and 4 % ahead of the pixel-major kernel alone; one layer lost 12 % by it, 24 -> 30 3x3 at 92x95, 32 images, whose few
-// channels leave three quarters of the epilogue's warps idle in a launch that it bounds: those keep the pixel-major kernel.
+// tile stand for the epilogue of an unsplit one. Over 225 drawn layers (operators with a residual and graph outputs, tf32 and bf16) the choice was
+// 5.6 % ahead of the pixel-major kernel alone; six lost more than 2 %, one-wave 1x1 layers at the line up to 19 % (tf32 32 -> 505 at 21x20, 7 images
+// 6.9 / 8.5, bf16 436 -> 442 at 17x17, 13 images 12.4 / 13.1), 384 -> 61 1x1 at 57x54, 24 images, bf16, 57.7 / 63.5. Few channels (24 -> 30
+// 3x3 at 92x95, 32 images, 12 % slower) leave three quarters of the epilogue's warps idle in a launch that it bounds: those keep the pixel-major kernel.
 // One wave of 1x1 tiles, which share no loads, has to be further ahead: tf32 322 -> 473 at 19x22, 8 images 14.9 pixel-major / 17.1 us, 311 -> 448 of
 // stride 2 at 39x40, 9 images 18.7 / 21.2, bf16 141 -> 129 at 84x84, 2 images 13.6 / 14.8; 110 -> 364 at 14x13, 15 images 11.6 / 11.3 and all of 22 drawn
-// layers of more waves (0.997 to 1.8 times) still take this form.
+// layers of more waves (0.997 to 1.8 times) still take this form. Where the pixel-major kernel's K blocks are narrower than 128 bytes (up to 32 bf16 or
+// 16 tf32 channels) its main loop is not modelled: those layers stay with it unless this whole launch is shorter than that epilogue (2 of 340
+// drawn ones; bf16 22 -> 254 1x1 at 28x29, 20 images, 13.3 / 10.4). Of 160 forced over, 1x1 layers to few channels lost, up to 0.69 times as
+// fast, and wide filters gained, 1.18 times in the mean of all: a model for them has yet to be fitted.
 //
 // NHWC results (layers of plans): each form's modelled clocks, the pixel-major one's with its epilogue, weighted by what launches of plans
 // measured. 3x3 layers, whose pixels the pixel-major kernel loads nine times over, are ahead of their model: tf32 128 -> 128 at 28x28 and
 // 256 -> 256 at 14x14 gained up to the line, 512 -> 512 at 7x7 (two images to a tile, the weights' rows bound both forms) lost where the model said
 // so: 32 images 39.7 / 77.1 us, 256 images 103.5 / 154.0. Split reductions of 1x1 layers lose 8 to 17 % up to a ratio of 1 (64 x 768 -> 160 at 7x7
-// 14.2 / 15.2) and gain from 1.15 on. Splits of wider filters over three and more CTAs keep what the models call level: 40 drawn layers of
-// ratios 0.86 to 1.02 were 0.985 to 1.43 times as fast here, bf16 192 -> 160 3x3 at 13x11, 28 images, 18.9 / 15.2 us, at 0.997. Launches of one channel
+// 14.2 / 15.2) and gain from 1.15 on. Splits of wider filters over three and more CTAs are left only where the models cross; 40 drawn layers
+// of ratios 0.86 to 1.02 were 0.985 to 1.43 times as fast here (bf16 192 -> 160 3x3 at 13x11, 28 images, ratio 0.997: 18.9 / 15.2 us). Launches of one channel
 // block that read and write more than they multiply are the epilogue's, of which 32 channels use a quarter: tf32 1x1 layers up to a ratio
 // of 1.5 (32 -> 32 at 90x88, 45 images 161.8 / 225.8, 32 -> 40 at 76x79, 56 images 160.8 / 174.1; all 23 drawn ones lost) and 3x3 layers of 17 to 32 channels
 // from about 100 tiles on (32 -> 32 at 40x42, 61 images 66.9 / 81.2, 0.82 to 1.10; fewer tiles 1.04 to 1.18), bf16 1x1 layers of 17 to 32 channels and more

@@ -42,7 +42,7 @@
 // and shuffles (6300 clocks of work), the issue of the MMAs (5200), the converters (4700). Before the rows came by bulk copies (they came
 // by each converter's own cp.async, read back one at a time) and the maximum moved in front of bias and rounding a strip took 9400: the epilogue worked for
 // 8100, the converters for 7000. A launch in ResNet-18, us, before / now: bf16 1 image 11.9 / 9.9, 32: 34.2 / 25.1, 128: 74.5 / 61.5; tf32 1: 16.9 / 12.7, 32:
-// 55.3 / 38.1, 128: 154.9 / 111.8; whole networks gain 2 to 4.5 % (1024 images, where the power limit sets the clock, 2 %). Tried: fp32 rows prefetched in registers instead
+// 55.3 / 38.1, 128: 154.9 / 111.8; whole networks gain 2 to 4.5 % (at 1024 images, where the power limit sets the clock, they are level). Tried: fp32 rows prefetched in registers instead
 // (two rows ahead: 10500 clocks a strip, memory latency), packed pixels stored without bank conflicts (no change).
 //
 // bf16 strips have four pooled rows; two where that leaves no SM a second strip (up to five images of 224 x 224), whose time is

@@ -88,7 +88,7 @@ struct TcConfig {
     // 1 (tf32 only): the operands come as tf32 high and low parts and hi*hi, hi*lo and lo*hi are summed in one launch. The
     // low activations lie N images after the high ones (one tensor map covers both), tmB2 describes the low weights.
     int x3 = 0;
-    double clocks = 0.0;  // modelled time of the launch (choose_split), into the reference's layout up to its last K block; int8: not modelled
+    double clocks = 0.0;  // modelled time of the launch (choose_split), into the reference's layout up to its last K block; 0, not modelled: int8, K blocks below 128 bytes
     int mt = 1;    // 2: two pixel tiles per work item share each B tile (two accumulate chains in flight)
 };
 

@@ -77,7 +77,7 @@ struct Vec<FullF32> {
 
 // Three-pass tf32: a value that convolutions read has its tf32 high parts `parts * 2` and its low parts `parts` elements before its
 // full form (0: it has none). Written here they cost no launch and no second reading (a launch of 2 us and, behind the pooling of 32
-// images of 64 x 112 x 112, 10 us; ResNet-18, us, with them / so: one image 197.9 / 193.6, 8: 384.2 / 379.3, 32: 981.3 / 974.5, 64: 1707.7 / 1692.6).
+// images of 64 x 112 x 112, 10 us; ResNet-18, us, with them / so: one image 197.9 / 193.6, 8: 384.2 / 379.3; from 32 on level with the runs' spread).
 template <typename T>
 __device__ __forceinline__ void store_parts(T* p, const float (&f)[Vec<T>::kLanes], int64_t parts) {
     Vec<T>::store(p, f);
