@@ -795,8 +795,10 @@ bool choose(CmPlan* plan, TcDType dtype, const ConvDims& d) {
 // block that read and write more than they multiply are the epilogue's, of which 32 channels use a quarter: tf32 1x1 layers up to a ratio
 // of 1.5 (32 -> 32 at 90x88, 45 images 161.8 / 225.8, 32 -> 40 at 76x79, 56 images 160.8 / 174.1; all 23 drawn ones lost) and 3x3 layers of 17 to 32 channels
 // from about 100 tiles on (32 -> 32 at 40x42, 61 images 66.9 / 81.2, 0.82 to 1.10; fewer tiles 1.04 to 1.18), bf16 1x1 layers of 17 to 32 channels and more
-// than one wave (64 -> 32 at 95x95, 33 images 92.4 / 100.4, 0.92 to 0.95; 16 channels gain 16 to 23 %). Of 626 drawn layers these lines
-// let 178 through, which were 1.13 times as fast (nine lost more than 3 %, the worst bf16 480 -> 416 1x1 at 33x31, 8 images, 34.8 / 39.6).
+// than one wave (64 -> 32 at 95x95, 33 images 92.4 / 100.4, 0.92 to 0.95; 16 channels gain 16 to 23 %). bf16 1x1 layers to
+// more channels gain from a ratio of 1.6 on (1.0 to 1.25 times, with a residual and without; below it 0.92 to 1.02: 384 -> 384 at 17x14, 63 images, 52.0 /
+// 56.4). Of 840 drawn layers these lines let 264 through, which were 1.12 times as fast (seven lost more than 3 %, the worst tf32 64 -> 32 3x3 of stride 2 at
+// 45x48, 39 images, 29.5 / 32.6).
 // ResNet-18 tf32 32 images 476.8 / 419.6 us, 64: 739 / 661, 256: 2156 / 2028; bf16 32: 265.7 / 254.2, 128: 552 / 545. bf16 layers of stride 2
 // keep the pixel-major kernel: with a 1x1 layer beside them they are one launch of it (two outputs), and alone they give the same bits as there.
 const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcOutMode out_mode) {
@@ -843,7 +845,8 @@ const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcO
             const double ahead = d.KH * d.KW == 1 && tiles(e.plan.g, c.BW, c.BH, c.BNI) <= kNumSMs ? 2800.0 : 1000.0;
             e.use = rc == KXC_B200_OK && (d.O > 32 || e.plan.g.cblocks > 1) && c.cost + ahead < cfg.clocks + epilogue;
         } else {
-            const double ahead = d.KH * d.KW == 1 ? (p.split > 1 ? 1.15 : 0.80) : (p.split > 2 ? 1.0 : (d.SH == 1 ? 0.83 : 0.95));
+            const double ahead = d.KH * d.KW == 1 ? (p.split > 1 ? 1.15 : (dtype == kTcBF16 && d.O > 32 ? 1.6 : 0.80))
+                                                  : (p.split > 2 ? 1.0 : (d.SH == 1 ? 0.83 : 0.95));
             const long long items = tiles(e.plan.g, e.plan.c.BW, e.plan.c.BH, e.plan.c.BNI);
             const bool few = d.O > 16 && d.O <= 32;  // channels
             bool stays = dtype == kTcBF16 && d.SH == 2;
