@@ -25,7 +25,7 @@
 // every second (int8: fourth) chunk of 32 columns. Two accumulators of 256 columns. Every wait is bounded.
 //
 // What bounds it: the operands' way out of shared memory (an instruction fetches 128 + N rows of 32 bytes at about 64 bytes a clock) where N
-// is large, the one issuing thread where it is small (~70 clocks an instruction, ~100 for the hand-over of a group of taps; a loop that
+// is large, the issuing warp where it is small (elect_one in sm100.cuh; ~100 clocks for the hand-over of a group of taps; a loop that
 // waited and committed per tap took 300 a tap), in fp32 launches of many tiles the epilogue's 4-byte accesses (~18 clocks per channel and 32
 // pixels with a residual, as in the pixel-major kernel). Device time of a call, pixel-major kernel / this one, us: tf32 72 -> 120 3x3
 // at 45x51, 9 images, with a residual 26.9 / 17.5 (135 tiles of 51x3 pixels in one wave, before 208 tiles of 51x2 in two); int8 128 -> 128 3x3
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // (a uniform value, as the compiler then knows)
     const int lane = threadIdx.x & 31;
     // pixels, weights, staging: an MMA may read up to 15 rows past a pixel slot (N is rounded up) and up to 120 past a weight slot
     // (rows beyond the last channel); both stay inside this allocation, and those columns and rows are not stored
@@ -182,116 +182,121 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
     volatile int* abort_ptr = &abort_flag;
     pdl_launch_dependents();
 
+    auto wait = [&](uint64_t* bar, uint32_t phase) { return __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(bar), phase, abort_ptr)) != 0; };
     const int items = p.tiles_c * p.tiles_w * p.tiles_h * p.tiles_n;
 
     if (warp == 0) {
-        if (lane == 0) {
-            tma_prefetch_desc(&p.tmA[0]);
-            pdl_wait();
-            int slot = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
-                const Item t = item_at(p, item);
-                for (int cb = 0; ok && cb < p.cblocks; ++cb)
-                    for (int l = 0; l < p.loads; ++l) {
-                        if (!mbar_wait_bounded(smem_u32(&bar_px_empty[slot]), phase ^ 1u, abort_ptr)) {
-                            ok = false;
-                            break;
-                        }
-                        const uint32_t full = smem_u32(&bar_px_full[slot]);
-                        mbar_arrive_expect_tx(full, (uint32_t)p.px_bytes);
-                        tma_load_4d(px_smem + (uint32_t)(slot * p.px_slot_bytes), &p.tmA[p.load_map[l]], full, cb * p.kb_elems, t.ow0 + p.load_w[l],
-                                    t.oh0 + p.load_h[l], t.n0);
-                        if (++slot == p.px_slots) { slot = 0; phase ^= 1u; }
+        const bool lead = elect_one();
+        if (lead) tma_prefetch_desc(&p.tmA[0]);
+        pdl_wait();
+        int slot = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int item = (int)blockIdx.x; ok && item < items; item += (int)gridDim.x) {
+            const Item t = item_at(p, item);
+            for (int cb = 0; ok && cb < p.cblocks; ++cb)
+                for (int l = 0; l < p.loads; ++l) {
+                    if (!wait(&bar_px_empty[slot], phase ^ 1u)) {
+                        ok = false;
+                        break;
                     }
-            }
+                    const uint32_t full = smem_u32(&bar_px_full[slot]);
+                    const uint32_t dst = px_smem + (uint32_t)(slot * p.px_slot_bytes);
+                    if (lead) {
+                        mbar_arrive_expect_tx(full, (uint32_t)p.px_bytes);
+                        tma_load_4d(dst, &p.tmA[p.load_map[l]], full, cb * p.kb_elems, t.ow0 + p.load_w[l], t.oh0 + p.load_h[l], t.n0);
+                    }
+                    __syncwarp();
+                    if (++slot == p.px_slots) { slot = 0; phase ^= 1u; }
+                }
         }
     } else if (warp == 2) {
-        if (lane == 0) {
-            tma_prefetch_desc(&p.tmW);
-            if (!p.weights_ready) pdl_wait();
-            int slot = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
-                const int co0 = item_at(p, item).ct * kM;
-                for (int cb = 0; ok && cb < p.cblocks; ++cb)
-                    for (int g = 0; g < p.groups; ++g) {
-                        if (!mbar_wait_bounded(smem_u32(&bar_w_empty[slot]), phase ^ 1u, abort_ptr)) {
-                            ok = false;
-                            break;
-                        }
-                        const uint32_t full = smem_u32(&bar_w_full[slot]);
-                        const int count = p.group[g].count;
+        const bool lead = elect_one();
+        if (lead) tma_prefetch_desc(&p.tmW);
+        if (!p.weights_ready) pdl_wait();
+        int slot = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int item = (int)blockIdx.x; ok && item < items; item += (int)gridDim.x) {
+            const int co0 = item_at(p, item).ct * kM;
+            for (int cb = 0; ok && cb < p.cblocks; ++cb)
+                for (int g = 0; g < p.groups; ++g) {
+                    if (!wait(&bar_w_empty[slot], phase ^ 1u)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t full = smem_u32(&bar_w_full[slot]);
+                    const int count = p.group[g].count;
+                    if (lead) {
                         mbar_arrive_expect_tx(full, (uint32_t)(count * p.w_tap_bytes));
                         for (int j = 0; j < count; ++j)
                             tma_load_3d(w_smem + (uint32_t)(slot * p.w_slot_bytes + j * p.w_tap_bytes), &p.tmW, full, cb * p.kb_elems, co0, p.group[g].tap[j]);
-                        if (++slot == p.w_slots) { slot = 0; phase ^= 1u; }
                     }
-            }
+                    __syncwarp();
+                    if (++slot == p.w_slots) { slot = 0; phase ^= 1u; }
+                }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = make_instr_desc(kKind == MmaKind::F16 ? kFmtBF16 : (kKind == MmaKind::TF32 ? kFmtTF32 : kFmtS8),
-                                                   kKind == MmaKind::I8 ? kAccS32 : kAccF32, (uint32_t)p.n_cols);
-            const uint32_t hi = desc_hi(8 * kRow, kLayoutSw128);
-            const uint32_t px_lo0 = desc_lo(px_smem, 16), w_lo0 = desc_lo(w_smem, 16);
-            const uint32_t tap_step = (uint32_t)p.w_tap_bytes >> 4;
-            const int groups = p.groups, w_slots = p.w_slots, px_slots = p.px_slots;
-            int ps = 0, ws = 0, acc = 0;
-            uint32_t pphase = 0, wphase = 0, acc_phase = 0;
-            uint32_t px_lo = px_lo0, w_lo = w_lo0;
-            bool ok = true;
-            for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
-                if (!mbar_wait_bounded(smem_u32(&bar_acc_empty[acc]), acc_phase ^ 1u, abort_ptr)) break;
-                tc_fence_after_sync();
-                const uint32_t d = tmem_base + (uint32_t)(acc * kAccCols);
-                uint32_t accumulate = 0;
-                for (int cb = 0; ok && cb < p.cblocks; ++cb) {
-                    const int steps = cb + 1 == p.cblocks ? p.last_steps : kRow / 32;
-                    CmParams::Group g = p.group[0];
-                    for (int i = 0; i < groups; ++i) {
-                        const CmParams::Group next = p.group[i + 1];  // (one more than there are: read ahead of its use)
-                        if (g.first && !mbar_wait_bounded(smem_u32(&bar_px_full[ps]), pphase, abort_ptr)) {
-                            ok = false;
-                            break;
-                        }
-                        if (!mbar_wait_bounded(smem_u32(&bar_w_full[ws]), wphase, abort_ptr)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after_sync();
+        const bool lead = elect_one();
+        const uint32_t idesc = make_instr_desc(kKind == MmaKind::F16 ? kFmtBF16 : (kKind == MmaKind::TF32 ? kFmtTF32 : kFmtS8),
+                                               kKind == MmaKind::I8 ? kAccS32 : kAccF32, (uint32_t)p.n_cols);
+        const uint32_t hi = desc_hi(8 * kRow, kLayoutSw128);
+        const uint32_t px_lo0 = desc_lo(px_smem, 16), w_lo0 = desc_lo(w_smem, 16);
+        const uint32_t tap_step = (uint32_t)p.w_tap_bytes >> 4;
+        const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const int groups = p.groups, w_slots = p.w_slots, px_slots = p.px_slots;
+        int ps = 0, ws = 0, acc = 0;
+        uint32_t pphase = 0, wphase = 0, acc_phase = 0;
+        uint32_t px_lo = px_lo0, w_lo = w_lo0;
+        bool ok = true;
+        for (int item = (int)blockIdx.x; ok && item < items; item += (int)gridDim.x) {
+            if (!wait(&bar_acc_empty[acc], acc_phase ^ 1u)) break;
+            tc_fence_after_sync();
+            const uint32_t d = tmem + (uint32_t)(acc * kAccCols);
+            uint32_t accumulate = 0;
+            for (int cb = 0; ok && cb < p.cblocks; ++cb) {
+                const int steps = cb + 1 == p.cblocks ? p.last_steps : kRow / 32;
+                CmParams::Group g = p.group[0];
+                for (int i = 0; i < groups; ++i) {
+                    const CmParams::Group next = p.group[i + 1];  // (one more than there are: read ahead of its use)
+                    if ((g.first && !wait(&bar_px_full[ps], pphase)) || !wait(&bar_w_full[ws], wphase)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                    if (lead) {
 #pragma unroll
                         for (int j = 0; j < CmParams::kMaxGroup; ++j) {
                             if (j >= g.count) break;
                             const uint32_t a = w_lo + (uint32_t)j * tap_step, b = px_lo + g.shift[j];
                             if (steps == kRow / 32) {
 #pragma unroll
-                                for (int k = 0; k < kRow / 32; ++k) mma_step<kKind>(d, a + 2 * k, b + 2 * k, hi, idesc, k == 0 ? accumulate : 1u);
+                                for (int k = 0; k < kRow / 32; ++k) mma_step<kKind>(d, a + 2 * k, b + 2 * k, hi, idesc, k == 0 && j == 0 ? accumulate : 1u);
                             } else {
-                                mma_step<kKind>(d, a, b, hi, idesc, accumulate);
+                                mma_step<kKind>(d, a, b, hi, idesc, j == 0 ? accumulate : 1u);
                                 if (steps > 1) mma_step<kKind>(d, a + 2, b + 2, hi, idesc, 1u);
                                 if (steps > 2) mma_step<kKind>(d, a + 4, b + 4, hi, idesc, 1u);
                             }
-                            accumulate = 1;
                         }
                         umma_commit(smem_u32(&bar_w_empty[ws]));
-                        w_lo += (uint32_t)p.w_slot_bytes >> 4;
-                        if (++ws == w_slots) { ws = 0; wphase ^= 1u; w_lo = w_lo0; }
-                        if (g.last) {
-                            umma_commit(smem_u32(&bar_px_empty[ps]));
-                            px_lo += (uint32_t)p.px_slot_bytes >> 4;
-                            if (++ps == px_slots) { ps = 0; pphase ^= 1u; px_lo = px_lo0; }
-                        }
-                        g = next;
+                        if (g.last) umma_commit(smem_u32(&bar_px_empty[ps]));
                     }
+                    __syncwarp();
+                    accumulate = 1;
+                    w_lo += (uint32_t)p.w_slot_bytes >> 4;
+                    if (++ws == w_slots) { ws = 0; wphase ^= 1u; w_lo = w_lo0; }
+                    if (g.last) {
+                        px_lo += (uint32_t)p.px_slot_bytes >> 4;
+                        if (++ps == px_slots) { ps = 0; pphase ^= 1u; px_lo = px_lo0; }
+                    }
+                    g = next;
                 }
-                if (!ok) break;
-                umma_commit(smem_u32(&bar_acc_full[acc]));
-                acc ^= 1;
-                if (acc == 0) acc_phase ^= 1u;
             }
+            if (!ok) break;
+            if (lead) umma_commit(smem_u32(&bar_acc_full[acc]));
+            __syncwarp();
+            acc ^= 1;
+            if (acc == 0) acc_phase ^= 1u;
         }
     } else {
         constexpr int kEpiParts = kEpiWarps<kKind> / 4;
