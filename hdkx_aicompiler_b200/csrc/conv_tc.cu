@@ -1,9 +1,10 @@
 // Implicit-GEMM convolution / dense on tcgen05 tensor cores with TMEM accumulators and TMA operand
 // loads (see conv_tc.cuh for the GEMM view). Persistent, warp-specialised CTAs, one per SM:
 //
-//   warp 0      TMA producer   one lane issues cp.async.bulk.tensor loads into a ring of swizzled
+//   warp 0      TMA producer   its elected lane issues cp.async.bulk.tensor loads into a ring of swizzled
 //                              shared-memory stages, each guarded by a full/empty mbarrier pair
-//   warp 1      MMA issuer     one lane issues tcgen05.mma (M = 128, N = BN, K = 32 bytes per
+//   warp 1      MMA issuer     its elected lane (elect_one in sm100.cuh: both loops run on the whole warp; int8 256 -> 256 3x3 at 14x14,
+//                              256 images, a loop of one lane 26.4 us, so 23.1) issues tcgen05.mma (M = 128, N = BN, K = 32 bytes per
 //                              instruction) into one of two TMEM accumulators; tcgen05.commit
 //                              releases stages and publishes finished accumulators; owns TMEM alloc
 //   warps 2..9  epilogue       tcgen05.ld the accumulator (two warps per 32-lane quadrant, each half
@@ -99,7 +100,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
     __shared__ int abort_flag;
     [[maybe_unused]] __shared__ int requant_ok;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // (a uniform value, as the compiler then knows)
     const int lane = threadIdx.x & 31;
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t cta_rank = kPair ? cluster_cta_rank() : 0u;
@@ -131,8 +132,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
     __syncthreads();
     if constexpr (kPair) cluster_sync_all();  // the peer's barriers are initialised before anything signals them
     tc_fence_after_sync();
-    const uint32_t tmem_base = tmem_base_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
     volatile int* abort_ptr = &abort_flag;
+    auto wait = [&](uint64_t* bar, uint32_t phase) { return __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(bar), phase, abort_ptr)) != 0; };
     pdl_launch_dependents();  // the next kernel's CTAs may take over SMs this grid has left; they wait before touching memory
 
     const int num_kb_main = p.taps_h * p.taps_w * p.cblocks;
@@ -147,114 +149,121 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
 
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
-        if (lane == 0) {
+        const bool lead = elect_one();
+        if (lead) {
             tma_prefetch_desc(&p.tmB);
             tma_prefetch_desc(&p.tmA[0]);
             if constexpr (kDual || kX3) tma_prefetch_desc(&p.tmB2);
-            const uint32_t tx_bytes = (uint32_t)((kX3 ? 2 : kMT) * rows_used * KB_BYTES + G::kBBytes);
-            pdl_wait();  // the activations come from the previous kernel
-            int stage = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int item = first_tile; ok && item < total_tiles; item += tile_step) {
-                const int tile = p.reverse ? total_tiles - 1 - item : item;
-                const int ct = tile % p.tiles_c;
-                int ow0[kMT], oh0[kMT], n0[kMT];
+        }
+        const uint32_t tx_bytes = (uint32_t)((kX3 ? 2 : kMT) * rows_used * KB_BYTES + G::kBBytes);
+        pdl_wait();  // the activations come from the previous kernel
+        int stage = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int item = first_tile; ok && item < total_tiles; item += tile_step) {
+            const int tile = p.reverse ? total_tiles - 1 - item : item;
+            const int ct = tile % p.tiles_c;
+            int ow0[kMT], oh0[kMT], n0[kMT];
 #pragma unroll
-                for (int t = 0; t < kMT; ++t) {
-                    int r = ((tile / p.tiles_c) * kCtas + (int)cta_rank) * kMT + t;
-                    const int tw = r % p.tiles_w; r /= p.tiles_w;
-                    const int th = r % p.tiles_h;
-                    const int tn = r / p.tiles_h;
-                    ow0[t] = tw * p.BW; oh0[t] = th * p.BH; n0[t] = tn * p.BNI;
-                }
-                const int co0 = ct * BN + (int)cta_rank * (BN / kCtas);
-                int kb = 0;
-                for (int kh = 0; ok && kh < p.taps_h; ++kh) {
-                    for (int kw = 0; ok && kw < p.taps_w; ++kw) {
-                        const int dh = kh * p.dil_h - p.pad_h;
-                        const int dw = kw * p.dil_w - p.pad_w;
-                        int map = 0, ch = dh, cw = dw;  // offsets of this tap's box from the tile's first pixel
-                        if (p.stride == 2) {
-                            const int hp = dh & 1, wp = dw & 1;
-                            map = hp * 2 + wp;
-                            ch = (dh - hp) >> 1;
-                            cw = (dw - wp) >> 1;
-                        }
-                        for (int cb = 0; cb < p.cblocks; ++cb, ++kb) {
-                            if (!mbar_wait_bounded(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_ptr)) {
-                                ok = false;
-                                break;
-                            }
-                            const uint32_t full = smem_u32(&bar_full[stage]);
-                            const uint32_t a_dst = ring + (uint32_t)stage * G::kStageBytes;
-                            if constexpr (kPair) {
-                                if (leader) mbar_arrive_expect_tx(full, 2u * tx_bytes);
-                                const uint32_t full0 = map_to_cta(full, 0);
-#pragma unroll
-                                for (int t = 0; t < kMT; ++t)
-                                    tma_load_4d_pair(a_dst + t * G::kATileBytes, &p.tmA[map], full0, cb * p.kb_elems, ow0[t] + cw,
-                                                     oh0[t] + ch, n0[t]);
-                                tma_load_2d_pair(a_dst + G::kABytes, &p.tmB, full0, kb * p.kb_elems, co0);
-                            } else {
-                                mbar_arrive_expect_tx(full, tx_bytes);
-#pragma unroll
-                                for (int t = 0; t < kMT; ++t)
-                                    tma_load_4d(a_dst + t * G::kATileBytes, &p.tmA[map], full, cb * p.kb_elems, ow0[t] + cw, oh0[t] + ch,
-                                                n0[t]);
-                                tma_load_2d(a_dst + G::kABytes, &p.tmB, full, kb * p.kb_elems, co0);
-                                if constexpr (kX3) {
-                                    tma_load_4d(a_dst + G::kATileBytes, &p.tmA[map], full, cb * p.kb_elems, ow0[0] + cw, oh0[0] + ch,
-                                                n0[0] + p.N);
-                                    tma_load_2d(a_dst + G::kABytes + G::kBTileBytes, &p.tmB2, full, kb * p.kb_elems, co0);
-                                }
-                            }
-                            if (++stage == kStages) { stage = 0; phase ^= 1u; }
-                        }
-                    }
-                }
-                if constexpr (kDual) {
-                    // second output: the centre tap's pixels (the 1x1 convolution's only tap) against tmB2
-                    const int dh = (p.taps_h / 2) * p.dil_h - p.pad_h, dw = (p.taps_w / 2) * p.dil_w - p.pad_w;  // 0, 0
-                    int map = 0, ch = oh0[0] + dh, cw = ow0[0] + dw;
+            for (int t = 0; t < kMT; ++t) {
+                int r = ((tile / p.tiles_c) * kCtas + (int)cta_rank) * kMT + t;
+                const int tw = r % p.tiles_w; r /= p.tiles_w;
+                const int th = r % p.tiles_h;
+                const int tn = r / p.tiles_h;
+                ow0[t] = tw * p.BW; oh0[t] = th * p.BH; n0[t] = tn * p.BNI;
+            }
+            const int co0 = ct * BN + (int)cta_rank * (BN / kCtas);
+            int kb = 0;
+            for (int kh = 0; ok && kh < p.taps_h; ++kh) {
+                for (int kw = 0; ok && kw < p.taps_w; ++kw) {
+                    const int dh = kh * p.dil_h - p.pad_h;
+                    const int dw = kw * p.dil_w - p.pad_w;
+                    int map = 0, ch = dh, cw = dw;  // offsets of this tap's box from the tile's first pixel
                     if (p.stride == 2) {
                         const int hp = dh & 1, wp = dw & 1;
                         map = hp * 2 + wp;
-                        ch = oh0[0] + ((dh - hp) >> 1);
-                        cw = ow0[0] + ((dw - wp) >> 1);
+                        ch = (dh - hp) >> 1;
+                        cw = (dw - wp) >> 1;
                     }
-                    for (int cb = 0; ok && cb < p.cblocks; ++cb) {
-                        if (!mbar_wait_bounded(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_ptr)) {
+                    for (int cb = 0; cb < p.cblocks; ++cb, ++kb) {
+                        if (!wait(&bar_empty[stage], phase ^ 1u)) {
                             ok = false;
                             break;
                         }
                         const uint32_t full = smem_u32(&bar_full[stage]);
                         const uint32_t a_dst = ring + (uint32_t)stage * G::kStageBytes;
+                        if (!lead) {
+                        } else if constexpr (kPair) {
+                            if (leader) mbar_arrive_expect_tx(full, 2u * tx_bytes);
+                            const uint32_t full0 = map_to_cta(full, 0);
+#pragma unroll
+                            for (int t = 0; t < kMT; ++t)
+                                tma_load_4d_pair(a_dst + t * G::kATileBytes, &p.tmA[map], full0, cb * p.kb_elems, ow0[t] + cw,
+                                                 oh0[t] + ch, n0[t]);
+                            tma_load_2d_pair(a_dst + G::kABytes, &p.tmB, full0, kb * p.kb_elems, co0);
+                        } else {
+                            mbar_arrive_expect_tx(full, tx_bytes);
+#pragma unroll
+                            for (int t = 0; t < kMT; ++t)
+                                tma_load_4d(a_dst + t * G::kATileBytes, &p.tmA[map], full, cb * p.kb_elems, ow0[t] + cw, oh0[t] + ch,
+                                            n0[t]);
+                            tma_load_2d(a_dst + G::kABytes, &p.tmB, full, kb * p.kb_elems, co0);
+                            if constexpr (kX3) {
+                                tma_load_4d(a_dst + G::kATileBytes, &p.tmA[map], full, cb * p.kb_elems, ow0[0] + cw, oh0[0] + ch,
+                                            n0[0] + p.N);
+                                tma_load_2d(a_dst + G::kABytes + G::kBTileBytes, &p.tmB2, full, kb * p.kb_elems, co0);
+                            }
+                        }
+                        __syncwarp();
+                        if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                    }
+                }
+            }
+            if constexpr (kDual) {
+                // second output: the centre tap's pixels (the 1x1 convolution's only tap) against tmB2
+                const int dh = (p.taps_h / 2) * p.dil_h - p.pad_h, dw = (p.taps_w / 2) * p.dil_w - p.pad_w;  // 0, 0
+                int map = 0, ch = oh0[0] + dh, cw = ow0[0] + dw;
+                if (p.stride == 2) {
+                    const int hp = dh & 1, wp = dw & 1;
+                    map = hp * 2 + wp;
+                    ch = oh0[0] + ((dh - hp) >> 1);
+                    cw = ow0[0] + ((dw - wp) >> 1);
+                }
+                for (int cb = 0; ok && cb < p.cblocks; ++cb) {
+                    if (!wait(&bar_empty[stage], phase ^ 1u)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t full = smem_u32(&bar_full[stage]);
+                    const uint32_t a_dst = ring + (uint32_t)stage * G::kStageBytes;
+                    if (lead) {
                         mbar_arrive_expect_tx(full, tx_bytes);
                         tma_load_4d(a_dst, &p.tmA[map], full, cb * p.kb_elems, cw, ch, n0[0]);
                         tma_load_2d(a_dst + G::kABytes, &p.tmB2, full, cb * p.kb_elems, co0);
-                        if (++stage == kStages) { stage = 0; phase ^= 1u; }
                     }
+                    __syncwarp();
+                    if (++stage == kStages) { stage = 0; phase ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0 && leader) {
+        if (leader) {
+            const bool lead = elect_one();
             int stage = 0;
             uint32_t phase = 0;
             int acc = 0;
             uint32_t acc_phase = 0;
             bool ok = true;
             for (int tile = first_tile; ok && tile < total_tiles; tile += tile_step) {
-                if (!mbar_wait_bounded(smem_u32(&bar_acc_empty[acc]), acc_phase ^ 1u, abort_ptr)) break;
+                if (!wait(&bar_acc_empty[acc], acc_phase ^ 1u)) break;
                 tc_fence_after_sync();
                 const uint32_t d_main = tmem_base + (uint32_t)(acc * kAccCols);
                 for (int kb = 0; kb < num_kb; ++kb) {
                     const bool second = kDual && kb >= num_kb_main;
                     const uint32_t d_tmem = second ? d_main + (uint32_t)BN : d_main;
                     const int kb_local = second ? kb - num_kb_main : kb;
-                    if (!mbar_wait_bounded(smem_u32(&bar_full[stage]), phase, abort_ptr)) {
+                    if (!wait(&bar_full[stage], phase)) {
                         ok = false;
                         break;
                     }
@@ -262,33 +271,39 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                     const uint32_t a_addr = ring + (uint32_t)stage * G::kStageBytes;
                     const uint64_t a_desc = make_smem_desc(a_addr, KB_BYTES);
                     const uint64_t b_desc = make_smem_desc(a_addr + G::kABytes, KB_BYTES);
+                    if (lead) {
 #pragma unroll
-                    for (int k = 0; k < KB_BYTES / 32; ++k) {
-                        if constexpr (kX3) {
-                            const uint64_t a_k = a_desc + (uint64_t)(2 * k), b_k = b_desc + (uint64_t)(2 * k);
-                            umma<kKind>(d_tmem, a_k, b_k, kIdescWide, (kb_local | k) != 0 ? 1u : 0u);
-                            umma<kKind>(d_tmem + (uint32_t)BN, a_k + (uint64_t)(G::kATileBytes >> 4), b_k, kIdesc, 1u);
-                        } else {
+                        for (int k = 0; k < KB_BYTES / 32; ++k) {
+                            if constexpr (kX3) {
+                                const uint64_t a_k = a_desc + (uint64_t)(2 * k), b_k = b_desc + (uint64_t)(2 * k);
+                                umma<kKind>(d_tmem, a_k, b_k, kIdescWide, (kb_local | k) != 0 ? 1u : 0u);
+                                umma<kKind>(d_tmem + (uint32_t)BN, a_k + (uint64_t)(G::kATileBytes >> 4), b_k, kIdesc, 1u);
+                            } else {
 #pragma unroll
-                        for (int t = 0; t < kMT; ++t) {
-                            // advancing 32 bytes along K inside the swizzle span = +2 in the (addr >> 4) field;
-                            // the next pixel tile of the stage is kATileBytes further on
-                            const uint64_t a_k = a_desc + (uint64_t)(2 * k) + (uint64_t)(t * (G::kATileBytes >> 4));
-                            const uint32_t d_t = d_tmem + (uint32_t)(t * BN);
-                            if constexpr (kPair)
-                                umma_pair<kKind>(d_t, a_k, b_desc + (uint64_t)(2 * k), kIdesc, (kb_local | k) != 0 ? 1u : 0u);
-                            else
-                                umma<kKind>(d_t, a_k, b_desc + (uint64_t)(2 * k), kIdesc, (kb_local | k) != 0 ? 1u : 0u);
+                            for (int t = 0; t < kMT; ++t) {
+                                // advancing 32 bytes along K inside the swizzle span = +2 in the (addr >> 4) field;
+                                // the next pixel tile of the stage is kATileBytes further on
+                                const uint64_t a_k = a_desc + (uint64_t)(2 * k) + (uint64_t)(t * (G::kATileBytes >> 4));
+                                const uint32_t d_t = d_tmem + (uint32_t)(t * BN);
+                                if constexpr (kPair)
+                                    umma_pair<kKind>(d_t, a_k, b_desc + (uint64_t)(2 * k), kIdesc, (kb_local | k) != 0 ? 1u : 0u);
+                                else
+                                    umma<kKind>(d_t, a_k, b_desc + (uint64_t)(2 * k), kIdesc, (kb_local | k) != 0 ? 1u : 0u);
+                            }
+                            }
                         }
-                        }
+                        if constexpr (kPair) umma_commit_pair(smem_u32(&bar_empty[stage]), 3);
+                        else umma_commit(smem_u32(&bar_empty[stage]));
                     }
-                    if constexpr (kPair) umma_commit_pair(smem_u32(&bar_empty[stage]), 3);
-                    else umma_commit(smem_u32(&bar_empty[stage]));
+                    __syncwarp();
                     if (++stage == kStages) { stage = 0; phase ^= 1u; }
                 }
                 if (!ok) break;
-                if constexpr (kPair) umma_commit_pair(smem_u32(&bar_acc_full[acc]), 3);
-                else umma_commit(smem_u32(&bar_acc_full[acc]));
+                if (lead) {
+                    if constexpr (kPair) umma_commit_pair(smem_u32(&bar_acc_full[acc]), 3);
+                    else umma_commit(smem_u32(&bar_acc_full[acc]));
+                }
+                __syncwarp();
                 if (++acc == kBufs) {
                     acc = 0;
                     acc_phase ^= 1u;
