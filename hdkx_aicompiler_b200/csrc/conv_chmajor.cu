@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
     volatile int* abort_ptr = &abort_flag;
     pdl_launch_dependents();
 
-    auto wait = [&](uint64_t* bar, uint32_t phase) { return __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(bar), phase, abort_ptr)) != 0; };
+    auto wait = [&](uint64_t* bar, uint32_t phase) { return mbar_wait_warp(smem_u32(bar), phase, abort_ptr); };
     const int items = p.tiles_c * p.tiles_w * p.tiles_h * p.tiles_n;
 
     if (warp == 0) {

@@ -13,6 +13,9 @@
 // 4: 204.0 / 189.5, 32: 491.6 / 476.7), and 16-byte st.async from the accumulator to the owners (slower than the fetches from two
 // images on, tf32 32: 524).
 //
+// Both issuing loops run on whole warps (elect_one in sm100.cuh): ResNet-18 tf32 one image 147.4 -> 134.8 us, bf16 109.7 -> 102.4; 512 -> 512 3x3
+// at 7x7, tf32, 8 images 14.4 -> 11.8.
+//
 //   warp 0      TMA producer; loads the weights of the first stages before it waits for the previous kernel (weights of a
 //               plan do not come from that kernel), so only the pixels are on the critical path of a layer
 //   warp 1      MMA issuer, TMEM owner
@@ -224,7 +227,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __g
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // (a uniform value, as the compiler then knows)
     const int lane = threadIdx.x & 31;
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const int rank = (int)cluster_cta_rank();
@@ -258,7 +261,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __g
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = tmem_base_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
     volatile int* abort_ptr = &abort_flag;
     // First cluster barrier: every CTA's receive buffer and its mbarrier are ready. Arrived at here, or when the ring is idle.
     if constexpr (G::kOwnBuffer) cluster_arrive();
@@ -277,14 +280,24 @@ __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __g
     const int ow0 = tw * p.BW, oh0 = th * p.BH, n0 = tn * p.BNI;
 
     if (warp == 0) {
-        if (lane == 0) {
-            tma_prefetch_desc(&p.tmB);
-            tma_prefetch_desc(&p.tmA[0]);
-            if constexpr (kDual || kX3) tma_prefetch_desc(&p.tmB2);
+        // The three-pass form of 128 channels keeps a loop of one lane: its stages of 64 KB, asked for any faster, arrive later (512 -> 512 at 7x7,
+        // 32 images 45.5 us, 47.2 with the whole warp; 51.2 with the pixels' loads before the weights').
+        constexpr bool kWhole = !(kX3 && BN == 128);
+        const bool lead = kWhole ? elect_one() : lane == 0;
+        auto converge = [] {
+            if constexpr (kWhole) __syncwarp();
+        };
+        if (kWhole || lead) {
+            if (lead) {
+                tma_prefetch_desc(&p.tmB);
+                tma_prefetch_desc(&p.tmA[0]);
+                if constexpr (kDual || kX3) tma_prefetch_desc(&p.tmB2);
+            }
             const uint32_t tx_bytes = (uint32_t)((kX3 ? 2 : 1) * (rows_used * kKB + G::kBTile));
             auto load_weights = [&](int kb, int stage) {
                 const uint32_t full = smem_u32(&bar_full[stage]);
                 const uint32_t dst = ring + (uint32_t)stage * G::kStageBytes + G::kABytes;
+                if (!lead) return;
                 mbar_arrive_expect_tx(full, tx_bytes);
                 if (kDual && kb >= kb_main) {
                     tma_load_2d(dst, &p.tmB2, full, (kb - kb_main) * p.kb_elems, ct * BN);
@@ -315,38 +328,43 @@ __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __g
                 }
                 const uint32_t full = smem_u32(&bar_full[stage]);
                 const uint32_t dst = ring + (uint32_t)stage * G::kStageBytes;
+                if (!lead) return;
                 tma_load_4d(dst, &p.tmA[map], full, cb * p.kb_elems, ow0 + cw, oh0 + ch, n0);
                 if constexpr (kX3) tma_load_4d(dst + G::kATile, &p.tmA[map], full, cb * p.kb_elems, ow0 + cw, oh0 + ch, n0 + p.N);
             };
             const int early = p.weights_ready ? (kb1 - kb0 < kStages ? kb1 - kb0 : kStages) : 0;
             for (int i = 0; i < early; ++i) load_weights(kb0 + i, i);
+            converge();
             pdl_wait();  // the pixels come from the previous kernel
             for (int i = 0; i < early; ++i) load_pixels(kb0 + i, i);
+            converge();
             int stage = early == kStages ? 0 : early;
             uint32_t phase = early == kStages ? 1u : 0u;
             for (int kb = kb0 + early; kb < kb1; ++kb) {
-                if (!mbar_wait_bounded(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_ptr)) break;
+                if (!(kWhole ? mbar_wait_warp(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_ptr) : mbar_wait_bounded(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_ptr))) break;
                 load_weights(kb, stage);
                 load_pixels(kb, stage);
+                converge();
                 if (++stage == kStages) { stage = 0; phase ^= 1u; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int kb = kb0; kb < kb1; ++kb) {
-                if (!mbar_wait_bounded(smem_u32(&bar_full[stage]), phase, abort_ptr)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after_sync();
-                const bool second = kDual && kb >= kb_main;
-                const bool first_of_sum = kb == kb0 || (kDual && kb == kb_main);
-                const uint32_t d = tmem_base + (second ? (uint32_t)BN : 0u);
-                const uint32_t a_addr = ring + (uint32_t)stage * G::kStageBytes;
-                const uint64_t a_desc = make_smem_desc(a_addr, kKB), b_desc = make_smem_desc(a_addr + G::kABytes, kKB);
+        const bool lead = elect_one();
+        int stage = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int kb = kb0; kb < kb1; ++kb) {
+            if (!mbar_wait_warp(smem_u32(&bar_full[stage]), phase, abort_ptr)) {
+                ok = false;
+                break;
+            }
+            tc_fence_after_sync();
+            const bool second = kDual && kb >= kb_main;
+            const bool first_of_sum = kb == kb0 || (kDual && kb == kb_main);
+            const uint32_t d = tmem_base + (second ? (uint32_t)BN : 0u);
+            const uint32_t a_addr = ring + (uint32_t)stage * G::kStageBytes;
+            const uint64_t a_desc = make_smem_desc(a_addr, kKB), b_desc = make_smem_desc(a_addr + G::kABytes, kKB);
+            if (lead) {
 #pragma unroll
                 for (int k = 0; k < kKB / 32; ++k) {
                     const uint64_t a_k = a_desc + (uint64_t)(2 * k), b_k = b_desc + (uint64_t)(2 * k);
@@ -359,10 +377,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) conv_splitk_kernel(const __g
                     }
                 }
                 umma_commit(smem_u32(&bar_empty[stage]));
-                if (++stage == kStages) { stage = 0; phase ^= 1u; }
             }
-            if (ok) umma_commit(smem_u32(&bar_acc));
+            __syncwarp();
+            if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
+        if (ok && lead) umma_commit(smem_u32(&bar_acc));
     } else {
         // this CTA's partial sums into its ring and on to the owners of their rows: every load has landed and every MMA has read it
         // once bar_acc completes

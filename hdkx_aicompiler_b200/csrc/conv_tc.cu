@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
     tc_fence_after_sync();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
     volatile int* abort_ptr = &abort_flag;
-    auto wait = [&](uint64_t* bar, uint32_t phase) { return __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(bar), phase, abort_ptr)) != 0; };
+    auto wait = [&](uint64_t* bar, uint32_t phase) { return mbar_wait_warp(smem_u32(bar), phase, abort_ptr); };
     pdl_launch_dependents();  // the next kernel's CTAs may take over SMs this grid has left; they wait before touching memory
 
     const int num_kb_main = p.taps_h * p.taps_w * p.cblocks;
