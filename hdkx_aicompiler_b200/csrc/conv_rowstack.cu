@@ -22,7 +22,9 @@
 //   * the 72 KiB of weights stay resident, ordered [kw][r][cout][cin] by nine TMA loads of the ordinary packed tensor.
 //
 // Roles as in conv_tc.cu: warp 0 producer, warp 1 MMA issuer + TMEM owner, warps 2..17 epilogue (two sets); two TMEM
-// accumulators (the epilogue of one tile overlaps the next tile's MMAs); every wait bounded.
+// accumulators (the epilogue of one tile overlaps the next tile's MMAs); every wait bounded. The producer's and the issuer's loops run on whole
+// warps (elect_one in sm100.cuh): a launch of 128 images at 56x56 27.8 -> 26.2 us, 30.5 -> 29.8 with a residual. (The 128-channel form, whose
+// pairs issue 24 instructions for a hand-over, is level in bf16 so and 4 % slower in tf32: it keeps loops of one lane.)
 #include "conv_rowstack.cuh"
 
 #include <climits>
@@ -78,7 +80,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack_kernel(const __g
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // (a uniform value, as the compiler then knows)
     const int lane = threadIdx.x & 31;
     const uint32_t w_smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t halo_smem = w_smem + kWeightBytes;
@@ -110,14 +112,15 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack_kernel(const __g
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = tmem_base_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
     volatile int* abort_ptr = &abort_flag;
     pdl_launch_dependents();
 
     const int total_tiles = p.tiles_w * p.tiles_h * p.tiles_n;
 
     if (warp == 0) {
-        if (lane == 0) {
+        const bool lead = elect_one();
+        if (lead) {
             tma_prefetch_desc(&p.tmA[0]);
             tma_prefetch_desc(&p.tmB);
             if (has_res) tma_prefetch_desc(&p.tmA[1]);
@@ -126,44 +129,51 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack_kernel(const __g
             for (int kw = 0; kw < 3; ++kw)
                 for (int r = 0; r < 3; ++r)
                     tma_load_2d(w_smem + kw * kTapBytes + r * (kO * 128), &p.tmB, smem_u32(&bar_w), (r * 3 + kw) * kC, 0);
-            pdl_wait();  // the weights are constants; the activations come from the previous kernel
-            int stage = 0, rb = 0;
-            uint32_t phase = 0, rphase = 0;
-            for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-                int r = p.reverse ? total_tiles - 1 - tile : tile;
-                const int tw = r % p.tiles_w; r /= p.tiles_w;
-                const int th = r % p.tiles_h;
-                const int tn = r / p.tiles_h;
-                if (!mbar_wait_bounded(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_ptr)) break;
-                const uint32_t full = smem_u32(&bar_full[stage]);
+        }
+        pdl_wait();  // the weights are constants; the activations come from the previous kernel
+        int stage = 0, rb = 0;
+        uint32_t phase = 0, rphase = 0;
+        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
+            int r = p.reverse ? total_tiles - 1 - tile : tile;
+            const int tw = r % p.tiles_w; r /= p.tiles_w;
+            const int th = r % p.tiles_h;
+            const int tn = r / p.tiles_h;
+            if (!mbar_wait_warp(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_ptr)) break;
+            const uint32_t full = smem_u32(&bar_full[stage]);
+            if (lead) {
                 mbar_arrive_expect_tx(full, kHaloBytes);
                 // tensor map dimensions: channel, ROW, column, image
                 tma_load_4d(halo_smem + stage * kHaloBytes, &p.tmA[0], full, 0, th * kOutRows - 1, tw * kTileW - 1, tn);
-                if (++stage == kStages) { stage = 0; phase ^= 1u; }
-                if (has_res) {  // the residual pixels of the same output tile, two to three tiles ahead of their use
-                    if (!mbar_wait_bounded(smem_u32(&bar_res_empty[rb]), rphase ^ 1u, abort_ptr)) break;
-                    const uint32_t rfull = smem_u32(&bar_res_full[rb]);
+            }
+            __syncwarp();
+            if (++stage == kStages) { stage = 0; phase ^= 1u; }
+            if (has_res) {  // the residual pixels of the same output tile, two to three tiles ahead of their use
+                if (!mbar_wait_warp(smem_u32(&bar_res_empty[rb]), rphase ^ 1u, abort_ptr)) break;
+                const uint32_t rfull = smem_u32(&bar_res_full[rb]);
+                if (lead) {
                     mbar_arrive_expect_tx(rfull, kBoxBytes);
                     tma_load_4d(res_smem + rb * kBoxBytes, &p.tmA[1], rfull, 0, th * kOutRows, tw * kTileW, tn);
-                    if (++rb == kResBufs) { rb = 0; rphase ^= 1u; }
                 }
+                __syncwarp();
+                if (++rb == kResBufs) { rb = 0; rphase ^= 1u; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            bool ok = mbar_wait_bounded(smem_u32(&bar_w), 0, abort_ptr);
-            const uint32_t hi = desc_hi(1024, kLayoutSw128);  // both operands: 8-row groups of contiguous 128-byte rows
-            const uint32_t b_lo0 = desc_lo(w_smem, 16);
-            int stage = 0;
-            uint32_t phase = 0;
-            int acc = 0;
-            uint32_t acc_phase = 0;
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-                if (!mbar_wait_bounded(smem_u32(&bar_acc_empty[acc]), acc_phase ^ 1u, abort_ptr)) break;
-                if (!mbar_wait_bounded(smem_u32(&bar_full[stage]), phase, abort_ptr)) break;
-                tc_fence_after_sync();
-                const uint32_t d = tmem_base + (uint32_t)(acc * kAccStride);
-                const uint32_t a_lo0 = desc_lo(halo_smem + stage * kHaloBytes, 16);
+        const bool lead = elect_one();
+        bool ok = mbar_wait_warp(smem_u32(&bar_w), 0, abort_ptr);
+        const uint32_t hi = desc_hi(1024, kLayoutSw128);  // both operands: 8-row groups of contiguous 128-byte rows
+        const uint32_t b_lo0 = desc_lo(w_smem, 16);
+        int stage = 0;
+        uint32_t phase = 0;
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
+            if (!mbar_wait_warp(smem_u32(&bar_acc_empty[acc]), acc_phase ^ 1u, abort_ptr)) break;
+            if (!mbar_wait_warp(smem_u32(&bar_full[stage]), phase, abort_ptr)) break;
+            tc_fence_after_sync();
+            const uint32_t d = tmem_base + (uint32_t)(acc * kAccStride);
+            const uint32_t a_lo0 = desc_lo(halo_smem + stage * kHaloBytes, 16);
+            if (lead) {
 #pragma unroll
                 for (int kw = 0; kw < 3; ++kw) {
 #pragma unroll
@@ -175,10 +185,11 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack_kernel(const __g
                 }
                 umma_commit(smem_u32(&bar_empty[stage]));
                 umma_commit(smem_u32(&bar_acc_full[acc]));
-                if (++stage == kStages) { stage = 0; phase ^= 1u; }
-                acc ^= 1;
-                if (acc == 0) acc_phase ^= 1u;
             }
+            __syncwarp();
+            if (++stage == kStages) { stage = 0; phase ^= 1u; }
+            acc ^= 1;
+            if (acc == 0) acc_phase ^= 1u;
         }
     } else {
         const int quad = warp & 3;
@@ -333,7 +344,7 @@ __global__ void __launch_bounds__(kThreads8, 1) conv3x3_rowstack_s8_kernel(const
     __shared__ __align__(16) int4 q_tab[kO];
     __shared__ int q_fast;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // (a uniform value, as the compiler then knows)
     const int lane = threadIdx.x & 31;
     const uint32_t w_smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t halo_smem = w_smem + kWeightBytes8;
@@ -365,51 +376,58 @@ __global__ void __launch_bounds__(kThreads8, 1) conv3x3_rowstack_s8_kernel(const
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = tmem_base_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
     volatile int* abort_ptr = &abort_flag;
     pdl_launch_dependents();
 
     const int total_tiles = p.tiles_w * p.tiles_h * p.tiles_n;
 
     if (warp == 0) {
-        if (lane == 0) {
+        const bool lead = elect_one();
+        if (lead) {
             tma_prefetch_desc(&p.tmA[0]);
             tma_prefetch_desc(&p.tmB);
-            if (!p.weights_ready) pdl_wait();  // weights that the previous kernel packs
+        }
+        if (!p.weights_ready) pdl_wait();  // weights that the previous kernel packs
+        if (lead) {
             mbar_arrive_expect_tx(smem_u32(&bar_w), kWeightBytes8);
             for (int kw = 0; kw < 3; ++kw)
                 for (int r = 0; r < 3; ++r)
                     tma_load_2d(w_smem + kw * kTapBytes8 + r * (kO * kPx8), &p.tmB, smem_u32(&bar_w), (r * 3 + kw) * kC, 0);
-            pdl_wait();
-            int stage = 0;
-            uint32_t phase = 0;
-            for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-                int r = tile;
-                const int tw = r % p.tiles_w; r /= p.tiles_w;
-                const int th = r % p.tiles_h;
-                const int tn = r / p.tiles_h;
-                if (!mbar_wait_bounded(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_ptr)) break;
-                const uint32_t full = smem_u32(&bar_full[stage]);
+        }
+        pdl_wait();
+        int stage = 0;
+        uint32_t phase = 0;
+        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
+            int r = tile;
+            const int tw = r % p.tiles_w; r /= p.tiles_w;
+            const int th = r % p.tiles_h;
+            const int tn = r / p.tiles_h;
+            if (!mbar_wait_warp(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_ptr)) break;
+            const uint32_t full = smem_u32(&bar_full[stage]);
+            if (lead) {
                 mbar_arrive_expect_tx(full, kHaloBytes8);
                 tma_load_4d(halo_smem + stage * kHaloBytes8, &p.tmA[0], full, 0, th * kOutRows - 1, tw * kTileW - 1, tn);
-                if (++stage == kStages8) { stage = 0; phase ^= 1u; }
             }
+            __syncwarp();
+            if (++stage == kStages8) { stage = 0; phase ^= 1u; }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            bool ok = mbar_wait_bounded(smem_u32(&bar_w), 0, abort_ptr);
-            const uint32_t hi = desc_hi(8 * kPx8, kLayoutSw64);  // both operands: 8-row groups of contiguous 64-byte rows
-            const uint32_t b_lo0 = desc_lo(w_smem, 16);
-            int stage = 0;
-            uint32_t phase = 0;
-            int acc = 0;
-            uint32_t acc_phase = 0;
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-                if (!mbar_wait_bounded(smem_u32(&bar_acc_empty[acc]), acc_phase ^ 1u, abort_ptr)) break;
-                if (!mbar_wait_bounded(smem_u32(&bar_full[stage]), phase, abort_ptr)) break;
-                tc_fence_after_sync();
-                const uint32_t d = tmem_base + (uint32_t)(acc * kAccStride);
-                const uint32_t a_lo0 = desc_lo(halo_smem + stage * kHaloBytes8, 16);
+        const bool lead = elect_one();
+        bool ok = mbar_wait_warp(smem_u32(&bar_w), 0, abort_ptr);
+        const uint32_t hi = desc_hi(8 * kPx8, kLayoutSw64);  // both operands: 8-row groups of contiguous 64-byte rows
+        const uint32_t b_lo0 = desc_lo(w_smem, 16);
+        int stage = 0;
+        uint32_t phase = 0;
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
+            if (!mbar_wait_warp(smem_u32(&bar_acc_empty[acc]), acc_phase ^ 1u, abort_ptr)) break;
+            if (!mbar_wait_warp(smem_u32(&bar_full[stage]), phase, abort_ptr)) break;
+            tc_fence_after_sync();
+            const uint32_t d = tmem_base + (uint32_t)(acc * kAccStride);
+            const uint32_t a_lo0 = desc_lo(halo_smem + stage * kHaloBytes8, 16);
+            if (lead) {
 #pragma unroll
                 for (int kw = 0; kw < 3; ++kw) {
 #pragma unroll
@@ -421,10 +439,11 @@ __global__ void __launch_bounds__(kThreads8, 1) conv3x3_rowstack_s8_kernel(const
                 }
                 umma_commit(smem_u32(&bar_empty[stage]));
                 umma_commit(smem_u32(&bar_acc_full[acc]));
-                if (++stage == kStages8) { stage = 0; phase ^= 1u; }
-                acc ^= 1;
-                if (acc == 0) acc_phase ^= 1u;
             }
+            __syncwarp();
+            if (++stage == kStages8) { stage = 0; phase ^= 1u; }
+            acc ^= 1;
+            if (acc == 0) acc_phase ^= 1u;
         }
     } else {
         const int quad = warp & 3;
