@@ -546,4 +546,69 @@ __device__ __forceinline__ void epilogue_coalesced_bf16(const EpiParams& p, cons
     }
 }
 
+// fp32 results in NHWC: the same by way of a tile of 32 rows x 128 bytes. A thread's own 128 bytes, 16 at a time, were 32 lines to a warp's access
+// and half a sector of each: 128 pixels of 256 channels took 19000 clocks, 25000 with a residual, 98 KB of a three-pass tile as long as its
+// main loop. Here eight neighbouring threads cover a pixel's 128 bytes. Thread `lane` handles, in step j (0..7), piece (lane & 7) of row
+// 4 j + (lane >> 3).
+constexpr size_t kNoPixel = ~(size_t)0;
+// those rows' first elements, from the threads that own them
+__device__ __forceinline__ void make_row_map_f32(size_t pix, bool valid, int cout, int lane, size_t (&at)[8]) {
+    const size_t own = valid ? pix * (size_t)cout : kNoPixel;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) at[j] = (size_t)__shfl_sync(0xffffffffu, (unsigned long long)own, 4 * j + (lane >> 3));
+}
+__device__ __forceinline__ void residual_fetch_rows_f32(const TcParams& p, const size_t (&at)[8], int c0, int lane, uint4 (&res)[8]) {
+    const int c = c0 + (lane & 7) * 4;
+    const float* base = static_cast<const float*>(p.residual) + c;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) res[j] = at[j] != kNoPixel && c < p.Cout ? __ldg(reinterpret_cast<const uint4*>(base + at[j])) : make_uint4(0, 0, 0, 0);
+}
+// Whole warp, converged; Cout a multiple of four, all pointers 16-byte aligned. kSplit: as in epilogue_chunk.
+template <bool kSplit>
+__device__ __forceinline__ void epilogue_coalesced_f32(const TcParams& p, const uint32_t (&v)[32], int c0, uint32_t tile, int lane, const size_t (&at)[8],
+                                                       const uint4 (&res)[8], bool has_res) {
+#pragma unroll
+    for (int g = 0; g < 8; ++g)
+        st_shared_v4(tile + (uint32_t)(lane * 128 + ((g ^ (lane & 7)) << 4)), make_uint4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]));
+    __syncwarp();
+    const int piece = lane & 7, c = c0 + 4 * piece;
+    const bool has_bias = p.bias != nullptr, mine = c < p.Cout;
+    const float4 b = has_bias && mine ? __ldg(reinterpret_cast<const float4*>(p.bias + c)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int row = 4 * j + (lane >> 3);
+        const uint4 q = ld_shared_v4(tile + (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)));
+        float f[4] = {__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w)};
+        if (has_bias) {
+            f[0] = __fadd_rn(f[0], b.x); f[1] = __fadd_rn(f[1], b.y); f[2] = __fadd_rn(f[2], b.z); f[3] = __fadd_rn(f[3], b.w);
+        }
+        if (has_res) {
+            f[0] = __fadd_rn(f[0], __uint_as_float(res[j].x)); f[1] = __fadd_rn(f[1], __uint_as_float(res[j].y));
+            f[2] = __fadd_rn(f[2], __uint_as_float(res[j].z)); f[3] = __fadd_rn(f[3], __uint_as_float(res[j].w));
+        }
+        if (p.relu) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) f[k] = f[k] > 0.0f ? f[k] : 0.0f;
+        }
+        if (p.round_out_tf32) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) f[k] = tf32_rne(f[k]);
+        }
+        if (at[j] == kNoPixel || !mine) continue;
+        if constexpr (kSplit) {
+            if (p.out_hi != nullptr) {
+                float h[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) h[k] = tf32_rne(f[k]);
+                float* hi = p.out_hi + at[j] + c;
+                *reinterpret_cast<float4*>(hi) = make_float4(h[0], h[1], h[2], h[3]);
+                *reinterpret_cast<float4*>(hi + p.out_lo_offset) = make_float4(tf32_low_part(f[0], h[0]), tf32_low_part(f[1], h[1]), tf32_low_part(f[2], h[2]), tf32_low_part(f[3], h[3]));
+            }
+            if (p.out == nullptr) continue;
+        }
+        *reinterpret_cast<float4*>(static_cast<float*>(p.out) + at[j] + c) = make_float4(f[0], f[1], f[2], f[3]);
+    }
+    __syncwarp();  // the tile may be overwritten (next chunk)
+}
+
 }  // namespace kxc_b200

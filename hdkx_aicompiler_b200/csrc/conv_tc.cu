@@ -44,8 +44,8 @@ struct StageGeom {
     static constexpr int kStageBytes = kABytes + kBBytes;
     // per epilogue warp a 4 KiB box (32 pixels x 64 channels, SWIZZLE_128B) that TMA stores read; its first half
     // doubles as the staging tile of the per-thread store path
-    // (or, into the reference's layout, holds the bias; the three-pass kernels have no other use for it)
-    static constexpr int kEpilogueBytes = kX3 ? (kNchw ? kStoreBoxBytes : 0) : 8 * kStoreBoxBytes;
+    // (fp32 NHWC: all of it; into the reference's layout it holds the bias, the three-pass kernels' only use for it there)
+    static constexpr int kEpilogueBytes = kX3 && kNchw ? kStoreBoxBytes : 8 * kStoreBoxBytes;
     static constexpr int kStagesRaw = (kSmemLimit - 2048 - kEpilogueBytes) / kStageBytes;
     static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
     static constexpr int kSmemBytes = kStages * kStageBytes + kEpilogueBytes + 1024;  // + slack to align the ring to 1024 B
@@ -322,6 +322,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
         const int h_l = rem / p.BW;
         const int w_l = rem - h_l * p.BW;
         const bool fast = (kOutMode == kOutNHWC_BF16) && p.vec_ok && ((p.Cout & 31) == 0);
+        const bool wide = kOutMode == kOutNHWC_F32 && p.vec_ok && (p.Cout & 3) == 0;  // fp32 NHWC in 16-byte pieces
         const bool has_res = p.residual != nullptr;
         const EpiParams ep = {p.bias, p.residual, p.out, p.Cout, p.relu};
         const uint32_t stage_tile = ring + (uint32_t)(kStages * G::kStageBytes) + (uint32_t)((warp - 2) * kStoreBoxBytes);
@@ -387,6 +388,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                     __syncwarp();  // (lanes beyond the image's edge skipped the loads; the reads of tensor memory want the whole warp)
                 }
             }
+            [[maybe_unused]] size_t at32[8];  // kOutNHWC_F32 only
+            [[maybe_unused]] uint4 res32[8] = {}, next32[8] = {};
+            if constexpr (kOutMode == kOutNHWC_F32) {
+                if (wide) {
+                    make_row_map_f32(pix, valid, p.Cout, lane, at32);
+                    if (has_res && c_base < p.Cout) residual_fetch_rows_f32(p, at32, c_base, lane, res32);
+                }
+            }
             RowMap rows;
             if (fast && !boxed) {
                 rows = make_row_map(pix, valid, lane);
@@ -439,6 +448,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                 uint4 res_next[4] = {};
                 if (fast && has_res && (i + 1 < kChunksPerWarp) && (c0 + 32 < p.Cout))
                     residual_fetch_rows(ep, rows, c0 + 32, lane, res_next);
+                if constexpr (kOutMode == kOutNHWC_F32) {
+                    if (wide && has_res && i + 1 < kChunksPerWarp && c0 + 32 < p.Cout) residual_fetch_rows_f32(p, at32, c0 + 32, lane, next32);
+                }
                 if constexpr (kOutMode == kOutNCHW_F32) {
                     if (has_res && i + 1 < kChunksPerWarp && c0 + 32 < p.Cout) residual_fetch_nchw(p, c0 + 32, valid, n, oh, ow, nchw_next);
                 }
@@ -468,6 +480,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                     }
                 } else if (fast) {
                     if (c0 < p.Cout) epilogue_coalesced_bf16<32>(ep, v, c0, stage_tile, lane, rows, res_cur, has_res);
+                } else if (wide) {
+                    if constexpr (kOutMode == kOutNHWC_F32) {
+                        if (c0 < p.Cout) epilogue_coalesced_f32<kX3>(p, v, c0, stage_tile, lane, at32, res32, has_res);
+                    }
                 } else if (kKind == MmaKind::I8 && q_tab != nullptr) {
                     if constexpr (kKind == MmaKind::I8) {
                         if (valid && c0 < p.Cout) {
@@ -487,6 +503,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                 }
 #pragma unroll
                 for (int g = 0; g < 4; ++g) res_cur[g] = res_next[g];
+                if constexpr (kOutMode == kOutNHWC_F32) {
+#pragma unroll
+                    for (int g = 0; g < 8; ++g) res32[g] = next32[g];
+                }
                 if constexpr (kOutMode == kOutNCHW_F32) {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) nchw_cur[j] = nchw_next[j];
