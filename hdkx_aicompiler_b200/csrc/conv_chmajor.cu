@@ -20,6 +20,11 @@
 // Channels beyond the last whole 32 bytes of a pixel are not multiplied: the last channel block of a tap issues only the
 // instructions that have channels (72 tf32 channels: 9 of 12).
 //
+// CTA pairs (tcgen05 cta_group::2; NHWC results of more than 128 channels): 256 channels and two boxes of pixels to a tile. Each CTA holds its 128
+// channels' weights and one box, an instruction reads both boxes, and each CTA's tensor memory takes its channels of both. Weights, most of what a
+// tile loads, then serve twice the pixels that a CTA's shared memory and ring hold. The leader issues, all loads count on its barriers,
+// commits arrive on both CTAs', and the second CTA's epilogue releases accumulators on the leader's (as in conv_tc.cu).
+//
 // Roles: warp 0 loads pixels, warp 1 issues MMAs and owns TMEM, warp 2 loads weights (a ring of its own, ahead of the previous kernel's
 // end where the weights are old), the others are the epilogue: warp (quad, part) takes TMEM lanes = channels [32 quad, 32 quad + 32) and
 // every second (int8: fourth) chunk of 32 columns. Two accumulators of 256 columns. Every wait is bounded.
@@ -68,6 +73,12 @@ constexpr int kSmemLimit = 227 * 1024 - 1024;                  // (static shared
 template <MmaKind kKind>
 constexpr int kStagingBytes = kEpiWarps<kKind> * (kKind == MmaKind::I8 ? kS8Tile : kF32Tile);
 
+// (pair form, as tma_load_4d_pair)
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* m, uint32_t cluster_bar, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
+                 "l"(reinterpret_cast<uint64_t>(m)), "r"(cluster_bar), "r"(c0), "r"(c1), "r"(c2)
+                 : "memory");
+}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
                  "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
@@ -114,21 +125,25 @@ __device__ __noinline__ uint32_t requantize_any(uint32_t acc, int32_t bias, int3
     return (uint32_t)(uint8_t)requantize_s8((int32_t)(acc + (uint32_t)bias), mult, shift, relu);
 }
 
-struct Item {
-    int ct, ow0, oh0, n0;
+// First result of a tile's box of pixels; a box beyond the last one (the second of a pair's last tile) lies beyond the last image.
+struct Corner {
+    int ow0, oh0, n0;
 };
-__device__ __forceinline__ Item item_at(const CmParams& p, int item) {
-    Item t;
-    const int r = (int)p.by_c.quotient((unsigned)item), row = (int)p.by_w.quotient((unsigned)r), n = (int)p.by_h.quotient((unsigned)row);
-    t.ct = item - r * p.tiles_c;
-    t.ow0 = (r - row * p.tiles_w) * p.BW; t.oh0 = (row - n * p.tiles_h) * p.BH; t.n0 = n * p.BNI;
-    return t;
+__device__ __forceinline__ Corner corner_of(const CmParams& p, int box) {
+    const int row = (int)p.by_w.quotient((unsigned)box), n = (int)p.by_h.quotient((unsigned)row);
+    return {(box - row * p.tiles_w) * p.BW, (row - n * p.tiles_h) * p.BH, n * p.BNI};
 }
 
 // One instruction of M = 128; the upper words of both descriptors are the same constant.
-template <MmaKind kKind>
+template <MmaKind kKind, bool kPair>
 __device__ __forceinline__ void mma_step(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
-    umma<kKind>(d, (uint64_t)hi << 32 | a_lo, (uint64_t)hi << 32 | b_lo, idesc, accumulate);
+    if constexpr (kPair) umma_pair<kKind>(d, (uint64_t)hi << 32 | a_lo, (uint64_t)hi << 32 | b_lo, idesc, accumulate);
+    else umma<kKind>(d, (uint64_t)hi << 32 | a_lo, (uint64_t)hi << 32 | b_lo, idesc, accumulate);
+}
+template <bool kPair>
+__device__ __forceinline__ void commit(uint32_t bar) {
+    if constexpr (kPair) umma_commit_pair(bar, 3);
+    else umma_commit(bar);
 }
 
 // How results leave. Planes: the reference's layout, element by element, neighbouring lanes side by side. PlanesVec: rows, planes and
@@ -136,9 +151,10 @@ __device__ __forceinline__ void mma_step(uint32_t d, uint32_t a_lo, uint32_t b_l
 // fp32, words for int8. Pixels (bf16 and tf32 plans): NHWC, bf16 or fp32; the staging tile turns 32 channels x 32 pixels, and lanes take 16
 // bytes of a pixel each.
 enum class CmForm { Planes, PlanesVec, Pixels };
-template <MmaKind kKind, CmForm kForm>
+template <MmaKind kKind, CmForm kForm, bool kPair>
 __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const __grid_constant__ CmParams p) {
     constexpr bool kVec = kForm == CmForm::PlanesVec;
+    constexpr int kCtas = kPair ? 2 : 1;
     static_assert(kForm != CmForm::Pixels || kKind != MmaKind::I8, "int8 results leave in planes");
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bar_px_full[kMaxSlots], bar_px_empty[kMaxSlots];
@@ -149,6 +165,7 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // (a uniform value, as the compiler then knows)
     const int lane = threadIdx.x & 31;
+    const int rank = kPair ? (int)cluster_cta_rank() : 0;
     // pixels, weights, staging: an MMA may read up to 15 rows past a pixel slot (N is rounded up) and up to 120 past a weight slot
     // (rows beyond the last channel); both stay inside this allocation, and those columns and rows are not stored
     const uint32_t px_smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -167,23 +184,37 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(smem_u32(&bar_acc_full[a]), 1);
-            mbar_init(smem_u32(&bar_acc_empty[a]), kEpiWarps<kKind>);
+            mbar_init(smem_u32(&bar_acc_empty[a]), kCtas * kEpiWarps<kKind>);
         }
         mbar_fence_init();
     }
     if (warp == 1) {
-        tmem_alloc(smem_u32(&tmem_base_slot), 2 * kAccCols);
-        tmem_relinquish();
+        if constexpr (kPair) {
+            tmem_alloc_pair(smem_u32(&tmem_base_slot), 2 * kAccCols);
+            tmem_relinquish_pair();
+        } else {
+            tmem_alloc(smem_u32(&tmem_base_slot), 2 * kAccCols);
+            tmem_relinquish();
+        }
+    }
+    if (p.zero_bytes > 0) {  // the halo behind a box, which no load writes
+        uint8_t* boxes = smem_raw + (px_smem - smem_u32(smem_raw)) + p.px_bytes;
+        for (int s = 0; s < p.px_slots; ++s)
+            for (int i = (int)threadIdx.x * 16; i < p.zero_bytes; i += kThreads<kKind> * 16)
+                *reinterpret_cast<uint4*>(boxes + (size_t)s * p.px_slot_bytes + i) = make_uint4(0, 0, 0, 0);
+        fence_proxy_async_shared();
     }
     tc_fence_before_sync();
     __syncthreads();
+    if constexpr (kPair) cluster_sync_all();  // the other CTA's barriers are initialised before anything signals them
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
     volatile int* abort_ptr = &abort_flag;
     pdl_launch_dependents();
 
     auto wait = [&](uint64_t* bar, uint32_t phase) { return mbar_wait_warp(smem_u32(bar), phase, abort_ptr); };
-    const int items = p.tiles_c * p.tiles_w * p.tiles_h * p.tiles_n;
+    const int items = p.tiles_c * ((p.tiles_w * p.tiles_h * p.tiles_n + kCtas - 1) / kCtas);
+    const int first = kPair ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, step = kPair ? (int)(gridDim.x >> 1) : (int)gridDim.x;
 
     if (warp == 0) {
         const bool lead = elect_one();
@@ -192,8 +223,8 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
         int slot = 0;
         uint32_t phase = 0;
         bool ok = true;
-        for (int item = (int)blockIdx.x; ok && item < items; item += (int)gridDim.x) {
-            const Item t = item_at(p, item);
+        for (int item = first; ok && item < items; item += step) {
+            const Corner t = corner_of(p, (int)p.by_c.quotient((unsigned)item) * kCtas + rank);
             for (int cb = 0; ok && cb < p.cblocks; ++cb)
                 for (int l = 0; l < p.loads; ++l) {
                     if (!wait(&bar_px_empty[slot], phase ^ 1u)) {
@@ -203,8 +234,13 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
                     const uint32_t full = smem_u32(&bar_px_full[slot]);
                     const uint32_t dst = px_smem + (uint32_t)(slot * p.px_slot_bytes);
                     if (lead) {
-                        mbar_arrive_expect_tx(full, (uint32_t)p.px_bytes);
-                        tma_load_4d(dst, &p.tmA[p.load_map[l]], full, cb * p.kb_elems, t.ow0 + p.load_w[l], t.oh0 + p.load_h[l], t.n0);
+                        if constexpr (kPair) {  // (both CTAs' bytes count on the leader's barrier)
+                            if (rank == 0) mbar_arrive_expect_tx(full, 2u * (uint32_t)p.px_bytes);
+                            tma_load_4d_pair(dst, &p.tmA[p.load_map[l]], map_to_cta(full, 0), cb * p.kb_elems, t.ow0 + p.load_w[l], t.oh0 + p.load_h[l], t.n0);
+                        } else {
+                            mbar_arrive_expect_tx(full, (uint32_t)p.px_bytes);
+                            tma_load_4d(dst, &p.tmA[p.load_map[l]], full, cb * p.kb_elems, t.ow0 + p.load_w[l], t.oh0 + p.load_h[l], t.n0);
+                        }
                     }
                     __syncwarp();
                     if (++slot == p.px_slots) { slot = 0; phase ^= 1u; }
@@ -217,8 +253,8 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
         int slot = 0;
         uint32_t phase = 0;
         bool ok = true;
-        for (int item = (int)blockIdx.x; ok && item < items; item += (int)gridDim.x) {
-            const int co0 = item_at(p, item).ct * kM;
+        for (int item = first; ok && item < items; item += step) {
+            const int co0 = ((item - (int)p.by_c.quotient((unsigned)item) * p.tiles_c) * kCtas + rank) * kM;
             for (int cb = 0; ok && cb < p.cblocks; ++cb)
                 for (int g = 0; g < p.groups; ++g) {
                     if (!wait(&bar_w_empty[slot], phase ^ 1u)) {
@@ -228,75 +264,80 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
                     const uint32_t full = smem_u32(&bar_w_full[slot]);
                     const int count = p.group[g].count;
                     if (lead) {
-                        mbar_arrive_expect_tx(full, (uint32_t)(count * p.w_tap_bytes));
-                        for (int j = 0; j < count; ++j)
-                            tma_load_3d(w_smem + (uint32_t)(slot * p.w_slot_bytes + j * p.w_tap_bytes), &p.tmW, full, cb * p.kb_elems, co0, p.group[g].tap[j]);
+                        if (rank == 0) mbar_arrive_expect_tx(full, (uint32_t)(kCtas * count * p.w_tap_bytes));
+                        for (int j = 0; j < count; ++j) {
+                            const uint32_t dst = w_smem + (uint32_t)(slot * p.w_slot_bytes + j * p.w_tap_bytes);
+                            if constexpr (kPair) tma_load_3d_pair(dst, &p.tmW, map_to_cta(full, 0), cb * p.kb_elems, co0, p.group[g].tap[j]);
+                            else tma_load_3d(dst, &p.tmW, full, cb * p.kb_elems, co0, p.group[g].tap[j]);
+                        }
                     }
                     __syncwarp();
                     if (++slot == p.w_slots) { slot = 0; phase ^= 1u; }
                 }
         }
     } else if (warp == 1) {
-        const bool lead = elect_one();
-        const uint32_t idesc = make_instr_desc(kKind == MmaKind::F16 ? kFmtBF16 : (kKind == MmaKind::TF32 ? kFmtTF32 : kFmtS8),
-                                               kKind == MmaKind::I8 ? kAccS32 : kAccF32, (uint32_t)p.n_cols);
-        const uint32_t hi = desc_hi(8 * kRow, kLayoutSw128);
-        const uint32_t px_lo0 = desc_lo(px_smem, 16), w_lo0 = desc_lo(w_smem, 16);
-        const uint32_t tap_step = (uint32_t)p.w_tap_bytes >> 4;
-        const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
-        const int groups = p.groups, w_slots = p.w_slots, px_slots = p.px_slots;
-        int ps = 0, ws = 0, acc = 0;
-        uint32_t pphase = 0, wphase = 0, acc_phase = 0;
-        uint32_t px_lo = px_lo0, w_lo = w_lo0;
-        bool ok = true;
-        for (int item = (int)blockIdx.x; ok && item < items; item += (int)gridDim.x) {
-            if (!wait(&bar_acc_empty[acc], acc_phase ^ 1u)) break;
-            tc_fence_after_sync();
-            const uint32_t d = tmem + (uint32_t)(acc * kAccCols);
-            uint32_t accumulate = 0;
-            for (int cb = 0; ok && cb < p.cblocks; ++cb) {
-                const int steps = cb + 1 == p.cblocks ? p.last_steps : kRow / 32;
-                CmParams::Group g = p.group[0];
-                for (int i = 0; i < groups; ++i) {
-                    const CmParams::Group next = p.group[i + 1];  // (one more than there are: read ahead of its use)
-                    if ((g.first && !wait(&bar_px_full[ps], pphase)) || !wait(&bar_w_full[ws], wphase)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    if (lead) {
-#pragma unroll
-                        for (int j = 0; j < CmParams::kMaxGroup; ++j) {
-                            if (j >= g.count) break;
-                            const uint32_t a = w_lo + (uint32_t)j * tap_step, b = px_lo + g.shift[j];
-                            if (steps == kRow / 32) {
-#pragma unroll
-                                for (int k = 0; k < kRow / 32; ++k) mma_step<kKind>(d, a + 2 * k, b + 2 * k, hi, idesc, k == 0 && j == 0 ? accumulate : 1u);
-                            } else {
-                                mma_step<kKind>(d, a, b, hi, idesc, j == 0 ? accumulate : 1u);
-                                if (steps > 1) mma_step<kKind>(d, a + 2, b + 2, hi, idesc, 1u);
-                                if (steps > 2) mma_step<kKind>(d, a + 4, b + 4, hi, idesc, 1u);
-                            }
+        if (rank == 0) {
+            const bool lead = elect_one();
+            const uint32_t idesc = make_instr_desc(kKind == MmaKind::F16 ? kFmtBF16 : (kKind == MmaKind::TF32 ? kFmtTF32 : kFmtS8),
+                                                   kKind == MmaKind::I8 ? kAccS32 : kAccF32, (uint32_t)p.n_cols, kCtas * kM);
+            const uint32_t hi = desc_hi(8 * kRow, kLayoutSw128);
+            const uint32_t px_lo0 = desc_lo(px_smem, 16), w_lo0 = desc_lo(w_smem, 16);
+            const uint32_t tap_step = (uint32_t)p.w_tap_bytes >> 4;
+            const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+            const int groups = p.groups, w_slots = p.w_slots, px_slots = p.px_slots;
+            int ps = 0, ws = 0, acc = 0;
+            uint32_t pphase = 0, wphase = 0, acc_phase = 0;
+            uint32_t px_lo = px_lo0, w_lo = w_lo0;
+            bool ok = true;
+            for (int item = first; ok && item < items; item += step) {
+                if (!wait(&bar_acc_empty[acc], acc_phase ^ 1u)) break;
+                tc_fence_after_sync();
+                const uint32_t d = tmem + (uint32_t)(acc * kAccCols);
+                uint32_t accumulate = 0;
+                for (int cb = 0; ok && cb < p.cblocks; ++cb) {
+                    const int steps = cb + 1 == p.cblocks ? p.last_steps : kRow / 32;
+                    CmParams::Group g = p.group[0];
+                    for (int i = 0; i < groups; ++i) {
+                        const CmParams::Group next = p.group[i + 1];  // (one more than there are: read ahead of its use)
+                        if ((g.first && !wait(&bar_px_full[ps], pphase)) || !wait(&bar_w_full[ws], wphase)) {
+                            ok = false;
+                            break;
                         }
-                        umma_commit(smem_u32(&bar_w_empty[ws]));
-                        if (g.last) umma_commit(smem_u32(&bar_px_empty[ps]));
+                        tc_fence_after_sync();
+                        if (lead) {
+#pragma unroll
+                            for (int j = 0; j < CmParams::kMaxGroup; ++j) {
+                                if (j >= g.count) break;
+                                const uint32_t a = w_lo + (uint32_t)j * tap_step, b = px_lo + g.shift[j];
+                                if (steps == kRow / 32) {
+#pragma unroll
+                                    for (int k = 0; k < kRow / 32; ++k) mma_step<kKind, kPair>(d, a + 2 * k, b + 2 * k, hi, idesc, k == 0 && j == 0 ? accumulate : 1u);
+                                } else {
+                                    mma_step<kKind, kPair>(d, a, b, hi, idesc, j == 0 ? accumulate : 1u);
+                                    if (steps > 1) mma_step<kKind, kPair>(d, a + 2, b + 2, hi, idesc, 1u);
+                                    if (steps > 2) mma_step<kKind, kPair>(d, a + 4, b + 4, hi, idesc, 1u);
+                                }
+                            }
+                            commit<kPair>(smem_u32(&bar_w_empty[ws]));
+                            if (g.last) commit<kPair>(smem_u32(&bar_px_empty[ps]));
+                        }
+                        __syncwarp();
+                        accumulate = 1;
+                        w_lo += (uint32_t)p.w_slot_bytes >> 4;
+                        if (++ws == w_slots) { ws = 0; wphase ^= 1u; w_lo = w_lo0; }
+                        if (g.last) {
+                            px_lo += (uint32_t)p.px_slot_bytes >> 4;
+                            if (++ps == px_slots) { ps = 0; pphase ^= 1u; px_lo = px_lo0; }
+                        }
+                        g = next;
                     }
-                    __syncwarp();
-                    accumulate = 1;
-                    w_lo += (uint32_t)p.w_slot_bytes >> 4;
-                    if (++ws == w_slots) { ws = 0; wphase ^= 1u; w_lo = w_lo0; }
-                    if (g.last) {
-                        px_lo += (uint32_t)p.px_slot_bytes >> 4;
-                        if (++ps == px_slots) { ps = 0; pphase ^= 1u; px_lo = px_lo0; }
-                    }
-                    g = next;
                 }
+                if (!ok) break;
+                if (lead) commit<kPair>(smem_u32(&bar_acc_full[acc]));
+                __syncwarp();
+                acc ^= 1;
+                if (acc == 0) acc_phase ^= 1u;
             }
-            if (!ok) break;
-            if (lead) umma_commit(smem_u32(&bar_acc_full[acc]));
-            __syncwarp();
-            acc ^= 1;
-            if (acc == 0) acc_phase ^= 1u;
         }
     } else {
         constexpr int kEpiParts = kEpiWarps<kKind> / 4;
@@ -308,13 +349,15 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
         // A lane stores the columns from `col` on of a chunk (four with kVec, else one) for every kLanesC-th channel from `sub` on.
         constexpr int kLanesPx = kVec ? kChunk / 4 : kChunk, kLanesC = 32 / kLanesPx, kStores = 32 / kLanesC;
         const int col = lane % kLanesPx * (kVec ? 4 : 1), sub = lane / kLanesPx;
-        // where those columns lie in the box: image << 16 | row << 8 | column, -1: not a result
+        // where those columns lie in their box: (second box) << 28 | image << 16 | row << 8 | column, -1: not a result
         int place[kMine];
 #pragma unroll
         for (int i = 0; i < kMine; ++i) {
-            const int j = (part + i * kEpiParts) * kChunk + col;
+            int j = (part + i * kEpiParts) * kChunk + col;
+            const int second = kPair && j >= p.n_cols / 2 ? 1 : 0;
+            j -= second * (p.n_cols / 2);
             const int hw = p.HB * p.WB, n_l = j / hw, r = j - n_l * hw, h_l = r / p.WB, w_l = r - h_l * p.WB;
-            place[i] = n_l < p.BNI && h_l < p.BH && w_l < p.BW ? n_l << 16 | h_l << 8 | w_l : -1;
+            place[i] = n_l < p.BNI && h_l < p.BH && w_l < p.BW ? second << 28 | n_l << 16 | h_l << 8 | w_l : -1;
         }
         // of this lane's channel, in the tile `held`: the bias; int8: also K = bias * M + rounding term as in requant_prepare, M, shift - 1
         int held = -1;
@@ -325,19 +368,29 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
         pdl_wait();  // residual reads and result writes must not overtake earlier kernels
         int acc = 0;
         uint32_t acc_phase = 0;
-        for (int item = blockIdx.x; item < items; item += gridDim.x) {
-            const Item t = item_at(p, item);
-            const int c0 = t.ct * kM + quad * 32;
+        for (int item = first; item < items; item += step) {
+            const int group = (int)p.by_c.quotient((unsigned)item), ct = (item - group * p.tiles_c) * kCtas + rank;
+            const Corner t = corner_of(p, group * kCtas);
+            [[maybe_unused]] Corner t2 = t;
+            if constexpr (kPair) t2 = corner_of(p, group * kCtas + 1);
+            // the pixel of this lane's columns of chunk i, and whether there is one
+            auto pixel_of = [&](int i, int* n, int* oh, int* ow) {
+                int at = place[0];
+#pragma unroll
+                for (int k = 1; k < kMine; ++k) at = i == k ? place[k] : at;
+                const bool second = kPair && (at >> 28 & 1) != 0;
+                *n = (second ? t2.n0 : t.n0) + (at >> 16 & 0xfff); *oh = (second ? t2.oh0 : t.oh0) + (at >> 8 & 255); *ow = (second ? t2.ow0 : t.ow0) + (at & 255);
+                return at >= 0 && *n < p.N && *oh < p.OH && *ow < p.OW;
+            };
+            const int c0 = ct * kM + quad * 32;
             const int nch = p.Cout - c0 < 32 ? p.Cout - c0 : 32;
             const uint32_t t_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * kAccCols);
             // the element that this lane's columns of chunk i have in its first channel, and whether there is one
             auto pixel = [&](int i, uint32_t* off) {
-                int at = place[0];
-#pragma unroll
-                for (int k = 1; k < kMine; ++k) at = i == k ? place[k] : at;
-                const int n = t.n0 + (at >> 16), oh = t.oh0 + ((at >> 8) & 255), ow = t.ow0 + (at & 255);
+                int n, oh, ow;
+                const bool there = pixel_of(i, &n, &oh, &ow);
                 *off = ((uint32_t)(n * p.Cout + c0 + sub) * (uint32_t)p.OH + (uint32_t)oh) * (uint32_t)p.OW + (uint32_t)ow;
-                return at >= 0 && n < p.N && oh < p.OH && ow < p.OW;
+                return there;
             };
             auto wait = [&] {
                 const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&bar_acc_full[acc]), acc_phase, abort_ptr));
@@ -347,7 +400,10 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
             auto release = [&] {  // this warp has read its part of the accumulator
                 tc_fence_before_sync();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[acc]));
+                if (lane == 0) {
+                    if constexpr (kPair) mbar_arrive_cluster(map_to_cta(smem_u32(&bar_acc_empty[acc]), 0));
+                    else mbar_arrive(smem_u32(&bar_acc_empty[acc]));
+                }
             };
             const int mine = nch > 0 && part < chunks ? (chunks - part + kEpiParts - 1) / kEpiParts : 0;
             if constexpr (kForm == CmForm::Pixels) {
@@ -356,18 +412,16 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
                 const int ch = lane % kLanes * kElems, px = lane / kLanes;
                 const bool has_bias = p.bias != nullptr, has_res = p.residual != nullptr, relu = p.relu != 0, round = p.round_out_tf32 != 0;
                 constexpr int kBytes = kKind == MmaKind::F16 ? 2 : 4;
-                if (t.ct != held) {
-                    held = t.ct;
+                if (ct != held) {
+                    held = ct;
                     if (has_bias) bias_f = lane < nch ? __ldg(p.bias + c0 + lane) : 0.0f;
                 }
                 // the element of this warp's first channel in the pixel of this lane's column, all ones: no pixel
                 auto element = [&](int i) {
-                    int at = place[0];
-#pragma unroll
-                    for (int k = 1; k < kMine; ++k) at = i == k ? place[k] : at;
-                    const int n = t.n0 + (at >> 16), oh = t.oh0 + ((at >> 8) & 255), ow = t.ow0 + (at & 255);
+                    int n, oh, ow;
+                    const bool there = pixel_of(i, &n, &oh, &ow);
                     const uint32_t e = ((uint32_t)(n * p.OH + oh) * (uint32_t)p.OW + (uint32_t)ow) * (uint32_t)p.Cout + (uint32_t)c0;
-                    return at >= 0 && n < p.N && oh < p.OH && ow < p.OW ? e : 0xffffffffu;
+                    return there ? e : 0xffffffffu;
                 };
                 auto fetch = [&](int i, uint4(&res)[kSteps]) {
                     const uint32_t mine_at = element(i);
@@ -434,8 +488,8 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
                 const float* res_base = static_cast<const float*>(p.residual);
                 float* out = static_cast<float*>(p.out);
                 const bool has_bias = p.bias != nullptr, has_res = res_base != nullptr, relu = p.relu != 0;
-                if (t.ct != held) {
-                    held = t.ct;
+                if (ct != held) {
+                    held = ct;
                     if (has_bias) bias_f = lane < nch ? __ldg(p.bias + c0 + lane) : 0.0f;
                 }
                 auto fetch = [&](int i, float(&res)[32]) {
@@ -510,8 +564,8 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
                     for (int k = 0; k < 32; ++k) res[k] = next[k];
                 }
             } else {
-                if (t.ct != held) {
-                    held = t.ct;
+                if (ct != held) {
+                    held = ct;
                     bias = 0; mult = 0; shift = 2;
                     if (lane < nch) {
                         bias = __ldg(p.bias_i32 + c0 + lane);
@@ -589,24 +643,31 @@ __global__ void __launch_bounds__(kThreads<kKind>, 1) conv_chmajor_kernel(const 
     }
     tc_fence_before_sync();
     __syncthreads();
+    // neither CTA of a pair may release its tensor or shared memory while the other one can still signal or read it
+    if constexpr (kPair) cluster_sync_all();
     tc_fence_after_sync();
     if (warp == 1) {
         __syncwarp();
-        tmem_dealloc(tmem_base, 2 * kAccCols);
+        if constexpr (kPair) tmem_dealloc_pair(tmem_base, 2 * kAccCols);
+        else tmem_dealloc(tmem_base, 2 * kAccCols);
     }
     if (threadIdx.x == 0 && *abort_ptr && p.status != nullptr) atomicExch(p.status, KXC_B200_ERR_DEVICE_WAIT);
 }
 
-template <MmaKind kKind, CmForm kForm>
+template <MmaKind kKind, CmForm kForm, bool kPair>
 int32_t launch(const CmParams& p, cudaStream_t stream) {
     static PerDeviceOnce smem_once;
-    auto kernel = conv_chmajor_kernel<kKind, kForm>;
+    auto kernel = conv_chmajor_kernel<kKind, kForm, kPair>;
     KXC_TRY(smem_opt_in(smem_once, kernel, kSmemLimit));
-    const long long items = (long long)p.tiles_c * p.tiles_w * p.tiles_h * p.tiles_n;
+    const int ctas = kPair ? 2 : 1;
+    const long long boxes = (long long)p.tiles_w * p.tiles_h * p.tiles_n, items = p.tiles_c * ((boxes + ctas - 1) / ctas);
     if (items <= 0) return KXC_B200_OK;
     const int bytes = 1024 + p.px_slots * p.px_slot_bytes + p.w_slots * p.w_slot_bytes + kStagingBytes<kKind>;
-    if (bytes > kSmemLimit || items > INT_MAX) return fail(KXC_B200_ERR_INVALID, "channel-major conv: %d bytes of shared memory, %lld tiles", bytes, items);
-    KXC_CUDA_TRY(launch_kernel(kernel, dim3((unsigned)(items < kNumSMs ? items : kNumSMs)), dim3(kThreads<kKind>), bytes, stream, /*pdl=*/true, 1, p));
+    if (bytes > kSmemLimit || boxes + 1 > INT_MAX || items > INT_MAX) return fail(KXC_B200_ERR_INVALID, "channel-major conv: %d bytes of shared memory, %lld tiles", bytes, items);
+    // (pairs: as many as are resident at once, every form of these kernels takes an SM to itself)
+    const int units = kPair ? tc_split_capacity(2) : kNumSMs;
+    if (units <= 0) return fail(KXC_B200_ERR_CUDA, "channel-major conv: no room for CTA pairs");
+    KXC_CUDA_TRY(launch_kernel(kernel, dim3((unsigned)(ctas * (items < units ? items : units))), dim3(kThreads<kKind>), bytes, stream, /*pdl=*/true, ctas, p));
     return check_launch("conv_chmajor_kernel");
 }
 
@@ -618,16 +679,19 @@ int32_t launch_kind(const CmParams& p, cudaStream_t stream) {
     if constexpr (kKind != MmaKind::I8) {
         if (p.pixels) {
             if ((addr & 15u) != 0 || p.Cout % (kKind == MmaKind::F16 ? 8 : 4) != 0) return fail(KXC_B200_ERR_INVALID, "channel-major conv: NHWC results need 16-byte pixels");
-            return launch<kKind, CmForm::Pixels>(p, stream);
+            return p.ctas == 2 ? launch<kKind, CmForm::Pixels, true>(p, stream) : launch<kKind, CmForm::Pixels, false>(p, stream);
         }
     }
-    return vec ? launch<kKind, CmForm::PlanesVec>(p, stream) : launch<kKind, CmForm::Planes>(p, stream);
+    return vec ? launch<kKind, CmForm::PlanesVec, false>(p, stream) : launch<kKind, CmForm::Planes, false>(p, stream);
 }
 
 int div_up(int a, int b) { return (a + b - 1) / b; }
-long long tiles(const CmGeometry& g, int BW, int BH, int BNI) {
-    return (long long)div_up(g.Cout, kM) * div_up(g.OW, BW) * div_up(g.OH, BH) * div_up(g.N, BNI);
+// work items of a launch: tiles of one CTA, or of a pair
+long long tiles(const CmGeometry& g, int BW, int BH, int BNI, int ctas) {
+    const long long boxes = (long long)div_up(g.OW, BW) * div_up(g.OH, BH) * div_up(g.N, BNI);
+    return (long long)div_up(g.Cout, ctas * kM) * ((boxes + ctas - 1) / ctas);
 }
+long long tiles(const CmPlan& plan) { return tiles(plan.g, plan.c.BW, plan.c.BH, plan.c.BNI, plan.c.ctas); }
 int floor_half(int v) { return (v - (v & 1)) / 2; }
 
 // The taps of a filter as loads: those that share a box (all of them at stride 1, those of one row and column parity at stride 2) or
@@ -672,24 +736,33 @@ bool group_taps(const CmGeometry& g, bool shared, Grouping* out) {
 }
 
 struct Box {
-    double cost = -1.0;
-    int BW = 0, BH = 0, BNI = 0, HB = 0, WB = 0, n = 0, px_slots = 0, w_slots = 0, group = 0;
+    double cost = -1.0, clocks = -1.0;
+    int BW = 0, BH = 0, BNI = 0, HB = 0, WB = 0, n = 0, zero_rows = 0, px_slots = 0, w_slots = 0, group = 0;
 };
 
-// Columns of a loaded box: a multiple of four where the rows of the result are (kVec).
-int box_width(const CmGeometry& g, const Grouping& t, int BW) {
+// Columns of a loaded box: a multiple of four where the rows of the result are (kVec). A pair's box that spans the plane shares its padding: what
+// lies behind a row, and behind an image, is what lies before the next one, and a tap's view runs on into it (7x7 planes of a 3x3
+// filter: 8x8 pixels instead of 9x9, two images in 119 columns instead of 142).
+int box_width(const CmGeometry& g, const Grouping& t, int ctas, int BW) {
+    if (ctas == 2) return BW + t.extra_w - (g.stride == 1 && BW == g.OW && t.extra_w >= g.pad_w ? g.pad_w : 0);
     return (g.OW & 3) == 0 && (BW & 3) == 0 ? div_up(BW + t.extra_w, 4) * 4 : BW + t.extra_w;
+}
+int box_height(const CmGeometry& g, const Grouping& t, int ctas, int BH) {
+    return BH + t.extra_h - (ctas == 2 && g.stride == 1 && BH == g.OH && t.extra_h >= g.pad_h ? g.pad_h : 0);
 }
 
 // Modelled cycles of a launch and the slots of its rings for one tile box; false where shared memory does not hold it.
-bool box_cost(const CmGeometry& g, const Grouping& t, int staging, int BW, int BH, int BNI, Box* b) {
+bool box_cost(const CmGeometry& g, const Grouping& t, int staging, int ctas, int BW, int BH, int BNI, Box* b) {
     b->BW = BW; b->BH = BH; b->BNI = BNI;
-    b->HB = BH + t.extra_h; b->WB = box_width(g, t, BW);
+    b->HB = box_height(g, t, ctas, BH); b->WB = box_width(g, t, ctas, BW);
     const int n = ((BNI - 1) * b->HB + BH - 1) * b->WB + BW;  // the last pixel's flat place, and one
-    if (n > kMaxN || b->WB > 256 || b->HB > 256) return false;
-    b->n = div_up(n, 16) * 16;
+    const int step = 16 / ctas;  // (of a pair's columns each CTA's box has half)
+    if (n > kMaxN / ctas || b->WB > 256 || b->HB > 256) return false;
+    b->n = div_up(n, step) * step;
     const int rows_w = g.Cout < kM ? div_up(g.Cout, 8) * 8 : kM, rows_px = b->HB * b->WB * BNI;
-    const int px_bytes = div_up(rows_px * kRow, 1024) * 1024, tap_bytes = rows_w * kRow;
+    const int last = n + t.extra_h * b->WB + t.extra_w;  // rows that the last tap's view reaches
+    b->zero_rows = ctas == 2 && last > rows_px ? last - rows_px : 0;
+    const int px_bytes = div_up((rows_px + b->zero_rows) * kRow, 1024) * 1024, tap_bytes = rows_w * kRow;
     const int budget = kSmemLimit - 1024 - staging;
     int px_slots, w_slots;
     b->group = 1;
@@ -708,26 +781,37 @@ bool box_cost(const CmGeometry& g, const Grouping& t, int staging, int BW, int B
     b->w_slots = w_slots < kMaxSlots ? w_slots : kMaxSlots;
     int groups = 0;
     for (int l = 0; l < t.loads; ++l) groups += div_up((l + 1 < t.loads ? t.first[l + 1] : t.taps) - t.first[l], b->group);
-    const long long items = tiles(g, BW, BH, BNI);
+    const long long items = tiles(g, BW, BH, BNI, ctas);
     // What a tile costs: its rows at the rate the copies reach shared memory, or its instructions, which fetch 128 + n rows of 32 bytes at
     // 64 bytes a clock, and the hand-over of a group; then its epilogue, which overlaps the next tile. (Boxes chosen so over 200 drawn layers.)
     const double fill = (double)g.cblocks * ((double)t.loads * rows_px + (double)t.taps * rows_w) * 2.6;
     const double mma = (double)t.taps * ((g.cblocks - 1) * 4 + g.last_steps) * (64.0 + 0.5 * b->n);
     const double main_loop = (fill > mma ? fill : mma) + 100.0 * g.cblocks * groups;
     const double epilogue = 1500.0 + 700.0 * div_up(div_up(b->n, kChunk), g.epi_parts);
-    const double waves = (double)((items + kNumSMs - 1) / kNumSMs);
+    const double waves = (double)((items + kNumSMs / ctas - 1) / (kNumSMs / ctas));
     b->cost = main_loop + (waves - 1.0) * (main_loop > epilogue ? main_loop : epilogue) + epilogue + 1e-3 * (double)items;
+    // The same in clocks of 1.85 GHz, with what a launch costs besides: fitted to 753 launches of 381 drawn layers in either form (9 to 12 % rms) after the
+    // loops had come to run on whole warps; for the choice between pairs and the others. (A pair's instruction takes a clock for each
+    // column of a box, 45 at least; a single one half that.)
+    if (g.eb > 1) {
+        const bool pair = ctas == 2;
+        const double rows = (double)g.cblocks * ((double)t.loads * rows_px + (double)t.taps * rows_w) * (pair ? 0.82 : 1.15);
+        const double steps = (double)t.taps * ((g.cblocks - 1) * 4 + g.last_steps) * (pair ? (b->n > 45 ? b->n : 45.0) : 4.0 + 0.463 * b->n);
+        const double loop = (rows > steps ? rows : steps) + (pair ? 190.0 : 553.0) * g.cblocks * groups;
+        const double end = 390.0 + (!g.pixels ? 2600.0 : (g.eb == 2 ? 1610.0 : 2730.0)) * div_up(div_up(b->n * ctas, kChunk), g.epi_parts);
+        b->clocks = (pair ? 6580.0 : 2810.0) + loop + (waves - 1.0) * (loop > end ? loop : end) + end;
+    }
     return true;
 }
 
-// The tile box of a launch; false where the form does not apply.
-bool choose(CmPlan* plan, TcDType dtype, const ConvDims& d) {
+// The tile box of a launch, of single CTAs or of pairs; false where the form does not apply.
+bool choose(CmPlan* plan, TcDType dtype, const ConvDims& d, bool pixels, int ctas) {
     CmGeometry* g = &plan->g;
     CmChoice* best = &plan->c;
     const int eb = tc_elem_bytes(dtype), N = d.N, C = d.C, KH = d.KH, KW = d.KW;
     g->N = N; g->H = d.H; g->W = d.W; g->Cout = d.O; g->KH = KH; g->KW = KW; g->stride = d.SH;
     g->pad_h = d.PH; g->pad_w = d.PW; g->dil_h = d.DH; g->dil_w = d.DW;
-    g->OH = d.OH; g->OW = d.OW;
+    g->OH = d.OH; g->OW = d.OW; g->pixels = pixels ? 1 : 0; g->eb = eb;
     // (elements are counted in 32 bits)
     if (d.SH != d.SW || (d.SH != 1 && d.SH != 2) || g->OH <= 0 || g->OW <= 0 || (unsigned long long)N * d.O * g->OH * g->OW >= (1ull << 32)) return false;
     g->kb_elems = kRow / eb;
@@ -736,32 +820,36 @@ bool choose(CmPlan* plan, TcDType dtype, const ConvDims& d) {
     g->epi_parts = (dtype == kTcS8 ? kEpiWarps<MmaKind::I8> : kEpiWarps<MmaKind::F16>) / 4;
     const int staging = dtype == kTcS8 ? kStagingBytes<MmaKind::I8> : kStagingBytes<MmaKind::F16>;
     best->cost = -1.0;
-    for (int shared = 0; shared < 2; ++shared) {
+    best->ctas = ctas;
+    const int columns = kMaxN / ctas;
+    for (int shared = ctas == 2 ? 1 : 0; shared < 2; ++shared) {
         Grouping t;
         if ((shared && KH * KW == 1) || !group_taps(*g, shared != 0, &t)) continue;
         // widths and heights that divide the plane evenly, from the widest that fits down
-        for (int tw = div_up(d.OW, kMaxN), last_w = 0; tw <= d.OW; ++tw) {
+        for (int tw = div_up(d.OW, columns), last_w = 0; tw <= d.OW; ++tw) {
             const int BW = (d.OW & 3) == 0 ? div_up(div_up(d.OW, tw), 4) * 4 : div_up(d.OW, tw);
             if (BW == last_w) continue;
             last_w = BW;
             if (BW < 8 && tw > 1) break;
-            const int WB = box_width(*g, t, BW), most_h = (kMaxN - BW) / WB + 1;
+            if (BW > columns) continue;
+            const int WB = box_width(*g, t, ctas, BW), most_h = (columns - BW) / WB + 1;
             for (int th = div_up(d.OH, most_h), last_h = 0; th <= d.OH; ++th) {
                 const int BH = div_up(d.OH, th);
                 if (BH == last_h) continue;
                 last_h = BH;
-                if (th > 1 && BW * BH < 48 && best->cost >= 0.0) break;
+                if (th > 1 && BW * BH < 48 / ctas && best->cost >= 0.0) break;
                 int most = 1;
                 if (BH == d.OH) {
-                    most = 1 + (kMaxN - ((BH - 1) * WB + BW)) / ((BH + t.extra_h) * WB);
+                    most = 1 + (columns - ((BH - 1) * WB + BW)) / (box_height(*g, t, ctas, BH) * WB);
                     if (most > N) most = N;
                 }
                 for (int bni = most; bni >= 1; bni = bni > 1 ? bni / 2 : 0) {
                     Box b;
-                    if (box_cost(*g, t, staging, BW, BH, bni, &b) && (best->cost < 0.0 || b.cost < best->cost)) {
-                        best->cost = b.cost;
+                    if (!box_cost(*g, t, staging, ctas, BW, BH, bni, &b)) continue;
+                    if (best->cost < 0.0 || (ctas == 2 ? b.clocks < best->clocks : b.cost < best->cost)) {
+                        best->cost = b.cost; best->clocks = b.clocks;
                         best->shared = shared;
-                        best->BW = BW; best->BH = BH; best->BNI = bni; best->HB = b.HB; best->WB = b.WB; best->n = b.n;
+                        best->BW = BW; best->BH = BH; best->BNI = bni; best->HB = b.HB; best->WB = b.WB; best->n = b.n; best->zero_rows = b.zero_rows;
                         best->px_slots = b.px_slots; best->w_slots = b.w_slots; best->group = b.group;
                     }
                 }
@@ -804,13 +892,19 @@ bool choose(CmPlan* plan, TcDType dtype, const ConvDims& d) {
 // more channels gain from a ratio of 1.6 on (1.0 to 1.25 times, with a residual and without; below it 0.92 to 1.02: 384 -> 384 at 17x14, 63 images, 52.0 /
 // 56.4). Of 840 drawn layers these lines let 264 through, which were 1.12 times as fast (seven lost more than 3 %, the worst tf32 64 -> 32 3x3 of stride 2 at
 // 45x48, 39 images, 29.5 / 32.6).
+// CTA pairs: 3x3 layers of stride 1 and at least four channel blocks, where their fitted clocks (box_cost) are 5.5 % below the other form's
+// (tc_modelled_clocks, or those of single CTAs), not where the reduction is split over three and more. Of 200 drawn layers and those of ResNet-18 at 1 to 512
+// images 73 took them, 1.12 times as fast in the mean (0.86 to 1.37; four lost more than 3 %): 512 -> 512 at 7x7, 64 images, bf16 23.2 / 16.9 us (split
+// in two), tf32 35.3 / 28.1; 256 -> 256 at 14x14, 128 images, 28.7 / 25.7 and 52.6 / 45.0. With fewer channel blocks they lost up to 20 % (32 -> 256 at
+// 17x15, 97 images, tf32 15.8 / 19.9), at stride 2 up to 35 % (256 -> 512 at 14x14, 256 images, tf32 52.7 / 71.2), with 5x5 filters up to 40 %; into planes one
+// of 71 layers gained, int8 planes lost 13 % in the mean.
 // ResNet-18 tf32 32 images 476.8 / 419.6 us, 64: 739 / 661, 256: 2156 / 2028; bf16 32: 265.7 / 254.2, 128: 552 / 545. bf16 layers of stride 2
 // keep the pixel-major kernel: with a 1x1 layer beside them they are one launch of it (two outputs), and alone they give the same bits as there.
-const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcOutMode out_mode) {
+const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcOutMode out_mode, bool residual) {
     // The choices of the last geometries: sets of four, so that the layers of a network called one by one keep theirs (of 11 ResNet-18 layers
     // in 128 single entries, two met in 45 of 128 combinations of batch and precision, and each call of these chose anew: 3 to 20 us).
     struct Entry {
-        int key[17] = {-1};
+        int key[18] = {-1};
         bool use = false;
         CmPlan plan;
     };
@@ -824,7 +918,7 @@ const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcO
         cudaGetLastError();
         return nullptr;
     }
-    const int key[17] = {(int)dtype, d.N, d.C, d.H, d.W, d.O, d.KH, d.KW, d.SH, d.SW, d.PH, d.PW, d.DH, d.DW, weights_ready, (int)out_mode, dev};
+    const int key[18] = {(int)dtype, d.N, d.C, d.H, d.W, d.O, d.KH, d.KW, d.SH, d.SW, d.PH, d.PW, d.DH, d.DW, weights_ready, (int)out_mode, (int)residual, dev};
     uint32_t hash = 0;  // (each step carries the upper bits down: extents are multiples of large powers of two)
     for (const int v : key) {
         hash = (hash ^ (uint32_t)v) * 0x9e3779b1u;
@@ -835,7 +929,8 @@ const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcO
         if (memcmp(w.key, key, sizeof(key)) == 0) return w.use ? &w.plan : nullptr;
     Entry& e = set.way[set.next++ % 4];  // (in turn: the oldest)
     memcpy(e.key, key, sizeof(key));
-    e.use = choose(&e.plan, dtype, d);
+    const bool pixels = out_mode == kOutNHWC_BF16 || out_mode == kOutNHWC_F32;
+    e.use = choose(&e.plan, dtype, d, pixels, 1);
     if (e.use && dtype != kTcS8) {
         TcParams p{};
         TcConfig cfg{};
@@ -847,12 +942,12 @@ const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcO
         if (out_mode == kOutNCHW_F32) {
             const double epilogue = p.split > 1 ? 0.0 : 30.0 * (d.O < cfg.bn ? d.O : cfg.bn);
             const CmChoice& c = e.plan.c;
-            const double ahead = d.KH * d.KW == 1 && tiles(e.plan.g, c.BW, c.BH, c.BNI) <= kNumSMs ? 2800.0 : 1000.0;
+            const double ahead = d.KH * d.KW == 1 && tiles(e.plan) <= kNumSMs ? 2800.0 : 1000.0;
             e.use = rc == KXC_B200_OK && (d.O > 32 || e.plan.g.cblocks > 1) && c.cost + ahead < cfg.clocks + epilogue;
         } else {
             const double ahead = d.KH * d.KW == 1 ? (p.split > 1 ? 1.15 : (dtype == kTcBF16 && d.O > 32 ? 1.6 : 0.80))
                                                   : (p.split > 2 ? 1.0 : (d.SH == 1 ? 0.83 : 0.95));
-            const long long items = tiles(e.plan.g, e.plan.c.BW, e.plan.c.BH, e.plan.c.BNI);
+            const long long items = tiles(e.plan);
             const bool few = d.O > 16 && d.O <= 32;  // channels
             bool stays = dtype == kTcBF16 && d.SH == 2;
             if (e.plan.g.cblocks == 1 && d.SH == 1) {
@@ -860,6 +955,15 @@ const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcO
                 else if (few && d.KH * d.KW == 1 && items > kNumSMs) stays = true;
             }
             e.use = rc == KXC_B200_OK && cfg.clocks >= ahead * e.plan.c.cost && !stays;
+            CmPlan pair;
+            if (rc == KXC_B200_OK && d.O > kM && e.plan.g.cblocks >= 4 && d.KH * d.KW > 1 && d.KH * d.KW <= 9 && d.SH == 1 && p.split <= 2 && tc_split_capacity(2) > 0 &&
+                choose(&pair, dtype, d, true, 2)) {
+                const double other = e.use ? e.plan.c.clocks : tc_modelled_clocks(p, cfg, residual);
+                if (pair.c.clocks < 0.945 * other) {
+                    e.plan = pair;
+                    e.use = true;
+                }
+            }
         }
         // (what a failed query of the device decided is not kept)
         if (rc != KXC_B200_OK || tc_split_capacity(2) <= 0) e.key[0] = -1;
@@ -869,7 +973,7 @@ const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcO
 
 int cm_weight_pad(TcDType t, int c, const CmPlan& plan) {
     const int e128 = kRow / tc_elem_bytes(t);
-    return tiles(plan.g, plan.c.BW, plan.c.BH, plan.c.BNI) > kNumSMs ? div_up(c, e128) * e128 : cm_channel_pad(t, c);
+    return plan.c.ctas * tiles(plan) > kNumSMs ? div_up(c, e128) * e128 : cm_channel_pad(t, c);
 }
 
 int32_t cm_setup(CmParams* p, TcDType dtype, const CmPlan& plan, const void* act_nhwc, const void* w_packed, int cpad, int w_cpad, int* status_word) {
@@ -882,13 +986,14 @@ int32_t cm_setup(CmParams* p, TcDType dtype, const CmPlan& plan, const void* act
     if (px % 16 != 0 || tap % 16 != 0) return fail(KXC_B200_ERR_INVALID, "channel-major conv: %d, %d padded channels x %d bytes", cpad, w_cpad, eb);
     p->N = g.N; p->OH = g.OH; p->OW = g.OW; p->Cout = g.Cout;
     p->kb_elems = g.kb_elems; p->cblocks = g.cblocks; p->last_steps = g.last_steps;
-    p->BW = c.BW; p->BH = c.BH; p->BNI = c.BNI; p->HB = c.HB; p->WB = c.WB; p->n_cols = c.n;
+    p->BW = c.BW; p->BH = c.BH; p->BNI = c.BNI; p->HB = c.HB; p->WB = c.WB; p->ctas = c.ctas; p->n_cols = c.ctas * c.n;
     p->tiles_w = div_up(g.OW, c.BW);
-    p->tiles_h = div_up(g.OH, c.BH); p->tiles_n = div_up(g.N, c.BNI); p->tiles_c = div_up(g.Cout, kM);
+    p->tiles_h = div_up(g.OH, c.BH); p->tiles_n = div_up(g.N, c.BNI); p->tiles_c = div_up(g.Cout, c.ctas * kM);
     p->by_c = Divisor((unsigned)p->tiles_c); p->by_w = Divisor((unsigned)p->tiles_w); p->by_h = Divisor((unsigned)p->tiles_h);
     const int rows_w = g.Cout < kM ? div_up(g.Cout, 8) * 8 : kM;
     p->px_bytes = c.HB * c.WB * c.BNI * kRow;
-    p->px_slot_bytes = div_up(p->px_bytes, 1024) * 1024;
+    p->zero_bytes = c.zero_rows * kRow;
+    p->px_slot_bytes = div_up(p->px_bytes + p->zero_bytes, 1024) * 1024;
     p->w_tap_bytes = rows_w * kRow;
     p->w_slot_bytes = c.group * p->w_tap_bytes;
     p->px_slots = c.px_slots; p->w_slots = c.w_slots;

@@ -27,9 +27,11 @@ struct alignas(64) CmParams {
     int kb_elems, cblocks, last_steps;  // elements of a channel block; blocks; MMAs of the last block
     int BW, BH, BNI;                    // tile box: columns x rows x images of results
     int HB, WB;                         // rows and columns of a loaded box (the tile and the halo of its taps)
-    int n_cols;                         // columns of the accumulator: flat pixels of the loaded box, a multiple of 16
+    int ctas;                           // 2: a pair of CTAs, 256 channels and two boxes to a tile
+    int n_cols;                         // columns of the accumulator: flat pixels of the loaded boxes, a multiple of 16
     int tiles_w, tiles_h, tiles_n, tiles_c;
     Divisor by_c, by_w, by_h;           // of the first three extents of a tile's number: tiles_c, tiles_w, tiles_h
+    int zero_bytes;                     // behind a box: padding that its last taps read
     int px_bytes, px_slot_bytes, px_slots, w_tap_bytes, w_slot_bytes, w_slots;
     int loads, groups;                  // per channel block
     int relu;
@@ -50,11 +52,11 @@ struct alignas(64) CmParams {
 };
 
 struct CmGeometry {
-    int N, H, W, Cout, KH, KW, stride, pad_h, pad_w, dil_h, dil_w, OH, OW, kb_elems, cblocks, last_steps, epi_parts;
+    int N, H, W, Cout, KH, KW, stride, pad_h, pad_w, dil_h, dil_w, OH, OW, pixels, eb, kb_elems, cblocks, last_steps, epi_parts;
 };
 struct CmChoice {
-    double cost;  // modelled clocks
-    int shared, BW, BH, BNI, HB, WB, n, px_slots, w_slots, group;
+    double cost, clocks;  // modelled clocks of single CTAs; of either form (box_cost)
+    int shared, ctas, BW, BH, BNI, HB, WB, n, zero_rows, px_slots, w_slots, group;
 };
 
 struct CmPlan {
@@ -64,7 +66,7 @@ struct CmPlan {
 
 // Whether a convolution into the reference's layout or NHWC (`out_mode`) takes this form, and its tile box; null: it does not. Looked up in the calling thread's
 // last choices, which depend on the geometry and the device alone; valid until the thread's next call.
-const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcOutMode out_mode = kOutNCHW_F32);
+const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcOutMode out_mode = kOutNCHW_F32, bool residual = false);
 // `status_word`: as in tc_setup_conv.
 int32_t cm_setup(CmParams* p, TcDType dtype, const CmPlan& plan, const void* act_nhwc, const void* w_packed, int cpad, int w_cpad, int* status_word = nullptr);
 int32_t cm_launch(TcDType dtype, const CmParams& p, cudaStream_t stream);

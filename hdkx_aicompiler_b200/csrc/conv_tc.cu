@@ -980,6 +980,33 @@ int32_t choose_split(TcParams* p, TcConfig* cfg, const void* w, const void* w_lo
 }
 }  // namespace
 
+// Per form: what a launch costs besides, a K block, the epilogue of a tile (it overlaps the next tile's main loop) NHWC and what a residual adds to it,
+// and both into the reference's layout. Fits over the launches of 381 drawn layers (plans' layers with and without a residual, graph outputs,
+// operators with their conversion apart; 1 to 512 images), 2 to 9 % rms each. Choosing between this and the channel-major kernel's clocks (box_cost
+// there, 12 % rms) lost 1.004 to 1.02 in the mean of each kind of layer against the faster form of each; weighted ratios of older models with lines
+// of their own per kind of layer 1.02 to 1.04.
+double tc_modelled_clocks(const TcParams& p, const TcConfig& cfg, bool residual) {
+    struct Form {
+        double once, block, epilogue, with_residual, planes, planes_with_residual;
+    };
+    const bool bf16 = cfg.dtype == kTcBF16;
+    static constexpr Form kWhole[2][3] = {{{2640, 405, 2720, 0, 2865, 593}, {2700, 427, 6230, 680, 5200, 2080}, {1420, 596, 14080, 2720, 11900, 9160}},    // tf32 64, 128, 256
+                                          {{2620, 417, 2660, 0, 2750, 470}, {2700, 430, 4500, 680, 5200, 2080}, {5480, 590, 6680, 3020, 12950, 8470}}};   // bf16
+    static constexpr Form kTwoTiles[2] = {{2050, 703, 6150, 0, 6600, 490}, {5740, 791, 8070, 1630, 5110, 2360}};                                          // tf32 64, 128
+    static constexpr Form kTwoTilesBf16 = {500, 859, 7770, 2280, 7770, 2280}, k192 = {2530, 477, 5180, 1510, 10630, 5920};
+    static constexpr Form kSplit[2][3] = {{{4520, 401, 4580, 0, 5000, 380}, {5580, 482, 6570, 0, 6530, 660}, {5850, 660, 12950, 0, 9000, 3600}},           // tf32
+                                          {{4660, 489, 3680, 0, 4830, 140}, {5720, 425, 6450, 0, 4820, 2280}, {6100, 751, 10590, 0, 6660, 3610}}};         // bf16
+    const int width = cfg.bn == 64 ? 0 : (cfg.bn == 128 ? 1 : 2);
+    const Form& f = p.split > 1 ? kSplit[bf16][width] : (cfg.mt == 2 ? (bf16 ? kTwoTilesBf16 : kTwoTiles[width == 0 ? 0 : 1]) : (cfg.bn == 192 ? k192 : kWhole[bf16][width]));
+    const long long m_tiles = (long long)p.tiles_w * p.tiles_h * p.tiles_n;
+    const int kb = p.taps_h * p.taps_w * p.cblocks;
+    const long long group = (long long)cfg.ctas * cfg.mt, items = p.tiles_c * ((m_tiles + group - 1) / group), slots = kNumSMs / cfg.ctas;
+    const double waves = p.split > 1 ? 1.0 : (double)((items + slots - 1) / slots);
+    const double main_loop = f.block * (p.split > 1 ? (kb + p.split - 1) / p.split : kb);
+    const double epilogue = cfg.out_mode == kOutNCHW_F32 ? f.planes + (residual ? f.planes_with_residual : 0.0) : f.epilogue + (residual ? f.with_residual : 0.0);
+    return f.once + main_loop + (waves - 1.0) * (main_loop > epilogue ? main_loop : epilogue) + epilogue;
+}
+
 bool tc_dual_applicable(TcDType dtype, TcOutMode out_mode, int cpad, int Cout, int KH, int KW, int stride, int pad_h, int pad_w,
                         int dil_h, int dil_w) {
     // the second output's only tap must be the main filter's centre tap

@@ -107,6 +107,9 @@ int32_t tc_launch_split(const TcConfig& cfg, const TcParams& p, cudaStream_t str
 // Clusters of `split` CTAs that the current device holds at once (whole GPCs' worth: fewer than 148 / split).
 int tc_split_capacity(int split);
 
+// Modelled time of a set-up launch of bf16 or tf32 operands, in clocks of 1.85 GHz, for the comparison with the channel-major kernel's CTA pairs.
+double tc_modelled_clocks(const TcParams& p, const TcConfig& cfg, bool residual);
+
 // Tile box selection: maximise the fraction of the 128 rows that are real output pixels.
 void tc_pick_tile(int N, int OH, int OW, int* BW, int* BH, int* BNI);
 

@@ -1008,7 +1008,7 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
                 } else if (pl->x3) {
                     KXC_TRY(tc_setup_conv_x3(&st.params, &st.cfg, om, pl->storage(st.in0), pw.ptr, pw.ptr_lo, st.N, st.H, st.W, st.cpad, pw.O,
                                              pw.KH, pw.KW, st.pool.strides[0], st.pad_h, st.pad_w, st.pool.pool_size[0], st.pool.pool_size[1]));
-                } else if (const CmPlan* cm = cm_wanted(dt, conv_dims(st, pw), st.params.weights_ready, om)) {
+                } else if (const CmPlan* cm = cm_wanted(dt, conv_dims(st, pw), st.params.weights_ready, om, st.in1 >= 0)) {
                     st.direct = 6;
                     KXC_TRY(cm_setup(&st.cm, dt, *cm, pl->storage(st.in0), pw.ptr, st.cpad, st.cpad));
                     st.cm.relu = st.relu ? 1 : 0;
@@ -1020,6 +1020,7 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
                     st.params.stride = st.pool.strides[0];  // (these as launch_info shows them)
                     st.params.BW = st.cm.BW; st.params.BH = st.cm.BH; st.params.BNI = st.cm.BNI;
                     st.cfg = TcConfig{dt, 128, 128, om};
+                    st.cfg.ctas = st.cm.ctas;
                 } else
                 KXC_TRY(tc_setup_conv(&st.params, &st.cfg, dt, om, pl->storage(st.in0), pw.ptr, st.N, st.H, st.W, st.cpad, pw.O,
                                       pw.KH, pw.KW, st.pool.strides[0], st.pad_h, st.pad_w, st.pool.pool_size[0], st.pool.pool_size[1]));

@@ -91,6 +91,24 @@ CHMAJOR_LAYERS = [
 ]
 
 
+# 3x3 layers of a plan that its CTA pairs take: (images, h, w, channels, residual). pair_layers is a 1x1 layer to those channels, the 3x3 layer, with the
+# first one's result as residual or without, and a pooling that keeps the result NHWC. Boxes of part of a plane and of whole ones, which share their
+# padding, one and two images to a box, an odd number of boxes, and channels that leave the second CTA a part, or nothing, of a tile.
+CHMAJOR_PAIRS = [("tf32", (48, 9, 9, 160, False)), ("tf32", (21, 14, 14, 160, True)), ("tf32", (47, 9, 10, 160, True)), ("tf32", (61, 7, 7, 288, True)),
+                 ("bf16", (10, 14, 15, 320, True)), ("bf16", (195, 4, 4, 320, False))]
+
+
+def pair_layers(relay, case, to_constant, weights, biases):
+    n, h, w, _, residual = case
+    x = relay.Var("input", (n, weights[0].shape[1], h, w))
+    conv = lambda d, i, k: relay.Call("nn_conv2d", [d, relay.Constant(to_constant(weights[i])), relay.Constant(to_constant(biases[i]))],
+                                      relay.Conv2DAttrs((1, 1), (k // 2,) * 4, (1, 1), 1))
+    y = relay.Call("nn_relu", [conv(x, 0, 1)])
+    z = conv(y, 1, 3)
+    z = relay.Call("nn_relu", [relay.Call("add", [z, y]) if residual else z])
+    return relay.Function([x], relay.Call("nn_max_pool2d", [z], relay.MaxPool2DAttrs((1, 1), (1, 1, 1, 1), (1, 1), (3, 3), "NCHW", False)))
+
+
 def chmajor_layers(relay, case, to_constant, weights, biases):
     n, c, h, w, _, k, s = case
     x = relay.Var("input", (n, c, h, w))
