@@ -63,6 +63,11 @@ inline int64_t pool_out_dim(int64_t in, int64_t k, int64_t s, int64_t p0, int64_
 
 // Launch with optional programmatic dependent launch (the kernel must call sm100::pdl_wait() before it touches
 // memory other kernels produce or consume) and an optional cluster of `cluster_x` CTAs.
+// The operators of one pass over memory (pooling, sums, copies, casts, transposes) wait first and name no point before their end at
+// which the next kernel may start: only its launch is prepared meanwhile. us, back to back in one stream: 3x3 max pool + add + ReLU of
+// 1x17x100x54 2.11 -> 1.68 and of 32x64x112x112 26.8 -> 26.6; pool, copy, dense layer and softmax of 32x512x7x7 (1000 classes) 11.6 ->
+// 11.0, and called one by one 18.4 -> 15.6. Letting the next kernel's blocks in at the start of each made those of the dense layer take
+// the shared memory of the pool before them: 13.1, and 72x802x5x5 20.9 for 16.4.
 // KXC_B200_PDL=0 in the environment launches everything fully serialized.
 bool pdl_enabled();
 template <typename... KArgs, typename... Args>

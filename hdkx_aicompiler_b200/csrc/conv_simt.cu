@@ -7,6 +7,7 @@
 // fp32 results are bit-identical to the reference's CPU lowering. They also serve shapes the
 // tensor-core path does not take (dilation, channel counts that do not fill a K block).
 #include "common.cuh"
+#include "sm100.cuh"
 #include "conv_common.cuh"
 
 #include <type_traits>
@@ -33,6 +34,7 @@ template <typename TIn, typename TAcc, typename Epilogue>
 __global__ void __launch_bounds__(kThreads) conv2d_direct_kernel(const TIn* __restrict__ data,
                                                                  const TIn* __restrict__ weight, ConvDims d,
                                                                  Epilogue epi) {
+    sm100::pdl_wait();
     const int64_t total = (int64_t)d.N * d.O * d.OH * d.OW;
     for (int64_t lin = (int64_t)blockIdx.x * kThreads + threadIdx.x; lin < total; lin += (int64_t)gridDim.x * kThreads) {
         const int ow = (int)(lin % d.OW);
@@ -148,6 +150,7 @@ template <int kKW, int kTO, int kTP, int kOG, int kPG, int kMul, int kDeep, type
 __global__ void __launch_bounds__(2 * kOG * kPG, !ExactStage<kKW, kMul>::kAsync && kTO * kTP <= 16 ? 4 : 2)
     conv2d_tiled_f32_kernel(const float* __restrict__ data, const float* __restrict__ weight, ConvDims d, float neg_zero_arg,
                             Epilogue epi) {
+    sm100::pdl_wait();
     using Tile = ExactTile<kTO, kTP, kOG, kPG>;
     using Stage = ExactStage<kKW, kMul>;
     using Smem = ExactSmem<kKW, kTO, kTP, kOG, kPG, kMul, kDeep>;
@@ -482,6 +485,7 @@ __global__ void __launch_bounds__(kThreads) gemm_direct_kernel(const float* __re
                                                                const float* __restrict__ c, float* __restrict__ out,
                                                                int M, int N, int K, float alpha, float beta, int transB,
                                                                int has_c) {
+    sm100::pdl_wait();
     const int64_t total = (int64_t)M * N;
     for (int64_t lin = (int64_t)blockIdx.x * kThreads + threadIdx.x; lin < total; lin += (int64_t)gridDim.x * kThreads) {
         const int j = (int)(lin % N);
@@ -553,7 +557,7 @@ int32_t launch_exact(const float* data, const float* weight, const ConvDims& d, 
     KXC_TRY(smem_opt_in(smem_once, kernel, kBytes));
     const int64_t P = (int64_t)d.N * d.OH * d.OW;
     const dim3 grid((unsigned)((P + Tile::kP - 1) / Tile::kP), (unsigned)((d.O + Tile::kO - 1) / Tile::kO), 1u);
-    kernel<<<grid, 2 * Tile::kThreads, kBytes, s>>>(data, weight, d, -0.0f, epi);
+    KXC_CUDA_TRY(launch_kernel(kernel, grid, dim3(2 * Tile::kThreads), kBytes, s, /*pdl=*/true, 1, data, weight, d, -0.0f, epi));
     return check_launch("nn_conv2d (fp32, tiled)");
 }
 
@@ -601,7 +605,8 @@ int32_t conv2d_fp32_exact(const float* data, const float* weight, const float* b
     if (total == 0) return KXC_B200_OK;
     EpilogueF32 epi{bias, residual, out, relu};
     if (tiled_f32_ok(d)) return launch_tiled_f32(data, weight, d, epi, s);
-    conv2d_direct_kernel<float, float, EpilogueF32><<<grid_for(total), kThreads, 0, s>>>(data, weight, d, epi);
+    KXC_CUDA_TRY(launch_kernel(conv2d_direct_kernel<float, float, EpilogueF32>, dim3(grid_for(total)), dim3(kThreads), 0, s, /*pdl=*/true, 1, data,
+                               weight, d, epi));
     return check_launch("nn_conv2d (fp32)");
 }
 
@@ -610,7 +615,8 @@ int32_t conv2d_s8_exact(const int8_t* data, const int8_t* weight, const int32_t*
     const int64_t total = (int64_t)d.N * d.O * d.OH * d.OW;
     if (total == 0) return KXC_B200_OK;
     EpilogueS8 epi{bias, multiplier, shift, out, relu};
-    conv2d_direct_kernel<int8_t, int32_t, EpilogueS8><<<grid_for(total), kThreads, 0, s>>>(data, weight, d, epi);
+    KXC_CUDA_TRY(launch_kernel(conv2d_direct_kernel<int8_t, int32_t, EpilogueS8>, dim3(grid_for(total)), dim3(kThreads), 0, s, /*pdl=*/true, 1, data,
+                               weight, d, epi));
     return check_launch("nn_conv2d_s8 (direct)");
 }
 
@@ -622,7 +628,8 @@ int32_t gemm_fp32_exact(const float* a, const float* b, const float* c, float* o
     const bool plain = !g.has_c || ((double)g.alpha == 1.0 && (double)g.beta == 1.0);
     const ConvDims d{g.m, g.k, 1, 1, g.n, 1, 1, 1, 1, 0, 0, 1, 1, 1, 1};
     if (g.transB && plain && g.k > 0 && tiled_f32_ok(d)) return launch_tiled_f32(a, b, d, EpilogueF32{g.has_c ? c : nullptr, nullptr, out, 0}, s);
-    gemm_direct_kernel<<<grid_for(total), kThreads, 0, s>>>(a, b, c, out, g.m, g.n, g.k, g.alpha, g.beta, g.transB, g.has_c);
+    KXC_CUDA_TRY(launch_kernel(gemm_direct_kernel, dim3(grid_for(total)), dim3(kThreads), 0, s, /*pdl=*/true, 1, a, b, c, out, g.m, g.n, g.k, g.alpha,
+                               g.beta, g.transB, g.has_c));
     return check_launch("nn_gemm (fp32)");
 }
 

@@ -551,6 +551,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_kernel(const __gri
 // channel e%4; zero for kw >= KW or c >= C.
 __global__ void stem_pack_weights_core_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ out, int O, int C,
                                               int KH, int KW) {
+    sm100::pdl_wait();
     const int total = KH * 4 * kBN * 8;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int e = i & 7, o = (i >> 3) & (kBN - 1), j = (i >> 9) & 3, kh = i >> 11;
@@ -566,6 +567,7 @@ __global__ void stem_pack_weights_core_kernel(const float* __restrict__ w, __nv_
 template <bool kNhwcIn>
 __global__ void __launch_bounds__(256) stem_pack_s8_kernel(const int8_t* __restrict__ x, uint2* __restrict__ out, int N, int C, int H,
                                                             int W, int Hp, int Wp, int pad_h, int pad_w) {
+    sm100::pdl_wait();
     const int64_t total = (int64_t)N * Hp * Wp;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
         const int wp = (int)(i % Wp);
@@ -591,6 +593,7 @@ __global__ void __launch_bounds__(256) stem_pack_s8_kernel(const int8_t* __restr
 // (kOhwi: the weights are [O,KH,KW,C] instead of [O,C,KH,KW])
 template <bool kOhwi>
 __global__ void stem_pack_weights_core_s8_kernel(const int8_t* __restrict__ w, int8_t* __restrict__ out, int O, int C, int KH, int KW) {
+    sm100::pdl_wait();
     const int total = KH * 4 * kBN * 16;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int e = i & 15, o = (i >> 4) & (kBN - 1), j = (i >> 10) & 3, kh = i >> 12;
@@ -615,13 +618,17 @@ int32_t stem_direct_s8_pack(const int8_t* x, const int8_t* w, void* packed_x, vo
     if (blocks > (int64_t)kNumSMs * 16) blocks = (int64_t)kNumSMs * 16;
     const int wblocks = (KH * 4 * kBN * 16 + 255) / 256;
     if (nhwc) {
-        stem_pack_s8_kernel<true><<<(int)blocks, 256, 0, s>>>(x, static_cast<uint2*>(packed_x), N, C, H, W, Hp, Wp, pad_h, pad_w);
+        KXC_CUDA_TRY(launch_kernel(stem_pack_s8_kernel<true>, dim3((int)blocks), dim3(256), 0, s, /*pdl=*/true, 1, x, static_cast<uint2*>(packed_x),
+                                   N, C, H, W, Hp, Wp, pad_h, pad_w));
         KXC_TRY(check_launch("stem_pack_s8"));
-        stem_pack_weights_core_s8_kernel<true><<<wblocks, 256, 0, s>>>(w, static_cast<int8_t*>(packed_w), O, C, KH, KW);
+        KXC_CUDA_TRY(launch_kernel(stem_pack_weights_core_s8_kernel<true>, dim3(wblocks), dim3(256), 0, s, /*pdl=*/true, 1, w,
+                                   static_cast<int8_t*>(packed_w), O, C, KH, KW));
     } else {
-        stem_pack_s8_kernel<false><<<(int)blocks, 256, 0, s>>>(x, static_cast<uint2*>(packed_x), N, C, H, W, Hp, Wp, pad_h, pad_w);
+        KXC_CUDA_TRY(launch_kernel(stem_pack_s8_kernel<false>, dim3((int)blocks), dim3(256), 0, s, /*pdl=*/true, 1, x, static_cast<uint2*>(packed_x),
+                                   N, C, H, W, Hp, Wp, pad_h, pad_w));
         KXC_TRY(check_launch("stem_pack_s8"));
-        stem_pack_weights_core_s8_kernel<false><<<wblocks, 256, 0, s>>>(w, static_cast<int8_t*>(packed_w), O, C, KH, KW);
+        KXC_CUDA_TRY(launch_kernel(stem_pack_weights_core_s8_kernel<false>, dim3(wblocks), dim3(256), 0, s, /*pdl=*/true, 1, w,
+                                   static_cast<int8_t*>(packed_w), O, C, KH, KW));
     }
     return check_launch("stem_pack_weights_core_s8");
 }
@@ -652,7 +659,8 @@ bool stem_direct_applicable(TcDType dtype, int C, int O, int KH, int KW, int OW,
 size_t stem_direct_weight_bytes(int KH) { return (size_t)KH * 4 * kBN * 16; }
 
 int32_t stem_direct_pack_weights(const float* w, void* out, int O, int C, int KH, int KW, cudaStream_t s) {
-    stem_pack_weights_core_kernel<<<(KH * 4 * kBN * 8 + 255) / 256, 256, 0, s>>>(w, static_cast<__nv_bfloat16*>(out), O, C, KH, KW);
+    KXC_CUDA_TRY(launch_kernel(stem_pack_weights_core_kernel, dim3((KH * 4 * kBN * 8 + 255) / 256), dim3(256), 0, s, /*pdl=*/true, 1, w,
+                               static_cast<__nv_bfloat16*>(out), O, C, KH, KW));
     return check_launch("stem_pack_weights_core");
 }
 

@@ -6,6 +6,7 @@
 //   relu : `x > 0 ? x : 0`  (NaN -> 0, -0 -> +0)            include/te/topi/nn.h:19-30
 //   add  : one IEEE fp32 add per element (__fadd_rn, never contracted)   include/te/topi/broadcast.h:90-109
 #include "common.cuh"
+#include "sm100.cuh"
 
 namespace kxc_b200 {
 namespace {
@@ -33,6 +34,7 @@ __device__ __forceinline__ void stg_stream(float4* p, float4 v) { __stcs(p, v); 
 template <bool kRelu>
 __global__ void __launch_bounds__(kThreads) relu_vec_kernel(const float4* __restrict__ x, float4* __restrict__ out,
                                                             int64_t nvec) {
+    sm100::pdl_wait();
     // a block's kUnroll loads cover one contiguous run of kUnroll * kThreads vectors (measured 6 % faster than loads a
     // whole grid apart: the memory system sees one linear sweep)
     const int64_t stride = kThreads;
@@ -51,6 +53,7 @@ __global__ void __launch_bounds__(kThreads) relu_vec_kernel(const float4* __rest
 // copy, 7.3 with the kernel; on the device 1.8 and 2.0)
 __global__ void __launch_bounds__(kThreads) copy_kernel(const float* __restrict__ x, float* __restrict__ out, int64_t n, int vec) {
     const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    sm100::pdl_wait();
     if (vec) {
         if (4 * i + 3 < n) reinterpret_cast<float4*>(out)[i] = __ldg(reinterpret_cast<const float4*>(x) + i);
         else
@@ -65,6 +68,7 @@ __global__ void __launch_bounds__(kThreads) copy_kernel(const float* __restrict_
 }
 
 __global__ void relu_scalar_kernel(const float* __restrict__ x, float* __restrict__ out, int64_t begin, int64_t n) {
+    sm100::pdl_wait();
     for (int64_t i = begin + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = relu1(x[i]);
 }
@@ -72,6 +76,7 @@ __global__ void relu_scalar_kernel(const float* __restrict__ x, float* __restric
 template <bool kRelu>
 __global__ void __launch_bounds__(kThreads) add_vec_kernel(const float4* __restrict__ a, const float4* __restrict__ b,
                                                            float4* __restrict__ out, int64_t nvec) {
+    sm100::pdl_wait();
     const int64_t stride = kThreads;
     for (int64_t i = (int64_t)blockIdx.x * (kUnrollAdd * kThreads) + threadIdx.x; i < nvec; i += (int64_t)gridDim.x * kUnrollAdd * kThreads) {
         float4 va[kUnrollAdd], vb[kUnrollAdd];
@@ -103,6 +108,7 @@ struct BroadcastDims {
 template <bool kRelu>
 __global__ void add_broadcast_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out,
                                      BroadcastDims d, int64_t begin, int64_t total) {
+    sm100::pdl_wait();
     for (int64_t lin = begin + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; lin < total;
          lin += (int64_t)gridDim.x * blockDim.x) {
         int64_t rem = lin, ai = 0, bi = 0;
@@ -146,11 +152,12 @@ extern "C" int32_t kxc_b200_nn_relu(void** packed_args, int64_t numel, void* str
         const int64_t nvec = numel / 4;
         vec_elems = nvec * 4;
         if (nvec > 0)
-            relu_vec_kernel<true><<<grid_for((nvec + kUnroll - 1) / kUnroll), kThreads, 0, s>>>(reinterpret_cast<const float4*>(x),
-                                                                        reinterpret_cast<float4*>(out), nvec);
+            KXC_CUDA_TRY(launch_kernel(relu_vec_kernel<true>, dim3(grid_for((nvec + kUnroll - 1) / kUnroll)), dim3(kThreads), 0, s, /*pdl=*/true, 1,
+                                       reinterpret_cast<const float4*>(x), reinterpret_cast<float4*>(out), nvec));
     }
     if (vec_elems < numel)
-        relu_scalar_kernel<<<grid_for(numel - vec_elems), kThreads, 0, s>>>(x, out, vec_elems, numel);
+        KXC_CUDA_TRY(launch_kernel(relu_scalar_kernel, dim3(grid_for(numel - vec_elems)), dim3(kThreads), 0, s, /*pdl=*/true, 1, x, out, vec_elems,
+                                   numel));
     return check_launch("nn_relu");
 }
 
@@ -160,9 +167,9 @@ extern "C" int32_t kxc_b200_nn_flatten(void** packed_args, int64_t numel, void* 
     if (numel == 0 || packed_args[0] == packed_args[1]) return KXC_B200_OK;
     if (!packed_args[0] || !packed_args[1]) return fail(KXC_B200_ERR_INVALID, "nn_flatten: null tensor pointer");
     if (numel <= 1 << 20) {
-        copy_kernel<<<(unsigned)((numel + 4 * kThreads - 1) / (4 * kThreads)), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const float*>(packed_args[0]), static_cast<float*>(packed_args[1]), numel,
-            aligned16(packed_args[0]) && aligned16(packed_args[1]) ? 1 : 0);
+        KXC_CUDA_TRY(launch_kernel(copy_kernel, dim3((unsigned)((numel + 4 * kThreads - 1) / (4 * kThreads))), dim3(kThreads), 0,
+                                   static_cast<cudaStream_t>(stream), /*pdl=*/true, 1, static_cast<const float*>(packed_args[0]),
+                                   static_cast<float*>(packed_args[1]), numel, aligned16(packed_args[0]) && aligned16(packed_args[1]) ? 1 : 0));
         return check_launch("nn_flatten");
     }
     KXC_CUDA_TRY(cudaMemcpyAsync(packed_args[1], packed_args[0], (size_t)numel * sizeof(float),
@@ -215,16 +222,20 @@ extern "C" int32_t kxc_b200_add(void** packed_args, const kxc_b200_add_desc* des
             auto* b4 = reinterpret_cast<const float4*>(b);
             auto* o4 = reinterpret_cast<float4*>(out);
             if (relu)
-                add_vec_kernel<true><<<grid_for((nvec + kUnrollAdd - 1) / kUnrollAdd), kThreads, 0, s>>>(a4, b4, o4, nvec);
+                KXC_CUDA_TRY(launch_kernel(add_vec_kernel<true>, dim3(grid_for((nvec + kUnrollAdd - 1) / kUnrollAdd)), dim3(kThreads), 0, s,
+                                           /*pdl=*/true, 1, a4, b4, o4, nvec));
             else
-                add_vec_kernel<false><<<grid_for((nvec + kUnrollAdd - 1) / kUnrollAdd), kThreads, 0, s>>>(a4, b4, o4, nvec);
+                KXC_CUDA_TRY(launch_kernel(add_vec_kernel<false>, dim3(grid_for((nvec + kUnrollAdd - 1) / kUnrollAdd)), dim3(kThreads), 0, s,
+                                           /*pdl=*/true, 1, a4, b4, o4, nvec));
         }
     }
     if (done < total) {
         if (relu)
-            add_broadcast_kernel<true><<<grid_for(total - done), kThreads, 0, s>>>(a, b, out, d, done, total);
+            KXC_CUDA_TRY(launch_kernel(add_broadcast_kernel<true>, dim3(grid_for(total - done)), dim3(kThreads), 0, s, /*pdl=*/true, 1, a, b, out, d,
+                                       done, total));
         else
-            add_broadcast_kernel<false><<<grid_for(total - done), kThreads, 0, s>>>(a, b, out, d, done, total);
+            KXC_CUDA_TRY(launch_kernel(add_broadcast_kernel<false>, dim3(grid_for(total - done)), dim3(kThreads), 0, s, /*pdl=*/true, 1, a, b, out, d,
+                                       done, total));
     }
     return check_launch("add");
 }

@@ -158,6 +158,7 @@ __global__ void __launch_bounds__(256) convert_operands_kernel(const float* __re
 // Weights alone: constants of a plan, packed once.
 template <typename TIn, typename TOut, bool kSplit>
 __global__ void __launch_bounds__(256) pack_weights_kernel(PackArgs pack) {
+    sm100::pdl_wait();
     pack_weights_block<TIn, TOut, kSplit>(static_cast<const TIn*>(pack.w), static_cast<TOut*>(pack.out), static_cast<TOut*>(pack.lo), pack, blockIdx.x);
 }
 
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(256) pack_weights_kernel(PackArgs pack) {
 // 16-byte accesses (bound by memory: 4 bytes read and 8 written per value).
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ in, float* __restrict__ hi, float* __restrict__ lo, int64_t rows,
                                                          int cols, int cpad) {
+    sm100::pdl_wait();
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (cols == cpad && (cols & 3) == 0) {
@@ -357,6 +359,7 @@ __global__ void __launch_bounds__(256) transpose_bytes_kernel(TransposeArgs a, P
 
 template <typename TOut>
 __global__ void convert_rows_kernel(const float* __restrict__ in, TOut* __restrict__ out, int64_t rows, int cols, int cpad) {
+    sm100::pdl_wait();
     const int64_t total = rows * cpad;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int c = (int)(i % cpad);
@@ -371,6 +374,7 @@ __global__ void convert_rows_kernel(const float* __restrict__ in, TOut* __restri
 template <typename TOut>
 __global__ void __launch_bounds__(256) convert_two_kernel(const float* __restrict__ a, TOut* __restrict__ out_a, int64_t quads_a,
                                                           const float* __restrict__ b, TOut* __restrict__ out_b, int64_t quads_b) {
+    sm100::pdl_wait();
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < quads_a + quads_b; i += step) {
         const bool first = i < quads_a;
@@ -485,9 +489,11 @@ int32_t convert_rows_two(const float* a, void* out_a, int64_t rows_a, const floa
     const int64_t qa = rows_a * cols / 4, qb = rows_b * cols / 4;
     const int grid = grid_1d(qa + qb, 256);
     if (dtype == kTcBF16)
-        convert_two_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(a, static_cast<__nv_bfloat16*>(out_a), qa, b, static_cast<__nv_bfloat16*>(out_b), qb);
+        KXC_CUDA_TRY(launch_kernel(convert_two_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, s, /*pdl=*/true, 1, a,
+                                   static_cast<__nv_bfloat16*>(out_a), qa, b, static_cast<__nv_bfloat16*>(out_b), qb));
     else
-        convert_two_kernel<float><<<grid, 256, 0, s>>>(a, static_cast<float*>(out_a), qa, b, static_cast<float*>(out_b), qb);
+        KXC_CUDA_TRY(launch_kernel(convert_two_kernel<float>, dim3(grid), dim3(256), 0, s, /*pdl=*/true, 1, a, static_cast<float*>(out_a), qa, b,
+                                   static_cast<float*>(out_b), qb));
     return check_launch("convert_rows_two");
 }
 
@@ -499,7 +505,8 @@ int32_t split_rows(const float* in, float* hi, float* lo, int64_t rows, int cols
         KXC_TRY(convert_rows(in, hi, kTcTF32, rows, cols, cpad, s, false));
         return convert_rows(in, lo, kTcTF32, rows, cols, cpad, s, true);
     }
-    split_rows_kernel<<<grid_1d(vec ? rows * cols / 4 : rows * cpad, 256), 256, 0, s>>>(in, hi, lo, rows, cols, cpad);
+    KXC_CUDA_TRY(launch_kernel(split_rows_kernel, dim3(grid_1d(vec ? rows * cols / 4 : rows * cpad, 256)), dim3(256), 0, s, /*pdl=*/true, 1, in, hi,
+                               lo, rows, cols, cpad));
     return check_launch("split_rows");
 }
 
@@ -540,7 +547,7 @@ int32_t nhwc_to_nchw_s8(const int8_t* in, int8_t* out, int N, int C, int pitch, 
 int32_t pack_weights_ohwi(const WeightPack& w, TcDType dtype, cudaStream_t s) {
     auto go = [&](auto kernel, const PackArgs& p) -> int32_t {
         if (p.blocks == 0) return KXC_B200_OK;
-        kernel<<<p.blocks, 256, 0, s>>>(p);
+        KXC_CUDA_TRY(launch_kernel(kernel, dim3(p.blocks), dim3(256), 0, s, /*pdl=*/true, 1, p));
         return check_launch("pack_weights");
     };
     switch (dtype) {
@@ -558,11 +565,14 @@ int32_t convert_rows(const float* in, void* out, TcDType dtype, int64_t rows, in
     if (total == 0) return KXC_B200_OK;
     const int grid = grid_1d(total, 256);
     if (dtype == kTcBF16)
-        convert_rows_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(in, static_cast<__nv_bfloat16*>(out), rows, cols, cpad);
+        KXC_CUDA_TRY(launch_kernel(convert_rows_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, s, /*pdl=*/true, 1, in,
+                                   static_cast<__nv_bfloat16*>(out), rows, cols, cpad));
     else if (dtype == kTcTF32 && tf32_lo)
-        convert_rows_kernel<Tf32Lo><<<grid, 256, 0, s>>>(in, static_cast<Tf32Lo*>(out), rows, cols, cpad);
+        KXC_CUDA_TRY(launch_kernel(convert_rows_kernel<Tf32Lo>, dim3(grid), dim3(256), 0, s, /*pdl=*/true, 1, in, static_cast<Tf32Lo*>(out), rows,
+                                   cols, cpad));
     else if (dtype == kTcTF32)
-        convert_rows_kernel<float><<<grid, 256, 0, s>>>(in, static_cast<float*>(out), rows, cols, cpad);
+        KXC_CUDA_TRY(launch_kernel(convert_rows_kernel<float>, dim3(grid), dim3(256), 0, s, /*pdl=*/true, 1, in, static_cast<float*>(out), rows, cols,
+                                   cpad));
     else
         return fail(KXC_B200_ERR_INVALID, "convert_rows: dtype");
     return check_launch("convert_rows");

@@ -98,6 +98,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) maxpool_nhwc_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int H,
                                                                 int W, int C, int OH, int OW, int KH, int KW, int SH, int SW,
                                                                 int PT, int PL, int64_t parts) {
+    sm100::pdl_wait();
     constexpr int L = Vec<T>::kLanes;
     const int cg = C / L;
     const int64_t total = (int64_t)N * OH * OW * cg;
@@ -136,6 +137,7 @@ __global__ void __launch_bounds__(kThreads) maxpool_nhwc_kernel(const T* __restr
 template <typename T>
 __global__ void __launch_bounds__(kThreads) maxpool3x3s2p1_nhwc_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int H,
                                                                        int W, int C, int OH, int OW, int64_t parts) {
+    sm100::pdl_wait();
     constexpr int L = Vec<T>::kLanes;
     const int cg = C / L, ow2n = OW / 2, oh2n = OH / 2;
     const int64_t total = (int64_t)N * oh2n * ow2n * cg;
@@ -249,6 +251,7 @@ __global__ void __launch_bounds__(kThreads) gap_nhwc_split_kernel(const T* __res
 template <typename T>
 __global__ void __launch_bounds__(kThreads) eltwise_nhwc_kernel(const T* __restrict__ a, const T* __restrict__ b,
                                                                 T* __restrict__ out, int64_t nvec, int relu, int64_t parts) {
+    sm100::pdl_wait();
     constexpr int L = Vec<T>::kLanes;
     for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < nvec; i += (int64_t)gridDim.x * kThreads) {
         float va[L];
@@ -270,6 +273,7 @@ __global__ void __launch_bounds__(kThreads) eltwise_nhwc_kernel(const T* __restr
 // NHWC (bf16/fp32) -> NCHW fp32 through a shared-memory transpose tile; grid (ceil(HW/32), ceil(C/32), N)
 template <typename T>
 __global__ void nhwc_to_nchw_kernel(const T* __restrict__ in, float* __restrict__ out, int C, int HW) {
+    sm100::pdl_wait();
     __shared__ float tile[32][33];
     const int n = blockIdx.z, hw0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
     const T* src = in + (size_t)n * HW * C;
@@ -347,6 +351,7 @@ __global__ void __launch_bounds__(kThreads) stem_pack_kernel(const float* __rest
 // Stem weights: OIHW fp32 [O,C<=4,KH,KW<=8] -> [O][KH][8][4] operand type, zero for kw >= KW or c >= C
 template <typename T>
 __global__ void stem_pack_weights_kernel(const float* __restrict__ w, T* __restrict__ out, int O, int C, int KH, int KW, int low) {
+    sm100::pdl_wait();
     const int total = O * KH * 32;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int c = i & 3, kw = (i >> 2) & 7;
@@ -395,12 +400,12 @@ int32_t maxpool_nhwc(const void* x, void* out, TcDType dt, int N, int H, int W, 
     if (items == 0) return KXC_B200_OK;
     if (KH == 3 && KW == 3 && SH == 2 && SW == 2 && PT == 1 && PL == 1 && (OH % 2) == 0 && (OW % 2) == 0 && OH == (H + 2 - 3) / 2 + 1 &&
         OW == (W + 2 - 3) / 2 + 1) {
-        KXC_DISPATCH_STORED(dt, full, (maxpool3x3s2p1_nhwc_kernel<T><<<grid_for(items / 4, 16), kThreads, 0, s>>>(
-                                 static_cast<const T*>(x), static_cast<T*>(out), N, H, W, C, OH, OW, parts)));
+        KXC_DISPATCH_STORED(dt, full, KXC_CUDA_TRY(launch_kernel(maxpool3x3s2p1_nhwc_kernel<T>, dim3(grid_for(items / 4, 16)), dim3(kThreads), 0, s,
+                                   /*pdl=*/true, 1, static_cast<const T*>(x), static_cast<T*>(out), N, H, W, C, OH, OW, parts)));
         return check_launch("maxpool3x3s2p1_nhwc");
     }
-    KXC_DISPATCH_STORED(dt, full, (maxpool_nhwc_kernel<T><<<grid_for(items, 16), kThreads, 0, s>>>(
-                             static_cast<const T*>(x), static_cast<T*>(out), N, H, W, C, OH, OW, KH, KW, SH, SW, PT, PL, parts)));
+    KXC_DISPATCH_STORED(dt, full, KXC_CUDA_TRY(launch_kernel(maxpool_nhwc_kernel<T>, dim3(grid_for(items, 16)), dim3(kThreads), 0, s, /*pdl=*/true, 1,
+                               static_cast<const T*>(x), static_cast<T*>(out), N, H, W, C, OH, OW, KH, KW, SH, SW, PT, PL, parts)));
     return check_launch("maxpool_nhwc");
 }
 
@@ -422,8 +427,8 @@ int32_t eltwise_nhwc(const void* a, const void* b, void* out, TcDType dt, int64_
     if (numel % lanes != 0) return fail(KXC_B200_ERR_UNSUPPORTED, "NHWC elementwise: %lld elements is not a multiple of %d", (long long)numel, lanes);
     const int64_t nvec = numel / lanes;
     if (nvec == 0) return KXC_B200_OK;
-    KXC_DISPATCH_STORED(dt, full, (eltwise_nhwc_kernel<T><<<grid_for(nvec, 16), kThreads, 0, s>>>(
-                             static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), nvec, relu, parts)));
+    KXC_DISPATCH_STORED(dt, full, KXC_CUDA_TRY(launch_kernel(eltwise_nhwc_kernel<T>, dim3(grid_for(nvec, 16)), dim3(kThreads), 0, s, /*pdl=*/true, 1,
+                               static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), nvec, relu, parts)));
     return check_launch("eltwise_nhwc");
 }
 
@@ -431,7 +436,8 @@ int32_t nhwc_to_nchw_f32(const void* in, float* out, TcDType dt, int N, int C, i
     if (N == 0) return KXC_B200_OK;
     if (N > 65535) return fail(KXC_B200_ERR_UNSUPPORTED, "layout transform: batch %d exceeds the grid limit", N);
     const dim3 grid((HW + 31) / 32, (C + 31) / 32, N), block(32, 8);
-    KXC_DISPATCH_ACT(dt, (nhwc_to_nchw_kernel<T><<<grid, block, 0, s>>>(static_cast<const T*>(in), out, C, HW)));
+    KXC_DISPATCH_ACT(dt, KXC_CUDA_TRY(launch_kernel(nhwc_to_nchw_kernel<T>, grid, block, 0, s, /*pdl=*/true, 1, static_cast<const T*>(in), out, C,
+                               HW)));
     return check_launch("nhwc_to_nchw");
 }
 
@@ -448,8 +454,8 @@ int32_t stem_pack(const float* x, void* out, TcDType dt, int N, int C, int H, in
 }
 
 int32_t stem_pack_weights(const float* w, void* out, TcDType dt, int O, int C, int KH, int KW, cudaStream_t s, bool tf32_lo) {
-    KXC_DISPATCH_ACT(dt, (stem_pack_weights_kernel<T><<<grid_for((int64_t)O * KH * 32), kThreads, 0, s>>>(w, static_cast<T*>(out), O,
-                                                                                                          C, KH, KW, tf32_lo ? 1 : 0)));
+    KXC_DISPATCH_ACT(dt, KXC_CUDA_TRY(launch_kernel(stem_pack_weights_kernel<T>, dim3(grid_for((int64_t)O * KH * 32)), dim3(kThreads), 0, s,
+                               /*pdl=*/true, 1, w, static_cast<T*>(out), O, C, KH, KW, tf32_lo ? 1 : 0)));
     return check_launch("stem_pack_weights");
 }
 

@@ -7,6 +7,7 @@
 //   gap : s = 0; for h, w: s = s + x; out = s / (float)(H*W)                    include/te/topi/nn.h:260-287
 //         (sequential per plane; planes are staged through shared memory so HBM reads stay coalesced)
 #include "common.cuh"
+#include "sm100.cuh"
 
 #include <cmath>
 
@@ -32,6 +33,7 @@ __global__ void __launch_bounds__(kThreads) pool_generic_kernel(const float* __r
     const int64_t total = d.planes * d.OH * d.OW;
     const float pad_value = -1e30f;
     const float div = (float)(d.KH * d.KW);
+    sm100::pdl_wait();
     for (int64_t lin = (int64_t)blockIdx.x * kThreads + threadIdx.x; lin < total; lin += (int64_t)gridDim.x * kThreads) {
         const int ow = (int)(lin % d.OW);
         const int64_t t = lin / d.OW;
@@ -74,6 +76,7 @@ __global__ void __launch_bounds__(kThreads) maxpool_3x3s2p1_kernel(const float* 
     const int row_pairs = OH >> 1;     // OH is even when this kernel is chosen
     const Index total = (Index)(planes * row_pairs * groups);
     const float pad_value = -1e30f;
+    sm100::pdl_wait();
     for (Index lin = (Index)blockIdx.x * kThreads + threadIdx.x; lin < total; lin += (Index)gridDim.x * kThreads) {
         const Index t = lin / (Index)groups;
         const int g = (int)(lin - t * (Index)groups);
@@ -135,6 +138,7 @@ __global__ void __launch_bounds__(kThreads) maxpool_3x3s2p1_ragged_kernel(const 
                                                                           float* __restrict__ out, uint32_t total, int H, int W, int OH, int OW) {
     const uint32_t row_pairs = (uint32_t)(OH + 1) >> 1;
     const float pad_value = -1e30f;
+    sm100::pdl_wait();
     const uint32_t lin = blockIdx.x * kThreads + threadIdx.x;
     if (lin >= total) return;
     const uint32_t t = lin / (uint32_t)OW;
@@ -183,6 +187,7 @@ __global__ void __launch_bounds__(128) gap_staged_kernel(const float* __restrict
                                                          int64_t planes, int HW, int planes_per_cta, int pitch) {
     extern __shared__ __align__(16) float tile[];
     const float div = (float)HW;
+    sm100::pdl_wait();
     for (int64_t p0 = (int64_t)blockIdx.x * planes_per_cta; p0 < planes; p0 += (int64_t)gridDim.x * planes_per_cta) {
         const int np = (int)((planes - p0 < planes_per_cta) ? (planes - p0) : planes_per_cta);
         const float* src = x + p0 * HW;
@@ -226,6 +231,7 @@ __global__ void __launch_bounds__(128) gap_staged_kernel(const float* __restrict
 // Planes too large to stage: each thread still walks its plane sequentially (exact), uncoalesced.
 __global__ void gap_direct_kernel(const float* __restrict__ x, float* __restrict__ out, int64_t planes, int64_t HW) {
     const float div = (float)HW;
+    sm100::pdl_wait();
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < planes; p += (int64_t)gridDim.x * blockDim.x) {
         const float* row = x + p * HW;
         float s = 0.0f;
@@ -269,15 +275,17 @@ int32_t launch_max_pool(const float* x, const float* res, float* out, const kxc_
         // one item per thread (no grid-stride iterations) up to 64 blocks per SM: the hardware block scheduler
         // balances these short kernels at a finer grain than a persistent loop would
         auto kernel = items < (1ll << 31) ? maxpool_3x3s2p1_kernel<kAddRelu, uint32_t> : maxpool_3x3s2p1_kernel<kAddRelu, int64_t>;
-        kernel<<<grid_for(items, kThreads, 64), kThreads, 0, s>>>(x, res, out, pd.planes, pd.H, pd.W, pd.OH, pd.OW);
+        KXC_CUDA_TRY(launch_kernel(kernel, dim3(grid_for(items, kThreads, 64)), dim3(kThreads), 0, s, /*pdl=*/true, 1, x, res, out, pd.planes, pd.H, pd.W,
+                                   pd.OH, pd.OW));
     } else if (d->kh == 3 && d->kw == 3 && d->stride_h == 2 && d->stride_w == 2 && d->pad_top == 1 && d->pad_left == 1 &&
                pd.planes * ((pd.OH + 1) / 2) * pd.OW < (1ll << 31)) {
         const int64_t items = pd.planes * ((pd.OH + 1) / 2) * pd.OW;
-        maxpool_3x3s2p1_ragged_kernel<kAddRelu><<<(unsigned)((items + kThreads - 1) / kThreads), kThreads, 0, s>>>(x, res, out, (uint32_t)items,
-                                                                                                                pd.H, pd.W, pd.OH, pd.OW);
+        KXC_CUDA_TRY(launch_kernel(maxpool_3x3s2p1_ragged_kernel<kAddRelu>, dim3((unsigned)((items + kThreads - 1) / kThreads)), dim3(kThreads), 0, s,
+                                   /*pdl=*/true, 1, x, res, out, (uint32_t)items, pd.H, pd.W, pd.OH, pd.OW));
     } else {
         const int64_t items = pd.planes * pd.OH * pd.OW;
-        pool_generic_kernel<true, kAddRelu><<<grid_for(items, kThreads, 8), kThreads, 0, s>>>(x, res, out, pd);
+        KXC_CUDA_TRY(launch_kernel(pool_generic_kernel<true, kAddRelu>, dim3(grid_for(items, kThreads, 8)), dim3(kThreads), 0, s, /*pdl=*/true, 1, x, res,
+                                   out, pd));
     }
     return check_launch(name);
 }
@@ -317,8 +325,8 @@ extern "C" int32_t kxc_b200_nn_avg_pool2d(void** packed_args, const kxc_b200_poo
     if (!packed_args || !packed_args[0] || !packed_args[1]) return fail(KXC_B200_ERR_INVALID, "nn_avg_pool2d: null tensor pointer");
     if (pd.planes == 0) return KXC_B200_OK;
     const int64_t items = pd.planes * pd.OH * pd.OW;
-    pool_generic_kernel<false, false><<<grid_for(items, kThreads, 8), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const float*>(packed_args[0]), nullptr, static_cast<float*>(packed_args[1]), pd);
+    KXC_CUDA_TRY(launch_kernel(pool_generic_kernel<false, false>, dim3(grid_for(items, kThreads, 8)), dim3(kThreads), 0, static_cast<cudaStream_t>(stream),
+                               /*pdl=*/true, 1, static_cast<const float*>(packed_args[0]), nullptr, static_cast<float*>(packed_args[1]), pd));
     return check_launch("nn_avg_pool2d");
 }
 
@@ -345,12 +353,10 @@ extern "C" int32_t kxc_b200_nn_global_avg_pool2d(void** packed_args, int32_t n, 
         // one CTA per group of planes (no grid-stride loop unless the count exceeds the grid limit): the hardware
         // hands out CTAs as SMs free up, which balances better than a fixed 3-or-4 iterations per resident CTA
         const int grid = (int)(ctas < 0x7fffffff ? ctas : 0x7fffffff);
-        if (linear)
-            gap_staged_kernel<true><<<grid, 128, (size_t)per_cta * pitch * 4, s>>>(x, out, planes, (int)HW, per_cta, (int)pitch);
-        else
-            gap_staged_kernel<false><<<grid, 128, (size_t)per_cta * pitch * 4, s>>>(x, out, planes, (int)HW, per_cta, (int)pitch);
+        KXC_CUDA_TRY(launch_kernel(linear ? gap_staged_kernel<true> : gap_staged_kernel<false>, dim3(grid), dim3(128), (size_t)per_cta * pitch * 4, s,
+                                   /*pdl=*/true, 1, x, out, planes, (int)HW, per_cta, (int)pitch));
     } else {
-        gap_direct_kernel<<<grid_for(planes, 128, 8), 128, 0, s>>>(x, out, planes, HW);
+        KXC_CUDA_TRY(launch_kernel(gap_direct_kernel, dim3(grid_for(planes, 128, 8)), dim3(128), 0, s, /*pdl=*/true, 1, x, out, planes, HW));
     }
     return check_launch("nn_global_avg_pool2d");
 }

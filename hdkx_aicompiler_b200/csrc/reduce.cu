@@ -12,6 +12,7 @@
 //               the same reference defect applies unless the reduced axes are the trailing ones, so keepdims = 1 is
 //               accepted for trailing axes only.
 #include "common.cuh"
+#include "sm100.cuh"
 
 namespace kxc_b200 {
 namespace {
@@ -22,6 +23,7 @@ __global__ void __launch_bounds__(kSoftmaxThreads) softmax_rows_kernel(const flo
                                                                      int64_t rows, int len) {
     __shared__ float warp_sum[kSoftmaxThreads / 32];
     __shared__ float total;
+    sm100::pdl_wait();
     for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
         const float* xp = x + r * len;
         float* op = out + r * len;
@@ -51,6 +53,7 @@ __global__ void __launch_bounds__(kSoftmaxThreads) softmax_rows_reg_kernel(const
                                                                          int64_t rows, int len) {
     __shared__ float warp_sum[2][kSoftmaxThreads / 32];
     int phase = 0;
+    sm100::pdl_wait();
     for (int64_t r = blockIdx.x; r < rows; r += gridDim.x, phase ^= 1) {
         const float* xp = x + r * len;
         float* op = out + r * len;
@@ -92,6 +95,7 @@ struct ReduceDims {
 };
 
 __global__ void reduce_mean_kernel(const float* __restrict__ x, float* __restrict__ out, ReduceDims d) {
+    sm100::pdl_wait();
     const float div = (float)d.count;
     for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < d.nout; o += (int64_t)gridDim.x * blockDim.x) {
         int64_t rem = o, base = 0;
@@ -143,14 +147,11 @@ extern "C" int32_t kxc_b200_softmax(void** packed_args, const kxc_b200_softmax_d
     const float* xin = static_cast<const float*>(packed_args[0]);
     float* yout = static_cast<float*>(packed_args[1]);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (len <= 4 * kSoftmaxThreads)
-        softmax_rows_reg_kernel<4><<<grid, kSoftmaxThreads, 0, s>>>(xin, yout, rows, (int)len);
-    else if (len <= 8 * kSoftmaxThreads)
-        softmax_rows_reg_kernel<8><<<grid, kSoftmaxThreads, 0, s>>>(xin, yout, rows, (int)len);
-    else if (len <= 16 * kSoftmaxThreads)
-        softmax_rows_reg_kernel<16><<<grid, kSoftmaxThreads, 0, s>>>(xin, yout, rows, (int)len);
-    else
-        softmax_rows_kernel<<<grid, kSoftmaxThreads, 0, s>>>(xin, yout, rows, (int)len);
+    auto kernel = len <= 4 * kSoftmaxThreads    ? softmax_rows_reg_kernel<4>
+                  : len <= 8 * kSoftmaxThreads  ? softmax_rows_reg_kernel<8>
+                  : len <= 16 * kSoftmaxThreads ? softmax_rows_reg_kernel<16>
+                                                : softmax_rows_kernel;
+    KXC_CUDA_TRY(launch_kernel(kernel, dim3(grid), dim3(kSoftmaxThreads), 0, s, /*pdl=*/true, 1, xin, yout, rows, (int)len));
     return check_launch("softmax");
 }
 
@@ -202,7 +203,7 @@ extern "C" int32_t kxc_b200_reduce_mean(void** packed_args, const kxc_b200_reduc
     }
     const int64_t blocks = (d.nout + 127) / 128;
     const int grid = (int)(blocks < (int64_t)kNumSMs * 16 ? blocks : (int64_t)kNumSMs * 16);
-    reduce_mean_kernel<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const float*>(packed_args[0]),
-                                                                          static_cast<float*>(packed_args[1]), d);
+    KXC_CUDA_TRY(launch_kernel(reduce_mean_kernel, dim3(grid), dim3(128), 0, static_cast<cudaStream_t>(stream), /*pdl=*/true, 1,
+                               static_cast<const float*>(packed_args[0]), static_cast<float*>(packed_args[1]), d));
     return check_launch("reduce_mean");
 }

@@ -13,6 +13,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "sm100.cuh"
 
 namespace kxc_b200 {
 namespace {
@@ -48,6 +49,7 @@ __device__ __forceinline__ int64_t transpose_src_offset(I o, const TransposeDims
 
 template <typename T, typename I>
 __global__ void __launch_bounds__(256) transpose_rows_kernel(const T* __restrict__ in, T* __restrict__ out, TransposeDims d) {
+    sm100::pdl_wait();
     const I total = (I)d.total, stride = (I)gridDim.x * 256;
     I o = (I)blockIdx.x * 256 + threadIdx.x;
     for (; o + stride < total; o += 2 * stride) {
@@ -70,6 +72,7 @@ struct TileDims {
 
 template <typename T>
 __global__ void __launch_bounds__(kTile* kTileRows) transpose_tiles_kernel(const T* __restrict__ in, T* __restrict__ out, TileDims d) {
+    sm100::pdl_wait();
     __shared__ T tile[kTile][kTile + 1];
     const int tx = threadIdx.x & (kTile - 1), ty = threadIdx.x / kTile;
     for (int64_t t = blockIdx.x; t < d.tiles; t += gridDim.x) {
@@ -118,6 +121,7 @@ constexpr int kVTile = 64;
 
 __global__ void __launch_bounds__(256) transpose_tiles_vec4_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                                   TileDims d) {
+    sm100::pdl_wait();
     __shared__ uint32_t tile[kVTile][kVTile + 1];  // tile[x][y]
     const int lane16 = threadIdx.x & 15, row16 = threadIdx.x >> 4;  // 16 float4 per 64-element row, 16 rows per pass
     for (int64_t t = blockIdx.x; t < d.tiles; t += gridDim.x) {
@@ -175,9 +179,11 @@ template <typename T>
 int32_t rows_launch(const void* in, void* out, const TransposeDims& m, cudaStream_t s) {
     const int grid = grid_for((m.total + 511) / 512);
     if (m.total < (int64_t)1 << 31)
-        transpose_rows_kernel<T, uint32_t><<<grid, 256, 0, s>>>(static_cast<const T*>(in), static_cast<T*>(out), m);
+        KXC_CUDA_TRY(launch_kernel(transpose_rows_kernel<T, uint32_t>, dim3(grid), dim3(256), 0, s, /*pdl=*/true, 1, static_cast<const T*>(in),
+                                   static_cast<T*>(out), m));
     else
-        transpose_rows_kernel<T, int64_t><<<grid, 256, 0, s>>>(static_cast<const T*>(in), static_cast<T*>(out), m);
+        KXC_CUDA_TRY(launch_kernel(transpose_rows_kernel<T, int64_t>, dim3(grid), dim3(256), 0, s, /*pdl=*/true, 1, static_cast<const T*>(in),
+                                   static_cast<T*>(out), m));
     return check_launch("transpose");
 }
 
@@ -209,7 +215,8 @@ int32_t transpose_launch(const void* in, void* out, const TransposeDims& m, cons
             d.tiles_y = (d.Y + kVTile - 1) / kVTile;
             d.tiles = d.tiles_x * d.tiles_y;
             for (int j = 0; j < d.nb; ++j) d.tiles *= d.bshape[j];
-            transpose_tiles_vec4_kernel<<<grid_for(d.tiles), 256, 0, s>>>(static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), d);
+            KXC_CUDA_TRY(launch_kernel(transpose_tiles_vec4_kernel, dim3(grid_for(d.tiles)), dim3(256), 0, s, /*pdl=*/true, 1,
+                                       static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), d));
             return check_launch("transpose");
         }
     }
@@ -217,7 +224,8 @@ int32_t transpose_launch(const void* in, void* out, const TransposeDims& m, cons
     d.tiles_y = (d.Y + kTile - 1) / kTile;
     d.tiles = d.tiles_x * d.tiles_y;
     for (int j = 0; j < d.nb; ++j) d.tiles *= d.bshape[j];
-    transpose_tiles_kernel<T><<<grid_for(d.tiles), kTile * kTileRows, 0, s>>>(static_cast<const T*>(in), static_cast<T*>(out), d);
+    KXC_CUDA_TRY(launch_kernel(transpose_tiles_kernel<T>, dim3(grid_for(d.tiles)), dim3(kTile * kTileRows), 0, s, /*pdl=*/true, 1,
+                               static_cast<const T*>(in), static_cast<T*>(out), d));
     return check_launch("transpose");
 }
 
@@ -246,6 +254,7 @@ __device__ __forceinline__ D convert_elem(S v) {
 
 template <typename S, typename D>
 __global__ void __launch_bounds__(256) cast_kernel(const S* __restrict__ in, D* __restrict__ out, int64_t n) {
+    sm100::pdl_wait();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (; i + 3 * stride < n; i += 4 * stride) {  // four independent loads in flight per thread
@@ -266,6 +275,7 @@ struct alignas(sizeof(T) * V) ElemVec {
 
 template <typename S, typename D, int V>
 __global__ void __launch_bounds__(256) cast_vec_kernel(const S* __restrict__ in, D* __restrict__ out, int64_t n) {
+    sm100::pdl_wait();
     const int64_t nv = n / V;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const ElemVec<S, V>* in_v = reinterpret_cast<const ElemVec<S, V>*>(in);
@@ -301,9 +311,11 @@ int32_t cast_launch(const void* in, void* out, int64_t n, cudaStream_t s) {
     const bool aligned = (reinterpret_cast<uintptr_t>(in) % (sizeof(S) * V) == 0) && (reinterpret_cast<uintptr_t>(out) % (sizeof(D) * V) == 0);
     if (aligned && n >= V) {
         const int64_t nv = n / V;
-        cast_vec_kernel<S, D, V><<<grid_for((nv + 511) / 512), 256, 0, s>>>(static_cast<const S*>(in), static_cast<D*>(out), n);
+        KXC_CUDA_TRY(launch_kernel(cast_vec_kernel<S, D, V>, dim3(grid_for((nv + 511) / 512)), dim3(256), 0, s, /*pdl=*/true, 1,
+                                   static_cast<const S*>(in), static_cast<D*>(out), n));
     } else {
-        cast_kernel<S, D><<<grid_for((n + 1023) / 1024), 256, 0, s>>>(static_cast<const S*>(in), static_cast<D*>(out), n);
+        KXC_CUDA_TRY(launch_kernel(cast_kernel<S, D>, dim3(grid_for((n + 1023) / 1024)), dim3(256), 0, s, /*pdl=*/true, 1, static_cast<const S*>(in),
+                                   static_cast<D*>(out), n));
     }
     return check_launch("cast");
 }

@@ -995,3 +995,39 @@ def test_native_calls_leave_modes_and_subclasses_alone(ops):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(z, x.clamp(min=0))
+
+
+@pytest.mark.parametrize("n,c,hw", [(1, 5, 9), (3, 33, 20), (16, 64, 56)])
+@pytest.mark.parametrize("captured", [False, True])
+def test_queued_operators_wait_for_one_another(ops, rng, n, c, hw, captured):
+    """Each launch is prepared while the kernel before it runs: operators that read what the one before wrote, into memory that
+    the allocator has just taken from an earlier result, give what they give one by one."""
+    x, b = dev(rng.normal(size=(n, c, hw, hw)).astype(f32)), dev(rng.normal(size=21).astype(f32))
+    w = dev(rng.normal(0, 0.01, (21, c)).astype(f32))  # (the softmax takes exp of the values themselves: at most 16 |x| * 64 |w| < 88)
+
+    def chain(after):
+        out = []
+        for _ in range(8):
+            y = x
+            for f in (lambda t: ops.add(t, t, relu=True), ops.nn_relu, lambda t: ops.add(t, t[:1, :, :1]),
+                      lambda t: ops.cast(ops.cast(t, torch.float64), torch.float32), lambda t: ops.transpose(t, (0, 2, 3, 1)),
+                      lambda t: ops.transpose(t, (0, 3, 1, 2)), lambda t: ops.nn_max_pool2d(t, (3, 3), (2, 2), (1, 1, 1, 1)),
+                      lambda t: ops.max_pool2d_add_relu(t, ops.nn_max_pool2d(t, (3, 3), (2, 2), (1, 1, 1, 1)), (3, 3), (2, 2), (1, 1, 1, 1)),
+                      lambda t: ops.nn_avg_pool2d(t, (2, 2), (1, 1)), lambda t: ops.add(t, ops.reduce_mean(t, [0], keepdims=False)), ops.nn_global_avg_pool2d,
+                      ops.nn_flatten, lambda t: ops.nn_gemm(t, w, b, transB=1, precision="fp32"), ops.softmax):
+                y = f(y)
+                after()
+            out.append(y)
+        return out
+
+    expected = [t.cpu() for t in chain(torch.cuda.synchronize)]
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = chain(lambda: None)
+        graph.replay()
+    else:
+        got = chain(lambda: None)
+    torch.cuda.synchronize()
+    for g, e in zip(got, expected):
+        assert torch.isfinite(e).all() and torch.equal(g.cpu(), e)
