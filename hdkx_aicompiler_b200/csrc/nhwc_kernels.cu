@@ -392,6 +392,9 @@ int grid_for(int64_t items, int per_sm = 8) {
     } else                                                   \
         KXC_DISPATCH_ACT(dtype, __VA_ARGS__)
 
+// Pooling and sums of plans are launched when the kernel before them has ended: that one, a convolution, lets the next one's blocks in at its own
+// start, and these loops over a fixed grid then run where an SM came free first, not evenly (112x112x64 fp32, three-pass plans: 4 images 7.0 us, 10.2
+// launched ahead; 32: 36.4 / 40.2, 64: 68.4 / 75.0).
 int32_t maxpool_nhwc(const void* x, void* out, TcDType dt, int N, int H, int W, int C, int OH, int OW, int KH, int KW, int SH,
                      int SW, int PT, int PL, cudaStream_t s, bool full, int64_t parts) {
     const int lanes = dt == kTcBF16 ? 8 : 4;
@@ -401,10 +404,10 @@ int32_t maxpool_nhwc(const void* x, void* out, TcDType dt, int N, int H, int W, 
     if (KH == 3 && KW == 3 && SH == 2 && SW == 2 && PT == 1 && PL == 1 && (OH % 2) == 0 && (OW % 2) == 0 && OH == (H + 2 - 3) / 2 + 1 &&
         OW == (W + 2 - 3) / 2 + 1) {
         KXC_DISPATCH_STORED(dt, full, KXC_CUDA_TRY(launch_kernel(maxpool3x3s2p1_nhwc_kernel<T>, dim3(grid_for(items / 4, 16)), dim3(kThreads), 0, s,
-                                   /*pdl=*/true, 1, static_cast<const T*>(x), static_cast<T*>(out), N, H, W, C, OH, OW, parts)));
+                                   /*pdl=*/false, 1, static_cast<const T*>(x), static_cast<T*>(out), N, H, W, C, OH, OW, parts)));
         return check_launch("maxpool3x3s2p1_nhwc");
     }
-    KXC_DISPATCH_STORED(dt, full, KXC_CUDA_TRY(launch_kernel(maxpool_nhwc_kernel<T>, dim3(grid_for(items, 16)), dim3(kThreads), 0, s, /*pdl=*/true, 1,
+    KXC_DISPATCH_STORED(dt, full, KXC_CUDA_TRY(launch_kernel(maxpool_nhwc_kernel<T>, dim3(grid_for(items, 16)), dim3(kThreads), 0, s, /*pdl=*/false, 1,
                                static_cast<const T*>(x), static_cast<T*>(out), N, H, W, C, OH, OW, KH, KW, SH, SW, PT, PL, parts)));
     return check_launch("maxpool_nhwc");
 }
@@ -427,7 +430,7 @@ int32_t eltwise_nhwc(const void* a, const void* b, void* out, TcDType dt, int64_
     if (numel % lanes != 0) return fail(KXC_B200_ERR_UNSUPPORTED, "NHWC elementwise: %lld elements is not a multiple of %d", (long long)numel, lanes);
     const int64_t nvec = numel / lanes;
     if (nvec == 0) return KXC_B200_OK;
-    KXC_DISPATCH_STORED(dt, full, KXC_CUDA_TRY(launch_kernel(eltwise_nhwc_kernel<T>, dim3(grid_for(nvec, 16)), dim3(kThreads), 0, s, /*pdl=*/true, 1,
+    KXC_DISPATCH_STORED(dt, full, KXC_CUDA_TRY(launch_kernel(eltwise_nhwc_kernel<T>, dim3(grid_for(nvec, 16)), dim3(kThreads), 0, s, /*pdl=*/false, 1,
                                static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), nvec, relu, parts)));
     return check_launch("eltwise_nhwc");
 }
