@@ -68,17 +68,20 @@ struct StageGeom {
 // kX3 (three-pass tf32): every stage carries the high and low parts of both operands, so a tap's pixels and weights cross
 // L2 -> shared memory twice instead of three times and no partial sum leaves the chip. The B tile is [w_hi; w_lo] (2 BN
 // rows): ONE instruction of N = 2 BN multiplies a_hi with both and fills the accumulators hi*hi | hi*lo side by side, a
-// second of N = BN adds a_lo * w_hi to the latter. The two sums meet in one rounded fp32 add in the epilogue. An
-// instruction costs ~140 / 205 cycles at N = 128 / 256 and ~96 / 140 at 64 / 128 (operand fetch), so a stage of four K steps
-// is ~950 (BN 64) or ~1400 cycles (BN 128), just above the ~50 B/clk at which an SM's stage (48 / 64 KB) arrives.
+// second of N = BN adds a_lo * w_hi to the latter. The two sums meet in one rounded fp32 add in the epilogue. A stage of four K steps
+// is 448 cycles of the tensor pipe with 64 channels (64 + 48 a step) and 768 with 128, but takes 650 to 850 and 1030: its 48 or 64 KB
+// arrive at ~60 bytes a cycle.
+// Pairs (64 channels): 40 KB a stage and CTA, whose half of the B tile is [w_hi; w_lo] of 32 channels. The wide instruction then
+// gives hi*hi | hi*lo of either half, so lo*hi has columns of its own and the epilogue adds three sums. 630 to 790 cycles a stage: ResNet-18's layers, us,
+// 32 images 28x28 45.3 -> 40.0 (128 channels a tile before), 56x56 50.5 -> 47.5, 64 images 14x14 81 -> 73; whole networks 32: 873 -> 841, 48: 1260 -> 1204.
 template <MmaKind kKind, int KB_BYTES, int BN, int kOutMode, int kCtas, bool kDual = false, int kMT = 1, bool kX3 = false>
 __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_constant__ TcParams p) {
     using G = StageGeom<KB_BYTES, BN, kCtas, kMT, kX3, kOutMode == kOutNCHW_F32>;
     static_assert(!(kDual && kMT != 1), "the two-output kernel works on one pixel tile at a time");
-    static_assert(!kX3 || (kKind == MmaKind::TF32 && kCtas == 1 && !kDual && kMT == 1 && BN <= 128), "three-pass form: tf32, single CTAs");
+    static_assert(!kX3 || (kKind == MmaKind::TF32 && !kDual && kMT == 1 && BN <= 128 / kCtas), "three-pass form: tf32, one pixel tile, pairs of 64 channels");
     constexpr bool kPair = kCtas == 2;
     constexpr int kStages = G::kStages;
-    constexpr int kAccCols = (kDual || kX3 ? 2 : kMT) * BN;  // TMEM columns of one accumulator buffer
+    constexpr int kAccCols = (kX3 && kPair ? 3 : (kDual || kX3 ? 2 : kMT)) * BN;  // TMEM columns of one accumulator buffer
     // two accumulator buffers (the epilogue of one work item overlaps the next item's main loop) where TMEM's 512
     // columns allow it, else one
     constexpr int kBufs = 2 * kAccCols <= 512 ? 2 : 1;
@@ -89,7 +92,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
     constexpr uint32_t kIdesc =
         make_instr_desc(kKind == MmaKind::F16 ? kFmtBF16 : (kKind == MmaKind::TF32 ? kFmtTF32 : kFmtS8),
                         kKind == MmaKind::I8 ? kAccS32 : kAccF32, BN, 128u * kCtas);
-    [[maybe_unused]] constexpr uint32_t kIdescWide = make_instr_desc(kFmtTF32, kAccF32, 2 * BN <= 256 ? 2 * BN : 256, 128u);  // x3: [w_hi; w_lo]
+    [[maybe_unused]] constexpr uint32_t kIdescWide = make_instr_desc(kFmtTF32, kAccF32, 2 * BN <= 256 ? 2 * BN : 256, 128u * kCtas);  // x3: [w_hi; w_lo]
 
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[kStages];
@@ -200,7 +203,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                             for (int t = 0; t < kMT; ++t)
                                 tma_load_4d_pair(a_dst + t * G::kATileBytes, &p.tmA[map], full0, cb * p.kb_elems, ow0[t] + cw,
                                                  oh0[t] + ch, n0[t]);
-                            tma_load_2d_pair(a_dst + G::kABytes, &p.tmB, full0, kb * p.kb_elems, co0);
+                            if constexpr (kX3) {
+                                tma_load_4d_pair(a_dst + G::kATileBytes, &p.tmA[map], full0, cb * p.kb_elems, ow0[0] + cw, oh0[0] + ch, n0[0] + p.N);
+                                tma_load_2d_pair(a_dst + G::kABytes, &p.tmB, full0, kb * p.kb_elems, co0);
+                                tma_load_2d_pair(a_dst + G::kABytes + G::kBTileBytes, &p.tmB2, full0, kb * p.kb_elems, co0);
+                            } else {
+                                tma_load_2d_pair(a_dst + G::kABytes, &p.tmB, full0, kb * p.kb_elems, co0);
+                            }
                         } else {
                             mbar_arrive_expect_tx(full, tx_bytes);
 #pragma unroll
@@ -275,9 +284,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
 #pragma unroll
                         for (int k = 0; k < KB_BYTES / 32; ++k) {
                             if constexpr (kX3) {
-                                const uint64_t a_k = a_desc + (uint64_t)(2 * k), b_k = b_desc + (uint64_t)(2 * k);
-                                umma<kKind>(d_tmem, a_k, b_k, kIdescWide, (kb_local | k) != 0 ? 1u : 0u);
-                                umma<kKind>(d_tmem + (uint32_t)BN, a_k + (uint64_t)(G::kATileBytes >> 4), b_k, kIdesc, 1u);
+                                const uint64_t a_k = a_desc + (uint64_t)(2 * k), b_k = b_desc + (uint64_t)(2 * k), a_lo = a_k + (uint64_t)(G::kATileBytes >> 4);
+                                if constexpr (kPair) {
+                                    umma_pair<kKind>(d_tmem, a_k, b_k, kIdescWide, (kb_local | k) != 0 ? 1u : 0u);
+                                    umma_pair<kKind>(d_tmem + (uint32_t)(2 * BN), a_lo, b_k, kIdesc, (kb_local | k) != 0 ? 1u : 0u);
+                                } else {
+                                    umma<kKind>(d_tmem, a_k, b_k, kIdescWide, (kb_local | k) != 0 ? 1u : 0u);
+                                    umma<kKind>(d_tmem + (uint32_t)BN, a_lo, b_k, kIdesc, 1u);
+                                }
                             } else {
 #pragma unroll
                             for (int t = 0; t < kMT; ++t) {
@@ -410,7 +424,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                 }
                 tc_fence_after_sync();
             }
-            const uint32_t t_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * kAccCols + t * BN + col0);
+            // (x3 pairs: of either half of the channels hi*hi and hi*lo, then lo*hi of all)
+            const uint32_t t_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * kAccCols + t * BN + col0 + (kX3 && kPair ? half * (BN / 2) : 0));
+            [[maybe_unused]] const uint32_t u_addr = t_addr + (uint32_t)(kPair ? BN / 2 : BN), w_addr = t_addr + (uint32_t)(2 * BN - half * (BN / 2));
             if (kOutMode == kOutNCHW_F32 && small_nchw) {
                 if constexpr (kOutMode == kOutNCHW_F32) {
                     // unrolled: the two chunks of residual values in flight then need not be moved
@@ -427,7 +443,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                         __syncwarp();
                         if constexpr (kX3) {
                             uint32_t u[32];
-                            tmem_ld_32x32(t_addr + (uint32_t)(BN + i * 32), u);
+                            tmem_ld_32x32(u_addr + (uint32_t)(i * 32), u);
+                            if constexpr (kPair) {
+                                uint32_t w[32];
+                                tmem_ld_32x32(w_addr + (uint32_t)(i * 32), w);
+                                tmem_ld_wait();
+#pragma unroll
+                                for (int j = 0; j < 32; ++j) u[j] = __float_as_uint(__fadd_rn(__uint_as_float(u[j]), __uint_as_float(w[j])));
+                            }
                             tmem_ld_wait();
 #pragma unroll
                             for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j])));
@@ -456,7 +479,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                 }
                 if constexpr (kX3) {
                     uint32_t u[32];
-                    tmem_ld_32x32(t_addr + (uint32_t)(BN + i * 32), u);
+                    tmem_ld_32x32(u_addr + (uint32_t)(i * 32), u);
+                    if constexpr (kPair) {
+                        uint32_t w[32];
+                        tmem_ld_32x32(w_addr + (uint32_t)(i * 32), w);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) u[j] = __float_as_uint(__fadd_rn(__uint_as_float(u[j]), __uint_as_float(w[j])));
+                    }
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j])));
@@ -636,11 +666,11 @@ int32_t launch_by_out(const TcConfig& cfg, const TcParams& p, cudaStream_t s) {
     return fail(KXC_B200_ERR_INVALID, "tensor-core conv: output mode %d does not fit dtype %d", (int)cfg.out_mode, (int)cfg.dtype);
 }
 
-template <int KB_BYTES, int BN>
+template <int KB_BYTES, int BN, int kCtas>
 int32_t launch_x3(const TcConfig& cfg, const TcParams& p, cudaStream_t s) {
     switch (cfg.out_mode) {
-        case kOutNHWC_F32: return launch_one<MmaKind::TF32, KB_BYTES, BN, kOutNHWC_F32, 1, false, 1, true>(p, s);
-        case kOutNCHW_F32: return launch_one<MmaKind::TF32, KB_BYTES, BN, kOutNCHW_F32, 1, false, 1, true>(p, s);
+        case kOutNHWC_F32: return launch_one<MmaKind::TF32, KB_BYTES, BN, kOutNHWC_F32, kCtas, false, 1, true>(p, s);
+        case kOutNCHW_F32: return launch_one<MmaKind::TF32, KB_BYTES, BN, kOutNCHW_F32, kCtas, false, 1, true>(p, s);
         default: return fail(KXC_B200_ERR_INVALID, "tensor-core conv: output mode %d has no three-pass form", (int)cfg.out_mode);
     }
 }
@@ -649,8 +679,11 @@ template <MmaKind kKind, int KB_BYTES>
 int32_t launch_by_bn(const TcConfig& cfg, const TcParams& p, cudaStream_t s) {
     if (cfg.x3) {
         if constexpr (kKind == MmaKind::TF32) {
+            if constexpr (KB_BYTES == 128) {
+                if (cfg.ctas == 2 && cfg.mt == 1 && !cfg.dual && cfg.bn == 64) return launch_x3<KB_BYTES, 64, 2>(cfg, p, s);
+            }
             if (cfg.ctas == 1 && cfg.mt == 1 && !cfg.dual && (cfg.bn == 64 || cfg.bn == 128))
-                return cfg.bn == 64 ? launch_x3<KB_BYTES, 64>(cfg, p, s) : launch_x3<KB_BYTES, 128>(cfg, p, s);
+                return cfg.bn == 64 ? launch_x3<KB_BYTES, 64, 1>(cfg, p, s) : launch_x3<KB_BYTES, 128, 1>(cfg, p, s);
         }
         return fail(KXC_B200_ERR_INVALID, "tensor-core conv: no three-pass kernel for this configuration");
     }
@@ -939,7 +972,7 @@ int32_t choose_split(TcParams* p, TcConfig* cfg, const void* w, const void* w_lo
     const long long m_tiles = (long long)p->tiles_w * p->tiles_h * p->tiles_n;
     const int kb = p->taps_h * p->taps_w * p->cblocks;
     const bool wide_items = cfg->mt == 2;
-    const long long block = cfg->x3 ? (cfg->bn == 64 ? 830 : 1050)
+    const long long block = cfg->x3 ? (cfg->ctas == 2 ? 660 : (cfg->bn == 64 ? 830 : 1050))
                             : wide_items ? (cfg->dtype == kTcBF16 ? 760 : (cfg->bn == 64 ? 820 : 1100))
                                          : (cfg->bn == 64 ? 550 : (cfg->bn == 128 ? 590 : (cfg->bn == 192 ? 500 : 620)));
     const long long tail = (cfg->bn == 64 ? 0 : (cfg->bn == 128 ? 2000 : (cfg->bn == 192 ? 4000 : 8000))) + (wide_items ? 2800 : 0);
@@ -1202,16 +1235,24 @@ int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_m
 }
 
 int32_t tc_finish_x3(TcParams* p, TcConfig* cfg, const void* w_hi, const void* w_lo, int Cout, int k_elems) {
-    // The tile whose waves cost least: a stage takes ~950 cycles with 64 channels and ~1400 with 128 (see the kernel).
+    // The tile whose waves cost least. Single CTAs: by 950 cycles a stage with 64 channels and 1400 with 128; pairs of 64 channels
+    // where by what the forms measured (660, and 760 / 1030 for single ones, over ResNet-18's layers of 1 to 64 images) they are ahead. 250 launches of
+    // 150 drawn layers (operators and plans, 1 to 64 images, 32 to 512 channels): pairs took 62, 1.09 times as fast in the mean, 0.98 to 1.30 (a
+    // 64 -> 128 3x3 at 80x79, one image, before it was split in two). Fewer than 12 K blocks lose up to 10 % (the stem 73 / 78 us), 1x1 layers were 0.94 to 1.04 times as fast. Pairs of 128 channels
+    // have one accumulator buffer and were level or behind (28x28, 32 images 45 / 52).
     const long long m_tiles = (long long)p->tiles_w * p->tiles_h * p->tiles_n;
     auto waves = [&](int bn) { return (m_tiles * ((Cout + bn - 1) / bn) + kNumSMs - 1) / kNumSMs; };
-    const int bn = Cout > 64 && waves(128) * 1400 <= waves(64) * 950 ? 128 : 64;
-    cfg->bn = bn; cfg->ctas = 1; cfg->mt = 1; cfg->dual = 0; cfg->x3 = 1;
+    int bn = Cout > 64 && waves(128) * 1400 <= waves(64) * 950 ? 128 : 64;
+    const long long pair_waves = ((m_tiles + 1) / 2 * ((Cout + 63) / 64) + kNumSMs / 2 - 1) / (kNumSMs / 2);
+    const bool pair = cfg->kb_bytes == 128 && m_tiles > 1 && p->taps_h * p->taps_w > 1 && p->taps_h * p->taps_w * p->cblocks >= 12 &&
+                      pair_waves * 660 < waves(bn) * (bn == 64 ? 760 : 1030) && tc_split_capacity(2) > 0;
+    if (pair) bn = 64;
+    cfg->bn = bn; cfg->ctas = pair ? 2 : 1; cfg->mt = 1; cfg->dual = 0; cfg->x3 = 1;
     p->tiles_c = (Cout + bn - 1) / bn;
     const uint64_t ktot = (uint64_t)k_elems;
     const uint64_t bdims[2] = {ktot, (uint64_t)Cout};
     const uint64_t bstrides[1] = {ktot * 4};
-    const uint32_t bbox[2] = {(uint32_t)p->kb_elems, (uint32_t)bn};
+    const uint32_t bbox[2] = {(uint32_t)p->kb_elems, (uint32_t)(bn / cfg->ctas)};
     KXC_TRY(tc_make_tmap(&p->tmB, kTcTF32, 2, const_cast<void*>(w_hi), bdims, bstrides, bbox, cfg->kb_bytes));
     KXC_TRY(tc_make_tmap(&p->tmB2, kTcTF32, 2, const_cast<void*>(w_lo), bdims, bstrides, bbox, cfg->kb_bytes));
     return choose_split(p, cfg, w_hi, w_lo, k_elems);

@@ -98,6 +98,12 @@ CHMAJOR_PAIRS = [("tf32", (48, 9, 9, 160, False)), ("tf32", (21, 14, 14, 160, Tr
                  ("bf16", (10, 14, 15, 320, True)), ("bf16", (195, 4, 4, 320, False))]
 
 
+# Three-pass layers that pairs of the implicit-GEMM kernel take: of a plan (pair_layers), and operators (images, channels, h, w, outputs, kernel, stride, residual). An
+# odd number of pixel tiles, channels that fill no tile of 64 or leave nothing to the second CTA's half of it, several tiles to a CTA and fewer than CTAs.
+THREE_PASS_PAIRS = [(9, 39, 36, 64, True), (15, 40, 23, 64, False), (12, 15, 31, 160, True), (14, 25, 23, 96, True)]
+THREE_PASS_OPERATORS = [(2, 81, 42, 42, 70, 3, 1, True), (7, 40, 45, 40, 33, 5, 1, False), (28, 74, 18, 19, 186, 3, 2, True), (32, 44, 11, 10, 131, 5, 1, False)]
+
+
 def pair_layers(relay, case, to_constant, weights, biases):
     n, h, w, _, residual = case
     x = relay.Var("input", (n, weights[0].shape[1], h, w))

@@ -827,6 +827,18 @@ def test_conv2d_tf32x3_tiles(ops, rng, case):
     assert max_rel <= 1e-4, f"conv tf32x3 {case}: {max_abs:.3e} {max_rel:.3e}"
 
 
+@pytest.mark.parametrize("case", dispatch_cases.THREE_PASS_OPERATORS)
+def test_conv2d_three_pass_pairs(ops, rng, case):
+    n, c, h, w, o, k, s, with_res = case
+    x, wt, b = conv_inputs(rng, n, c, h, w, o, k, k)
+    oh, ow = port.conv_out_dim(h, k, s, k // 2, 1), port.conv_out_dim(w, k, s, k // 2, 1)
+    res = rng.uniform(-1, 1, (n, o, oh, ow)).astype(f32) if with_res else None
+    got = host(ops.nn_conv2d(dev(x), dev(wt), dev(b), (s, s), (k // 2, k // 2), residual=None if res is None else dev(res), relu=True, precision="tf32x3"))
+    assert ops.device_status() == 0
+    max_abs, max_rel = ref_metric(got, conv_expect(x, wt, b, res, True, s, k // 2, 1, None))
+    assert min(max_abs, max_rel) <= 1e-4, f"{case}: {max_abs:.3e} {max_rel:.3e}"
+
+
 def test_conv2d_config1_tf32x3_vs_single_pass(ops, rng):
     """BASELINE config 1 (U(-1,1) data): the three-pass form is ~1000x closer to the fp32 reference than one pass."""
     x = rng.uniform(-1, 1, (1, 64, 56, 56)).astype(f32)
