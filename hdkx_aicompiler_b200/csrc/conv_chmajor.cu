@@ -29,8 +29,8 @@
 // end where the weights are old), the others are the epilogue: warp (quad, part) takes TMEM lanes = channels [32 quad, 32 quad + 32) and
 // every second (int8: fourth) chunk of 32 columns. Two accumulators of 256 columns. Every wait is bounded.
 //
-// What bounds it: the operands' way out of shared memory (an instruction fetches 128 + N rows of 32 bytes at about 64 bytes a clock) where N
-// is large, the issuing warp where it is small (elect_one in sm100.cuh; ~100 clocks for the hand-over of a group of taps; a loop that
+// What bounds it: the instructions where N is large (142 clocks for N = 224 in a launch of seven tiles a CTA; 112 alone, with nothing else in shared
+// memory), the issuing warp where it is small (elect_one in sm100.cuh; ~100 clocks for the hand-over of a group of taps; a loop that
 // waited and committed per tap took 300 a tap), in fp32 launches of many tiles the epilogue's 4-byte accesses (~18 clocks per channel and 32
 // pixels with a residual, as in the pixel-major kernel). Device time of a call, pixel-major kernel / this one, us: tf32 72 -> 120 3x3
 // at 45x51, 9 images, with a residual 26.9 / 17.5 (135 tiles of 51x3 pixels in one wave, before 208 tiles of 51x2 in two); int8 128 -> 128 3x3
@@ -782,8 +782,8 @@ bool box_cost(const CmGeometry& g, const Grouping& t, int staging, int ctas, int
     int groups = 0;
     for (int l = 0; l < t.loads; ++l) groups += div_up((l + 1 < t.loads ? t.first[l + 1] : t.taps) - t.first[l], b->group);
     const long long items = tiles(g, BW, BH, BNI, ctas);
-    // What a tile costs: its rows at the rate the copies reach shared memory, or its instructions, which fetch 128 + n rows of 32 bytes at
-    // 64 bytes a clock, and the hand-over of a group; then its epilogue, which overlaps the next tile. (Boxes chosen so over 200 drawn layers.)
+    // What a tile costs: its rows at the rate the copies reach shared memory, or its instructions, 64 + n / 2 clocks each (a fit), and the hand-over of a
+    // group; then its epilogue, which overlaps the next tile. (Boxes chosen so over 200 drawn layers.)
     const double fill = (double)g.cblocks * ((double)t.loads * rows_px + (double)t.taps * rows_w) * 2.6;
     const double mma = (double)t.taps * ((g.cblocks - 1) * 4 + g.last_steps) * (64.0 + 0.5 * b->n);
     const double main_loop = (fill > mma ? fill : mma) + 100.0 * g.cblocks * groups;

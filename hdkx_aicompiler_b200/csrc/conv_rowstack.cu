@@ -1,17 +1,17 @@
 // 3x3 / stride-1 / pad-1 convolution for 64 -> 64 channel layers (bf16 NHWC) with the three filter ROWS stacked along
 // the MMA's N dimension, on tcgen05 + TMEM.
 //
-// A tcgen05.mma fetches its A operand (128 pixels x 32 bytes) and its B operand (N x 32 bytes) from shared memory for
-// every instruction, at roughly 64 bytes per clock, so with only 64 output channels (N = 64) an instruction spends
-// ~96 cycles fetching for 32 cycles of math and two thirds of what it fetches is the A tile. Here one instruction
-// multiplies the A tile with the weights of THREE taps at once:
+// An instruction of M = 128 takes 48 / 64 / 96 / 128 cycles at N = 64 / 128 / 192 / 256 (bf16, tf32 and int8 alike), so with only
+// 64 output channels (N = 64) a third of the tensor pipe is idle, each one has to be issued, and two thirds of what it reads from
+// shared memory is the A tile (128 pixels x 32 bytes, B: N x 32). Here one instruction multiplies the A tile with the weights of
+// THREE taps at once:
 //
 //     D_r[i, w] = sum_kw W(r, kw) . X[i, w + kw - 1]        r = 0, 1, 2 (filter row), i = input row
 //     out[oh, ow] = D_0[oh - 1, ow] + D_1[oh, ow] + D_2[oh + 1, ow]
 //
 // For a fixed kw the three D_r share the A operand X[i, w + kw - 1], so B = [W(0,kw); W(1,kw); W(2,kw)] (192 rows) and
 // the accumulator holds D_0 | D_1 | D_2 in 192 TMEM columns: 12 instructions of N = 192 per tile instead of 36 of
-// N = 64, i.e. 12 x 10 KB instead of 36 x 6 KB of operand fetch. The sum over r is taken in the epilogue, where it
+// N = 64, i.e. 12 x 96 cycles and 12 x 10 KB of operands instead of 36 x 48 and 36 x 6 KB. The sum over r is taken in the epilogue, where it
 // is a shift by one accumulator ROW: the tile's pixels are ordered column-major (TMEM lane = 16 * column + row), so
 // rows i - 1 and i + 1 of the same column are the neighbouring lanes of the same warp (two warp shuffles per value).
 //
