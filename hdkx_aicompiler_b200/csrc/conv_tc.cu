@@ -69,10 +69,10 @@ struct StageGeom {
 // L2 -> shared memory twice instead of three times and no partial sum leaves the chip. The B tile is [w_hi; w_lo] (2 BN
 // rows): ONE instruction of N = 2 BN multiplies a_hi with both and fills the accumulators hi*hi | hi*lo side by side, a
 // second of N = BN adds a_lo * w_hi to the latter. The two sums meet in one rounded fp32 add in the epilogue. A stage of four K steps
-// is 448 cycles of the tensor pipe with 64 channels (64 + 48 a step) and 768 with 128, but takes 650 to 850 and 1030: its 48 or 64 KB
-// arrive at ~60 bytes a cycle.
-// Pairs (64 channels): 40 KB a stage and CTA, whose half of the B tile is [w_hi; w_lo] of 32 channels. The wide instruction then
-// gives hi*hi | hi*lo of either half, so lo*hi has columns of its own and the epilogue adds three sums. 630 to 790 cycles a stage: ResNet-18's layers, us,
+// is 448 cycles of the tensor pipe with 64 channels (64 + 48 a step) and 768 with 128, but takes 850 and 1150: what crosses shared
+// memory, 56 or 80 KB of operands that the instructions read and 48 or 64 KB of copies, does so at 125 to 128 bytes a cycle.
+// Pairs (64 channels): 44 and 40 KB a stage and CTA, whose half of the B tile is [w_hi; w_lo] of 32 channels. The wide instruction then
+// gives hi*hi | hi*lo of either half, so lo*hi has columns of its own and the epilogue adds three sums. 680 to 790 cycles a stage: ResNet-18's layers, us,
 // 32 images 28x28 45.3 -> 40.0 (128 channels a tile before), 56x56 50.5 -> 47.5, 64 images 14x14 81 -> 73; whole networks 32: 873 -> 841, 48: 1260 -> 1204.
 template <MmaKind kKind, int KB_BYTES, int BN, int kOutMode, int kCtas, bool kDual = false, int kMT = 1, bool kX3 = false>
 __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_constant__ TcParams p) {
