@@ -80,16 +80,6 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_direct_kernel(const __g
     const uint32_t strip_smem = w_smem + kWeightBytes;
 
     const int KH = p.taps_h;
-    if constexpr (kKind == MmaKind::I8) {
-        if (threadIdx.x == 0) q_fast = 1;
-        __syncthreads();
-        // |accumulator| <= 128 * 128 * (KH rows * 8 columns * 8 channels); the constants are call arguments
-        if (threadIdx.x >= 64 && threadIdx.x < 64 + kBN) {
-            const int c = threadIdx.x - 64;
-            if (!requant_prepare(__ldg(p.bias_i32 + c), __ldg(p.multiplier + c), __ldg(p.shift + c), 128ll * 128 * 64 * KH, &q_tab[c]))
-                q_fast = 0;
-        }
-    }
     const int row_bytes = p.aux_row_bytes;          // Wp * 8
     const int Hp = p.aux_hp;
     const int strips_per_image = (p.OH + kStripRows - 1) / kStripRows;
@@ -98,6 +88,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_direct_kernel(const __g
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
+        if constexpr (kKind == MmaKind::I8) q_fast = 1;
         mbar_init(smem_u32(&bar_w), 1);
         for (int s = 0; s < kStages; ++s) {
             mbar_init(smem_u32(&bar_full[s]), 1);
@@ -130,8 +121,9 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_direct_kernel(const __g
     if (warp == 0) {
         if (lane == 0) {
             const uint32_t wbytes = (uint32_t)(KH * 4 * kBN * 16);
+            if (!p.weights_ready) pdl_wait();  // the operator's, which the kernel before this one packs
             mbar_arrive_expect_tx(smem_u32(&bar_w), wbytes);
-            bulk_copy_g2s(w_smem, p.aux_w, wbytes, smem_u32(&bar_w));  // constants: no need to wait for the previous kernel
+            bulk_copy_g2s(w_smem, p.aux_w, wbytes, smem_u32(&bar_w));
             pdl_wait();
             int stage = 0;
             uint32_t phase = 0;
@@ -196,6 +188,13 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_direct_kernel(const __g
         const int c0 = half * 32;
         const bool col_ok = ow < p.OW;
         pdl_wait();
+        if constexpr (kKind == MmaKind::I8) {  // (the quantization constants are the caller's: the kernel before may have written them)
+            const int c = (int)threadIdx.x - 64;
+            // |accumulator| <= 128 * 128 * (KH rows * 8 columns * 8 channels)
+            if (c < kBN && !requant_prepare(__ldg(p.bias_i32 + c), __ldg(p.multiplier + c), __ldg(p.shift + c), 128ll * 128 * 64 * KH, &q_tab[c]))
+                q_fast = 0;
+            named_barrier(1, kThreads - 64);
+        }
         int acc = 0;
         uint32_t acc_phase = 0;
         bool ok = true;

@@ -1043,3 +1043,21 @@ def test_queued_operators_wait_for_one_another(ops, rng, n, c, hw, captured):
     torch.cuda.synchronize()
     for g, e in zip(got, expected):
         assert torch.isfinite(e).all() and torch.equal(g.cpu(), e)
+
+
+@pytest.mark.parametrize("nhwc", [False, True])
+def test_first_layers_wait_for_their_weights(ops, rng, nhwc):
+    """The int8 first layer packs its weights on each call: calls with other weights, queued one behind the other, give what each gives by itself."""
+    x = dev(rng.integers(-128, 128, (2, 30, 26, 3) if nhwc else (2, 3, 30, 26), dtype=np.int8))
+    calls = []
+    for _ in range(12):
+        w = dev(rng.integers(-127, 128, (64, 7, 7, 3) if nhwc else (64, 3, 7, 7), dtype=np.int8))
+        b, m = dev(rng.integers(-1000, 1000, 64, dtype=np.int32)), dev(rng.integers(1 << 30, (1 << 31) - 1, 64, dtype=np.int32))
+        calls.append(lambda w=w, b=b, m=m: ops.nn_conv2d_s8(x, w, b, m, torch.full_like(b, 9), (2, 2), (3, 3), nhwc=nhwc))
+    expected = []
+    for call in calls:
+        expected.append(call())
+        torch.cuda.synchronize()
+    for got, e in zip([call() for call in calls], expected):
+        assert torch.equal(got, e)
+    assert ops.device_status() == 0 and len({bytes(e.cpu().numpy()) for e in expected}) == len(calls)

@@ -2,6 +2,8 @@
 word it reports into, the once-per-device kernel set-up, and the threading contract of the per-operator entry
 points (the reference calls the same kernel entry from several host threads: src/runtime/kernel_runner.cc:17-30)."""
 import ctypes
+import os
+import re
 import threading
 
 import numpy as np
@@ -16,6 +18,37 @@ def test_per_device_once_bookkeeping():
     from hdkx_aicompiler_b200 import _lib
     lib = _lib.load()
     assert lib.kxc_b200_selftest_per_device_once() == 0, _lib.last_error()
+
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "hdkx_aicompiler_b200", "csrc")
+
+
+def reads_before_the_wait(file, kernel):
+    """The reads of global memory (__ldg, copies of weights) in a kernel's text that no griddepcontrol.wait of their block, or of one around it,
+    precedes. Copies of weights may also follow a wait on condition of weights_ready."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, file)).read())
+    text = text[re.search(r"__global__[^;{]*?\b" + kernel + r"\(", text).start():]
+    waited, found = [], []
+    for m in re.finditer(r"\{|\}|if \(!p\.weights_ready\) pdl_wait\(\)|pdl_wait\(\)|__ldg\(|&p\.tm[BW]2?, |p\.aux_w, ", text):
+        token = m.group()
+        if token == "{":
+            waited.append(set(waited[-1]) if waited else set())
+        elif token == "}":
+            waited.pop()
+            if not waited:
+                return found
+        elif token == "pdl_wait()":
+            waited[-1] |= {"all", "weights"}
+        elif "pdl_wait" in token:
+            waited[-1].add("weights")
+        elif ("all" if token == "__ldg(" else "weights") not in waited[-1]:
+            found.append(text[m.start():m.start() + 60])
+
+
+# Kernels of operators, whose weights and constants the kernel before may have written
+@pytest.mark.parametrize("file,kernel", [("conv_stem.cu", "conv_stem_direct_kernel")])
+def test_operands_are_read_after_the_wait(file, kernel):
+    assert reads_before_the_wait(file, kernel) == []
 
 
 @pytest.mark.gpu
