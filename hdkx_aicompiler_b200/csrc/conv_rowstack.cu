@@ -349,15 +349,9 @@ __global__ void __launch_bounds__(kThreads8, 1) conv3x3_rowstack_s8_kernel(const
     const uint32_t w_smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t halo_smem = w_smem + kWeightBytes8;
 
-    if (threadIdx.x == 0) q_fast = 1;
-    __syncthreads();
-    if (threadIdx.x >= 64 && threadIdx.x < 64 + kO) {  // the quantization constants are call arguments, not a producer's output
-        const int c = threadIdx.x - 64;
-        // |accumulator| <= 128 * 128 * (9 taps * 64 channels)
-        if (!requant_prepare(__ldg(p.bias_i32 + c), __ldg(p.multiplier + c), __ldg(p.shift + c), 128ll * 128 * 9 * kC, &q_tab[c])) q_fast = 0;
-    }
     if (threadIdx.x == 0) {
         abort_flag = 0;
+        q_fast = 1;
         mbar_init(smem_u32(&bar_w), 1);
         for (int s = 0; s < kStages8; ++s) {
             mbar_init(smem_u32(&bar_full[s]), 1);
@@ -388,14 +382,13 @@ __global__ void __launch_bounds__(kThreads8, 1) conv3x3_rowstack_s8_kernel(const
             tma_prefetch_desc(&p.tmA[0]);
             tma_prefetch_desc(&p.tmB);
         }
-        if (!p.weights_ready) pdl_wait();  // weights that the previous kernel packs
+        pdl_wait();  // pixels and weights are the caller's: the kernel before may have written either
         if (lead) {
             mbar_arrive_expect_tx(smem_u32(&bar_w), kWeightBytes8);
             for (int kw = 0; kw < 3; ++kw)
                 for (int r = 0; r < 3; ++r)
                     tma_load_2d(w_smem + kw * kTapBytes8 + r * (kO * kPx8), &p.tmB, smem_u32(&bar_w), (r * 3 + kw) * kC, 0);
         }
-        pdl_wait();
         int stage = 0;
         uint32_t phase = 0;
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
@@ -454,8 +447,14 @@ __global__ void __launch_bounds__(kThreads8, 1) conv3x3_rowstack_s8_kernel(const
         const bool in_box = (h_l >= 1) && (h_l <= kOutRows);
         int8_t* out = static_cast<int8_t*>(p.out);
         const int32_t lo = p.relu ? 0 : INT32_MIN;
-        const bool fast = q_fast != 0;
         pdl_wait();
+        const int channel = (int)threadIdx.x - 64;
+        // |accumulator| <= 128 * 128 * (9 taps * 64 channels)
+        if (channel < kO &&
+            !requant_prepare(__ldg(p.bias_i32 + channel), __ldg(p.multiplier + channel), __ldg(p.shift + channel), 128ll * 128 * 9 * kC, &q_tab[channel]))
+            q_fast = 0;
+        named_barrier(1, kThreads8 - 64);
+        const bool fast = q_fast != 0;
         uint32_t acc_phase = 0;
         // this set's tiles: blockIdx.x + (2 i + set) gridDim.x; the tile coordinates advance by a fixed step with carries
         const int step = 2 * (int)gridDim.x;

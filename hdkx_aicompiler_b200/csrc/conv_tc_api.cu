@@ -195,7 +195,6 @@ int32_t conv2d_s8_dispatch(const int8_t* data, const int8_t* weight, const int32
         }();
         if (rowstack_enabled && rowstack3x3_s8_applicable(d.C, d.O, d.KH, d.KW, d.SH, d.PH, d.PW, d.DH, d.DW)) {
             KXC_TRY(rowstack3x3_s8_setup(&p, data, weight, d.N, d.H, d.W));
-            p.weights_ready = 1;
             p.bias_i32 = bias;
             p.multiplier = multiplier;
             p.shift = shift;

@@ -1061,3 +1061,20 @@ def test_first_layers_wait_for_their_weights(ops, rng, nhwc):
     for got, e in zip([call() for call in calls], expected):
         assert torch.equal(got, e)
     assert ops.device_status() == 0 and len({bytes(e.cpu().numpy()) for e in expected}) == len(calls)
+
+
+def test_filters_that_a_kernel_in_flight_writes(ops, rng):
+    """The filters of a resident int8 layer are the result of a long convolution on a few SMs, which lets the kernel behind it start when it starts itself."""
+    x = dev(rng.integers(-128, 128, (3, 28, 28, 64), dtype=np.int8))
+    image, filters = (dev(rng.integers(-127, 128, s, dtype=np.int8)) for s in ((64, 3, 3, 512), (64, 7, 7, 512)))
+    zero, m = torch.zeros(64, dtype=torch.int32, device="cuda"), torch.full((64,), 1 << 30, dtype=torch.int32, device="cuda")
+    biases = [torch.full_like(zero, 50000 * i) for i in range(8)]
+    expected, got = [], []
+    for out, wait in ((expected, torch.cuda.synchronize), (got, lambda: None)):
+        for b in biases:
+            w = ops.nn_conv2d_s8(image, filters, b, m, torch.full_like(zero, 13), (1, 1), (3, 3), nhwc=True)
+            wait()
+            out.append(ops.nn_conv2d_s8(x, w, zero, m, torch.full_like(zero, 13), (1, 1), (1, 1), nhwc=True))
+            wait()
+    assert ops.device_status() == 0 and len({bytes(e.cpu().numpy()) for e in expected}) == len(biases)
+    assert all(torch.equal(g, e) for g, e in zip(got, expected))

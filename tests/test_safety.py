@@ -46,7 +46,7 @@ def reads_before_the_wait(file, kernel):
 
 
 # Kernels of operators, whose weights and constants the kernel before may have written
-@pytest.mark.parametrize("file,kernel", [("conv_stem.cu", "conv_stem_direct_kernel")])
+@pytest.mark.parametrize("file,kernel", [("conv_stem.cu", "conv_stem_direct_kernel"), ("conv_rowstack.cu", "conv3x3_rowstack_s8_kernel")])
 def test_operands_are_read_after_the_wait(file, kernel):
     assert reads_before_the_wait(file, kernel) == []
 
