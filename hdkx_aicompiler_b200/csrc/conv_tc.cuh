@@ -73,8 +73,8 @@ struct alignas(64) TcParams {
     long long out_lo_offset;
     int out_pitch;               // kOutNHWC_S8: channels per stored pixel (0: Cout), a multiple of 16
     int split;                   // 2..kMaxSplit: the reduction is split over clusters of that many CTAs (conv_splitk.cu); 0: it is not
-    // the packed weights were written long before this launch: they may be read ahead of its predecessor's end (set before the
-    // set-up functions, which weigh it)
+    // The weights are a plan's: whatever packed them had ended before the launch ahead of this one began, so they may be read ahead of that
+    // one's end (set before the set-up functions, which weigh it). Everything a caller passes is read after the wait.
     int weights_ready;
 };
 

@@ -942,7 +942,7 @@ static int32_t finalize_core(kxc_b200_plan* pl) {
     }
     // ---- tensor maps and launch parameters ----
     for (auto& st : pl->steps) {
-        st.params.weights_ready = 1;  // packed by ordinary launches ahead of the run's first kernel
+        st.params.weights_ready = 1;  // (plan_run_core lets no step begin before they are packed)
         if (st.kind == SKind::Conv) {
             PackedWeight& pw = pl->weights[st.weight];
             Value* ov = pl->find(st.out);
@@ -1105,6 +1105,8 @@ static int64_t split_parts(kxc_b200_plan* pl, int id) {
     return pl->x3 && v->split ? (int64_t)v->elems : 0;
 }
 
+__global__ void weights_packed_kernel() {}
+
 static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream, cudaEvent_t* events) {
     if (!pl || !pl->finalized) return fail(KXC_B200_ERR_INVALID, "plan_run: plan is not finalized");
     if (pl->precision == KXC_B200_PREC_FP32) return run_exact(pl, packed_args, stream, events);
@@ -1122,9 +1124,11 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
     auto arg_of = [&](int id) -> void* { return packed_args[pl->find(id)->arg_index]; };
 
     // (re)pack constants whose source pointer changed
+    bool packed = false;
     for (auto& w : pl->weights) {
         const void* src = arg_of(w.const_id);
         if (src == w.source) continue;
+        packed = true;
         switch (w.mode) {
             case 0: KXC_TRY(pack_weights_ohwi(WeightPack{src, w.ptr, w.ptr_lo, w.O, w.C, w.KH * w.KW, w.cpad}, dt, s)); break;
             case 1: KXC_TRY(stem_pack_weights(static_cast<const float*>(src), w.ptr, dt, w.O, w.C, w.KH, w.KW, s)); break;
@@ -1142,6 +1146,12 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
             }
         }
         w.source = src;
+    }
+    // The steps read packed weights ahead of their waits. A step behind the last packing kernel could start with that one's blocks gone and what they
+    // wrote not yet visible; an empty kernel launched in order ends after all of it.
+    if (packed) {
+        weights_packed_kernel<<<1, 32, 0, s>>>();
+        KXC_TRY(check_launch("weights_packed"));
     }
 
     // Tensor-core launches alternate the direction in which they walk their work items (KXC_B200_TILE_ORDER=0: all

@@ -29,11 +29,11 @@ void* address(size_t bytes) {
     next_address += (bytes + 4095) & ~(size_t)4095;
     return reinterpret_cast<void*>(p);
 }
-cudaError_t launch(const void* func, dim3 g, dim3 b, size_t smem, unsigned cluster) {
+cudaError_t launch(const void* func, dim3 g, dim3 b, size_t smem, unsigned cluster, int ahead = 0) {
     if (g.x == 0 || g.y == 0 || g.z == 0 || g.x > 0x7fffffffu || g.y > 65535u || g.z > 65535u || b.x * b.y * b.z > 1024u)
         return result(cudaErrorInvalidConfiguration);
     char line[512];
-    snprintf(line, sizeof(line), "%s grid %u %u %u block %u smem %zu cluster %u\n", kernels[func].c_str(), g.x, g.y, g.z, b.x * b.y * b.z, smem, cluster);
+    snprintf(line, sizeof(line), "%s grid %u %u %u block %u smem %zu ahead %d cluster %u\n", kernels[func].c_str(), g.x, g.y, g.z, b.x * b.y * b.z, smem, ahead, cluster);
     log_text += line;
     return cudaSuccess;
 }
@@ -74,9 +74,12 @@ cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* smem, void* s) 
 cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3 b, void**, size_t smem, cudaStream_t) { return launch(f, g, b, smem, 1); }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
     unsigned cluster = 1;
-    for (unsigned i = 0; i < c->numAttrs; ++i)
+    int ahead = 0;  // of the end of the kernel before
+    for (unsigned i = 0; i < c->numAttrs; ++i) {
         if (c->attrs[i].id == cudaLaunchAttributeClusterDimension) cluster = c->attrs[i].val.clusterDim.x;
-    return launch(f, c->gridDim, c->blockDim, c->dynamicSmemBytes, cluster);
+        if (c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization) ahead = c->attrs[i].val.programmaticStreamSerializationAllowed;
+    }
+    return launch(f, c->gridDim, c->blockDim, c->dynamicSmemBytes, cluster, ahead);
 }
 cudaError_t cudaGetLastError(void) { const cudaError_t e = last; last = cudaSuccess; return e; }
 const char* cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAllocation ? "out of memory" : e == cudaErrorInvalidConfiguration ? "invalid configuration argument" : "error"; }
