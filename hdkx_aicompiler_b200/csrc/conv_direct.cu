@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_direct_kernel(const __gri
             // resident weights: nine 64x64 tap blocks
             mbar_arrive_expect_tx(smem_u32(&bar_w), kWeightBytes);
             for (int t = 0; t < kTaps; ++t) tma_load_2d(w_smem + t * (kBN * 128), &p.tmB, smem_u32(&bar_w), t * kC, 0);
-            pdl_wait();  // the weights are constants; the activations come from the previous kernel
+            pdl_wait();  // the weights are the plan's (TcParams::weights_ready); the activations come from the previous kernel
             int stage = 0;
             uint32_t phase = 0;
             for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {

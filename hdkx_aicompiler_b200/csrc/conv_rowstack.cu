@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack_kernel(const __g
                 for (int r = 0; r < 3; ++r)
                     tma_load_2d(w_smem + kw * kTapBytes + r * (kO * 128), &p.tmB, smem_u32(&bar_w), (r * 3 + kw) * kC, 0);
         }
-        pdl_wait();  // the weights are constants; the activations come from the previous kernel
+        pdl_wait();  // the weights are the plan's (TcParams::weights_ready); the activations come from the previous kernel
         int stage = 0, rb = 0;
         uint32_t phase = 0, rphase = 0;
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {

@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
                         tma_load_2d_pair(w_smem + (uint32_t)((kw * 2 + pl) * kWBlockBytes + 32 * j * 128), &p.tmB, wbar,
                                          (r * 3 + kw) * kC + pl * kPlaneC, half * kOH + co0);
                     }
-            pdl_wait();  // the weights are constants; the activations come from the previous kernel
+            pdl_wait();  // the weights are the plan's (TcParams::weights_ready); the activations come from the previous kernel
             int stage = 0, rb = 0;
             uint32_t phase = 0, rphase = 0;
             for (int tp = first_tp; tp < tile_pairs; tp += tp_step) {
@@ -247,10 +247,10 @@ __global__ void __launch_bounds__(kThreads, 1) conv3x3_rowstack128_kernel(const 
         const uint32_t sw = box_row & 7u;
         const uint32_t acc_empty0 = map_to_cta(smem_u32(&bar_acc_empty[0]), 0);
         const uint32_t acc_empty1 = map_to_cta(smem_u32(&bar_acc_empty[1]), 0);
+        pdl_wait();
         float bias[kCh];
 #pragma unroll
         for (int j = 0; j < kCh; ++j) bias[j] = p.bias != nullptr ? __ldg(p.bias + half * kOH + c0 + j) : 0.0f;
-        pdl_wait();
         int acc = 0, rb = group, ob = group;
         uint32_t acc_phase = 0, rphase = 0;
         for (int tp = first_tp; tp < tile_pairs; tp += tp_step) {

@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_kernel(const __gri
         if (lane == 0) {
             const uint32_t wbytes = (uint32_t)(KH * 4 * kBN * 16);
             mbar_arrive_expect_tx(smem_u32(&bar_w), wbytes);
-            bulk_copy_g2s(w_smem, p.aux_w, wbytes, smem_u32(&bar_w));  // constants: no need to wait for the previous kernel
+            bulk_copy_g2s(w_smem, p.aux_w, wbytes, smem_u32(&bar_w));  // the plan's (TcParams::weights_ready)
             pdl_wait();
             int stage = 0;
             uint32_t phase = 0;
@@ -433,10 +433,10 @@ __global__ void __launch_bounds__(kThreads, 1) conv_stem_pool_kernel(const __gri
         const int POH = p.OH / 2, POW = p.OW / 2;
         __nv_bfloat16* pooled = static_cast<__nv_bfloat16*>(p.out);
         const bool centre = (lane & 1) == 0 && ow < p.OW;  // even conv columns are the pooling windows' centres
+        pdl_wait();
         float bias[32];
 #pragma unroll
         for (int e = 0; e < 32; ++e) bias[e] = p.bias != nullptr ? __ldg(p.bias + c0 + e) : 0.0f;
-        pdl_wait();
         int acc = 0;
         uint32_t acc_phase = 0;
         uint32_t row_ctr = 0;  // conv rows handled so far (parity picks the exchange slot)

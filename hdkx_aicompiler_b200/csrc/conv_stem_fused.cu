@@ -250,10 +250,6 @@ __global__ void __launch_bounds__(StemGeom<kF32, kPooledRows>::kThreads, 1) conv
         const uint32_t addr = strip_smem + i * 16;
         asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0u) : "memory");
     }
-    if (threadIdx.x < kBN) {
-        const float b = p.bias != nullptr ? __ldg(p.bias + threadIdx.x) : 0.0f;
-        asm volatile("st.shared.f32 [%0], %1;" ::"r"(bias_smem + threadIdx.x * 4u), "f"(b) : "memory");
-    }
     fence_proxy_async_shared();
     tc_fence_before_sync();
     __syncthreads();
@@ -286,7 +282,7 @@ __global__ void __launch_bounds__(StemGeom<kF32, kPooledRows>::kThreads, 1) conv
         // A slot's rows of a plane lie one after the other in the image: one bulk copy per channel.
         if (lane == 0) {
             mbar_arrive_expect_tx(smem_u32(&bar_w), (uint32_t)kWeightBytes);
-            bulk_copy_g2s(w_smem, p.aux_w, (uint32_t)kWeightBytes, smem_u32(&bar_w));
+            bulk_copy_g2s(w_smem, p.aux_w, (uint32_t)kWeightBytes, smem_u32(&bar_w));  // the plan's (TcParams::weights_ready)
             pdl_wait();
             int slot = 0;
             uint32_t phase = 0;
@@ -461,6 +457,11 @@ __global__ void __launch_bounds__(StemGeom<kF32, kPooledRows>::kThreads, 1) conv
         const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
         const bool odd = (lane & 1) != 0;
         pdl_wait();
+        if (ow < kPartCols) {  // the bias of this part's channels, for its four warps
+            const float b = p.bias != nullptr ? __ldg(p.bias + c0 + ow) : 0.0f;
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(bias_smem + (uint32_t)(c0 + ow) * 4u), "f"(b) : "memory");
+        }
+        named_barrier(1 + part, 128);
         uint32_t blk = 0;
         uint32_t fin = 0;  // pooled rows finished so far (parity picks the exchange slot)
         bool bad = false;  // a wait ran out: carried to the next 128-thread barrier, where the four warps of this part leave together
