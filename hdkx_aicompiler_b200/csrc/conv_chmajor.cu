@@ -956,7 +956,7 @@ const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcO
             }
             e.use = rc == KXC_B200_OK && cfg.clocks >= ahead * e.plan.c.cost && !stays;
             CmPlan pair;
-            if (rc == KXC_B200_OK && d.O > kM && e.plan.g.cblocks >= 4 && d.KH * d.KW > 1 && d.KH * d.KW <= 9 && d.SH == 1 && p.split <= 2 && tc_split_capacity(2) > 0 &&
+            if (rc == KXC_B200_OK && d.O > kM && e.plan.g.cblocks >= 4 && d.KH * d.KW > 1 && d.KH * d.KW <= 9 && d.SH == 1 && p.split <= 2 && tc_cta_pairs() && tc_split_capacity(2) > 0 &&
                 choose(&pair, dtype, d, true, 2)) {
                 const double other = e.use ? e.plan.c.clocks : tc_modelled_clocks(p, cfg, residual);
                 if (pair.c.clocks < 0.945 * other) {

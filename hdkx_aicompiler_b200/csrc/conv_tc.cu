@@ -1013,6 +1013,14 @@ int32_t choose_split(TcParams* p, TcConfig* cfg, const void* w, const void* w_lo
 }
 }  // namespace
 
+bool tc_cta_pairs() {
+    static const bool on = [] {
+        const char* e = getenv("KXC_B200_CTA_PAIR");
+        return !(e != nullptr && e[0] == '0');
+    }();
+    return on;
+}
+
 // Per form: what a launch costs besides, a K block, the epilogue of a tile (it overlaps the next tile's main loop) NHWC and what a residual adds to it,
 // and both into the reference's layout. Fits over the launches of 381 drawn layers (plans' layers with and without a residual, graph outputs,
 // operators with their conversion apart; 1 to 512 images), 2 to 9 % rms each. Choosing between this and the channel-major kernel's clocks (box_cost
@@ -1145,16 +1153,12 @@ int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_m
         }
     }
     // CTA pairs (tcgen05 cta_group::2): each CTA fetches half of the B tile, which relieves the L2 -> shared-memory
-    // fill rate that bounds the wide tiles. KXC_B200_CTA_PAIR=0 switches them off (for measurements).
-    static const bool pair_enabled = [] {
-        const char* e = getenv("KXC_B200_CTA_PAIR");
-        return !(e != nullptr && e[0] == '0');
-    }();
+    // fill rate that bounds the wide tiles.
     const long long m_tiles = (long long)p->tiles_w * p->tiles_h * p->tiles_n;
     // Measured: pairs gain 5-7 % with the 256-wide tile and lose 3-10 % with the 128-wide one (the pair's MMA is
     // no faster there and the handshakes cross SMs), so only the 256-wide tile uses them. "2" forces them for 128 too.
     static const bool pair_all = [] { const char* e = getenv("KXC_B200_CTA_PAIR"); return e != nullptr && e[0] == '2'; }();
-    int ctas = (pair_enabled && bn >= (pair_all ? 128 : 256) && kb_bytes == 128 && m_tiles >= 2) ? 2 : 1;
+    int ctas = (tc_cta_pairs() && bn >= (pair_all ? 128 : 256) && kb_bytes == 128 && m_tiles >= 2) ? 2 : 1;
     // Launches with few tiles (small per-GPU batches in the deep layers): the 256-wide tile leaves SMs idle, e.g. 98 tiles
     // (49-50 pairs) on 148 SMs. 512 channels in 192-wide tiles on 49 pixel tiles are 147 CTAs, one wave, and an
     // M = 128, K = 16 instruction takes ~99 cycles at N = 192 against ~131 at N = 256 (measured). The narrower tile is
@@ -1244,7 +1248,7 @@ int32_t tc_finish_x3(TcParams* p, TcConfig* cfg, const void* w_hi, const void* w
     int bn = Cout > 64 && waves(128) * 1400 <= waves(64) * 950 ? 128 : 64;
     const long long pair_waves = ((m_tiles + 1) / 2 * ((Cout + 63) / 64) + kNumSMs / 2 - 1) / (kNumSMs / 2);
     const bool pair = cfg->kb_bytes == 128 && m_tiles > 1 && p->taps_h * p->taps_w > 1 && p->taps_h * p->taps_w * p->cblocks >= 12 &&
-                      pair_waves * 660 < waves(bn) * (bn == 64 ? 760 : 1030) && tc_split_capacity(2) > 0;
+                      pair_waves * 660 < waves(bn) * (bn == 64 ? 760 : 1030) && tc_cta_pairs() && tc_split_capacity(2) > 0;
     if (pair) bn = 64;
     cfg->bn = bn; cfg->ctas = pair ? 2 : 1; cfg->mt = 1; cfg->dual = 0; cfg->x3 = 1;
     p->tiles_c = (Cout + bn - 1) / bn;

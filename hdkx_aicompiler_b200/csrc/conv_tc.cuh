@@ -107,6 +107,9 @@ int32_t tc_launch_split(const TcConfig& cfg, const TcParams& p, cudaStream_t str
 // Clusters of `split` CTAs that the current device holds at once (whole GPCs' worth: fewer than 148 / split).
 int tc_split_capacity(int split);
 
+// Whether launches may take CTA pairs: KXC_B200_CTA_PAIR=0 switches those of the implicit-GEMM and channel-major kernels off (for measurements).
+bool tc_cta_pairs();
+
 // Modelled time of a set-up launch of bf16 or tf32 operands, in clocks of 1.85 GHz, for the comparison with the channel-major kernel's CTA pairs.
 double tc_modelled_clocks(const TcParams& p, const TcConfig& cfg, bool residual);
 
