@@ -895,9 +895,11 @@ bool choose(CmPlan* plan, TcDType dtype, const ConvDims& d, bool pixels, int cta
 // CTA pairs: 3x3 layers of stride 1 and at least four channel blocks, where their fitted clocks (box_cost) are 5.5 % below the other form's
 // (tc_modelled_clocks, or those of single CTAs), not where the reduction is split over three and more. Of 200 drawn layers and those of ResNet-18 at 1 to 512
 // images 73 took them, 1.12 times as fast in the mean (0.86 to 1.37; four lost more than 3 %): 512 -> 512 at 7x7, 64 images, bf16 23.2 / 16.9 us (split
-// in two), tf32 35.3 / 28.1; 256 -> 256 at 14x14, 128 images, 28.7 / 25.7 and 52.6 / 45.0. With fewer channel blocks they lost up to 20 % (32 -> 256 at
+// in two), tf32 35.3 / 28.1; 256 -> 256 at 14x14, 128 images, 28.7 / 25.7 and 52.6 / 45.0. 110 others that took them: 1.12 (0.93 to 1.37, two lost more than
+// 3 %), 48 of other paddings and dilations 1.08 (0.93 to 1.33, six). With fewer channel blocks they lost up to 20 % (32 -> 256 at
 // 17x15, 97 images, tf32 15.8 / 19.9), at stride 2 up to 35 % (256 -> 512 at 14x14, 256 images, tf32 52.7 / 71.2), with 5x5 filters up to 40 %; into planes one
-// of 71 layers gained, int8 planes lost 13 % in the mean.
+// of 71 layers gained, int8 planes lost 13 % in the mean. Filters of two to nine taps that are not 3x3, which the fit has none of: 80 that it would take
+// over were 0.97 times as fast in the mean (288 -> 288 1x5 at 15x17, 41 images, tf32 27.4 / 42.7; 192 -> 192 5x1 at 17x15, 118 images, 28.9 / 42.4).
 // ResNet-18 tf32 32 images 476.8 / 419.6 us, 64: 739 / 661, 256: 2156 / 2028; bf16 32: 265.7 / 254.2, 128: 552 / 545. bf16 layers of stride 2
 // keep the pixel-major kernel: with a 1x1 layer beside them they are one launch of it (two outputs), and alone they give the same bits as there.
 const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcOutMode out_mode, bool residual) {
@@ -956,7 +958,7 @@ const CmPlan* cm_wanted(TcDType dtype, const ConvDims& d, int weights_ready, TcO
             }
             e.use = rc == KXC_B200_OK && cfg.clocks >= ahead * e.plan.c.cost && !stays;
             CmPlan pair;
-            if (rc == KXC_B200_OK && d.O > kM && e.plan.g.cblocks >= 4 && d.KH * d.KW > 1 && d.KH * d.KW <= 9 && d.SH == 1 && p.split <= 2 && tc_cta_pairs() && tc_split_capacity(2) > 0 &&
+            if (rc == KXC_B200_OK && d.O > kM && e.plan.g.cblocks >= 4 && d.KH == 3 && d.KW == 3 && d.SH == 1 && p.split <= 2 && tc_cta_pairs() && tc_split_capacity(2) > 0 &&
                 choose(&pair, dtype, d, true, 2)) {
                 const double other = e.use ? e.plan.c.clocks : tc_modelled_clocks(p, cfg, residual);
                 if (pair.c.clocks < 0.945 * other) {

@@ -96,6 +96,13 @@ CHMAJOR_LAYERS = [
 # padding, one and two images to a box, an odd number of boxes, and channels that leave the second CTA a part, or nothing, of a tile.
 CHMAJOR_PAIRS = [("tf32", (48, 9, 9, 160, False)), ("tf32", (21, 14, 14, 160, True)), ("tf32", (47, 9, 10, 160, True)), ("tf32", (61, 7, 7, 288, True)),
                  ("bf16", (10, 14, 15, 320, True)), ("bf16", (195, 4, 4, 320, False))]
+# ... of other paddings and dilations (the last two entries): no padding, in one direction or both, more than the filter's reach, taps two apart; planes in part and
+# whole, two and three images to a box
+CHMAJOR_PAIR_PADDINGS = [
+    ("tf32", (41, 12, 15, 160, False, (0, 0), (1, 1))), ("tf32", (97, 4, 8, 160, False, (2, 2), (1, 1))), ("tf32", (13, 17, 13, 160, False, (3, 1), (1, 1))),
+    ("tf32", (97, 6, 6, 160, False, (3, 1), (1, 1))), ("tf32", (97, 4, 15, 160, False, (2, 2), (2, 2))), ("tf32", (41, 12, 15, 160, False, (1, 1), (2, 2))),
+    ("tf32", (25, 13, 16, 160, False, (2, 1), (2, 1))), ("tf32", (211, 2, 5, 160, False, (2, 2), (1, 1))), ("bf16", (151, 6, 5, 320, False, (0, 1), (1, 1))),
+    ("bf16", (151, 4, 7, 320, False, (1, 0), (1, 1))), ("bf16", (211, 4, 4, 320, False, (2, 2), (2, 2))), ("bf16", (211, 6, 6, 320, False, (0, 0), (1, 1)))]
 
 
 # Three-pass layers that pairs of the implicit-GEMM kernel take: of a plan (pair_layers), and operators (images, channels, h, w, outputs, kernel, stride, residual). An
@@ -105,12 +112,13 @@ THREE_PASS_OPERATORS = [(2, 81, 42, 42, 70, 3, 1, True), (7, 40, 45, 40, 33, 5, 
 
 
 def pair_layers(relay, case, to_constant, weights, biases):
-    n, h, w, _, residual = case
+    n, h, w, _, residual = case[:5]
+    padding, dilation = case[5:] or ((1, 1), (1, 1))
     x = relay.Var("input", (n, weights[0].shape[1], h, w))
-    conv = lambda d, i, k: relay.Call("nn_conv2d", [d, relay.Constant(to_constant(weights[i])), relay.Constant(to_constant(biases[i]))],
-                                      relay.Conv2DAttrs((1, 1), (k // 2,) * 4, (1, 1), 1))
-    y = relay.Call("nn_relu", [conv(x, 0, 1)])
-    z = conv(y, 1, 3)
+    conv = lambda d, i, p, dil: relay.Call("nn_conv2d", [d, relay.Constant(to_constant(weights[i])), relay.Constant(to_constant(biases[i]))],
+                                           relay.Conv2DAttrs((1, 1), p * 2, dil, 1))
+    y = relay.Call("nn_relu", [conv(x, 0, (0, 0), (1, 1))])
+    z = conv(y, 1, padding, dilation)
     z = relay.Call("nn_relu", [relay.Call("add", [z, y]) if residual else z])
     return relay.Function([x], relay.Call("nn_max_pool2d", [z], relay.MaxPool2DAttrs((1, 1), (1, 1, 1, 1), (1, 1), (3, 3), "NCHW", False)))
 
