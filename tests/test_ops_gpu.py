@@ -1013,7 +1013,8 @@ def test_native_calls_leave_modes_and_subclasses_alone(ops):
 @pytest.mark.parametrize("captured", [False, True])
 def test_queued_operators_wait_for_one_another(ops, rng, n, c, hw, captured):
     """Each launch is prepared while the kernel before it runs: operators that read what the one before wrote, into memory that
-    the allocator has just taken from an earlier result, give what they give one by one."""
+    the allocator has just taken from an earlier result, give what they give one by one. (None of them lets the next one's blocks in before its end; a
+    wait that is missing shows in test_operators_wait_for_a_convolution_in_flight.)"""
     x, b = dev(rng.normal(size=(n, c, hw, hw)).astype(f32)), dev(rng.normal(size=21).astype(f32))
     w = dev(rng.normal(0, 0.01, (21, c)).astype(f32))  # (the softmax takes exp of the values themselves: at most 16 |x| * 64 |w| < 88)
 
@@ -1078,3 +1079,114 @@ def test_filters_that_a_kernel_in_flight_writes(ops, rng):
             wait()
     assert ops.device_status() == 0 and len({bytes(e.cpu().numpy()) for e in expected}) == len(biases)
     assert all(torch.equal(g, e) for g, e in zip(got, expected))
+
+
+def operators_behind_a_convolution(ops, rng):
+    """Operators of one pass over memory, by the kernel they take, as functions of a large fp32 result: they read its end, which is written last."""
+    u = lambda *shape: dev(rng.uniform(-1, 1, shape).astype(f32))
+
+    def end(t, *shape, before=0):  # (16-byte aligned where the elements from its start to the result's end are a multiple of four)
+        flat, n = t.view(-1), int(np.prod(shape))
+        return flat[flat.numel() - n - before:flat.numel() - before].view(shape)
+
+    square, odd = (16, 64, 32, 32), (16, 63, 31, 33)
+    b, res, w, wt, filters = u(1, 64, 1, 32), u(16, 64, 16, 16), u(512, 512), u(40, 300), u(24, 64, 3, 3)
+    pool = ((3, 3), (2, 2), (1, 1, 1, 1))
+    return {
+        "relu": lambda t: ops.nn_relu(end(t, *square)), "relu, ragged": lambda t: ops.nn_relu(end(t, 100001, before=3)),
+        "add": lambda t: ops.add(end(t, *square), end(t, *square), relu=True), "add, broadcast": lambda t: ops.add(end(t, *square), b),
+        "copy": lambda t: ops.nn_flatten(end(t, 16, 64, 8, 8)), "copy, ragged": lambda t: ops.nn_flatten(end(t, 7, 3, 9, 11)),
+        "max pool": lambda t: ops.nn_max_pool2d(end(t, *square), *pool), "max pool, ragged": lambda t: ops.nn_max_pool2d(end(t, *odd), *pool),
+        "max pool, any": lambda t: ops.nn_max_pool2d(end(t, *square), (2, 2), (1, 1)), "avg pool": lambda t: ops.nn_avg_pool2d(end(t, *square), (2, 2), (1, 1)),
+        "pool, add, relu": lambda t: ops.max_pool2d_add_relu(end(t, *square), res, *pool),
+        "mean of planes, odd": lambda t: ops.nn_global_avg_pool2d(end(t, 16, 64, 7, 7)), "mean of planes": lambda t: ops.nn_global_avg_pool2d(end(t, 16, 64, 8, 8)),
+        "mean of planes, large": lambda t: ops.nn_global_avg_pool2d(end(t, 4, 2, 300, 300)), "mean": lambda t: ops.reduce_mean(end(t, *square), [1], keepdims=False),
+        "softmax 300": lambda t: ops.softmax(end(t, 64, 300)), "softmax 1000": lambda t: ops.softmax(end(t, 64, 1000)),
+        "softmax 4000": lambda t: ops.softmax(end(t, 64, 4000)), "softmax 9000": lambda t: ops.softmax(end(t, 64, 9000)),
+        "transpose": lambda t: ops.transpose(end(t, *square), (0, 2, 3, 1)), "transpose, ragged": lambda t: ops.transpose(end(t, *odd), (0, 2, 3, 1)),
+        "transpose, rows": lambda t: ops.transpose(end(t, *square), (1, 0, 2, 3)), "cast": lambda t: ops.cast(end(t, *square), torch.float64),
+        "cast, ragged": lambda t: ops.cast(end(t, 100003), torch.float64), "dense fp32": lambda t: ops.nn_dense(end(t, 96, 512), w, precision="fp32"),
+        "matrix product fp32": lambda t: ops.matmul(end(t, 96, 512), w, precision="fp32"), "dense tf32": lambda t: ops.nn_dense(end(t, 8, 300), wt),
+        "dense bf16": lambda t: ops.nn_dense(end(t, 700, 512), w, precision="bf16"), "dense tf32x3": lambda t: ops.nn_dense(end(t, 700, 512), w, precision="tf32x3"),
+        "convolution fp32": lambda t: ops.nn_conv2d(end(t, *square), filters, None, (1, 1), (1, 1), precision="fp32"),
+        "convolution fp32, dilated": lambda t: ops.nn_conv2d(end(t, 4, 64, 32, 32), filters, None, (2, 1), (2, 2), (2, 2), precision="fp32"),
+        "convolution tf32": lambda t: ops.nn_conv2d(end(t, *square), filters, None, (1, 1), (1, 1), precision="tf32"),
+    }
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_operators_wait_for_a_convolution_in_flight(ops, rng, captured):
+    """A convolution lets the launch behind it start when it starts itself: operators that read its result, of which nothing is left from another run, wait
+    for it; one that writes where it reads its residual too."""
+    x, w = dev(rng.uniform(-1, 1, (64, 64, 56, 56)).astype(f32)), dev(rng.normal(0, 0.05, (64, 64, 3, 3)).astype(f32))
+    result, held = torch.empty(64, 64, 56, 56, device="cuda"), dev(rng.uniform(-1, 1, (64, 64, 56, 56)).astype(f32))
+    residual = held.clone()
+
+    def convolve():
+        residual.copy_(held)
+        result.fill_(float("nan"))
+        return ops.nn_conv2d(x, w, None, (1, 1), (1, 1), residual=residual, precision="bf16", out=result)
+
+    expected = convolve().clone()
+    overwritten = residual.view(-1)[-64 * 64 * 14 * 14:].view(64, 64, 14, 14)  # (the end of the residual, which the convolution reads last)
+    small, added = dev(rng.uniform(-1, 1, (64, 64, 28, 28)).astype(f32)), dev(rng.uniform(-1, 1, (64, 64, 14, 14)).astype(f32))
+    calls = operators_behind_a_convolution(ops, rng)
+    calls["into its residual"] = lambda t: (ops.max_pool2d_add_relu(small, added, (3, 3), (2, 2), (1, 1, 1, 1), out=overwritten), t)[1]
+    for name, call in calls.items():
+        torch.cuda.synchronize()
+        want = call(expected)
+        torch.cuda.synchronize()
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                got = call(convolve())
+            graph.replay()
+        else:
+            got = call(convolve())
+        torch.cuda.synchronize()
+        assert torch.equal(got, want), name
+    assert ops.device_status() == 0
+
+
+def test_captured_branches_join_in_operators(ops, rng):
+    """Two convolutions and two poolings on streams of their own, captured: the sum where they join, and what forks behind it, read finished results."""
+    x = [dev(rng.uniform(-1, 1, (n, 64, 56, 56)).astype(f32)) for n in (32, 32)]
+    w = [dev(rng.normal(0, 0.05, (64, 64, 3, 3)).astype(f32)) for _ in range(2)]
+    y = [torch.empty(32, 64, 56, 56, device="cuda") for _ in range(2)]
+    side = torch.cuda.Stream()
+
+    def run(fork, join):
+        outs = [None, None]
+        for t in y:
+            t.fill_(float("nan"))
+        fork()
+        ops.nn_conv2d(x[0], w[0], None, (1, 1), (1, 1), precision="bf16", out=y[0])
+        with torch.cuda.stream(side):
+            ops.nn_conv2d(x[1], w[1], None, (1, 1), (1, 1), precision="tf32", out=y[1])
+        join()
+        total = ops.add(y[0], y[1], relu=True)
+        fork()
+        outs[0] = ops.nn_max_pool2d(total, (3, 3), (2, 2), (1, 1, 1, 1))
+        with torch.cuda.stream(side):
+            outs[1] = ops.transpose(total, (0, 2, 3, 1))
+        join()
+        return outs + [ops.add(ops.nn_max_pool2d(ops.transpose(outs[1], (0, 3, 1, 2)), (3, 3), (2, 2), (1, 1, 1, 1)), outs[0])]
+
+    def settle():
+        torch.cuda.synchronize()
+
+    expected = run(settle, settle)
+    settle()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        main = torch.cuda.current_stream()
+        got = run(lambda: side.wait_stream(main), lambda: main.wait_stream(side))
+    for _ in range(3):
+        for t in got:
+            t.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(g, e) for g, e in zip(got, expected))
+    got = run(lambda: side.wait_stream(torch.cuda.current_stream()), lambda: torch.cuda.current_stream().wait_stream(side))
+    settle()
+    assert all(torch.equal(g, e) for g, e in zip(got, expected)) and ops.device_status() == 0
