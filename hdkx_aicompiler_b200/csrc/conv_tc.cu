@@ -203,13 +203,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                             for (int t = 0; t < kMT; ++t)
                                 tma_load_4d_pair(a_dst + t * G::kATileBytes, &p.tmA[map], full0, cb * p.kb_elems, ow0[t] + cw,
                                                  oh0[t] + ch, n0[t]);
-                            if constexpr (kX3) {
+                            if constexpr (kX3)
                                 tma_load_4d_pair(a_dst + G::kATileBytes, &p.tmA[map], full0, cb * p.kb_elems, ow0[0] + cw, oh0[0] + ch, n0[0] + p.N);
-                                tma_load_2d_pair(a_dst + G::kABytes, &p.tmB, full0, kb * p.kb_elems, co0);
-                                tma_load_2d_pair(a_dst + G::kABytes + G::kBTileBytes, &p.tmB2, full0, kb * p.kb_elems, co0);
-                            } else {
-                                tma_load_2d_pair(a_dst + G::kABytes, &p.tmB, full0, kb * p.kb_elems, co0);
-                            }
+                            tma_load_2d_pair(a_dst + G::kABytes, &p.tmB, full0, kb * p.kb_elems, co0);
+                            if constexpr (kX3) tma_load_2d_pair(a_dst + G::kABytes + G::kBTileBytes, &p.tmB2, full0, kb * p.kb_elems, co0);
                         } else {
                             mbar_arrive_expect_tx(full, tx_bytes);
 #pragma unroll
@@ -294,16 +291,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) conv_igemm_kernel(const __grid_
                                 }
                             } else {
 #pragma unroll
-                            for (int t = 0; t < kMT; ++t) {
-                                // advancing 32 bytes along K inside the swizzle span = +2 in the (addr >> 4) field;
-                                // the next pixel tile of the stage is kATileBytes further on
-                                const uint64_t a_k = a_desc + (uint64_t)(2 * k) + (uint64_t)(t * (G::kATileBytes >> 4));
-                                const uint32_t d_t = d_tmem + (uint32_t)(t * BN);
-                                if constexpr (kPair)
-                                    umma_pair<kKind>(d_t, a_k, b_desc + (uint64_t)(2 * k), kIdesc, (kb_local | k) != 0 ? 1u : 0u);
-                                else
-                                    umma<kKind>(d_t, a_k, b_desc + (uint64_t)(2 * k), kIdesc, (kb_local | k) != 0 ? 1u : 0u);
-                            }
+                                for (int t = 0; t < kMT; ++t) {
+                                    // advancing 32 bytes along K inside the swizzle span = +2 in the (addr >> 4) field;
+                                    // the next pixel tile of the stage is kATileBytes further on
+                                    const uint64_t a_k = a_desc + (uint64_t)(2 * k) + (uint64_t)(t * (G::kATileBytes >> 4));
+                                    const uint32_t d_t = d_tmem + (uint32_t)(t * BN);
+                                    if constexpr (kPair)
+                                        umma_pair<kKind>(d_t, a_k, b_desc + (uint64_t)(2 * k), kIdesc, (kb_local | k) != 0 ? 1u : 0u);
+                                    else
+                                        umma<kKind>(d_t, a_k, b_desc + (uint64_t)(2 * k), kIdesc, (kb_local | k) != 0 ? 1u : 0u);
+                                }
                             }
                         }
                         if constexpr (kPair) umma_commit_pair(smem_u32(&bar_empty[stage]), 3);

@@ -98,7 +98,6 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) maxpool_nhwc_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int H,
                                                                 int W, int C, int OH, int OW, int KH, int KW, int SH, int SW,
                                                                 int PT, int PL, int64_t parts) {
-    sm100::pdl_wait();
     constexpr int L = Vec<T>::kLanes;
     const int cg = C / L;
     const int64_t total = (int64_t)N * OH * OW * cg;
@@ -137,7 +136,6 @@ __global__ void __launch_bounds__(kThreads) maxpool_nhwc_kernel(const T* __restr
 template <typename T>
 __global__ void __launch_bounds__(kThreads) maxpool3x3s2p1_nhwc_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int H,
                                                                        int W, int C, int OH, int OW, int64_t parts) {
-    sm100::pdl_wait();
     constexpr int L = Vec<T>::kLanes;
     const int cg = C / L, ow2n = OW / 2, oh2n = OH / 2;
     const int64_t total = (int64_t)N * oh2n * ow2n * cg;
@@ -251,7 +249,6 @@ __global__ void __launch_bounds__(kThreads) gap_nhwc_split_kernel(const T* __res
 template <typename T>
 __global__ void __launch_bounds__(kThreads) eltwise_nhwc_kernel(const T* __restrict__ a, const T* __restrict__ b,
                                                                 T* __restrict__ out, int64_t nvec, int relu, int64_t parts) {
-    sm100::pdl_wait();
     constexpr int L = Vec<T>::kLanes;
     for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < nvec; i += (int64_t)gridDim.x * kThreads) {
         float va[L];
