@@ -70,6 +70,8 @@ inline int64_t pool_out_dim(int64_t in, int64_t k, int64_t s, int64_t p0, int64_
 // the shared memory of the pool before them: 13.1, and 72x802x5x5 20.9 for 16.4.
 // KXC_B200_PDL=0 in the environment launches everything fully serialized.
 bool pdl_enabled();
+// The calling thread's next launch_kernel waits for the end of the kernel before it, whatever its caller asks for.
+inline thread_local bool next_launch_in_order = false;
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl,
                                  int cluster_x, Args&&... args) {
@@ -83,7 +85,9 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
         attr[n].val.clusterDim.z = 1;
         ++n;
     }
-    if (pdl && pdl_enabled()) {
+    const bool in_order = next_launch_in_order;
+    next_launch_in_order = false;
+    if (pdl && !in_order && pdl_enabled()) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n].val.programmaticStreamSerializationAllowed = 1;
         ++n;

@@ -1105,8 +1105,6 @@ static int64_t split_parts(kxc_b200_plan* pl, int id) {
     return pl->x3 && v->split ? (int64_t)v->elems : 0;
 }
 
-__global__ void weights_packed_kernel() {}
-
 static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream, cudaEvent_t* events) {
     if (!pl || !pl->finalized) return fail(KXC_B200_ERR_INVALID, "plan_run: plan is not finalized");
     if (pl->precision == KXC_B200_PREC_FP32) return run_exact(pl, packed_args, stream, events);
@@ -1147,12 +1145,9 @@ static int32_t plan_run_core(kxc_b200_plan* pl, void** packed_args, void* stream
         }
         w.source = src;
     }
-    // The steps read packed weights ahead of their waits. A step behind the last packing kernel could start with that one's blocks gone and what they
-    // wrote not yet visible; an empty kernel launched in order ends after all of it.
-    if (packed) {
-        weights_packed_kernel<<<1, 32, 0, s>>>();
-        KXC_TRY(check_launch("weights_packed"));
-    }
+    // The steps read packed weights ahead of their waits. The first one could start with the last packing kernel's blocks gone and what they wrote not
+    // yet visible, and the others with it: it is launched in order. (An empty kernel between them took 3 us of a first pass.)
+    next_launch_in_order = packed;
 
     // Tensor-core launches alternate the direction in which they walk their work items (KXC_B200_TILE_ORDER=0: all
     // forward): a launch then begins with the images its producer finished last, whose lines are still in L2.
