@@ -782,8 +782,9 @@ bool box_cost(const CmGeometry& g, const Grouping& t, int staging, int ctas, int
     int groups = 0;
     for (int l = 0; l < t.loads; ++l) groups += div_up((l + 1 < t.loads ? t.first[l + 1] : t.taps) - t.first[l], b->group);
     const long long items = tiles(g, BW, BH, BNI, ctas);
-    // What a tile costs: its rows at the rate the copies reach shared memory, or its instructions, 64 + n / 2 clocks each (a fit), and the hand-over of a
-    // group; then its epilogue, which overlaps the next tile. (Boxes chosen so over 200 drawn layers.)
+    // What a tile costs: its rows at the rate the copies reach shared memory, or its instructions, 64 + n / 2 clocks each, and the hand-over of a
+    // group; then its epilogue, which overlaps the next tile. (Boxes chosen so over 200 drawn layers. A fit of the loops of one lane: the boxes of single CTAs, and the
+    // lines of cm_wanted but that of the pairs, still go by it.)
     const double fill = (double)g.cblocks * ((double)t.loads * rows_px + (double)t.taps * rows_w) * 2.6;
     const double mma = (double)t.taps * ((g.cblocks - 1) * 4 + g.last_steps) * (64.0 + 0.5 * b->n);
     const double main_loop = (fill > mma ? fill : mma) + 100.0 * g.cblocks * groups;

@@ -943,9 +943,13 @@ bool split_fits(long long tiles, int s, long long* late) {
 // Whether a set-up launch (tile width, store form and so on already chosen for the persistent kernel) is better off with its
 // reduction split over a cluster, and the set-up of that form: the cheaper of the two in modelled cycles, the split one 5 % ahead.
 // The figures are fits over 320 launches timed in every form that fits the chip (7 layers in a row, NHWC, and one layer
-// into NCHW; 16 to 144 K blocks; 1 to 96 images), in clocks of 1.9 GHz:
+// into NCHW; 16 to 144 K blocks; 1 to 96 images), in clocks of 1.9 GHz, and older than the loops of whole warps, which take 400 to 490 clocks a block at 64
+// and 128 channels in either form (tc_modelled_clocks below, which only the choice of CTA pairs uses): this model splits from 14 K blocks on in two parts of one
+// wave, that one from 18 to 24. Which is right there has not been timed:
 //   a K block of 128 bytes per row     550 / 590 / 500 / 620 at 64 / 128 / 192 / 256 channels, 650 at 256 in the split kernel;
-//                                      760 with two bf16 pixel tiles, 820 / 1100 with two tf32 ones; three passes 830 / 1050, split 830 / 930
+//                                      760 with two bf16 pixel tiles, 820 / 1100 with two tf32 ones; three passes 830 / 1050, split 830 / 930, pairs
+//                                      660 (of the loops of whole warps: 148 launches that pairs took over were 1.11 times as fast with them in
+//                                      the mean, 0.94 to 1.8, the 22 that would be split 1.18, 0.98 to 1.8)
 //   what follows the last K block      unsplit 0 / 2000 / 4000 / 8000 (the epilogue of that many channels), 2800 more with two pixel
 //                                      tiles; split 3000 / 5500 / 10000 (the exchange of the partial sums over distributed shared
 //                                      memory and the epilogue, which grow with the width; refitted over 170 layers when the
@@ -1152,8 +1156,8 @@ int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_m
     // CTA pairs (tcgen05 cta_group::2): each CTA fetches half of the B tile, which relieves the L2 -> shared-memory
     // fill rate that bounds the wide tiles.
     const long long m_tiles = (long long)p->tiles_w * p->tiles_h * p->tiles_n;
-    // Measured: pairs gain 5-7 % with the 256-wide tile and lose 3-10 % with the 128-wide one (the pair's MMA is
-    // no faster there and the handshakes cross SMs), so only the 256-wide tile uses them. "2" forces them for 128 too.
+    // Measured: pairs gain 5-7 % with the 256-wide tile, so that one uses them. With the 128-wide one they lost 3-10 % when one lane issued and
+    // are level since (ResNet-18 bf16, 1024 images 3322 us, with them 3328; 64 to 256 level). "2" forces them for 128 too.
     static const bool pair_all = [] { const char* e = getenv("KXC_B200_CTA_PAIR"); return e != nullptr && e[0] == '2'; }();
     int ctas = (tc_cta_pairs() && bn >= (pair_all ? 128 : 256) && kb_bytes == 128 && m_tiles >= 2) ? 2 : 1;
     // Launches with few tiles (small per-GPU batches in the deep layers): the 256-wide tile leaves SMs idle, e.g. 98 tiles
@@ -1190,8 +1194,9 @@ int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_m
     cfg->mt = (mt_enabled && bn == 128 && dtype == kTcBF16 && out_mode == kOutNHWC_BF16 && kb_bytes == 128 && m_tiles >= 2 * ctas) ? 2 : 1;
     // tf32 and int8: the tiles of such a launch reach shared memory at 7 to 8 TB/s over all SMs whatever the MMAs do, and two
     // pixel tiles against one weight tile are 20 / 24 KB per tile instead of 24 / 32 (64 / 128 channels). Taken when the
-    // modelled makespan gains: a stage of two tiles costs 820 / 1100 cycles against 490 / 655. ResNet-18 tf32, 32 images: layer 1 42 -> 34 us per convolution, layer 2 31 -> 30; int8 128 -> 128,
-    // 28x28, 256 images: 52 -> 46.
+    // modelled makespan gains: a stage of two tiles cost 820 / 1100 cycles against 490 / 655 when one lane issued (a whole warp: 703 / 791 against 405 / 427,
+    // tc_modelled_clocks; not fitted again). ResNet-18 tf32, 32 images: layer 1 42 -> 34 us per convolution, layer 2 31 -> 30; int8 128 -> 128, 28x28, 256
+    // images: 52 -> 46.
     if (mt_enabled && ctas == 1 && kb_bytes == 128 &&
         ((dtype == kTcTF32 && (bn == 64 || bn == 128)) || (dtype == kTcS8 && bn == 128 && out_mode == kOutNHWC_S8))) {
         const long long tc = (Cout + bn - 1) / bn;
@@ -1235,8 +1240,8 @@ int32_t tc_setup_conv(TcParams* p, TcConfig* cfg, TcDType dtype, TcOutMode out_m
 }
 
 int32_t tc_finish_x3(TcParams* p, TcConfig* cfg, const void* w_hi, const void* w_lo, int Cout, int k_elems) {
-    // The tile whose waves cost least. Single CTAs: by 950 cycles a stage with 64 channels and 1400 with 128; pairs of 64 channels
-    // where by what the forms measured (660, and 760 / 1030 for single ones, over ResNet-18's layers of 1 to 64 images) they are ahead. 250 launches of
+    // The tile whose waves cost least. Single CTAs: by 950 cycles a stage with 64 channels and 1400 with 128 (of the loops of one lane, not fitted again); pairs
+    // of 64 channels where by what the forms measured since (660, and 760 / 1030 for single ones, over ResNet-18's layers of 1 to 64 images) they are ahead. 250 launches of
     // 150 drawn layers (operators and plans, 1 to 64 images, 32 to 512 channels): pairs took 62, 1.09 times as fast in the mean, 0.98 to 1.30 (a
     // 64 -> 128 3x3 at 80x79, one image, before it was split in two). Fewer than 12 K blocks lose up to 10 % (the stem 73 / 78 us), 1x1 layers were 0.94 to 1.04 times as fast. Pairs of 128 channels
     // have one accumulator buffer and were level or behind (28x28, 32 images 45 / 52).

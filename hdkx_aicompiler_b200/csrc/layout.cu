@@ -98,8 +98,8 @@ __device__ __forceinline__ void pack_weights_block(const TIn* __restrict__ w, TO
 //
 // Programmatic launch on both sides: the blocks wait for the previous kernel before they touch memory, and with `overlap` then
 // let the next kernel's CTAs set themselves up. Weights packed here are not TcParams::weights_ready for the kernel after it (it
-// waits before it reads them); those of a plan come from launches before this one, which have ended by the time its blocks let
-// go. A launch that packs a plan's weights does not let go early: the kernel after the next may read them ahead.
+// waits before it reads them); those of a plan have been packed before its first step begins. A launch that packs a plan's weights does not let go
+// early: the kernel after the next may read them ahead.
 //
 // kSub: only the pixels that a 1x1 convolution of stride `st` without padding reads, so that it runs with stride 1 over a quarter of the
 // pixels: rows it skips are never touched, and a quarter is written (67 -> 56 at 91x94, 60 images, bf16: 102 -> 49 us a call).

@@ -183,8 +183,9 @@ __device__ __forceinline__ bool named_barrier_or(int id, int count, bool pred) {
 
 // One lane of the (converged) warp, the same one every time. The loops that issue copies and MMAs run on a whole warp: the warp's number comes from
 // a shuffle, waits end in a vote, and only the instructions themselves are the elected lane's. Their operands are uniform registers. In a branch of
-// one lane (lane == 0) the compiler cannot tell that a value is uniform and moves every operand there first: 130 to 170 clocks an MMA in the
-// loops of conv_chmajor.cu, 70 to 100 so (tf32 256 -> 256 3x3 at 14x14, 32 images, a launch 23.5 -> 20.0 us).
+// one lane (lane == 0) the compiler cannot tell that a value is uniform and moves every operand there first. Four MMAs of N = 64 and the hand-over of
+// their stage, in a loop alone: 480 clocks so, 283 by a whole warp; in the launches of conv_chmajor.cu 130 to 170 clocks an MMA, 70 to 100 now
+// (tf32 256 -> 256 3x3 at 14x14, 32 images, a launch 23.5 -> 20.0 us).
 __device__ __forceinline__ bool elect_one() {
     uint32_t is;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
